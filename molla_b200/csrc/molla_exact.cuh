@@ -121,7 +121,6 @@ __device__ __forceinline__ void block_argmax(CX &c, float &v, int &i) {
 
 // bitonic sort, descending, of n2 (power of two) keys in shared memory
 __device__ void bitonic_desc(unsigned long long *k, int n2, int tid) {
-    IN_SHARED(k);
     // A warp's 32 consecutive pair indices cover 64 consecutive keys whenever the stride is at
     // most 16, the same 64 for every such stride: those stages only need the warp to agree.
     bool local = false;  // the previous stage was such a stage

@@ -1,0 +1,1825 @@
+// The ordinary entry points' path: a batch of logit rows through four small kernels.
+//
+//   tile_stats   every tile of 1024 logits: its maximum, where it lies, and an estimate of the tile's
+//                sum of exponentials                                     (reads the block from HBM)
+//   row_plan     every row: the maximum, the answer of greedy rows, an estimate of the running softmax
+//                sum before every tile, what is too small to matter there, and a value that the
+//                `need` largest elements reach
+//   tile_exp     every tile again (from L2 where the block fits it): the exponentials of what can
+//                matter, the head's candidates, and a short program ("items") that says how the exact
+//                sequential sum goes through the tile
+//   row_finish   every row: one thread runs the items, which gives the exact softmax denominator, then
+//                the sorted head, the filters and the draw, or the walks past the head over the list
+//                of exponentials
+//
+// A tile belongs to one warp and no warp waits for another (except around bias and penalty patches),
+// so any number of rows, from one to thousands, fills the chip, and nothing but the last kernel has
+// a serial part. The reference's sequential fp32 sums are reproduced bit for bit: see "Items" below.
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stddef.h>
+#include <stdint.h>
+#include <stdio.h>
+
+#include "molla_exact.cuh"
+#include "molla_rows.h"
+
+namespace {
+
+constexpr int TILE = 1024;                 // logits of a tile: 32 per lane, consecutive
+constexpr int PITCH = 36;                  // words per lane in shared memory: float4 accesses without bank conflicts
+constexpr int SPAN_THREADS = 256;          // a block of the tile kernels: eight warps, eight tiles
+constexpr int SPAN = SPAN_THREADS * 32;    // logits per block
+constexpr int MAX_TILES = 704;             // V <= 720896
+constexpr int ITEMS_PER_TILE = 66;         // a run and a careful chunk per lane at most, and one more run
+constexpr int HEADCAP = 2048;              // candidates of the sorted head at most
+constexpr int HEAD_MOST = 1026;            // the sorted head covers top-k + 1 up to this many
+constexpr int ITEM_CAP = 512;              // items of a row that fit shared memory
+constexpr int CARE_CAP = 64;               // careful chunks whose entries are fetched ahead
+constexpr int TIE_CAP = 64;                // rounding ties a walk resolves by parity; more send it the slow way
+constexpr int PLAN_GROUPS = 300 * 32;      // group maxima row_plan looks at, at most
+
+enum { PLAN_DONE = 0, PLAN_SAMPLED = 1 };
+enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8 };
+
+struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
+struct __align__(8) TilePlan { float thr, est; };
+struct __align__(16) TileOut { unsigned int emax; float esum; unsigned short cnt, nitem; unsigned int pad; };
+struct __align__(16) RowPlan { int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; int pad; };
+
+// Items: the exact sequential sum of a tile's values as a short program. While the running sum s
+// stays in one binade, fl(s + v) is s plus rne(v / ulp) units, an integer that does not depend on s;
+// in the bit pattern of s, adding k units is the integer addition of k. So a run of lanes whose
+// values all round by themselves is one number (kind RUN). A lane near the end of a binade carries
+// the numbers of both binades (DUAL); a lane with a rounding tie, a value of a quarter of the sum or
+// a guess that spans more is added value by value (STEP). The binades are guessed from the estimated
+// sum before the tile; whoever runs the items checks every guess against the exact sum and adds the
+// values one by one where it was wrong.
+enum { K_RUN = 0, K_DUAL = 1, K_STEP = 2 };
+struct __align__(16) Item {
+    unsigned int ka, kb;   // units of binade jb (RUN, DUAL) and of the next one (DUAL)
+    unsigned int meta;     // biased exponent of the binade (8 bits), kind (2 bits)
+    unsigned int oc;       // first entry in the tile's list << 16 | entries
+};
+
+struct RowsArgs {
+    BatchArgs a;
+    int r0, rows;            // batch rows [r0, r0 + rows) are in flight
+    int ntile, nspan, glog;  // glog: log2 of the lanes whose maxima row_plan joins
+    int oG, oVc, oL;         // see F_NARROW
+    TileStat *ts;            // [rows][ntile]
+    float *gmax;             // [rows][ntile * 32] the lanes' maxima
+    TilePlan *tp;            // [rows][ntile]
+    RowPlan *plan;           // [rows]
+    int *ncand;              // [rows]
+    unsigned long long *cand;  // [rows][HEADCAP]
+    TileOut *to;             // [rows][ntile]
+    Item *items;             // [rows][ntile][ITEMS_PER_TILE]
+    float *elist;            // [rows][ntile][TILE] values kept, in vocabulary order, packed per tile
+    unsigned int *kmask;     // [rows][ntile][32] which logits they are
+};
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---- settings ---------------------------------------------------------------------------------
+struct RowCfg {
+    int q; long long lrow;
+    float T, P, minp, typ, rp, fp, pp;
+    int k, ring_n, H, b0, nb, npatch;
+    const long long *histp;
+    long long n_lim;
+    bool greedy, topp_on, pure, open_row;
+    unsigned int status;
+};
+
+// Where row r's settings live and what they are; status bits for a row that cannot be sampled
+// (the rules of SamplerConfig.check, sample.mojo:140-154; NaN fails every test).
+__device__ __forceinline__ RowCfg row_cfg(const BatchArgs &a, int r) {
+    RowCfg c;
+    c.status = 0;
+    c.q = a.slot ? a.slot[r] : r;
+    c.lrow = a.rows ? (long long)a.rows[r] : (long long)r;
+    const bool idx_ok = (!a.slot || (c.q >= 0 && (a.n_slots <= 0 || c.q < a.n_slots))) &&
+                        (!a.rows || (c.lrow >= 0 && (a.n_logit_rows <= 0 || c.lrow < a.n_logit_rows)));
+    const int q = idx_ok ? c.q : 0;   // a stale row or slot index: nothing of that row or slot is touched
+    if (!idx_ok) {
+        c.T = 0; c.P = 1; c.minp = 0; c.typ = 1; c.rp = 1; c.fp = c.pp = 0; c.k = 0; c.ring_n = c.H = c.b0 = c.nb = c.npatch = 0;
+        c.histp = nullptr; c.n_lim = a.V; c.greedy = true; c.topp_on = c.pure = c.open_row = false;
+        c.status = MOLLA_ROW_INVALID_CONFIG | 0x80000000u;
+        return c;
+    }
+    c.T = a.temperature ? a.temperature[q] : 0.0f;
+    c.k = a.top_k ? a.top_k[q] : 0;
+    c.P = a.top_p ? a.top_p[q] : 1.0f;
+    c.minp = a.min_p ? a.min_p[q] : 0.0f;
+    c.typ = a.typical_p ? a.typical_p[q] : 1.0f;
+    c.rp = a.repeat_penalty ? a.repeat_penalty[q] : 1.0f;
+    c.fp = a.frequency_penalty ? a.frequency_penalty[q] : 0.0f;
+    c.pp = a.presence_penalty ? a.presence_penalty[q] : 0.0f;
+    c.ring_n = a.ring ? min(max(a.ring_len[q], 0), a.ring_cap) : 0;
+    const bool won = a.ring ? (c.ring_n > 0) : (a.window_on ? (a.window_on[q] != 0) : true);
+    const int h0 = (a.hist && a.hist_off) ? a.hist_off[q] : 0;
+    // a window kept on the device fills from its first slot (sample.mojo:246-258): the first
+    // `filled` entries are the window, whatever the head is
+    c.histp = a.ring ? a.ring + (size_t)q * (size_t)a.ring_cap : (a.hist ? a.hist + h0 : nullptr);
+    c.H = a.ring ? min(max(a.ring_filled[q], 0), c.ring_n) : ((a.hist && a.hist_off) ? (a.hist_off[q + 1] - h0) : 0);
+    c.b0 = (a.bias_ids && a.bias_off) ? a.bias_off[q] : 0;
+    c.nb = (a.bias_ids && a.bias_off) ? (a.bias_off[q + 1] - c.b0) : 0;
+    const bool valid = (c.T >= 0.0f) && (c.k >= 0) && (c.P > 0.0f && c.P <= 1.0f) && (c.minp >= 0.0f && c.minp <= 1.0f) &&
+                       (c.typ > 0.0f && c.typ <= 1.0f) && (c.rp > 0.0f) && c.H >= 0 && c.nb >= 0;
+    c.greedy = !(c.T > 0.0f);
+    const bool penalizing = won && c.H > 0 && (c.rp != 1.0f || c.fp != 0.0f || c.pp != 0.0f);
+    c.npatch = (penalizing ? c.H : 0) + c.nb;
+    if (!valid) c.status |= MOLLA_ROW_INVALID_CONFIG;
+    // typical-p is done on rows an earlier filter sorted and cut to a set inside the sorted head
+    else if (!c.greedy && c.typ < 1.0f && !((c.k > 0 && c.k < a.V) || c.P < 1.0f)) c.status |= MOLLA_ROW_UNSUPPORTED;
+    if (c.npatch > PATCH_MAX) c.status |= MOLLA_ROW_UNSUPPORTED;
+    c.n_lim = (c.k > 0 && c.k < a.V) ? (long long)c.k : (long long)a.V;
+    c.open_row = c.n_lim == (long long)a.V;
+    c.topp_on = c.P < 1.0f && c.n_lim > 1;
+    c.pure = !c.topp_on && c.open_row;
+    return c;
+}
+
+// The end of every row, one thread: the answer, then `_took` (sample.mojo:361-363).
+__device__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
+                           float dtarget, float dp) {
+    if (status & 0x80000000u) {  // a stale index
+        a.tokens[r] = -1; a.row_status[r] = status & 0x7fffffffu;
+        return;
+    }
+    if (status & (MOLLA_ROW_LOAD_TIMEOUT | MOLLA_ROW_DEGENERATE | MOLLA_ROW_INVALID_CONFIG | MOLLA_ROW_UNSUPPORTED | MOLLA_ROW_EMPTY)) token = -1;
+    a.tokens[r] = token;
+    a.row_status[r] = status;
+    if (a.ring && token >= 0) {
+        const int q = c.q;
+        if (c.ring_n > 0) {  // `observe` (:246-258)
+            const int hd = a.ring_head[q];
+            const int at = (hd >= 0 && hd < c.ring_n) ? hd : 0;
+            a.ring[(size_t)q * (size_t)a.ring_cap + at] = (long long)token;
+            a.ring_head[q] = (at + 1) % c.ring_n;
+            const int f = a.ring_filled[q];
+            a.ring_filled[q] = f < c.ring_n ? f + 1 : c.ring_n;
+        }
+        a.drawn_rw[q] += 1ull;
+        if (a.stopped) a.stopped[r] = (a.stop_token && a.stop_token[q] == (long long)token) ? 1 : 0;
+    }
+    if (a.diag) { a.diag[4 * r] = dZ; a.diag[4 * r + 1] = dsum; a.diag[4 * r + 2] = dtarget; a.diag[4 * r + 3] = dp; }
+}
+
+// ---- arithmetic -------------------------------------------------------------------------------
+// x / d, correctly rounded, for many x and one d: two steps of the division by a reciprocal with
+// fused multiply-adds of Markstein (IBM J. Res. Dev. 34, 1990): with y = RN(1/d) the first step is
+// within an ulp, its remainder is exact, and the second step rounds correctly. Five operations in
+// place of a division's own sequence. Holds while nothing under- or overflows on the way: the
+// callers see to that (F_FASTDIV).
+__device__ __forceinline__ float div_by(float x, float d, float y) {
+    const float q0 = __fmul_rn(x, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-q0, d, x), y, q0);
+    return __fmaf_rn(__fmaf_rn(-q1, d, x), y, q1);
+}
+// a probability e / Z (Z between 1 and the vocabulary's size; e in [0, 1])
+__device__ __forceinline__ float prob_of(float e, float Z, float y) {
+    return e > 1.0e-20f ? div_by(e, Z, y) : __fdiv_rn(e, Z);
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float warp_max_key(float v) { return fkey_inv(__reduce_max_sync(0xffffffffu, fkey(v))); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// ---- a span of a row in shared memory -----------------------------------------------------------
+__device__ __forceinline__ void cp16(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp4(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+struct SpanScratch {
+    unsigned int cnt[SPAN / 2];         // per logit 16 bits: times in the window, top bit: named by a bias
+    unsigned short hits[PATCH_MAX];     // the patched logits of the span
+    int nhits;
+};
+
+// Logits [c0, c0 + SPAN) of row r, capped, masked, biased and penalised, to `sx`: lane l of tile w
+// finds its 32 at sx[(32 w + l) * PITCH]. What lies past the row's end is -inf. Threads
+// 0..SPAN_THREADS-1 work (`active`), all threads of the block take part in the barriers; each warp
+// may then use its own tile. 16-byte asynchronous copies where the row starts on such a boundary,
+// 4-byte ones elsewhere.
+__device__ void load_span(const BatchArgs &a, const RowCfg &c, int r, int c0, float *sx, SpanScratch *s, bool active) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float *src = a.logits + c.lrow * a.row_stride + c0;
+    const int n = min(SPAN, a.V - c0);
+    const int e0 = warp * TILE;
+    float *mine = sx + (size_t)tid * PITCH;
+    if (active) {
+        if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int ch = i * 32 + lane, e = e0 + ch * 4;
+                float *dst = sx + (warp * 32 + (ch >> 3)) * PITCH + (ch & 7) * 4;
+                if (e + 4 <= n) cp16(dst, src + e);
+                else {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) dst[u] = (e + u < n) ? __ldg(src + e + u) : -INFINITY;
+                }
+            }
+        } else {
+#pragma unroll 8
+            for (int i = 0; i < 32; i++) {
+                const int e = e0 + i * 32 + lane;
+                float *dst = sx + (warp * 32 + i) * PITCH + lane;
+                if (e < n) cp4(dst, src + e);
+                else *dst = -INFINITY;
+            }
+        }
+    }
+    const bool patching = c.npatch > 0;
+    if (patching) {
+        if (active) {
+            uint4 *z = reinterpret_cast<uint4 *>(s->cnt);
+#pragma unroll
+            for (int i = 0; i < SPAN / 8 / SPAN_THREADS; i++) z[tid + i * SPAN_THREADS] = make_uint4(0, 0, 0, 0);
+            if (tid == 0) s->nhits = 0;
+        }
+        __syncthreads();
+        if (active)
+            for (int i = tid; i < c.npatch; i += SPAN_THREADS) {
+                const bool is_bias = i < c.nb;
+                const long long t64 = (is_bias ? a.bias_ids[c.b0 + i] : c.histp[i - c.nb]) - (long long)c0;
+                if (t64 < 0 || t64 >= n) continue;
+                const int t = (int)t64, sh = (t & 1) * 16;
+                const unsigned int old = is_bias ? atomicOr(&s->cnt[t >> 1], 0x8000u << sh) : atomicAdd(&s->cnt[t >> 1], 1u << sh);
+                if (((old >> sh) & 0xffffu) == 0u) s->hits[satom_add(&s->nhits, 1)] = (unsigned short)t;
+            }
+        __syncthreads();
+    }
+    if (active) {
+        cp_wait();
+        __syncwarp();
+        const int m = n - (e0 + lane * 32);  // this lane's logits that exist
+        if (a.softcap > 0.0f) {
+            for (int j = 0; j < min(32, m); j++) mine[j] = softcap_pinned(mine[j], a.softcap);
+            __syncwarp();
+        }
+        if (a.mask && m > 0) {
+            // `_mask` (sample.mojo:371-379): what the grammar forbids is no candidate at all. A logit of
+            // -inf is exactly that here: it wins no maximum, no bias or penalty brings it back, its
+            // exponential is zero, and zeros are absent from every sum, count and walk.
+            const unsigned int w = __ldg(a.mask + (long long)r * a.mask_stride + ((c0 + e0 + lane * 32) >> 5));
+#pragma unroll
+            for (int g = 0; g < 8; g++) {
+                float4 x = *reinterpret_cast<float4 *>(mine + 4 * g);
+                if (!((w >> (4 * g)) & 1u)) x.x = -INFINITY;
+                if (!((w >> (4 * g + 1)) & 1u)) x.y = -INFINITY;
+                if (!((w >> (4 * g + 2)) & 1u)) x.z = -INFINITY;
+                if (!((w >> (4 * g + 3)) & 1u)) x.w = -INFINITY;
+                *reinterpret_cast<float4 *>(mine + 4 * g) = x;
+            }
+        }
+    }
+    if (patching) {
+        __syncthreads();
+        if (active) {
+            const int nh = s->nhits;
+            for (int i = tid; i < nh; i += SPAN_THREADS) {
+                const int t = s->hits[i];
+                const int nw = (int)((s->cnt[t >> 1] >> ((t & 1) * 16)) & 0x7fffu);
+                float v = sx[(t >> 5) * PITCH + (t & 31)];
+                for (int b = 0; b < c.nb; b++)  // duplicates add up, in the order they were given
+                    if (a.bias_ids[c.b0 + b] == (long long)t + c0) v = __fadd_rn(v, a.bias_vals[c.b0 + b]);
+                if (nw > 0) {
+                    if (v > 0.0f) v = __fdiv_rn(v, c.rp);
+                    else v = __fmul_rn(v, c.rp);
+                    v = __fsub_rn(v, __fmul_rn((float)nw, c.fp));
+                    v = __fsub_rn(v, c.pp);
+                }
+                sx[(t >> 5) * PITCH + (t & 31)] = v;
+            }
+        }
+        __syncthreads();
+    } else {
+        __syncwarp();
+    }
+}
+
+// =============================================================================
+// Kernel 1: the tiles' maxima and estimated sums. Bound: HBM (4 bytes per logit, once).
+// =============================================================================
+struct SpanShared {
+    float x[SPAN_THREADS * PITCH];
+    SpanScratch s;
+};
+
+__global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __grid_constant__ RowsArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SpanShared *S = reinterpret_cast<SpanShared *>(smem_raw);
+    pdl_next();
+    pdl_wait();
+    const int rr = blockIdx.x / A.nspan, span = blockIdx.x - rr * A.nspan, r = A.r0 + rr;
+    const BatchArgs &a = A.a;
+    const RowCfg c = row_cfg(a, r);
+    if (c.status) return;
+    load_span(a, c, r, span * SPAN, S->x, &S->s, true);
+    const int lane = threadIdx.x & 31, tile = span * (SPAN / TILE) + (threadIdx.x >> 5);
+    if (tile >= A.ntile) return;
+    const float *mine = S->x + threadIdx.x * PITCH;
+    float x[32];
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+        const float4 v = *reinterpret_cast<const float4 *>(mine + 4 * g);
+        x[4 * g] = v.x; x[4 * g + 1] = v.y; x[4 * g + 2] = v.z; x[4 * g + 3] = v.w;
+    }
+    float m = x[0];
+#pragma unroll
+    for (int j = 1; j < 32; j++) m = fmaxf(m, x[j]);
+    const float tmax = warp_max_key(m);
+    const unsigned int who = __ballot_sync(0xffffffffu, m == tmax);
+    const int first = who ? __ffs((int)who) - 1 : 0;
+    int at = 0;
+    if (lane == first) {
+#pragma unroll
+        for (int j = 31; j >= 0; j--)
+            if (x[j] == tmax) at = j;
+    }
+    at = __shfl_sync(0xffffffffu, at, first) + first * 32 + tile * TILE;
+    const bool sampled = !c.greedy && c.n_lim > 1;
+    int eq = 0;
+    float sum = 0.0f;
+    if (sampled) {
+        // an estimate is enough (it only guesses binades and bounds what is dropped): hardware exponentials
+        if (tmax > -INFINITY) {
+            const float f = fminf(1.44269504f / c.T, 1.0e30f);
+            float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+                s0 += ex2_approx((x[j] - tmax) * f);
+                s1 += ex2_approx((x[j + 1] - tmax) * f);
+            }
+            sum = warp_sum(s0 + s1);
+        }
+        if (!c.pure) A.gmax[((size_t)rr * A.ntile + tile) * 32 + lane] = m;
+    } else if (!c.greedy) {  // only a top-k of one asks how many share the maximum
+#pragma unroll
+        for (int j = 0; j < 32; j++) eq += x[j] == tmax ? 1 : 0;
+        eq = __reduce_add_sync(0xffffffffu, eq);
+    }
+    if (lane == 0) {
+        TileStat t;
+        t.tmax = tmax; t.tsum = sum; t.tidx = at; t.teq = eq;
+        A.ts[(size_t)rr * A.ntile + tile] = t;
+    }
+}
+
+// =============================================================================
+// Kernel 2: one block per row.
+// =============================================================================
+struct PlanShared {
+    float g[PLAN_GROUPS];
+    float wsf[NWARP + 1];
+    int wsi[NWARP + 1];
+};
+
+// Exclusive scan over the block without a subtraction (the terms span many orders of magnitude).
+__device__ __forceinline__ float block_excl_scan_plus(float v, float *ws, float *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float inc = warp_incl_scan(v, lane);
+    float ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) ex = 0.0f;
+    __syncthreads();
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    float b = 0.0f, t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < NWARP; w++) {
+        if (w == warp) b = t;
+        t += ws[w];
+    }
+    *total = t;
+    return b + ex;
+}
+
+__global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ RowsArgs A) {
+    __shared__ PlanShared S;
+    pdl_next();
+    const int rr = blockIdx.x, r = A.r0 + rr, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const BatchArgs &a = A.a;
+    pdl_wait();
+    RowCfg c = row_cfg(a, r);
+    if (MOLLA_KNOB(a, 16) && !c.status) c.status |= MOLLA_ROW_LOAD_TIMEOUT;  // testing build: a wait that ran out
+    RowPlan pl;
+    pl.kind = PLAN_DONE; pl.flags = 0; pl.top = 0; pl.tau_bits = 1u; pl.xmax = 0; pl.imax = 0; pl.need = 0; pl.pad = 0;
+    if (c.status) {
+        if (tid == 0) { finish_row(a, r, c, c.status, -1, 0, 0, 0, 0); A.plan[rr] = pl; }
+        return;
+    }
+    // the maximum and its first index (kernel.mojo:571-585, sample.mojo:342-346)
+    const TileStat *ts = A.ts + (size_t)rr * A.ntile;
+    float tm[2], tsum[2], xmax = -INFINITY;
+    int te[2], imax = 0x7fffffff;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int t = 2 * tid + u;
+        TileStat s;
+        s.tmax = -INFINITY; s.tsum = 0.0f; s.tidx = 0x7fffffff; s.teq = 0;
+        if (t < A.ntile) s = ts[t];
+        tm[u] = s.tmax; tsum[u] = s.tsum; te[u] = s.teq;
+        if (s.tmax > xmax) { xmax = s.tmax; imax = s.tidx; }
+    }
+    warp_argmax(xmax, imax);
+    if (lane == 0) { S.wsf[warp] = xmax; S.wsi[warp] = imax; }
+    __syncthreads();
+    xmax = S.wsf[0]; imax = S.wsi[0];
+#pragma unroll
+    for (int w = 1; w < NWARP; w++)
+        if (S.wsf[w] > xmax || (S.wsf[w] == xmax && S.wsi[w] < imax)) { xmax = S.wsf[w]; imax = S.wsi[w]; }
+    if (imax == 0x7fffffff) imax = 0;
+    unsigned int status = 0;
+    bool done = c.greedy || c.n_lim == 1;
+    if (a.mask && !(xmax > -INFINITY)) { status |= MOLLA_ROW_EMPTY; done = true; }  // every candidate was filtered out
+    else if (!c.greedy && c.n_lim == 1) {
+        // top-k of one: the sort's first element is a maximum (sample.mojo:485-490)
+        int eq = 0;
+#pragma unroll
+        for (int u = 0; u < 2; u++) eq += tm[u] == xmax ? te[u] : 0;
+        eq = __reduce_add_sync(0xffffffffu, eq);
+        __syncthreads();
+        if (lane == 0) S.wsi[warp] = eq;
+        __syncthreads();
+        eq = 0;
+        for (int w = 0; w < NWARP; w++) eq += S.wsi[w];
+        if (eq > 1) status |= MOLLA_ROW_TOPK_TIE;
+    }
+    if (done) {
+        if (tid == 0) { finish_row(a, r, c, status, imax, 0, 0, 0, 0); A.plan[rr] = pl; }
+        return;
+    }
+    const float top = (c.T == 1.0f) ? xmax : __fdiv_rn(xmax, c.T);
+    const bool filter_ok = fabsf(top) < 1.0e5f;
+    long long need = c.open_row ? (long long)HEAD_NEED : c.n_lim + 1;
+    if (need > HEAD_MOST) need = HEAD_MOST;
+    if (need > a.V) need = a.V;
+    // estimated sum before every tile, relative to the row's maximum
+    const float f = fminf(1.44269504f / c.T, 1.0e30f);
+    float e[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) e[u] = (tm[u] > -INFINITY) ? tsum[u] * ex2_approx((tm[u] - xmax) * f) : 0.0f;
+    float total;
+    const float ex = block_excl_scan_plus(e[0] + e[1], S.wsf, &total);
+    const float est[2] = {ex, ex + e[0]};
+    // A logit below half an ulp of the running sum adds nothing to it, whatever order: 17.6 is above
+    // 25 ln 2, the tenth taken off the estimate covers what rounding loses. Below top - 105 the
+    // exponential is exactly zero.
+    const float thr_zero = filter_ok ? c.T * (top - 105.0f) : -INFINITY;
+    auto thr_of = [&](float s) -> float {
+        const float rel = (filter_ok && s > 0.0f) ? c.T * (top + logf(0.9f * s) - REL_MARGIN) : -INFINITY;
+        return fmaxf(rel, thr_zero);
+    };
+    // The head: a value that at least `need` of the lanes' maxima reach bounds the need-th largest
+    // element from below, and few more elements than that reach it.
+    float tau_x = INFINITY;
+    bool narrow = false;
+    if (!c.pure) {
+        const int gl = A.glog, ng = (A.ntile * 32) >> gl;
+        const float *gm = A.gmax + (size_t)rr * A.ntile * 32;
+        for (int i = tid; i < ng; i += NT) {
+            float v = gm[i << gl];
+            for (int u = 1; u < (1 << gl); u++) v = fmaxf(v, gm[(i << gl) + u]);
+            S.g[i] = v;
+        }
+        __syncthreads();
+        auto count = [&](float t) -> int {
+            int n = 0;
+            for (int i = tid; i < ng; i += NT) n += S.g[i] >= t ? 1 : 0;
+            n = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0) S.wsi[warp] = n;
+            __syncthreads();
+            n = 0;
+#pragma unroll
+            for (int w = 0; w < NWARP; w++) n += S.wsi[w];
+            __syncthreads();
+            return n;
+        };
+        float lo = xmax - 32.0f, hi = xmax;
+        tau_x = -INFINITY;
+        if (fabsf(xmax) < 65536.0f && count(lo) >= need) {
+            const int enough = (int)need + (int)need / 32;
+            for (int it = 0; it < 24; it++) {
+                const float mid = 0.5f * (lo + hi);
+                if (!(mid > lo) || !(mid < hi)) break;
+                const int n = count(mid);
+                if (n >= need) { lo = mid; if (n <= enough) break; } else hi = mid;
+            }
+            tau_x = lo;
+        }
+        // F_NARROW: a top-k so wide for the vocabulary that fewer ranges than candidates exist (one range
+        // per thread of the widest layout: oG blocks of NT threads with oL logits each). Such rows report
+        // the order of equal probabilities the way the descending walk sees it.
+        if (need > HEAD_NEED && A.oG > 0) {
+            int have = 0, allowed = 0;
+            for (int i = tid; i < A.oG * NT; i += NT) {
+                const int g = i / NT, l0 = (i - g * NT) * A.oL, n_g = max(0, min(A.oVc, a.V - g * A.oVc));
+                if (l0 >= n_g) continue;
+                int bits = min(A.oL, n_g - l0);
+                if (a.mask) {
+                    const unsigned int *mrow = a.mask + (long long)r * a.mask_stride;
+                    int b = 0;
+                    for (int j = 0; j < bits; j++) { const int t = g * A.oVc + l0 + j; b += (__ldg(mrow + (t >> 5)) >> (t & 31)) & 1u; }
+                    bits = b;
+                }
+                have += bits > 0 ? 1 : 0;
+                allowed += bits;
+            }
+            have = __reduce_add_sync(0xffffffffu, have);
+            allowed = __reduce_add_sync(0xffffffffu, allowed);
+            if (lane == 0) { S.wsi[warp] = have; S.wsf[warp] = __int_as_float(allowed); }
+            __syncthreads();
+            have = allowed = 0;
+            for (int w = 0; w < NWARP; w++) { have += S.wsi[w]; allowed += __float_as_int(S.wsf[w]); }
+            narrow = have < need && allowed > HEADCAP;
+            __syncthreads();
+        }
+    }
+    const float tv = (c.T == 1.0f) ? tau_x : __fdiv_rn(tau_x, c.T);
+    const unsigned int tb = c.pure ? 0xffffffffu : __float_as_uint(expf_pinned(__fsub_rn(tv, top)));
+    TilePlan *tp = A.tp + (size_t)rr * A.ntile;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int t = 2 * tid + u;
+        if (t < A.ntile) { TilePlan p; p.thr = fminf(thr_of(est[u]), tau_x); p.est = est[u]; tp[t] = p; }
+    }
+    if (tid == 0) {
+        pl.kind = PLAN_SAMPLED;
+        const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
+        // (too few lanes to bound the head: row_finish narrows it down from the list)
+        pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) |
+                   ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
+        pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
+        pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
+        A.plan[rr] = pl;
+        A.ncand[rr] = 0;
+    }
+}
+
+// =============================================================================
+// Kernel 3: exponentials, candidates, items.
+// =============================================================================
+// The items of a tile whose lane `lane` holds `cnt` values v(0..cnt-1) (padded with zeros to a multiple
+// of four), estimated sum before the tile `est`. `off` = the lane's first entry in the tile's list.
+// Returns the number of items; `care` = this lane's values are wanted one by one.
+__device__ __forceinline__ int tile_items(const float *row, int cnt, int off, int total, float csum, float est, Item *out, bool &care) {
+    const int lane = threadIdx.x & 31;
+    const float inc = warp_incl_scan(csum, lane);
+    float ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) ex = 0.0f;
+    const float sst = est + ex;
+    const bool nonempty = cnt > 0 && csum > 0.0f;
+    // the estimate counts what was dropped (it adds nothing to the true sum), so it is high rather than low
+    const float lo = sst * (1.0f - 1.0f / 512.0f), hi = (sst + csum) * (1.0f + 1.0f / 2048.0f);
+    const int jl = fexpo(lo), jh = fexpo(hi);
+    const bool usable = nonempty && lo > 0.0f && jh <= jl + 1 && jl >= -100 && jh <= 100;
+    const bool two = usable && jh == jl + 1;
+    bool bad = false;
+    float da = 0.0f, db = 0.0f;
+    if (__any_sync(0xffffffffu, two)) {
+        if (usable) {
+            const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
+            const float C2 = __fmul_rn(1.5f, fpow2(jl + 1)), h2 = fpow2(jl - 23);
+            for (int i = 0; i < cnt; i += 4) {
+                const float4 v4 = *reinterpret_cast<const float4 *>(row + i);
+                const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const float q = __fsub_rn(__fadd_rn(v[u], C1), C1);
+                    bad |= (fabsf(__fsub_rn(v[u], q)) == h1) | (v[u] >= b1);
+                    da = __fadd_rn(da, q);
+                    const float q2 = __fsub_rn(__fadd_rn(v[u], C2), C2);
+                    bad |= two & (fabsf(__fsub_rn(v[u], q2)) == h2);
+                    db = __fadd_rn(db, q2);
+                }
+            }
+        }
+    } else if (usable) {
+        const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
+        float d1 = 0.0f;
+        for (int i = 0; i < cnt; i += 4) {
+            const float4 v4 = *reinterpret_cast<const float4 *>(row + i);
+            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float q = __fsub_rn(__fadd_rn(v[u], C1), C1);
+                bad |= (fabsf(__fsub_rn(v[u], q)) == h1) | (v[u] >= b1);
+                if (u & 1) d1 = __fadd_rn(d1, q); else da = __fadd_rn(da, q);
+            }
+        }
+        da = __fadd_rn(da, d1);
+    }
+    const bool step = nonempty && (!usable || bad);
+    const unsigned int ne = __ballot_sync(0xffffffffu, nonempty);
+    // lanes that round by themselves inside one binade form runs; two neighbours that disagree about
+    // the binade do not belong to one run
+    const unsigned int below = ne & ((1u << lane) - 1u);
+    const int prev = below ? 31 - __clz((int)below) : lane;
+    const int pj = __shfl_sync(0xffffffffu, jl, prev);
+    const bool prev_alone = ((__ballot_sync(0xffffffffu, step || two) >> prev) & 1u) != 0u;
+    care = step || two || (nonempty && below && !prev_alone && pj != jl);
+    const unsigned int cm = __ballot_sync(0xffffffffu, care);
+    const float units = fpow2(max(min(23 - jl, 127), -126));
+    const unsigned int ka = (usable && !bad) ? __float2uint_rn(__fmul_rn(da, units)) : 0u;   // da is a multiple of 2^(jl-23), below 2^24 of them
+    if (cm == 0u) {
+        const unsigned int k = __reduce_add_sync(0xffffffffu, ka);
+        if (k == 0u) return 0;
+        const int j0 = __shfl_sync(0xffffffffu, jl, __ffs((int)ne) - 1);
+        if (lane == 0) {
+            Item it;
+            it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8); it.oc = (unsigned int)total;
+            out[0] = it;
+        }
+        return 1;
+    }
+    int n = 0;
+    unsigned int left = cm;
+    int from = 0;
+    for (int round = 0; round < 33; round++) {
+        const int cl = left ? __ffs((int)left) - 1 : 32;
+        const unsigned int span = (cl == 32 ? 0xffffffffu : ((1u << cl) - 1u)) & ~((from == 0) ? 0u : (from == 32 ? 0xffffffffu : ((1u << from) - 1u)));
+        const unsigned int in = span & ne;
+        if (in) {
+            const unsigned int k = __reduce_add_sync(0xffffffffu, ((in >> lane) & 1u) ? ka : 0u);
+            if (k) {
+                const int l0 = __ffs((int)in) - 1, l1 = 31 - __clz((int)in);
+                const int j0 = __shfl_sync(0xffffffffu, jl, l0), o0 = __shfl_sync(0xffffffffu, off, l0), o1 = __shfl_sync(0xffffffffu, off + cnt, l1);
+                if (lane == 0) {
+                    Item it;
+                    it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8); it.oc = ((unsigned int)o0 << 16) | (unsigned int)(o1 - o0);
+                    out[n] = it;
+                }
+                n++;
+            }
+        }
+        if (cl == 32) break;
+        if (lane == cl) {
+            Item it;
+            const bool dual = two && !bad;
+            it.ka = dual ? ka : 0u;
+            it.kb = dual ? __float2uint_rn(__fmul_rn(db, fpow2(max(min(22 - jl, 127), -126)))) : 0u;
+            it.meta = dual ? ((unsigned int)(jl + 127) | (K_DUAL << 8)) : (unsigned int)(K_STEP << 8);
+            it.oc = ((unsigned int)off << 16) | (unsigned int)cnt;
+            out[n] = it;
+        }
+        n++;
+        from = cl + 1;
+        left &= left - 1u;
+    }
+    return n;
+}
+
+struct TileEval { int cnt, off, total; unsigned int keep; float csum; unsigned int emax; };
+
+// The exponentials (temperature and softmax numerator, sample.mojo:419-434) of a tile's logits that
+// reach `thr`, packed to the front of every lane's own part of shared memory.
+template <class TAKE>
+__device__ __forceinline__ TileEval tile_eval(float *mine, float thr, float T, float rT, float top, bool fast, TAKE take) {
+    const int lane = threadIdx.x & 31;
+    unsigned int m = 0;
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+        const float4 v = *reinterpret_cast<const float4 *>(mine + 4 * g);
+        m |= (v.x >= thr ? 1u : 0u) << (4 * g) | (v.y >= thr ? 1u : 0u) << (4 * g + 1) | (v.z >= thr ? 1u : 0u) << (4 * g + 2) | (v.w >= thr ? 1u : 0u) << (4 * g + 3);
+    }
+    TileEval r;
+    r.cnt = 0; r.keep = 0; r.csum = 0.0f; r.emax = 0;
+    const bool one = T == 1.0f;
+    for (int round = 0; round < 32 && __any_sync(0xffffffffu, m != 0u); round++) {
+        if (m) {
+            const int b = __ffs((int)m) - 1;
+            m &= m - 1u;
+            const float x = mine[b];
+            const float v = one ? x : (fast ? div_by(x, T, rT) : __fdiv_rn(x, T));
+            const float e = expf_pinned_nonpos(__fsub_rn(v, top));  // no logit of the row exceeds its maximum
+            if (e > 0.0f) {
+                mine[r.cnt] = e;
+                r.cnt++;
+                r.csum += e;
+                r.keep |= 1u << b;
+                const unsigned int eb = __float_as_uint(e);
+                r.emax = max(r.emax, eb);
+                take(eb, lane * 32 + b);
+            }
+        }
+    }
+    for (int i = r.cnt; i < ((r.cnt + 3) & ~3); i++) mine[i] = 0.0f;
+    const int inc = warp_incl_scan(r.cnt, lane);
+    r.off = inc - r.cnt;
+    r.total = __shfl_sync(0xffffffffu, inc, 31);
+    __syncwarp();
+    return r;
+}
+
+// A tile's packed values to its place in the list: dense lanes are written by the whole warp.
+__device__ __forceinline__ void tile_store(const float *tile_rows, const TileEval &t, float *dst, unsigned int lanes) {
+    const int lane = threadIdx.x & 31;
+    const float *mine = tile_rows + lane * PITCH;
+    const bool wide = __reduce_max_sync(0xffffffffu, (unsigned int)t.cnt) > 6u;
+    if (!wide) {
+        if ((lanes >> lane) & 1u)
+            for (int i = 0; i < t.cnt; i++) dst[t.off + i] = mine[i];
+        return;
+    }
+    unsigned int left = __ballot_sync(0xffffffffu, t.cnt > 0) & lanes;
+    while (left) {
+        const int l = __ffs((int)left) - 1;
+        left &= left - 1u;
+        const int n = __shfl_sync(0xffffffffu, t.cnt, l), o = __shfl_sync(0xffffffffu, t.off, l);
+        if (lane < n) dst[o + lane] = tile_rows[l * PITCH + lane];
+    }
+}
+
+__global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_constant__ RowsArgs A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SpanShared *S = reinterpret_cast<SpanShared *>(smem_raw);
+    pdl_next();
+    pdl_wait();
+    const int rr = blockIdx.x / A.nspan, span = blockIdx.x - rr * A.nspan, r = A.r0 + rr;
+    const RowPlan pl = A.plan[rr];
+    if (pl.kind == PLAN_DONE) return;
+    const BatchArgs &a = A.a;
+    const RowCfg c = row_cfg(a, r);
+    load_span(a, c, r, span * SPAN, S->x, &S->s, true);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
+    if (tile >= A.ntile) return;
+    const size_t gt = (size_t)rr * A.ntile + tile;
+    const TilePlan tp = A.tp[gt];
+    float *mine = S->x + threadIdx.x * PITCH;
+    const unsigned int tau = pl.tau_bits;
+    unsigned long long *cand = A.cand + (size_t)rr * HEADCAP;
+    const TileEval t = tile_eval(mine, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
+        [&](unsigned int eb, int i) {
+            if (eb >= tau) {
+                const int pos = atomicAdd(&A.ncand[rr], 1);
+                if (pos < HEADCAP) cand[pos] = make_key(eb, tile * TILE + i);
+            }
+        });
+    bool care;
+    const int ni = tile_items(mine, t.cnt, t.off, t.total, t.csum, tp.est, A.items + gt * ITEMS_PER_TILE, care);
+    const unsigned int lanes = (pl.flags & F_LIST) ? 0xffffffffu : __ballot_sync(0xffffffffu, care);
+    if (lanes) tile_store(S->x + (size_t)warp * 32 * PITCH, t, A.elist + gt * TILE, lanes);
+    if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = t.keep;
+    const float esum = warp_sum(t.csum);
+    const unsigned int emax = __reduce_max_sync(0xffffffffu, t.emax);
+    if (lane == 0) {
+        TileOut o;
+        o.emax = emax; o.esum = esum; o.cnt = (unsigned short)t.total; o.nitem = (unsigned short)ni; o.pad = 0;
+        A.to[gt] = o;
+    }
+}
+
+// =============================================================================
+// Kernel 4: one block per sampled row.
+// =============================================================================
+struct __align__(16) AuxF {
+    union {
+        float tile[NWARP * 32 * PITCH];    // tiles being worked on, one per warp (a span and its scratch use the same space)
+        struct {
+            union {
+                struct { unsigned int hq[NBINS], hqh[NBINS], hc[NBINS]; } h;
+            } u;
+            unsigned long long cand[NC];   // the head's, then a bin's candidates
+            unsigned long long tmp[NC];
+            float pc[NC];
+            float pre[HEADCAP];
+            unsigned int hidx[HEADCAP];
+        };
+    };
+    Item items[ITEM_CAP + 1];
+    unsigned int isrc[ITEM_CAP];           // tile << 8 | slot of the fetched entries (255: none)
+    float care[CARE_CAP * 32];
+    unsigned short careidx[CARE_CAP];
+    float ebuf[TILE];
+    unsigned short tcnt[MAX_TILES];        // entries in the tile's list
+    unsigned short tni[MAX_TILES];         // items of the tile
+    int toff[MAX_TILES + 1];               // first item of the tile
+    float tsum[MAX_TILES];
+    double wsd[2 * (NWARP + 1)];
+    unsigned long long wsu[NWARP + 1];
+    float wsf[NWARP + 1];
+    int wsi[NWARP + 1];
+    int ncand, ncare, evt_thread, specbin, hit_bin;
+    unsigned long long hit_qbefore, hit_cbefore, tot_q, tot_c;
+    float b_s; int b_event; int b_idx; float b_p; long long b_pos; int b_aux;
+    float b_sum, b_target;
+    unsigned int w_sb; int w_i, w_need, w_found, w_tile, w_at;   // the items' runner
+    int ntie; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP];
+    unsigned long long tpqm[TIE_CAP], tabove[TIE_CAP], tc[TIE_CAP];
+    unsigned int tbits[NBINS / 32];
+};
+static_assert(sizeof(SpanScratch) + (size_t)SPAN_THREADS * PITCH * 4 <= sizeof(float) * NWARP * 32 * PITCH, "a span and its scratch fit the tiles' space");
+
+struct CtxF {
+    int tid, lane, warp;
+    AuxF *A;
+    unsigned int status;
+    const RowsArgs *R;
+    int rr, r;
+    RowCfg cfg;
+    RowPlan pl;
+    float *list;                 // this row's [ntile][TILE]
+    Item *gitems;                // this row's [ntile][ITEMS_PER_TILE]
+    const unsigned int *kmask;   // this row's [ntile][32]
+};
+
+// One entry of the list, as a token id: the nth logit its tile kept.
+__device__ int token_of(const CtxF &c, int tile, int nth) {
+    const uint4 *m = reinterpret_cast<const uint4 *>(c.kmask + (size_t)tile * 32);
+    int at = 0;
+    uint4 w[8];
+#pragma unroll
+    for (int g = 0; g < 8; g++) w[g] = m[g];
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+        const unsigned int v[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int n = __popc(v[u]);
+            if (nth >= at && nth < at + n) return tile * TILE + (4 * g + u) * 32 + (int)__fns(v[u], 0, nth - at + 1);
+            at += n;
+        }
+    }
+    return tile * TILE;
+}
+__device__ __forceinline__ int token_of(const CtxF &c, int pos) { return token_of(c, pos >> 10, pos & (TILE - 1)); }
+
+// Tile `t` evaluated again, as kernel 3 did it: by warp t % 8, its values packed into dst.
+__device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    const RowsArgs &R = *c.R;
+    const int span = t0 / (SPAN / TILE);
+    SpanScratch *s = reinterpret_cast<SpanScratch *>(A->tile + SPAN_THREADS * PITCH);
+    __syncthreads();
+    load_span(R.a, c.cfg, c.r, span * SPAN, A->tile, s, c.tid < SPAN_THREADS);
+    const int t = span * (SPAN / TILE) + c.warp;
+    if (c.warp < SPAN / TILE && t >= t0 && t < t1) {
+        const float thr = R.tp[(size_t)c.rr * R.ntile + t].thr;
+        const TileEval e = tile_eval(A->tile + (size_t)c.tid * PITCH, thr, c.cfg.T, __fdiv_rn(1.0f, c.cfg.T), c.pl.top,
+                                     (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, int) {});
+        tile_store(A->tile + (size_t)c.warp * 32 * PITCH, e, to_list ? c.list + (size_t)t * TILE : dst, 0xffffffffu);
+        if (to_list) const_cast<unsigned int *>(c.kmask)[(size_t)t * 32 + c.lane] = e.keep;
+    }
+    __syncthreads();
+}
+
+// v[0..n) added one by one to the sum with bit pattern A->w_sb (thread 0). With `locate`, stops at the
+// first value behind which the sum exceeds `target`.
+__device__ __forceinline__ void run_values(AuxF *A, unsigned int &sb, const float *v, int n, int off, int tile, bool locate, float target) {
+    float s = __uint_as_float(sb);
+    for (int i = 0; i < n; i += 8) {
+        float x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = i + u < n ? v[i + u] : 0.0f;   // (adding nothing changes nothing)
+        const float s0 = s;
+#pragma unroll
+        for (int u = 0; u < 8; u++) s = __fadd_rn(s, x[u]);
+        if (locate && target < s) {
+            s = s0;
+            for (int u = 0; u < 8; u++) {
+                s = __fadd_rn(s, v[i + u]);
+                if (target < s) { A->w_found = 1; A->w_tile = tile; A->w_at = off + i + u; break; }
+            }
+            break;
+        }
+    }
+    sb = __float_as_uint(s);
+}
+
+// Thread 0: the items of the batch in shared memory from A->w_i on. Ends with A->w_need = -1 (the batch
+// is through, or the target is found) or the item whose values are wanted.
+__device__ void run_items(AuxF *A, int n, bool locate, float target) {
+    IN_SHARED(A);
+    unsigned int sb = A->w_sb;
+    int i = A->w_found ? n : A->w_i;
+    A->w_need = -1;
+    Item nx = A->items[min(i, n)];
+    while (i < n) {
+        const Item it = nx;
+        nx = A->items[i + 1];
+        const unsigned int jb = it.meta & 0xffu, kind = it.meta >> 8, e = sb >> 23;
+        unsigned int to = sb + it.ka;
+        bool ok = kind != K_STEP && e == jb && (to >> 23) == jb;
+        if (kind == K_DUAL && e == jb + 1u) { to = sb + it.kb; ok = (to >> 23) == e; }
+        if (ok && !(locate && target < __uint_as_float(to))) { sb = to; i++; continue; }
+        const unsigned int src = A->isrc[i];
+        if ((src & 0xffu) == 255u) { A->w_need = i; break; }
+        run_values(A, sb, A->care + (src & 0xffu) * 32, (int)(it.oc & 0xffffu), (int)(it.oc >> 16), (int)(src >> 8), locate, target);
+        i++;
+        if (A->w_found) break;
+    }
+    A->w_sb = sb; A->w_i = i;
+}
+
+// The exact sequential fp32 sum over the row's items (A->tni of each tile in the row's item space).
+// Returns it; with `locate`, A->w_found says whether the running sum exceeded `target` and A->w_tile,
+// A->w_at at which list entry.
+__device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    const RowsArgs &R = *c.R;
+    __syncthreads();
+    int total;
+    {
+        const int t = 2 * c.tid;
+        const int n0 = t < R.ntile ? A->tni[t] : 0, n1 = t + 1 < R.ntile ? A->tni[t + 1] : 0;
+        const int ex = block_excl_scan<int>(n0 + n1, A->wsi, &total);
+        if (t < R.ntile) A->toff[t] = ex;
+        if (t + 1 < R.ntile) A->toff[t + 1] = ex + n0;
+    }
+    if (c.tid == 0) { A->w_sb = 0u; A->w_found = 0; A->w_tile = 0; A->w_at = 0; }
+    for (int b0 = 0; b0 < total; b0 += ITEM_CAP) {
+        const int n = min(ITEM_CAP, total - b0);
+        __syncthreads();
+        if (c.tid == 0) { A->ncare = 0; A->w_i = 0; }
+        for (int t = c.tid; t < R.ntile; t += NT) {
+            const int o = A->toff[t] - b0, m = A->tni[t];
+            for (int j = max(0, -o); j < m && o + j < n; j++) {
+                A->items[o + j] = c.gitems[(size_t)t * ITEMS_PER_TILE + j];
+                A->isrc[o + j] = ((unsigned int)t << 8) | 255u;
+            }
+        }
+        __syncthreads();
+        for (int i = c.tid; i < n; i += NT)
+            if ((A->items[i].meta >> 8) != K_RUN) {
+                const int s = satom_add(&A->ncare, 1);
+                if (s < CARE_CAP) { A->careidx[s] = (unsigned short)i; A->isrc[i] = (A->isrc[i] & ~0xffu) | (unsigned int)s; }
+            }
+        __syncthreads();
+        const int ncare = min(A->ncare, CARE_CAP);
+        for (int s = c.warp; s < ncare; s += NWARP) {
+            const int i = A->careidx[s];
+            const unsigned int oc = A->items[i].oc, t = A->isrc[i] >> 8;
+            if (c.lane < (int)(oc & 0xffffu)) A->care[s * 32 + c.lane] = c.list[(size_t)t * TILE + (oc >> 16) + c.lane];
+        }
+        for (int round = 0; round <= n; round++) {   // (each round but the last is for one more item)
+            __syncthreads();
+            if (c.tid == 0) run_items(A, n, locate, target);
+            __syncthreads();
+            const int want = A->w_need;
+            if (want < 0 || A->w_found) break;
+            // a run whose guess was wrong, or that holds the target: its values, one by one
+            const Item it = A->items[want];
+            const int t = (int)(A->isrc[want] >> 8), off = (int)(it.oc >> 16), m = (int)(it.oc & 0xffffu);
+            const float *v = A->ebuf;
+            if ((c.pl.flags & F_LIST) || (it.meta >> 8) != K_RUN) {
+                for (int i = c.tid; i < m; i += NT) A->ebuf[i] = c.list[(size_t)t * TILE + off + i];
+                __syncthreads();
+            } else {
+                tile_again(c, t, t + 1, A->ebuf, false);
+                v = A->ebuf + off;
+            }
+            if (c.tid == 0) {
+                unsigned int sb = A->w_sb;
+                run_values(A, sb, v, m, off, t, locate, target);
+                A->w_sb = sb; A->w_i = want + 1;
+            }
+        }
+        if (A->w_found) break;
+    }
+    __syncthreads();
+    return __uint_as_float(A->w_sb);
+}
+
+// Calls f(values, first position) for the row's list, four entries of a lane at a time (zero: none);
+// entry u of lane l is at first position + l + 32 u. All lanes of a warp make the same calls.
+template <class F>
+__device__ __forceinline__ void for_list4(const CtxF &c, F f) {
+    const AuxF *A = c.A;
+    IN_SHARED(A);
+    for (int t = c.warp; t < c.R->ntile; t += NWARP) {
+        const int n = A->tcnt[t];
+        float *src = c.list + (size_t)t * TILE;
+        for (int i0 = 0; i0 < n; i0 += 128) {
+            unsigned int eb[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) eb[u] = (i0 + u * 32 + c.lane < n) ? __float_as_uint(src[i0 + u * 32 + c.lane]) : 0u;
+            f(eb, t * TILE + i0, src + i0);
+        }
+    }
+}
+
+// More candidates than the head holds (few lanes for a wide top-k, or many equal values): a finer
+// edge from the values themselves. Returns the number of candidates written to `cand` and moves the
+// row's edge up, or a number above HEADCAP where one bin of values alone is too full.
+__device__ __noinline__ int narrow_head(CtxF &c, unsigned long long *cand) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    __syncthreads();
+    for (int i = c.tid; i < NBINS; i += NT) A->u.h.hc[i] = 0u;
+    if (c.tid == 0) { A->ncand = 0; A->evt_thread = -1; }
+    __syncthreads();
+    for_list4(c, [&](const unsigned int (&eb)[4], int, float *) {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (eb[u]) sred_add(&A->u.h.hc[eb[u] >> BIN_SHIFT], 1u);
+    });
+    __syncthreads();
+    int n[BPT], sum = 0, tot;
+#pragma unroll
+    for (int i = 0; i < BPT; i++) { n[i] = (int)A->u.h.hc[NBINS - 1 - BPT * c.tid - i]; sum += n[i]; }
+    int run = block_excl_scan<int>(sum, A->wsi, &tot);
+    const int need = min(c.pl.need, tot);
+#pragma unroll
+    for (int i = 0; i < BPT; i++) {
+        if (run < need && run + n[i] >= need) { A->evt_thread = NBINS - 1 - BPT * c.tid - i; A->b_idx = run + n[i]; }
+        run += n[i];
+    }
+    __syncthreads();
+    if (A->evt_thread < 0 || A->b_idx > HEADCAP) return HEADCAP + 1;
+    const unsigned int edge = (unsigned int)A->evt_thread << BIN_SHIFT;
+    c.pl.tau_bits = edge > 1u ? edge : 1u;
+    for (int t = c.warp; t < c.R->ntile; t += NWARP) {
+        unsigned int m = c.kmask[(size_t)t * 32 + c.lane];
+        const float *src = c.list + (size_t)t * TILE + (warp_incl_scan(__popc(m), c.lane) - __popc(m));
+        for (int i = 0; m; i++, m &= m - 1u) {
+            const unsigned int eb = __float_as_uint(src[i]);
+            if (eb >= c.pl.tau_bits) cand[satom_add(&A->ncand, 1)] = make_key(eb, t * TILE + c.lane * 32 + __ffs((int)m) - 1);
+        }
+    }
+    __syncthreads();
+    return A->ncand;
+}
+
+// The descending walk past the sorted head (sample.mojo:492-506 and :580-590) over the row's list of
+// probabilities. State: exact running sum, elements consumed, and tau: everything with probability
+// bits >= tau is consumed. Every phase histograms what remains by value bin, consumes whole bins up
+// to the first one holding an event, gathers that bin, sorts it and adds it element by element.
+//
+// An element whose addition would be a rounding tie (its value is an odd multiple of half the
+// running sum's unit) rounds up or down with the parity of the sum before it. Such elements do
+// not stop a phase: they are listed, a second pass adds up what precedes each of them inside
+// its own bin, and one thread then resolves them from the top down, each from the exact integer
+// sum before it; their contributions go into their bins' masses before the event is searched.
+struct FWalk {
+    float s; long long pos; unsigned int tau;
+    int event; int idx; float p; int tie;   // idx: position in the list, or (crowded) the same
+};
+// Where a walk's last phase began. The draw walk adds up the same elements in the same order as
+// the cut walk before it, so when its target is not reached before that point it starts there,
+// on the bin tables that are still standing, and skips the passes that built them.
+struct FResume {
+    int valid;
+    float s; long long pos; unsigned int tau;
+    int lvl; unsigned int lo; int shift; int tie_mode; int ntie;
+};
+
+// position of the (nth+1)-th entry, in vocabulary order, whose bits equal `eb`
+__device__ int list_nth_equal(CtxF &c, unsigned int eb, int nth) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    __syncthreads();
+    for (int t = c.warp; t < c.R->ntile; t += NWARP) {
+        int n = 0;
+        for (int i = c.lane; i < A->tcnt[t]; i += 32) n += __float_as_uint(c.list[(size_t)t * TILE + i]) == eb ? 1 : 0;
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (c.lane == 0) A->toff[t] = n;
+    }
+    __syncthreads();
+    if (c.tid == 0) {
+        int seen = 0, at = 0;
+        for (int t = 0; t < c.R->ntile; t++) {
+            if (nth < seen + A->toff[t]) {
+                for (int i = 0; i < A->tcnt[t]; i++)
+                    if (__float_as_uint(c.list[(size_t)t * TILE + i]) == eb && seen++ == nth) { at = t * TILE + i; break; }
+                break;
+            }
+            seen += A->toff[t];
+        }
+        A->b_idx = at;
+    }
+    __syncthreads();
+    return A->b_idx;
+}
+
+__device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long long nstop, FResume &rs, bool try_resume) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    const bool counting = nstop >= 0;
+    int lvl = 1;
+    unsigned int lo = 0u;
+    int shift = BIN_SHIFT;
+    bool tie_mode = true;
+    const bool resumed = try_resume && rs.valid && !counting && x_ge >= 3.0e38f && !(x_gt < rs.s);
+    if (resumed) {
+        w.s = rs.s; w.pos = rs.pos; w.tau = rs.tau;
+        lvl = rs.lvl; lo = rs.lo; shift = rs.shift; tie_mode = rs.tie_mode != 0;
+    }
+    for (int phase = 0; phase < 8192; phase++) {
+        const bool reuse = resumed && phase == 0;  // this phase's tables stand already
+        __syncthreads();
+        if (!reuse) {
+            for (int i = c.tid; i < NBINS; i += NT) { A->u.h.hq[i] = 0u; A->u.h.hqh[i] = 0u; A->u.h.hc[i] = 0u; }
+            for (int i = c.tid; i < NBINS / 32; i += NT) A->tbits[i] = 0u;
+            rs.valid = 1; rs.s = w.s; rs.pos = w.pos; rs.tau = w.tau;
+            rs.lvl = lvl; rs.lo = lo; rs.shift = shift; rs.tie_mode = tie_mode ? 1 : 0; rs.ntie = 0;
+        }
+        if (c.tid == 0) {
+            if (!reuse) A->specbin = -1;
+            A->ncand = 0; A->ntie = 0;
+        }
+        __syncthreads();
+        const bool have_s = w.s > 0.0f;
+        const int j = have_s ? fexpo(w.s) : 0;
+        const bool binade_ok = have_s && j >= -100 && j <= 100;
+        const float Cm = __fmul_rn(1.5f, fpow2(j)), halfu = fpow2(j - 24), bigthr = fpow2(j - 1);
+        const float inv_u = fpow2(23 - j);
+        const unsigned int cm_bits = __float_as_uint(Cm);
+        const bool ties_listed = tie_mode && lvl == 1 && binade_ok;
+        const unsigned int wtau = w.tau;
+        int ntie = rs.ntie;
+        if (!reuse) {
+            const bool count_all = counting || !binade_ok;
+            for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+                bool rare = false;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned int eb = ebs[u];
+                    const bool live = eb != 0u && eb < wtau && eb >= lo;
+                    const int bin = (int)((eb - lo) >> shift);
+                    const float p = __uint_as_float(eb);
+                    const float tq = __fadd_rn(p, Cm);
+                    const float rr = __fsub_rn(p, __fsub_rn(tq, Cm));
+                    const bool special = (fabsf(rr) == halfu) || (p >= bigthr);
+                    // below bigthr, p + Cm stays in Cm's binade, whose unit is the sum's: the difference
+                    // of the two bit patterns is the count of units
+                    const unsigned int qu = __float_as_uint(tq) - cm_bits;
+                    if (live && count_all) sred_add(&A->u.h.hc[bin], 1u);
+                    const bool plain = live && binade_ok && !special;
+                    if (plain && (qu & MASS_LO_MASK)) sred_add(&A->u.h.hq[bin], qu & MASS_LO_MASK);
+                    if (plain && (qu >> MASS_SPLIT)) sred_add(&A->u.h.hqh[bin], qu >> MASS_SPLIT);
+                    rare |= live && binade_ok && special;
+                }
+                if (__any_sync(0xffffffffu, rare)) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const unsigned int eb = ebs[u];
+                        if (!(eb != 0u && eb < wtau && eb >= lo)) continue;
+                        const int bin = (int)((eb - lo) >> shift);
+                        const float p = __uint_as_float(eb);
+                        const float q = __fsub_rn(__fadd_rn(p, Cm), Cm);
+                        const bool tie = fabsf(__fsub_rn(p, q)) == halfu;
+                        if ((p >= bigthr) || (tie && !ties_listed)) { sred_max(&A->specbin, bin); continue; }
+                        if (tie) {
+                            const int pos = satom_add(&A->ntie, 1);
+                            if (pos < TIE_CAP) { A->tkey[pos] = make_key(eb, pos0 + c.lane + 32 * u); A->tbin[pos] = bin; }
+                        }
+                    }
+                }
+            });
+            __syncthreads();
+            ntie = ties_listed ? A->ntie : 0;
+            rs.ntie = ntie;
+            if (ntie > TIE_CAP) { tie_mode = false; c.status |= MOLLA_ROW_SLOW_PATH; continue; }  // too many: they stop phases instead
+            if (ntie > 0) {
+                // what precedes each listed element inside its own bin (descending value, then ascending id)
+                if (c.tid < ntie) {
+                    const int b = A->tbin[c.tid];
+                    A->tpq_lo[c.tid] = 0u; A->tpq_hi[c.tid] = 0u;
+                    sred_or(&A->tbits[b >> 5], 1u << (b & 31));
+                }
+                __syncthreads();
+                int tb_lo = NBINS, tb_hi = -1;
+                for (int t = 0; t < ntie; t++) { tb_lo = min(tb_lo, A->tbin[t]); tb_hi = max(tb_hi, A->tbin[t]); }
+                const unsigned int tb_span = (unsigned int)(tb_hi - tb_lo);
+                for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+                    bool near = false;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const unsigned int eb = ebs[u];
+                        const int bin = (int)((eb - lo) >> shift);
+                        near |= eb != 0u && eb < wtau && eb >= lo && (unsigned int)(bin - tb_lo) <= tb_span;
+                    }
+                    if (!__any_sync(0xffffffffu, near)) return;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const unsigned int eb = ebs[u];
+                        if (eb == 0u || eb >= wtau || eb < lo) continue;
+                        const int bin = (int)((eb - lo) >> shift);
+                        if (!((A->tbits[bin >> 5] >> (bin & 31)) & 1u)) continue;
+                        const float p = __uint_as_float(eb);
+                        const float tq = __fadd_rn(p, Cm);
+                        const float rr = __fsub_rn(p, __fsub_rn(tq, Cm));
+                        if (fabsf(rr) == halfu || p >= bigthr) continue;
+                        const unsigned int qu = __float_as_uint(tq) - cm_bits;
+                        const unsigned long long key = make_key(eb, pos0 + c.lane + 32 * u);
+                        for (int t = 0; t < ntie; t++)
+                            if (A->tbin[t] == bin && key > A->tkey[t] && qu) {  // two halves, as in the bin tables
+                                sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
+                                if (qu >> MASS_SPLIT) sred_add(&A->tpq_hi[t], qu >> MASS_SPLIT);
+                            }
+                    }
+                });
+                __syncthreads();
+            }
+        }
+        BinQuery qy;
+        qy.bin_hi = NBINS; qy.spec_bits = nullptr;
+        qy.hq = A->u.h.hq; qy.hqh = A->u.h.hqh; qy.hc = A->u.h.hc;
+        qy.pos0 = (unsigned long long)w.pos;
+        qy.nstop = counting ? (unsigned long long)nstop : ~0ull;
+        qy.m0 = 0; qy.xq = ~0ull;
+        if (binade_ok) {
+            qy.m0 = (unsigned long long)((double)w.s * (double)inv_u);
+            unsigned long long xq = 1ull << 24;  // leaving the binade
+            if (x_ge < 3.0e38f) {
+                double t = ceil((double)x_ge * (double)inv_u);
+                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
+            }
+            if (x_gt < 3.0e38f) {
+                double t = floor((double)x_gt * (double)inv_u) + 1.0;
+                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
+            }
+            qy.xq = xq;
+        } else {
+            qy.pos0 = 0; qy.nstop = 1;  // nothing consumed yet: take the highest non-empty bin
+        }
+        if (c.tid < ntie) {
+            if (!reuse) A->tpqm[c.tid] = (unsigned long long)A->tpq_lo[c.tid] + ((unsigned long long)A->tpq_hi[c.tid] << MASS_SPLIT);
+            A->tc[c.tid] = 0ull;
+        }
+        __syncthreads();
+        qy.specbin = A->specbin;
+        find_event_bin_adj(c, qy,
+            [&](int b, unsigned long long &q, unsigned long long &n) {
+                q = (unsigned long long)qy.hq[b] + ((unsigned long long)qy.hqh[b] << MASS_SPLIT);
+                n = qy.hc[b];
+            },
+            [&](unsigned long long (&q)[BPT], unsigned long long eq) -> bool {
+                if (ntie == 0) return false;
+                // the mass before each listed element: the bins above its own (the thread that
+                // owns the bin knows), and what precedes it inside the bin
+                unsigned long long run = eq;
+#pragma unroll
+                for (int i = 0; i < BPT; i++) {
+                    const int b = NBINS - 1 - BPT * c.tid - i;
+                    for (int t = 0; t < ntie; t++)
+                        if (A->tbin[t] == b) A->tabove[t] = run;
+                    run += q[i];
+                }
+                __syncthreads();
+                if (c.tid == 0) {
+                    // from the top down (what lies below an event never matters: the walk stops there)
+                    unsigned long long done = 0ull, carried = 0ull;
+                    for (int round = 0; round < ntie; round++) {
+                        int best = -1;
+                        for (int t = 0; t < ntie; t++)
+                            if (!((done >> t) & 1ull) && (best < 0 || A->tkey[t] > A->tkey[best])) best = t;
+                        done |= 1ull << best;
+                        const float p = key_val(A->tkey[best]);
+                        const float qf = __fsub_rn(__fadd_rn(p, Cm), Cm);
+                        unsigned long long k = (unsigned long long)__float2uint_rn(__fmul_rn(qf, inv_u));
+                        if (qf > p) k -= 1ull;  // the multiple of the unit below p
+                        const unsigned long long mb = qy.m0 + A->tabove[best] + A->tpqm[best] + carried;
+                        if (qy.xq != ~0ull && mb >= qy.xq) break;
+                        const unsigned long long ct = k + ((mb + k) & 1ull);
+                        A->tc[best] = ct;
+                        carried += ct;
+                        if (qy.xq != ~0ull && mb + ct >= qy.xq) break;
+                    }
+                }
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < BPT; i++) {
+                    const int b = NBINS - 1 - BPT * c.tid - i;
+                    for (int t = 0; t < ntie; t++)
+                        if (A->tbin[t] == b) q[i] += A->tc[t];
+                }
+                return true;
+            });
+        const int hb = A->hit_bin;
+        if (hb < 0) {
+            // nothing left in this range triggers an event: consume it whole
+            if (binade_ok) w.s = (float)((double)(qy.m0 + A->tot_q) * (double)fpow2(j - 23));
+            w.pos += (long long)A->tot_c;
+            if (lvl == 1) { w.tau = 0; w.event = EV_EXHAUSTED; return; }
+            w.tau = lo; lvl = 1; lo = 0u; shift = BIN_SHIFT;  // back to the coarse bins below this range
+            continue;
+        }
+        const unsigned long long qb = A->hit_qbefore, cb = A->hit_cbefore;
+        const unsigned int blo = lo + ((unsigned int)hb << shift);
+        const unsigned long long bhi64 = (unsigned long long)lo + ((unsigned long long)(hb + 1) << shift);
+        const unsigned int bhi = bhi64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (unsigned int)bhi64;
+        const unsigned int gtau = wtau < bhi ? wtau : bhi;  // the bin's entries: blo <= value < gtau, and not zero (an absent element)
+        for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < 4; u++) any |= ebs[u] != 0u && ebs[u] >= blo && ebs[u] < gtau;
+            if (!__any_sync(0xffffffffu, any)) return;  // one bin of 2048: most warps pass most elements by
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const unsigned int eb = ebs[u];
+                if (eb != 0u && eb >= blo && eb < gtau) {
+                    const int pos = satom_add(&A->ncand, 1);
+                    if (pos < NC) A->cand[pos] = make_key(eb, pos0 + c.lane + 32 * u);
+                }
+            }
+        });
+        __syncthreads();
+        const int nb = A->ncand;
+        const bool crowded = nb > NC;
+        // what lies above the bin is consumed without an event either way
+        const float s_bin = binade_ok ? (float)((double)(qy.m0 + qb) * (double)fpow2(j - 23)) : w.s;
+        const long long pos_bin = w.pos + ((counting || !binade_ok) ? (long long)cb : 0);
+        if (crowded && lvl < 3) {
+            w.s = s_bin; w.pos = pos_bin;
+            w.tau = bhi < w.tau ? bhi : w.tau;
+            lo = blo; shift = (lvl == 1) ? BIN_SHIFT2 : 0; lvl++;
+            c.status |= MOLLA_ROW_SLOW_PATH;
+            continue;
+        }
+        if (crowded) {
+            // one value, more copies than the buffer holds: add them one at a time (thread 0), then
+            // find which copy, in token order, the event fell on
+            c.status |= MOLLA_ROW_SLOW_PATH;
+            const float pv = __uint_as_float(blo);
+            if (c.tid == 0) {
+                float s = s_bin;
+                long long pos = pos_bin;
+                int ev = EV_NONE, at = -1;
+                for (int i = 0; i < nb; i++) {
+                    s = __fadd_rn(s, pv);
+                    pos++;
+                    if (s >= x_ge) ev = EV_CUT;
+                    else if (x_gt < s) ev = EV_DRAW;
+                    else if (counting && pos >= nstop) ev = EV_LIMIT;
+                    if (ev != EV_NONE) { at = i; break; }
+                }
+                A->b_event = ev; A->b_s = s; A->b_pos = pos; A->b_aux = at;
+            }
+            __syncthreads();
+            const int ev = A->b_event, at = A->b_aux;
+            w.s = A->b_s; w.pos = A->b_pos;
+            if (ev != EV_NONE) {
+                w.event = ev; w.idx = list_nth_equal(c, blo, at); w.p = pv; w.tie = 1;
+                return;
+            }
+            w.tau = blo;
+            continue;
+        }
+        sort_cands(c, nb);
+        walk_sorted(c, nb, s_bin, pos_bin, x_ge, x_gt, counting, nstop);
+        w.s = A->b_s; w.pos = A->b_pos; w.tau = blo;
+        const int ev = A->b_event;
+        if (ev != EV_NONE) {
+            w.event = ev; w.idx = A->b_idx; w.p = A->b_p; w.tie = A->b_aux;
+            __syncthreads();
+            return;
+        }
+        if (phase > 8) c.status |= MOLLA_ROW_SLOW_PATH;
+    }
+    w.event = EV_DEGENERATE;
+    c.status |= MOLLA_ROW_DEGENERATE;
+}
+
+__global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant__ RowsArgs R) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CtxF c;
+    c.tid = threadIdx.x; c.lane = c.tid & 31; c.warp = c.tid >> 5; c.status = 0;
+    c.A = reinterpret_cast<AuxF *>(smem_raw);
+    c.R = &R;
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    pdl_next();
+    pdl_wait();
+    c.rr = blockIdx.x; c.r = R.r0 + c.rr;
+    c.pl = R.plan[c.rr];
+    if (c.pl.kind == PLAN_DONE) return;
+    const BatchArgs &a = R.a;
+    c.cfg = row_cfg(a, c.r);
+    c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
+    c.gitems = R.items + (size_t)c.rr * R.ntile * ITEMS_PER_TILE;
+    c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
+    const RowCfg &g = c.cfg;
+    const int ntile = R.ntile, imax = c.pl.imax;
+    for (int t = c.tid; t < ntile; t += NT) {
+        const TileOut o = R.to[(size_t)c.rr * ntile + t];
+        A->tcnt[t] = o.cnt; A->tni[t] = o.nitem;
+    }
+    unsigned long long *gcand = R.cand + (size_t)c.rr * HEADCAP;
+    int nc_all = g.pure ? 0 : R.ncand[c.rr];
+    if (nc_all > HEADCAP) {
+        if (!(c.pl.flags & F_LIST)) {
+            for (int t = 0; t < ntile; t += SPAN / TILE) tile_again(c, t, min(t + SPAN / TILE, ntile), nullptr, true);
+            c.pl.flags |= F_LIST;
+        }
+        nc_all = narrow_head(c, gcand);
+    }
+    const bool head_overflow = nc_all > HEADCAP;  // thousands of equal values at the head's edge
+    const bool narrow = (c.pl.flags & F_NARROW) != 0;
+    if (narrow) c.status |= MOLLA_ROW_SLOW_PATH;
+
+    float dZ = 0.0f, dsum = 0.0f, dtarget = 0.0f, dp = 0.0f;
+    int token = -1;
+    auto finish = [&]() { if (c.tid == 0) finish_row(a, c.r, g, c.status, token, dZ, dsum, dtarget, dp); };
+
+    // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
+    const float Z = exact_sum(c, false, 0.0f);
+    dZ = Z;
+    const float yZ = __fdiv_rn(1.0f, Z);
+    const float u01 = draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull);
+
+    // min-p (sample.mojo:508-523) keeps a prefix of the sorted order: the entries whose probability
+    // reaches p_max * min_p. Below 2.2e-8 the list no longer holds them all.
+    long long n_use = g.n_lim;
+    unsigned int minp_pbits = 0u, e_floor = 0u;
+    if (g.minp > 0.0f) {
+        const float p_top = __fdiv_rn(expf_pinned(__fsub_rn(c.pl.top, c.pl.top)), Z);
+        const float floor_p = __fmul_rn(p_top, g.minp);
+        minp_pbits = __float_as_uint(floor_p);
+        if (!(floor_p >= 2.2e-8f)) { c.status |= MOLLA_ROW_UNSUPPORTED; finish(); return; }
+        if (!g.pure) {
+            unsigned int lo_b = 0u, hi_b = 0x3F800000u;
+            for (int it = 0; it < 32 && lo_b < hi_b; it++) {
+                const unsigned int mid = lo_b + ((hi_b - lo_b) >> 1);
+                if (__fdiv_rn(__uint_as_float(mid), Z) >= floor_p) hi_b = mid; else lo_b = mid + 1u;
+            }
+            e_floor = hi_b;
+            int n = 0, tot;
+            if (c.pl.flags & F_LIST) {
+                for_list4(c, [&](const unsigned int (&eb)[4], int, float *) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) n += (eb[u] >= e_floor && eb[u] != 0u) ? 1 : 0;
+                });
+            } else {
+                // the head holds the row's largest, more of them than top-k keeps: a floor below all of it changes nothing
+                for (int i = c.tid; i < nc_all; i += NT) n += (unsigned int)(gcand[i] >> 32) >= e_floor ? 1 : 0;
+            }
+            (void)block_excl_scan<int>(n, A->wsi, &tot);
+            const long long n_ge = tot < 1 ? 1 : tot;  // never empties
+            if (n_ge < n_use) n_use = n_ge;
+        }
+    }
+
+    if (g.pure) {
+        // ---- nothing sorted: the draw walks the vocabulary in order (sample.mojo:365-369, 580-594):
+        // probabilities p = e / Z (:437-438), what min-p drops becomes zero
+        for (int t = c.warp; t < ntile; t += NWARP) {
+            const int n = A->tcnt[t];
+            float *src = c.list + (size_t)t * TILE;
+            float s = 0.0f;
+            for (int i = c.lane; i < n; i += 32) {
+                float p = prob_of(src[i], Z, yZ);
+                if (__float_as_uint(p) < minp_pbits) p = 0.0f;
+                src[i] = p;
+                s += p;
+            }
+            s = warp_sum(s);
+            if (c.lane == 0) A->tsum[t] = s;
+        }
+        __syncthreads();
+        {
+            const int t = 2 * c.tid;
+            const float s0 = t < ntile ? A->tsum[t] : 0.0f, s1 = t + 1 < ntile ? A->tsum[t + 1] : 0.0f;
+            float tot;
+            const float ex = block_excl_scan_plus(s0 + s1, A->wsf, &tot);
+            __syncthreads();
+            if (t < ntile) A->tsum[t] = ex;
+            if (t + 1 < ntile) A->tsum[t + 1] = ex + s0;
+        }
+        __syncthreads();
+        float *mine = A->tile + (size_t)c.tid * PITCH;
+        for (int t = c.warp; t < ntile; t += NWARP) {
+            const int n = A->tcnt[t], per = (n + 31) >> 5, off = min(n, c.lane * per), cnt = min(per, n - off);
+            const float *src = c.list + (size_t)t * TILE;
+            float s = 0.0f;
+            for (int i = 0; i < ((cnt + 3) & ~3); i++) {
+                const float p = i < cnt ? src[off + i] : 0.0f;
+                mine[i] = p;
+                s += p;
+            }
+            __syncwarp();
+            bool care;
+            const int ni = tile_items(mine, cnt, off, n, s, A->tsum[t], c.gitems + (size_t)t * ITEMS_PER_TILE, care);
+            if (c.lane == 0) A->tni[t] = (unsigned short)ni;
+            __syncwarp();
+        }
+        __syncthreads();
+        const float sum = exact_sum(c, false, 0.0f);
+        const float target = __fmul_rn(u01, sum);
+        (void)exact_sum(c, true, target);
+        dsum = sum; dtarget = target;
+        if (A->w_found) {
+            if (c.tid == 0) token = token_of(c, A->w_tile, A->w_at);
+        } else {
+            // the walk fell off the end: the reference returns the last token of the vocabulary,
+            // whether or not it could matter to any sum ... or the last one min-p left
+            token = a.V - 1;
+            if (minp_pbits) {
+                int last = -1;
+                for_list4(c, [&](const unsigned int (&pb)[4], int pos0, float *) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (pb[u] >= minp_pbits && pb[u] != 0u) last = max(last, pos0 + c.lane + 32 * u);
+                });
+                last = __reduce_max_sync(0xffffffffu, last);
+                __syncthreads();
+                if (c.lane == 0) A->wsi[c.warp] = last;
+                __syncthreads();
+                for (int w = 0; w < NWARP; w++) last = max(last, A->wsi[w]);
+                token = last >= 0 ? token_of(c, last) : imax;
+            }
+        }
+        finish();
+        return;
+    }
+
+    // ---- sorted order: the head's candidates as probabilities
+    const int nc = head_overflow ? 0 : nc_all;
+    if (head_overflow) c.status |= MOLLA_ROW_SLOW_PATH;  // no head: the descending walk takes everything from the top
+    {
+        for (int i = c.tid; i < nc; i += NT) {
+            const unsigned long long kk = gcand[i];
+            A->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(kk), Z, yZ)) << 32) | (kk & 0xFFFFFFFFull);
+        }
+    }
+    sort_cands(c, nc);
+    for (int i = c.tid; i < nc; i += NT) {
+        const float p = A->pc[i];
+        const bool eq = (i > 0 && A->pc[i - 1] == p) || (i + 1 < nc && A->pc[i + 1] == p);
+        A->hidx[i] = (unsigned int)key_idx(A->cand[i]) | (eq ? 0x80000000u : 0u);
+    }
+    __syncthreads();
+#ifdef MOLLA_SAMPLE_TESTING
+    if (a.topk_out) {
+        for (int i = c.tid; i < a.topk_cap; i += NT)
+            a.topk_out[(long long)c.r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? (int)(A->hidx[i] & 0x7fffffffu) : -1;
+    }
+#endif
+    const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST);
+    const bool typ_on = g.typ < 1.0f;
+    if (c.tid == 0) {
+        float s = 0.0f;
+        int cut = -1, tie = 0;
+        bool by_mass = false;
+        // the prefix sums of the sorted head (sample.mojo:497-506), eight loads ahead of the
+        // additions; at most n_use elements are added
+        const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
+        int i = 0;
+        while (i < lim && cut < 0) {
+            float v[8];
+            const int m = min(8, lim - i);
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[q] = (q < m) ? A->pc[i + q] : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                if (q < m && cut < 0) {
+                    s = __fadd_rn(s, v[q]);
+                    A->pre[i + q] = s;
+                    if (g.topp_on && s >= g.P) { cut = i + q + 1; by_mass = true; }
+                }
+            }
+            i += m;
+        }
+        const long long pos = (cut >= 0) ? (long long)cut : (long long)lim;
+        auto equal_next_to = [&](int x) { return (A->hidx[x] & 0x80000000u) != 0u; };
+        if (by_mass) {
+            if (narrow ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && A->pc[cut] == A->pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
+        } else if (lim > 0 && (long long)lim >= n_use) {
+            cut = lim;  // the count limit
+            if (narrow && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
+        }
+        if (cut < 0 && !p3row && !head_overflow) cut = nc;  // everything that can matter is in the head
+        if (!narrow && n_use < (long long)a.V && (long long)nc > n_use && A->pc[n_use] == A->pc[n_use - 1])
+            tie |= MOLLA_ROW_TOPK_TIE;
+        A->b_s = s; A->b_pos = pos; A->b_event = EV_NONE; A->b_idx = -1; A->b_p = 0.0f;
+        if (typ_on) {
+            A->ncand = narrow ? -1 : cut;  // the typical-p filter takes over from here
+        } else if (cut > 0) {
+            const float sum = A->pre[cut - 1];
+            const float target = __fmul_rn(u01, sum);
+            int at = cut - 1;
+            for (int i0 = 0; i0 < cut && at == cut - 1; i0 += 8) {
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[q] = (i0 + q < cut) ? A->pre[i0 + q] : 0.0f;
+#pragma unroll
+                for (int q = 7; q >= 0; q--)
+                    if (i0 + q < cut && target < v[q]) at = i0 + q;  // the first one wins
+            }
+            A->b_event = EV_DRAW; A->b_idx = (int)(A->hidx[at] & 0x7fffffffu); A->b_p = A->pc[at];
+            if (narrow ? equal_next_to(at) : ((at > 0 && A->pc[at - 1] == A->pc[at]) || (at + 1 < cut && A->pc[at + 1] == A->pc[at])))
+                tie |= MOLLA_ROW_CHOSEN_TIE;
+            A->b_sum = sum; A->b_target = target;
+        }
+        A->b_aux = tie;
+    }
+    __syncthreads();
+    c.status |= (unsigned int)A->b_aux;
+    const float head_s = A->b_s;
+    const long long head_pos = A->b_pos;
+    if (typ_on) {
+        const int m = A->ncand;
+        __syncthreads();
+        if (m <= 0 || m > HEADC) {
+            c.status |= MOLLA_ROW_UNSUPPORTED;  // what the earlier filters left reaches past the head, or is wider than the filter's scratch
+        } else {
+            typical_head(c, m, g.typ, u01);
+            token = A->b_idx; dp = A->b_p; dsum = A->b_sum; dtarget = A->b_target;
+            c.status |= (unsigned int)A->b_aux;
+        }
+        finish();
+        return;
+    }
+    if (A->b_event == EV_DRAW) {
+        token = A->b_idx; dp = A->b_p; dsum = A->b_sum; dtarget = A->b_target;
+        finish();
+        return;
+    }
+
+    // ---- past the head: the cut walk, then the draw walk, over the probabilities
+    // (sample.mojo:437-438); what the head took is consumed
+    const unsigned int tau_bits = head_overflow ? 0xffffffffu : c.pl.tau_bits;
+    for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (eb[u]) src[u * 32 + c.lane] = eb[u] >= tau_bits ? 0.0f : prob_of(__uint_as_float(eb[u]), Z, yZ);
+    });
+    __syncthreads();
+    const bool limited = n_use < (long long)a.V;
+    FWalk w;
+    FResume resume;
+    resume.valid = 0;
+    int cut_event = EV_NONE, cut_idx = -1;
+    float cut_p = 0.0f, sum = 0.0f, target = 0.0f;
+    bool settled = false;    // the token is known, or the row is degenerate
+    bool resolved = false;
+    for (int leg = 0; leg < 2; leg++) {   // (one call site for both walks)
+        w.s = head_s; w.pos = head_pos; w.tau = 0xFFFFFFFFu;
+        w.event = EV_NONE; w.idx = -1; w.p = 0; w.tie = 0;
+        const bool cut_round = leg == 0;
+        descend_list(c, w, (cut_round && g.topp_on) ? g.P : 3.4e38f, cut_round ? 3.4e38f : target,
+                     (cut_round && limited) ? n_use : -1, resume, !cut_round);
+        if (!cut_round) {
+            if (w.event == EV_DRAW) {
+                token = token_of(c, w.idx); dp = w.p; resolved = true;
+                if (w.tie) c.status |= MOLLA_ROW_CHOSEN_TIE;
+            } else if (w.event == EV_DEGENERATE) {
+                resolved = true;
+            }
+            break;
+        }
+        cut_event = w.event; cut_idx = w.idx; cut_p = w.p;
+        if (cut_event == EV_DEGENERATE) { settled = true; break; }
+        if (cut_event == EV_CUT && w.tie) c.status |= MOLLA_ROW_TOPP_TIE;
+        if (cut_event == EV_LIMIT && w.tie) c.status |= MOLLA_ROW_TOPK_TIE;
+        sum = w.s;
+        target = __fmul_rn(u01, sum);
+        dsum = sum; dtarget = target;
+        // is the drawn element in the head? (the first prefix sum above the target)
+        __syncthreads();
+        if (c.tid == 0) A->evt_thread = 0x7fffffff;
+        __syncthreads();
+        for (int i = c.tid; i < nc; i += NT)
+            if (target < A->pre[i]) { atomicMin(&A->evt_thread, i); break; }
+        __syncthreads();
+        if (A->evt_thread != 0x7fffffff) {
+            const int at = A->evt_thread;
+            token = (int)(A->hidx[at] & 0x7fffffffu);
+            dp = __fsub_rn(A->pre[at], at > 0 ? A->pre[at - 1] : 0.0f);
+            if (A->hidx[at] & 0x80000000u) c.status |= MOLLA_ROW_CHOSEN_TIE;
+            settled = true;
+            break;
+        }
+        if (!(target < sum)) break;
+    }
+    if (!settled && !resolved) {
+        // the walk falls off the end: the last kept candidate (sample.mojo:591-594)
+        if (cut_event == EV_CUT || cut_event == EV_LIMIT) {
+            token = token_of(c, cut_idx); dp = cut_p;
+        } else {
+            // everything listed was kept: its smallest value, highest id last
+            unsigned long long best = ~0ull;
+            for_list4(c, [&](const unsigned int (&pb)[4], int pos0, float *) {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (pb[u]) { const unsigned long long kk = make_key(pb[u], pos0 + c.lane + 32 * u); best = kk < best ? kk : best; }
+            });
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+                best = ob < best ? ob : best;
+            }
+            __syncthreads();
+            if (c.lane == 0) A->wsu[c.warp] = best;
+            __syncthreads();
+            for (int v = 0; v < NWARP; v++) best = A->wsu[v] < best ? A->wsu[v] : best;
+            token = (best != ~0ull) ? token_of(c, key_idx(best)) : imax;
+        }
+    }
+    finish();
+}
+
+// ---- host side --------------------------------------------------------------------------------
+// The widest layout of one row over thread blocks that F_NARROW speaks of: blocks of at most 38400
+// logits, 1, 2, 4 or 8 of them; more than the row needs where the batch leaves the chip idle.
+void narrow_layout(int V, int B, int sms, int &oG, int &oVc, int &oL) {
+    oG = 0; oVc = 0; oL = 0;
+    for (int G = 1; G <= 8; G *= 2) {
+        const int Vc = ((((V + G - 1) / G) + 3) / 4) * 4;
+        int L = (Vc + NT - 1) / NT;
+        if ((L & 1) == 0) L += 1;
+        if (L > 75) continue;
+        if (oG == 0 || ((long long)B * G * 9 <= (long long)sms * 8 && L >= 9)) { oG = G; oVc = Vc; oL = L; }
+    }
+}
+
+constexpr long long IN_FLIGHT = 1ll << 27;   // logits whose intermediate results the workspace holds at a time
+
+long long most_in_flight(int V) {
+    const long long per = (long long)((V + TILE - 1) / TILE) * TILE;
+    return IN_FLIGHT / per > 1 ? IN_FLIGHT / per : 1;
+}
+int rows_in_flight(int B, int V) {   // a batch that does not fit goes in equal parts
+    const long long most = most_in_flight(V), parts = (B + most - 1) / most;
+    return (int)((B + parts - 1) / parts);
+}
+size_t al(size_t n) { return (n + 255) & ~(size_t)255; }
+
+// Lays the rows' intermediate results over the workspace; returns the bytes they take.
+size_t lay_out(RowsArgs &A, char *ws, int rows, int V) {
+    const size_t nt = (size_t)((V + TILE - 1) / TILE), n = (size_t)rows * nt;
+    size_t o = 0;
+    auto take = [&](size_t bytes) { char *p = ws + o; o += al(bytes); return p; };
+    A.elist = (float *)take(n * TILE * sizeof(float));
+    A.items = (Item *)take(n * ITEMS_PER_TILE * sizeof(Item));
+    A.gmax = (float *)take(n * 32 * sizeof(float));
+    A.kmask = (unsigned int *)take(n * 32 * sizeof(unsigned int));
+    A.ts = (TileStat *)take(n * sizeof(TileStat));
+    A.tp = (TilePlan *)take(n * sizeof(TilePlan));
+    A.to = (TileOut *)take(n * sizeof(TileOut));
+    A.cand = (unsigned long long *)take((size_t)rows * HEADCAP * sizeof(unsigned long long));
+    A.plan = (RowPlan *)take((size_t)rows * sizeof(RowPlan));
+    A.ncand = (int *)take((size_t)rows * sizeof(int));
+    return o;
+}
+
+template <class K>
+cudaError_t launch(K kernel, unsigned int blocks, unsigned int threads, size_t smem, cudaStream_t st, const RowsArgs &A) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    // every kernel waits for the one before it by itself: its blocks are on the SMs by then
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, A);
+}
+
+}  // namespace
+
+size_t molla_rows_workspace_bytes(int B, int V) {
+    RowsArgs A;
+    const long long most = most_in_flight(V);
+    return lay_out(A, nullptr, (int)(B < 1 ? 1 : (B < most ? B : most)), V);
+}
+
+int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, char *err, size_t errlen) {
+    static bool ready[64] = {};
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && (dev >= 64 || !ready[dev])) {
+        e = cudaFuncSetAttribute(tile_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_exp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AuxF));
+        if (e == cudaSuccess && dev < 64) ready[dev] = true;
+    }
+    RowsArgs A;
+    A.a = a;
+    A.a.Vg = a.V; A.a.col0 = 0; A.a.mode = 0;
+    A.ntile = (a.V + TILE - 1) / TILE;
+    A.nspan = (a.V + SPAN - 1) / SPAN;
+    A.glog = A.ntile * 32 <= PLAN_GROUPS ? 0 : 2;
+    narrow_layout(a.V, a.B, sms, A.oG, A.oVc, A.oL);
+    const int rows = rows_in_flight(a.B, a.V);
+    lay_out(A, (char *)d_workspace, rows, a.V);
+    for (A.r0 = 0; A.r0 < a.B && e == cudaSuccess; A.r0 += rows) {
+        A.rows = a.B - A.r0 < rows ? a.B - A.r0 : rows;
+        const unsigned int spans = (unsigned int)A.rows * (unsigned int)A.nspan;
+        e = launch(tile_stats_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
+        if (e == cudaSuccess) e = launch(row_plan_kernel, (unsigned int)A.rows, NT, 0, st, A);
+        if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
+        if (e == cudaSuccess) e = launch(row_finish_kernel, (unsigned int)A.rows, NT, sizeof(AuxF), st, A);
+    }
+    if (e != cudaSuccess) {
+        snprintf(err, errlen, "kernel launch failed: %s", cudaGetErrorString(e));
+        return MOLLA_ERR_CUDA;
+    }
+    return MOLLA_OK;
+}

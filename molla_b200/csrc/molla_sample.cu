@@ -46,7 +46,7 @@
 #endif
 #include "molla_device.cuh"
 #include "molla_exact.cuh"
-#include "molla_cluster.h"
+#include "molla_rows.h"
 
 using namespace molla;
 
@@ -56,6 +56,8 @@ constexpr int LT = 11;               // elements per lane per piece (odd: confli
 constexpr int PIECE = 32 * LT;       // 352 floats = 1408 bytes: what one warp fetches at a time
 constexpr int NSTAGE = 4;            // pieces in flight per warp
 constexpr int MAX_PIECES = 128;      // per warp: V <= 16 * 128 * 352 = 720896
+constexpr int MAX_VOCAB = NWARP * MAX_PIECES * PIECE;
+constexpr int MAX_MASKED_VOCAB = 307200;
 constexpr int STAGE_FLOATS = NWARP * NSTAGE * PIECE;       // 22528 floats = 90112 bytes
 constexpr int SLIST_CAP = STAGE_FLOATS / 2;                 // list entries that fit the stage area
 constexpr int SA_WORDS = 3 + NWARP + HEAD_NEED + 1;  // max, argmax, ties, region maxima, top thread maxima
@@ -1960,7 +1962,9 @@ constexpr size_t WS_HEADER = 256 + (size_t)ORDER_CAP * 4;
 size_t help_bytes(size_t ctas) { return ctas * (sizeof(HelpSlot) + (size_t)HELP_TABLE_WORDS * 4); }
 size_t batch_workspace_bytes(int B, int V, int sms) {
     const size_t ctas = (size_t)(B < sms ? B : sms);
-    return WS_HEADER + ctas * 2 * (size_t)NWARP * (size_t)region_floats(V) * 8 + help_bytes(ctas);
+    const size_t lists = WS_HEADER + ctas * 2 * (size_t)NWARP * (size_t)region_floats(V) * 8 + help_bytes(ctas);
+    const size_t rows = molla_rows_workspace_bytes(B, V);
+    return lists > rows ? lists : rows;
 }
 
 int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, int max_ctas = 0x7fffffff, bool with_help = false) {
@@ -2005,13 +2009,11 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
     return MOLLA_OK;
 }
 
-// The ordinary entry points' launch: the cluster kernel when the vocabulary fits a cluster, else
-// the streaming kernel with its lists in the workspace.
-int launch_sampling(const BatchArgs &args_in, void *d_workspace, cudaStream_t st) {
-    const int rc = molla_cluster_launch(args_in, d_workspace, st, g_err, sizeof(g_err));
-    if (rc != MOLLA_CLUSTER_DECLINED) return rc;
-    if (args_in.mask) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies a thread-block cluster can hold%s");
-    return launch_rows(args_in, d_workspace, st, 0x7fffffff, true);
+// The ordinary entry points' launch.
+int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st) {
+    if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
+    if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
+    return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err));
 }
 
 }  // namespace
