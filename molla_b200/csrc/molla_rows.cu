@@ -34,10 +34,11 @@ constexpr int MAX_TILES = 704;             // V <= 720896
 constexpr int ITEMS_PER_TILE = 66;         // a run and a careful chunk per lane at most, and one more run
 constexpr int HEADCAP = 2048;              // candidates of the sorted head at most
 constexpr int HEAD_MOST = 1026;            // the sorted head covers top-k + 1 up to this many
-constexpr int ITEM_CAP = 512;              // items of a row that fit shared memory
-constexpr int CARE_CAP = 64;               // careful chunks whose entries are fetched ahead
+constexpr int ITEM_CAP = 384;              // items of a row that fit shared memory
+constexpr int CARE_CAP = 48;               // careful chunks whose entries are fetched ahead
 constexpr int TIE_CAP = 64;                // rounding ties a walk resolves by parity; more send it the slow way
-constexpr int PLAN_GROUPS = 300 * 32;      // group maxima row_plan looks at, at most
+constexpr int PLAN_BINS = 1024;            // row_plan: bins of the lanes' maxima by distance below the row's,
+constexpr float PLAN_RES = 32.0f;          // 32 per unit of logit
 
 enum { PLAN_DONE = 0, PLAN_SAMPLED = 1 };
 enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8 };
@@ -45,7 +46,6 @@ enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8 };
 struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
 struct __align__(8) TilePlan { float thr, est; };
 struct __align__(16) TileOut { unsigned int emax; float esum; unsigned short cnt, nitem; unsigned int pad; };
-struct __align__(16) RowPlan { int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; int pad; };
 
 // Items: the exact sequential sum of a tile's values as a short program. While the running sum s
 // stays in one binade, fl(s + v) is s plus rne(v / ulp) units, an integer that does not depend on s;
@@ -62,10 +62,24 @@ struct __align__(16) Item {
     unsigned int oc;       // first entry in the tile's list << 16 | entries
 };
 
+// ---- settings ---------------------------------------------------------------------------------
+struct __align__(16) RowCfg {
+    long long lrow;
+    float T, P, minp, typ, rp, fp, pp;
+    int q, k, ring_n, H, b0, nb, npatch;
+    const long long *histp;
+    long long n_lim;
+    bool greedy, topp_on, pure, open_row;
+    unsigned int status;
+};
+
+// What row_plan hands to the kernels behind it.
+struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; int pad; };
+
 struct RowsArgs {
     BatchArgs a;
     int r0, rows;            // batch rows [r0, r0 + rows) are in flight
-    int ntile, nspan, glog;  // glog: log2 of the lanes whose maxima row_plan joins
+    int ntile, nspan;
     int oG, oVc, oL;         // see F_NARROW
     TileStat *ts;            // [rows][ntile]
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
@@ -81,17 +95,6 @@ struct RowsArgs {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// ---- settings ---------------------------------------------------------------------------------
-struct RowCfg {
-    int q; long long lrow;
-    float T, P, minp, typ, rp, fp, pp;
-    int k, ring_n, H, b0, nb, npatch;
-    const long long *histp;
-    long long n_lim;
-    bool greedy, topp_on, pure, open_row;
-    unsigned int status;
-};
 
 // Where row r's settings live and what they are; status bits for a row that cannot be sampled
 // (the rules of SamplerConfig.check, sample.mojo:140-154; NaN fails every test).
@@ -384,7 +387,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
 // Kernel 2: one block per row.
 // =============================================================================
 struct PlanShared {
-    float g[PLAN_GROUPS];
+    unsigned int hist[PLAN_BINS];
+    int edge;
     float wsf[NWARP + 1];
     int wsi[NWARP + 1];
 };
@@ -417,6 +421,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     RowCfg c = row_cfg(a, r);
     if (MOLLA_KNOB(a, 16) && !c.status) c.status |= MOLLA_ROW_LOAD_TIMEOUT;  // testing build: a wait that ran out
     RowPlan pl;
+    pl.c = c;
     pl.kind = PLAN_DONE; pl.flags = 0; pl.top = 0; pl.tau_bits = 1u; pl.xmax = 0; pl.imax = 0; pl.need = 0; pl.pad = 0;
     if (c.status) {
         if (tid == 0) { finish_row(a, r, c, c.status, -1, 0, 0, 0, 0); A.plan[rr] = pl; }
@@ -489,38 +494,36 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     float tau_x = INFINITY;
     bool narrow = false;
     if (!c.pure) {
-        const int gl = A.glog, ng = (A.ntile * 32) >> gl;
-        const float *gm = A.gmax + (size_t)rr * A.ntile * 32;
-        for (int i = tid; i < ng; i += NT) {
-            float v = gm[i << gl];
-            for (int u = 1; u < (1 << gl); u++) v = fmaxf(v, gm[(i << gl) + u]);
-            S.g[i] = v;
+        const int ng = A.ntile * 32;
+        const float *gm = A.gmax + (size_t)rr * ng;
+        // one histogram of the lanes' maxima by distance below the row's
+        for (int i = tid; i < PLAN_BINS; i += NT) S.hist[i] = 0u;
+        if (tid == 0) S.edge = -1;
+        __syncthreads();
+        for (int i0 = 0; i0 < ng; i0 += 8 * NT) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = (i0 + u * NT + tid < ng) ? gm[i0 + u * NT + tid] : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const float d = (xmax - v[u]) * PLAN_RES;
+                if (d < (float)PLAN_BINS) sred_add(&S.hist[(int)d], 1u);
+            }
         }
         __syncthreads();
-        auto count = [&](float t) -> int {
-            int n = 0;
-            for (int i = tid; i < ng; i += NT) n += S.g[i] >= t ? 1 : 0;
-            n = __reduce_add_sync(0xffffffffu, n);
-            if (lane == 0) S.wsi[warp] = n;
-            __syncthreads();
-            n = 0;
+        constexpr int PER = PLAN_BINS / NT;
+        int n[PER], sum = 0, tot;
 #pragma unroll
-            for (int w = 0; w < NWARP; w++) n += S.wsi[w];
-            __syncthreads();
-            return n;
-        };
-        float lo = xmax - 32.0f, hi = xmax;
-        tau_x = -INFINITY;
-        if (fabsf(xmax) < 65536.0f && count(lo) >= need) {
-            const int enough = (int)need + (int)need / 32;
-            for (int it = 0; it < 24; it++) {
-                const float mid = 0.5f * (lo + hi);
-                if (!(mid > lo) || !(mid < hi)) break;
-                const int n = count(mid);
-                if (n >= need) { lo = mid; if (n <= enough) break; } else hi = mid;
-            }
-            tau_x = lo;
+        for (int i = 0; i < PER; i++) { n[i] = (int)S.hist[PER * tid + i]; sum += n[i]; }
+        int run = block_excl_scan<int>(sum, S.wsi, &tot);
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            if (run < need && run + n[i] >= need) S.edge = PER * tid + i;
+            run += n[i];
         }
+        __syncthreads();
+        // (a bin's lower end, and a little below it: the subtraction and the product above were rounded)
+        tau_x = (S.edge >= 0 && fabsf(xmax) < 65536.0f) ? xmax - ((float)(S.edge + 1) + 0.25f) * (1.0f / PLAN_RES) : -INFINITY;
         // F_NARROW: a top-k so wide for the vocabulary that fewer ranges than candidates exist (one range
         // per thread of the widest layout: oG blocks of NT threads with oL logits each). Such rows report
         // the order of equal probabilities the way the descending walk sees it.
@@ -753,7 +756,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     const RowPlan pl = A.plan[rr];
     if (pl.kind == PLAN_DONE) return;
     const BatchArgs &a = A.a;
-    const RowCfg c = row_cfg(a, r);
+    const RowCfg &c = pl.c;
     load_span(a, c, r, span * SPAN, S->x, &S->s, true);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
     if (tile >= A.ntile) return;
@@ -795,16 +798,17 @@ struct __align__(16) AuxF {
             } u;
             unsigned long long cand[NC];   // the head's, then a bin's candidates
             unsigned long long tmp[NC];
-            float pc[NC];
-            float pre[HEADCAP];
+            unsigned int sbin[NBINS];
+            __align__(16) float pc[NC];
+            __align__(16) float pre[HEADCAP];
             unsigned int hidx[HEADCAP];
         };
     };
     Item items[ITEM_CAP + 1];
     unsigned int isrc[ITEM_CAP];           // tile << 8 | slot of the fetched entries (255: none)
-    float care[CARE_CAP * 32];
+    __align__(16) float care[CARE_CAP * 32];
     unsigned short careidx[CARE_CAP];
-    float ebuf[TILE];
+    __align__(16) float ebuf[TILE];
     unsigned short tcnt[MAX_TILES];        // entries in the tile's list
     unsigned short tni[MAX_TILES];         // items of the tile
     int toff[MAX_TILES + 1];               // first item of the tile
@@ -823,6 +827,15 @@ struct __align__(16) AuxF {
     unsigned int tbits[NBINS / 32];
 };
 static_assert(sizeof(SpanScratch) + (size_t)SPAN_THREADS * PITCH * 4 <= sizeof(float) * NWARP * 32 * PITCH, "a span and its scratch fit the tiles' space");
+
+// Profiling stamps exist in the testing build only (per row 32 slots of clock readings and counts).
+#ifdef MOLLA_SAMPLE_TESTING
+#define FSTAMP(i) do { if (c.R->a.prof && c.tid == 0) c.R->a.prof[(long long)c.r * 32 + (i)] = clock64(); } while (0)
+#define FCOUNT(i, v) do { if (c.R->a.prof && c.tid == 0) c.R->a.prof[(long long)c.r * 32 + (i)] += (v); } while (0)
+#else
+#define FSTAMP(i) do { } while (0)
+#define FCOUNT(i, v) do { } while (0)
+#endif
 
 struct CtxF {
     int tid, lane, warp;
@@ -858,7 +871,7 @@ __device__ int token_of(const CtxF &c, int tile, int nth) {
 }
 __device__ __forceinline__ int token_of(const CtxF &c, int pos) { return token_of(c, pos >> 10, pos & (TILE - 1)); }
 
-// Tile `t` evaluated again, as kernel 3 did it: by warp t % 8, its values packed into dst.
+// Tiles [t0, t1) of one span evaluated again, as kernel 3 did it: their values packed into dst or the list.
 __device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
     AuxF *A = c.A;
     IN_SHARED(A);
@@ -878,52 +891,78 @@ __device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
     __syncthreads();
 }
 
-// v[0..n) added one by one to the sum with bit pattern A->w_sb (thread 0). With `locate`, stops at the
-// first value behind which the sum exceeds `target`.
-__device__ __forceinline__ void run_values(AuxF *A, unsigned int &sb, const float *v, int n, int off, int tile, bool locate, float target) {
+// n values, four at a time from a 16-byte aligned place that is padded with zeros, added one by one to
+// the sum with bit pattern `sb`. Every lane of the warp does the same. With `locate`, stops at the first
+// value behind which the sum exceeds `target`; returns its number, or -1.
+__device__ __forceinline__ int run_values(unsigned int &sb, const float *v, int n, bool locate, float target) {
+    const float4 *v4 = reinterpret_cast<const float4 *>(v);
     float s = __uint_as_float(sb);
     for (int i = 0; i < n; i += 8) {
-        float x[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) x[u] = i + u < n ? v[i + u] : 0.0f;   // (adding nothing changes nothing)
+        const float4 x = v4[i >> 2], y = v4[(i >> 2) + 1];
         const float s0 = s;
-#pragma unroll
-        for (int u = 0; u < 8; u++) s = __fadd_rn(s, x[u]);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x.x), x.y), x.z), x.w);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, y.x), y.y), y.z), y.w);
         if (locate && target < s) {
             s = s0;
             for (int u = 0; u < 8; u++) {
                 s = __fadd_rn(s, v[i + u]);
-                if (target < s) { A->w_found = 1; A->w_tile = tile; A->w_at = off + i + u; break; }
+                if (target < s) { sb = __float_as_uint(s); return i + u; }
             }
-            break;
         }
     }
     sb = __float_as_uint(s);
+    return -1;
 }
 
-// Thread 0: the items of the batch in shared memory from A->w_i on. Ends with A->w_need = -1 (the batch
-// is through, or the target is found) or the item whose values are wanted.
+// One warp: the items of the batch in shared memory from A->w_i on, 32 at a time. Runs in the sum's
+// binade are consumed by a scan of their units, whatever needs care one by one. Ends with A->w_need = -1
+// (the batch is through, or the target is found) or the item whose values are wanted.
 __device__ void run_items(AuxF *A, int n, bool locate, float target) {
     IN_SHARED(A);
+    const int lane = threadIdx.x & 31;
     unsigned int sb = A->w_sb;
-    int i = A->w_found ? n : A->w_i;
-    A->w_need = -1;
-    Item nx = A->items[min(i, n)];
-    while (i < n) {
-        const Item it = nx;
-        nx = A->items[i + 1];
-        const unsigned int jb = it.meta & 0xffu, kind = it.meta >> 8, e = sb >> 23;
-        unsigned int to = sb + it.ka;
-        bool ok = kind != K_STEP && e == jb && (to >> 23) == jb;
-        if (kind == K_DUAL && e == jb + 1u) { to = sb + it.kb; ok = (to >> 23) == e; }
-        if (ok && !(locate && target < __uint_as_float(to))) { sb = to; i++; continue; }
-        const unsigned int src = A->isrc[i];
-        if ((src & 0xffu) == 255u) { A->w_need = i; break; }
-        run_values(A, sb, A->care + (src & 0xffu) * 32, (int)(it.oc & 0xffffu), (int)(it.oc >> 16), (int)(src >> 8), locate, target);
-        i++;
-        if (A->w_found) break;
+    int i = A->w_found ? n : A->w_i, need = -1;
+    bool found = false;
+    while (i < n && need < 0 && !found) {
+        const int i0 = i;
+        Item it;
+        it.ka = 0u; it.kb = 0u; it.meta = 0u; it.oc = 0u;
+        if (i0 + lane < n) it = A->items[i0 + lane];
+        const unsigned int jb = it.meta & 0xffu, kind = it.meta >> 8;
+        const bool exists = i0 + lane < n;
+        const unsigned int incl = warp_incl_scan(kind == K_RUN ? it.ka : 0u, lane);
+        int at = 0;
+        unsigned int base = 0u;      // units of the runs before `at`
+        while (at < 32 && i0 + at < n && need < 0 && !found) {
+            const unsigned int j = sb >> 23, to = sb + (incl - base);
+            const bool fits = exists && kind == K_RUN && jb == j && (to >> 23) == j && !(locate && target < __uint_as_float(to));
+            const unsigned int stop = ~__ballot_sync(0xffffffffu, fits) & ~((1u << at) - 1u);
+            const int f = stop ? __ffs((int)stop) - 1 : 32;
+            if (f > at) { sb = __shfl_sync(0xffffffffu, to, f - 1); at = f; }
+            if (at >= 32 || i0 + at >= n) break;
+            const unsigned int ka = __shfl_sync(0xffffffffu, it.ka, at), kb = __shfl_sync(0xffffffffu, it.kb, at);
+            const unsigned int meta = __shfl_sync(0xffffffffu, it.meta, at), oc = __shfl_sync(0xffffffffu, it.oc, at);
+            base = __shfl_sync(0xffffffffu, incl, at);
+            const unsigned int kd = meta >> 8, jx = meta & 0xffu, e = sb >> 23;
+            bool ok = false;
+            unsigned int nx = sb;
+            if (kd == K_DUAL) {
+                if (e == jx) { nx = sb + ka; ok = (nx >> 23) == e; }
+                else if (e == jx + 1u) { nx = sb + kb; ok = (nx >> 23) == e; }
+            }
+            if (ok && !(locate && target < __uint_as_float(nx))) { sb = nx; at++; continue; }
+            const unsigned int src = A->isrc[i0 + at];
+            if ((src & 0xffu) == 255u) { need = i0 + at; break; }
+            const int hit = run_values(sb, A->care + (src & 0xffu) * 32, (int)(oc & 0xffffu), locate, target);
+            at++;
+            if (hit >= 0) {
+                found = true;
+                if (lane == 0) { A->w_found = 1; A->w_tile = (int)(src >> 8); A->w_at = (int)(oc >> 16) + hit; }
+            }
+        }
+        i = i0 + at;
     }
-    A->w_sb = sb; A->w_i = i;
+    if (lane == 0) { A->w_sb = sb; A->w_i = i; A->w_need = need; }
 }
 
 // The exact sequential fp32 sum over the row's items (A->tni of each tile in the row's item space).
@@ -947,47 +986,58 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
         const int n = min(ITEM_CAP, total - b0);
         __syncthreads();
         if (c.tid == 0) { A->ncare = 0; A->w_i = 0; }
-        for (int t = c.tid; t < R.ntile; t += NT) {
-            const int o = A->toff[t] - b0, m = A->tni[t];
-            for (int j = max(0, -o); j < m && o + j < n; j++) {
-                A->items[o + j] = c.gitems[(size_t)t * ITEMS_PER_TILE + j];
-                A->isrc[o + j] = ((unsigned int)t << 8) | 255u;
-            }
-        }
         __syncthreads();
-        for (int i = c.tid; i < n; i += NT)
-            if ((A->items[i].meta >> 8) != K_RUN) {
-                const int s = satom_add(&A->ncare, 1);
-                if (s < CARE_CAP) { A->careidx[s] = (unsigned short)i; A->isrc[i] = (A->isrc[i] & ~0xffu) | (unsigned int)s; }
+        // an item per thread: its tile is found in the tiles' offsets
+        for (int i = c.tid; i < n; i += NT) {
+            int lo = 0, hi = R.ntile - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (A->toff[mid] <= b0 + i) lo = mid; else hi = mid - 1;
             }
+            const Item it = c.gitems[(size_t)lo * ITEMS_PER_TILE + (b0 + i - A->toff[lo])];
+            unsigned int slot = 255u;
+            if ((it.meta >> 8) != K_RUN) {
+                const int q = satom_add(&A->ncare, 1);
+                if (q < CARE_CAP) { slot = (unsigned int)q; A->careidx[q] = (unsigned short)i; }
+            }
+            A->items[i] = it;
+            A->isrc[i] = ((unsigned int)lo << 8) | slot;
+        }
         __syncthreads();
         const int ncare = min(A->ncare, CARE_CAP);
-        for (int s = c.warp; s < ncare; s += NWARP) {
-            const int i = A->careidx[s];
+        for (int q = c.warp; q < ncare; q += NWARP) {
+            const int i = A->careidx[q];
             const unsigned int oc = A->items[i].oc, t = A->isrc[i] >> 8;
-            if (c.lane < (int)(oc & 0xffffu)) A->care[s * 32 + c.lane] = c.list[(size_t)t * TILE + (oc >> 16) + c.lane];
+            A->care[q * 32 + c.lane] = c.lane < (int)(oc & 0xffffu) ? c.list[(size_t)t * TILE + (oc >> 16) + c.lane] : 0.0f;
         }
+        FCOUNT(20, n); FCOUNT(21, ncare); if (!locate) FSTAMP(2);
         for (int round = 0; round <= n; round++) {   // (each round but the last is for one more item)
             __syncthreads();
-            if (c.tid == 0) run_items(A, n, locate, target);
+            if (c.warp == 0) run_items(A, n, locate, target);
             __syncthreads();
             const int want = A->w_need;
             if (want < 0 || A->w_found) break;
             // a run whose guess was wrong, or that holds the target: its values, one by one
             const Item it = A->items[want];
             const int t = (int)(A->isrc[want] >> 8), off = (int)(it.oc >> 16), m = (int)(it.oc & 0xffffu);
-            const float *v = A->ebuf;
+            FCOUNT(23, 1);
             if ((c.pl.flags & F_LIST) || (it.meta >> 8) != K_RUN) {
-                for (int i = c.tid; i < m; i += NT) A->ebuf[i] = c.list[(size_t)t * TILE + off + i];
-                __syncthreads();
+                for (int i = c.tid; i < ((m + 7) & ~7); i += NT) A->ebuf[i] = i < m ? c.list[(size_t)t * TILE + off + i] : 0.0f;
             } else {
                 tile_again(c, t, t + 1, A->ebuf, false);
-                v = A->ebuf + off;
+                float x[TILE / NT];
+                for (int i = c.tid, u = 0; u < TILE / NT; i += NT, u++) x[u] = i < m ? A->ebuf[off + i] : 0.0f;
+                __syncthreads();
+                for (int i = c.tid, u = 0; u < TILE / NT; i += NT, u++) A->ebuf[i] = x[u];
             }
-            if (c.tid == 0) {
+            __syncthreads();
+            if (c.warp == 0) {
                 unsigned int sb = A->w_sb;
-                run_values(A, sb, v, m, off, t, locate, target);
-                A->w_sb = sb; A->w_i = want + 1;
+                const int hit = run_values(sb, A->ebuf, m, locate, target);
+                if (c.lane == 0) {
+                    A->w_sb = sb; A->w_i = want + 1;
+                    if (hit >= 0) { A->w_found = 1; A->w_tile = t; A->w_at = off + hit; }
+                }
             }
         }
         if (A->w_found) break;
@@ -1012,6 +1062,72 @@ __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
             f(eb, t * TILE + i0, src + i0);
         }
     }
+}
+
+// Sorts A->cand[0..n) (descending value, ascending id) and leaves the values in A->pc, padded with zeros
+// to a multiple of eight. Short lists: every key counts the keys above it. Longer ones go through bins of
+// value first (a few keys each: about four keys to a bin at n = 1400) and count within their bin: 1.4 us
+// for 1400 keys, where a sorting network over the block took 17 us.
+__device__ __noinline__ void sort_head(CtxF &c, int n) {
+    AuxF *A = c.A;
+    IN_SHARED(A);
+    __syncthreads();
+    if (n <= 96) {
+        const unsigned long long mine = (c.tid < n) ? A->cand[c.tid] : 0ull;
+        int rank = 0;
+        if (c.tid < n)
+            for (int j = 0; j < n; j++) rank += A->cand[j] > mine ? 1 : 0;
+        __syncthreads();
+        if (c.tid < n) { A->cand[rank] = mine; A->pc[rank] = key_val(mine); }
+    } else {
+        constexpr int KPT = NC / NT;
+        unsigned long long k[KPT];
+        unsigned int lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+        for (int u = 0; u < KPT; u++) {
+            const int i = c.tid + u * NT;
+            k[u] = i < n ? A->cand[i] : 0ull;
+            if (i < n) { lo = min(lo, (unsigned int)(k[u] >> 32)); hi = max(hi, (unsigned int)(k[u] >> 32)); }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (c.lane == 0) { A->wsi[c.warp] = (int)lo; A->wsf[c.warp] = __uint_as_float(hi); }
+#pragma unroll
+        for (int i = 0; i < BPT; i++) A->sbin[c.tid + i * NT] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NWARP; w++) { lo = min(lo, (unsigned int)A->wsi[w]); hi = max(hi, __float_as_uint(A->wsf[w])); }
+        const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
+        unsigned int bin[KPT], slot[KPT];
+#pragma unroll
+        for (int u = 0; u < KPT; u++) {
+            bin[u] = NBINS - 1 - (((unsigned int)(k[u] >> 32) - lo) >> shift);   // descending
+            if (c.tid + u * NT < n) slot[u] = atomicAdd(&A->sbin[bin[u]], 1u);
+        }
+        __syncthreads();
+        unsigned int cnt[BPT], sum = 0u, tot;
+#pragma unroll
+        for (int i = 0; i < BPT; i++) { cnt[i] = A->sbin[BPT * c.tid + i]; sum += cnt[i]; }
+        unsigned int at = block_excl_scan<unsigned int>(sum, reinterpret_cast<unsigned int *>(A->wsi), &tot);
+#pragma unroll
+        for (int i = 0; i < BPT; i++) { A->sbin[BPT * c.tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (c.tid + u * NT < n) A->tmp[(A->sbin[bin[u]] & 0xffffu) + slot[u]] = k[u];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (c.tid + u * NT < n) {
+                const unsigned int b = A->sbin[bin[u]], b0 = b & 0xffffu, m = b >> 16;
+                unsigned int rank = b0;
+                for (unsigned int j = 0; j < m; j++) rank += A->tmp[b0 + j] > k[u] ? 1u : 0u;
+                A->cand[rank] = k[u];
+                A->pc[rank] = key_val(k[u]);
+            }
+    }
+    if (c.tid < 8 && n + c.tid < NC) A->pc[n + c.tid] = 0.0f;
+    __syncthreads();
 }
 
 // More candidates than the head holds (few lanes for a wide top-k, or many equal values): a finer
@@ -1121,6 +1237,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         lvl = rs.lvl; lo = rs.lo; shift = rs.shift; tie_mode = rs.tie_mode != 0;
     }
     for (int phase = 0; phase < 8192; phase++) {
+        FCOUNT(22, 1);
         const bool reuse = resumed && phase == 0;  // this phase's tables stand already
         __syncthreads();
         if (!reuse) {
@@ -1372,7 +1489,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             w.tau = blo;
             continue;
         }
-        sort_cands(c, nb);
+        sort_head(c, nb);
         walk_sorted(c, nb, s_bin, pos_bin, x_ge, x_gt, counting, nstop);
         w.s = A->b_s; w.pos = A->b_pos; w.tau = blo;
         const int ev = A->b_event;
@@ -1401,7 +1518,8 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
     c.pl = R.plan[c.rr];
     if (c.pl.kind == PLAN_DONE) return;
     const BatchArgs &a = R.a;
-    c.cfg = row_cfg(a, c.r);
+    FSTAMP(0);
+    c.cfg = c.pl.c;
     c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
     c.gitems = R.items + (size_t)c.rr * R.ntile * ITEMS_PER_TILE;
     c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
@@ -1426,10 +1544,12 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
 
     float dZ = 0.0f, dsum = 0.0f, dtarget = 0.0f, dp = 0.0f;
     int token = -1;
-    auto finish = [&]() { if (c.tid == 0) finish_row(a, c.r, g, c.status, token, dZ, dsum, dtarget, dp); };
+    auto finish = [&]() { FSTAMP(10); if (c.tid == 0) finish_row(a, c.r, g, c.status, token, dZ, dsum, dtarget, dp); };
 
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
+    FSTAMP(1);
     const float Z = exact_sum(c, false, 0.0f);
+    FSTAMP(3);
     dZ = Z;
     const float yZ = __fdiv_rn(1.0f, Z);
     const float u01 = draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull);
@@ -1548,7 +1668,8 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
             A->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(kk), Z, yZ)) << 32) | (kk & 0xFFFFFFFFull);
         }
     }
-    sort_cands(c, nc);
+    FSTAMP(4);
+    sort_head(c, nc);
     for (int i = c.tid; i < nc; i += NT) {
         const float p = A->pc[i];
         const bool eq = (i > 0 && A->pc[i - 1] == p) || (i + 1 < nc && A->pc[i + 1] == p);
@@ -1563,28 +1684,30 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
 #endif
     const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST);
     const bool typ_on = g.typ < 1.0f;
+    FSTAMP(5);
     if (c.tid == 0) {
         float s = 0.0f;
         int cut = -1, tie = 0;
         bool by_mass = false;
-        // the prefix sums of the sorted head (sample.mojo:497-506), eight loads ahead of the
-        // additions; at most n_use elements are added
+        // the prefix sums of the sorted head (sample.mojo:497-506), eight at a time; at most n_use
+        // elements are added
         const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
-        int i = 0;
-        while (i < lim && cut < 0) {
-            float v[8];
-            const int m = min(8, lim - i);
+        for (int i = 0; i < lim && cut < 0; i += 8) {
+            const float4 *p4 = reinterpret_cast<const float4 *>(A->pc + i);
+            const float4 x = p4[0], y = p4[1];
+            const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            float t[8];
 #pragma unroll
-            for (int q = 0; q < 8; q++) v[q] = (q < m) ? A->pc[i + q] : 0.0f;
+            for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
+            float4 *o4 = reinterpret_cast<float4 *>(A->pre + i);
+            o4[0] = make_float4(t[0], t[1], t[2], t[3]);
+            o4[1] = make_float4(t[4], t[5], t[6], t[7]);
+            if (g.topp_on && s >= g.P) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                if (q < m && cut < 0) {
-                    s = __fadd_rn(s, v[q]);
-                    A->pre[i + q] = s;
-                    if (g.topp_on && s >= g.P) { cut = i + q + 1; by_mass = true; }
-                }
+                for (int q = 7; q >= 0; q--)
+                    if (t[q] >= g.P) { cut = i + q + 1; s = t[q]; }   // the first one wins
+                by_mass = true;
             }
-            i += m;
         }
         const long long pos = (cut >= 0) ? (long long)cut : (long long)lim;
         auto equal_next_to = [&](int x) { return (A->hidx[x] & 0x80000000u) != 0u; };
@@ -1603,14 +1726,11 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
         } else if (cut > 0) {
             const float sum = A->pre[cut - 1];
             const float target = __fmul_rn(u01, sum);
-            int at = cut - 1;
-            for (int i0 = 0; i0 < cut && at == cut - 1; i0 += 8) {
-                float v[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) v[q] = (i0 + q < cut) ? A->pre[i0 + q] : 0.0f;
-#pragma unroll
-                for (int q = 7; q >= 0; q--)
-                    if (i0 + q < cut && target < v[q]) at = i0 + q;  // the first one wins
+            // the first prefix sum above the target (they never fall), or the last one kept
+            int at = 0, hi = cut - 1;
+            while (at < hi) {
+                const int mid = (at + hi) >> 1;
+                if (target < A->pre[mid]) hi = mid; else at = mid + 1;
             }
             A->b_event = EV_DRAW; A->b_idx = (int)(A->hidx[at] & 0x7fffffffu); A->b_p = A->pc[at];
             if (narrow ? equal_next_to(at) : ((at > 0 && A->pc[at - 1] == A->pc[at]) || (at + 1 < cut && A->pc[at + 1] == A->pc[at])))
@@ -1620,6 +1740,7 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
         A->b_aux = tie;
     }
     __syncthreads();
+    FSTAMP(6);
     c.status |= (unsigned int)A->b_aux;
     const float head_s = A->b_s;
     const long long head_pos = A->b_pos;
@@ -1651,6 +1772,7 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
             if (eb[u]) src[u * 32 + c.lane] = eb[u] >= tau_bits ? 0.0f : prob_of(__uint_as_float(eb[u]), Z, yZ);
     });
     __syncthreads();
+    FSTAMP(7);
     const bool limited = n_use < (long long)a.V;
     FWalk w;
     FResume resume;
@@ -1665,6 +1787,7 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
         const bool cut_round = leg == 0;
         descend_list(c, w, (cut_round && g.topp_on) ? g.P : 3.4e38f, cut_round ? 3.4e38f : target,
                      (cut_round && limited) ? n_use : -1, resume, !cut_round);
+        FSTAMP(8 + leg);
         if (!cut_round) {
             if (w.event == EV_DRAW) {
                 token = token_of(c, w.idx); dp = w.p; resolved = true;
@@ -1805,7 +1928,6 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     A.a.Vg = a.V; A.a.col0 = 0; A.a.mode = 0;
     A.ntile = (a.V + TILE - 1) / TILE;
     A.nspan = (a.V + SPAN - 1) / SPAN;
-    A.glog = A.ntile * 32 <= PLAN_GROUPS ? 0 : 2;
     narrow_layout(a.V, a.B, sms, A.oG, A.oVc, A.oL);
     const int rows = rows_in_flight(a.B, a.V);
     lay_out(A, (char *)d_workspace, rows, a.V);
