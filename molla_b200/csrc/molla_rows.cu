@@ -35,6 +35,7 @@ constexpr int ITEMS_PER_TILE = 66;         // a run and a careful chunk per lane
 constexpr int HEADCAP = 2048;              // candidates of the sorted head at most
 constexpr int HEAD_MOST = 1026;            // the sorted head covers top-k + 1 up to this many
 constexpr int ITEM_CAP = 384;              // items of a row that fit shared memory
+constexpr int CARE_PLACES = 192;           // careful chunks of a row whose values are handed on with the items
 constexpr int CARE_CAP = 48;               // careful chunks whose entries are fetched ahead
 constexpr int TIE_CAP = 64;                // rounding ties a walk resolves by parity; more send it the slow way
 constexpr int PLAN_BINS = 1024;            // row_plan: bins of the lanes' maxima by distance below the row's,
@@ -45,7 +46,7 @@ enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8 };
 
 struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
 struct __align__(8) TilePlan { float thr, est; };
-struct __align__(16) TileOut { unsigned int emax; float esum; unsigned short cnt, nitem; unsigned int pad; };
+struct __align__(8) TileOut { unsigned int ioff; unsigned short cnt, nitem; };   // its items in the row's, entries in its list
 
 // Items: the exact sequential sum of a tile's values as a short program. While the running sum s
 // stays in one binade, fl(s + v) is s plus rne(v / ulp) units, an integer that does not depend on s;
@@ -58,8 +59,15 @@ struct __align__(16) TileOut { unsigned int emax; float esum; unsigned short cnt
 enum { K_RUN = 0, K_DUAL = 1, K_STEP = 2 };
 struct __align__(16) Item {
     unsigned int ka, kb;   // units of binade jb (RUN, DUAL) and of the next one (DUAL)
-    unsigned int meta;     // biased exponent of the binade (8 bits), kind (2 bits)
-    unsigned int oc;       // first entry in the tile's list << 16 | entries
+    unsigned int meta;     // biased exponent of the binade (8 bits), kind (2), place of the values (8; 255: the list), tile (10)
+    unsigned int oc;       // entries (11 bits), first entry in the tile's list (10), number of the item in its tile (7)
+    __device__ __forceinline__ unsigned int jb() const { return meta & 0xffu; }
+    __device__ __forceinline__ unsigned int kind() const { return (meta >> 8) & 3u; }
+    __device__ __forceinline__ unsigned int place() const { return (meta >> 10) & 0xffu; }
+    __device__ __forceinline__ int tile() const { return (int)(meta >> 18); }
+    __device__ __forceinline__ int cnt() const { return (int)(oc & 0x7ffu); }
+    __device__ __forceinline__ int off() const { return (int)((oc >> 11) & 0x3ffu); }
+    __device__ __forceinline__ int num() const { return (int)(oc >> 21); }
 };
 
 // ---- settings ---------------------------------------------------------------------------------
@@ -76,6 +84,10 @@ struct __align__(16) RowCfg {
 // What row_plan hands to the kernels behind it.
 struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; int pad; };
 
+// A row's small results, together in memory: the kernels that read them wait once.
+//   RowHead | TileOut[ntile] | candidates[HEADCAP] | prefix sums[HEADCAP] | values of careful chunks[CARE_PLACES][32] | items
+struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; int pad[4]; };
+
 struct RowsArgs {
     BatchArgs a;
     int r0, rows;            // batch rows [r0, r0 + rows) are in flight
@@ -84,13 +96,16 @@ struct RowsArgs {
     TileStat *ts;            // [rows][ntile]
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
     TilePlan *tp;            // [rows][ntile]
-    RowPlan *plan;           // [rows]
-    int *ncand;              // [rows]
-    unsigned long long *cand;  // [rows][HEADCAP]
-    TileOut *to;             // [rows][ntile]
-    Item *items;             // [rows][ntile][ITEMS_PER_TILE]
+    char *box; long long box_stride;  // [rows]
+    int *queue;              // rows for row_tail: their number, then the rows
     float *elist;            // [rows][ntile][TILE] values kept, in vocabulary order, packed per tile
     unsigned int *kmask;     // [rows][ntile][32] which logits they are
+    __device__ __forceinline__ RowHead *head(int rr) const { return reinterpret_cast<RowHead *>(box + (long long)rr * box_stride); }
+    __device__ __forceinline__ TileOut *to(int rr) const { return reinterpret_cast<TileOut *>(head(rr) + 1); }
+    __device__ __forceinline__ unsigned long long *cand(int rr) const { return reinterpret_cast<unsigned long long *>(to(rr) + ((ntile + 1) & ~1)); }
+    __device__ __forceinline__ float *pre(int rr) const { return reinterpret_cast<float *>(cand(rr) + HEADCAP); }
+    __device__ __forceinline__ float *care(int rr) const { return pre(rr) + HEADCAP; }
+    __device__ __forceinline__ Item *items(int rr) const { return reinterpret_cast<Item *>(care(rr) + CARE_PLACES * 32); }
 };
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -412,6 +427,13 @@ __device__ __forceinline__ float block_excl_scan_plus(float v, float *ws, float 
     return b + ex;
 }
 
+__device__ __forceinline__ void store_plan(const RowsArgs &A, int rr, const RowPlan &pl) {
+    RowHead *h = A.head(rr);
+    h->plan = pl;
+    h->ncand = 0; h->nitem = 0; h->ncare = 0; h->state = 0;
+    if (rr == 0) A.queue[0] = 0;
+}
+
 __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ RowsArgs A) {
     __shared__ PlanShared S;
     pdl_next();
@@ -424,7 +446,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     pl.c = c;
     pl.kind = PLAN_DONE; pl.flags = 0; pl.top = 0; pl.tau_bits = 1u; pl.xmax = 0; pl.imax = 0; pl.need = 0; pl.pad = 0;
     if (c.status) {
-        if (tid == 0) { finish_row(a, r, c, c.status, -1, 0, 0, 0, 0); A.plan[rr] = pl; }
+        if (tid == 0) { finish_row(a, r, c, c.status, -1, 0, 0, 0, 0); store_plan(A, rr, pl); }
         return;
     }
     // the maximum and its first index (kernel.mojo:571-585, sample.mojo:342-346)
@@ -465,7 +487,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         if (eq > 1) status |= MOLLA_ROW_TOPK_TIE;
     }
     if (done) {
-        if (tid == 0) { finish_row(a, r, c, status, imax, 0, 0, 0, 0); A.plan[rr] = pl; }
+        if (tid == 0) { finish_row(a, r, c, status, imax, 0, 0, 0, 0); store_plan(A, rr, pl); }
         return;
     }
     const float top = (c.T == 1.0f) ? xmax : __fdiv_rn(xmax, c.T);
@@ -568,8 +590,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
                    ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
         pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
         pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
-        A.plan[rr] = pl;
-        A.ncand[rr] = 0;
+        store_plan(A, rr, pl);
     }
 }
 
@@ -579,7 +600,10 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
 // The items of a tile whose lane `lane` holds `cnt` values v(0..cnt-1) (padded with zeros to a multiple
 // of four), estimated sum before the tile `est`. `off` = the lane's first entry in the tile's list.
 // Returns the number of items; `care` = this lane's values are wanted one by one.
-__device__ __forceinline__ int tile_items(const float *row, int cnt, int off, int total, float csum, float est, Item *out, bool &care) {
+// `alloc(n, c)` is called by all lanes with the number of items and of careful chunks among them and
+// returns where the items go; place(i) says where the i-th careful chunk's values go (255: nowhere).
+template <class ALLOC, class PLACE>
+__device__ __forceinline__ int tile_items(const float *row, int cnt, int off, int total, float csum, float est, int tile, ALLOC alloc, PLACE place, bool &care, int &my_place) {
     const int lane = threadIdx.x & 31;
     const float inc = warp_incl_scan(csum, lane);
     float ex = __shfl_up_sync(0xffffffffu, inc, 1);
@@ -587,7 +611,7 @@ __device__ __forceinline__ int tile_items(const float *row, int cnt, int off, in
     const float sst = est + ex;
     const bool nonempty = cnt > 0 && csum > 0.0f;
     // the estimate counts what was dropped (it adds nothing to the true sum), so it is high rather than low
-    const float lo = sst * (1.0f - 1.0f / 512.0f), hi = (sst + csum) * (1.0f + 1.0f / 2048.0f);
+    const float lo = sst * (1.0f - 1.0f / 256.0f), hi = (sst + csum) * (1.0f + 1.0f / 2048.0f);
     const int jl = fexpo(lo), jh = fexpo(hi);
     const bool usable = nonempty && lo > 0.0f && jh <= jl + 1 && jl >= -100 && jh <= 100;
     const bool two = usable && jh == jl + 1;
@@ -638,55 +662,61 @@ __device__ __forceinline__ int tile_items(const float *row, int cnt, int off, in
     const unsigned int cm = __ballot_sync(0xffffffffu, care);
     const float units = fpow2(max(min(23 - jl, 127), -126));
     const unsigned int ka = (usable && !bad) ? __float2uint_rn(__fmul_rn(da, units)) : 0u;   // da is a multiple of 2^(jl-23), below 2^24 of them
+    my_place = 255;
     if (cm == 0u) {
         const unsigned int k = __reduce_add_sync(0xffffffffu, ka);
         if (k == 0u) return 0;
         const int j0 = __shfl_sync(0xffffffffu, jl, __ffs((int)ne) - 1);
+        Item *out = alloc(1, 0);
         if (lane == 0) {
             Item it;
-            it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8); it.oc = (unsigned int)total;
+            it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18); it.oc = (unsigned int)total;
             out[0] = it;
         }
         return 1;
     }
-    int n = 0;
-    unsigned int left = cm;
-    int from = 0;
-    for (int round = 0; round < 33; round++) {
-        const int cl = left ? __ffs((int)left) - 1 : 32;
-        const unsigned int span = (cl == 32 ? 0xffffffffu : ((1u << cl) - 1u)) & ~((from == 0) ? 0u : (from == 32 ? 0xffffffffu : ((1u << from) - 1u)));
-        const unsigned int in = span & ne;
-        if (in) {
-            const unsigned int k = __reduce_add_sync(0xffffffffu, ((in >> lane) & 1u) ? ka : 0u);
-            if (k) {
-                const int l0 = __ffs((int)in) - 1, l1 = 31 - __clz((int)in);
-                const int j0 = __shfl_sync(0xffffffffu, jl, l0), o0 = __shfl_sync(0xffffffffu, off, l0), o1 = __shfl_sync(0xffffffffu, off + cnt, l1);
-                if (lane == 0) {
-                    Item it;
-                    it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8); it.oc = ((unsigned int)o0 << 16) | (unsigned int)(o1 - o0);
-                    out[n] = it;
-                }
-                n++;
-            }
+    // the runs between the careful lanes: a run goes with the careful lane behind it, or closes the tile
+    const unsigned int kin = warp_incl_scan(care ? 0u : ka, lane);
+    const unsigned int lt = (1u << lane) - 1u, cb = cm & lt;
+    const int lastc = cb ? 31 - __clz((int)cb) : -1, last = 31 - __clz((int)cm);
+    const unsigned int kprev = __shfl_sync(0xffffffffu, kin, lastc < 0 ? 0 : lastc);
+    const unsigned int kin_up = __shfl_up_sync(0xffffffffu, kin, 1);
+    const unsigned int kr = (lane == 0 ? 0u : kin_up) - (lastc < 0 ? 0u : kprev);   // units of the run that ends before this lane
+    const unsigned int runm = __ballot_sync(0xffffffffu, care && kr != 0u);          // careful lanes with a run before them
+    const unsigned int ktail = __shfl_sync(0xffffffffu, kin, 31) - __shfl_sync(0xffffffffu, kin, last);
+    const int ncare = __popc(cm), n = ncare + __popc(runm) + (ktail ? 1 : 0);
+    Item *out = alloc(n, ncare);
+    // the first lane of a run that holds anything, for its binade and its first entry
+    auto first_in = [&](int from) { const unsigned int m = ne & ~(from < 0 ? 0u : (from == 31 ? 0xffffffffu : ((2u << from) - 1u))); return m ? __ffs((int)m) - 1 : 31; };
+    const int fl = first_in(lastc), tl = first_in(last);
+    const int fj = __shfl_sync(0xffffffffu, jl, fl), fo = __shfl_sync(0xffffffffu, off, fl);
+    const int tj = __shfl_sync(0xffffffffu, jl, tl), to = __shfl_sync(0xffffffffu, off, tl);
+    if (care) {
+        int i = __popc(cb) + __popc(runm & lt);
+        Item it;
+        if ((runm >> lane) & 1u) {
+            it.ka = kr; it.kb = 0; it.meta = (unsigned int)(fj + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18);
+            it.oc = (unsigned int)(off - fo) | ((unsigned int)fo << 11) | ((unsigned int)i << 21);
+            out[i++] = it;
         }
-        if (cl == 32) break;
-        if (lane == cl) {
-            Item it;
-            const bool dual = two && !bad;
-            it.ka = dual ? ka : 0u;
-            it.kb = dual ? __float2uint_rn(__fmul_rn(db, fpow2(max(min(22 - jl, 127), -126)))) : 0u;
-            it.meta = dual ? ((unsigned int)(jl + 127) | (K_DUAL << 8)) : (unsigned int)(K_STEP << 8);
-            it.oc = ((unsigned int)off << 16) | (unsigned int)cnt;
-            out[n] = it;
-        }
-        n++;
-        from = cl + 1;
-        left &= left - 1u;
+        my_place = place(__popc(cb));
+        const bool dual = two && !bad;
+        it.ka = dual ? ka : 0u;
+        it.kb = dual ? __float2uint_rn(__fmul_rn(db, fpow2(max(min(22 - jl, 127), -126)))) : 0u;
+        it.meta = (dual ? ((unsigned int)(jl + 127) | (K_DUAL << 8)) : (unsigned int)(K_STEP << 8)) | ((unsigned int)my_place << 10) | ((unsigned int)tile << 18);
+        it.oc = (unsigned int)cnt | ((unsigned int)off << 11) | ((unsigned int)i << 21);
+        out[i] = it;
+    }
+    if (ktail && lane == 0) {
+        Item it;
+        it.ka = ktail; it.kb = 0; it.meta = (unsigned int)(tj + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18);
+        it.oc = (unsigned int)(total - to) | ((unsigned int)to << 11) | ((unsigned int)(n - 1) << 21);
+        out[n - 1] = it;
     }
     return n;
 }
 
-struct TileEval { int cnt, off, total; unsigned int keep; float csum; unsigned int emax; };
+struct TileEval { int cnt, off, total; unsigned int keep; float csum; };
 
 // The exponentials (temperature and softmax numerator, sample.mojo:419-434) of a tile's logits that
 // reach `thr`, packed to the front of every lane's own part of shared memory.
@@ -700,7 +730,7 @@ __device__ __forceinline__ TileEval tile_eval(float *mine, float thr, float T, f
         m |= (v.x >= thr ? 1u : 0u) << (4 * g) | (v.y >= thr ? 1u : 0u) << (4 * g + 1) | (v.z >= thr ? 1u : 0u) << (4 * g + 2) | (v.w >= thr ? 1u : 0u) << (4 * g + 3);
     }
     TileEval r;
-    r.cnt = 0; r.keep = 0; r.csum = 0.0f; r.emax = 0;
+    r.cnt = 0; r.keep = 0; r.csum = 0.0f;
     const bool one = T == 1.0f;
     for (int round = 0; round < 32 && __any_sync(0xffffffffu, m != 0u); round++) {
         if (m) {
@@ -715,7 +745,6 @@ __device__ __forceinline__ TileEval tile_eval(float *mine, float thr, float T, f
                 r.csum += e;
                 r.keep |= 1u << b;
                 const unsigned int eb = __float_as_uint(e);
-                r.emax = max(r.emax, eb);
                 take(eb, lane * 32 + b);
             }
         }
@@ -753,7 +782,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     pdl_next();
     pdl_wait();
     const int rr = blockIdx.x / A.nspan, span = blockIdx.x - rr * A.nspan, r = A.r0 + rr;
-    const RowPlan pl = A.plan[rr];
+    RowHead *head = A.head(rr);
+    const RowPlan pl = head->plan;
     if (pl.kind == PLAN_DONE) return;
     const BatchArgs &a = A.a;
     const RowCfg &c = pl.c;
@@ -764,30 +794,407 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     const TilePlan tp = A.tp[gt];
     float *mine = S->x + threadIdx.x * PITCH;
     const unsigned int tau = pl.tau_bits;
-    unsigned long long *cand = A.cand + (size_t)rr * HEADCAP;
+    unsigned long long *cand = A.cand(rr);
     const TileEval t = tile_eval(mine, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
         [&](unsigned int eb, int i) {
             if (eb >= tau) {
-                const int pos = atomicAdd(&A.ncand[rr], 1);
+                const int pos = atomicAdd(&head->ncand, 1);
                 if (pos < HEADCAP) cand[pos] = make_key(eb, tile * TILE + i);
             }
         });
     bool care;
-    const int ni = tile_items(mine, t.cnt, t.off, t.total, t.csum, tp.est, A.items + gt * ITEMS_PER_TILE, care);
-    const unsigned int lanes = (pl.flags & F_LIST) ? 0xffffffffu : __ballot_sync(0xffffffffu, care);
+    int my_place, c0 = CARE_PLACES;
+    unsigned int i0 = 0;
+    const int ni = tile_items(mine, t.cnt, t.off, t.total, t.csum, tp.est, tile,
+        [&](int n, int nc) -> Item * {
+            if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, n); if (nc) c0 = atomicAdd(&head->ncare, nc); }
+            i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
+            return A.items(rr) + i0;
+        },
+        [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
+    // the careful lanes' values, padded with zeros
+    for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
+        const int l = __ffs((int)left) - 1, n = __shfl_sync(0xffffffffu, t.cnt, l), at = __shfl_sync(0xffffffffu, my_place, l);
+        A.care(rr)[at * 32 + lane] = lane < n ? S->x[(warp * 32 + l) * PITCH + lane] : 0.0f;
+    }
+    const unsigned int lanes = (pl.flags & F_LIST) ? 0xffffffffu : __ballot_sync(0xffffffffu, care && my_place == 255);
     if (lanes) tile_store(S->x + (size_t)warp * 32 * PITCH, t, A.elist + gt * TILE, lanes);
     if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = t.keep;
-    const float esum = warp_sum(t.csum);
-    const unsigned int emax = __reduce_max_sync(0xffffffffu, t.emax);
     if (lane == 0) {
         TileOut o;
-        o.emax = emax; o.esum = esum; o.cnt = (unsigned short)t.total; o.nitem = (unsigned short)ni; o.pad = 0;
-        A.to[gt] = o;
+        o.ioff = i0; o.cnt = (unsigned short)t.total; o.nitem = (unsigned short)ni;
+        A.to(rr)[tile] = o;
     }
 }
 
 // =============================================================================
-// Kernel 4: one block per sampled row.
+// Kernel 4: one small block per sampled row. The items give the softmax denominator, the candidates the
+// sorted head; most rows end here. Rows that go on (nothing sorted, a nucleus past the head, typical-p,
+// anything unusual) are queued for the last kernel. Bound: the latency of one warp's dependent additions
+// and of one round of loads, so the block is small and four of them share an SM.
+// =============================================================================
+constexpr int HT = 256, HW = HT / 32;
+constexpr int H_ITEMS = 512, H_CARE = 80;
+enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2 };   // what a queued row has: nothing, its denominator, its head too
+
+struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the last of them | kind | own binade | place
+
+struct __align__(16) HeadShared {
+    union {
+        struct { Item items[H_ITEMS]; float care[H_CARE * 32]; CareRec rec[H_CARE + 1]; } w;
+        unsigned int sbin[NBINS];
+    };
+    unsigned long long cand[HEADCAP];
+    union {
+        unsigned long long tmp[HEADCAP];
+        struct { float pc[HEADCAP]; float pre[HEADCAP]; } p;
+    };
+    unsigned short toff[MAX_TILES + 2];
+    unsigned int ws[HW + 1], ws2[HW + 1];
+    float Z; int ok, cut, n_ge;
+};
+
+// exclusive scan over the HT threads
+__device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *ws, unsigned int *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int inc = warp_incl_scan(v, lane);
+    __syncthreads();
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    unsigned int b = 0u, t = 0u;
+#pragma unroll
+    for (int w = 0; w < HW; w++) {
+        if (w == warp) b = t;
+        t += ws[w];
+    }
+    *total = t;
+    return b + inc - v;
+}
+
+// Sorts S->cand[0..n) (descending value, ascending id) and leaves the values in S->p.pc, padded with zeros
+// to a multiple of eight. Up to HT keys: every key counts the keys above it. More go through bins of value
+// first (a few keys each) and count within their bin.
+__device__ void head_sort(HeadShared *S, int n) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int KPT = HEADCAP / HT, PER = NBINS / HT;
+    if (n <= HT) {
+        const unsigned long long mine = tid < n ? S->cand[tid] : 0ull;
+        int rank = 0;
+        if (warp * 32 < n) {
+            int j = 0;
+            for (; j + 4 <= n; j += 4) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(S->cand + j), b = *reinterpret_cast<const ulonglong2 *>(S->cand + j + 2);
+                rank += (a.x > mine ? 1 : 0) + (a.y > mine ? 1 : 0) + (b.x > mine ? 1 : 0) + (b.y > mine ? 1 : 0);
+            }
+            for (; j < n; j++) rank += S->cand[j] > mine ? 1 : 0;
+        }
+        __syncthreads();
+        if (tid < n) { S->cand[rank] = mine; S->p.pc[rank] = key_val(mine); }
+    } else {
+        unsigned long long k[KPT];
+        unsigned int lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+        for (int u = 0; u < KPT; u++) {
+            const int i = tid + u * HT;
+            k[u] = i < n ? S->cand[i] : 0ull;
+            if (i < n) { lo = min(lo, (unsigned int)(k[u] >> 32)); hi = max(hi, (unsigned int)(k[u] >> 32)); }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) { S->ws[warp] = lo; S->ws2[warp] = hi; }
+#pragma unroll
+        for (int i = 0; i < PER; i++) S->sbin[tid + i * HT] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < HW; w++) { lo = min(lo, S->ws[w]); hi = max(hi, S->ws2[w]); }
+        const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
+        unsigned int slot[KPT];
+        auto bin_of = [&](unsigned long long key) { return NBINS - 1 - (((unsigned int)(key >> 32) - lo) >> shift); };   // descending
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * HT < n) slot[u] = atomicAdd(&S->sbin[bin_of(k[u])], 1u);
+        __syncthreads();
+        unsigned int cnt[PER], sum = 0u, tot;
+#pragma unroll
+        for (int i = 0; i < PER; i++) { cnt[i] = S->sbin[PER * tid + i]; sum += cnt[i]; }
+        unsigned int at = head_scan(sum, S->ws, &tot);
+#pragma unroll
+        for (int i = 0; i < PER; i++) { S->sbin[PER * tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * HT < n) S->tmp[(S->sbin[bin_of(k[u])] & 0xffffu) + slot[u]] = k[u];
+        __syncthreads();
+        unsigned int rank[KPT];
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * HT < n) {
+                const unsigned int b = S->sbin[bin_of(k[u])], b0 = b & 0xffffu, m = b >> 16;
+                rank[u] = b0;
+                for (unsigned int j = 0; j < m; j++) rank[u] += S->tmp[b0 + j] > k[u] ? 1u : 0u;
+            }
+        __syncthreads();   // the values take the space of the keys being read
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * HT < n) { S->cand[rank[u]] = k[u]; S->p.pc[rank[u]] = key_val(k[u]); }
+    }
+    if (tid < 8 && n + tid < HEADCAP) S->p.pc[n + tid] = 0.0f;
+    __syncthreads();
+}
+
+// One warp, all lanes alike: the sum through the careful chunks S->w.rec[0..nrec) and the runs between
+// them. Returns false where a run's binade was guessed wrong.
+__device__ bool walk_records(const HeadShared *S, int nrec, float &Z) {
+    unsigned int sb = 0u, kdone = 0u;
+    CareRec nx = S->w.rec[0];
+    for (int q = 0; q <= nrec; q++) {
+        const CareRec r = nx;
+        const float4 *v = reinterpret_cast<const float4 *>(S->w.care + ((r.meta >> 24) & 0xffu) * 32);
+        const unsigned int kind = (r.meta >> 8) & 3u;
+        float4 x[8];
+        if (q < nrec && kind != K_RUN) {   // asked for before it is known whether they are needed
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = v[i];
+        }
+        nx = S->w.rec[q < nrec ? q + 1 : q];
+        const unsigned int kx = r.k - kdone;
+        kdone = r.k;
+        if (kx) {
+            const unsigned int to = sb + kx, j = r.meta & 0xffu;
+            if ((sb >> 23) != j || (to >> 23) != j) return false;
+            sb = to;
+        }
+        if (q == nrec) break;
+        const unsigned int e = sb >> 23, jb = (r.meta >> 16) & 0xffu;
+        if (kind == K_RUN) {
+            const unsigned int to = sb + r.ka;
+            if (e != jb || (to >> 23) != jb) return false;
+            sb = to;
+            continue;
+        }
+        if (kind == K_DUAL) {
+            const unsigned int to = e == jb ? sb + r.ka : sb + r.kb;
+            if ((e == jb || e == jb + 1u) && (to >> 23) == e) { sb = to; continue; }
+        }
+        float s = __uint_as_float(sb);
+#pragma unroll
+        for (int i = 0; i < 8; i++) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
+        sb = __float_as_uint(s);
+    }
+    Z = __uint_as_float(sb);
+    return true;
+}
+
+__global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__ RowsArgs R) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    HeadShared *S = reinterpret_cast<HeadShared *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rr = blockIdx.x, r = R.r0 + rr;
+    pdl_next();
+    pdl_wait();
+    RowHead *head = R.head(rr);
+    const BatchArgs &a = R.a;
+    const int ntile = R.ntile;
+    // everything that will be wanted, in one round of loads (what lies past the counts is not used)
+    const int ncand = head->ncand, nitem = head->nitem, ncare = head->ncare;
+    const RowPlan &pl = head->plan;
+    const int kind = pl.kind;
+    TileOut to[3];
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+        to[u].nitem = 0;
+        if (3 * tid + u < ntile) to[u] = R.to(rr)[3 * tid + u];
+    }
+    Item it[H_ITEMS / HT];
+#pragma unroll
+    for (int u = 0; u < H_ITEMS / HT; u++) it[u] = R.items(rr)[tid + u * HT];   // (a row has room for more)
+    constexpr int CV = (H_CARE * 8 + HT - 1) / HT;
+    float4 cv[CV];
+#pragma unroll
+    for (int u = 0; u < CV; u++)
+        if (tid + u * HT < H_CARE * 8) cv[u] = reinterpret_cast<const float4 *>(R.care(rr))[tid + u * HT];
+    unsigned long long key = R.cand(rr)[tid];
+    if (kind == PLAN_DONE) return;
+    const RowCfg &g = pl.c;
+    const bool narrow = (pl.flags & F_NARROW) != 0;
+    auto queue_row = [&](int state) {
+        if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
+    };
+    if (nitem > H_ITEMS || ncare > H_CARE || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING); return; }
+    // ---- the items in order, the careful ones among them as records
+    unsigned int total;
+    const unsigned int o = head_scan(to[0].nitem + to[1].nitem + to[2].nitem, S->ws, &total);
+    if (3 * tid < ntile) {
+        S->toff[3 * tid] = (unsigned short)o;
+        S->toff[3 * tid + 1] = (unsigned short)(o + to[0].nitem);
+        S->toff[3 * tid + 2] = (unsigned short)(o + to[0].nitem + to[1].nitem);
+    }
+#pragma unroll
+    for (int u = 0; u < CV; u++)
+        if (tid + u * HT < H_CARE * 8) reinterpret_cast<float4 *>(S->w.care)[tid + u * HT] = cv[u];
+    if (tid == 0) { S->ok = 1; S->n_ge = 0; }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < H_ITEMS / HT; u++)
+        if (tid + u * HT < nitem) S->w.items[S->toff[it[u].tile()] + it[u].num()] = it[u];
+    __syncthreads();
+    unsigned int nrec;
+    {
+        constexpr int IPT = H_ITEMS / HT;
+        bool care[IPT];
+        unsigned int pj[IPT], k = 0u, n = 0u;
+        Item mine[IPT];
+#pragma unroll
+        for (int u = 0; u < IPT; u++) {
+            const int i = IPT * tid + u;
+            care[u] = false; pj[u] = 0u;
+            if (i < nitem) {
+                mine[u] = S->w.items[i];
+                const bool run = mine[u].kind() == K_RUN;
+                bool prev_run = false;
+                if (i > 0) { const Item p = S->w.items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
+                care[u] = !run || (prev_run && pj[u] != mine[u].jb());   // (a change of binade between two runs: a wrong guess)
+                if (care[u]) { n++; if (!run && mine[u].place() >= (unsigned int)H_CARE) S->ok = 0; }
+                else k += mine[u].ka;
+            }
+        }
+        unsigned int ktot;
+        unsigned int kx = head_scan(k, S->ws, &ktot), nx = head_scan(n, S->ws2, &nrec);
+        if (nrec <= (unsigned int)H_CARE) {
+#pragma unroll
+            for (int u = 0; u < IPT; u++)
+                if (IPT * tid + u < nitem) {
+                    if (care[u]) {
+                        CareRec c;
+                        c.k = kx; c.ka = mine[u].ka; c.kb = mine[u].kb;
+                        c.meta = pj[u] | (mine[u].kind() << 8) | (mine[u].jb() << 16) | (mine[u].place() << 24);
+                        S->w.rec[nx++] = c;
+                    } else kx += mine[u].ka;
+                }
+            if (tid == 0) {
+                CareRec c;
+                c.k = ktot; c.ka = c.kb = 0u; c.meta = nitem > 0 ? S->w.items[nitem - 1].jb() : 0u;
+                S->w.rec[nrec] = c;
+            }
+        }
+    }
+    __syncthreads();
+    if (nrec > (unsigned int)H_CARE || !S->ok) { queue_row(ST_NOTHING); return; }
+    __syncthreads();
+    // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
+    if (warp == 0) {
+        float z = 0.0f;
+        const bool fine = walk_records(S, (int)nrec, z);
+        if (lane == 0) { S->Z = z; S->ok = fine ? 1 : 0; }
+    }
+    __syncthreads();
+    if (!S->ok) { queue_row(ST_NOTHING); return; }
+    const float Z = S->Z, yZ = __fdiv_rn(1.0f, Z);
+    if (tid == 0) head->Z = Z;
+    if (g.pure || g.typ < 1.0f) { queue_row(ST_SUM); return; }
+    // ---- sorted order: the head's candidates as probabilities
+    const int nc = ncand;
+    for (int i = tid; i < nc; i += HT) {
+        if (i >= HT) key = R.cand(rr)[i];
+        S->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(key), Z, yZ)) << 32) | (key & 0xFFFFFFFFull);
+    }
+    __syncthreads();
+    head_sort(S, nc);
+    // min-p (sample.mojo:508-523) keeps a prefix of the sorted order: what reaches p_max * min_p
+    long long n_use = g.n_lim;
+    bool all_above = false;   // every candidate does: how many others do is not known here
+    if (g.minp > 0.0f) {
+        const float floor_p = __fmul_rn(__fdiv_rn(expf_pinned(__fsub_rn(pl.top, pl.top)), Z), g.minp);
+        if (!(floor_p >= 2.2e-8f)) {
+            if (tid == 0) finish_row(a, r, g, MOLLA_ROW_UNSUPPORTED | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), -1, Z, 0, 0, 0);
+            return;
+        }
+        int n = 0;
+        for (int i = tid; i < nc; i += HT) n += S->p.pc[i] >= floor_p ? 1 : 0;
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0 && n) atomicAdd(&S->n_ge, n);
+        __syncthreads();
+        const int n_ge = max(1, S->n_ge);
+        all_above = S->n_ge == nc;
+        if (!all_above && n_ge < n_use) n_use = n_ge;
+    }
+#ifdef MOLLA_SAMPLE_TESTING
+    if (a.topk_out) {
+        for (int i = tid; i < a.topk_cap; i += HT)
+            a.topk_out[(long long)r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? key_idx(S->cand[i]) : -1;
+    }
+#endif
+    if (warp == 0) {
+        // the prefix sums of the sorted head (sample.mojo:497-506), eight at a time; at most n_use
+        // elements are added
+        const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST);
+        const bool topp_on = g.topp_on;
+        const float P = g.P;
+        const float *pc = S->p.pc;
+        float *pre = S->p.pre;
+        float s = 0.0f;
+        int cut = -1, tie = 0;
+        bool by_mass = false;
+        const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
+        const float4 *p4 = reinterpret_cast<const float4 *>(pc);
+        float4 x = p4[0], y = p4[1];
+        for (int i = 0; i < lim && cut < 0; i += 8) {
+            const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            if (i + 8 < lim) { x = p4[(i >> 2) + 2]; y = p4[(i >> 2) + 3]; }
+            float t[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
+            if (lane == 0) {
+                float4 *o4 = reinterpret_cast<float4 *>(pre + i);
+                o4[0] = make_float4(t[0], t[1], t[2], t[3]);
+                o4[1] = make_float4(t[4], t[5], t[6], t[7]);
+            }
+            if (topp_on && s >= P) {
+#pragma unroll
+                for (int q = 7; q >= 0; q--)
+                    if (t[q] >= P) { cut = i + q + 1; s = t[q]; }   // the first one wins
+                by_mass = true;
+            }
+        }
+        __syncwarp();
+        const int pos = cut >= 0 ? cut : lim;
+        auto equal_next_to = [&](int i) { return (i > 0 && pc[i - 1] == pc[i]) || (i + 1 < nc && pc[i + 1] == pc[i]); };
+        if (by_mass) {
+            if (narrow ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
+        } else if (lim > 0 && (long long)lim >= n_use) {
+            cut = lim;  // the count limit
+            if (narrow && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
+        }
+        if (cut < 0 && !p3row) cut = nc;  // everything that can matter is in the head
+        if (!narrow && n_use < (long long)a.V && (long long)nc > n_use && pc[n_use] == pc[n_use - 1]) tie |= MOLLA_ROW_TOPK_TIE;
+        if (cut > 0) {
+            const float sum = pre[cut - 1];
+            const float target = __fmul_rn(draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull), sum);
+            // the first prefix sum above the target (they never fall), or the last one kept
+            int at = 0, hi = cut - 1;
+            while (at < hi) {
+                const int mid = (at + hi) >> 1;
+                if (target < pre[mid]) hi = mid; else at = mid + 1;
+            }
+            if (narrow ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at])))
+                tie |= MOLLA_ROW_CHOSEN_TIE;
+            if (lane == 0)
+                finish_row(a, r, g, (unsigned int)tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), key_idx(S->cand[at]), Z, sum, target, pc[at]);
+        } else if (lane == 0) {
+            head->head_s = s; head->head_pos = pos;
+        }
+        if (lane == 0) S->cut = cut;
+    }
+    __syncthreads();
+    if (S->cut > 0) return;
+    if (all_above || nc == 0) { queue_row(ST_SUM); return; }
+    // past the head: the sorted candidates and their prefix sums go along
+    for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
+    queue_row(ST_HEAD);
+}
+
+// =============================================================================
+// Kernel 5: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
+// what it does not.
 // =============================================================================
 struct __align__(16) AuxF {
     union {
@@ -812,6 +1219,7 @@ struct __align__(16) AuxF {
     unsigned short tcnt[MAX_TILES];        // entries in the tile's list
     unsigned short tni[MAX_TILES];         // items of the tile
     int toff[MAX_TILES + 1];               // first item of the tile
+    unsigned int tio[MAX_TILES];           // where its items begin
     float tsum[MAX_TILES];
     double wsd[2 * (NWARP + 1)];
     unsigned long long wsu[NWARP + 1];
@@ -846,7 +1254,7 @@ struct CtxF {
     RowCfg cfg;
     RowPlan pl;
     float *list;                 // this row's [ntile][TILE]
-    Item *gitems;                // this row's [ntile][ITEMS_PER_TILE]
+    Item *gitems;                // this row's items
     const unsigned int *kmask;   // this row's [ntile][32]
 };
 
@@ -928,7 +1336,7 @@ __device__ void run_items(AuxF *A, int n, bool locate, float target) {
         Item it;
         it.ka = 0u; it.kb = 0u; it.meta = 0u; it.oc = 0u;
         if (i0 + lane < n) it = A->items[i0 + lane];
-        const unsigned int jb = it.meta & 0xffu, kind = it.meta >> 8;
+        const unsigned int jb = it.jb(), kind = it.kind();
         const bool exists = i0 + lane < n;
         const unsigned int incl = warp_incl_scan(kind == K_RUN ? it.ka : 0u, lane);
         int at = 0;
@@ -943,7 +1351,7 @@ __device__ void run_items(AuxF *A, int n, bool locate, float target) {
             const unsigned int ka = __shfl_sync(0xffffffffu, it.ka, at), kb = __shfl_sync(0xffffffffu, it.kb, at);
             const unsigned int meta = __shfl_sync(0xffffffffu, it.meta, at), oc = __shfl_sync(0xffffffffu, it.oc, at);
             base = __shfl_sync(0xffffffffu, incl, at);
-            const unsigned int kd = meta >> 8, jx = meta & 0xffu, e = sb >> 23;
+            const unsigned int kd = (meta >> 8) & 3u, jx = meta & 0xffu, e = sb >> 23;
             bool ok = false;
             unsigned int nx = sb;
             if (kd == K_DUAL) {
@@ -953,11 +1361,11 @@ __device__ void run_items(AuxF *A, int n, bool locate, float target) {
             if (ok && !(locate && target < __uint_as_float(nx))) { sb = nx; at++; continue; }
             const unsigned int src = A->isrc[i0 + at];
             if ((src & 0xffu) == 255u) { need = i0 + at; break; }
-            const int hit = run_values(sb, A->care + (src & 0xffu) * 32, (int)(oc & 0xffffu), locate, target);
+            const int hit = run_values(sb, A->care + (src & 0xffu) * 32, (int)(oc & 0x7ffu), locate, target);
             at++;
             if (hit >= 0) {
                 found = true;
-                if (lane == 0) { A->w_found = 1; A->w_tile = (int)(src >> 8); A->w_at = (int)(oc >> 16) + hit; }
+                if (lane == 0) { A->w_found = 1; A->w_tile = (int)(src >> 8); A->w_at = (int)((oc >> 11) & 0x3ffu) + hit; }
             }
         }
         i = i0 + at;
@@ -994,9 +1402,9 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
                 const int mid = (lo + hi + 1) >> 1;
                 if (A->toff[mid] <= b0 + i) lo = mid; else hi = mid - 1;
             }
-            const Item it = c.gitems[(size_t)lo * ITEMS_PER_TILE + (b0 + i - A->toff[lo])];
+            const Item it = c.gitems[A->tio[lo] + (b0 + i - A->toff[lo])];
             unsigned int slot = 255u;
-            if ((it.meta >> 8) != K_RUN) {
+            if (it.kind() != K_RUN) {
                 const int q = satom_add(&A->ncare, 1);
                 if (q < CARE_CAP) { slot = (unsigned int)q; A->careidx[q] = (unsigned short)i; }
             }
@@ -1007,8 +1415,8 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
         const int ncare = min(A->ncare, CARE_CAP);
         for (int q = c.warp; q < ncare; q += NWARP) {
             const int i = A->careidx[q];
-            const unsigned int oc = A->items[i].oc, t = A->isrc[i] >> 8;
-            A->care[q * 32 + c.lane] = c.lane < (int)(oc & 0xffffu) ? c.list[(size_t)t * TILE + (oc >> 16) + c.lane] : 0.0f;
+            const Item it = A->items[i];
+            A->care[q * 32 + c.lane] = c.lane >= it.cnt() ? 0.0f : (it.place() != 255u ? R.care(c.rr)[it.place() * 32 + c.lane] : c.list[(size_t)it.tile() * TILE + it.off() + c.lane]);
         }
         FCOUNT(20, n); FCOUNT(21, ncare); if (!locate) FSTAMP(2);
         for (int round = 0; round <= n; round++) {   // (each round but the last is for one more item)
@@ -1019,9 +1427,11 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
             if (want < 0 || A->w_found) break;
             // a run whose guess was wrong, or that holds the target: its values, one by one
             const Item it = A->items[want];
-            const int t = (int)(A->isrc[want] >> 8), off = (int)(it.oc >> 16), m = (int)(it.oc & 0xffffu);
+            const int t = it.tile(), off = it.off(), m = it.cnt();
             FCOUNT(23, 1);
-            if ((c.pl.flags & F_LIST) || (it.meta >> 8) != K_RUN) {
+            if (it.place() != 255u) {
+                if (c.tid < 32) A->ebuf[c.tid] = c.tid < m ? R.care(c.rr)[it.place() * 32 + c.tid] : 0.0f;
+            } else if ((c.pl.flags & F_LIST) || it.kind() != K_RUN) {
                 for (int i = c.tid; i < ((m + 7) & ~7); i += NT) A->ebuf[i] = i < m ? c.list[(size_t)t * TILE + off + i] : 0.0f;
             } else {
                 tile_again(c, t, t + 1, A->ebuf, false);
@@ -1504,7 +1914,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
     c.status |= MOLLA_ROW_DEGENERATE;
 }
 
-__global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant__ RowsArgs R) {
+__device__ void tail_row(const RowsArgs &R, int rr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CtxF c;
     c.tid = threadIdx.x; c.lane = c.tid & 31; c.warp = c.tid >> 5; c.status = 0;
@@ -1512,26 +1922,26 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
     c.R = &R;
     AuxF *A = c.A;
     IN_SHARED(A);
-    pdl_next();
-    pdl_wait();
-    c.rr = blockIdx.x; c.r = R.r0 + c.rr;
-    c.pl = R.plan[c.rr];
-    if (c.pl.kind == PLAN_DONE) return;
+    c.rr = rr; c.r = R.r0 + rr;
+    const RowHead *head = R.head(rr);
+    c.pl = head->plan;
+    const int state = head->state;
     const BatchArgs &a = R.a;
     FSTAMP(0);
     c.cfg = c.pl.c;
     c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
-    c.gitems = R.items + (size_t)c.rr * R.ntile * ITEMS_PER_TILE;
+    c.gitems = R.items(rr);
     c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
     const RowCfg &g = c.cfg;
     const int ntile = R.ntile, imax = c.pl.imax;
     for (int t = c.tid; t < ntile; t += NT) {
-        const TileOut o = R.to[(size_t)c.rr * ntile + t];
-        A->tcnt[t] = o.cnt; A->tni[t] = o.nitem;
+        const TileOut o = R.to(rr)[t];
+        A->tcnt[t] = o.cnt; A->tni[t] = o.nitem; A->tio[t] = o.ioff;
     }
-    unsigned long long *gcand = R.cand + (size_t)c.rr * HEADCAP;
-    int nc_all = g.pure ? 0 : R.ncand[c.rr];
+    unsigned long long *gcand = R.cand(rr);
+    int nc_all = g.pure ? 0 : head->ncand;
     if (nc_all > HEADCAP) {
+        __syncthreads();
         if (!(c.pl.flags & F_LIST)) {
             for (int t = 0; t < ntile; t += SPAN / TILE) tile_again(c, t, min(t + SPAN / TILE, ntile), nullptr, true);
             c.pl.flags |= F_LIST;
@@ -1548,7 +1958,7 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
 
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
     FSTAMP(1);
-    const float Z = exact_sum(c, false, 0.0f);
+    const float Z = state != ST_NOTHING ? head->Z : exact_sum(c, false, 0.0f);
     FSTAMP(3);
     dZ = Z;
     const float yZ = __fdiv_rn(1.0f, Z);
@@ -1625,8 +2035,9 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
             }
             __syncwarp();
             bool care;
-            const int ni = tile_items(mine, cnt, off, n, s, A->tsum[t], c.gitems + (size_t)t * ITEMS_PER_TILE, care);
-            if (c.lane == 0) A->tni[t] = (unsigned short)ni;
+            int my_place;
+            const int ni = tile_items(mine, cnt, off, n, s, A->tsum[t], t, [&](int, int) { return c.gitems + (size_t)t * ITEMS_PER_TILE; }, [](int) { return 255; }, care, my_place);
+            if (c.lane == 0) { A->tni[t] = (unsigned short)ni; A->tio[t] = (unsigned int)(t * ITEMS_PER_TILE); }
             __syncwarp();
         }
         __syncthreads();
@@ -1662,6 +2073,18 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
     // ---- sorted order: the head's candidates as probabilities
     const int nc = head_overflow ? 0 : nc_all;
     if (head_overflow) c.status |= MOLLA_ROW_SLOW_PATH;  // no head: the descending walk takes everything from the top
+    float head_s;
+    long long head_pos;
+    if (state == ST_HEAD) {   // row_head has sorted it and added it up
+        head_s = head->head_s; head_pos = head->head_pos;
+        for (int i = c.tid; i < nc; i += NT) {
+            const unsigned int p = (unsigned int)(gcand[i] >> 32);
+            const bool eq = (i > 0 && (unsigned int)(gcand[i - 1] >> 32) == p) || (i + 1 < nc && (unsigned int)(gcand[i + 1] >> 32) == p);
+            A->pre[i] = R.pre(rr)[i];
+            A->hidx[i] = (unsigned int)key_idx(gcand[i]) | (eq ? 0x80000000u : 0u);
+        }
+        __syncthreads();
+    } else {
     {
         for (int i = c.tid; i < nc; i += NT) {
             const unsigned long long kk = gcand[i];
@@ -1742,8 +2165,8 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
     __syncthreads();
     FSTAMP(6);
     c.status |= (unsigned int)A->b_aux;
-    const float head_s = A->b_s;
-    const long long head_pos = A->b_pos;
+    head_s = A->b_s;
+    head_pos = A->b_pos;
     if (typ_on) {
         const int m = A->ncand;
         __syncthreads();
@@ -1761,6 +2184,7 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
         token = A->b_idx; dp = A->b_p; dsum = A->b_sum; dtarget = A->b_target;
         finish();
         return;
+    }
     }
 
     // ---- past the head: the cut walk, then the draw walk, over the probabilities
@@ -1848,6 +2272,16 @@ __global__ void __launch_bounds__(NT, 2) row_finish_kernel(const __grid_constant
     finish();
 }
 
+__global__ void __launch_bounds__(NT, 1) row_tail_kernel(const __grid_constant__ RowsArgs R) {
+    pdl_next();
+    pdl_wait();
+    const int n = R.queue[0];
+    for (int q = blockIdx.x; q < n; q += gridDim.x) {
+        tail_row(R, R.queue[1 + q]);
+        __syncthreads();
+    }
+}
+
 // ---- host side --------------------------------------------------------------------------------
 // The widest layout of one row over thread blocks that F_NARROW speaks of: blocks of at most 38400
 // logits, 1, 2, 4 or 8 of them; more than the row needs where the batch leaves the chip idle.
@@ -1880,15 +2314,15 @@ size_t lay_out(RowsArgs &A, char *ws, int rows, int V) {
     size_t o = 0;
     auto take = [&](size_t bytes) { char *p = ws + o; o += al(bytes); return p; };
     A.elist = (float *)take(n * TILE * sizeof(float));
-    A.items = (Item *)take(n * ITEMS_PER_TILE * sizeof(Item));
     A.gmax = (float *)take(n * 32 * sizeof(float));
     A.kmask = (unsigned int *)take(n * 32 * sizeof(unsigned int));
     A.ts = (TileStat *)take(n * sizeof(TileStat));
     A.tp = (TilePlan *)take(n * sizeof(TilePlan));
-    A.to = (TileOut *)take(n * sizeof(TileOut));
-    A.cand = (unsigned long long *)take((size_t)rows * HEADCAP * sizeof(unsigned long long));
-    A.plan = (RowPlan *)take((size_t)rows * sizeof(RowPlan));
-    A.ncand = (int *)take((size_t)rows * sizeof(int));
+    const size_t items = nt * ITEMS_PER_TILE > (size_t)H_ITEMS ? nt * ITEMS_PER_TILE : (size_t)H_ITEMS;
+    A.box_stride = (long long)al(sizeof(RowHead) + ((nt + 1) & ~(size_t)1) * sizeof(TileOut) + HEADCAP * (sizeof(unsigned long long) + sizeof(float)) +
+                                 CARE_PLACES * 32 * sizeof(float) + items * sizeof(Item));
+    A.box = (char *)take((size_t)rows * (size_t)A.box_stride);
+    A.queue = (int *)take((size_t)(rows + 1) * sizeof(int));
     return o;
 }
 
@@ -1920,7 +2354,8 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     if (e == cudaSuccess && (dev >= 64 || !ready[dev])) {
         e = cudaFuncSetAttribute(tile_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_exp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AuxF));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AuxF));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadShared));
         if (e == cudaSuccess && dev < 64) ready[dev] = true;
     }
     RowsArgs A;
@@ -1937,7 +2372,8 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         e = launch(tile_stats_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
         if (e == cudaSuccess) e = launch(row_plan_kernel, (unsigned int)A.rows, NT, 0, st, A);
         if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
-        if (e == cudaSuccess) e = launch(row_finish_kernel, (unsigned int)A.rows, NT, sizeof(AuxF), st, A);
+        if (e == cudaSuccess) e = launch(row_head_kernel, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
+        if (e == cudaSuccess) e = launch(row_tail_kernel, (unsigned int)(A.rows < sms ? A.rows : sms), NT, sizeof(AuxF), st, A);
     }
     if (e != cudaSuccess) {
         snprintf(err, errlen, "kernel launch failed: %s", cudaGetErrorString(e));
