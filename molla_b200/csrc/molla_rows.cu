@@ -35,7 +35,7 @@ constexpr int ITEMS_PER_TILE = 66;         // a run and a careful chunk per lane
 constexpr int HEADCAP = 2048;              // candidates of the sorted head at most
 constexpr int HEAD_MOST = 1026;            // the sorted head covers top-k + 1 up to this many
 constexpr int ITEM_CAP = 384;              // items of a row that fit shared memory
-constexpr int CARE_PLACES = 192;           // careful chunks of a row whose values are handed on with the items
+constexpr int CARE_PLACES = 255;           // careful chunks of a row whose values are handed on with the items
 constexpr int CARE_CAP = 48;               // careful chunks whose entries are fetched ahead
 constexpr int TIE_CAP = 64;                // rounding ties a walk resolves by parity; more send it the slow way
 constexpr int PLAN_BINS = 1024;            // row_plan: bins of the lanes' maxima by distance below the row's,
@@ -611,7 +611,7 @@ __device__ __forceinline__ int tile_items(const float *row, int cnt, int off, in
     const float sst = est + ex;
     const bool nonempty = cnt > 0 && csum > 0.0f;
     // the estimate counts what was dropped (it adds nothing to the true sum), so it is high rather than low
-    const float lo = sst * (1.0f - 1.0f / 256.0f), hi = (sst + csum) * (1.0f + 1.0f / 2048.0f);
+    const float lo = sst * (1.0f - 1.0f / 1024.0f), hi = (sst + csum) * (1.0f + 1.0f / 2048.0f);
     const int jl = fexpo(lo), jh = fexpo(hi);
     const bool usable = nonempty && lo > 0.0f && jh <= jl + 1 && jl >= -100 && jh <= 100;
     const bool two = usable && jh == jl + 1;
@@ -834,14 +834,14 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // and of one round of loads, so the block is small and four of them share an SM.
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
-constexpr int H_ITEMS = 512, H_CARE = 80;
+constexpr int H_ITEMS = 512, H_CARE = 80, H_REC = 320;   // careful chunks whose values are at hand, and all of them
 enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2 };   // what a queued row has: nothing, its denominator, its head too
 
 struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the last of them | kind | own binade | place
 
 struct __align__(16) HeadShared {
     union {
-        struct { Item items[H_ITEMS]; float care[H_CARE * 32]; CareRec rec[H_CARE + 1]; } w;
+        struct { Item items[H_ITEMS]; float care[H_CARE * 32]; CareRec rec[H_REC + 1]; } w;
         unsigned int sbin[NBINS];
     };
     unsigned long long cand[HEADCAP];
@@ -943,16 +943,16 @@ __device__ void head_sort(HeadShared *S, int n) {
 }
 
 // One warp, all lanes alike: the sum through the careful chunks S->w.rec[0..nrec) and the runs between
-// them. Returns false where a run's binade was guessed wrong.
-__device__ bool walk_records(const HeadShared *S, int nrec, float &Z) {
+// them; `more` holds the values of all of them. Returns false where a run's binade was guessed wrong.
+__device__ bool walk_records(const HeadShared *S, const float *more, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
     CareRec nx = S->w.rec[0];
     for (int q = 0; q <= nrec; q++) {
         const CareRec r = nx;
-        const float4 *v = reinterpret_cast<const float4 *>(S->w.care + ((r.meta >> 24) & 0xffu) * 32);
-        const unsigned int kind = (r.meta >> 8) & 3u;
+        const unsigned int kind = (r.meta >> 8) & 3u, place = r.meta >> 24;
+        const float4 *v = reinterpret_cast<const float4 *>(S->w.care + place * 32);
         float4 x[8];
-        if (q < nrec && kind != K_RUN) {   // asked for before it is known whether they are needed
+        if (q < nrec && kind != K_RUN && place < H_CARE) {   // asked for before it is known whether they are needed
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = v[i];
         }
@@ -975,6 +975,10 @@ __device__ bool walk_records(const HeadShared *S, int nrec, float &Z) {
         if (kind == K_DUAL) {
             const unsigned int to = e == jb ? sb + r.ka : sb + r.kb;
             if ((e == jb || e == jb + 1u) && (to >> 23) == e) { sb = to; continue; }
+        }
+        if (place >= H_CARE) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = reinterpret_cast<const float4 *>(more + place * 32)[i];
         }
         float s = __uint_as_float(sb);
 #pragma unroll
@@ -1016,10 +1020,13 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
     if (kind == PLAN_DONE) return;
     const RowCfg &g = pl.c;
     const bool narrow = (pl.flags & F_NARROW) != 0;
-    auto queue_row = [&](int state) {
+    auto queue_row = [&](int state, int why = 0) {
+#ifdef MOLLA_SAMPLE_TESTING
+        if (a.prof && tid == 0) { a.prof[(long long)r * 32 + 24] = why; a.prof[(long long)r * 32 + 25] = nitem; a.prof[(long long)r * 32 + 26] = ncare; a.prof[(long long)r * 32 + 27] = ncand; }
+#endif
         if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
     };
-    if (nitem > H_ITEMS || ncare > H_CARE || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING); return; }
+    if (nitem > H_ITEMS || ncare > CARE_PLACES || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
     // ---- the items in order, the careful ones among them as records
     unsigned int total;
     const unsigned int o = head_scan(to[0].nitem + to[1].nitem + to[2].nitem, S->ws, &total);
@@ -1031,7 +1038,7 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
 #pragma unroll
     for (int u = 0; u < CV; u++)
         if (tid + u * HT < H_CARE * 8) reinterpret_cast<float4 *>(S->w.care)[tid + u * HT] = cv[u];
-    if (tid == 0) { S->ok = 1; S->n_ge = 0; }
+    if (tid == 0) S->n_ge = 0;
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < H_ITEMS / HT; u++)
@@ -1053,13 +1060,13 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
                 bool prev_run = false;
                 if (i > 0) { const Item p = S->w.items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
                 care[u] = !run || (prev_run && pj[u] != mine[u].jb());   // (a change of binade between two runs: a wrong guess)
-                if (care[u]) { n++; if (!run && mine[u].place() >= (unsigned int)H_CARE) S->ok = 0; }
+                if (care[u]) n++;
                 else k += mine[u].ka;
             }
         }
         unsigned int ktot;
         unsigned int kx = head_scan(k, S->ws, &ktot), nx = head_scan(n, S->ws2, &nrec);
-        if (nrec <= (unsigned int)H_CARE) {
+        if (nrec <= (unsigned int)H_REC) {
 #pragma unroll
             for (int u = 0; u < IPT; u++)
                 if (IPT * tid + u < nitem) {
@@ -1078,19 +1085,19 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
         }
     }
     __syncthreads();
-    if (nrec > (unsigned int)H_CARE || !S->ok) { queue_row(ST_NOTHING); return; }
+    if (nrec > (unsigned int)H_REC) { queue_row(ST_NOTHING, 2); return; }
     __syncthreads();
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
     if (warp == 0) {
         float z = 0.0f;
-        const bool fine = walk_records(S, (int)nrec, z);
+        const bool fine = walk_records(S, R.care(rr), (int)nrec, z);
         if (lane == 0) { S->Z = z; S->ok = fine ? 1 : 0; }
     }
     __syncthreads();
-    if (!S->ok) { queue_row(ST_NOTHING); return; }
+    if (!S->ok) { queue_row(ST_NOTHING, 3); return; }
     const float Z = S->Z, yZ = __fdiv_rn(1.0f, Z);
     if (tid == 0) head->Z = Z;
-    if (g.pure || g.typ < 1.0f) { queue_row(ST_SUM); return; }
+    if (g.pure || g.typ < 1.0f) { queue_row(ST_SUM, 4); return; }
     // ---- sorted order: the head's candidates as probabilities
     const int nc = ncand;
     for (int i = tid; i < nc; i += HT) {
@@ -1186,10 +1193,10 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
     }
     __syncthreads();
     if (S->cut > 0) return;
-    if (all_above || nc == 0) { queue_row(ST_SUM); return; }
+    if (all_above || nc == 0) { queue_row(ST_SUM, 5); return; }
     // past the head: the sorted candidates and their prefix sums go along
     for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
-    queue_row(ST_HEAD);
+    queue_row(ST_HEAD, 6);
 }
 
 // =============================================================================
@@ -1938,6 +1945,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         const TileOut o = R.to(rr)[t];
         A->tcnt[t] = o.cnt; A->tni[t] = o.nitem; A->tio[t] = o.ioff;
     }
+    __syncthreads();
     unsigned long long *gcand = R.cand(rr);
     int nc_all = g.pure ? 0 : head->ncand;
     if (nc_all > HEADCAP) {
