@@ -86,6 +86,12 @@ struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned in
 
 // A row's small results, together in memory: the kernels that read them wait once.
 //   RowHead | TileOut[ntile] | candidates[HEADCAP] | prefix sums[HEADCAP] | values of careful chunks[CARE_PLACES][32] | items
+// A walk past the head: per binade of the running sum, the integer mass of every bin of values, and the
+// elements that would round on a tie there.
+constexpr int WALK_BINADES = 3;
+struct __align__(16) WalkTies { int n; int pad[3]; unsigned long long key[TIE_CAP]; };
+constexpr size_t WALK_BYTES = WALK_BINADES * (NBINS * sizeof(unsigned long long) + sizeof(WalkTies));
+
 struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; int pad[4]; };
 
 struct RowsArgs {
@@ -97,9 +103,12 @@ struct RowsArgs {
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
     TilePlan *tp;            // [rows][ntile]
     char *box; long long box_stride;  // [rows]
-    int *queue;              // rows for row_tail: their number, then the rows
+    int *queue;              // rows for tile_walk and row_tail: their number, then the rows
+    char *walk;              // [rows] tables and ties of a walk past the head
     float *elist;            // [rows][ntile][TILE] values kept, in vocabulary order, packed per tile
     unsigned int *kmask;     // [rows][ntile][32] which logits they are
+    __device__ __forceinline__ unsigned long long *table(int rr, int b) const { return reinterpret_cast<unsigned long long *>(walk + (size_t)rr * WALK_BYTES) + (size_t)b * NBINS; }
+    __device__ __forceinline__ WalkTies *ties(int rr) const { return reinterpret_cast<WalkTies *>(table(rr, WALK_BINADES)); }
     __device__ __forceinline__ RowHead *head(int rr) const { return reinterpret_cast<RowHead *>(box + (long long)rr * box_stride); }
     __device__ __forceinline__ TileOut *to(int rr) const { return reinterpret_cast<TileOut *>(head(rr) + 1); }
     __device__ __forceinline__ unsigned long long *cand(int rr) const { return reinterpret_cast<unsigned long long *>(to(rr) + ((ntile + 1) & ~1)); }
@@ -834,27 +843,41 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // and of one round of loads, so the block is small and four of them share an SM.
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
-constexpr int H_ITEMS = 512, H_CARE = 80, H_REC = 320;   // careful chunks whose values are at hand, and all of them
-enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2 };   // what a queued row has: nothing, its denominator, its head too
+constexpr int H_ITEMS = 768;               // items of a row
+constexpr int H_CARE = 80, H_REC = 512;    // careful chunks whose values are at hand, and all of them
+// What a queued row has: nothing; its denominator; its head too (tile_walk prepares the walk past it);
+// its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
+enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3 };
 
 struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the last of them | kind | own binade | place
 
+struct __align__(16) WalkShared {
+    Item items[H_ITEMS];
+    float care[H_CARE * 32];
+    CareRec rec[H_REC + 1];
+    unsigned int sbs[H_REC + 2];           // the sum before every record's runs
+    unsigned short toff[MAX_TILES + 4];
+    unsigned int ws[NWARP + 1], ws2[NWARP + 1];
+};
+
 struct __align__(16) HeadShared {
     union {
-        struct { Item items[H_ITEMS]; float care[H_CARE * 32]; CareRec rec[H_REC + 1]; } w;
+        WalkShared w;
         unsigned int sbin[NBINS];
+        struct { unsigned long long keys[HEADC]; float lg[HEADC], tt[HEADC]; } typ;
     };
     unsigned long long cand[HEADCAP];
     union {
         unsigned long long tmp[HEADCAP];
         struct { float pc[HEADCAP]; float pre[HEADCAP]; } p;
     };
-    unsigned short toff[MAX_TILES + 2];
     unsigned int ws[HW + 1], ws2[HW + 1];
-    float Z; int ok, cut, n_ge;
+    float Z; int ok, cut, n_ge; unsigned int tie;
+    float ent;
 };
 
-// exclusive scan over the HT threads
+// exclusive scan over N threads
+template <int N>
 __device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *ws, unsigned int *total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned int inc = warp_incl_scan(v, lane);
@@ -863,7 +886,7 @@ __device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *
     __syncthreads();
     unsigned int b = 0u, t = 0u;
 #pragma unroll
-    for (int w = 0; w < HW; w++) {
+    for (int w = 0; w < N / 32; w++) {
         if (w == warp) b = t;
         t += ws[w];
     }
@@ -917,7 +940,7 @@ __device__ void head_sort(HeadShared *S, int n) {
         unsigned int cnt[PER], sum = 0u, tot;
 #pragma unroll
         for (int i = 0; i < PER; i++) { cnt[i] = S->sbin[PER * tid + i]; sum += cnt[i]; }
-        unsigned int at = head_scan(sum, S->ws, &tot);
+        unsigned int at = head_scan<HT>(sum, S->ws, &tot);
 #pragma unroll
         for (int i = 0; i < PER; i++) { S->sbin[PER * tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
         __syncthreads();
@@ -942,21 +965,102 @@ __device__ void head_sort(HeadShared *S, int n) {
     __syncthreads();
 }
 
-// One warp, all lanes alike: the sum through the careful chunks S->w.rec[0..nrec) and the runs between
+// Everything about a row's items, in one round of loads by N threads (what lies past the counts is not used).
+template <int N>
+struct WalkLoads {
+    static constexpr int TPT = (MAX_TILES + N - 1) / N, IPT = (H_ITEMS + N - 1) / N, CV = (H_CARE * 8 + N - 1) / N;
+    TileOut to[TPT];
+    Item it[IPT];
+    float4 cv[CV];
+    __device__ __forceinline__ void load(const RowsArgs &R, int rr) {
+        const int tid = threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < TPT; u++) {
+            to[u].nitem = 0;
+            if (TPT * tid + u < R.ntile) to[u] = R.to(rr)[TPT * tid + u];
+        }
+#pragma unroll
+        for (int u = 0; u < IPT; u++)
+            if (tid + u * N < H_ITEMS) it[u] = R.items(rr)[tid + u * N];
+#pragma unroll
+        for (int u = 0; u < CV; u++)
+            if (tid + u * N < H_CARE * 8) cv[u] = reinterpret_cast<const float4 *>(R.care(rr))[tid + u * N];
+    }
+    // The items in order, the careful ones among them as records; returns the number of records.
+    __device__ __forceinline__ unsigned int order(WalkShared *W, int ntile, int nitem) {
+        const int tid = threadIdx.x;
+        unsigned int total, n0 = 0u;
+#pragma unroll
+        for (int u = 0; u < TPT; u++) n0 += to[u].nitem;
+        unsigned int o = head_scan<N>(n0, W->ws, &total);
+#pragma unroll
+        for (int u = 0; u < TPT; u++) {
+            if (TPT * tid + u < ntile) W->toff[TPT * tid + u] = (unsigned short)o;
+            o += to[u].nitem;
+        }
+#pragma unroll
+        for (int u = 0; u < CV; u++)
+            if (tid + u * N < H_CARE * 8) reinterpret_cast<float4 *>(W->care)[tid + u * N] = cv[u];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < IPT; u++)
+            if (tid + u * N < nitem) W->items[W->toff[it[u].tile()] + it[u].num()] = it[u];
+        __syncthreads();
+        unsigned int pj[IPT], k = 0u, n = 0u, care = 0u;
+#pragma unroll
+        for (int u = 0; u < IPT; u++) {
+            const int i = IPT * tid + u;
+            pj[u] = 0u;
+            if (i < nitem) {
+                it[u] = W->items[i];
+                const bool run = it[u].kind() == K_RUN;
+                bool prev_run = false;
+                if (i > 0) { const Item p = W->items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
+                if (!run || (prev_run && pj[u] != it[u].jb())) { care |= 1u << u; n++; }   // (a change of binade between two runs: a wrong guess)
+                else k += it[u].ka;
+            }
+        }
+        unsigned int ktot, nrec;
+        unsigned int kx = head_scan<N>(k, W->ws, &ktot), nx = head_scan<N>(n, W->ws2, &nrec);
+        if (nrec <= (unsigned int)H_REC) {
+#pragma unroll
+            for (int u = 0; u < IPT; u++) {
+                const int i = IPT * tid + u;
+                if (i >= nitem) break;
+                if ((care >> u) & 1u) {
+                    CareRec c;
+                    c.k = kx; c.ka = it[u].ka; c.kb = it[u].kb;
+                    c.meta = pj[u] | (it[u].kind() << 8) | (it[u].jb() << 16) | (it[u].place() << 24);
+                    W->rec[nx++] = c;
+                } else kx += it[u].ka;
+            }
+            if (tid == 0) {
+                CareRec c;
+                c.k = ktot; c.ka = c.kb = 0u; c.meta = nitem > 0 ? W->items[nitem - 1].jb() : 0u;
+                W->rec[nrec] = c;
+            }
+        }
+        __syncthreads();
+        return nrec;
+    }
+};
+
+// One warp, all lanes alike: the sum through the careful chunks W->rec[0..nrec) and the runs between
 // them; `more` holds the values of all of them. Returns false where a run's binade was guessed wrong.
-__device__ bool walk_records(const HeadShared *S, const float *more, int nrec, float &Z) {
+__device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
-    CareRec nx = S->w.rec[0];
+    CareRec nx = W->rec[0];
     for (int q = 0; q <= nrec; q++) {
         const CareRec r = nx;
         const unsigned int kind = (r.meta >> 8) & 3u, place = r.meta >> 24;
-        const float4 *v = reinterpret_cast<const float4 *>(S->w.care + place * 32);
+        const float4 *v = reinterpret_cast<const float4 *>(W->care + place * 32);
         float4 x[8];
         if (q < nrec && kind != K_RUN && place < H_CARE) {   // asked for before it is known whether they are needed
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = v[i];
         }
-        nx = S->w.rec[q < nrec ? q + 1 : q];
+        nx = W->rec[q < nrec ? q + 1 : q];
+        W->sbs[q] = sb;
         const unsigned int kx = r.k - kdone;
         kdone = r.k;
         if (kx) {
@@ -977,6 +1081,7 @@ __device__ bool walk_records(const HeadShared *S, const float *more, int nrec, f
             if ((e == jb || e == jb + 1u) && (to >> 23) == e) { sb = to; continue; }
         }
         if (place >= H_CARE) {
+            if (place == 255u) return false;
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = reinterpret_cast<const float4 *>(more + place * 32)[i];
         }
@@ -985,11 +1090,93 @@ __device__ bool walk_records(const HeadShared *S, const float *more, int nrec, f
         for (int i = 0; i < 8; i++) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
         sb = __float_as_uint(s);
     }
+    W->sbs[nrec + 1] = sb;
     Z = __uint_as_float(sb);
     return true;
 }
 
-__global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__ RowsArgs R) {
+// Typical-p (sample.mojo:525-567) on the m kept probabilities S->p.pc[0..m), descending, ids in S->cand:
+// entropy H = -sum p log p added up in that order, distance |-log p - H|, stable order by distance, the
+// smallest prefix whose probabilities add up to typ, the draw (:569-594) over that prefix in that order.
+__device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int r, const RowCfg &g, int m, float Z, unsigned int status) {
+    const int tid = threadIdx.x;
+    const float *pc = S->p.pc;
+    float *pre = S->p.pre;
+    unsigned long long *keys = S->typ.keys;
+    if (m <= 0 || m > HEADC) {   // what the earlier filters left reaches past the head, or is wider than the filter's scratch
+        if (tid == 0) finish_row(a, r, g, status | MOLLA_ROW_UNSUPPORTED, -1, Z, 0, 0, 0);
+        return;
+    }
+    __syncthreads();
+    for (int i = tid; i < m; i += HT) {
+        const float p = pc[i];
+        const float l = (p > 0.0f) ? logf_pinned(p) : 0.0f;
+        S->typ.lg[i] = l;
+        S->typ.tt[i] = (p > 0.0f) ? __fmul_rn(p, l) : 0.0f;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        float ent = 0.0f;
+        for (int i = 0; i < m; i++)
+            if (pc[i] > 0.0f) ent = __fsub_rn(ent, S->typ.tt[i]);
+        S->ent = ent;
+    }
+    __syncthreads();
+    const float ent = S->ent;
+    constexpr int KPT = HEADC / HT;
+    unsigned long long k[KPT];
+    int rank[KPT];
+#pragma unroll
+    for (int u = 0; u < KPT; u++) {
+        const int i = tid + u * HT;
+        k[u] = 0ull; rank[u] = 0;
+        if (i < m) {
+            const float sur = (pc[i] > 0.0f) ? -S->typ.lg[i] : 0.0f;
+            const float d = fabsf(__fsub_rn(sur, ent));
+            // descending keys = ascending distance, and among equal distances ascending position (stable)
+            k[u] = ((unsigned long long)(~__float_as_uint(d)) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned int)i);
+            keys[i] = k[u];
+        }
+    }
+    __syncthreads();
+    for (int j = 0; j < m; j++) {
+        const unsigned long long o = keys[j];
+#pragma unroll
+        for (int u = 0; u < KPT; u++) rank[u] += o > k[u] ? 1 : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < KPT; u++)
+        if (tid + u * HT < m) keys[rank[u]] = k[u];
+    __syncthreads();
+    if (tid == 0) {
+        auto at_of = [&](int j) { return (int)(0xFFFFFFFFu - (unsigned int)(keys[j] & 0xFFFFFFFFull)); };
+        float s = 0.0f;
+        int kept = m;
+        for (int j = 0; j < m; j++) {
+            s = __fadd_rn(s, pc[at_of(j)]);
+            pre[j] = s;
+            if (s >= g.typ) { kept = j + 1; break; }
+        }
+        const float sum = pre[kept - 1];
+        int at = kept - 1;
+        float target = 0.0f;
+        if (sum <= 0.0f) at = 0;  // sample.mojo:583-584
+        else {
+            target = __fmul_rn(draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull), sum);
+            for (int j = 0; j < kept; j++)
+                if (target < pre[j]) { at = j; break; }
+        }
+        const int i = at_of(at);
+        if ((i > 0 && pc[i - 1] == pc[i]) || (i + 1 < HEADCAP && pc[i + 1] == pc[i])) status |= MOLLA_ROW_CHOSEN_TIE;
+        // the last one kept and the first one dropped equally probable: which of them the reference
+        // keeps depends on the order its sort left them in
+        if (kept < m && pc[at_of(kept - 1)] == pc[at_of(kept)]) status |= MOLLA_ROW_TOPP_TIE;
+        finish_row(a, r, g, status, key_idx(S->cand[i]), Z, sum, target, pc[i]);
+    }
+}
+
+__global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__ RowsArgs R) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HeadShared *S = reinterpret_cast<HeadShared *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rr = blockIdx.x, r = R.r0 + rr;
@@ -1002,20 +1189,8 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
     const int ncand = head->ncand, nitem = head->nitem, ncare = head->ncare;
     const RowPlan &pl = head->plan;
     const int kind = pl.kind;
-    TileOut to[3];
-#pragma unroll
-    for (int u = 0; u < 3; u++) {
-        to[u].nitem = 0;
-        if (3 * tid + u < ntile) to[u] = R.to(rr)[3 * tid + u];
-    }
-    Item it[H_ITEMS / HT];
-#pragma unroll
-    for (int u = 0; u < H_ITEMS / HT; u++) it[u] = R.items(rr)[tid + u * HT];   // (a row has room for more)
-    constexpr int CV = (H_CARE * 8 + HT - 1) / HT;
-    float4 cv[CV];
-#pragma unroll
-    for (int u = 0; u < CV; u++)
-        if (tid + u * HT < H_CARE * 8) cv[u] = reinterpret_cast<const float4 *>(R.care(rr))[tid + u * HT];
+    WalkLoads<HT> wl;
+    wl.load(R, rr);
     unsigned long long key = R.cand(rr)[tid];
     if (kind == PLAN_DONE) return;
     const RowCfg &g = pl.c;
@@ -1027,77 +1202,25 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
         if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
     };
     if (nitem > H_ITEMS || ncare > CARE_PLACES || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
-    // ---- the items in order, the careful ones among them as records
-    unsigned int total;
-    const unsigned int o = head_scan(to[0].nitem + to[1].nitem + to[2].nitem, S->ws, &total);
-    if (3 * tid < ntile) {
-        S->toff[3 * tid] = (unsigned short)o;
-        S->toff[3 * tid + 1] = (unsigned short)(o + to[0].nitem);
-        S->toff[3 * tid + 2] = (unsigned short)(o + to[0].nitem + to[1].nitem);
-    }
-#pragma unroll
-    for (int u = 0; u < CV; u++)
-        if (tid + u * HT < H_CARE * 8) reinterpret_cast<float4 *>(S->w.care)[tid + u * HT] = cv[u];
     if (tid == 0) S->n_ge = 0;
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < H_ITEMS / HT; u++)
-        if (tid + u * HT < nitem) S->w.items[S->toff[it[u].tile()] + it[u].num()] = it[u];
-    __syncthreads();
-    unsigned int nrec;
-    {
-        constexpr int IPT = H_ITEMS / HT;
-        bool care[IPT];
-        unsigned int pj[IPT], k = 0u, n = 0u;
-        Item mine[IPT];
-#pragma unroll
-        for (int u = 0; u < IPT; u++) {
-            const int i = IPT * tid + u;
-            care[u] = false; pj[u] = 0u;
-            if (i < nitem) {
-                mine[u] = S->w.items[i];
-                const bool run = mine[u].kind() == K_RUN;
-                bool prev_run = false;
-                if (i > 0) { const Item p = S->w.items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
-                care[u] = !run || (prev_run && pj[u] != mine[u].jb());   // (a change of binade between two runs: a wrong guess)
-                if (care[u]) n++;
-                else k += mine[u].ka;
-            }
-        }
-        unsigned int ktot;
-        unsigned int kx = head_scan(k, S->ws, &ktot), nx = head_scan(n, S->ws2, &nrec);
-        if (nrec <= (unsigned int)H_REC) {
-#pragma unroll
-            for (int u = 0; u < IPT; u++)
-                if (IPT * tid + u < nitem) {
-                    if (care[u]) {
-                        CareRec c;
-                        c.k = kx; c.ka = mine[u].ka; c.kb = mine[u].kb;
-                        c.meta = pj[u] | (mine[u].kind() << 8) | (mine[u].jb() << 16) | (mine[u].place() << 24);
-                        S->w.rec[nx++] = c;
-                    } else kx += mine[u].ka;
-                }
-            if (tid == 0) {
-                CareRec c;
-                c.k = ktot; c.ka = c.kb = 0u; c.meta = nitem > 0 ? S->w.items[nitem - 1].jb() : 0u;
-                S->w.rec[nrec] = c;
-            }
-        }
-    }
-    __syncthreads();
+    const unsigned int nrec = wl.order(&S->w, ntile, nitem);
     if (nrec > (unsigned int)H_REC) { queue_row(ST_NOTHING, 2); return; }
-    __syncthreads();
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
     if (warp == 0) {
         float z = 0.0f;
-        const bool fine = walk_records(S, R.care(rr), (int)nrec, z);
+        const bool fine = walk_records(&S->w, R.care(rr), (int)nrec, z);
         if (lane == 0) { S->Z = z; S->ok = fine ? 1 : 0; }
     }
     __syncthreads();
     if (!S->ok) { queue_row(ST_NOTHING, 3); return; }
     const float Z = S->Z, yZ = __fdiv_rn(1.0f, Z);
     if (tid == 0) head->Z = Z;
-    if (g.pure || g.typ < 1.0f) { queue_row(ST_SUM, 4); return; }
+    if (g.pure) {
+        if (g.minp > 0.0f) { queue_row(ST_SUM, 4); return; }   // (what min-p leaves out is in no estimate)
+        if (tid == 0) { head->nitem = 0; head->ncare = 0; }
+        queue_row(ST_PURE, 4);
+        return;
+    }
     // ---- sorted order: the head's candidates as probabilities
     const int nc = ncand;
     for (int i = tid; i < nc; i += HT) {
@@ -1173,7 +1296,9 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
         }
         if (cut < 0 && !p3row) cut = nc;  // everything that can matter is in the head
         if (!narrow && n_use < (long long)a.V && (long long)nc > n_use && pc[n_use] == pc[n_use - 1]) tie |= MOLLA_ROW_TOPK_TIE;
-        if (cut > 0) {
+        if (g.typ < 1.0f) {
+            // the typical-p filter takes over from here
+        } else if (cut > 0) {
             const float sum = pre[cut - 1];
             const float target = __fmul_rn(draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull), sum);
             // the first prefix sum above the target (they never fall), or the last one kept
@@ -1189,18 +1314,150 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
         } else if (lane == 0) {
             head->head_s = s; head->head_pos = pos;
         }
-        if (lane == 0) S->cut = cut;
+        if (lane == 0) { S->cut = cut; S->tie = (unsigned int)tie; }
     }
     __syncthreads();
+    if (g.typ < 1.0f) {
+        typical_rows(S, a, r, g, narrow ? -1 : S->cut, Z, S->tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u));
+        return;
+    }
     if (S->cut > 0) return;
     if (all_above || nc == 0) { queue_row(ST_SUM, 5); return; }
-    // past the head: the sorted candidates and their prefix sums go along
+    // past the head: the sorted candidates and their prefix sums go along, and empty tables for tile_walk
+    {
+        ulonglong2 *z = reinterpret_cast<ulonglong2 *>(R.table(rr, 0));
+        for (int i = tid; i < WALK_BINADES * NBINS / 2; i += HT) z[i] = make_ulonglong2(0ull, 0ull);
+        if (tid < WALK_BINADES) R.ties(rr)[tid].n = 0;
+    }
     for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
     queue_row(ST_HEAD, 6);
 }
 
 // =============================================================================
-// Kernel 5: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
+// Kernel 5: the lists of queued rows, a tile per warp: exponentials become probabilities p = e / Z
+// (sample.mojo:437-438). Where nothing is sorted, the items of their sum in vocabulary order; past a
+// sorted head, the bin tables of the walk in the binades the sum will go through: an element adds
+// rne(p / ulp) units to whatever sum lies in the binade, so one histogram of those integers per binade
+// tells where the sum crosses anything. Blocks take spans from the queue as long as there are any.
+// =============================================================================
+struct __align__(16) WalkTileShared {
+    float x[SPAN_THREADS * PITCH];
+    unsigned int hq[WALK_BINADES][NBINS];   // the low MASS_SPLIT bits of the contributions, summed, and the rest
+    unsigned int hqh[WALK_BINADES][NBINS];
+};
+
+__global__ void __launch_bounds__(SPAN_THREADS, 2) tile_walk_kernel(const __grid_constant__ RowsArgs R) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    WalkTileShared *S = reinterpret_cast<WalkTileShared *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_next();
+    pdl_wait();
+    const int work = R.queue[0] * R.nspan;
+    for (int wi = blockIdx.x; wi < work; wi += gridDim.x) {
+        const int rr = R.queue[1 + wi / R.nspan], span = wi % R.nspan, tile = span * (SPAN / TILE) + warp;
+        RowHead *head = R.head(rr);
+        const int state = head->state;
+        if (state != ST_HEAD && state != ST_PURE) continue;
+        const float Z = head->Z, yZ = __fdiv_rn(1.0f, Z);
+        const size_t gt = (size_t)rr * R.ntile + tile;
+        const int n = tile < R.ntile ? (int)R.to(rr)[tile].cnt : 0;
+        float4 *src = reinterpret_cast<float4 *>(R.elist + gt * TILE);
+        float4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (4 * (lane + 32 * i) < n) v[i] = src[lane + 32 * i];
+        if (state == ST_PURE) {
+            if (tile >= R.ntile) continue;
+            // lane l's chunk: per values from l * per on
+            const int per = (n + 31) >> 5, off = min(n, lane * per), cnt = min(per, n - off);
+            float *rows = S->x + (size_t)warp * 32 * PITCH;
+            __syncwarp();
+            const unsigned int magic = per ? (unsigned int)((0x100000000ull + (unsigned long long)per - 1ull) / (unsigned long long)per) : 0u;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int e0 = 4 * (lane + 32 * i);
+                if (e0 >= n) continue;
+                float p[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    p[u] = e0 + u < n ? prob_of(p[u], Z, yZ) : 0.0f;
+                    const int e = e0 + u, q = per > 1 ? (int)__umulhi((unsigned int)e, magic) : e;   // e / per
+                    if (e < n) rows[q * PITCH + (e - q * per)] = p[u];
+                }
+                src[lane + 32 * i] = make_float4(p[0], p[1], p[2], p[3]);
+            }
+            __syncwarp();
+            float *mine = rows + lane * PITCH;
+            float s = 0.0f;
+            for (int i = cnt; i < ((cnt + 3) & ~3); i++) mine[i] = 0.0f;
+            for (int i = 0; i < cnt; i++) s += mine[i];
+            bool care;
+            int my_place, c0 = CARE_PLACES;
+            unsigned int i0 = 0;
+            const int ni = tile_items(mine, cnt, off, n, s, R.tp[gt].est * yZ, tile,
+                [&](int k, int nc) -> Item * {
+                    if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, k); if (nc) c0 = atomicAdd(&head->ncare, nc); }
+                    i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
+                    return R.items(rr) + i0;
+                },
+                [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
+            for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
+                const int l = __ffs((int)left) - 1, k = __shfl_sync(0xffffffffu, cnt, l), at = __shfl_sync(0xffffffffu, my_place, l);
+                R.care(rr)[at * 32 + lane] = lane < k ? rows[l * PITCH + lane] : 0.0f;
+            }
+            if (lane == 0) { R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = (unsigned short)ni; }
+            __syncwarp();
+            continue;
+        }
+        // ---- past a sorted head: what it took is consumed
+        const unsigned int tau = head->plan.tau_bits;
+        const float hs = head->head_s;
+        const int j0 = hs > 0.0f ? fexpo(hs) : 0, nb = (hs > 0.0f && j0 >= -30 && j0 < 0) ? min(WALK_BINADES, -j0) : 0;
+        __syncthreads();
+        for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) { (&S->hq[0][0])[i] = 0u; (&S->hqh[0][0])[i] = 0u; }
+        __syncthreads();
+        const float half0 = fpow2(j0 - 24);   // below half a unit of the first binade: adds nothing from here on
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int e0 = 4 * (lane + 32 * i);
+            if (e0 >= n) continue;
+            float p[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                p[u] = (e0 + u < n && __float_as_uint(p[u]) < tau) ? prob_of(p[u], Z, yZ) : 0.0f;
+                if (!(p[u] >= half0)) continue;
+                const unsigned int pb = __float_as_uint(p[u]);
+                const int bin = (int)(pb >> BIN_SHIFT);
+                for (int b = 0; b < nb; b++) {
+                    const float Cm = __fmul_rn(1.5f, fpow2(j0 + b));
+                    const float tq = __fadd_rn(p[u], Cm);
+                    const float rr_ = __fsub_rn(p[u], __fsub_rn(tq, Cm));
+                    if (fabsf(rr_) == fpow2(j0 + b - 24) || p[u] >= fpow2(j0 + b - 1)) {
+                        // a rounding tie: listed (an element of a quarter of the sum cannot follow a whole head)
+                        WalkTies *t = R.ties(rr) + b;
+                        const int at = atomicAdd(&t->n, 1);
+                        if (at < TIE_CAP) t->key[at] = make_key(pb, tile * TILE + e0 + u);
+                        continue;
+                    }
+                    // p + Cm stays in Cm's binade, whose unit is the sum's: the difference of the two bit
+                    // patterns is the count of units
+                    const unsigned int qu = __float_as_uint(tq) - __float_as_uint(Cm);
+                    if (qu & MASS_LO_MASK) sred_add(&S->hq[b][bin], qu & MASS_LO_MASK);
+                    if (qu >> MASS_SPLIT) sred_add(&S->hqh[b][bin], qu >> MASS_SPLIT);
+                }
+            }
+            src[lane + 32 * i] = make_float4(p[0], p[1], p[2], p[3]);
+        }
+        __syncthreads();
+        for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) {
+            const unsigned long long q = (unsigned long long)(&S->hq[0][0])[i] + ((unsigned long long)(&S->hqh[0][0])[i] << MASS_SPLIT);
+            if (q) atomicAdd(R.table(rr, 0) + i, q);
+        }
+    }
+}
+
+// =============================================================================
+// Kernel 6: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
 // what it does not.
 // =============================================================================
 struct __align__(16) AuxF {
@@ -1260,6 +1517,7 @@ struct CtxF {
     int rr, r;
     RowCfg cfg;
     RowPlan pl;
+    int tj0, tnb;                // binades that tile_walk has left tables for
     float *list;                 // this row's [ntile][TILE]
     Item *gitems;                // this row's items
     const unsigned int *kmask;   // this row's [ntile][32]
@@ -1463,21 +1721,38 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
     return __uint_as_float(A->w_sb);
 }
 
-// Calls f(values, first position) for the row's list, four entries of a lane at a time (zero: none);
-// entry u of lane l is at first position + l + 32 u. All lanes of a warp make the same calls.
+// Calls f(values, first position, where they are) for the row's list, four entries of a lane at a time
+// (zero: none); entry u of lane l is at first position + l + 32 u. All lanes of a warp make the same
+// calls. The next eight entries of every lane are on their way while f works on the ones before: a
+// block of 16 warps needs that many to cover the way to L2.
 template <class F>
 __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
     const AuxF *A = c.A;
     IN_SHARED(A);
-    for (int t = c.warp; t < c.R->ntile; t += NWARP) {
-        const int n = A->tcnt[t];
-        float *src = c.list + (size_t)t * TILE;
-        for (int i0 = 0; i0 < n; i0 += 128) {
-            unsigned int eb[4];
+    const int ntile = c.R->ntile;
+    int t = c.warp, i0 = 0;
+    auto settle = [&]() { while (t < ntile && i0 >= A->tcnt[t]) { t += NWARP; i0 = 0; } };
+    auto fetch = [&](unsigned int (&eb)[8]) {
+        const int n = t < ntile ? A->tcnt[t] : 0;
+        const float *src = c.list + (size_t)t * TILE + i0 + c.lane;
 #pragma unroll
-            for (int u = 0; u < 4; u++) eb[u] = (i0 + u * 32 + c.lane < n) ? __float_as_uint(src[i0 + u * 32 + c.lane]) : 0u;
-            f(eb, t * TILE + i0, src + i0);
-        }
+        for (int u = 0; u < 8; u++) eb[u] = (i0 + u * 32 + c.lane < n) ? __float_as_uint(src[u * 32]) : 0u;
+    };
+    settle();
+    unsigned int nx[8];
+    fetch(nx);
+    while (t < ntile) {
+        unsigned int lo[4], hi[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) { lo[u] = nx[u]; hi[u] = nx[u + 4]; }
+        const int pos = t * TILE + i0;
+        const bool second = i0 + 128 < A->tcnt[t];
+        float *at = c.list + pos;
+        i0 += 256;
+        settle();
+        fetch(nx);
+        f(lo, pos, at);
+        if (second) f(hi, pos + 128, at + 128);
     }
 }
 
@@ -1609,7 +1884,7 @@ struct FWalk {
 struct FResume {
     int valid;
     float s; long long pos; unsigned int tau;
-    int lvl; unsigned int lo; int shift; int tie_mode; int ntie;
+    int lvl; unsigned int lo; int shift; int tie_mode; int ntie; int tabbed;
 };
 
 // position of the (nth+1)-th entry, in vocabulary order, whose bits equal `eb`
@@ -1655,18 +1930,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
     }
     for (int phase = 0; phase < 8192; phase++) {
         FCOUNT(22, 1);
-        const bool reuse = resumed && phase == 0;  // this phase's tables stand already
-        __syncthreads();
-        if (!reuse) {
-            for (int i = c.tid; i < NBINS; i += NT) { A->u.h.hq[i] = 0u; A->u.h.hqh[i] = 0u; A->u.h.hc[i] = 0u; }
-            for (int i = c.tid; i < NBINS / 32; i += NT) A->tbits[i] = 0u;
-            rs.valid = 1; rs.s = w.s; rs.pos = w.pos; rs.tau = w.tau;
-            rs.lvl = lvl; rs.lo = lo; rs.shift = shift; rs.tie_mode = tie_mode ? 1 : 0; rs.ntie = 0;
-        }
-        if (c.tid == 0) {
-            if (!reuse) A->specbin = -1;
-            A->ncand = 0; A->ntie = 0;
-        }
+        const bool reuse = resumed && phase == 0 && !rs.tabbed;  // this phase's tables stand already
         __syncthreads();
         const bool have_s = w.s > 0.0f;
         const int j = have_s ? fexpo(w.s) : 0;
@@ -1676,8 +1940,73 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         const unsigned int cm_bits = __float_as_uint(Cm);
         const bool ties_listed = tie_mode && lvl == 1 && binade_ok;
         const unsigned int wtau = w.tau;
-        int ntie = rs.ntie;
+        // tile_walk's tables hold whole bins: they serve while what is consumed ends at a bin's edge
+        const WalkTies *tt = nullptr;
+        const unsigned long long *tab = nullptr;
+        int bin_hi = NBINS;
+        if (c.tnb > 0 && ties_listed && !counting && j >= c.tj0 && j < c.tj0 + c.tnb && (wtau == 0xFFFFFFFFu || (wtau & ((1u << BIN_SHIFT) - 1u)) == 0u)) {
+            tt = c.R->ties(c.rr) + (j - c.tj0);
+            if (tt->n <= TIE_CAP) {
+                tab = c.R->table(c.rr, j - c.tj0);
+                if (wtau != 0xFFFFFFFFu) bin_hi = (int)(wtau >> BIN_SHIFT);
+            }
+        }
+        const bool tabbed = tab != nullptr;
         if (!reuse) {
+            if (!tabbed)
+                for (int i = c.tid; i < NBINS; i += NT) { A->u.h.hq[i] = 0u; A->u.h.hqh[i] = 0u; A->u.h.hc[i] = 0u; }
+            for (int i = c.tid; i < NBINS / 32; i += NT) A->tbits[i] = 0u;
+            rs.valid = 1; rs.s = w.s; rs.pos = w.pos; rs.tau = w.tau;
+            rs.lvl = lvl; rs.lo = lo; rs.shift = shift; rs.tie_mode = tie_mode ? 1 : 0; rs.ntie = 0; rs.tabbed = tabbed ? 1 : 0;
+        }
+        if (c.tid == 0) {
+            if (!reuse) A->specbin = -1;
+            A->ncand = 0; A->ntie = 0;
+        }
+        __syncthreads();
+        BinQuery qy;
+        qy.bin_hi = bin_hi; qy.spec_bits = nullptr; qy.specbin = -1;
+        qy.hq = A->u.h.hq; qy.hqh = A->u.h.hqh; qy.hc = A->u.h.hc;
+        qy.pos0 = (unsigned long long)w.pos;
+        qy.nstop = counting ? (unsigned long long)nstop : ~0ull;
+        qy.m0 = 0; qy.xq = ~0ull;
+        if (binade_ok) {
+            qy.m0 = (unsigned long long)((double)w.s * (double)inv_u);
+            unsigned long long xq = 1ull << 24;  // leaving the binade
+            if (x_ge < 3.0e38f) {
+                double t = ceil((double)x_ge * (double)inv_u);
+                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
+            }
+            if (x_gt < 3.0e38f) {
+                double t = floor((double)x_gt * (double)inv_u) + 1.0;
+                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
+            }
+            qy.xq = xq;
+        } else {
+            qy.pos0 = 0; qy.nstop = 1;  // nothing consumed yet: take the highest non-empty bin
+        }
+        auto bin_load = [&](int b, unsigned long long &q, unsigned long long &n) {
+            if (tabbed) { q = tab[b]; n = 0ull; return; }
+            q = (unsigned long long)qy.hq[b] + ((unsigned long long)qy.hqh[b] << MASS_SPLIT);
+            n = qy.hc[b];
+        };
+        int ntie = rs.ntie;
+        bool searched = false;
+        if (tabbed) {
+            // without the ties first: they only add, so the event lies in the bin found here or in a higher
+            // one, and a tie below that bin changes nothing
+            find_event_bin_with(c, qy, bin_load);
+            const int b0 = A->hit_bin;
+            if (c.tid < tt->n) {
+                const unsigned long long key = tt->key[c.tid];
+                const int b = (int)((unsigned int)(key >> 32) >> BIN_SHIFT);
+                if (b < bin_hi && b >= b0) { const int at = satom_add(&A->ntie, 1); A->tkey[at] = key; A->tbin[at] = b; }
+            }
+            __syncthreads();
+            ntie = A->ntie;
+            rs.ntie = ntie;
+            searched = ntie == 0;
+        } else if (!reuse) {
             const bool count_all = counting || !binade_ok;
             for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
                 bool rare = false;
@@ -1720,80 +2049,56 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             ntie = ties_listed ? A->ntie : 0;
             rs.ntie = ntie;
             if (ntie > TIE_CAP) { tie_mode = false; c.status |= MOLLA_ROW_SLOW_PATH; continue; }  // too many: they stop phases instead
-            if (ntie > 0) {
-                // what precedes each listed element inside its own bin (descending value, then ascending id)
-                if (c.tid < ntie) {
-                    const int b = A->tbin[c.tid];
-                    A->tpq_lo[c.tid] = 0u; A->tpq_hi[c.tid] = 0u;
-                    sred_or(&A->tbits[b >> 5], 1u << (b & 31));
-                }
-                __syncthreads();
-                int tb_lo = NBINS, tb_hi = -1;
-                for (int t = 0; t < ntie; t++) { tb_lo = min(tb_lo, A->tbin[t]); tb_hi = max(tb_hi, A->tbin[t]); }
-                const unsigned int tb_span = (unsigned int)(tb_hi - tb_lo);
-                for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
-                    bool near = false;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const unsigned int eb = ebs[u];
-                        const int bin = (int)((eb - lo) >> shift);
-                        near |= eb != 0u && eb < wtau && eb >= lo && (unsigned int)(bin - tb_lo) <= tb_span;
-                    }
-                    if (!__any_sync(0xffffffffu, near)) return;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const unsigned int eb = ebs[u];
-                        if (eb == 0u || eb >= wtau || eb < lo) continue;
-                        const int bin = (int)((eb - lo) >> shift);
-                        if (!((A->tbits[bin >> 5] >> (bin & 31)) & 1u)) continue;
-                        const float p = __uint_as_float(eb);
-                        const float tq = __fadd_rn(p, Cm);
-                        const float rr = __fsub_rn(p, __fsub_rn(tq, Cm));
-                        if (fabsf(rr) == halfu || p >= bigthr) continue;
-                        const unsigned int qu = __float_as_uint(tq) - cm_bits;
-                        const unsigned long long key = make_key(eb, pos0 + c.lane + 32 * u);
-                        for (int t = 0; t < ntie; t++)
-                            if (A->tbin[t] == bin && key > A->tkey[t] && qu) {  // two halves, as in the bin tables
-                                sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
-                                if (qu >> MASS_SPLIT) sred_add(&A->tpq_hi[t], qu >> MASS_SPLIT);
-                            }
-                    }
-                });
-                __syncthreads();
-            }
         }
-        BinQuery qy;
-        qy.bin_hi = NBINS; qy.spec_bits = nullptr;
-        qy.hq = A->u.h.hq; qy.hqh = A->u.h.hqh; qy.hc = A->u.h.hc;
-        qy.pos0 = (unsigned long long)w.pos;
-        qy.nstop = counting ? (unsigned long long)nstop : ~0ull;
-        qy.m0 = 0; qy.xq = ~0ull;
-        if (binade_ok) {
-            qy.m0 = (unsigned long long)((double)w.s * (double)inv_u);
-            unsigned long long xq = 1ull << 24;  // leaving the binade
-            if (x_ge < 3.0e38f) {
-                double t = ceil((double)x_ge * (double)inv_u);
-                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
+        if (!reuse && ntie > 0) {
+            // what precedes each listed element inside its own bin (descending value, then ascending id)
+            if (c.tid < ntie) {
+                const int b = A->tbin[c.tid];
+                A->tpq_lo[c.tid] = 0u; A->tpq_hi[c.tid] = 0u;
+                sred_or(&A->tbits[b >> 5], 1u << (b & 31));
             }
-            if (x_gt < 3.0e38f) {
-                double t = floor((double)x_gt * (double)inv_u) + 1.0;
-                if (t < (double)xq) xq = (t <= 0.0) ? 0ull : (unsigned long long)t;
-            }
-            qy.xq = xq;
-        } else {
-            qy.pos0 = 0; qy.nstop = 1;  // nothing consumed yet: take the highest non-empty bin
+            __syncthreads();
+            int tb_lo = NBINS, tb_hi = -1;
+            for (int t = 0; t < ntie; t++) { tb_lo = min(tb_lo, A->tbin[t]); tb_hi = max(tb_hi, A->tbin[t]); }
+            const unsigned int tb_span = (unsigned int)(tb_hi - tb_lo);
+            for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+                bool near = false;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned int eb = ebs[u];
+                    const int bin = (int)((eb - lo) >> shift);
+                    near |= eb != 0u && eb < wtau && eb >= lo && (unsigned int)(bin - tb_lo) <= tb_span;
+                }
+                if (!__any_sync(0xffffffffu, near)) return;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned int eb = ebs[u];
+                    if (eb == 0u || eb >= wtau || eb < lo) continue;
+                    const int bin = (int)((eb - lo) >> shift);
+                    if (!((A->tbits[bin >> 5] >> (bin & 31)) & 1u)) continue;
+                    const float p = __uint_as_float(eb);
+                    const float tq = __fadd_rn(p, Cm);
+                    const float rr = __fsub_rn(p, __fsub_rn(tq, Cm));
+                    if (fabsf(rr) == halfu || p >= bigthr) continue;
+                    const unsigned int qu = __float_as_uint(tq) - cm_bits;
+                    const unsigned long long key = make_key(eb, pos0 + c.lane + 32 * u);
+                    for (int t = 0; t < ntie; t++)
+                        if (A->tbin[t] == bin && key > A->tkey[t] && qu) {  // two halves, as in the bin tables
+                            sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
+                            if (qu >> MASS_SPLIT) sred_add(&A->tpq_hi[t], qu >> MASS_SPLIT);
+                        }
+                }
+            });
+            __syncthreads();
         }
         if (c.tid < ntie) {
             if (!reuse) A->tpqm[c.tid] = (unsigned long long)A->tpq_lo[c.tid] + ((unsigned long long)A->tpq_hi[c.tid] << MASS_SPLIT);
             A->tc[c.tid] = 0ull;
         }
         __syncthreads();
-        qy.specbin = A->specbin;
-        find_event_bin_adj(c, qy,
-            [&](int b, unsigned long long &q, unsigned long long &n) {
-                q = (unsigned long long)qy.hq[b] + ((unsigned long long)qy.hqh[b] << MASS_SPLIT);
-                n = qy.hc[b];
-            },
+        if (!tabbed) qy.specbin = A->specbin;
+        if (!searched)
+        find_event_bin_adj(c, qy, bin_load,
             [&](unsigned long long (&q)[BPT], unsigned long long eq) -> bool {
                 if (ntie == 0) return false;
                 // the mass before each listed element: the bins above its own (the thread that
@@ -1921,6 +2226,94 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
     c.status |= MOLLA_ROW_DEGENERATE;
 }
 
+// A row that sorts nothing, once tile_walk has written the items of its probabilities: the walk to their
+// sum leaves the sum before every stretch, so the draw (sample.mojo:580-590) is a search among those and
+// then inside one stretch. Returns false where the general way has to be gone.
+__device__ bool tail_pure(CtxF &c, float u01, float Z) {
+    const RowsArgs &R = *c.R;
+    WalkShared *W = reinterpret_cast<WalkShared *>(c.A->tile);
+    AuxF *A = c.A;
+    RowHead *head = R.head(c.rr);
+    const int nitem = head->nitem;
+    if (nitem > H_ITEMS || head->ncare > CARE_PLACES) return false;
+    WalkLoads<NT> wl;
+    wl.load(R, c.rr);
+    __syncthreads();
+    const unsigned int nrec = wl.order(W, R.ntile, nitem);
+    if (nrec > (unsigned int)H_REC) return false;
+    if (c.warp == 0) {
+        float z = 0.0f;
+        const bool fine = walk_records(W, R.care(c.rr), (int)nrec, z);
+        if (c.lane == 0) { A->b_s = z; A->b_event = fine ? 1 : 0; A->evt_thread = 0x7fffffff; }
+    }
+    __syncthreads();
+    if (!A->b_event) return false;
+    const float sum = A->b_s, target = __fmul_rn(u01, sum);
+    // the first stretch (runs, then a careful chunk) behind which the sum exceeds the target
+    for (int q = c.tid; q <= (int)nrec; q += NT)
+        if (target < __uint_as_float(W->sbs[q + 1])) { atomicMin(&A->evt_thread, q); break; }
+    __syncthreads();
+    const int q = A->evt_thread;
+    if (c.warp != 0) return true;
+    if (q == 0x7fffffff) {   // the walk fell off the end: the reference returns the last token of the vocabulary
+        if (c.lane == 0) finish_row(R.a, c.r, c.cfg, c.status, R.a.V - 1, Z, sum, target, 0.0f);
+        return true;
+    }
+    unsigned int sb = W->sbs[q];
+    // the stretch's items: behind the record before it, up to its own
+    const unsigned int k0 = q > 0 ? W->rec[q - 1].k : 0u;
+    int lo = 0, seen = 0;
+    // (records are items in order: find the q-th one, counting as order() did)
+    for (int i0 = 0; i0 < nitem && seen < q; i0 += 32) {
+        const int i = i0 + c.lane;
+        bool care = false;
+        if (i < nitem) {
+            const Item it = W->items[i];
+            care = it.kind() != K_RUN;
+            if (!care && i > 0) { const Item p = W->items[i - 1]; care = p.kind() == K_RUN && p.jb() != it.jb(); }
+        }
+        const unsigned int m = __ballot_sync(0xffffffffu, care);
+        const int n = __popc(m);
+        if (seen + n >= q) { lo = i0 + (int)__fns(m, 0, q - seen) + 1; seen = q; }
+        else seen += n;
+    }
+    (void)k0;
+    // item by item from there
+    int tile = -1, at = 0;
+    for (int i = lo; i < nitem && tile < 0; i++) {
+        const Item it = W->items[i];
+        const int n = it.cnt(), off = it.off();
+        if (it.kind() == K_RUN && !(target < __uint_as_float(sb + it.ka))) { sb += it.ka; continue; }
+        const float *v = c.list + (size_t)it.tile() * TILE + off;
+        float s = __uint_as_float(sb);
+        if (it.kind() == K_RUN) {
+            // the values of a run round by themselves: each lane adds up the units of its share
+            const int j = fexpo(s), per = (n + 31) >> 5, b0 = min(n, c.lane * per), b1 = min(n, b0 + per);
+            const float Cm = __fmul_rn(1.5f, fpow2(j));
+            unsigned int k = 0u;
+            for (int e = b0; e < b1; e++) k += __float_as_uint(__fadd_rn(v[e], Cm)) - __float_as_uint(Cm);
+            const unsigned int inc = warp_incl_scan(k, c.lane);
+            const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(sb + inc));
+            const int l = hit ? __ffs((int)hit) - 1 : 31;
+            const unsigned int before = __shfl_sync(0xffffffffu, inc - k, l);
+            s = __uint_as_float(sb + before);
+            const int e0 = min(n, l * per), e1 = min(n, e0 + per);
+            for (int e = e0; e < e1 && tile < 0; e++) {
+                s = __fadd_rn(s, v[e]);
+                if (target < s) { tile = it.tile(); at = off + e; }
+            }
+        } else {
+            for (int e = 0; e < n && tile < 0; e++) {
+                s = __fadd_rn(s, v[e]);
+                if (target < s) { tile = it.tile(); at = off + e; }
+            }
+        }
+        sb = __float_as_uint(s);
+    }
+    if (c.lane == 0) finish_row(R.a, c.r, c.cfg, c.status, tile < 0 ? R.a.V - 1 : token_of(c, tile, at), Z, sum, target, 0.0f);
+    return true;
+}
+
 __device__ void tail_row(const RowsArgs &R, int rr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CtxF c;
@@ -2004,6 +2397,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         }
     }
 
+    if (state == ST_PURE && tail_pure(c, u01, Z)) return;
     if (g.pure) {
         // ---- nothing sorted: the draw walks the vocabulary in order (sample.mojo:365-369, 580-594):
         // probabilities p = e / Z (:437-438), what min-p drops becomes zero
@@ -2012,9 +2406,12 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
             float *src = c.list + (size_t)t * TILE;
             float s = 0.0f;
             for (int i = c.lane; i < n; i += 32) {
-                float p = prob_of(src[i], Z, yZ);
-                if (__float_as_uint(p) < minp_pbits) p = 0.0f;
-                src[i] = p;
+                float p = src[i];
+                if (state != ST_PURE) {   // (else tile_walk has done it)
+                    p = prob_of(p, Z, yZ);
+                    if (__float_as_uint(p) < minp_pbits) p = 0.0f;
+                    src[i] = p;
+                }
                 s += p;
             }
             s = warp_sum(s);
@@ -2198,7 +2595,9 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     // ---- past the head: the cut walk, then the draw walk, over the probabilities
     // (sample.mojo:437-438); what the head took is consumed
     const unsigned int tau_bits = head_overflow ? 0xffffffffu : c.pl.tau_bits;
-    for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
+    c.tnb = 0; c.tj0 = 0;
+    if (state == ST_HEAD && head_s > 0.0f && fexpo(head_s) >= -30 && fexpo(head_s) < 0) { c.tj0 = fexpo(head_s); c.tnb = min(WALK_BINADES, -c.tj0); }
+    if (state != ST_HEAD) for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
 #pragma unroll
         for (int u = 0; u < 4; u++)
             if (eb[u]) src[u * 32 + c.lane] = eb[u] >= tau_bits ? 0.0f : prob_of(__uint_as_float(eb[u]), Z, yZ);
@@ -2330,6 +2729,7 @@ size_t lay_out(RowsArgs &A, char *ws, int rows, int V) {
     A.box_stride = (long long)al(sizeof(RowHead) + ((nt + 1) & ~(size_t)1) * sizeof(TileOut) + HEADCAP * (sizeof(unsigned long long) + sizeof(float)) +
                                  CARE_PLACES * 32 * sizeof(float) + items * sizeof(Item));
     A.box = (char *)take((size_t)rows * (size_t)A.box_stride);
+    A.walk = take((size_t)rows * WALK_BYTES);
     A.queue = (int *)take((size_t)(rows + 1) * sizeof(int));
     return o;
 }
@@ -2363,6 +2763,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         e = cudaFuncSetAttribute(tile_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_exp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(row_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AuxF));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkTileShared));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(row_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadShared));
         if (e == cudaSuccess && dev < 64) ready[dev] = true;
     }
@@ -2381,6 +2782,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         if (e == cudaSuccess) e = launch(row_plan_kernel, (unsigned int)A.rows, NT, 0, st, A);
         if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
         if (e == cudaSuccess) e = launch(row_head_kernel, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
+        if (e == cudaSuccess) e = launch(tile_walk_kernel, spans < 2u * (unsigned int)sms ? spans : 2u * (unsigned int)sms, SPAN_THREADS, sizeof(WalkTileShared), st, A);
         if (e == cudaSuccess) e = launch(row_tail_kernel, (unsigned int)(A.rows < sms ? A.rows : sms), NT, sizeof(AuxF), st, A);
     }
     if (e != cudaSuccess) {
