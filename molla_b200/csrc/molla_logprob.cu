@@ -1,0 +1,312 @@
+// Logprobs of the raw logits (sample.mojo:268-293) for rows of 4096 logits and more: the chosen token's,
+// the top N's, or a whole row's. A tile of 1024 logits belongs to one warp, so a few rows fill the chip
+// as well as many: one block per row, as for short rows, took 97 us for 64 rows of 151936 logits and left
+// half of the SMs idle.
+//
+//   lp_tiles  every tile: its maximum and the sum of exp(z - maximum), accumulated in fp64
+//                                           (bound: HBM, 4 bytes per logit, and an exponential per logit)
+//   lp_rows   every row: maximum, logarithm of the sum, the chosen token, the top N. The N-th largest of
+//             the tiles' maxima bounds the N-th largest logit from below, so only tiles whose maximum
+//             reaches it, N of them but for ties, are looked at again
+//   lp_write  every tile of a whole row's logprobs: z - maximum - logarithm (bound: HBM, 8 bytes per logit)
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+#include <stdio.h>
+
+#include "molla_exact.cuh"
+#include "molla_logprob.h"
+
+namespace {
+
+constexpr int LT_ = 256;          // threads of a block: eight warps, eight tiles
+constexpr int LTILE = 1024;
+constexpr int LREST = 64;         // a row's last piece of fewer logits goes with the tile before it
+constexpr int LMAX_TILES = 704;
+constexpr int LCAND = 512;
+
+struct LpArgs {
+    const float *logits; long long row_stride; int B, V;
+    const int *tokens; int top_n; float *chosen; int *top_ids; float *top_lps;
+    const int *rows; int n_logit_rows; float softcap;
+    float *out;                   // whole rows' logprobs, or nullptr
+    float *stats; long long stats_row, stats_tile;   // tile t of row r: four floats at stats + r * stats_row + t * stats_tile
+    int ntile;
+};
+
+__device__ __forceinline__ float *stat_of(const LpArgs &a, int r, int t) { return a.stats + (long long)r * a.stats_row + (long long)t * a.stats_tile; }
+// which row of the block batch row r reads; -1 for a stale index (the row's sampling call has reported it)
+__device__ __forceinline__ long long logit_row(const LpArgs &a, int r) {
+    const long long l = a.rows ? (long long)a.rows[r] : (long long)r;
+    return (a.rows && (l < 0 || (a.n_logit_rows > 0 && l >= a.n_logit_rows))) ? -1 : l;
+}
+__device__ __forceinline__ int tile_end(const LpArgs &a, int t) { return t == a.ntile - 1 ? a.V : (t + 1) * LTILE; }
+__device__ __forceinline__ float capped(const LpArgs &a, float x) { return a.softcap > 0.0f ? softcap_pinned(x, a.softcap) : x; }
+
+__global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
+    const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
+    if (t >= a.ntile) return;
+    const long long lrow = logit_row(a, r);
+    if (lrow < 0) return;
+    const float *z = a.logits + lrow * a.row_stride + (long long)t * LTILE;
+    const int n = tile_end(a, t) - t * LTILE;
+    float x[34];
+    if ((reinterpret_cast<uintptr_t>(z) & 15u) == 0 && n >= LTILE) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(z) + lane + 32 * i);
+            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++) x[i] = lane + 32 * i < n ? __ldg(z + lane + 32 * i) : -INFINITY;
+    }
+    x[32] = LTILE + lane < n ? __ldg(z + LTILE + lane) : -INFINITY;
+    x[33] = LTILE + 32 + lane < n ? __ldg(z + LTILE + 32 + lane) : -INFINITY;
+    float m = -INFINITY;
+    if (a.softcap > 0.0f) {
+#pragma unroll
+        for (int i = 0; i < 34; i++) if (x[i] > -INFINITY) x[i] = softcap_pinned(x[i], a.softcap);
+    }
+#pragma unroll
+    for (int i = 0; i < 34; i++) m = fmaxf(m, x[i]);
+    m = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(m)));
+    double s0 = 0.0, s1 = 0.0;
+    if (m > -INFINITY) {
+#pragma unroll
+        for (int i = 0; i < 34; i += 2) {
+            s0 += (double)expf_pinned_nonpos(__fsub_rn(x[i], m));
+            s1 += (double)expf_pinned_nonpos(__fsub_rn(x[i + 1], m));
+        }
+    }
+    s0 += s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    if (lane == 0) {   // (whole rows' logprobs keep this in the tile's own output, which need not be aligned)
+        float *o = stat_of(a, r, t);
+        const unsigned long long b = (unsigned long long)__double_as_longlong(s0);
+        o[0] = m; o[1] = __uint_as_float((unsigned int)b); o[2] = __uint_as_float((unsigned int)(b >> 32));
+    }
+}
+
+__global__ void __launch_bounds__(LT_) lp_rows(const __grid_constant__ LpArgs a) {
+    __shared__ float tm[LMAX_TILES];
+    __shared__ unsigned short pick[LMAX_TILES];
+    __shared__ unsigned long long cand[LCAND];
+    __shared__ double wsd[LT_ / 32];
+    __shared__ float wsf[LT_ / 32];
+    __shared__ int wsi[LT_ / 32];
+    __shared__ int npick, ncand;
+    __shared__ float s_thr;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, top_n = a.top_n;
+    const long long lrow = logit_row(a, r);
+    if (lrow < 0) {
+        if (a.chosen && tid == 0) a.chosen[r] = 0.0f;
+        for (int i = tid; i < top_n; i += LT_) { a.top_ids[(long long)r * top_n + i] = -1; a.top_lps[(long long)r * top_n + i] = 0.0f; }
+        return;
+    }
+    const float *z = a.logits + lrow * a.row_stride;
+    constexpr int PER = (LMAX_TILES + LT_ - 1) / LT_;
+    double sum[PER];
+    float m[PER], top = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int t = tid + u * LT_;
+        sum[u] = 0.0; m[u] = -INFINITY;
+        if (t < a.ntile) {
+            const float *o = stat_of(a, r, t);
+            m[u] = o[0];
+            sum[u] = __longlong_as_double((long long)((unsigned long long)__float_as_uint(o[1]) | ((unsigned long long)__float_as_uint(o[2]) << 32)));
+            tm[t] = m[u];
+        }
+        top = fmaxf(top, m[u]);
+    }
+    top = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(top)));
+    if (lane == 0) wsf[warp] = top;
+    if (tid == 0) { npick = 0; ncand = 0; s_thr = -INFINITY; }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < LT_ / 32; w++) top = fmaxf(top, wsf[w]);
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < PER; u++)
+        if (m[u] > -INFINITY) s += sum[u] * exp((double)m[u] - (double)top);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) wsd[warp] = s;
+    __syncthreads();
+    s = 0.0;
+#pragma unroll
+    for (int w = 0; w < LT_ / 32; w++) s += wsd[w];
+    const float offset = (float)log(s);
+    if (a.out) {   // a copy for every tile, in the tile's own output
+        for (int t = tid; t < a.ntile; t += LT_) { float *o = stat_of(a, r, t); o[0] = top; o[1] = offset; }
+        return;
+    }
+    if (a.chosen && a.tokens && tid == 0) {
+        const int t = a.tokens[r];
+        a.chosen[r] = (t >= 0 && t < a.V) ? __fsub_rn(__fsub_rn(capped(a, __ldg(z + t)), top), offset) : 0.0f;
+    }
+    if (top_n == 0) return;
+    // the tiles whose maximum is among the top_n largest; equal maxima count in order
+    if (a.ntile >= top_n) {
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int t = tid + u * LT_;
+            if (t >= a.ntile) break;
+            int above = 0;
+            for (int o = 0; o < a.ntile; o++) above += (tm[o] > m[u] || (tm[o] == m[u] && o < t)) ? 1 : 0;
+            if (above == top_n - 1) s_thr = m[u];
+        }
+    }
+    __syncthreads();
+    const float thr = s_thr;
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int t = tid + u * LT_;
+        if (t < a.ntile && m[u] >= thr) pick[satom_add(&npick, 1)] = (unsigned short)t;
+    }
+    __syncthreads();
+    for (int i = warp; i < npick; i += LT_ / 32) {
+        const int t = pick[i], e1 = tile_end(a, t);
+        for (int e = t * LTILE + lane; e < e1; e += 32 * 8) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = e + 32 * u < e1 ? __ldg(z + e + 32 * u) : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (e + 32 * u >= e1) continue;
+                const float x = capped(a, v[u]);
+                if (x >= thr) {
+                    const int pos = satom_add(&ncand, 1);
+                    if (pos < LCAND) cand[pos] = ((unsigned long long)fkey(x) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned int)(e + 32 * u));
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const int n = ncand;
+    if (n <= LCAND) {
+        for (int i = tid; i < n; i += LT_) {
+            const unsigned long long mine = cand[i];
+            int rank = 0;
+            for (int j = 0; j < n; j++) rank += cand[j] > mine ? 1 : 0;
+            if (rank < top_n) {
+                const int id = (int)(0xFFFFFFFFu - (unsigned int)(mine & 0xFFFFFFFFull));
+                a.top_ids[(long long)r * top_n + rank] = id;
+                a.top_lps[(long long)r * top_n + rank] = __fsub_rn(__fsub_rn(fkey_inv((unsigned int)(mine >> 32)), top), offset);
+            }
+        }
+        for (int i = n + tid; i < top_n; i += LT_) { a.top_ids[(long long)r * top_n + i] = -1; a.top_lps[(long long)r * top_n + i] = 0.0f; }
+        return;
+    }
+    // More logits at or above the threshold than the buffer holds (a flat or heavily quantised row): the N
+    // largest one after the other, each the first in the order (value descending, index ascending) behind
+    // the one before it. A pass per pick.
+    float lastv = INFINITY;
+    int lasti = -1;
+    for (int k = 0; k < top_n; k++) {
+        float bv = -INFINITY;
+        int bi = 0x7fffffff;
+        for (int i = tid; i < a.V; i += LT_) {
+            const float x = capped(a, __ldg(z + i));
+            const bool behind = x < lastv || (x == lastv && i > lasti);
+            if (behind && (x > bv || (x == bv && i < bi))) { bv = x; bi = i; }
+        }
+        warp_argmax(bv, bi);
+        __syncthreads();
+        if (lane == 0) { wsf[warp] = bv; wsi[warp] = bi; }
+        __syncthreads();
+        bv = wsf[0]; bi = wsi[0];
+        for (int w = 1; w < LT_ / 32; w++)
+            if (wsf[w] > bv || (wsf[w] == bv && wsi[w] < bi)) { bv = wsf[w]; bi = wsi[w]; }
+        const bool found = bi != 0x7fffffff;
+        if (tid == 0) {
+            a.top_ids[(long long)r * top_n + k] = found ? bi : -1;
+            a.top_lps[(long long)r * top_n + k] = found ? __fsub_rn(__fsub_rn(bv, top), offset) : 0.0f;
+        }
+        lastv = bv; lasti = bi;
+        if (!found) lastv = -INFINITY;
+    }
+}
+
+__global__ void __launch_bounds__(LT_) lp_write(const __grid_constant__ LpArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
+    const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
+    if (t >= a.ntile) return;
+    const float *z = a.logits + (long long)r * a.row_stride + (long long)t * LTILE;
+    float *o = stat_of(a, r, t);   // this is also where the tile's logprobs go
+    const int n = tile_end(a, t) - t * LTILE;
+    const float top = o[0], offset = o[1];
+    float x[34];
+    const bool vec = (reinterpret_cast<uintptr_t>(z) & 15u) == 0 && (reinterpret_cast<uintptr_t>(o) & 15u) == 0 && n >= LTILE;
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(z) + lane + 32 * i);
+            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++) x[i] = lane + 32 * i < n ? __ldg(z + lane + 32 * i) : 0.0f;
+    }
+    x[32] = LTILE + lane < n ? __ldg(z + LTILE + lane) : 0.0f;
+    x[33] = LTILE + 32 + lane < n ? __ldg(z + LTILE + 32 + lane) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 34; i++) x[i] = __fsub_rn(__fsub_rn(x[i], top), offset);
+    __syncwarp();   // every lane has read the tile's copy
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) __stcs(reinterpret_cast<float4 *>(o) + lane + 32 * i, make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++)
+            if (lane + 32 * i < n) __stcs(o + lane + 32 * i, x[i]);
+    }
+    if (LTILE + lane < n) o[LTILE + lane] = x[32];
+    if (LTILE + 32 + lane < n) o[LTILE + 32 + lane] = x[33];
+}
+
+cudaError_t lp_launch(void (*kernel)(LpArgs), unsigned int blocks, cudaStream_t st, const LpArgs &a) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(LT_); cfg.stream = st;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+int tiles_of(int V) {
+    const int full = V / LTILE, rest = V % LTILE;
+    return full + (rest >= LREST ? 1 : 0);
+}
+
+}  // namespace
+
+bool molla_logprob_tiled(int V) { return V >= 4096 && tiles_of(V) <= LMAX_TILES; }
+size_t molla_logprob_workspace_bytes(int B, int V) { return (size_t)B * (size_t)tiles_of(V) * 4 * sizeof(float); }
+
+cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int B, int V, const int *tokens, int top_n, float *chosen,
+                                 int *top_ids, float *top_lps, const int *rows, int n_logit_rows, float softcap, void *workspace,
+                                 float *full_out, cudaStream_t st) {
+    LpArgs a = {};
+    a.logits = logits; a.row_stride = row_stride; a.B = B; a.V = V;
+    a.tokens = tokens; a.top_n = top_n; a.chosen = chosen; a.top_ids = top_ids; a.top_lps = top_lps;
+    a.rows = rows; a.n_logit_rows = n_logit_rows; a.softcap = softcap; a.out = full_out;
+    a.ntile = tiles_of(V);
+    if (full_out) { a.stats = full_out; a.stats_row = V; a.stats_tile = LTILE; }
+    else { a.stats = (float *)workspace; a.stats_row = 4ll * a.ntile; a.stats_tile = 4; }
+    const unsigned int blocks = (unsigned int)B * (unsigned int)((a.ntile + 7) / 8);
+    cudaError_t e = lp_launch(lp_tiles, blocks, st, a);
+    if (e == cudaSuccess) e = lp_launch(lp_rows, (unsigned int)B, st, a);
+    if (e == cudaSuccess && full_out) e = lp_launch(lp_write, blocks, st, a);
+    return e;
+}

@@ -1,0 +1,14 @@
+// Logprobs of rows that are long enough to be cut into tiles (molla_logprob.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+// Whether rows of V logits go this way; shorter ones are one block's work.
+bool molla_logprob_tiled(int V);
+size_t molla_logprob_workspace_bytes(int B, int V);
+
+// The chosen tokens' and the top N's logprobs (workspace of molla_logprob_workspace_bytes), or with
+// `full_out` [B x V] whole rows' (no workspace; rows = batch rows, no softcap).
+cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int B, int V, const int *tokens, int top_n, float *chosen,
+                                 int *top_ids, float *top_lps, const int *rows, int n_logit_rows, float softcap, void *workspace,
+                                 float *full_out, cudaStream_t st);

@@ -237,39 +237,43 @@ struct SpanScratch {
     int nhits;
 };
 
-// Logits [c0, c0 + SPAN) of row r, capped, masked, biased and penalised, to `sx`: lane l of tile w
-// finds its 32 at sx[(32 w + l) * PITCH]. What lies past the row's end is -inf. Threads
-// 0..SPAN_THREADS-1 work (`active`), all threads of the block take part in the barriers; each warp
-// may then use its own tile. 16-byte asynchronous copies where the row starts on such a boundary,
-// 4-byte ones elsewhere.
-__device__ void load_span(const BatchArgs &a, const RowCfg &c, int r, int c0, float *sx, SpanScratch *s, bool active) {
+// Logits [c0, c0 + SPAN) of logit row `lrow` on their way to `sx`: lane l of tile w will find its 32 at
+// sx[(32 w + l) * PITCH]. What lies past the row's end is -inf. 16-byte asynchronous copies where the row
+// starts on such a boundary, 4-byte ones elsewhere.
+__device__ __forceinline__ void span_fetch(const BatchArgs &a, long long lrow, int c0, float *sx) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float *src = a.logits + c.lrow * a.row_stride + c0;
+    const float *src = a.logits + lrow * a.row_stride + c0;
+    const int n = min(SPAN, a.V - c0), e0 = warp * TILE;
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int ch = i * 32 + lane, e = e0 + ch * 4;
+            float *dst = sx + (warp * 32 + (ch >> 3)) * PITCH + (ch & 7) * 4;
+            if (e + 4 <= n) cp16(dst, src + e);
+            else {
+#pragma unroll
+                for (int u = 0; u < 4; u++) dst[u] = (e + u < n) ? __ldg(src + e + u) : -INFINITY;
+            }
+        }
+    } else {
+#pragma unroll 8
+        for (int i = 0; i < 32; i++) {
+            const int e = e0 + i * 32 + lane;
+            float *dst = sx + (warp * 32 + i) * PITCH + lane;
+            if (e < n) cp4(dst, src + e);
+            else *dst = -INFINITY;
+        }
+    }
+}
+
+// Waits for what span_fetch asked for and caps, masks, biases and penalises it. Threads
+// 0..SPAN_THREADS-1 work (`active`), all threads of the block take part in the barriers; each warp may
+// then use its own tile.
+__device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, float *sx, SpanScratch *s, bool active) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(SPAN, a.V - c0);
     const int e0 = warp * TILE;
     float *mine = sx + (size_t)tid * PITCH;
-    if (active) {
-        if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int ch = i * 32 + lane, e = e0 + ch * 4;
-                float *dst = sx + (warp * 32 + (ch >> 3)) * PITCH + (ch & 7) * 4;
-                if (e + 4 <= n) cp16(dst, src + e);
-                else {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) dst[u] = (e + u < n) ? __ldg(src + e + u) : -INFINITY;
-                }
-            }
-        } else {
-#pragma unroll 8
-            for (int i = 0; i < 32; i++) {
-                const int e = e0 + i * 32 + lane;
-                float *dst = sx + (warp * 32 + i) * PITCH + lane;
-                if (e < n) cp4(dst, src + e);
-                else *dst = -INFINITY;
-            }
-        }
-    }
     const bool patching = c.npatch > 0;
     if (patching) {
         if (active) {
@@ -354,9 +358,13 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
     pdl_wait();
     const int rr = blockIdx.x / A.nspan, span = blockIdx.x - rr * A.nspan, r = A.r0 + rr;
     const BatchArgs &a = A.a;
+    {   // the logits first: what the settings say about them can wait
+        const long long lrow = a.rows ? (long long)a.rows[r] : (long long)r;
+        if (lrow >= 0 && (!a.rows || a.n_logit_rows <= 0 || lrow < a.n_logit_rows)) span_fetch(a, lrow, span * SPAN, S->x);
+    }
     const RowCfg c = row_cfg(a, r);
-    if (c.status) return;
-    load_span(a, c, r, span * SPAN, S->x, &S->s, true);
+    if (c.status) { cp_wait(); return; }
+    span_ready(a, c, r, span * SPAN, S->x, &S->s, true);
     const int lane = threadIdx.x & 31, tile = span * (SPAN / TILE) + (threadIdx.x >> 5);
     if (tile >= A.ntile) return;
     const float *mine = S->x + threadIdx.x * PITCH;
@@ -606,13 +614,34 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
 // =============================================================================
 // Kernel 3: exponentials, candidates, items.
 // =============================================================================
-// The items of a tile whose lane `lane` holds `cnt` values v(0..cnt-1) (padded with zeros to a multiple
-// of four), estimated sum before the tile `est`. `off` = the lane's first entry in the tile's list.
-// Returns the number of items; `care` = this lane's values are wanted one by one.
+// A tile's list in shared memory: entry e at list[skew(e)] (a word is left out after every 32, so that
+// lanes that read their own chunks meet different banks). Lane l's chunk is entries [off, off + cnt):
+// equal shares of an odd number, or 32.
+__device__ __forceinline__ int skew(int e) { return e + (e >> 5); }
+struct TileChunk { int cnt, off, total; float csum; };
+__device__ __forceinline__ TileChunk tile_chunk(const float *list, int total) {
+    TileChunk c;
+    int per = (total + 31) >> 5;
+    if (per < 32) per |= 1;
+    c.total = total;
+    c.off = min(total, (int)(threadIdx.x & 31) * per);
+    c.cnt = min(per, total - c.off);
+    float s0 = 0.0f, s1 = 0.0f;
+    int i = 0;
+    for (; i + 2 <= c.cnt; i += 2) { s0 += list[skew(c.off + i)]; s1 += list[skew(c.off + i + 1)]; }
+    if (i < c.cnt) s0 += list[skew(c.off + i)];
+    c.csum = s0 + s1;
+    return c;
+}
+
+// The items of a tile's list cut into chunks, `est` = the estimated sum before the tile. Returns the
+// number of items; `care` = this lane's values are wanted one by one.
 // `alloc(n, c)` is called by all lanes with the number of items and of careful chunks among them and
 // returns where the items go; place(i) says where the i-th careful chunk's values go (255: nowhere).
 template <class ALLOC, class PLACE>
-__device__ __forceinline__ int tile_items(const float *row, int cnt, int off, int total, float csum, float est, int tile, ALLOC alloc, PLACE place, bool &care, int &my_place) {
+__device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch, float est, int tile, ALLOC alloc, PLACE place, bool &care, int &my_place) {
+    const int cnt = ch.cnt, off = ch.off, total = ch.total;
+    const float csum = ch.csum;
     const int lane = threadIdx.x & 31;
     const float inc = warp_incl_scan(csum, lane);
     float ex = __shfl_up_sync(0xffffffffu, inc, 1);
@@ -630,34 +659,25 @@ __device__ __forceinline__ int tile_items(const float *row, int cnt, int off, in
         if (usable) {
             const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
             const float C2 = __fmul_rn(1.5f, fpow2(jl + 1)), h2 = fpow2(jl - 23);
-            for (int i = 0; i < cnt; i += 4) {
-                const float4 v4 = *reinterpret_cast<const float4 *>(row + i);
-                const float v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const float q = __fsub_rn(__fadd_rn(v[u], C1), C1);
-                    bad |= (fabsf(__fsub_rn(v[u], q)) == h1) | (v[u] >= b1);
-                    da = __fadd_rn(da, q);
-                    const float q2 = __fsub_rn(__fadd_rn(v[u], C2), C2);
-                    bad |= two & (fabsf(__fsub_rn(v[u], q2)) == h2);
-                    db = __fadd_rn(db, q2);
-                }
+            for (int i = 0; i < cnt; i++) {
+                const float v = list[skew(off + i)];
+                const float q = __fsub_rn(__fadd_rn(v, C1), C1);
+                bad |= (fabsf(__fsub_rn(v, q)) == h1) | (v >= b1);
+                da = __fadd_rn(da, q);
+                const float q2 = __fsub_rn(__fadd_rn(v, C2), C2);
+                bad |= two & (fabsf(__fsub_rn(v, q2)) == h2);
+                db = __fadd_rn(db, q2);
             }
         }
     } else if (usable) {
         const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
-        float d1 = 0.0f;
-        for (int i = 0; i < cnt; i += 4) {
-            const float4 v4 = *reinterpret_cast<const float4 *>(row + i);
-            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const float q = __fsub_rn(__fadd_rn(v[u], C1), C1);
-                bad |= (fabsf(__fsub_rn(v[u], q)) == h1) | (v[u] >= b1);
-                if (u & 1) d1 = __fadd_rn(d1, q); else da = __fadd_rn(da, q);
-            }
+#pragma unroll 4
+        for (int i = 0; i < cnt; i++) {
+            const float v = list[skew(off + i)];
+            const float q = __fsub_rn(__fadd_rn(v, C1), C1);
+            bad |= (fabsf(__fsub_rn(v, q)) == h1) | (v >= b1);
+            da = __fadd_rn(da, q);
         }
-        da = __fadd_rn(da, d1);
     }
     const bool step = nonempty && (!usable || bad);
     const unsigned int ne = __ballot_sync(0xffffffffu, nonempty);
@@ -725,13 +745,17 @@ __device__ __forceinline__ int tile_items(const float *row, int cnt, int off, in
     return n;
 }
 
-struct TileEval { int cnt, off, total; unsigned int keep; float csum; };
+struct TileEval { int total; unsigned int keep; };
 
 // The exponentials (temperature and softmax numerator, sample.mojo:419-434) of a tile's logits that
-// reach `thr`, packed to the front of every lane's own part of shared memory.
+// reach `thr`, packed into the tile's list (over the logits: entry e never lies behind a logit that is
+// still to be read). The warp first lists what is kept and then evaluates it in full warps, two of them
+// at a time; a tile that keeps three quarters and more keeps all (a value too small to matter adds
+// nothing). `idx` holds 1024 positions.
 template <class TAKE>
-__device__ __forceinline__ TileEval tile_eval(float *mine, float thr, float T, float rT, float top, bool fast, TAKE take) {
+__device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, float thr, float T, float rT, float top, bool fast, TAKE take) {
     const int lane = threadIdx.x & 31;
+    const float *mine = tile + lane * PITCH;
     unsigned int m = 0;
 #pragma unroll
     for (int g = 0; g < 8; g++) {
@@ -739,49 +763,45 @@ __device__ __forceinline__ TileEval tile_eval(float *mine, float thr, float T, f
         m |= (v.x >= thr ? 1u : 0u) << (4 * g) | (v.y >= thr ? 1u : 0u) << (4 * g + 1) | (v.z >= thr ? 1u : 0u) << (4 * g + 2) | (v.w >= thr ? 1u : 0u) << (4 * g + 3);
     }
     TileEval r;
-    r.cnt = 0; r.keep = 0; r.csum = 0.0f;
-    const bool one = T == 1.0f;
-    for (int round = 0; round < 32 && __any_sync(0xffffffffu, m != 0u); round++) {
-        if (m) {
-            const int b = __ffs((int)m) - 1;
+    const int cnt = __popc(m), inc = warp_incl_scan(cnt, lane);
+    r.total = __shfl_sync(0xffffffffu, inc, 31);
+    const bool all = r.total >= 3 * TILE / 4;
+    if (all) { m = 0xffffffffu; r.total = TILE; }
+    r.keep = m;
+    if (!all) {
+        unsigned short *o = idx + (inc - cnt);
+        while (m) {
+            *o++ = (unsigned short)(lane * 32 + __ffs((int)m) - 1);
             m &= m - 1u;
-            const float x = mine[b];
-            const float v = one ? x : (fast ? div_by(x, T, rT) : __fdiv_rn(x, T));
-            const float e = expf_pinned_nonpos(__fsub_rn(v, top));  // no logit of the row exceeds its maximum
-            if (e > 0.0f) {
-                mine[r.cnt] = e;
-                r.cnt++;
-                r.csum += e;
-                r.keep |= 1u << b;
-                const unsigned int eb = __float_as_uint(e);
-                take(eb, lane * 32 + b);
-            }
         }
     }
-    for (int i = r.cnt; i < ((r.cnt + 3) & ~3); i++) mine[i] = 0.0f;
-    const int inc = warp_incl_scan(r.cnt, lane);
-    r.off = inc - r.cnt;
-    r.total = __shfl_sync(0xffffffffu, inc, 31);
     __syncwarp();
+    const bool one = T == 1.0f;
+    auto value = [&](float x) -> float {
+        // (what is not there is -inf, which div_by cannot take; everything so far down becomes zero)
+        const float v = one ? x : (fast ? div_by(fmaxf(x, -1.0e20f), T, rT) : __fdiv_rn(x, T));
+        return expf_pinned_nonpos(__fsub_rn(v, top));  // no logit of the row exceeds its maximum
+    };
+    for (int i0 = 0; i0 < r.total; i0 += 64) {
+        const int i = i0 + lane, j = i + 32;
+        const int p = all ? i : (i < r.total ? (int)idx[i] : 0), q = all ? j : (j < r.total ? (int)idx[j] : 0);
+        const float x = tile[p + 4 * (p >> 5)], y = tile[q + 4 * (q >> 5)];
+        const float ex = value(x), ey = value(y);
+        __syncwarp();
+        if (i < r.total) { tile[skew(i)] = ex; take(__float_as_uint(ex), p); }
+        if (j < r.total) { tile[skew(j)] = ey; take(__float_as_uint(ey), q); }
+        __syncwarp();
+    }
     return r;
 }
 
-// A tile's packed values to its place in the list: dense lanes are written by the whole warp.
-__device__ __forceinline__ void tile_store(const float *tile_rows, const TileEval &t, float *dst, unsigned int lanes) {
+// The careful lanes' values to their places, padded with zeros.
+__device__ __forceinline__ void store_care(float *care, const float *list, const TileChunk &ch, int my_place) {
     const int lane = threadIdx.x & 31;
-    const float *mine = tile_rows + lane * PITCH;
-    const bool wide = __reduce_max_sync(0xffffffffu, (unsigned int)t.cnt) > 6u;
-    if (!wide) {
-        if ((lanes >> lane) & 1u)
-            for (int i = 0; i < t.cnt; i++) dst[t.off + i] = mine[i];
-        return;
-    }
-    unsigned int left = __ballot_sync(0xffffffffu, t.cnt > 0) & lanes;
-    while (left) {
-        const int l = __ffs((int)left) - 1;
-        left &= left - 1u;
-        const int n = __shfl_sync(0xffffffffu, t.cnt, l), o = __shfl_sync(0xffffffffu, t.off, l);
-        if (lane < n) dst[o + lane] = tile_rows[l * PITCH + lane];
+    for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
+        const int l = __ffs((int)left) - 1, n = __shfl_sync(0xffffffffu, ch.cnt, l), o = __shfl_sync(0xffffffffu, ch.off, l);
+        const int at = __shfl_sync(0xffffffffu, my_place, l);
+        care[at * 32 + lane] = lane < n ? list[skew(o + lane)] : 0.0f;
     }
 }
 
@@ -796,38 +816,38 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     if (pl.kind == PLAN_DONE) return;
     const BatchArgs &a = A.a;
     const RowCfg &c = pl.c;
-    load_span(a, c, r, span * SPAN, S->x, &S->s, true);
+    span_fetch(a, c.lrow, span * SPAN, S->x);
+    span_ready(a, c, r, span * SPAN, S->x, &S->s, true);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
     if (tile >= A.ntile) return;
     const size_t gt = (size_t)rr * A.ntile + tile;
     const TilePlan tp = A.tp[gt];
-    float *mine = S->x + threadIdx.x * PITCH;
+    float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = pl.tau_bits;
     unsigned long long *cand = A.cand(rr);
-    const TileEval t = tile_eval(mine, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
+    const TileEval t = tile_eval(list, reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top,
+        (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
         [&](unsigned int eb, int i) {
             if (eb >= tau) {
                 const int pos = atomicAdd(&head->ncand, 1);
                 if (pos < HEADCAP) cand[pos] = make_key(eb, tile * TILE + i);
             }
         });
+    const TileChunk ch = tile_chunk(list, t.total);
     bool care;
     int my_place, c0 = CARE_PLACES;
     unsigned int i0 = 0;
-    const int ni = tile_items(mine, t.cnt, t.off, t.total, t.csum, tp.est, tile,
+    const int ni = tile_items(list, ch, tp.est, tile,
         [&](int n, int nc) -> Item * {
             if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, n); if (nc) c0 = atomicAdd(&head->ncare, nc); }
             i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
             return A.items(rr) + i0;
         },
         [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
-    // the careful lanes' values, padded with zeros
-    for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
-        const int l = __ffs((int)left) - 1, n = __shfl_sync(0xffffffffu, t.cnt, l), at = __shfl_sync(0xffffffffu, my_place, l);
-        A.care(rr)[at * 32 + lane] = lane < n ? S->x[(warp * 32 + l) * PITCH + lane] : 0.0f;
-    }
-    const unsigned int lanes = (pl.flags & F_LIST) ? 0xffffffffu : __ballot_sync(0xffffffffu, care && my_place == 255);
-    if (lanes) tile_store(S->x + (size_t)warp * 32 * PITCH, t, A.elist + gt * TILE, lanes);
+    store_care(A.care(rr), list, ch, my_place);
+    const bool whole = (pl.flags & F_LIST) || __any_sync(0xffffffffu, care && my_place == 255);
+    if (whole)
+        for (int i = lane; i < t.total; i += 32) A.elist[gt * TILE + i] = list[skew(i)];
     if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = t.keep;
     if (lane == 0) {
         TileOut o;
@@ -1340,13 +1360,15 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
 // rne(p / ulp) units to whatever sum lies in the binade, so one histogram of those integers per binade
 // tells where the sum crosses anything. Blocks take spans from the queue as long as there are any.
 // =============================================================================
-struct __align__(16) WalkTileShared {
+union __align__(16) WalkTileShared {
     float x[SPAN_THREADS * PITCH];
-    unsigned int hq[WALK_BINADES][NBINS];   // the low MASS_SPLIT bits of the contributions, summed, and the rest
-    unsigned int hqh[WALK_BINADES][NBINS];
+    struct {
+        unsigned int hq[WALK_BINADES][NBINS];   // the low MASS_SPLIT bits of the contributions, summed, and the rest
+        unsigned int hqh[WALK_BINADES][NBINS];
+    };
 };
 
-__global__ void __launch_bounds__(SPAN_THREADS, 2) tile_walk_kernel(const __grid_constant__ RowsArgs R) {
+__global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid_constant__ RowsArgs R) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WalkTileShared *S = reinterpret_cast<WalkTileShared *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1366,13 +1388,11 @@ __global__ void __launch_bounds__(SPAN_THREADS, 2) tile_walk_kernel(const __grid
 #pragma unroll
         for (int i = 0; i < 8; i++)
             if (4 * (lane + 32 * i) < n) v[i] = src[lane + 32 * i];
+        __syncthreads();
         if (state == ST_PURE) {
             if (tile >= R.ntile) continue;
-            // lane l's chunk: per values from l * per on
-            const int per = (n + 31) >> 5, off = min(n, lane * per), cnt = min(per, n - off);
-            float *rows = S->x + (size_t)warp * 32 * PITCH;
+            float *list = S->x + (size_t)warp * 32 * PITCH;
             __syncwarp();
-            const unsigned int magic = per ? (unsigned int)((0x100000000ull + (unsigned long long)per - 1ull) / (unsigned long long)per) : 0u;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int e0 = 4 * (lane + 32 * i);
@@ -1381,30 +1401,23 @@ __global__ void __launch_bounds__(SPAN_THREADS, 2) tile_walk_kernel(const __grid
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     p[u] = e0 + u < n ? prob_of(p[u], Z, yZ) : 0.0f;
-                    const int e = e0 + u, q = per > 1 ? (int)__umulhi((unsigned int)e, magic) : e;   // e / per
-                    if (e < n) rows[q * PITCH + (e - q * per)] = p[u];
+                    list[skew(e0 + u)] = p[u];
                 }
                 src[lane + 32 * i] = make_float4(p[0], p[1], p[2], p[3]);
             }
             __syncwarp();
-            float *mine = rows + lane * PITCH;
-            float s = 0.0f;
-            for (int i = cnt; i < ((cnt + 3) & ~3); i++) mine[i] = 0.0f;
-            for (int i = 0; i < cnt; i++) s += mine[i];
+            const TileChunk ch = tile_chunk(list, n);
             bool care;
             int my_place, c0 = CARE_PLACES;
             unsigned int i0 = 0;
-            const int ni = tile_items(mine, cnt, off, n, s, R.tp[gt].est * yZ, tile,
+            const int ni = tile_items(list, ch, R.tp[gt].est * yZ, tile,
                 [&](int k, int nc) -> Item * {
                     if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, k); if (nc) c0 = atomicAdd(&head->ncare, nc); }
                     i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
                     return R.items(rr) + i0;
                 },
                 [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
-            for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
-                const int l = __ffs((int)left) - 1, k = __shfl_sync(0xffffffffu, cnt, l), at = __shfl_sync(0xffffffffu, my_place, l);
-                R.care(rr)[at * 32 + lane] = lane < k ? rows[l * PITCH + lane] : 0.0f;
-            }
+            store_care(R.care(rr), list, ch, my_place);
             if (lane == 0) { R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = (unsigned short)ni; }
             __syncwarp();
             continue;
@@ -1552,13 +1565,16 @@ __device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
     const int span = t0 / (SPAN / TILE);
     SpanScratch *s = reinterpret_cast<SpanScratch *>(A->tile + SPAN_THREADS * PITCH);
     __syncthreads();
-    load_span(R.a, c.cfg, c.r, span * SPAN, A->tile, s, c.tid < SPAN_THREADS);
+    if (c.tid < SPAN_THREADS) span_fetch(R.a, c.cfg.lrow, span * SPAN, A->tile);
+    span_ready(R.a, c.cfg, c.r, span * SPAN, A->tile, s, c.tid < SPAN_THREADS);
     const int t = span * (SPAN / TILE) + c.warp;
     if (c.warp < SPAN / TILE && t >= t0 && t < t1) {
         const float thr = R.tp[(size_t)c.rr * R.ntile + t].thr;
-        const TileEval e = tile_eval(A->tile + (size_t)c.tid * PITCH, thr, c.cfg.T, __fdiv_rn(1.0f, c.cfg.T), c.pl.top,
+        float *list = A->tile + (size_t)c.warp * 32 * PITCH;
+        const TileEval e = tile_eval(list, reinterpret_cast<unsigned short *>(s->cnt) + c.warp * TILE, thr, c.cfg.T, __fdiv_rn(1.0f, c.cfg.T), c.pl.top,
                                      (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, int) {});
-        tile_store(A->tile + (size_t)c.warp * 32 * PITCH, e, to_list ? c.list + (size_t)t * TILE : dst, 0xffffffffu);
+        float *to = to_list ? c.list + (size_t)t * TILE : dst;
+        for (int i = c.lane; i < e.total; i += 32) to[i] = list[skew(i)];
         if (to_list) const_cast<unsigned int *>(c.kmask)[(size_t)t * 32 + c.lane] = e.keep;
     }
     __syncthreads();
@@ -1721,38 +1737,37 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
     return __uint_as_float(A->w_sb);
 }
 
-// Calls f(values, first position, where they are) for the row's list, four entries of a lane at a time
-// (zero: none); entry u of lane l is at first position + l + 32 u. All lanes of a warp make the same
-// calls. The next eight entries of every lane are on their way while f works on the ones before: a
-// block of 16 warps needs that many to cover the way to L2.
+// Calls f(values, position of the first, where they are) for the row's list, four neighbouring entries of
+// a lane at a time (zero: none). All lanes of a warp make the same calls. A lane's share of the next tile
+// is on its way while f works on the one before: a block of 16 warps needs up to 64 KB under way to
+// cover the latency of L2 (two rounds of loads of 256 entries took 25 k cycles for 66 k entries).
 template <class F>
 __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
     const AuxF *A = c.A;
     IN_SHARED(A);
     const int ntile = c.R->ntile;
-    int t = c.warp, i0 = 0;
-    auto settle = [&]() { while (t < ntile && i0 >= A->tcnt[t]) { t += NWARP; i0 = 0; } };
-    auto fetch = [&](unsigned int (&eb)[8]) {
+    uint4 nx[8];
+    auto fetch = [&](int t) {
         const int n = t < ntile ? A->tcnt[t] : 0;
-        const float *src = c.list + (size_t)t * TILE + i0 + c.lane;
+        const uint4 *src = reinterpret_cast<const uint4 *>(c.list + (size_t)t * TILE) + c.lane;
 #pragma unroll
-        for (int u = 0; u < 8; u++) eb[u] = (i0 + u * 32 + c.lane < n) ? __float_as_uint(src[u * 32]) : 0u;
+        for (int i = 0; i < 8; i++)
+            if (4 * (c.lane + 32 * i) < n) nx[i] = src[32 * i];
     };
-    settle();
-    unsigned int nx[8];
-    fetch(nx);
-    while (t < ntile) {
-        unsigned int lo[4], hi[4];
+    fetch(c.warp);
+    for (int t = c.warp; t < ntile; t += NWARP) {
+        uint4 v[8];
 #pragma unroll
-        for (int u = 0; u < 4; u++) { lo[u] = nx[u]; hi[u] = nx[u + 4]; }
-        const int pos = t * TILE + i0;
-        const bool second = i0 + 128 < A->tcnt[t];
-        float *at = c.list + pos;
-        i0 += 256;
-        settle();
-        fetch(nx);
-        f(lo, pos, at);
-        if (second) f(hi, pos + 128, at + 128);
+        for (int i = 0; i < 8; i++) v[i] = nx[i];
+        fetch(t + NWARP);
+        const int n = A->tcnt[t];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (128 * i >= n) break;
+            const int e0 = 4 * (c.lane + 32 * i);
+            const unsigned int eb[4] = {e0 < n ? v[i].x : 0u, e0 + 1 < n ? v[i].y : 0u, e0 + 2 < n ? v[i].z : 0u, e0 + 3 < n ? v[i].w : 0u};
+            f(eb, t * TILE + e0, c.list + (size_t)t * TILE + e0);
+        }
     }
 }
 
@@ -2040,7 +2055,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                         if ((p >= bigthr) || (tie && !ties_listed)) { sred_max(&A->specbin, bin); continue; }
                         if (tie) {
                             const int pos = satom_add(&A->ntie, 1);
-                            if (pos < TIE_CAP) { A->tkey[pos] = make_key(eb, pos0 + c.lane + 32 * u); A->tbin[pos] = bin; }
+                            if (pos < TIE_CAP) { A->tkey[pos] = make_key(eb, pos0 + u); A->tbin[pos] = bin; }
                         }
                     }
                 }
@@ -2081,7 +2096,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                     const float rr = __fsub_rn(p, __fsub_rn(tq, Cm));
                     if (fabsf(rr) == halfu || p >= bigthr) continue;
                     const unsigned int qu = __float_as_uint(tq) - cm_bits;
-                    const unsigned long long key = make_key(eb, pos0 + c.lane + 32 * u);
+                    const unsigned long long key = make_key(eb, pos0 + u);
                     for (int t = 0; t < ntie; t++)
                         if (A->tbin[t] == bin && key > A->tkey[t] && qu) {  // two halves, as in the bin tables
                             sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
@@ -2141,6 +2156,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                 }
                 return true;
             });
+        if (phase < 2 && !try_resume) FSTAMP(11 + 3 * phase);
         const int hb = A->hit_bin;
         if (hb < 0) {
             // nothing left in this range triggers an event: consume it whole
@@ -2165,11 +2181,12 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                 const unsigned int eb = ebs[u];
                 if (eb != 0u && eb >= blo && eb < gtau) {
                     const int pos = satom_add(&A->ncand, 1);
-                    if (pos < NC) A->cand[pos] = make_key(eb, pos0 + c.lane + 32 * u);
+                    if (pos < NC) A->cand[pos] = make_key(eb, pos0 + u);
                 }
             }
         });
         __syncthreads();
+        if (phase < 2 && !try_resume) FSTAMP(12 + 3 * phase);
         const int nb = A->ncand;
         const bool crowded = nb > NC;
         // what lies above the bin is consumed without an event either way
@@ -2213,6 +2230,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         }
         sort_head(c, nb);
         walk_sorted(c, nb, s_bin, pos_bin, x_ge, x_gt, counting, nstop);
+        if (phase < 2 && !try_resume) FSTAMP(13 + 3 * phase);
         w.s = A->b_s; w.pos = A->b_pos; w.tau = blo;
         const int ev = A->b_event;
         if (ev != EV_NONE) {
@@ -2241,6 +2259,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
     __syncthreads();
     const unsigned int nrec = wl.order(W, R.ntile, nitem);
     if (nrec > (unsigned int)H_REC) return false;
+    FSTAMP(17);
     if (c.warp == 0) {
         float z = 0.0f;
         const bool fine = walk_records(W, R.care(c.rr), (int)nrec, z);
@@ -2254,6 +2273,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
         if (target < __uint_as_float(W->sbs[q + 1])) { atomicMin(&A->evt_thread, q); break; }
     __syncthreads();
     const int q = A->evt_thread;
+    FSTAMP(18);
     if (c.warp != 0) return true;
     if (q == 0x7fffffff) {   // the walk fell off the end: the reference returns the last token of the vocabulary
         if (c.lane == 0) finish_row(R.a, c.r, c.cfg, c.status, R.a.V - 1, Z, sum, target, 0.0f);
@@ -2310,6 +2330,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
         }
         sb = __float_as_uint(s);
     }
+    FSTAMP(10);
     if (c.lane == 0) finish_row(R.a, c.r, c.cfg, c.status, tile < 0 ? R.a.V - 1 : token_of(c, tile, at), Z, sum, target, 0.0f);
     return true;
 }
@@ -2428,20 +2449,16 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
             if (t + 1 < ntile) A->tsum[t + 1] = ex + s0;
         }
         __syncthreads();
-        float *mine = A->tile + (size_t)c.tid * PITCH;
+        float *list = A->tile + (size_t)c.warp * 32 * PITCH;
         for (int t = c.warp; t < ntile; t += NWARP) {
-            const int n = A->tcnt[t], per = (n + 31) >> 5, off = min(n, c.lane * per), cnt = min(per, n - off);
+            const int n = A->tcnt[t];
             const float *src = c.list + (size_t)t * TILE;
-            float s = 0.0f;
-            for (int i = 0; i < ((cnt + 3) & ~3); i++) {
-                const float p = i < cnt ? src[off + i] : 0.0f;
-                mine[i] = p;
-                s += p;
-            }
+            for (int i = c.lane; i < n; i += 32) list[skew(i)] = src[i];
             __syncwarp();
+            const TileChunk ch = tile_chunk(list, n);
             bool care;
             int my_place;
-            const int ni = tile_items(mine, cnt, off, n, s, A->tsum[t], t, [&](int, int) { return c.gitems + (size_t)t * ITEMS_PER_TILE; }, [](int) { return 255; }, care, my_place);
+            const int ni = tile_items(list, ch, A->tsum[t], t, [&](int, int) { return c.gitems + (size_t)t * ITEMS_PER_TILE; }, [](int) { return 255; }, care, my_place);
             if (c.lane == 0) { A->tni[t] = (unsigned short)ni; A->tio[t] = (unsigned int)(t * ITEMS_PER_TILE); }
             __syncwarp();
         }
@@ -2461,7 +2478,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
                 for_list4(c, [&](const unsigned int (&pb)[4], int pos0, float *) {
 #pragma unroll
                     for (int u = 0; u < 4; u++)
-                        if (pb[u] >= minp_pbits && pb[u] != 0u) last = max(last, pos0 + c.lane + 32 * u);
+                        if (pb[u] >= minp_pbits && pb[u] != 0u) last = max(last, pos0 + u);
                 });
                 last = __reduce_max_sync(0xffffffffu, last);
                 __syncthreads();
@@ -2600,7 +2617,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     if (state != ST_HEAD) for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (eb[u]) src[u * 32 + c.lane] = eb[u] >= tau_bits ? 0.0f : prob_of(__uint_as_float(eb[u]), Z, yZ);
+            if (eb[u]) src[u] = eb[u] >= tau_bits ? 0.0f : prob_of(__uint_as_float(eb[u]), Z, yZ);
     });
     __syncthreads();
     FSTAMP(7);
@@ -2662,7 +2679,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
             for_list4(c, [&](const unsigned int (&pb)[4], int pos0, float *) {
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (pb[u]) { const unsigned long long kk = make_key(pb[u], pos0 + c.lane + 32 * u); best = kk < best ? kk : best; }
+                    if (pb[u]) { const unsigned long long kk = make_key(pb[u], pos0 + u); best = kk < best ? kk : best; }
             });
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -2782,7 +2799,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         if (e == cudaSuccess) e = launch(row_plan_kernel, (unsigned int)A.rows, NT, 0, st, A);
         if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
         if (e == cudaSuccess) e = launch(row_head_kernel, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
-        if (e == cudaSuccess) e = launch(tile_walk_kernel, spans < 2u * (unsigned int)sms ? spans : 2u * (unsigned int)sms, SPAN_THREADS, sizeof(WalkTileShared), st, A);
+        if (e == cudaSuccess) e = launch(tile_walk_kernel, spans < 4u * (unsigned int)sms ? spans : 4u * (unsigned int)sms, SPAN_THREADS, sizeof(WalkTileShared), st, A);
         if (e == cudaSuccess) e = launch(row_tail_kernel, (unsigned int)(A.rows < sms ? A.rows : sms), NT, sizeof(AuxF), st, A);
     }
     if (e != cudaSuccess) {

@@ -46,6 +46,7 @@
 #endif
 #include "molla_device.cuh"
 #include "molla_exact.cuh"
+#include "molla_logprob.h"
 #include "molla_rows.h"
 
 using namespace molla;
@@ -1963,8 +1964,9 @@ size_t help_bytes(size_t ctas) { return ctas * (sizeof(HelpSlot) + (size_t)HELP_
 size_t batch_workspace_bytes(int B, int V, int sms) {
     const size_t ctas = (size_t)(B < sms ? B : sms);
     const size_t lists = WS_HEADER + ctas * 2 * (size_t)NWARP * (size_t)region_floats(V) * 8 + help_bytes(ctas);
-    const size_t rows = molla_rows_workspace_bytes(B, V);
-    return lists > rows ? lists : rows;
+    const size_t rows = molla_rows_workspace_bytes(B, V), lp = molla_logprob_workspace_bytes(B, V);
+    const size_t most = rows > lp ? rows : lp;
+    return lists > most ? lists : most;
 }
 
 int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, int max_ctas = 0x7fffffff, bool with_help = false) {
@@ -2014,6 +2016,23 @@ int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
     return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err));
+}
+
+// The chosen tokens' and the top N's logprobs behind a sampling launch, which is done with the workspace.
+int launch_logprobs(const float *logits, int64_t row_stride, int B, int V, const int *tokens, int top_n, float *chosen, int *top_ids,
+                    float *top_lps, const int *rows, int n_logit_rows, float softcap, void *d_workspace, cudaStream_t st) {
+    if (!chosen && top_n == 0) return MOLLA_OK;
+    cudaError_t e;
+    if (molla_logprob_tiled(V)) {
+        e = molla_logprob_launch(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, rows, n_logit_rows, softcap,
+                                 d_workspace, nullptr, st);
+    } else {
+        const int sms = sm_count();
+        logprob_kernel<<<sms > 0 && B > sms ? sms : B, NT, 0, st>>>(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, nullptr,
+                                                                    rows, n_logit_rows, softcap);
+        e = cudaGetLastError();
+    }
+    return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
 }
 
 }  // namespace
@@ -2073,17 +2092,8 @@ int32_t molla_sample_batch_masked(const uint32_t *d_mask, int64_t mask_stride_wo
     MOLLA_SET_TESTING_ARGS(a);
     int rc = launch_sampling(a, d_workspace, st);
     if (rc != MOLLA_OK) return rc;
-    if (d_chosen_logprob || top_n > 0) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int grid = B < sms ? B : sms;
-        logprob_kernel<<<grid, NT, 0, st>>>(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob,
-                                            d_top_ids, d_top_logprobs, nullptr, nullptr, 0, 0.0f);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
-    }
-    return MOLLA_OK;
+    return launch_logprobs(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob, d_top_ids, d_top_logprobs, nullptr, 0, 0.0f,
+                           d_workspace, st);
 }
 
 int32_t molla_sample_batch(const float *d_logits, int64_t row_stride, int32_t B, int32_t V,
@@ -2153,17 +2163,8 @@ int32_t molla_sample_decode_step(const float *d_logits, int64_t row_stride, int3
     }
     int rc = launch_sampling(a, d_workspace, st);
     if (rc != MOLLA_OK) return rc;
-    if (d_chosen_logprob || top_n > 0) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int grid = B < sms ? B : sms;
-        logprob_kernel<<<grid, NT, 0, st>>>(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob,
-                                            d_top_ids, d_top_logprobs, nullptr, d_rows, n_logit_rows, final_softcap);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
-    }
-    return MOLLA_OK;
+    return launch_logprobs(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob, d_top_ids, d_top_logprobs, d_rows, n_logit_rows, final_softcap,
+                           d_workspace, st);
 }
 
 int32_t molla_sample_batch_noalloc(const float *d_logits, int64_t row_stride, int32_t B, int32_t V,
@@ -2222,16 +2223,8 @@ int32_t molla_sample_batch_noalloc(const float *d_logits, int64_t row_stride, in
     // at zero); the row order and the lists behind it are written before they are read
     int rc = launch_rows(a, ws, st, max_ctas);
     if (rc != MOLLA_OK) return rc;
-    if (d_chosen_logprob || top_n > 0) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int grid = B < sms ? B : sms;
-        logprob_kernel<<<grid, NT, 0, st>>>(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob,
-                                            d_top_ids, d_top_logprobs, nullptr, nullptr, 0, 0.0f);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
-    }
-    return MOLLA_OK;
+    static_assert((size_t)MOLLA_NOALLOC_MAX_ROWS * (MOLLA_NOALLOC_MAX_VOCAB / 1024 + 1) * 16 <= MOLLA_NOALLOC_SCRATCH_BYTES, "the logprobs' tile results fit");
+    return launch_logprobs(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob, d_top_ids, d_top_logprobs, nullptr, 0, 0.0f, ws, st);
 }
 
 // ---- vocab-sharded form ------------------------------------------------------------
@@ -2544,12 +2537,14 @@ int32_t molla_sample_logprobs(const float *d_logits, int64_t row_stride, int32_t
     g_err[0] = 0;
     if (!d_logits || !d_out || B < 0 || V <= 0 || row_stride < V) return fail(MOLLA_ERR_ARGUMENT, "bad arguments to logprobs%s");
     if (B == 0) return MOLLA_OK;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int grid = B < sms ? B : sms;
-    logprob_kernel<<<grid, NT, 0, (cudaStream_t)stream>>>(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr,
-                                                          nullptr, d_out, nullptr, 0, 0.0f);
+    if (molla_logprob_tiled(V)) {
+        const cudaError_t e = molla_logprob_launch(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0.0f,
+                                                   nullptr, d_out, (cudaStream_t)stream);
+        return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
+    }
+    const int sms = sm_count();
+    logprob_kernel<<<sms > 0 && B > sms ? sms : B, NT, 0, (cudaStream_t)stream>>>(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr,
+                                                                                  nullptr, d_out, nullptr, 0, 0.0f);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
     return MOLLA_OK;
