@@ -90,7 +90,10 @@ struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned in
 // elements that would round on a tie there.
 constexpr int WALK_BINADES = 3;
 struct __align__(16) WalkTies { int n; int pad[3]; unsigned long long key[TIE_CAP]; };
-constexpr size_t WALK_BYTES = WALK_BINADES * (NBINS * sizeof(unsigned long long) + sizeof(WalkTies));
+// The bins whose elements the walk will want one by one, and those elements.
+constexpr int PICKS = 8, PICK_CAP = NC;
+struct __align__(16) WalkPicks { int n, arrived, pad[2]; int bin[PICKS]; int cnt[PICKS]; };
+constexpr size_t WALK_BYTES = WALK_BINADES * (NBINS * sizeof(unsigned long long) + sizeof(WalkTies)) + sizeof(WalkPicks) + (size_t)PICKS * PICK_CAP * sizeof(unsigned long long);
 
 struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; int pad[4]; };
 
@@ -109,6 +112,8 @@ struct RowsArgs {
     unsigned int *kmask;     // [rows][ntile][32] which logits they are
     __device__ __forceinline__ unsigned long long *table(int rr, int b) const { return reinterpret_cast<unsigned long long *>(walk + (size_t)rr * WALK_BYTES) + (size_t)b * NBINS; }
     __device__ __forceinline__ WalkTies *ties(int rr) const { return reinterpret_cast<WalkTies *>(table(rr, WALK_BINADES)); }
+    __device__ __forceinline__ WalkPicks *picks(int rr) const { return reinterpret_cast<WalkPicks *>(ties(rr) + WALK_BINADES); }
+    __device__ __forceinline__ unsigned long long *picked(int rr, int i) const { return reinterpret_cast<unsigned long long *>(picks(rr) + 1) + (size_t)i * PICK_CAP; }
     __device__ __forceinline__ RowHead *head(int rr) const { return reinterpret_cast<RowHead *>(box + (long long)rr * box_stride); }
     __device__ __forceinline__ TileOut *to(int rr) const { return reinterpret_cast<TileOut *>(head(rr) + 1); }
     __device__ __forceinline__ unsigned long long *cand(int rr) const { return reinterpret_cast<unsigned long long *>(to(rr) + ((ntile + 1) & ~1)); }
@@ -1348,6 +1353,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         ulonglong2 *z = reinterpret_cast<ulonglong2 *>(R.table(rr, 0));
         for (int i = tid; i < WALK_BINADES * NBINS / 2; i += HT) z[i] = make_ulonglong2(0ull, 0ull);
         if (tid < WALK_BINADES) R.ties(rr)[tid].n = 0;
+        if (tid == 0) { R.picks(rr)->n = 0; R.picks(rr)->arrived = 0; }
     }
     for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
     queue_row(ST_HEAD, 6);
@@ -1368,9 +1374,129 @@ union __align__(16) WalkTileShared {
     };
 };
 
+// Which bins the walk past row rr's head will look into element by element: from the tables alone the
+// sum before every bin is known to within the rounding inside one bin and a few ties, so the bins where it
+// crosses into the next binade, reaches top-p, or passes the drawn target are known but for a neighbour.
+// What is left out here is only slower: row_tail then looks for it in the list.
+__device__ __noinline__ void plan_picks(const RowsArgs &R, int rr, float hs, int j0, int nb) {
+    __shared__ double ws[SPAN_THREADS / 32];
+    __shared__ int s_bin[4];
+    __shared__ double s_before[2];
+    __shared__ int picked[PICKS];
+    __shared__ int npick;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = NBINS / SPAN_THREADS;
+    const RowHead *head = R.head(rr);
+    const RowCfg &g = head->plan.c;
+    if (tid == 0) npick = 0;
+    auto want = [&](int b) {   // thread 0
+        if (b < 0 || b >= NBINS) return;
+        for (int i = 0; i < npick; i++) if (picked[i] == b) return;
+        if (npick < PICKS) picked[npick++] = b;
+    };
+    // For the table of binade j0 + p below bin `hi`, with m0 units before it: the first bin (descending)
+    // whose end reaches x units, the units before it, and its neighbours that hold anything.
+    double q[PER];
+    auto load = [&](int p, int hi) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int b = NBINS - 1 - PER * tid - i;
+            q[i] = b < hi ? (double)__ldcg(R.table(rr, p) + b) : 0.0;
+        }
+    };
+    double total = 0.0;
+    auto find = [&](double m0, double x) -> int {   // all threads; results in s_bin[0..2], s_before
+        double sum = 0.0;
+#pragma unroll
+        for (int i = 0; i < PER; i++) sum += q[i];
+        const double inc = warp_incl_scan(sum, lane);
+        __syncthreads();
+        if (lane == 31) ws[warp] = inc;
+        if (tid == 0) { s_bin[0] = -1; s_bin[1] = -1; s_bin[2] = -1; }
+        __syncthreads();
+        double b0 = 0.0, t = 0.0;
+#pragma unroll
+        for (int w = 0; w < SPAN_THREADS / 32; w++) { if (w == warp) b0 = t; t += ws[w]; }
+        total = t;
+        double c = m0 + b0 + (inc - sum);
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int b = NBINS - 1 - PER * tid - i;
+            if (q[i] > 0.0) {
+                if (c < x && c + q[i] >= x) { s_bin[0] = b; s_before[0] = c; s_before[1] = c + q[i]; }
+                if (c + q[i] < x) atomicMin(reinterpret_cast<unsigned int *>(&s_bin[1]), (unsigned int)b);   // the last one before it
+                if (c >= x) atomicMax(&s_bin[2], b);                                                          // the first one behind it
+            }
+            c += q[i];
+        }
+        __syncthreads();
+        return s_bin[0];
+    };
+    const double slack = 96.0;
+    double start[WALK_BINADES + 1];
+    int hi_of[WALK_BINADES], low_of[WALK_BINADES];
+    double s = (double)hs, sum_lo = 0.0, sum_hi = 0.0;
+    int hi = NBINS, phases = 0;
+    bool cut = false;
+    __syncthreads();
+    for (int p = 0; p < nb && !cut; p++) {
+        const double unit = dpow2(j0 + p - 23), m0 = s / unit;
+        double x = 16777216.0;
+        bool by_cut = false;
+        if (g.topp_on) { const double t = ceil((double)g.P / unit); if (t <= x) { x = t; by_cut = true; } }
+        load(p, hi);
+        const int hb = find(m0, x);
+        start[p] = s; hi_of[p] = hi; low_of[p] = hb < 0 ? 0 : hb;
+        phases = p + 1;
+        if (hb < 0) { sum_lo = (m0 + total) * unit; sum_hi = sum_lo; break; }
+        if (tid == 0) {
+            want(hb);
+            if (x - s_before[0] < slack) want(s_bin[1]);
+            if (s_before[1] - x < slack) want(s_bin[2]);
+        }
+        if (by_cut) { cut = true; sum_lo = x * unit; sum_hi = fmin(s_before[1] * unit, (x + slack) * unit + (double)__uint_as_float((unsigned int)(hb + 1) << BIN_SHIFT)); }
+        s = s_before[1] * unit;
+        sum_lo = cut ? sum_lo : s; sum_hi = cut ? sum_hi : s;
+        hi = hb;
+        __syncthreads();
+    }
+    // the draw
+    const BatchArgs &a = R.a;
+    const double u01 = (double)draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull);
+    const double tg[2] = {u01 * sum_lo * (1.0 - 1.0e-6), u01 * sum_hi * (1.0 + 1.0e-6)};
+    int last = -1;
+    for (int k = 0; k < 2; k++) {
+        if (tg[k] < (double)hs) continue;   // in the head
+        int p = 0;
+        while (p + 1 < phases && tg[k] >= start[p + 1]) p++;
+        const double unit = dpow2(j0 + p - 23);
+        load(p, hi_of[p]);
+        const int b = find(start[p] / unit, tg[k] / unit);
+        if (tid == 0) { want(b); want(last); }
+        last = b;
+        __syncthreads();
+    }
+    // ties at or above the lowest bin of their binade's stretch: what precedes them in their bins is wanted
+    if (tid == 0) {
+        for (int p = 0; p < phases; p++) {
+            const WalkTies *t = R.ties(rr) + p;
+            const int n = min(__ldcg(&t->n), TIE_CAP);
+            for (int i = 0; i < n; i++) {
+                const int b = (int)((unsigned int)(__ldcg(&t->key[i]) >> 32) >> BIN_SHIFT);
+                if (b >= low_of[p] && b < hi_of[p]) want(b);
+            }
+        }
+        WalkPicks *o = R.picks(rr);
+        for (int i = 0; i < npick; i++) { o->bin[i] = picked[i]; o->cnt[i] = 0; }
+        o->n = npick;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid_constant__ RowsArgs R) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WalkTileShared *S = reinterpret_cast<WalkTileShared *>(smem_raw);
+    __shared__ int S_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_next();
     pdl_wait();
@@ -1466,11 +1592,64 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             const unsigned long long q = (unsigned long long)(&S->hq[0][0])[i] + ((unsigned long long)(&S->hqh[0][0])[i] << MASS_SPLIT);
             if (q) atomicAdd(R.table(rr, 0) + i, q);
         }
+        // the block that finishes a row's tables works out which bins the walk will want
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) S_last = atomicAdd(&R.picks(rr)->arrived, 1) == R.nspan - 1 ? 1 : 0;
+        __syncthreads();
+        if (S_last && nb > 0) {
+            __threadfence();
+            plan_picks(R, rr, hs, j0, nb);
+        }
     }
 }
 
 // =============================================================================
-// Kernel 6: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
+// Kernel 6: the elements of the wanted bins of every walk, gathered over the whole chip.
+// =============================================================================
+__global__ void __launch_bounds__(SPAN_THREADS, 4) tile_pick_kernel(const __grid_constant__ RowsArgs R) {
+    __shared__ unsigned char slot[NBINS];   // 0: not wanted
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_next();
+    pdl_wait();
+    const int work = R.queue[0] * R.nspan;
+    for (int wi = blockIdx.x; wi < work; wi += gridDim.x) {
+        const int rr = R.queue[1 + wi / R.nspan], span = wi % R.nspan, tile = span * (SPAN / TILE) + warp;
+        if (R.head(rr)->state != ST_HEAD) continue;
+        WalkPicks *pk = R.picks(rr);
+        const int npick = pk->n;
+        if (npick == 0) continue;
+        const int n = tile < R.ntile ? (int)R.to(rr)[tile].cnt : 0;
+        const uint4 *src = reinterpret_cast<const uint4 *>(R.elist + ((size_t)rr * R.ntile + tile) * TILE);
+        uint4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (4 * (lane + 32 * i) < n) v[i] = src[lane + 32 * i];
+        __syncthreads();
+        for (int i = tid; i < NBINS / 4; i += SPAN_THREADS) reinterpret_cast<unsigned int *>(slot)[i] = 0u;
+        __syncthreads();
+        if (tid < npick) slot[pk->bin[tid]] = (unsigned char)(tid + 1);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int e0 = 4 * (lane + 32 * i);
+            if (e0 >= n) continue;
+            const unsigned int p[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (e0 + u >= n || p[u] == 0u) continue;
+                const int k = slot[p[u] >> BIN_SHIFT];
+                if (k) {
+                    const int at = atomicAdd(&pk->cnt[k - 1], 1);
+                    if (at < PICK_CAP) R.picked(rr, k - 1)[at] = make_key(p[u], tile * TILE + e0 + u);
+                }
+            }
+        }
+    }
+}
+
+// =============================================================================
+// Kernel 7: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
 // what it does not.
 // =============================================================================
 struct __align__(16) AuxF {
@@ -1531,6 +1710,7 @@ struct CtxF {
     RowCfg cfg;
     RowPlan pl;
     int tj0, tnb;                // binades that tile_walk has left tables for
+    int npick;                   // bins that tile_pick has gathered
     float *list;                 // this row's [ntile][TILE]
     Item *gitems;                // this row's items
     const unsigned int *kmask;   // this row's [ntile][32]
@@ -1738,29 +1918,18 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
 }
 
 // Calls f(values, position of the first, where they are) for the row's list, four neighbouring entries of
-// a lane at a time (zero: none). All lanes of a warp make the same calls. A lane's share of the next tile
-// is on its way while f works on the one before: a block of 16 warps needs up to 64 KB under way to
-// cover the latency of L2 (two rounds of loads of 256 entries took 25 k cycles for 66 k entries).
+// a lane at a time (zero: none). All lanes of a warp make the same calls. A whole tile is asked for at once.
 template <class F>
 __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
     const AuxF *A = c.A;
     IN_SHARED(A);
-    const int ntile = c.R->ntile;
-    uint4 nx[8];
-    auto fetch = [&](int t) {
-        const int n = t < ntile ? A->tcnt[t] : 0;
+    for (int t = c.warp; t < c.R->ntile; t += NWARP) {
+        const int n = A->tcnt[t];
         const uint4 *src = reinterpret_cast<const uint4 *>(c.list + (size_t)t * TILE) + c.lane;
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (4 * (c.lane + 32 * i) < n) nx[i] = src[32 * i];
-    };
-    fetch(c.warp);
-    for (int t = c.warp; t < ntile; t += NWARP) {
         uint4 v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = nx[i];
-        fetch(t + NWARP);
-        const int n = A->tcnt[t];
+        for (int i = 0; i < 8; i++)
+            if (4 * (c.lane + 32 * i) < n) v[i] = src[32 * i];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             if (128 * i >= n) break;
@@ -2065,6 +2234,12 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             rs.ntie = ntie;
             if (ntie > TIE_CAP) { tie_mode = false; c.status |= MOLLA_ROW_SLOW_PATH; continue; }  // too many: they stop phases instead
         }
+        const WalkPicks *pk = c.R->picks(c.rr);
+        auto pick_of = [&](int b) -> int {   // the bin's place among the gathered ones, -1: not there
+            for (int i = 0; i < c.npick; i++)
+                if (pk->bin[i] == b && pk->cnt[i] <= PICK_CAP) return i;
+            return -1;
+        };
         if (!reuse && ntie > 0) {
             // what precedes each listed element inside its own bin (descending value, then ascending id)
             if (c.tid < ntie) {
@@ -2076,7 +2251,26 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             int tb_lo = NBINS, tb_hi = -1;
             for (int t = 0; t < ntie; t++) { tb_lo = min(tb_lo, A->tbin[t]); tb_hi = max(tb_hi, A->tbin[t]); }
             const unsigned int tb_span = (unsigned int)(tb_hi - tb_lo);
-            for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+            bool gathered = tabbed;
+            for (int t = 0; t < ntie && gathered; t++) gathered = pick_of(A->tbin[t]) >= 0;
+            if (gathered) {
+                for (int t = 0; t < ntie; t++) {
+                    const int k = pick_of(A->tbin[t]), m = pk->cnt[k];
+                    const unsigned long long *keys = c.R->picked(c.rr, k), tk = A->tkey[t];
+                    for (int i = c.tid; i < m; i += NT) {
+                        const unsigned long long key = keys[i];
+                        const unsigned int eb = (unsigned int)(key >> 32);
+                        const float p = __uint_as_float(eb);
+                        const float tq = __fadd_rn(p, Cm);
+                        if (eb >= wtau || !(key > tk) || fabsf(__fsub_rn(p, __fsub_rn(tq, Cm))) == halfu || p >= bigthr) continue;
+                        const unsigned int qu = __float_as_uint(tq) - cm_bits;
+                        if (qu) {
+                            sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
+                            if (qu >> MASS_SPLIT) sred_add(&A->tpq_hi[t], qu >> MASS_SPLIT);
+                        }
+                    }
+                }
+            } else for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
                 bool near = false;
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
@@ -2171,7 +2365,16 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         const unsigned long long bhi64 = (unsigned long long)lo + ((unsigned long long)(hb + 1) << shift);
         const unsigned int bhi = bhi64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (unsigned int)bhi64;
         const unsigned int gtau = wtau < bhi ? wtau : bhi;  // the bin's entries: blo <= value < gtau, and not zero (an absent element)
-        for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
+        const int hk = lvl == 1 ? pick_of(hb) : -1;
+        if (hk >= 0) {
+            const unsigned long long *keys = c.R->picked(c.rr, hk);
+            const int m = pk->cnt[hk];
+            for (int i = c.tid; i < m; i += NT) {
+                const unsigned long long key = keys[i];
+                const unsigned int eb = (unsigned int)(key >> 32);
+                if (eb >= blo && eb < gtau) A->cand[satom_add(&A->ncand, 1)] = key;
+            }
+        } else for_list4(c, [&](const unsigned int (&ebs)[4], int pos0, float *) {
             bool any = false;
 #pragma unroll
             for (int u = 0; u < 4; u++) any |= ebs[u] != 0u && ebs[u] >= blo && ebs[u] < gtau;
@@ -2612,7 +2815,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     // ---- past the head: the cut walk, then the draw walk, over the probabilities
     // (sample.mojo:437-438); what the head took is consumed
     const unsigned int tau_bits = head_overflow ? 0xffffffffu : c.pl.tau_bits;
-    c.tnb = 0; c.tj0 = 0;
+    c.tnb = 0; c.tj0 = 0; c.npick = state == ST_HEAD ? R.picks(rr)->n : 0;
     if (state == ST_HEAD && head_s > 0.0f && fexpo(head_s) >= -30 && fexpo(head_s) < 0) { c.tj0 = fexpo(head_s); c.tnb = min(WALK_BINADES, -c.tj0); }
     if (state != ST_HEAD) for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
 #pragma unroll
@@ -2800,6 +3003,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
         if (e == cudaSuccess) e = launch(row_head_kernel, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
         if (e == cudaSuccess) e = launch(tile_walk_kernel, spans < 4u * (unsigned int)sms ? spans : 4u * (unsigned int)sms, SPAN_THREADS, sizeof(WalkTileShared), st, A);
+        if (e == cudaSuccess) e = launch(tile_pick_kernel, spans < 4u * (unsigned int)sms ? spans : 4u * (unsigned int)sms, SPAN_THREADS, 0, st, A);
         if (e == cudaSuccess) e = launch(row_tail_kernel, (unsigned int)(A.rows < sms ? A.rows : sms), NT, sizeof(AuxF), st, A);
     }
     if (e != cudaSuccess) {
