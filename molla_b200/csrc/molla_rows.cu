@@ -175,7 +175,7 @@ __device__ __forceinline__ RowCfg row_cfg(const BatchArgs &a, int r) {
 }
 
 // The end of every row, one thread: the answer, then `_took` (sample.mojo:361-363).
-__device__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
+__device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
                            float dtarget, float dp) {
     if (status & 0x80000000u) {  // a stale index
         a.tokens[r] = -1; a.row_status[r] = status & 0x7fffffffu;
@@ -211,9 +211,12 @@ __device__ __forceinline__ float div_by(float x, float d, float y) {
     const float q1 = __fmaf_rn(__fmaf_rn(-q0, d, x), y, q0);
     return __fmaf_rn(__fmaf_rn(-q1, d, x), y, q1);
 }
+// (out of line: the compiler's division is long, and a row's code is read from L2 once per SM)
+__device__ __noinline__ float softcap_slow(float x, float cap) { return softcap_pinned(x, cap); }
+__device__ __noinline__ float div_slow(float x, float d) { return __fdiv_rn(x, d); }
 // a probability e / Z (Z between 1 and the vocabulary's size; e in [0, 1])
 __device__ __forceinline__ float prob_of(float e, float Z, float y) {
-    return e > 1.0e-20f ? div_by(e, Z, y) : __fdiv_rn(e, Z);
+    return e > 1.0e-20f || e == 0.0f ? div_by(e, Z, y) : div_slow(e, Z);
 }
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
@@ -249,19 +252,13 @@ __device__ __forceinline__ void span_fetch(const BatchArgs &a, long long lrow, i
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *src = a.logits + lrow * a.row_stride + c0;
     const int n = min(SPAN, a.V - c0), e0 = warp * TILE;
-    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0 && e0 + TILE <= n) {
+        float *dst = sx + (warp * 32 + (lane >> 3)) * PITCH + (lane & 7) * 4;
+        const float *from = src + e0 + lane * 4;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int ch = i * 32 + lane, e = e0 + ch * 4;
-            float *dst = sx + (warp * 32 + (ch >> 3)) * PITCH + (ch & 7) * 4;
-            if (e + 4 <= n) cp16(dst, src + e);
-            else {
-#pragma unroll
-                for (int u = 0; u < 4; u++) dst[u] = (e + u < n) ? __ldg(src + e + u) : -INFINITY;
-            }
-        }
+        for (int i = 0; i < 8; i++) cp16(dst + i * 4 * PITCH, from + i * 128);
     } else {
-#pragma unroll 8
+#pragma unroll 4
         for (int i = 0; i < 32; i++) {
             const int e = e0 + i * 32 + lane;
             float *dst = sx + (warp * 32 + i) * PITCH + lane;
@@ -289,6 +286,7 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
         }
         __syncthreads();
         if (active)
+#pragma unroll 1
             for (int i = tid; i < c.npatch; i += SPAN_THREADS) {
                 const bool is_bias = i < c.nb;
                 const long long t64 = (is_bias ? a.bias_ids[c.b0 + i] : c.histp[i - c.nb]) - (long long)c0;
@@ -304,7 +302,8 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
         __syncwarp();
         const int m = n - (e0 + lane * 32);  // this lane's logits that exist
         if (a.softcap > 0.0f) {
-            for (int j = 0; j < min(32, m); j++) mine[j] = softcap_pinned(mine[j], a.softcap);
+#pragma unroll 1
+            for (int j = 0; j < min(32, m); j++) mine[j] = softcap_slow(mine[j], a.softcap);
             __syncwarp();
         }
         if (a.mask && m > 0) {
@@ -327,10 +326,12 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
         __syncthreads();
         if (active) {
             const int nh = s->nhits;
+#pragma unroll 1
             for (int i = tid; i < nh; i += SPAN_THREADS) {
                 const int t = s->hits[i];
                 const int nw = (int)((s->cnt[t >> 1] >> ((t & 1) * 16)) & 0x7fffu);
                 float v = sx[(t >> 5) * PITCH + (t & 31)];
+#pragma unroll 1
                 for (int b = 0; b < c.nb; b++)  // duplicates add up, in the order they were given
                     if (a.bias_ids[c.b0 + b] == (long long)t + c0) v = __fadd_rn(v, a.bias_vals[c.b0 + b]);
                 if (nw > 0) {
@@ -541,9 +542,11 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         const int ng = A.ntile * 32;
         const float *gm = A.gmax + (size_t)rr * ng;
         // one histogram of the lanes' maxima by distance below the row's
+#pragma unroll 1
         for (int i = tid; i < PLAN_BINS; i += NT) S.hist[i] = 0u;
         if (tid == 0) S.edge = -1;
         __syncthreads();
+#pragma unroll 1
         for (int i0 = 0; i0 < ng; i0 += 8 * NT) {
             float v[8];
 #pragma unroll
@@ -573,6 +576,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         // the order of equal probabilities the way the descending walk sees it.
         if (need > HEAD_NEED && A.oG > 0) {
             int have = 0, allowed = 0;
+#pragma unroll 1
             for (int i = tid; i < A.oG * NT; i += NT) {
                 const int g = i / NT, l0 = (i - g * NT) * A.oL, n_g = max(0, min(A.oVc, a.V - g * A.oVc));
                 if (l0 >= n_g) continue;
@@ -580,6 +584,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
                 if (a.mask) {
                     const unsigned int *mrow = a.mask + (long long)r * a.mask_stride;
                     int b = 0;
+#pragma unroll 1
                     for (int j = 0; j < bits; j++) { const int t = g * A.oVc + l0 + j; b += (__ldg(mrow + (t >> 5)) >> (t & 31)) & 1u; }
                     bits = b;
                 }
@@ -633,6 +638,7 @@ __device__ __forceinline__ TileChunk tile_chunk(const float *list, int total) {
     c.cnt = min(per, total - c.off);
     float s0 = 0.0f, s1 = 0.0f;
     int i = 0;
+#pragma unroll 1
     for (; i + 2 <= c.cnt; i += 2) { s0 += list[skew(c.off + i)]; s1 += list[skew(c.off + i + 1)]; }
     if (i < c.cnt) s0 += list[skew(c.off + i)];
     c.csum = s0 + s1;
@@ -664,6 +670,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
         if (usable) {
             const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
             const float C2 = __fmul_rn(1.5f, fpow2(jl + 1)), h2 = fpow2(jl - 23);
+#pragma unroll 1
             for (int i = 0; i < cnt; i++) {
                 const float v = list[skew(off + i)];
                 const float q = __fsub_rn(__fadd_rn(v, C1), C1);
@@ -784,9 +791,10 @@ __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, 
     const bool one = T == 1.0f;
     auto value = [&](float x) -> float {
         // (what is not there is -inf, which div_by cannot take; everything so far down becomes zero)
-        const float v = one ? x : (fast ? div_by(fmaxf(x, -1.0e20f), T, rT) : __fdiv_rn(x, T));
+        const float v = one ? x : (fast ? div_by(fmaxf(x, -1.0e20f), T, rT) : div_slow(x, T));
         return expf_pinned_nonpos(__fsub_rn(v, top));  // no logit of the row exceeds its maximum
     };
+#pragma unroll 1
     for (int i0 = 0; i0 < r.total; i0 += 64) {
         const int i = i0 + lane, j = i + 32;
         const int p = all ? i : (i < r.total ? (int)idx[i] : 0), q = all ? j : (j < r.total ? (int)idx[j] : 0);
@@ -803,6 +811,7 @@ __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, 
 // The careful lanes' values to their places, padded with zeros.
 __device__ __forceinline__ void store_care(float *care, const float *list, const TileChunk &ch, int my_place) {
     const int lane = threadIdx.x & 31;
+#pragma unroll 1
     for (unsigned int left = __ballot_sync(0xffffffffu, my_place != 255); left; left &= left - 1u) {
         const int l = __ffs((int)left) - 1, n = __shfl_sync(0xffffffffu, ch.cnt, l), o = __shfl_sync(0xffffffffu, ch.off, l);
         const int at = __shfl_sync(0xffffffffu, my_place, l);
@@ -852,6 +861,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     store_care(A.care(rr), list, ch, my_place);
     const bool whole = (pl.flags & F_LIST) || __any_sync(0xffffffffu, care && my_place == 255);
     if (whole)
+#pragma unroll 1
         for (int i = lane; i < t.total; i += 32) A.elist[gt * TILE + i] = list[skew(i)];
     if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = t.keep;
     if (lane == 0) {
@@ -930,10 +940,12 @@ __device__ void head_sort(HeadShared *S, int n) {
         int rank = 0;
         if (warp * 32 < n) {
             int j = 0;
+#pragma unroll 1
             for (; j + 4 <= n; j += 4) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(S->cand + j), b = *reinterpret_cast<const ulonglong2 *>(S->cand + j + 2);
                 rank += (a.x > mine ? 1 : 0) + (a.y > mine ? 1 : 0) + (b.x > mine ? 1 : 0) + (b.y > mine ? 1 : 0);
             }
+#pragma unroll 1
             for (; j < n; j++) rank += S->cand[j] > mine ? 1 : 0;
         }
         __syncthreads();
@@ -979,6 +991,7 @@ __device__ void head_sort(HeadShared *S, int n) {
             if (tid + u * HT < n) {
                 const unsigned int b = S->sbin[bin_of(k[u])], b0 = b & 0xffffu, m = b >> 16;
                 rank[u] = b0;
+#pragma unroll 1
                 for (unsigned int j = 0; j < m; j++) rank[u] += S->tmp[b0 + j] > k[u] ? 1u : 0u;
             }
         __syncthreads();   // the values take the space of the keys being read
@@ -1075,6 +1088,7 @@ struct WalkLoads {
 __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
     CareRec nx = W->rec[0];
+#pragma unroll 1
     for (int q = 0; q <= nrec; q++) {
         const CareRec r = nx;
         const unsigned int kind = (r.meta >> 8) & 3u, place = r.meta >> 24;
@@ -1133,6 +1147,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
         return;
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = tid; i < m; i += HT) {
         const float p = pc[i];
         const float l = (p > 0.0f) ? logf_pinned(p) : 0.0f;
@@ -1142,6 +1157,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
     __syncthreads();
     if (tid == 0) {
         float ent = 0.0f;
+#pragma unroll 1
         for (int i = 0; i < m; i++)
             if (pc[i] > 0.0f) ent = __fsub_rn(ent, S->typ.tt[i]);
         S->ent = ent;
@@ -1164,6 +1180,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
         }
     }
     __syncthreads();
+#pragma unroll 1
     for (int j = 0; j < m; j++) {
         const unsigned long long o = keys[j];
 #pragma unroll
@@ -1178,6 +1195,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
         auto at_of = [&](int j) { return (int)(0xFFFFFFFFu - (unsigned int)(keys[j] & 0xFFFFFFFFull)); };
         float s = 0.0f;
         int kept = m;
+#pragma unroll 1
         for (int j = 0; j < m; j++) {
             s = __fadd_rn(s, pc[at_of(j)]);
             pre[j] = s;
@@ -1189,6 +1207,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
         if (sum <= 0.0f) at = 0;  // sample.mojo:583-584
         else {
             target = __fmul_rn(draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull), sum);
+#pragma unroll 1
             for (int j = 0; j < kept; j++)
                 if (target < pre[j]) { at = j; break; }
         }
@@ -1248,6 +1267,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     }
     // ---- sorted order: the head's candidates as probabilities
     const int nc = ncand;
+#pragma unroll 1
     for (int i = tid; i < nc; i += HT) {
         if (i >= HT) key = R.cand(rr)[i];
         S->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(key), Z, yZ)) << 32) | (key & 0xFFFFFFFFull);
@@ -1264,6 +1284,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
             return;
         }
         int n = 0;
+#pragma unroll 1
         for (int i = tid; i < nc; i += HT) n += S->p.pc[i] >= floor_p ? 1 : 0;
         n = __reduce_add_sync(0xffffffffu, n);
         if (lane == 0 && n) atomicAdd(&S->n_ge, n);
@@ -1274,6 +1295,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     }
 #ifdef MOLLA_SAMPLE_TESTING
     if (a.topk_out) {
+#pragma unroll 1
         for (int i = tid; i < a.topk_cap; i += HT)
             a.topk_out[(long long)r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? key_idx(S->cand[i]) : -1;
     }
@@ -1292,6 +1314,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
         const float4 *p4 = reinterpret_cast<const float4 *>(pc);
         float4 x = p4[0], y = p4[1];
+#pragma unroll 1
         for (int i = 0; i < lim && cut < 0; i += 8) {
             const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
             if (i + 8 < lim) { x = p4[(i >> 2) + 2]; y = p4[(i >> 2) + 3]; }
@@ -1351,10 +1374,12 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     // past the head: the sorted candidates and their prefix sums go along, and empty tables for tile_walk
     {
         ulonglong2 *z = reinterpret_cast<ulonglong2 *>(R.table(rr, 0));
+#pragma unroll 1
         for (int i = tid; i < WALK_BINADES * NBINS / 2; i += HT) z[i] = make_ulonglong2(0ull, 0ull);
         if (tid < WALK_BINADES) R.ties(rr)[tid].n = 0;
         if (tid == 0) { R.picks(rr)->n = 0; R.picks(rr)->arrived = 0; }
     }
+#pragma unroll 1
     for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
     queue_row(ST_HEAD, 6);
 }
@@ -1374,121 +1399,124 @@ union __align__(16) WalkTileShared {
     };
 };
 
+struct PlanFind { double ws[SPAN_THREADS / 32]; double before, end, total; int hit; unsigned int prev; int next; int pick[PICKS], n; };
+
+// In a walk's table `tab` below bin `hi`, with m0 units before it: the first bin from the top whose end
+// reaches x units (F.hit, or -1), the units before and behind it, its neighbours that hold anything, and
+// the units of all bins.
+__device__ __noinline__ void plan_find(PlanFind &F, const unsigned long long *tab, int hi, double m0, double x) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = NBINS / SPAN_THREADS;
+    const int top = NBINS - 1 - PER * tid;
+    unsigned long long q[PER], sum = 0ull;
+#pragma unroll
+    for (int i = 0; i < PER; i++) { q[i] = top - i < hi ? __ldcg(tab + top - i) : 0ull; sum += q[i]; }
+    const double inc = warp_incl_scan((double)sum, lane);
+    __syncthreads();
+    if (lane == 31) F.ws[warp] = inc;
+    if (tid == 0) { F.hit = -1; F.prev = 0xffffffffu; F.next = -1; }
+    __syncthreads();
+    double b0 = 0.0, t = 0.0;
+#pragma unroll 1
+    for (int w = 0; w < SPAN_THREADS / 32; w++) { if (w == warp) b0 = t; t += F.ws[w]; }
+    if (tid == 0) F.total = t;
+    double c = m0 + b0 + (inc - (double)sum);
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int b = top - i;
+        const double v = (double)q[i];
+        if (v > 0.0) {
+            if (c < x && c + v >= x) { F.hit = b; F.before = c; F.end = c + v; }
+            if (c + v < x) atomicMin(&F.prev, (unsigned int)b);   // the last one before it
+            if (c >= x) atomicMax(&F.next, b);                    // the first one behind it
+        }
+        c += v;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void plan_want(PlanFind &F, int b) {   // one thread
+    if (b < 0 || b >= NBINS) return;
+#pragma unroll 1
+    for (int i = 0; i < F.n; i++) if (F.pick[i] == b) return;
+    if (F.n < PICKS) F.pick[F.n++] = b;
+}
+
 // Which bins the walk past row rr's head will look into element by element: from the tables alone the
 // sum before every bin is known to within the rounding inside one bin and a few ties, so the bins where it
 // crosses into the next binade, reaches top-p, or passes the drawn target are known but for a neighbour.
 // What is left out here is only slower: row_tail then looks for it in the list.
 __device__ __noinline__ void plan_picks(const RowsArgs &R, int rr, float hs, int j0, int nb) {
-    __shared__ double ws[SPAN_THREADS / 32];
-    __shared__ int s_bin[4];
-    __shared__ double s_before[2];
-    __shared__ int picked[PICKS];
-    __shared__ int npick;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int PER = NBINS / SPAN_THREADS;
-    const RowHead *head = R.head(rr);
-    const RowCfg &g = head->plan.c;
-    if (tid == 0) npick = 0;
-    auto want = [&](int b) {   // thread 0
-        if (b < 0 || b >= NBINS) return;
-        for (int i = 0; i < npick; i++) if (picked[i] == b) return;
-        if (npick < PICKS) picked[npick++] = b;
-    };
-    // For the table of binade j0 + p below bin `hi`, with m0 units before it: the first bin (descending)
-    // whose end reaches x units, the units before it, and its neighbours that hold anything.
-    double q[PER];
-    auto load = [&](int p, int hi) {
-#pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int b = NBINS - 1 - PER * tid - i;
-            q[i] = b < hi ? (double)__ldcg(R.table(rr, p) + b) : 0.0;
-        }
-    };
-    double total = 0.0;
-    auto find = [&](double m0, double x) -> int {   // all threads; results in s_bin[0..2], s_before
-        double sum = 0.0;
-#pragma unroll
-        for (int i = 0; i < PER; i++) sum += q[i];
-        const double inc = warp_incl_scan(sum, lane);
-        __syncthreads();
-        if (lane == 31) ws[warp] = inc;
-        if (tid == 0) { s_bin[0] = -1; s_bin[1] = -1; s_bin[2] = -1; }
-        __syncthreads();
-        double b0 = 0.0, t = 0.0;
-#pragma unroll
-        for (int w = 0; w < SPAN_THREADS / 32; w++) { if (w == warp) b0 = t; t += ws[w]; }
-        total = t;
-        double c = m0 + b0 + (inc - sum);
-#pragma unroll
-        for (int i = 0; i < PER; i++) {
-            const int b = NBINS - 1 - PER * tid - i;
-            if (q[i] > 0.0) {
-                if (c < x && c + q[i] >= x) { s_bin[0] = b; s_before[0] = c; s_before[1] = c + q[i]; }
-                if (c + q[i] < x) atomicMin(reinterpret_cast<unsigned int *>(&s_bin[1]), (unsigned int)b);   // the last one before it
-                if (c >= x) atomicMax(&s_bin[2], b);                                                          // the first one behind it
-            }
-            c += q[i];
-        }
-        __syncthreads();
-        return s_bin[0];
-    };
+    __shared__ PlanFind F;
+    const int tid = threadIdx.x;
+    const RowCfg &g = R.head(rr)->plan.c;
     const double slack = 96.0;
-    double start[WALK_BINADES + 1];
+    double start[WALK_BINADES];
     int hi_of[WALK_BINADES], low_of[WALK_BINADES];
-    double s = (double)hs, sum_lo = 0.0, sum_hi = 0.0;
+    double s = (double)hs, sum_lo = s, sum_hi = s;
     int hi = NBINS, phases = 0;
-    bool cut = false;
-    __syncthreads();
-    for (int p = 0; p < nb && !cut; p++) {
-        const double unit = dpow2(j0 + p - 23), m0 = s / unit;
+    if (tid == 0) F.n = 0;
+    // stretch p: the running sum in binade j0 + p
+#pragma unroll
+    for (int p = 0; p < WALK_BINADES; p++) {
+        start[p] = s; hi_of[p] = hi; low_of[p] = 0;
+        if (p >= nb || hi <= 0) continue;
+        const double unit = dpow2(j0 + p - 23), inv = dpow2(23 - j0 - p);
         double x = 16777216.0;
-        bool by_cut = false;
-        if (g.topp_on) { const double t = ceil((double)g.P / unit); if (t <= x) { x = t; by_cut = true; } }
-        load(p, hi);
-        const int hb = find(m0, x);
-        start[p] = s; hi_of[p] = hi; low_of[p] = hb < 0 ? 0 : hb;
+        const double cut = g.topp_on ? ceil((double)g.P * inv) : 1.0e30;
+        const bool by_cut = cut <= x;
+        if (by_cut) x = cut;
+        plan_find(F, R.table(rr, p), hi, s * inv, x);
         phases = p + 1;
-        if (hb < 0) { sum_lo = (m0 + total) * unit; sum_hi = sum_lo; break; }
+        const int hb = F.hit;
+        if (hb < 0) { s = s + F.total * unit; sum_lo = sum_hi = s; hi = 0; continue; }
+        low_of[p] = hb;
         if (tid == 0) {
-            want(hb);
-            if (x - s_before[0] < slack) want(s_bin[1]);
-            if (s_before[1] - x < slack) want(s_bin[2]);
+            plan_want(F, hb);
+            if (x - F.before < slack) plan_want(F, (int)F.prev);
+            if (F.end - x < slack) plan_want(F, F.next);
         }
-        if (by_cut) { cut = true; sum_lo = x * unit; sum_hi = fmin(s_before[1] * unit, (x + slack) * unit + (double)__uint_as_float((unsigned int)(hb + 1) << BIN_SHIFT)); }
-        s = s_before[1] * unit;
-        sum_lo = cut ? sum_lo : s; sum_hi = cut ? sum_hi : s;
-        hi = hb;
+        s = F.end * unit;
+        sum_lo = sum_hi = s;
+        if (by_cut) { sum_lo = x * unit; sum_hi = fmin(s, (x + slack) * unit + (double)__uint_as_float((unsigned int)(hb + 1) << BIN_SHIFT)); }
+        hi = by_cut ? 0 : hb;
         __syncthreads();
     }
     // the draw
     const BatchArgs &a = R.a;
     const double u01 = (double)draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull);
-    const double tg[2] = {u01 * sum_lo * (1.0 - 1.0e-6), u01 * sum_hi * (1.0 + 1.0e-6)};
     int last = -1;
+#pragma unroll 1
     for (int k = 0; k < 2; k++) {
-        if (tg[k] < (double)hs) continue;   // in the head
+        const double tg = k == 0 ? u01 * sum_lo * (1.0 - 1.0e-6) : u01 * sum_hi * (1.0 + 1.0e-6);
+        if (tg < (double)hs) continue;   // in the head
         int p = 0;
-        while (p + 1 < phases && tg[k] >= start[p + 1]) p++;
-        const double unit = dpow2(j0 + p - 23);
-        load(p, hi_of[p]);
-        const int b = find(start[p] / unit, tg[k] / unit);
-        if (tid == 0) { want(b); want(last); }
-        last = b;
+        double st = start[0];
+        int h = hi_of[0];
+#pragma unroll
+        for (int i = 1; i < WALK_BINADES; i++)
+            if (i < phases && tg >= start[i]) { p = i; st = start[i]; h = hi_of[i]; }
+        const double inv = dpow2(23 - j0 - p);
+        plan_find(F, R.table(rr, p), h, st * inv, tg * inv);
+        if (tid == 0) { plan_want(F, F.hit); plan_want(F, last); }
+        last = F.hit;
         __syncthreads();
     }
     // ties at or above the lowest bin of their binade's stretch: what precedes them in their bins is wanted
     if (tid == 0) {
-        for (int p = 0; p < phases; p++) {
+#pragma unroll
+        for (int p = 0; p < WALK_BINADES; p++) {
             const WalkTies *t = R.ties(rr) + p;
-            const int n = min(__ldcg(&t->n), TIE_CAP);
+            const int n = p < phases ? min(__ldcg(&t->n), TIE_CAP) : 0;
+#pragma unroll 4
             for (int i = 0; i < n; i++) {
                 const int b = (int)((unsigned int)(__ldcg(&t->key[i]) >> 32) >> BIN_SHIFT);
-                if (b >= low_of[p] && b < hi_of[p]) want(b);
+                if (b >= low_of[p] && b < hi_of[p]) plan_want(F, b);
             }
         }
         WalkPicks *o = R.picks(rr);
-        for (int i = 0; i < npick; i++) { o->bin[i] = picked[i]; o->cnt[i] = 0; }
-        o->n = npick;
+#pragma unroll 1
+        for (int i = 0; i < F.n; i++) { o->bin[i] = F.pick[i]; o->cnt[i] = 0; }
+        o->n = F.n;
     }
     __syncthreads();
 }
@@ -1501,6 +1529,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
     pdl_next();
     pdl_wait();
     const int work = R.queue[0] * R.nspan;
+#pragma unroll 1
     for (int wi = blockIdx.x; wi < work; wi += gridDim.x) {
         const int rr = R.queue[1 + wi / R.nspan], span = wi % R.nspan, tile = span * (SPAN / TILE) + warp;
         RowHead *head = R.head(rr);
@@ -1510,26 +1539,23 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
         const size_t gt = (size_t)rr * R.ntile + tile;
         const int n = tile < R.ntile ? (int)R.to(rr)[tile].cnt : 0;
         float4 *src = reinterpret_cast<float4 *>(R.elist + gt * TILE);
-        float4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (4 * (lane + 32 * i) < n) v[i] = src[lane + 32 * i];
         __syncthreads();
         if (state == ST_PURE) {
             if (tile >= R.ntile) continue;
             float *list = S->x + (size_t)warp * 32 * PITCH;
             __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int e0 = 4 * (lane + 32 * i);
-                if (e0 >= n) continue;
-                float p[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+            float4 nx = 4 * lane < n ? src[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+            for (int e0 = 4 * lane; e0 < n; e0 += 128) {
+                const float4 v = nx;
+                if (e0 + 128 < n) nx = src[(e0 >> 2) + 32];
+                float p[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     p[u] = e0 + u < n ? prob_of(p[u], Z, yZ) : 0.0f;
                     list[skew(e0 + u)] = p[u];
                 }
-                src[lane + 32 * i] = make_float4(p[0], p[1], p[2], p[3]);
+                src[e0 >> 2] = make_float4(p[0], p[1], p[2], p[3]);
             }
             __syncwarp();
             const TileChunk ch = tile_chunk(list, n);
@@ -1553,20 +1579,23 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
         const float hs = head->head_s;
         const int j0 = hs > 0.0f ? fexpo(hs) : 0, nb = (hs > 0.0f && j0 >= -30 && j0 < 0) ? min(WALK_BINADES, -j0) : 0;
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) { (&S->hq[0][0])[i] = 0u; (&S->hqh[0][0])[i] = 0u; }
         __syncthreads();
+        float4 nx = 4 * lane < n ? src[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const float half0 = fpow2(j0 - 24);   // below half a unit of the first binade: adds nothing from here on
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int e0 = 4 * (lane + 32 * i);
-            if (e0 >= n) continue;
-            float p[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll 1
+        for (int e0 = 4 * lane; e0 < n; e0 += 128) {
+            const float4 v = nx;
+            if (e0 + 128 < n) nx = src[(e0 >> 2) + 32];
+            float p[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 p[u] = (e0 + u < n && __float_as_uint(p[u]) < tau) ? prob_of(p[u], Z, yZ) : 0.0f;
                 if (!(p[u] >= half0)) continue;
                 const unsigned int pb = __float_as_uint(p[u]);
                 const int bin = (int)(pb >> BIN_SHIFT);
+#pragma unroll 1
                 for (int b = 0; b < nb; b++) {
                     const float Cm = __fmul_rn(1.5f, fpow2(j0 + b));
                     const float tq = __fadd_rn(p[u], Cm);
@@ -1585,9 +1614,10 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
                     if (qu >> MASS_SPLIT) sred_add(&S->hqh[b][bin], qu >> MASS_SPLIT);
                 }
             }
-            src[lane + 32 * i] = make_float4(p[0], p[1], p[2], p[3]);
+            src[e0 >> 2] = make_float4(p[0], p[1], p[2], p[3]);
         }
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) {
             const unsigned long long q = (unsigned long long)(&S->hq[0][0])[i] + ((unsigned long long)(&S->hqh[0][0])[i] << MASS_SPLIT);
             if (q) atomicAdd(R.table(rr, 0) + i, q);
@@ -1613,6 +1643,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_pick_kernel(const __grid
     pdl_next();
     pdl_wait();
     const int work = R.queue[0] * R.nspan;
+#pragma unroll 1
     for (int wi = blockIdx.x; wi < work; wi += gridDim.x) {
         const int rr = R.queue[1 + wi / R.nspan], span = wi % R.nspan, tile = span * (SPAN / TILE) + warp;
         if (R.head(rr)->state != ST_HEAD) continue;
@@ -1626,6 +1657,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_pick_kernel(const __grid
         for (int i = 0; i < 8; i++)
             if (4 * (lane + 32 * i) < n) v[i] = src[lane + 32 * i];
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < NBINS / 4; i += SPAN_THREADS) reinterpret_cast<unsigned int *>(slot)[i] = 0u;
         __syncthreads();
         if (tid < npick) slot[pk->bin[tid]] = (unsigned char)(tid + 1);
@@ -1686,6 +1718,7 @@ struct __align__(16) AuxF {
     float b_s; int b_event; int b_idx; float b_p; long long b_pos; int b_aux;
     float b_sum, b_target;
     unsigned int w_sb; int w_i, w_need, w_found, w_tile, w_at;   // the items' runner
+    WalkTies ties[WALK_BINADES]; WalkPicks picks;   // row_tail's copies
     int ntie; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP];
     unsigned long long tpqm[TIE_CAP], tabove[TIE_CAP], tc[TIE_CAP];
     unsigned int tbits[NBINS / 32];
@@ -1711,34 +1744,29 @@ struct CtxF {
     RowPlan pl;
     int tj0, tnb;                // binades that tile_walk has left tables for
     int npick;                   // bins that tile_pick has gathered
+    bool first_table;            // the table of binade tj0 is in shared memory
     float *list;                 // this row's [ntile][TILE]
     Item *gitems;                // this row's items
     const unsigned int *kmask;   // this row's [ntile][32]
 };
 
 // One entry of the list, as a token id: the nth logit its tile kept.
-__device__ int token_of(const CtxF &c, int tile, int nth) {
-    const uint4 *m = reinterpret_cast<const uint4 *>(c.kmask + (size_t)tile * 32);
-    int at = 0;
-    uint4 w[8];
-#pragma unroll
-    for (int g = 0; g < 8; g++) w[g] = m[g];
-#pragma unroll
-    for (int g = 0; g < 8; g++) {
-        const unsigned int v[4] = {w[g].x, w[g].y, w[g].z, w[g].w};
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int n = __popc(v[u]);
-            if (nth >= at && nth < at + n) return tile * TILE + (4 * g + u) * 32 + (int)__fns(v[u], 0, nth - at + 1);
-            at += n;
-        }
+__device__ __noinline__ int token_of(const CtxF &c, int tile, int nth) {
+    const unsigned int *m = c.kmask + (size_t)tile * 32;
+#pragma unroll 8
+    for (int g = 0; g < 32; g++) {
+        unsigned int w = m[g];
+        const int n = __popc(w);
+        if (nth >= n) { nth -= n; continue; }
+        while (nth-- > 0) w &= w - 1u;
+        return tile * TILE + g * 32 + __ffs((int)w) - 1;
     }
     return tile * TILE;
 }
 __device__ __forceinline__ int token_of(const CtxF &c, int pos) { return token_of(c, pos >> 10, pos & (TILE - 1)); }
 
 // Tiles [t0, t1) of one span evaluated again, as kernel 3 did it: their values packed into dst or the list.
-__device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
+__device__ __noinline__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
     AuxF *A = c.A;
     IN_SHARED(A);
     const RowsArgs &R = *c.R;
@@ -1754,6 +1782,7 @@ __device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
         const TileEval e = tile_eval(list, reinterpret_cast<unsigned short *>(s->cnt) + c.warp * TILE, thr, c.cfg.T, __fdiv_rn(1.0f, c.cfg.T), c.pl.top,
                                      (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, int) {});
         float *to = to_list ? c.list + (size_t)t * TILE : dst;
+#pragma unroll 1
         for (int i = c.lane; i < e.total; i += 32) to[i] = list[skew(i)];
         if (to_list) const_cast<unsigned int *>(c.kmask)[(size_t)t * 32 + c.lane] = e.keep;
     }
@@ -1766,6 +1795,7 @@ __device__ void tile_again(CtxF &c, int t0, int t1, float *dst, bool to_list) {
 __device__ __forceinline__ int run_values(unsigned int &sb, const float *v, int n, bool locate, float target) {
     const float4 *v4 = reinterpret_cast<const float4 *>(v);
     float s = __uint_as_float(sb);
+#pragma unroll 1
     for (int i = 0; i < n; i += 8) {
         const float4 x = v4[i >> 2], y = v4[(i >> 2) + 1];
         const float s0 = s;
@@ -1773,6 +1803,7 @@ __device__ __forceinline__ int run_values(unsigned int &sb, const float *v, int 
         s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, y.x), y.y), y.z), y.w);
         if (locate && target < s) {
             s = s0;
+#pragma unroll 1
             for (int u = 0; u < 8; u++) {
                 s = __fadd_rn(s, v[i + u]);
                 if (target < s) { sb = __float_as_uint(s); return i + u; }
@@ -1851,12 +1882,14 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
         if (t + 1 < R.ntile) A->toff[t + 1] = ex + n0;
     }
     if (c.tid == 0) { A->w_sb = 0u; A->w_found = 0; A->w_tile = 0; A->w_at = 0; }
+#pragma unroll 1
     for (int b0 = 0; b0 < total; b0 += ITEM_CAP) {
         const int n = min(ITEM_CAP, total - b0);
         __syncthreads();
         if (c.tid == 0) { A->ncare = 0; A->w_i = 0; }
         __syncthreads();
         // an item per thread: its tile is found in the tiles' offsets
+#pragma unroll 1
         for (int i = c.tid; i < n; i += NT) {
             int lo = 0, hi = R.ntile - 1;
             while (lo < hi) {
@@ -1874,12 +1907,14 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
         }
         __syncthreads();
         const int ncare = min(A->ncare, CARE_CAP);
+#pragma unroll 1
         for (int q = c.warp; q < ncare; q += NWARP) {
             const int i = A->careidx[q];
             const Item it = A->items[i];
             A->care[q * 32 + c.lane] = c.lane >= it.cnt() ? 0.0f : (it.place() != 255u ? R.care(c.rr)[it.place() * 32 + c.lane] : c.list[(size_t)it.tile() * TILE + it.off() + c.lane]);
         }
         FCOUNT(20, n); FCOUNT(21, ncare); if (!locate) FSTAMP(2);
+#pragma unroll 1
         for (int round = 0; round <= n; round++) {   // (each round but the last is for one more item)
             __syncthreads();
             if (c.warp == 0) run_items(A, n, locate, target);
@@ -1893,12 +1928,15 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
             if (it.place() != 255u) {
                 if (c.tid < 32) A->ebuf[c.tid] = c.tid < m ? R.care(c.rr)[it.place() * 32 + c.tid] : 0.0f;
             } else if ((c.pl.flags & F_LIST) || it.kind() != K_RUN) {
+#pragma unroll 1
                 for (int i = c.tid; i < ((m + 7) & ~7); i += NT) A->ebuf[i] = i < m ? c.list[(size_t)t * TILE + off + i] : 0.0f;
             } else {
                 tile_again(c, t, t + 1, A->ebuf, false);
                 float x[TILE / NT];
+#pragma unroll 1
                 for (int i = c.tid, u = 0; u < TILE / NT; i += NT, u++) x[u] = i < m ? A->ebuf[off + i] : 0.0f;
                 __syncthreads();
+#pragma unroll 1
                 for (int i = c.tid, u = 0; u < TILE / NT; i += NT, u++) A->ebuf[i] = x[u];
             }
             __syncthreads();
@@ -1918,23 +1956,24 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
 }
 
 // Calls f(values, position of the first, where they are) for the row's list, four neighbouring entries of
-// a lane at a time (zero: none). All lanes of a warp make the same calls. A whole tile is asked for at once.
+// a lane at a time (zero: none). All lanes of a warp make the same calls. (Kept small: it is rarely needed, and cold code
+// is fetched from L2.)
 template <class F>
 __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
     const AuxF *A = c.A;
     IN_SHARED(A);
+#pragma unroll 1
     for (int t = c.warp; t < c.R->ntile; t += NWARP) {
         const int n = A->tcnt[t];
         const uint4 *src = reinterpret_cast<const uint4 *>(c.list + (size_t)t * TILE) + c.lane;
-        uint4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (4 * (c.lane + 32 * i) < n) v[i] = src[32 * i];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            if (128 * i >= n) break;
+        uint4 nx = make_uint4(0u, 0u, 0u, 0u);
+        if (4 * c.lane < n) nx = src[0];
+#pragma unroll 1
+        for (int i = 0; 128 * i < n; i++) {
+            const uint4 v = nx;
             const int e0 = 4 * (c.lane + 32 * i);
-            const unsigned int eb[4] = {e0 < n ? v[i].x : 0u, e0 + 1 < n ? v[i].y : 0u, e0 + 2 < n ? v[i].z : 0u, e0 + 3 < n ? v[i].w : 0u};
+            if (e0 + 128 < n) nx = src[32 * (i + 1)];
+            const unsigned int eb[4] = {e0 < n ? v.x : 0u, e0 + 1 < n ? v.y : 0u, e0 + 2 < n ? v.z : 0u, e0 + 3 < n ? v.w : 0u};
             f(eb, t * TILE + e0, c.list + (size_t)t * TILE + e0);
         }
     }
@@ -1952,6 +1991,7 @@ __device__ __noinline__ void sort_head(CtxF &c, int n) {
         const unsigned long long mine = (c.tid < n) ? A->cand[c.tid] : 0ull;
         int rank = 0;
         if (c.tid < n)
+#pragma unroll 1
             for (int j = 0; j < n; j++) rank += A->cand[j] > mine ? 1 : 0;
         __syncthreads();
         if (c.tid < n) { A->cand[rank] = mine; A->pc[rank] = key_val(mine); }
@@ -1997,6 +2037,7 @@ __device__ __noinline__ void sort_head(CtxF &c, int n) {
             if (c.tid + u * NT < n) {
                 const unsigned int b = A->sbin[bin[u]], b0 = b & 0xffffu, m = b >> 16;
                 unsigned int rank = b0;
+#pragma unroll 1
                 for (unsigned int j = 0; j < m; j++) rank += A->tmp[b0 + j] > k[u] ? 1u : 0u;
                 A->cand[rank] = k[u];
                 A->pc[rank] = key_val(k[u]);
@@ -2013,6 +2054,7 @@ __device__ __noinline__ int narrow_head(CtxF &c, unsigned long long *cand) {
     AuxF *A = c.A;
     IN_SHARED(A);
     __syncthreads();
+#pragma unroll 1
     for (int i = c.tid; i < NBINS; i += NT) A->u.h.hc[i] = 0u;
     if (c.tid == 0) { A->ncand = 0; A->evt_thread = -1; }
     __syncthreads();
@@ -2036,9 +2078,11 @@ __device__ __noinline__ int narrow_head(CtxF &c, unsigned long long *cand) {
     if (A->evt_thread < 0 || A->b_idx > HEADCAP) return HEADCAP + 1;
     const unsigned int edge = (unsigned int)A->evt_thread << BIN_SHIFT;
     c.pl.tau_bits = edge > 1u ? edge : 1u;
+#pragma unroll 1
     for (int t = c.warp; t < c.R->ntile; t += NWARP) {
         unsigned int m = c.kmask[(size_t)t * 32 + c.lane];
         const float *src = c.list + (size_t)t * TILE + (warp_incl_scan(__popc(m), c.lane) - __popc(m));
+#pragma unroll 1
         for (int i = 0; m; i++, m &= m - 1u) {
             const unsigned int eb = __float_as_uint(src[i]);
             if (eb >= c.pl.tau_bits) cand[satom_add(&A->ncand, 1)] = make_key(eb, t * TILE + c.lane * 32 + __ffs((int)m) - 1);
@@ -2072,12 +2116,14 @@ struct FResume {
 };
 
 // position of the (nth+1)-th entry, in vocabulary order, whose bits equal `eb`
-__device__ int list_nth_equal(CtxF &c, unsigned int eb, int nth) {
+__device__ __noinline__ int list_nth_equal(CtxF &c, unsigned int eb, int nth) {
     AuxF *A = c.A;
     IN_SHARED(A);
     __syncthreads();
+#pragma unroll 1
     for (int t = c.warp; t < c.R->ntile; t += NWARP) {
         int n = 0;
+#pragma unroll 1
         for (int i = c.lane; i < A->tcnt[t]; i += 32) n += __float_as_uint(c.list[(size_t)t * TILE + i]) == eb ? 1 : 0;
         n = __reduce_add_sync(0xffffffffu, n);
         if (c.lane == 0) A->toff[t] = n;
@@ -2085,8 +2131,10 @@ __device__ int list_nth_equal(CtxF &c, unsigned int eb, int nth) {
     __syncthreads();
     if (c.tid == 0) {
         int seen = 0, at = 0;
+#pragma unroll 1
         for (int t = 0; t < c.R->ntile; t++) {
             if (nth < seen + A->toff[t]) {
+#pragma unroll 1
                 for (int i = 0; i < A->tcnt[t]; i++)
                     if (__float_as_uint(c.list[(size_t)t * TILE + i]) == eb && seen++ == nth) { at = t * TILE + i; break; }
                 break;
@@ -2099,7 +2147,7 @@ __device__ int list_nth_equal(CtxF &c, unsigned int eb, int nth) {
     return A->b_idx;
 }
 
-__device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long long nstop, FResume &rs, bool try_resume) {
+__device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long long nstop, FResume &rs, bool try_resume) {
     AuxF *A = c.A;
     IN_SHARED(A);
     const bool counting = nstop >= 0;
@@ -2112,6 +2160,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         w.s = rs.s; w.pos = rs.pos; w.tau = rs.tau;
         lvl = rs.lvl; lo = rs.lo; shift = rs.shift; tie_mode = rs.tie_mode != 0;
     }
+#pragma unroll 1
     for (int phase = 0; phase < 8192; phase++) {
         FCOUNT(22, 1);
         const bool reuse = resumed && phase == 0 && !rs.tabbed;  // this phase's tables stand already
@@ -2129,16 +2178,19 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         const unsigned long long *tab = nullptr;
         int bin_hi = NBINS;
         if (c.tnb > 0 && ties_listed && !counting && j >= c.tj0 && j < c.tj0 + c.tnb && (wtau == 0xFFFFFFFFu || (wtau & ((1u << BIN_SHIFT) - 1u)) == 0u)) {
-            tt = c.R->ties(c.rr) + (j - c.tj0);
+            tt = A->ties + (j - c.tj0);
             if (tt->n <= TIE_CAP) {
-                tab = c.R->table(c.rr, j - c.tj0);
+                tab = (j == c.tj0 && c.first_table) ? reinterpret_cast<const unsigned long long *>(&A->u.h) : c.R->table(c.rr, j - c.tj0);
                 if (wtau != 0xFFFFFFFFu) bin_hi = (int)(wtau >> BIN_SHIFT);
             }
         }
         const bool tabbed = tab != nullptr;
         if (!reuse) {
+            if (!tabbed) c.first_table = false;
             if (!tabbed)
+#pragma unroll 1
                 for (int i = c.tid; i < NBINS; i += NT) { A->u.h.hq[i] = 0u; A->u.h.hqh[i] = 0u; A->u.h.hc[i] = 0u; }
+#pragma unroll 1
             for (int i = c.tid; i < NBINS / 32; i += NT) A->tbits[i] = 0u;
             rs.valid = 1; rs.s = w.s; rs.pos = w.pos; rs.tau = w.tau;
             rs.lvl = lvl; rs.lo = lo; rs.shift = shift; rs.tie_mode = tie_mode ? 1 : 0; rs.ntie = 0; rs.tabbed = tabbed ? 1 : 0;
@@ -2234,8 +2286,9 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             rs.ntie = ntie;
             if (ntie > TIE_CAP) { tie_mode = false; c.status |= MOLLA_ROW_SLOW_PATH; continue; }  // too many: they stop phases instead
         }
-        const WalkPicks *pk = c.R->picks(c.rr);
+        const WalkPicks *pk = &A->picks;
         auto pick_of = [&](int b) -> int {   // the bin's place among the gathered ones, -1: not there
+#pragma unroll 1
             for (int i = 0; i < c.npick; i++)
                 if (pk->bin[i] == b && pk->cnt[i] <= PICK_CAP) return i;
             return -1;
@@ -2249,14 +2302,18 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
             }
             __syncthreads();
             int tb_lo = NBINS, tb_hi = -1;
+#pragma unroll 1
             for (int t = 0; t < ntie; t++) { tb_lo = min(tb_lo, A->tbin[t]); tb_hi = max(tb_hi, A->tbin[t]); }
             const unsigned int tb_span = (unsigned int)(tb_hi - tb_lo);
             bool gathered = tabbed;
+#pragma unroll 1
             for (int t = 0; t < ntie && gathered; t++) gathered = pick_of(A->tbin[t]) >= 0;
             if (gathered) {
+#pragma unroll 1
                 for (int t = 0; t < ntie; t++) {
                     const int k = pick_of(A->tbin[t]), m = pk->cnt[k];
                     const unsigned long long *keys = c.R->picked(c.rr, k), tk = A->tkey[t];
+#pragma unroll 1
                     for (int i = c.tid; i < m; i += NT) {
                         const unsigned long long key = keys[i];
                         const unsigned int eb = (unsigned int)(key >> 32);
@@ -2291,6 +2348,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                     if (fabsf(rr) == halfu || p >= bigthr) continue;
                     const unsigned int qu = __float_as_uint(tq) - cm_bits;
                     const unsigned long long key = make_key(eb, pos0 + u);
+#pragma unroll 1
                     for (int t = 0; t < ntie; t++)
                         if (A->tbin[t] == bin && key > A->tkey[t] && qu) {  // two halves, as in the bin tables
                             sred_add(&A->tpq_lo[t], qu & MASS_LO_MASK);
@@ -2316,6 +2374,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
 #pragma unroll
                 for (int i = 0; i < BPT; i++) {
                     const int b = NBINS - 1 - BPT * c.tid - i;
+#pragma unroll 1
                     for (int t = 0; t < ntie; t++)
                         if (A->tbin[t] == b) A->tabove[t] = run;
                     run += q[i];
@@ -2324,8 +2383,10 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                 if (c.tid == 0) {
                     // from the top down (what lies below an event never matters: the walk stops there)
                     unsigned long long done = 0ull, carried = 0ull;
+#pragma unroll 1
                     for (int round = 0; round < ntie; round++) {
                         int best = -1;
+#pragma unroll 1
                         for (int t = 0; t < ntie; t++)
                             if (!((done >> t) & 1ull) && (best < 0 || A->tkey[t] > A->tkey[best])) best = t;
                         done |= 1ull << best;
@@ -2345,6 +2406,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
 #pragma unroll
                 for (int i = 0; i < BPT; i++) {
                     const int b = NBINS - 1 - BPT * c.tid - i;
+#pragma unroll 1
                     for (int t = 0; t < ntie; t++)
                         if (A->tbin[t] == b) q[i] += A->tc[t];
                 }
@@ -2369,6 +2431,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
         if (hk >= 0) {
             const unsigned long long *keys = c.R->picked(c.rr, hk);
             const int m = pk->cnt[hk];
+#pragma unroll 1
             for (int i = c.tid; i < m; i += NT) {
                 const unsigned long long key = keys[i];
                 const unsigned int eb = (unsigned int)(key >> 32);
@@ -2411,6 +2474,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
                 float s = s_bin;
                 long long pos = pos_bin;
                 int ev = EV_NONE, at = -1;
+#pragma unroll 1
                 for (int i = 0; i < nb; i++) {
                     s = __fadd_rn(s, pv);
                     pos++;
@@ -2450,7 +2514,7 @@ __device__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x_gt, long lon
 // A row that sorts nothing, once tile_walk has written the items of its probabilities: the walk to their
 // sum leaves the sum before every stretch, so the draw (sample.mojo:580-590) is a search among those and
 // then inside one stretch. Returns false where the general way has to be gone.
-__device__ bool tail_pure(CtxF &c, float u01, float Z) {
+__device__ __noinline__ bool tail_pure(CtxF &c, float u01, float Z) {
     const RowsArgs &R = *c.R;
     WalkShared *W = reinterpret_cast<WalkShared *>(c.A->tile);
     AuxF *A = c.A;
@@ -2472,6 +2536,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
     if (!A->b_event) return false;
     const float sum = A->b_s, target = __fmul_rn(u01, sum);
     // the first stretch (runs, then a careful chunk) behind which the sum exceeds the target
+#pragma unroll 1
     for (int q = c.tid; q <= (int)nrec; q += NT)
         if (target < __uint_as_float(W->sbs[q + 1])) { atomicMin(&A->evt_thread, q); break; }
     __syncthreads();
@@ -2487,6 +2552,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
     const unsigned int k0 = q > 0 ? W->rec[q - 1].k : 0u;
     int lo = 0, seen = 0;
     // (records are items in order: find the q-th one, counting as order() did)
+#pragma unroll 1
     for (int i0 = 0; i0 < nitem && seen < q; i0 += 32) {
         const int i = i0 + c.lane;
         bool care = false;
@@ -2497,12 +2563,17 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
         }
         const unsigned int m = __ballot_sync(0xffffffffu, care);
         const int n = __popc(m);
-        if (seen + n >= q) { lo = i0 + (int)__fns(m, 0, q - seen) + 1; seen = q; }
-        else seen += n;
+        if (seen + n >= q) {
+            unsigned int w = m;
+#pragma unroll 1
+            for (int k = seen + 1; k < q; k++) w &= w - 1u;
+            lo = i0 + __ffs((int)w); seen = q;
+        } else seen += n;
     }
     (void)k0;
     // item by item from there
     int tile = -1, at = 0;
+#pragma unroll 1
     for (int i = lo; i < nitem && tile < 0; i++) {
         const Item it = W->items[i];
         const int n = it.cnt(), off = it.off();
@@ -2514,6 +2585,7 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
             const int j = fexpo(s), per = (n + 31) >> 5, b0 = min(n, c.lane * per), b1 = min(n, b0 + per);
             const float Cm = __fmul_rn(1.5f, fpow2(j));
             unsigned int k = 0u;
+#pragma unroll 1
             for (int e = b0; e < b1; e++) k += __float_as_uint(__fadd_rn(v[e], Cm)) - __float_as_uint(Cm);
             const unsigned int inc = warp_incl_scan(k, c.lane);
             const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(sb + inc));
@@ -2521,11 +2593,13 @@ __device__ bool tail_pure(CtxF &c, float u01, float Z) {
             const unsigned int before = __shfl_sync(0xffffffffu, inc - k, l);
             s = __uint_as_float(sb + before);
             const int e0 = min(n, l * per), e1 = min(n, e0 + per);
+#pragma unroll 1
             for (int e = e0; e < e1 && tile < 0; e++) {
                 s = __fadd_rn(s, v[e]);
                 if (target < s) { tile = it.tile(); at = off + e; }
             }
         } else {
+#pragma unroll 1
             for (int e = 0; e < n && tile < 0; e++) {
                 s = __fadd_rn(s, v[e]);
                 if (target < s) { tile = it.tile(); at = off + e; }
@@ -2558,6 +2632,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
     const RowCfg &g = c.cfg;
     const int ntile = R.ntile, imax = c.pl.imax;
+#pragma unroll 1
     for (int t = c.tid; t < ntile; t += NT) {
         const TileOut o = R.to(rr)[t];
         A->tcnt[t] = o.cnt; A->tni[t] = o.nitem; A->tio[t] = o.ioff;
@@ -2568,6 +2643,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     if (nc_all > HEADCAP) {
         __syncthreads();
         if (!(c.pl.flags & F_LIST)) {
+#pragma unroll 1
             for (int t = 0; t < ntile; t += SPAN / TILE) tile_again(c, t, min(t + SPAN / TILE, ntile), nullptr, true);
             c.pl.flags |= F_LIST;
         }
@@ -2600,6 +2676,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         if (!(floor_p >= 2.2e-8f)) { c.status |= MOLLA_ROW_UNSUPPORTED; finish(); return; }
         if (!g.pure) {
             unsigned int lo_b = 0u, hi_b = 0x3F800000u;
+#pragma unroll 1
             for (int it = 0; it < 32 && lo_b < hi_b; it++) {
                 const unsigned int mid = lo_b + ((hi_b - lo_b) >> 1);
                 if (__fdiv_rn(__uint_as_float(mid), Z) >= floor_p) hi_b = mid; else lo_b = mid + 1u;
@@ -2613,6 +2690,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
                 });
             } else {
                 // the head holds the row's largest, more of them than top-k keeps: a floor below all of it changes nothing
+#pragma unroll 1
                 for (int i = c.tid; i < nc_all; i += NT) n += (unsigned int)(gcand[i] >> 32) >= e_floor ? 1 : 0;
             }
             (void)block_excl_scan<int>(n, A->wsi, &tot);
@@ -2625,10 +2703,12 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     if (g.pure) {
         // ---- nothing sorted: the draw walks the vocabulary in order (sample.mojo:365-369, 580-594):
         // probabilities p = e / Z (:437-438), what min-p drops becomes zero
+#pragma unroll 1
         for (int t = c.warp; t < ntile; t += NWARP) {
             const int n = A->tcnt[t];
             float *src = c.list + (size_t)t * TILE;
             float s = 0.0f;
+#pragma unroll 1
             for (int i = c.lane; i < n; i += 32) {
                 float p = src[i];
                 if (state != ST_PURE) {   // (else tile_walk has done it)
@@ -2653,9 +2733,11 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         }
         __syncthreads();
         float *list = A->tile + (size_t)c.warp * 32 * PITCH;
+#pragma unroll 1
         for (int t = c.warp; t < ntile; t += NWARP) {
             const int n = A->tcnt[t];
             const float *src = c.list + (size_t)t * TILE;
+#pragma unroll 1
             for (int i = c.lane; i < n; i += 32) list[skew(i)] = src[i];
             __syncwarp();
             const TileChunk ch = tile_chunk(list, n);
@@ -2702,6 +2784,22 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     long long head_pos;
     if (state == ST_HEAD) {   // row_head has sorted it and added it up
         head_s = head->head_s; head_pos = head->head_pos;
+        // what the walk will look up, all at once: its ties, the gathered bins, the first binade's table
+        static_assert(sizeof(A->u.h) >= NBINS * sizeof(unsigned long long), "a table takes the space of the walk's own histograms");
+        const uint4 *from = reinterpret_cast<const uint4 *>(R.ties(rr));
+        uint4 *to = reinterpret_cast<uint4 *>(A->ties);
+        for (int i = c.tid; i < (int)(sizeof(A->ties) / 16); i += NT) to[i] = from[i];
+        from = reinterpret_cast<const uint4 *>(R.picks(rr));
+        to = reinterpret_cast<uint4 *>(&A->picks);
+        if (c.tid < (int)(sizeof(WalkPicks) / 16)) to[c.tid] = from[c.tid];
+        from = reinterpret_cast<const uint4 *>(R.table(rr, 0));
+        to = reinterpret_cast<uint4 *>(&A->u.h);
+        uint4 x[NBINS / 2 / NT];
+#pragma unroll
+        for (int i = 0; i < NBINS / 2 / NT; i++) x[i] = from[c.tid + i * NT];
+#pragma unroll
+        for (int i = 0; i < NBINS / 2 / NT; i++) to[c.tid + i * NT] = x[i];
+#pragma unroll 1
         for (int i = c.tid; i < nc; i += NT) {
             const unsigned int p = (unsigned int)(gcand[i] >> 32);
             const bool eq = (i > 0 && (unsigned int)(gcand[i - 1] >> 32) == p) || (i + 1 < nc && (unsigned int)(gcand[i + 1] >> 32) == p);
@@ -2711,6 +2809,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         __syncthreads();
     } else {
     {
+#pragma unroll 1
         for (int i = c.tid; i < nc; i += NT) {
             const unsigned long long kk = gcand[i];
             A->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(kk), Z, yZ)) << 32) | (kk & 0xFFFFFFFFull);
@@ -2718,6 +2817,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     }
     FSTAMP(4);
     sort_head(c, nc);
+#pragma unroll 1
     for (int i = c.tid; i < nc; i += NT) {
         const float p = A->pc[i];
         const bool eq = (i > 0 && A->pc[i - 1] == p) || (i + 1 < nc && A->pc[i + 1] == p);
@@ -2726,6 +2826,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     __syncthreads();
 #ifdef MOLLA_SAMPLE_TESTING
     if (a.topk_out) {
+#pragma unroll 1
         for (int i = c.tid; i < a.topk_cap; i += NT)
             a.topk_out[(long long)c.r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? (int)(A->hidx[i] & 0x7fffffffu) : -1;
     }
@@ -2740,6 +2841,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         // the prefix sums of the sorted head (sample.mojo:497-506), eight at a time; at most n_use
         // elements are added
         const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
+#pragma unroll 1
         for (int i = 0; i < lim && cut < 0; i += 8) {
             const float4 *p4 = reinterpret_cast<const float4 *>(A->pc + i);
             const float4 x = p4[0], y = p4[1];
@@ -2815,7 +2917,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     // ---- past the head: the cut walk, then the draw walk, over the probabilities
     // (sample.mojo:437-438); what the head took is consumed
     const unsigned int tau_bits = head_overflow ? 0xffffffffu : c.pl.tau_bits;
-    c.tnb = 0; c.tj0 = 0; c.npick = state == ST_HEAD ? R.picks(rr)->n : 0;
+    c.tnb = 0; c.tj0 = 0; c.npick = state == ST_HEAD ? A->picks.n : 0; c.first_table = state == ST_HEAD;
     if (state == ST_HEAD && head_s > 0.0f && fexpo(head_s) >= -30 && fexpo(head_s) < 0) { c.tj0 = fexpo(head_s); c.tnb = min(WALK_BINADES, -c.tj0); }
     if (state != ST_HEAD) for_list4(c, [&](const unsigned int (&eb)[4], int, float *src) {
 #pragma unroll
@@ -2832,6 +2934,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     float cut_p = 0.0f, sum = 0.0f, target = 0.0f;
     bool settled = false;    // the token is known, or the row is degenerate
     bool resolved = false;
+#pragma unroll 1
     for (int leg = 0; leg < 2; leg++) {   // (one call site for both walks)
         w.s = head_s; w.pos = head_pos; w.tau = 0xFFFFFFFFu;
         w.event = EV_NONE; w.idx = -1; w.p = 0; w.tie = 0;
@@ -2859,6 +2962,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         __syncthreads();
         if (c.tid == 0) A->evt_thread = 0x7fffffff;
         __syncthreads();
+#pragma unroll 1
         for (int i = c.tid; i < nc; i += NT)
             if (target < A->pre[i]) { atomicMin(&A->evt_thread, i); break; }
         __syncthreads();
@@ -2903,6 +3007,7 @@ __global__ void __launch_bounds__(NT, 1) row_tail_kernel(const __grid_constant__
     pdl_next();
     pdl_wait();
     const int n = R.queue[0];
+#pragma unroll 1
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
         tail_row(R, R.queue[1 + q]);
         __syncthreads();
