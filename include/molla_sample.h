@@ -265,8 +265,8 @@ int32_t molla_sample_batch_noalloc(
  * before returning. Settings are validated on the host first with the rules and
  * messages of `SamplerConfig.check` (sample.mojo:140-154) and `Sampler.bias`
  * (:225-232): MOLLA_ERR_CONFIG, nothing launched. `temperature` is required;
- * the other per-row arrays may be NULL as above. A block of 32 MB and more goes up in
- * eight pieces on a copy stream the library makes for itself (one per device and
+ * the other per-row arrays may be NULL as above. A block of 6 MB and more goes up in
+ * pieces on a copy stream the library makes for itself (one per device and
  * calling thread, on first use) while the pieces that have arrived are sampled on
  * `stream`; a row the library did not answer fails the call (MOLLA_ERR_DEVICE).
  */
@@ -281,6 +281,24 @@ int32_t molla_sample_batch_host(
     const int32_t *bias_off, int32_t top_n, void *d_workspace, int64_t workspace_bytes,
     void *stream, int32_t *h_tokens, float *h_chosen_logprob, int32_t *h_top_ids,
     float *h_top_logprobs, uint32_t *h_row_status);
+
+/*
+ * The per-row loop of the decode step (batch.mojo:509-511) for a caller that keeps its samplers on the
+ * host and its logits on the device: batch row r samples logit row rows[r] (NULL = r) of the block, the
+ * settings and windows come from host arrays (as in molla_sample_batch_host) and the tokens and status words go back to host arrays. Blocks until they are there. The settings travel as
+ * one copy through pinned memory of the library's own (per device and calling thread, at most 8 MB, given
+ * back when the thread ends). Rows report for themselves in their status words: a row whose settings are
+ * refused, or without an answer, does not fail the call.
+ */
+int64_t molla_sample_pick_workspace_bytes(int32_t B, int32_t V, int64_t n_hist, int64_t n_bias);
+int32_t molla_sample_pick_rows(
+    const float *d_logits, int64_t row_stride, int32_t n_logit_rows, int32_t V, const int32_t *rows, int32_t B,
+    const float *temperature, const int32_t *top_k, const float *top_p, const float *min_p,
+    const float *typical_p, const float *repeat_penalty, const float *frequency_penalty,
+    const float *presence_penalty, const uint8_t *window_on, const uint64_t *seed, const uint64_t *drawn,
+    const int64_t *hist, const int32_t *hist_off, const int64_t *bias_ids, const float *bias_vals,
+    const int32_t *bias_off, void *d_workspace, int64_t workspace_bytes, void *stream, int32_t *tokens,
+    uint32_t *row_status);
 
 /* The rows after logit bias and penalties, before temperature: what
  * `_bias` and `_penalise` (sample.mojo:381-417) leave in `vals`. Same arguments

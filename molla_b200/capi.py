@@ -36,7 +36,7 @@ EXPORTS = (
     "molla_sample_workspace_bytes", "molla_sample_batch", "molla_sample_batch_masked", "molla_sample_host_workspace_bytes",
     "molla_sample_batch_host", "molla_sample_batch_noalloc", "molla_sample_shard_summary_words",
     "molla_sample_shard_stage_a", "molla_sample_shard_merge", "molla_sample_shard_stage_b", "molla_sample_shard_stage_c", "molla_sample_penalised",
-    "molla_sample_decode_step", "molla_sample_logprobs", "molla_sample_expf", "molla_sample_logf", "molla_sample_sync",
+    "molla_sample_pick_workspace_bytes", "molla_sample_pick_rows", "molla_sample_decode_step", "molla_sample_logprobs", "molla_sample_expf", "molla_sample_logf", "molla_sample_sync",
     "molla_sample_nccl_unique_id", "molla_sample_nccl_comm_create", "molla_sample_nccl_comm_destroy",
     "molla_sample_sharded_last_error", "molla_sample_sharded_workspace_bytes", "molla_sample_sharded_step",
 )
@@ -107,6 +107,10 @@ def _load(path, testing):
     L.molla_sample_host_workspace_bytes.argtypes = [i32, i32, i64, i64, i32]
     L.molla_sample_batch_host.restype = i32
     L.molla_sample_batch_host.argtypes = [vp, i64, i32, i32] + [vp] * 16 + [i32, vp, i64, vp] + [vp] * 5
+    L.molla_sample_pick_workspace_bytes.restype = i64
+    L.molla_sample_pick_workspace_bytes.argtypes = [i32, i32, i64, i64]
+    L.molla_sample_pick_rows.restype = i32
+    L.molla_sample_pick_rows.argtypes = [vp, i64, i32, i32, vp, i32] + [vp] * 17 + [i64] + [vp] * 3
     L.molla_sample_batch_noalloc.restype = i32
     L.molla_sample_batch_noalloc.argtypes = [vp, i64, i32, i32] + [vp] * 16 + [i32, vp] + [vp] * 5
     L.molla_sample_shard_summary_words.restype = i32

@@ -3097,7 +3097,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     A.a.Vg = a.V; A.a.col0 = 0; A.a.mode = 0;
     A.ntile = (a.V + TILE - 1) / TILE;
     A.nspan = (a.V + SPAN - 1) / SPAN;
-    narrow_layout(a.V, a.B, sms, A.oG, A.oVc, A.oL);
+    narrow_layout(a.V, a.layout_B > 0 ? a.layout_B : a.B, sms, A.oG, A.oVc, A.oL);
     const int rows = rows_in_flight(a.B, a.V);
     lay_out(A, (char *)d_workspace, rows, a.V);
     for (A.r0 = 0; A.r0 < a.B && e == cudaSuccess; A.r0 += rows) {

@@ -2328,42 +2328,68 @@ int32_t molla_sample_shard_stage_c(int32_t B, int32_t V_global, const float *d_t
 // ---- host-buffer form ---------------------------------------------------------
 namespace {
 constexpr int CL_MAX_DEVICES_HOST = 64;
-// The library's own copy stream and events for the host-buffer form, one set per device and per
-// calling thread (calls from different threads never share them).
+// The library's own copy stream and events for the host-buffer form, and pinned memory in which a call's
+// small arrays travel as one: one set per device and per calling thread (calls from different threads
+// never share them, and every call that uses one waits for its end), given back when the thread ends.
+constexpr size_t LANE_PIN_MOST = (size_t)8 << 20;
 struct CopyLane {
+    int dev = -1;
     cudaStream_t stream = nullptr;
     cudaEvent_t ready = nullptr;
     cudaEvent_t arrived[8] = {};
-    bool ok = false;
+    unsigned char *pin = nullptr;
+    size_t pin_bytes = 0;
+    bool tried = false, ok = false;
+    bool streams() {
+        if (!tried) {
+            tried = true;
+            ok = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess;
+            ok = ok && cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) == cudaSuccess;
+            for (int i = 0; i < 8 && ok; i++) ok = cudaEventCreateWithFlags(&arrived[i], cudaEventDisableTiming) == cudaSuccess;
+            if (!ok) (void)cudaGetLastError();
+        }
+        return ok;
+    }
+    unsigned char *pinned(size_t n) {
+        if (n > LANE_PIN_MOST) return nullptr;
+        if (n > pin_bytes) {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr;
+            pin_bytes = 0;
+            size_t want = 64 << 10;
+            while (want < n) want <<= 1;
+            if (cudaHostAlloc((void **)&pin, want, cudaHostAllocDefault) != cudaSuccess) { (void)cudaGetLastError(); pin = nullptr; return nullptr; }
+            pin_bytes = want;
+        }
+        return pin;
+    }
+    ~CopyLane() {   // (at the process's end the driver may be gone: nothing is left to do then)
+        if (pin) cudaFreeHost(pin);
+        if (ready) cudaEventDestroy(ready);
+        for (cudaEvent_t e : arrived) if (e) cudaEventDestroy(e);
+        if (stream) cudaStreamDestroy(stream);
+    }
 };
 CopyLane *copy_lane() {
     static thread_local CopyLane lanes[CL_MAX_DEVICES_HOST];
-    static thread_local bool tried[CL_MAX_DEVICES_HOST] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= CL_MAX_DEVICES_HOST) return nullptr;
-    CopyLane &l = lanes[dev];
-    if (!tried[dev]) {
-        tried[dev] = true;
-        bool ok = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) == cudaSuccess;
-        ok = ok && cudaEventCreateWithFlags(&l.ready, cudaEventDisableTiming) == cudaSuccess;
-        for (int i = 0; i < 8 && ok; i++) ok = cudaEventCreateWithFlags(&l.arrived[i], cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) (void)cudaGetLastError();
-        l.ok = ok;
-    }
-    return l.ok ? &l : nullptr;
+    lanes[dev].dev = dev;
+    return &lanes[dev];
 }
 inline size_t al256(size_t n) { return (n + 255) & ~(size_t)255; }
 struct HostLayout {
-    size_t logits, f[8], win, seed, drawn, k, hist, hist_off, bias_ids, bias_vals, bias_off;
+    size_t logits, f[8], win, seed, drawn, k, rows, hist, hist_off, bias_ids, bias_vals, bias_off;
     size_t tokens, status, chosen, top_ids, top_lps, total, inner;
 };
-HostLayout host_layout(int B, int V, long long n_hist, long long n_bias, int top_n, int sms) {
+HostLayout host_layout(int B, int V, long long n_hist, long long n_bias, int top_n, int sms, bool with_logits = true) {
     HostLayout L;
     size_t o = al256(batch_workspace_bytes(B, V, sms));  // the batched call's own workspace comes first
     L.inner = o;
-    L.logits = o; o += al256((size_t)B * V * 4);
+    L.logits = o; o += with_logits ? al256((size_t)B * V * 4) : 0;
     for (int i = 0; i < 8; i++) { L.f[i] = o; o += al256((size_t)B * 4); }
     L.k = o; o += al256((size_t)B * 4);
+    L.rows = o; o += al256((size_t)B * 4);
     L.win = o; o += al256((size_t)B);
     L.seed = o; o += al256((size_t)B * 8);
     L.drawn = o; o += al256((size_t)B * 8);
@@ -2379,6 +2405,79 @@ HostLayout host_layout(int B, int V, long long n_hist, long long n_bias, int top
     L.top_lps = o; o += al256((size_t)B * (top_n > 0 ? top_n : 1) * 4);
     L.total = o;
     return L;
+}
+// A batch's settings in host memory.
+struct HostParams {
+    const float *temperature; const int32_t *top_k; const float *top_p, *min_p, *typical_p, *repeat_penalty, *frequency_penalty, *presence_penalty;
+    const uint8_t *window_on; const uint64_t *seed, *drawn; const int64_t *hist; const int32_t *hist_off;
+    const int64_t *bias_ids; const float *bias_vals; const int32_t *bias_off;
+};
+// SamplerConfig.check (sample.mojo:140-154) and Sampler.bias (:225-232), before anything is launched
+// (`values` = false leaves the settings to the rows' own status words)
+int check_params(const HostParams &h, int B, int V, bool values) {
+    for (int r = 0; values && r < B; r++) {
+        if (!(h.temperature[r] >= 0)) return fail(MOLLA_ERR_CONFIG, "a temperature cannot be negative%s");
+        if (h.top_k && h.top_k[r] < 0) return fail(MOLLA_ERR_CONFIG, "a top-k cannot be negative%s");
+        if (h.top_p && !(h.top_p[r] > 0 && h.top_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a top-p has to be above zero and at most one%s");
+        if (h.min_p && !(h.min_p[r] >= 0 && h.min_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a min-p has to be between zero and one%s");
+        if (h.typical_p && !(h.typical_p[r] > 0 && h.typical_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a typical-p has to be above zero and at most one%s");
+        if (h.repeat_penalty && !(h.repeat_penalty[r] > 0)) return fail(MOLLA_ERR_CONFIG, "a repetition penalty of zero or less erases a logit%s");
+    }
+    // the ragged windows and bias lists: offsets that start at zero and never go back
+    for (int pass = 0; pass < 2; pass++) {
+        const int32_t *off = pass ? h.bias_off : h.hist_off;
+        if (!off) continue;
+        if (off[0] != 0) return fail(MOLLA_ERR_ARGUMENT, "an offset array has to start at zero%s");
+        for (int r = 0; r < B; r++)
+            if (off[r + 1] < off[r]) return fail(MOLLA_ERR_ARGUMENT, "an offset array has to be non-decreasing%s");
+    }
+    const long long n_bias = values && h.bias_off ? h.bias_off[B] : 0;
+    for (long long j = 0; j < n_bias; j++)
+        if (h.bias_ids[j] < 0 || h.bias_ids[j] >= V) return fail(MOLLA_ERR_CONFIG, "a logit bias names a token outside the vocabulary%s");
+    return MOLLA_OK;
+}
+// The settings (and `rows`) to the device on `st`: gathered in the lane's pinned memory and sent as one
+// copy (seventeen small ones took 35 us of the calling thread and as much of the copy engine); one copy
+// per array where that memory cannot be had or would be too large.
+cudaError_t upload_params(CopyLane *lane, const HostParams &h, int B, long long n_hist, long long n_bias, const int32_t *rows,
+                          const HostLayout &L, char *w, cudaStream_t st) {
+    const size_t base = L.f[0], bytes = L.tokens - base;
+    unsigned char *pin = lane ? lane->pinned(al256(bytes) + (size_t)B * 8) : nullptr;
+    cudaError_t e = cudaSuccess;
+    size_t end = base;
+    auto put = [&](size_t off, const void *src, size_t n) {
+        if (!src || !n || e != cudaSuccess) return;
+        if (pin) { memcpy(pin + (off - base), src, n); if (off + n > end) end = off + n; }
+        else e = cudaMemcpyAsync(w + off, src, n, cudaMemcpyHostToDevice, st);
+    };
+    const float *f[7] = {h.temperature, h.top_p, h.min_p, h.typical_p, h.repeat_penalty, h.frequency_penalty, h.presence_penalty};
+    for (int i = 0; i < 7; i++) put(L.f[i], f[i], (size_t)B * 4);
+    put(L.k, h.top_k, (size_t)B * 4); put(L.rows, rows, (size_t)B * 4); put(L.win, h.window_on, (size_t)B);
+    put(L.seed, h.seed, (size_t)B * 8); put(L.drawn, h.drawn, (size_t)B * 8);
+    put(L.hist, h.hist, (size_t)n_hist * 8); put(L.hist_off, h.hist_off, (size_t)(B + 1) * 4);
+    put(L.bias_ids, h.bias_ids, (size_t)n_bias * 8); put(L.bias_vals, h.bias_vals, (size_t)n_bias * 4); put(L.bias_off, h.bias_off, (size_t)(B + 1) * 4);
+    if (pin && end > base) e = cudaMemcpyAsync(w + base, pin, end - base, cudaMemcpyHostToDevice, st);
+    return e;
+}
+// Rows [r0, r1) of the uploaded settings as the kernels take them: per-row arrays advance by r0 elements
+// (the window and bias offsets are absolute, so their arrays only shift).
+BatchArgs device_params(const HostParams &h, const HostLayout &L, char *w, int r0, int r1) {
+    auto dp = [&](size_t off, const void *src, size_t elem, int r) -> char * { return src ? w + off + elem * (size_t)r : nullptr; };
+    BatchArgs a;
+    memset(&a, 0, sizeof(a));
+    a.B = r1 - r0;
+    a.temperature = (const float *)dp(L.f[0], h.temperature, 4, r0); a.top_p = (const float *)dp(L.f[1], h.top_p, 4, r0);
+    a.min_p = (const float *)dp(L.f[2], h.min_p, 4, r0); a.typical_p = (const float *)dp(L.f[3], h.typical_p, 4, r0);
+    a.repeat_penalty = (const float *)dp(L.f[4], h.repeat_penalty, 4, r0); a.frequency_penalty = (const float *)dp(L.f[5], h.frequency_penalty, 4, r0);
+    a.presence_penalty = (const float *)dp(L.f[6], h.presence_penalty, 4, r0);
+    a.top_k = (const int *)dp(L.k, h.top_k, 4, r0); a.window_on = (const unsigned char *)dp(L.win, h.window_on, 1, r0);
+    a.seed = (const unsigned long long *)dp(L.seed, h.seed, 8, r0); a.drawn = (const unsigned long long *)dp(L.drawn, h.drawn, 8, r0);
+    a.hist = (const long long *)dp(L.hist, h.hist, 8, 0); a.hist_off = (const int *)dp(L.hist_off, h.hist_off, 4, r0);
+    a.bias_ids = (const long long *)dp(L.bias_ids, h.bias_ids, 8, 0); a.bias_vals = (const float *)dp(L.bias_vals, h.bias_vals, 4, 0);
+    a.bias_off = (const int *)dp(L.bias_off, h.bias_off, 4, r0);
+    a.tokens = (int *)(w + L.tokens) + r0; a.row_status = (unsigned int *)(w + L.status) + r0;
+    MOLLA_SET_TESTING_ARGS(a);
+    return a;
 }
 }  // namespace
 
@@ -2407,98 +2506,90 @@ int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32
     if ((hist == nullptr) != (hist_off == nullptr)) return fail(MOLLA_ERR_ARGUMENT, "history ids and offsets go together%s");
     if ((bias_ids == nullptr) != (bias_off == nullptr) || (bias_ids && !bias_vals)) return fail(MOLLA_ERR_ARGUMENT, "bias ids, values and offsets go together%s");
     if (B == 0) return MOLLA_OK;
-    // SamplerConfig.check (sample.mojo:140-154) and Sampler.bias (:225-232), before anything is launched
-    for (int r = 0; r < B; r++) {
-        if (!(temperature[r] >= 0)) return fail(MOLLA_ERR_CONFIG, "a temperature cannot be negative%s");
-        if (top_k && top_k[r] < 0) return fail(MOLLA_ERR_CONFIG, "a top-k cannot be negative%s");
-        if (top_p && !(top_p[r] > 0 && top_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a top-p has to be above zero and at most one%s");
-        if (min_p && !(min_p[r] >= 0 && min_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a min-p has to be between zero and one%s");
-        if (typical_p && !(typical_p[r] > 0 && typical_p[r] <= 1)) return fail(MOLLA_ERR_CONFIG, "a typical-p has to be above zero and at most one%s");
-        if (repeat_penalty && !(repeat_penalty[r] > 0)) return fail(MOLLA_ERR_CONFIG, "a repetition penalty of zero or less erases a logit%s");
-    }
-    // the ragged windows and bias lists: offsets that start at zero and never go back
-    for (int pass = 0; pass < 2; pass++) {
-        const int32_t *off = pass ? bias_off : hist_off;
-        if (!off) continue;
-        if (off[0] != 0) return fail(MOLLA_ERR_ARGUMENT, "an offset array has to start at zero%s");
-        for (int r = 0; r < B; r++)
-            if (off[r + 1] < off[r]) return fail(MOLLA_ERR_ARGUMENT, "an offset array has to be non-decreasing%s");
-    }
+    const HostParams h = {temperature, top_k, top_p, min_p, typical_p, repeat_penalty, frequency_penalty, presence_penalty, window_on,
+                          seed, drawn, hist, hist_off, bias_ids, bias_vals, bias_off};
+    int rc = check_params(h, B, V, true);
+    if (rc != MOLLA_OK) return rc;
     const long long n_hist = hist_off ? hist_off[B] : 0, n_bias = bias_off ? bias_off[B] : 0;
-    for (long long j = 0; j < n_bias; j++)
-        if (bias_ids[j] < 0 || bias_ids[j] >= V) return fail(MOLLA_ERR_CONFIG, "a logit bias names a token outside the vocabulary%s");
     const int sms = sm_count();
     if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
     const HostLayout L = host_layout(B, V, n_hist, n_bias, top_n, sms);
     if (!d_workspace || workspace_bytes < (int64_t)L.total) return fail(MOLLA_ERR_WORKSPACE, "workspace missing or too small%s");
     char *w = (char *)d_workspace;
     cudaStream_t st = (cudaStream_t)stream;
-    // A large block goes up in pieces on a stream of the library's own (one per device, made on first
-    // use) while the pieces that have arrived are sampled on the caller's stream; a small one in one go.
+    CopyLane *lane = copy_lane();
+    // A large block goes up in pieces on a stream of the library's own while the pieces that have arrived
+    // are sampled on the caller's stream. At the 55 GB/s of the link a piece of 3 MB takes the 55 us that a
+    // few rows take to be sampled: smaller ones would wait for the kernels, larger ones leave more of them
+    // behind the last copy (16 MB in one piece: 450 us, in pieces: 350).
     constexpr int MAXPIECE = 8;
-    int npiece = 1;
-    if ((size_t)B * V * 4 >= ((size_t)32 << 20) && B >= 2 * MAXPIECE) npiece = MAXPIECE;
-    CopyLane *lane = npiece > 1 ? copy_lane() : nullptr;
-    if (!lane) npiece = 1;
+    const size_t block = (size_t)B * V * 4;
+    int npiece = (int)(block / ((size_t)3 << 20) < MAXPIECE ? block / ((size_t)3 << 20) : MAXPIECE);
+    if (npiece > B) npiece = B;
+    if (npiece < 2 || !lane || !lane->streams()) npiece = 1;
     cudaError_t e = cudaSuccess;
-    if (npiece == 1)
-        e = cudaMemcpy2DAsync(w + L.logits, (size_t)V * 4, h_logits, (size_t)row_stride * 4, (size_t)V * 4, (size_t)B, cudaMemcpyHostToDevice, st);
-    const float *fsrc[8] = {temperature, top_p, min_p, typical_p, repeat_penalty, frequency_penalty, presence_penalty, nullptr};
-    for (int i = 0; i < 7 && e == cudaSuccess; i++)
-        if (fsrc[i]) e = cudaMemcpyAsync(w + L.f[i], fsrc[i], (size_t)B * 4, cudaMemcpyHostToDevice, st);
-    auto up = [&](size_t off, const void *src, size_t bytes) { if (src && bytes && e == cudaSuccess) e = cudaMemcpyAsync(w + off, src, bytes, cudaMemcpyHostToDevice, st); };
-    up(L.k, top_k, (size_t)B * 4); up(L.win, window_on, (size_t)B); up(L.seed, seed, (size_t)B * 8); up(L.drawn, drawn, (size_t)B * 8);
-    up(L.hist, hist, (size_t)n_hist * 8); up(L.hist_off, hist_off, (size_t)(B + 1) * 4);
-    up(L.bias_ids, bias_ids, (size_t)n_bias * 8); up(L.bias_vals, bias_vals, (size_t)n_bias * 4); up(L.bias_off, bias_off, (size_t)(B + 1) * 4);
-    if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(e));
-    // rows [r0, r1) of the block on the device: per-row arrays advance by r0 elements (the window and
-    // bias offsets are absolute, so their arrays only shift)
-    auto dp = [&](size_t off, const void *src, size_t elem, int r0) -> void * { return src ? (void *)(w + off + elem * (size_t)r0) : nullptr; };
-    auto sample_rows = [&](int r0, int r1) -> int {
-        return molla_sample_batch(
-            (const float *)(w + L.logits) + (size_t)r0 * V, V, r1 - r0, V, (const float *)dp(L.f[0], temperature, 4, r0),
-            (const int32_t *)dp(L.k, top_k, 4, r0), (const float *)dp(L.f[1], top_p, 4, r0), (const float *)dp(L.f[2], min_p, 4, r0),
-            (const float *)dp(L.f[3], typical_p, 4, r0), (const float *)dp(L.f[4], repeat_penalty, 4, r0),
-            (const float *)dp(L.f[5], frequency_penalty, 4, r0), (const float *)dp(L.f[6], presence_penalty, 4, r0),
-            (const uint8_t *)dp(L.win, window_on, 1, r0), (const uint64_t *)dp(L.seed, seed, 8, r0),
-            (const uint64_t *)dp(L.drawn, drawn, 8, r0), (const int64_t *)dp(L.hist, hist, 8, 0),
-            (const int32_t *)dp(L.hist_off, hist_off, 4, r0), (const int64_t *)dp(L.bias_ids, bias_ids, 8, 0),
-            (const float *)dp(L.bias_vals, bias_vals, 4, 0), (const int32_t *)dp(L.bias_off, bias_off, 4, r0), top_n, w,
-            (int64_t)L.inner, stream, (int32_t *)(w + L.tokens) + r0, h_chosen_logprob ? (float *)(w + L.chosen) + r0 : nullptr,
-            top_n > 0 ? (int32_t *)(w + L.top_ids) + (size_t)r0 * top_n : nullptr,
-            top_n > 0 ? (float *)(w + L.top_lps) + (size_t)r0 * top_n : nullptr, (uint32_t *)(w + L.status) + r0, nullptr);
-    };
-    int rc = MOLLA_OK;
-    if (npiece == 1) {
-        rc = sample_rows(0, B);
-    } else {
+    if (npiece > 1) {
         // the copies start once everything queued on the caller's stream so far is done (the workspace may still be in use)
         e = cudaEventRecord(lane->ready, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(lane->stream, lane->ready, 0);
-        for (int c = 0; c < npiece && e == cudaSuccess; c++) {
-            const int r0 = (int)((long long)B * c / npiece), r1 = (int)((long long)B * (c + 1) / npiece);
-            e = cudaMemcpy2DAsync(w + L.logits + (size_t)r0 * V * 4, (size_t)V * 4, h_logits + (size_t)r0 * row_stride,
-                                  (size_t)row_stride * 4, (size_t)V * 4, (size_t)(r1 - r0), cudaMemcpyHostToDevice, lane->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(lane->arrived[c], lane->stream);
-        }
-        if (e != cudaSuccess) { cudaStreamSynchronize(lane->stream); return fail(MOLLA_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(e)); }
-        for (int c = 0; c < npiece && rc == MOLLA_OK; c++) {
-            const int r0 = (int)((long long)B * c / npiece), r1 = (int)((long long)B * (c + 1) / npiece);
+    }
+    auto copy_rows = [&](int r0, int r1, cudaStream_t on) -> cudaError_t {
+        if (row_stride == V) return cudaMemcpyAsync(w + L.logits + (size_t)r0 * V * 4, h_logits + (size_t)r0 * V, (size_t)(r1 - r0) * V * 4, cudaMemcpyHostToDevice, on);
+        return cudaMemcpy2DAsync(w + L.logits + (size_t)r0 * V * 4, (size_t)V * 4, h_logits + (size_t)r0 * row_stride,
+                                 (size_t)row_stride * 4, (size_t)V * 4, (size_t)(r1 - r0), cudaMemcpyHostToDevice, on);
+    };
+    if (e == cudaSuccess) e = upload_params(lane, h, B, n_hist, n_bias, nullptr, L, w, st);
+    for (int c = 0; c < npiece && e == cudaSuccess; c++) {
+        const int r0 = (int)((long long)B * c / npiece), r1 = (int)((long long)B * (c + 1) / npiece);
+        e = copy_rows(r0, r1, npiece > 1 ? lane->stream : st);
+        if (e == cudaSuccess && npiece > 1) e = cudaEventRecord(lane->arrived[c], lane->stream);
+    }
+    if (e != cudaSuccess) {
+        if (npiece > 1) cudaStreamSynchronize(lane->stream);
+        cudaStreamSynchronize(st);
+        return fail(MOLLA_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(e));
+    }
+    const int layout_B = (block >= ((size_t)32 << 20) && B >= 16) ? (B + 7) / 8 : B;
+    for (int c = 0; c < npiece && rc == MOLLA_OK; c++) {
+        const int r0 = (int)((long long)B * c / npiece), r1 = (int)((long long)B * (c + 1) / npiece);
+        if (npiece > 1) {
             e = cudaStreamWaitEvent(st, lane->arrived[c], 0);
             if (e != cudaSuccess) { rc = fail(MOLLA_ERR_CUDA, "waiting for a piece of the block failed: %s", cudaGetErrorString(e)); break; }
-            rc = sample_rows(r0, r1);
         }
-        if (rc != MOLLA_OK) cudaStreamSynchronize(lane->stream);  // no copy of this call outlives it
+        BatchArgs a = device_params(h, L, w, r0, r1);
+        a.logits = (const float *)(w + L.logits) + (size_t)r0 * V; a.row_stride = V; a.V = V; a.layout_B = layout_B;
+        rc = launch_sampling(a, w, st);
+        if (rc == MOLLA_OK)
+            rc = launch_logprobs(a.logits, V, a.B, V, a.tokens, top_n, h_chosen_logprob ? (float *)(w + L.chosen) + r0 : nullptr,
+                                 top_n > 0 ? (int32_t *)(w + L.top_ids) + (size_t)r0 * top_n : nullptr,
+                                 top_n > 0 ? (float *)(w + L.top_lps) + (size_t)r0 * top_n : nullptr, nullptr, 0, 0.0f, w, st);
     }
-    if (rc != MOLLA_OK) return rc;
-    e = cudaMemcpyAsync(h_tokens, w + L.tokens, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_row_status, w + L.status, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && h_chosen_logprob) e = cudaMemcpyAsync(h_chosen_logprob, w + L.chosen, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && top_n > 0) {
-        e = cudaMemcpyAsync(h_top_ids, w + L.top_ids, (size_t)B * top_n * 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h_top_logprobs, w + L.top_lps, (size_t)B * top_n * 4, cudaMemcpyDeviceToHost, st);
+    if (rc != MOLLA_OK) {  // no copy of this call outlives it
+        if (npiece > 1) cudaStreamSynchronize(lane->stream);
+        cudaStreamSynchronize(st);
+        return rc;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    // the results lie together: one copy, through the pinned memory (the parameters in it are long on the device)
+    const size_t rbytes = L.total - L.tokens;
+    unsigned char *pin = lane ? lane->pinned(rbytes) : nullptr;
+    if (pin && pin == lane->pin && rbytes <= ((size_t)256 << 10)) {
+        e = cudaMemcpyAsync(pin, w + L.tokens, rbytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) {
+            auto down = [&](void *dst, size_t off, size_t n) { if (dst && n) memcpy(dst, pin + (off - L.tokens), n); };
+            down(h_tokens, L.tokens, (size_t)B * 4); down(h_row_status, L.status, (size_t)B * 4); down(h_chosen_logprob, L.chosen, (size_t)B * 4);
+            if (top_n > 0) { down(h_top_ids, L.top_ids, (size_t)B * top_n * 4); down(h_top_logprobs, L.top_lps, (size_t)B * top_n * 4); }
+        }
+    } else {
+        e = cudaMemcpyAsync(h_tokens, w + L.tokens, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_row_status, w + L.status, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && h_chosen_logprob) e = cudaMemcpyAsync(h_chosen_logprob, w + L.chosen, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && top_n > 0) {
+            e = cudaMemcpyAsync(h_top_ids, w + L.top_ids, (size_t)B * top_n * 4, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(h_top_logprobs, w + L.top_lps, (size_t)B * top_n * 4, cudaMemcpyDeviceToHost, st);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    }
     if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "device to host copy failed: %s", cudaGetErrorString(e));
     // a row the library did not answer (token -1) fails the call, as `pick` would have raised
     for (int r = 0; r < B; r++) {
@@ -2507,6 +2598,61 @@ int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32
         if (h_row_status[r] & (MOLLA_ROW_LOAD_TIMEOUT | MOLLA_ROW_DEGENERATE | MOLLA_ROW_INVALID_CONFIG | MOLLA_ROW_SHARD_OVERFLOW | MOLLA_ROW_EMPTY))
             return fail(MOLLA_ERR_DEVICE, "a row reported an error in its status word%s");
     }
+    return MOLLA_OK;
+}
+
+int64_t molla_sample_pick_workspace_bytes(int32_t B, int32_t V, int64_t n_hist, int64_t n_bias) {
+    if (B < 0 || V <= 0 || n_hist < 0 || n_bias < 0) return fail(MOLLA_ERR_ARGUMENT, "bad shape for the workspace query%s");
+    const int sms = sm_count();
+    if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
+    return (int64_t)host_layout(B, V, n_hist, n_bias, 0, sms, false).total;
+}
+
+int32_t molla_sample_pick_rows(const float *d_logits, int64_t row_stride, int32_t n_logit_rows, int32_t V, const int32_t *rows, int32_t B,
+                               const float *temperature, const int32_t *top_k, const float *top_p, const float *min_p,
+                               const float *typical_p, const float *repeat_penalty, const float *frequency_penalty,
+                               const float *presence_penalty, const uint8_t *window_on, const uint64_t *seed, const uint64_t *drawn,
+                               const int64_t *hist, const int32_t *hist_off, const int64_t *bias_ids, const float *bias_vals,
+                               const int32_t *bias_off, void *d_workspace, int64_t workspace_bytes, void *stream, int32_t *tokens,
+                               uint32_t *row_status) {
+    g_err[0] = 0;
+    if (!d_logits || !tokens || !row_status || !temperature) return fail(MOLLA_ERR_ARGUMENT, "logits, temperature, tokens and row status are required%s");
+    if (B < 0 || V <= 0 || row_stride < V || n_logit_rows < 0 || (!rows && B > n_logit_rows)) return fail(MOLLA_ERR_ARGUMENT, "bad block shape%s");
+    if ((hist == nullptr) != (hist_off == nullptr)) return fail(MOLLA_ERR_ARGUMENT, "history ids and offsets go together%s");
+    if ((bias_ids == nullptr) != (bias_off == nullptr) || (bias_ids && !bias_vals)) return fail(MOLLA_ERR_ARGUMENT, "bias ids, values and offsets go together%s");
+    if (B == 0) return MOLLA_OK;
+    for (int r = 0; rows && r < B; r++)
+        if (rows[r] < 0 || rows[r] >= n_logit_rows) return fail(MOLLA_ERR_ARGUMENT, "a row outside the block%s");
+    const HostParams h = {temperature, top_k, top_p, min_p, typical_p, repeat_penalty, frequency_penalty, presence_penalty, window_on,
+                          seed, drawn, hist, hist_off, bias_ids, bias_vals, bias_off};
+    int rc = check_params(h, B, V, false);
+    if (rc != MOLLA_OK) return rc;
+    const long long n_hist = hist_off ? hist_off[B] : 0, n_bias = bias_off ? bias_off[B] : 0;
+    const int sms = sm_count();
+    if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
+    const HostLayout L = host_layout(B, V, n_hist, n_bias, 0, sms, false);
+    if (!d_workspace || workspace_bytes < (int64_t)L.total) return fail(MOLLA_ERR_WORKSPACE, "workspace missing or too small%s");
+    char *w = (char *)d_workspace;
+    cudaStream_t st = (cudaStream_t)stream;
+    CopyLane *lane = copy_lane();
+    cudaError_t e = upload_params(lane, h, B, n_hist, n_bias, rows, L, w, st);
+    if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "host to device copy failed: %s", cudaGetErrorString(e));
+    BatchArgs a = device_params(h, L, w, 0, B);
+    a.logits = d_logits; a.row_stride = row_stride; a.V = V; a.layout_B = B;
+    if (rows) { a.rows = (const int *)(w + L.rows); a.n_logit_rows = n_logit_rows; }
+    // the answers straight into pinned host memory, behind the parameters there: eight bytes a row
+    const size_t behind = al256(L.tokens - L.f[0]);
+    unsigned char *pin = lane && lane->pin && lane->pin_bytes >= behind + (size_t)B * 8 ? lane->pin + behind : nullptr;
+    if (pin) { a.tokens = (int *)pin; a.row_status = (unsigned int *)(pin + (size_t)B * 4); }
+    rc = launch_sampling(a, w, st);
+    if (rc != MOLLA_OK) { cudaStreamSynchronize(st); return rc; }  // (the pinned memory is still being read)
+    if (!pin) {
+        e = cudaMemcpyAsync(tokens, w + L.tokens, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(row_status, w + L.status, (size_t)B * 4, cudaMemcpyDeviceToHost, st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(MOLLA_ERR_CUDA, "sampling failed: %s", cudaGetErrorString(e));
+    if (pin) { memcpy(tokens, pin, (size_t)B * 4); memcpy(row_status, pin + (size_t)B * 4, (size_t)B * 4); }
     return MOLLA_OK;
 }
 

@@ -12,7 +12,8 @@ PyTorch is used for device memory and streams only.
 """
 from __future__ import annotations
 
-import ctypes as C
+import threading
+from array import array
 from dataclasses import dataclass, replace
 from typing import Iterable, Sequence
 
@@ -76,11 +77,12 @@ def draw(seed: int, counter: int) -> float:
 
 
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
-def _stream_ptr(device) -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream_ptr(device) -> int:
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 class Workspace:
@@ -268,6 +270,37 @@ def upload_params(w: dict, device, pinned: bool = False) -> dict:
     return out
 
 
+class _Window(array):
+    """The recent tokens: a list of ints to its readers, machine words underneath, so that a window
+    goes to the device as one copy (an element at a time, 64 tokens took 2.5 us and 256 took 9)."""
+    __slots__ = ()
+
+    def __new__(cls, tokens=()):
+        return super().__new__(cls, "q", tokens)
+
+    def __mul__(self, n):
+        return _Window(array.__mul__(self, n))
+
+    def __getitem__(self, i):
+        got = array.__getitem__(self, i)
+        return got.tolist() if isinstance(i, slice) else got
+
+    def __eq__(self, other):
+        return self.tolist() == (other.tolist() if isinstance(other, array) else other)
+
+    def __ne__(self, other):
+        return not self == other
+
+    __hash__ = None
+
+    def __repr__(self):
+        return repr(self.tolist())
+
+    def filled(self, n: int):
+        """The first n tokens' bytes, not copied."""
+        return memoryview(self)[:n].cast("B") if n else b""
+
+
 class Sampler:
     """One sequence's sampler: its settings, its recent tokens, its counter
     (sample.mojo:157-363)."""
@@ -278,7 +311,7 @@ class Sampler:
             raise ValueError("a sampler needs a vocabulary")
         self.config = config.copy()
         self._vocab = int(vocab)
-        self.recent = [-1] * config.repeat_last_n
+        self.recent = _Window([-1]) * config.repeat_last_n
         self.head = 0
         self.filled = 0
         self.drawn = 0
@@ -343,59 +376,109 @@ def _check_block(logits: torch.Tensor, samplers: Sequence[Sampler], rows: Sequen
     return block
 
 
+_U64 = 2**64 - 1
+
+
+def _packed(samplers: Sequence[Sampler]):
+    """The samplers' state as machine words: the seven float arrays one behind the other, top-k, the
+    window switches, seeds, counters, and the ragged windows (as bytes) and bias lists."""
+    cs = [s.config for s in samplers]
+    f = array("f", [c.temperature for c in cs] + [c.top_p for c in cs] + [c.min_p for c in cs] + [c.typical_p for c in cs]
+              + [c.repeat_penalty for c in cs] + [c.frequency_penalty for c in cs] + [c.presence_penalty for c in cs])
+    k = array("i", [c.top_k if c.top_k < 2**31 else 2**31 - 1 for c in cs])
+    win = bytes([c.repeat_last_n > 0 for c in cs])
+    sd = array("Q", [c.seed & _U64 for c in cs] + [s.drawn & _U64 for s in samplers])
+    off, n, parts = [0], 0, []
+    boff, bi, bv = [0], [], []
+    for s in samplers:
+        if s.filled:
+            r = s.recent if isinstance(s.recent, _Window) else _Window(s.recent)
+            m = s.filled if s.filled < len(r) else len(r)
+            parts.append(r.filled(m))
+            n += m
+        off.append(n)
+        if s.bias_ids:
+            bi.extend(s.bias_ids)
+            bv.extend(s.bias_vals)
+        boff.append(len(bi))
+    return f, k, win, sd, b"".join(parts), array("i", off), array("q", bi), array("f", bv), array("i", boff)
+
+
 def params_of(samplers: Sequence[Sampler]) -> dict:
     """The samplers' state as the parallel arrays the C entry point takes."""
     n = len(samplers)
-    w = dict(
-        temperature=np.array([s.config.temperature for s in samplers], np.float32),
-        top_k=np.array([min(s.config.top_k, 2**31 - 1) for s in samplers], np.int32),
-        top_p=np.array([s.config.top_p for s in samplers], np.float32),
-        min_p=np.array([s.config.min_p for s in samplers], np.float32),
-        typical_p=np.array([s.config.typical_p for s in samplers], np.float32),
-        repeat_penalty=np.array([s.config.repeat_penalty for s in samplers], np.float32),
-        frequency_penalty=np.array([s.config.frequency_penalty for s in samplers], np.float32),
-        presence_penalty=np.array([s.config.presence_penalty for s in samplers], np.float32),
-        window_on=np.array([1 if s.config.repeat_last_n > 0 else 0 for s in samplers], np.uint8),
-        seed=np.array([s.config.seed & (2**64 - 1) for s in samplers], np.uint64),
-        drawn=np.array([s.drawn & (2**64 - 1) for s in samplers], np.uint64),
-    )
-    hist, off = [], [0]
-    for s in samplers:
-        hist.extend(s.recent[: s.filled])
-        off.append(len(hist))
-    w["hist"] = np.array(hist, np.int64)
-    w["hist_off"] = np.array(off, np.int32)
-    bi, bv, boff = [], [], [0]
-    for s in samplers:
-        bi.extend(s.bias_ids)
-        bv.extend(s.bias_vals)
-        boff.append(len(bi))
-    w["bias_ids"] = np.array(bi, np.int64)
-    w["bias_vals"] = np.array(bv, np.float32)
-    w["bias_off"] = np.array(boff, np.int32)
-    assert len(w["temperature"]) == n
+    f, k, win, sd, hist, off, bi, bv, boff = _packed(samplers)
+    f, sd = np.array(f, np.float32), np.array(sd, np.uint64)
+    names = ("temperature", "top_p", "min_p", "typical_p", "repeat_penalty", "frequency_penalty", "presence_penalty")
+    w = {name: f[i * n:(i + 1) * n] for i, name in enumerate(names)}
+    w.update(top_k=np.array(k, np.int32), window_on=np.frombuffer(win, np.uint8).copy(), seed=sd[:n], drawn=sd[n:],
+             hist=np.frombuffer(hist, np.int64).copy(), hist_off=np.array(off, np.int32), bias_ids=np.array(bi, np.int64),
+             bias_vals=np.array(bv, np.float32), bias_off=np.array(boff, np.int32))
     return w
 
 
+# Each thread's device scratch for `pick_rows`, per device: a call ends with its stream idle, so the next
+# one in the thread may use the same memory on any stream. Kept up to 64 MB, given back with the thread.
+_scratch = threading.local()
+_SCRATCH_MOST = 64 << 20
+
+
+def _pick_scratch(dev, need: int) -> torch.Tensor:
+    kept = _scratch.__dict__.setdefault("bufs", {})
+    buf = kept.get(dev)
+    if buf is None or buf.numel() < need:
+        kept.pop(dev, None)
+        buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
+        if buf.numel() <= _SCRATCH_MOST:
+            kept[dev] = buf
+    return buf
+
+
 def pick_rows(logits: torch.Tensor, samplers: Sequence[Sampler], rows: Iterable[int] | None = None):
-    """Sample row `rows[i]` of `logits` with `samplers[i]`, all in one launch, then record
-    each token in its sampler (`_took`, sample.mojo:361-363). The batched counterpart of
-    the loop at batch.mojo:509-511. Returns the tokens as a list of ints."""
+    """Sample row `rows[i]` of `logits` with `samplers[i]`, all in one call of the library
+    (`molla_sample_pick_rows`), then record each token in its sampler (`_took`,
+    sample.mojo:361-363). The batched counterpart of the loop at batch.mojo:509-511.
+    Returns the tokens as a list of ints."""
     samplers = list(samplers)
     rows = list(range(len(samplers))) if rows is None else list(rows)
     block = _check_block(logits, samplers, rows)
     if not samplers:
         return []
+    if not block.is_cuda or block.dtype != torch.float32:
+        raise ValueError("logits must be a 2-D fp32 CUDA tensor")
     dev = block.device
-    if rows == list(range(block.shape[0])):
-        sel = block
-    else:
-        sel = block.index_select(0, torch.tensor(rows, device=dev))
-    p = upload_params(params_of(samplers), dev)
-    res = sample_batch(sel, p)
-    toks = res["tokens"].cpu().tolist()
-    stat = res["row_status"].cpu().tolist()
-    for s, t, st in zip(samplers, toks, stat):
+    n_rows, V = block.shape
+    if block.stride(1) != 1 or block.stride(0) < V:
+        if rows == list(range(n_rows)):
+            raise ValueError("logit rows must be contiguous")
+        block = block.index_select(0, torch.tensor(rows, device=dev))
+        rows = list(range(len(rows)))
+        n_rows = len(rows)
+    B = min(len(samplers), len(rows))
+    samplers = samplers[:B]
+    f, k, win, sd, hist, off, bi, bv, boff = _packed(samplers)
+    at = lambda a: a.buffer_info()[0]
+    fp, sp = at(f), at(sd)
+    row_ids = array("i", rows[:B])
+    got = array("i", bytes(8 * B))
+    gp = at(got)
+    L = capi.lib()
+    buf = _pick_scratch(dev, 0)
+    while True:
+        rc = L.molla_sample_pick_rows(
+            block.data_ptr(), block.stride(0), n_rows, V, at(row_ids), B, fp, at(k), fp + 4 * B, fp + 8 * B, fp + 12 * B,
+            fp + 16 * B, fp + 20 * B, fp + 24 * B, win, sp, sp + 8 * B, hist or None, at(off) if hist else None,
+            at(bi) if bi else None, at(bv) if bi else None, at(boff) if bi else None, buf.data_ptr(), buf.numel(),
+            _stream_ptr(dev), gp, gp + 4 * B)
+        if rc != capi.ERR_WORKSPACE:
+            break
+        need = L.molla_sample_pick_workspace_bytes(B, V, off[-1], boff[-1])
+        if need <= buf.numel():
+            break
+        buf = _pick_scratch(dev, need)
+    capi.check(rc)
+    toks = got[:B].tolist()
+    for s, t, st in zip(samplers, toks, got[B:]):
         s.last_status = st & 0xFFFFFFFF
         if st & capi.ROW_UNSUPPORTED:
             raise NotImplementedError("this combination of settings is not implemented on the device "
