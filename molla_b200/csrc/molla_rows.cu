@@ -42,7 +42,7 @@ constexpr int PLAN_BINS = 1024;            // row_plan: bins of the lanes' maxim
 constexpr float PLAN_RES = 32.0f;          // 32 per unit of logit
 
 enum { PLAN_DONE = 0, PLAN_SAMPLED = 1 };
-enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8 };
+enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8, F_JUMP = 16 };
 
 struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
 struct __align__(8) TilePlan { float thr, est; };
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
             }
             sum = warp_sum(s0 + s1);
         }
-        if (!c.pure) A.gmax[((size_t)rr * A.ntile + tile) * 32 + lane] = m;
+        A.gmax[((size_t)rr * A.ntile + tile) * 32 + lane] = m;
     } else if (!c.greedy) {  // only a top-k of one asks how many share the maximum
 #pragma unroll
         for (int j = 0; j < 32; j++) eq += x[j] == tmax ? 1 : 0;
@@ -424,8 +424,9 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
 // =============================================================================
 // Kernel 2: one block per row.
 // =============================================================================
+struct JumpShared { float in[128], over[128], own[128], pref[128]; int hit[128]; };
 struct PlanShared {
-    unsigned int hist[PLAN_BINS];
+    union { unsigned int hist[PLAN_BINS]; JumpShared jump; };
     int edge;
     float wsf[NWARP + 1];
     int wsi[NWARP + 1];
@@ -448,6 +449,55 @@ __device__ __forceinline__ float block_excl_scan_plus(float v, float *ws, float 
     }
     *total = t;
     return b + ex;
+}
+
+// Rows whose running sum jumps: MOLLA_ROW_SLOW_PATH tells a caller that the guesses of the sum's binade
+// went wrong somewhere. They are made for ranges of oL logits, 32 ranges to a group, with a prefix over
+// the groups of a block that is taken by subtracting a group's own sum, in double precision; where that
+// sum is more than 2^40 times everything before it, too few bits are left of what came before. This finds the
+// groups where that may be: the estimated sum of their tiles (or of as many of the group's largest logit)
+// against the largest term before them. Only sharp rows (low temperatures) have one.
+// Block of NT threads, 4 to a group; hit[q] is set for group q (block q / 16 of the layout, warp q % 16).
+__device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, float xmax, JumpShared &J) {
+    const int tid = threadIdx.x, lane = tid & 31, q = tid >> 2, part = tid & 3, g = q >> 4, w = q & 15, V = A.a.V;
+    const float *gm = A.gmax + (size_t)rr * A.ntile * 32;
+    const int e = min(V, (g + 1) * A.oVc), a = min(e, g * A.oVc + w * 32 * A.oL), b = min(e, a + 32 * A.oL);
+    float in = -INFINITY, over = -INFINITY;
+    if (g < A.oG && b > a) {
+#pragma unroll 8
+        for (int k = (a >> 5) + part; k <= (b - 1) >> 5; k += 4) {
+            const float m = gm[k];
+            over = fmaxf(over, m);
+            if (k * 32 >= a && k * 32 + 32 <= b) in = fmaxf(in, m);
+        }
+    }
+    in = fmaxf(in, __shfl_xor_sync(0xffffffffu, in, 1)); over = fmaxf(over, __shfl_xor_sync(0xffffffffu, over, 1));
+    in = fmaxf(in, __shfl_xor_sync(0xffffffffu, in, 2)); over = fmaxf(over, __shfl_xor_sync(0xffffffffu, over, 2));
+    __syncthreads();
+    if (part == 0) {
+        float own = 0.0f;
+        if (over > -INFINITY)
+#pragma unroll 4
+            for (int t = a / TILE; t <= (b - 1) / TILE; t++) {
+                const TileStat st = A.ts[(size_t)rr * A.ntile + t];
+                if (st.tmax > -INFINITY) own += st.tsum * ex2_approx(fminf((st.tmax - over) * f, 60.0f));
+            }
+        J.in[q] = in; J.over[q] = over; J.own[q] = log2f(fminf(own, (float)(b - a))); J.hit[q] = 0;
+    }
+    __syncthreads();
+    bool any = false;
+    if (tid < 128) {
+        float pf = lane > 0 ? J.in[tid - 1] : -INFINITY;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float v = __shfl_up_sync(0xffffffffu, pf, o); if (lane >= o) pf = fmaxf(pf, v); }
+#pragma unroll 4
+        for (int i = 0; i < (tid & ~31); i++) pf = fmaxf(pf, J.in[i]);
+        J.pref[tid] = pf;
+        // (e^-105 and less is zero)
+        any = (tid & 15) != 0 && J.over[tid] > -INFINITY && pf > -INFINITY && (J.over[tid] - pf) * f + J.own[tid] > 39.9f && (xmax - pf) * f < 152.0f;
+        J.hit[tid] = any ? 1 : 0;
+    }
+    return __syncthreads_or(any) != 0;
 }
 
 __device__ __forceinline__ void store_plan(const RowsArgs &A, int rr, const RowPlan &pl) {
@@ -523,6 +573,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     float e[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) e[u] = (tm[u] > -INFINITY) ? tsum[u] * ex2_approx((tm[u] - xmax) * f) : 0.0f;
+    const float first = A.gmax[(size_t)rr * A.ntile * 32];   // of the first 32 logits
     float total;
     const float ex = block_excl_scan_plus(e[0] + e[1], S.wsf, &total);
     const float est[2] = {ex, ex + e[0]};
@@ -601,6 +652,11 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
             __syncthreads();
         }
     }
+    bool jump = false;
+    if (A.oG > 0 && !((xmax - first) * f <= 29.0f)) {
+        __syncthreads();
+        jump = find_jumps(A, rr, f, xmax, S.jump);
+    }
     const float tv = (c.T == 1.0f) ? tau_x : __fdiv_rn(tau_x, c.T);
     const unsigned int tb = c.pure ? 0xffffffffu : __float_as_uint(expf_pinned(__fsub_rn(tv, top)));
     TilePlan *tp = A.tp + (size_t)rr * A.ntile;
@@ -613,7 +669,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         pl.kind = PLAN_SAMPLED;
         const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
         // (too few lanes to bound the head: row_finish narrows it down from the list)
-        pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) |
+        pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
                    ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
         pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
         pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
@@ -882,7 +938,7 @@ constexpr int H_ITEMS = 768;               // items of a row
 constexpr int H_CARE = 80, H_REC = 512;    // careful chunks whose values are at hand, and all of them
 // What a queued row has: nothing; its denominator; its head too (tile_walk prepares the walk past it);
 // its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
-enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3 };
+enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3, ST_DONE = 4 };
 
 struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the last of them | kind | own binade | place
 
@@ -1281,6 +1337,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         const float floor_p = __fmul_rn(__fdiv_rn(expf_pinned(__fsub_rn(pl.top, pl.top)), Z), g.minp);
         if (!(floor_p >= 2.2e-8f)) {
             if (tid == 0) finish_row(a, r, g, MOLLA_ROW_UNSUPPORTED | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), -1, Z, 0, 0, 0);
+            if (pl.flags & F_JUMP) queue_row(ST_DONE, 7);
             return;
         }
         int n = 0;
@@ -1367,9 +1424,13 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     __syncthreads();
     if (g.typ < 1.0f) {
         typical_rows(S, a, r, g, narrow ? -1 : S->cut, Z, S->tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u));
+        if (pl.flags & F_JUMP) queue_row(ST_DONE, 7);
         return;
     }
-    if (S->cut > 0) return;
+    if (S->cut > 0) {
+        if (pl.flags & F_JUMP) queue_row(ST_DONE, 7);
+        return;
+    }
     if (all_above || nc == 0) { queue_row(ST_SUM, 5); return; }
     // past the head: the sorted candidates and their prefix sums go along, and empty tables for tile_walk
     {
@@ -2660,6 +2721,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
     FSTAMP(1);
     const float Z = state != ST_NOTHING ? head->Z : exact_sum(c, false, 0.0f);
+    if (state == ST_NOTHING && c.tid == 0) R.head(c.rr)->Z = Z;   // (for jump_status)
     FSTAMP(3);
     dZ = Z;
     const float yZ = __fdiv_rn(1.0f, Z);
@@ -3003,14 +3065,124 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     finish();
 }
 
+// A row that find_jumps has marked: is a guess of its sum's binade wrong? Every marked group's guesses are
+// made here as they would be made from that prefix, and held against the sum before them (in double precision,
+// added without a subtraction). Pure rows add up twice, exponentials and then probabilities.
+__device__ __noinline__ void jump_status(const RowsArgs &R, int rr) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    AuxF *A = reinterpret_cast<AuxF *>(smem_raw);
+    JumpShared &J = *reinterpret_cast<JumpShared *>(A->items);
+    static_assert(sizeof(JumpShared) <= sizeof(A->items), "the groups' maxima use the items' space");
+    const RowHead *head = R.head(rr);
+    const RowPlan pl = head->plan;
+    const RowCfg &cfg = pl.c;
+    const float T = cfg.T, Z = head->Z, f = fminf(1.44269504f / T, 1.0e30f);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = R.r0 + rr, L = R.oL;
+    float *list = R.elist + (size_t)rr * R.ntile * TILE;   // (the row is done: its list is free)
+    unsigned int minp = 0u;
+    if (cfg.minp > 0.0f) minp = __float_as_uint(__fmul_rn(__fdiv_rn(expf_pinned(__fsub_rn(pl.top, pl.top)), Z), cfg.minp));
+    auto prob = [&](float e) -> float {
+        const float p = __fdiv_rn(e, Z);
+        return __float_as_uint(p) < minp ? 0.0f : p;
+    };
+    __syncthreads();
+    if (!find_jumps(R, rr, f, pl.xmax, J)) return;
+    bool slow = false;
+#pragma unroll 1
+    for (int q = 1; q < 128 && !slow; q++) {
+        if (!J.hit[q]) continue;
+        const int blk0 = (q >> 4) * R.oVc, e = min(R.a.V, blk0 + R.oVc), ga = blk0 + (q & 15) * 32 * L, gb = min(e, ga + 32 * L);
+        const float least = J.pref[q] - 40.0f / f;   // tiles below this are nothing beside what comes before the group
+        double sum[4] = {0.0, 0.0, 0.0, 0.0};   // before the block, in the block before the group; of the probabilities
+#pragma unroll 1
+        for (int span = 0; span * SPAN < gb; span++) {
+            bool want = (span + 1) * SPAN > ga;
+            for (int t = 0; t < SPAN / TILE && !want; t++) want = R.ts[(size_t)rr * R.ntile + span * (SPAN / TILE) + t].tmax >= least;
+            if (!want) continue;
+            __syncthreads();
+            if (tid < SPAN_THREADS) span_fetch(R.a, cfg.lrow, span * SPAN, A->tile);
+            span_ready(R.a, cfg, r, span * SPAN, A->tile, reinterpret_cast<SpanScratch *>(A->tile + SPAN_THREADS * PITCH), tid < SPAN_THREADS);
+            if (tid < SPAN_THREADS)
+#pragma unroll 1
+                for (int j = 0; j < 32; j++) {
+                    const int i = span * SPAN + tid * 32 + j;
+                    const float x = A->tile[tid * PITCH + j];
+                    if (i >= gb) break;
+                    const float ev = x > -INFINITY ? expf_pinned_nonpos(__fsub_rn(T == 1.0f ? x : div_slow(x, T), pl.top)) : 0.0f;
+                    if (i >= ga) list[i - ga] = ev;
+                    else if (ev != 0.0f) {
+                        sum[i < blk0 ? 0 : 1] += (double)ev;
+                        if (cfg.pure) sum[i < blk0 ? 2 : 3] += (double)prob(ev);
+                    }
+                }
+        }
+        __syncthreads();
+        for (int i = tid; i < gb - ga; i += NT) A->tile[i] = list[i];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            double v = sum[k];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && warp < 8) A->wsd[k * 8 + warp] = v;
+        }
+        __syncthreads();
+        bool wrong = false;
+        if (warp == 0) {
+#pragma unroll 1
+            for (int pass = 0; pass < (cfg.pure ? 2 : 1); pass++) {
+                double base = 0.0, before = 0.0;
+                for (int w = 0; w < 8; w++) { base += A->wsd[pass * 16 + w]; before += A->wsd[pass * 16 + 8 + w]; }
+                const int n = gb - ga, i0 = min(n, lane * L), i1 = min(n, i0 + L);
+                auto val = [&](int i) { return pass ? prob(A->tile[i]) : A->tile[i]; };
+                float c4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+                for (int i = i0; i < i1; i++) { const int k = (i - i0) < ((i1 - i0) & ~3) ? (i - i0) & 3 : 0; const float v = val(i);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) if (k == u) c4[u] = __fadd_rn(c4[u], v); }
+                const float csum = __fadd_rn(__fadd_rn(c4[0], c4[1]), __fadd_rn(c4[2], c4[3]));
+                const double inc = warp_incl_scan((double)csum, lane), own = __shfl_sync(0xffffffffu, inc, 31);
+                double ex = __shfl_up_sync(0xffffffffu, inc, 1);
+                if (lane == 0) ex = 0.0;
+                const double left = (before + own) - own;   // what the subtraction leaves of `before`
+                const double sst = base + (left + (inc - (double)csum));
+                const float lo = (float)(sst * (1.0 - 1.0 / 4096.0)), hi = (float)((sst + (double)csum) * (1.0 + 1.0 / 4096.0));
+                if (!(lo > 0.0f) || csum == 0.0f) continue;
+                const int jl = fexpo(lo), j2 = fexpo(hi);
+                if (!(j2 <= jl + 1 && jl >= -100 && j2 <= 100)) continue;
+                const bool two = j2 == jl + 1;
+                bool bad = false, some = false;
+                const float C1 = __fmul_rn(1.5f, fpow2(jl)), C2 = __fmul_rn(1.5f, fpow2(jl + 1));
+#pragma unroll 1
+                for (int i = i0; i < i1; i++) {
+                    const float v = val(i);
+                    const float k1 = __fsub_rn(__fadd_rn(v, C1), C1), k2 = __fsub_rn(__fadd_rn(v, C2), C2);
+                    bad |= fabsf(__fsub_rn(v, k1)) == fpow2(jl - 24) || v >= fpow2(jl - 1) || (two && fabsf(__fsub_rn(v, k2)) == fpow2(jl - 23));
+                    some |= k1 != 0.0f || (two && k2 != 0.0f);
+                }
+                if (bad || !some) continue;
+                const double s0 = base + before + ex, s1 = s0 + (double)csum;
+                const int js = fexpo((float)s0);
+                const bool held = two ? (js == jl || js == jl + 1) && s1 < (double)fpow2(jl + 2) : js == jl && s1 < (double)fpow2(jl + 1);
+                wrong |= !held;
+            }
+        }
+        slow = __syncthreads_or(wrong) != 0;
+    }
+    if (slow && tid == 0) R.a.row_status[r] |= MOLLA_ROW_SLOW_PATH;
+}
+
 __global__ void __launch_bounds__(NT, 1) row_tail_kernel(const __grid_constant__ RowsArgs R) {
     pdl_next();
     pdl_wait();
     const int n = R.queue[0];
 #pragma unroll 1
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
-        tail_row(R, R.queue[1 + q]);
+        const int rr = R.queue[1 + q];
+        if (R.head(rr)->state != ST_DONE) tail_row(R, rr);
         __syncthreads();
+        if (R.head(rr)->plan.flags & F_JUMP) {
+            jump_status(R, rr);
+            __syncthreads();
+        }
     }
 }
 
