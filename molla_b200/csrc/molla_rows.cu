@@ -182,20 +182,22 @@ __device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg 
         return;
     }
     if (status & (MOLLA_ROW_LOAD_TIMEOUT | MOLLA_ROW_DEGENERATE | MOLLA_ROW_INVALID_CONFIG | MOLLA_ROW_UNSUPPORTED | MOLLA_ROW_EMPTY)) token = -1;
+    // (all loads before the stores: one round trip instead of four)
+    const bool took = a.ring && token >= 0, seen = took && c.ring_n > 0;
+    const int q = c.q, hd = seen ? a.ring_head[q] : 0, f = seen ? a.ring_filled[q] : 0;
+    const unsigned long long dn = took ? a.drawn_rw[q] : 0ull;
+    const long long stop = took && a.stopped && a.stop_token ? a.stop_token[q] : -1ll;
     a.tokens[r] = token;
     a.row_status[r] = status;
-    if (a.ring && token >= 0) {
-        const int q = c.q;
-        if (c.ring_n > 0) {  // `observe` (:246-258)
-            const int hd = a.ring_head[q];
+    if (took) {
+        if (seen) {  // `observe` (:246-258)
             const int at = (hd >= 0 && hd < c.ring_n) ? hd : 0;
             a.ring[(size_t)q * (size_t)a.ring_cap + at] = (long long)token;
             a.ring_head[q] = (at + 1) % c.ring_n;
-            const int f = a.ring_filled[q];
             a.ring_filled[q] = f < c.ring_n ? f + 1 : c.ring_n;
         }
-        a.drawn_rw[q] += 1ull;
-        if (a.stopped) a.stopped[r] = (a.stop_token && a.stop_token[q] == (long long)token) ? 1 : 0;
+        a.drawn_rw[q] = dn + 1ull;
+        if (a.stopped) a.stopped[r] = (a.stop_token && stop == (long long)token) ? 1 : 0;
     }
     if (a.diag) { a.diag[4 * r] = dZ; a.diag[4 * r + 1] = dsum; a.diag[4 * r + 2] = dtarget; a.diag[4 * r + 3] = dp; }
 }
@@ -985,7 +987,7 @@ __device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *
     return b + inc - v;
 }
 
-// Sorts S->cand[0..n) (descending value, ascending id) and leaves the values in S->p.pc, padded with zeros
+// Sorts S->cand[0..n) (descending value, ascending id; zeros behind them up to a multiple of 16) and leaves the values in S->p.pc, padded with zeros
 // to a multiple of eight. Up to HT keys: every key counts the keys above it. More go through bins of value
 // first (a few keys each) and count within their bin.
 __device__ void head_sort(HeadShared *S, int n) {
@@ -995,14 +997,14 @@ __device__ void head_sort(HeadShared *S, int n) {
         const unsigned long long mine = tid < n ? S->cand[tid] : 0ull;
         int rank = 0;
         if (warp * 32 < n) {
-            int j = 0;
 #pragma unroll 1
-            for (; j + 4 <= n; j += 4) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(S->cand + j), b = *reinterpret_cast<const ulonglong2 *>(S->cand + j + 2);
-                rank += (a.x > mine ? 1 : 0) + (a.y > mine ? 1 : 0) + (b.x > mine ? 1 : 0) + (b.y > mine ? 1 : 0);
+            for (int j = 0; j < n; j += 16) {   // (padded to a multiple of 16; eight loads at a time)
+                ulonglong2 o[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) o[u] = *reinterpret_cast<const ulonglong2 *>(S->cand + j + 2 * u);
+#pragma unroll
+                for (int u = 0; u < 8; u++) rank += (o[u].x > mine ? 1 : 0) + (o[u].y > mine ? 1 : 0);
             }
-#pragma unroll 1
-            for (; j < n; j++) rank += S->cand[j] > mine ? 1 : 0;
         }
         __syncthreads();
         if (tid < n) { S->cand[rank] = mine; S->p.pc[rank] = key_val(mine); }
@@ -1141,53 +1143,58 @@ struct WalkLoads {
 
 // One warp, all lanes alike: the sum through the careful chunks W->rec[0..nrec) and the runs between
 // them; `more` holds the values of all of them. Returns false where a run's binade was guessed wrong.
+// Bound: 32 dependent additions a careful chunk. A register that has been added takes the next
+// record's value at once, so that no load is waited for between two chunks (337 cycles a record when each
+// asked for its own; two sets of registers would spill).
 __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
-    CareRec nx = W->rec[0];
+    CareRec r = W->rec[0], nx = W->rec[min(1, nrec)];
+    auto values = [&](const CareRec &c) { return reinterpret_cast<const float4 *>(W->care + min(c.meta >> 24, (unsigned int)H_CARE - 1u) * 32); };
+    float4 x[8];
+    {
+        const float4 *v = values(r);
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = v[i];
+    }
+    bool fine = true;
 #pragma unroll 1
-    for (int q = 0; q <= nrec; q++) {
-        const CareRec r = nx;
-        const unsigned int kind = (r.meta >> 8) & 3u, place = r.meta >> 24;
-        const float4 *v = reinterpret_cast<const float4 *>(W->care + place * 32);
-        float4 x[8];
-        if (q < nrec && kind != K_RUN && place < H_CARE) {   // asked for before it is known whether they are needed
+    for (int q = 0; ; q++) {
+        const float4 *v = values(nx);   // the next record's
+        const CareRec c = r;
+        r = nx;
+        nx = W->rec[min(q + 2, nrec)];
+        W->sbs[q] = sb;
+        const unsigned int to = sb + (c.k - kdone), j = c.meta & 0xffu, kind = (c.meta >> 8) & 3u, jb = (c.meta >> 16) & 0xffu, place = c.meta >> 24;
+        if (c.k != kdone && ((sb >> 23) != j || (to >> 23) != j)) { fine = false; break; }
+        kdone = c.k;
+        sb = to;
+        if (q == nrec) break;
+        const unsigned int e = sb >> 23, ta = sb + c.ka, tb = sb + c.kb;
+        const bool run = kind == K_RUN, low = e == jb;
+        if (run && (!low || (ta >> 23) != jb)) { fine = false; break; }
+        const unsigned int td = low ? ta : tb;
+        if (run || (kind == K_DUAL && (low || e == jb + 1u) && (td >> 23) == e)) {
+            sb = td;
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = v[i];
-        }
-        nx = W->rec[q < nrec ? q + 1 : q];
-        W->sbs[q] = sb;
-        const unsigned int kx = r.k - kdone;
-        kdone = r.k;
-        if (kx) {
-            const unsigned int to = sb + kx, j = r.meta & 0xffu;
-            if ((sb >> 23) != j || (to >> 23) != j) return false;
-            sb = to;
-        }
-        if (q == nrec) break;
-        const unsigned int e = sb >> 23, jb = (r.meta >> 16) & 0xffu;
-        if (kind == K_RUN) {
-            const unsigned int to = sb + r.ka;
-            if (e != jb || (to >> 23) != jb) return false;
-            sb = to;
             continue;
         }
-        if (kind == K_DUAL) {
-            const unsigned int to = e == jb ? sb + r.ka : sb + r.kb;
-            if ((e == jb || e == jb + 1u) && (to >> 23) == e) { sb = to; continue; }
-        }
-        if (place >= H_CARE) {
-            if (place == 255u) return false;
+        if (place >= H_CARE) {   // (a row with many: their values are still in L2)
+            if (place == 255u) { fine = false; break; }
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = reinterpret_cast<const float4 *>(more + place * 32)[i];
         }
         float s = __uint_as_float(sb);
 #pragma unroll
-        for (int i = 0; i < 8; i++) s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
+        for (int i = 0; i < 8; i++) {
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
+            x[i] = v[i];
+        }
         sb = __float_as_uint(s);
     }
     W->sbs[nrec + 1] = sb;
     Z = __uint_as_float(sb);
-    return true;
+    return fine;
 }
 
 // Typical-p (sample.mojo:525-567) on the m kept probabilities S->p.pc[0..m), descending, ids in S->cand:
@@ -1302,6 +1309,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
     };
     if (nitem > H_ITEMS || ncare > CARE_PLACES || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
+    const unsigned long long seed = a.seed ? a.seed[g.q] : 0ull, drawn = a.drawn ? a.drawn[g.q] : 0ull;   // (not needed before the end)
     if (tid == 0) S->n_ge = 0;
     const unsigned int nrec = wl.order(&S->w, ntile, nitem);
     if (nrec > (unsigned int)H_REC) { queue_row(ST_NOTHING, 2); return; }
@@ -1328,6 +1336,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         if (i >= HT) key = R.cand(rr)[i];
         S->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(key), Z, yZ)) << 32) | (key & 0xFFFFFFFFull);
     }
+    if (tid < 16 && nc + tid < HEADCAP) S->cand[nc + tid] = 0ull;
     __syncthreads();
     head_sort(S, nc);
     // min-p (sample.mojo:508-523) keeps a prefix of the sorted order: what reaches p_max * min_p
@@ -1405,7 +1414,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
             // the typical-p filter takes over from here
         } else if (cut > 0) {
             const float sum = pre[cut - 1];
-            const float target = __fmul_rn(draw01(a.seed ? a.seed[g.q] : 0ull, a.drawn ? a.drawn[g.q] : 0ull), sum);
+            const float target = __fmul_rn(draw01(seed, drawn), sum);
             // the first prefix sum above the target (they never fall), or the last one kept
             int at = 0, hi = cut - 1;
             while (at < hi) {
@@ -2574,17 +2583,23 @@ __device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x
 
 // A row that sorts nothing, once tile_walk has written the items of its probabilities: the walk to their
 // sum leaves the sum before every stretch, so the draw (sample.mojo:580-590) is a search among those and
-// then inside one stretch. Returns false where the general way has to be gone.
-__device__ __noinline__ bool tail_pure(CtxF &c, float u01, float Z) {
+// then inside one stretch. Returns false where the general way has to be gone. Bound: latency, of one
+// round of loads, the careful chunks' additions, and two more rounds for the values of one item.
+__device__ __noinline__ bool tail_pure(CtxF &c) {
     const RowsArgs &R = *c.R;
     WalkShared *W = reinterpret_cast<WalkShared *>(c.A->tile);
     AuxF *A = c.A;
-    RowHead *head = R.head(c.rr);
-    const int nitem = head->nitem;
-    if (nitem > H_ITEMS || head->ncare > CARE_PLACES) return false;
+    const RowHead *head = R.head(c.rr);
     WalkLoads<NT> wl;
     wl.load(R, c.rr);
-    __syncthreads();
+    const int nitem = head->nitem, ncare = head->ncare;
+    const float Z = head->Z;
+    c.pl = head->plan;
+    c.cfg = c.pl.c;
+    c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
+    c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
+    const unsigned long long seed = R.a.seed ? R.a.seed[c.cfg.q] : 0ull, drawn = R.a.drawn ? R.a.drawn[c.cfg.q] : 0ull;
+    if (nitem > H_ITEMS || ncare > CARE_PLACES) return false;
     const unsigned int nrec = wl.order(W, R.ntile, nitem);
     if (nrec > (unsigned int)H_REC) return false;
     FSTAMP(17);
@@ -2595,7 +2610,7 @@ __device__ __noinline__ bool tail_pure(CtxF &c, float u01, float Z) {
     }
     __syncthreads();
     if (!A->b_event) return false;
-    const float sum = A->b_s, target = __fmul_rn(u01, sum);
+    const float sum = A->b_s, target = __fmul_rn(draw01(seed, drawn), sum);
     // the first stretch (runs, then a careful chunk) behind which the sum exceeds the target
 #pragma unroll 1
     for (int q = c.tid; q <= (int)nrec; q += NT)
@@ -2609,64 +2624,70 @@ __device__ __noinline__ bool tail_pure(CtxF &c, float u01, float Z) {
         return true;
     }
     unsigned int sb = W->sbs[q];
-    // the stretch's items: behind the record before it, up to its own
-    const unsigned int k0 = q > 0 ? W->rec[q - 1].k : 0u;
-    int lo = 0, seen = 0;
-    // (records are items in order: find the q-th one, counting as order() did)
+    // 32 items at a time, the records among them counted as order() did: the q-th record's item is the
+    // first of the stretch, and the draw falls on a run of the stretch or on the careful chunk at its end
+    int seen = 0, item = -1;
+    bool in = q == 0;
 #pragma unroll 1
-    for (int i0 = 0; i0 < nitem && seen < q; i0 += 32) {
+    for (int i0 = 0; i0 < nitem && item < 0; i0 += 32) {
         const int i = i0 + c.lane;
-        bool care = false;
+        bool rec = false;
+        unsigned int ka = 0u;
         if (i < nitem) {
             const Item it = W->items[i];
-            care = it.kind() != K_RUN;
-            if (!care && i > 0) { const Item p = W->items[i - 1]; care = p.kind() == K_RUN && p.jb() != it.jb(); }
+            rec = it.kind() != K_RUN;
+            ka = it.ka;
+            if (!rec && i > 0) { const Item p = W->items[i - 1]; rec = p.kind() == K_RUN && p.jb() != it.jb(); }
         }
-        const unsigned int m = __ballot_sync(0xffffffffu, care);
-        const int n = __popc(m);
-        if (seen + n >= q) {
+        const unsigned int m = __ballot_sync(0xffffffffu, rec);
+        int from = 0;
+        if (!in) {
+            const int n = __popc(m);
+            if (seen + n < q) { seen += n; continue; }
             unsigned int w = m;
 #pragma unroll 1
             for (int k = seen + 1; k < q; k++) w &= w - 1u;
-            lo = i0 + __ffs((int)w); seen = q;
-        } else seen += n;
+            from = __ffs((int)w);      // behind the record before the stretch (which sbs[q] includes)
+            in = true;
+        }
+        const unsigned int later = from < 32 ? m & (0xffffffffu << from) : 0u;
+        const int end = later ? __ffs((int)later) - 1 : 32;
+        const unsigned int inc = warp_incl_scan(c.lane >= from && c.lane < end ? ka : 0u, c.lane);
+        const unsigned int hit = __ballot_sync(0xffffffffu, i < nitem && c.lane >= from && c.lane < end && target < __uint_as_float(sb + inc));
+        const int l = hit ? __ffs((int)hit) - 1 : end;
+        if (hit) { item = i0 + l; sb += __shfl_sync(0xffffffffu, inc - ka, l); }
+        else {
+            sb += __shfl_sync(0xffffffffu, inc, 31);
+            if (end < 32) item = i0 + end;
+        }
     }
-    (void)k0;
-    // item by item from there
     int tile = -1, at = 0;
-#pragma unroll 1
-    for (int i = lo; i < nitem && tile < 0; i++) {
-        const Item it = W->items[i];
-        const int n = it.cnt(), off = it.off();
-        if (it.kind() == K_RUN && !(target < __uint_as_float(sb + it.ka))) { sb += it.ka; continue; }
-        const float *v = c.list + (size_t)it.tile() * TILE + off;
+    if (item >= 0) {
+        const Item it = W->items[item];
+        const float *v = c.list + (size_t)it.tile() * TILE + it.off();
+        int n = it.cnt(), e0 = 0;
         float s = __uint_as_float(sb);
-        if (it.kind() == K_RUN) {
+        if (n > 32) {
             // the values of a run round by themselves: each lane adds up the units of its share
             const int j = fexpo(s), per = (n + 31) >> 5, b0 = min(n, c.lane * per), b1 = min(n, b0 + per);
             const float Cm = __fmul_rn(1.5f, fpow2(j));
             unsigned int k = 0u;
-#pragma unroll 1
+#pragma unroll 8
             for (int e = b0; e < b1; e++) k += __float_as_uint(__fadd_rn(v[e], Cm)) - __float_as_uint(Cm);
             const unsigned int inc = warp_incl_scan(k, c.lane);
             const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(sb + inc));
             const int l = hit ? __ffs((int)hit) - 1 : 31;
-            const unsigned int before = __shfl_sync(0xffffffffu, inc - k, l);
-            s = __uint_as_float(sb + before);
-            const int e0 = min(n, l * per), e1 = min(n, e0 + per);
-#pragma unroll 1
-            for (int e = e0; e < e1 && tile < 0; e++) {
-                s = __fadd_rn(s, v[e]);
-                if (target < s) { tile = it.tile(); at = off + e; }
-            }
-        } else {
-#pragma unroll 1
-            for (int e = 0; e < n && tile < 0; e++) {
-                s = __fadd_rn(s, v[e]);
-                if (target < s) { tile = it.tile(); at = off + e; }
-            }
+            s = __uint_as_float(sb + __shfl_sync(0xffffffffu, inc - k, l));
+            e0 = min(n, l * per); n = min(n, e0 + per) - e0;
         }
-        sb = __float_as_uint(s);
+        const float mine = c.lane < n ? v[e0 + c.lane] : 0.0f;
+        int first = -1;
+#pragma unroll 8
+        for (int e = 0; e < 32; e++) {
+            s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+            if (first < 0 && e < n && target < s) first = e;
+        }
+        if (first >= 0) { tile = it.tile(); at = it.off() + e0 + first; }
     }
     FSTAMP(10);
     if (c.lane == 0) finish_row(R.a, c.r, c.cfg, c.status, tile < 0 ? R.a.V - 1 : token_of(c, tile, at), Z, sum, target, 0.0f);
@@ -2683,10 +2704,14 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     IN_SHARED(A);
     c.rr = rr; c.r = R.r0 + rr;
     const RowHead *head = R.head(rr);
-    c.pl = head->plan;
     const int state = head->state;
-    const BatchArgs &a = R.a;
     FSTAMP(0);
+    if (state == ST_PURE) {
+        if (tail_pure(c)) return;
+        __syncthreads();
+    }
+    c.pl = head->plan;
+    const BatchArgs &a = R.a;
     c.cfg = c.pl.c;
     c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
     c.gitems = R.items(rr);
@@ -2761,7 +2786,6 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         }
     }
 
-    if (state == ST_PURE && tail_pure(c, u01, Z)) return;
     if (g.pure) {
         // ---- nothing sorted: the draw walks the vocabulary in order (sample.mojo:365-369, 580-594):
         // probabilities p = e / Z (:437-438), what min-p drops becomes zero
