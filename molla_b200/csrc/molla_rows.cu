@@ -1143,9 +1143,32 @@ struct WalkLoads {
 
 // One warp, all lanes alike: the sum through the careful chunks W->rec[0..nrec) and the runs between
 // them; `more` holds the values of all of them. Returns false where a run's binade was guessed wrong.
-// Bound: 32 dependent additions a careful chunk. A register that has been added takes the next
-// record's value at once, so that no load is waited for between two chunks (337 cycles a record when each
-// asked for its own; two sets of registers would spill).
+// Bound: 32 dependent additions a careful chunk, and the fetch of instructions: one warp runs this, once.
+// A register that has been added takes the next record's value at once, so that no load is waited for
+// between two chunks (337 cycles a record when each asked for its own; two sets of registers spill).
+// Chunks whose sum may lie in either of two binades come in stretches wherever a row's sum stays near a
+// power of two for long, 188 in one row of 196: while the binade holds, 32 of them are one prefix sum over
+// the lanes (173 cycles each one after the other), out of line, because most rows have none.
+__device__ __forceinline__ unsigned int kind_of(const CareRec &c) { return (c.meta >> 8) & 3u; }
+// From record q on: how many records one prefix sum takes, and the sum behind them.
+__device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsigned int sb, unsigned int kdone) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int e = sb >> 23;
+    CareRec c;
+    c.k = 0u; c.meta = 0u; c.ka = c.kb = 0u;
+    if (q + lane < nrec) c = W->rec[q + lane];
+    unsigned int kp = __shfl_up_sync(0xffffffffu, c.k, 1);
+    if (lane == 0) kp = kdone;
+    const unsigned int runs = c.k - kp, jb = (c.meta >> 16) & 0xffu, d = runs + (e == jb ? c.ka : c.kb);
+    const bool can = q + lane < nrec && kind_of(c) == K_DUAL && (e == jb || e == jb + 1u) &&
+                     (runs == 0u || ((c.meta & 0xffu) == e && runs < (1u << 24)));
+    const unsigned int inc = warp_incl_scan(can ? d : 0u, lane);
+    const unsigned int stop = __ballot_sync(0xffffffffu, !can || ((sb + inc) >> 23) != e);
+    const int n = stop ? __ffs((int)stop) - 1 : 32;
+    if (lane < n) W->sbs[q + lane] = sb + inc - d;
+    if (n > 0) sb += __shfl_sync(0xffffffffu, inc, n - 1);
+    return make_uint2(sb, (unsigned int)n);
+}
 __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
     CareRec r = W->rec[0], nx = W->rec[min(1, nrec)];
@@ -1164,7 +1187,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, i
         r = nx;
         nx = W->rec[min(q + 2, nrec)];
         W->sbs[q] = sb;
-        const unsigned int to = sb + (c.k - kdone), j = c.meta & 0xffu, kind = (c.meta >> 8) & 3u, jb = (c.meta >> 16) & 0xffu, place = c.meta >> 24;
+        const unsigned int to = sb + (c.k - kdone), j = c.meta & 0xffu, kind = kind_of(c), jb = (c.meta >> 16) & 0xffu, place = c.meta >> 24;
         if (c.k != kdone && ((sb >> 23) != j || (to >> 23) != j)) { fine = false; break; }
         kdone = c.k;
         sb = to;
@@ -1175,6 +1198,15 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, i
         const unsigned int td = low ? ta : tb;
         if (run || (kind == K_DUAL && (low || e == jb + 1u) && (td >> 23) == e)) {
             sb = td;
+            if (kind_of(r) == K_DUAL && q + 1 < nrec) {
+                const uint2 t = dual_stretch(W, nrec, q + 1, sb, kdone);
+                sb = t.x;
+                q += (int)t.y;
+                kdone = t.y ? W->rec[q].k : kdone;
+                r = W->rec[q + 1];
+                nx = W->rec[min(q + 2, nrec)];
+                v = values(r);
+            }
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = v[i];
             continue;
