@@ -936,8 +936,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // and of one round of loads, so the block is small and four of them share an SM.
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
-constexpr int H_ITEMS = 768;               // items of a row
-constexpr int H_CARE = 80, H_REC = 512;    // careful chunks whose values are at hand, and all of them
+constexpr int H_ITEMS = 1024;              // items of a row
+constexpr int H_CARE = 64, H_REC = 704;    // careful chunks whose values are at hand, and all of them
 // What a queued row has: nothing; its denominator; its head too (tile_walk prepares the walk past it);
 // its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
 enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3, ST_DONE = 4 };
@@ -949,7 +949,7 @@ struct __align__(16) WalkShared {
     float care[H_CARE * 32];
     CareRec rec[H_REC + 1];
     unsigned int sbs[H_REC + 2];           // the sum before every record's runs
-    unsigned short toff[MAX_TILES + 4];
+    unsigned short toff[MAX_TILES + 4], ritem[H_REC];
     unsigned int ws[NWARP + 1], ws2[NWARP + 1];
 };
 
@@ -1127,6 +1127,7 @@ struct WalkLoads {
                     CareRec c;
                     c.k = kx; c.ka = it[u].ka; c.kb = it[u].kb;
                     c.meta = pj[u] | (it[u].kind() << 8) | (it[u].jb() << 16) | (it[u].place() << 24);
+                    W->ritem[nx] = (unsigned short)i;
                     W->rec[nx++] = c;
                 } else kx += it[u].ka;
             }
@@ -1169,7 +1170,14 @@ __device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsig
     if (n > 0) sb += __shfl_sync(0xffffffffu, inc, n - 1);
     return make_uint2(sb, (unsigned int)n);
 }
-__device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, int nrec, float &Z) {
+__device__ __noinline__ float add_listed(float s, const float *v, int n) {
+    const int lane = threadIdx.x & 31;
+    const float mine = lane < n ? v[lane] : 0.0f;
+#pragma unroll 8
+    for (int e = 0; e < 32; e++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+    return s;
+}
+__device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, const float *list, int nrec, float &Z) {
     unsigned int sb = 0u, kdone = 0u;
     CareRec r = W->rec[0], nx = W->rec[min(1, nrec)];
     auto values = [&](const CareRec &c) { return reinterpret_cast<const float4 *>(W->care + min(c.meta >> 24, (unsigned int)H_CARE - 1u) * 32); };
@@ -1212,7 +1220,13 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, i
             continue;
         }
         if (place >= H_CARE) {   // (a row with many: their values are still in L2)
-            if (place == 255u) { fine = false; break; }
+            if (place == 255u) {   // (past CARE_PLACES: in its tile's list)
+                const Item it = W->items[W->ritem[q]];
+                sb = __float_as_uint(add_listed(__uint_as_float(sb), list + (size_t)it.tile() * TILE + it.off(), it.cnt()));
+#pragma unroll
+                for (int i = 0; i < 8; i++) x[i] = v[i];
+                continue;
+            }
 #pragma unroll
             for (int i = 0; i < 8; i++) x[i] = reinterpret_cast<const float4 *>(more + place * 32)[i];
         }
@@ -1325,7 +1339,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     const BatchArgs &a = R.a;
     const int ntile = R.ntile;
     // everything that will be wanted, in one round of loads (what lies past the counts is not used)
-    const int ncand = head->ncand, nitem = head->nitem, ncare = head->ncare;
+    const int ncand = head->ncand, nitem = head->nitem;
     const RowPlan &pl = head->plan;
     const int kind = pl.kind;
     WalkLoads<HT> wl;
@@ -1336,11 +1350,11 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     const bool narrow = (pl.flags & F_NARROW) != 0;
     auto queue_row = [&](int state, int why = 0) {
 #ifdef MOLLA_SAMPLE_TESTING
-        if (a.prof && tid == 0) { a.prof[(long long)r * 32 + 24] = why; a.prof[(long long)r * 32 + 25] = nitem; a.prof[(long long)r * 32 + 26] = ncare; a.prof[(long long)r * 32 + 27] = ncand; }
+        if (a.prof && tid == 0) { a.prof[(long long)r * 32 + 24] = why; a.prof[(long long)r * 32 + 25] = nitem; a.prof[(long long)r * 32 + 26] = head->ncare; a.prof[(long long)r * 32 + 27] = ncand; }
 #endif
         if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
     };
-    if (nitem > H_ITEMS || ncare > CARE_PLACES || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
+    if (nitem > H_ITEMS || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
     const unsigned long long seed = a.seed ? a.seed[g.q] : 0ull, drawn = a.drawn ? a.drawn[g.q] : 0ull;   // (not needed before the end)
     if (tid == 0) S->n_ge = 0;
     const unsigned int nrec = wl.order(&S->w, ntile, nitem);
@@ -1348,7 +1362,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     // ---- the softmax denominator, exactly as the sequential loop rounds it (sample.mojo:431-434)
     if (warp == 0) {
         float z = 0.0f;
-        const bool fine = walk_records(&S->w, R.care(rr), (int)nrec, z);
+        const bool fine = walk_records(&S->w, R.care(rr), R.elist + (size_t)rr * ntile * TILE, (int)nrec, z);
         if (lane == 0) { S->Z = z; S->ok = fine ? 1 : 0; }
     }
     __syncthreads();
@@ -2624,20 +2638,20 @@ __device__ __noinline__ bool tail_pure(CtxF &c) {
     const RowHead *head = R.head(c.rr);
     WalkLoads<NT> wl;
     wl.load(R, c.rr);
-    const int nitem = head->nitem, ncare = head->ncare;
+    const int nitem = head->nitem;
     const float Z = head->Z;
     c.pl = head->plan;
     c.cfg = c.pl.c;
     c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
     c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
     const unsigned long long seed = R.a.seed ? R.a.seed[c.cfg.q] : 0ull, drawn = R.a.drawn ? R.a.drawn[c.cfg.q] : 0ull;
-    if (nitem > H_ITEMS || ncare > CARE_PLACES) return false;
+    if (nitem > H_ITEMS) return false;
     const unsigned int nrec = wl.order(W, R.ntile, nitem);
     if (nrec > (unsigned int)H_REC) return false;
     FSTAMP(17);
     if (c.warp == 0) {
         float z = 0.0f;
-        const bool fine = walk_records(W, R.care(c.rr), (int)nrec, z);
+        const bool fine = walk_records(W, R.care(c.rr), c.list, (int)nrec, z);
         if (c.lane == 0) { A->b_s = z; A->b_event = fine ? 1 : 0; A->evt_thread = 0x7fffffff; }
     }
     __syncthreads();
