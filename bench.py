@@ -262,11 +262,12 @@ class Timed:
         return self.out["tokens"].cpu().numpy(), self.out["row_status"].cpu().numpy()
 
     def launches_per_step(self):
-        sms = self.torch.cuda.get_device_properties(self.dev).multi_processor_count
-        # thread blocks per row (the smallest cluster whose blocks hold 38400 logits each); the kernel
-        # that ranks the rows runs when not all rows can start at once
-        groups = next(g for g in (1, 2, 4, 8, 8) if self.V <= 38400 * g or g == 8)
-        return 1 + (1 if self.B * groups > sms else 0) + (1 if (self.logprob or self.top_n) else 0)
+        # seven row kernels for every 2^27 logits of the block (rows go in equal parts), and three
+        # logprob kernels (one for rows too short for tiles)
+        per_row = -(-self.V // 1024) * 1024
+        parts = -(-self.B // max(1, (1 << 27) // per_row))
+        lp = (3 if self.V >= 4096 else 1) if (self.logprob or self.top_n) else 0
+        return 7 * parts + lp
 
 
 def measure_e2e(w, dev, steps, barrier, top_n=0, logprob=False):
@@ -373,8 +374,8 @@ def run_ours(args):
                        "params": "per-row settings, windows and draw counters resident on the device, uploaded once "
                                  "outside the timed region (the decode loop keeps them there)",
                        "timed_region_ms": ms, "ms_per_step_of_3_more_runs": repeats},
-            "roofline": roofline(abytes_rank, ms_step, "sample_rows_cluster_kernel",
-                                 f"sample_rows_cluster_kernel:{args.config}" if args.rows is None else None),
+            "roofline": roofline(abytes_rank, ms_step, "tile_stats .. row_tail (all row kernels)",
+                                 f"row_kernels:{args.config}" if args.rows is None else None),
             "e2e": None if e2e_ms is None else {
                 "value": B_total * e2e_steps / (e2e_max / 1e3), "unit": "tokens/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": e2e_max / e2e_steps, "steps": e2e_steps,
@@ -411,7 +412,7 @@ def other_configs(dev, barrier):
         top_n = int(w.get("top_n", 0))
         t = Timed(w, dev, top_n, top_n > 0)
         ms = t.run(steps, 3, barrier) / steps
-        rf = roofline(algorithmic_bytes(w, top_n, top_n > 0), ms, "sample_rows_cluster_kernel", None)
+        rf = roofline(algorithmic_bytes(w, top_n, top_n > 0), ms, "tile_stats .. row_tail (all row kernels)", None)
         out[cfg] = {"workload": w["name"], "ms_per_step": ms, "tokens_per_s": w["B"] / (ms / 1e3),
                     "achieved_GBs": rf["achieved"], "frac_of_measured_peak": rf["frac"],
                     "launches_per_step": t.launches_per_step(), "blocks_rotated": t.nbuf}

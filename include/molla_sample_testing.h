@@ -12,8 +12,7 @@ extern "C" {
 #endif
 
 /* Experiment switches of the row kernels. Streaming kernel: bit 1 no last-use hint on the second
- * pass over a row, bit 2 no keep hint on list traffic, bit 3 no help from idle blocks. Both
- * kernels: bit 4 pretends, after the row has arrived, that one warp's bounded wait ran out
+ * pass over a row, bit 2 no keep hint on list traffic. All of them: bit 4 pretends, after the row has arrived, that one warp's bounded wait ran out
  * (nothing is withheld and nothing is left waiting): the row must come back with
  * MOLLA_ROW_LOAD_TIMEOUT, token -1 and its sampler state untouched. 0 = production behaviour. */
 void molla_sample_debug_knobs(int32_t knobs);

@@ -32,10 +32,6 @@ struct BatchArgs {
     int knobs;                   // experiment switches (0 = production behaviour)
     int *topk_out; int topk_cap; // optional [B x cap] ids of the sorted head after top-k
 #endif
-    // thread blocks that ran out of rows help the ones still converting a long list (HelpSlot)
-    void *help;                  // [grid] HelpSlot, one per thread block, or nullptr
-    unsigned int *help_tables;   // [grid x HELP_TABLE_WORDS]
-    int *rows_done;              // rows finished so far (zeroed before the launch)
     // decode-step form: which row of the logit block each batch row reads, which slot of the
     // per-stream arrays (settings and state) it uses, the final-logit softcap, and the state
     const int *rows;             // [B] or nullptr (row r reads logit row r)
@@ -473,8 +469,7 @@ struct BinQuery {
     const unsigned int *hq, *hqh, *hc;  // per bin: integer mass (low MASS_SPLIT bits summed, the rest summed) and count
 };
 
-// `bin_load(b, q, n)` gives bin b's integer mass and count (one thread block's tables, or the
-// sum over the tables of a cluster's thread blocks).
+// `bin_load(b, q, n)` gives bin b's integer mass and count.
 struct NoAdjust {};
 // `adjust(q, eq)` may change the masses of the thread's bins once their sum before the bins (eq)
 // is known; it returns whether it did (the same answer in every thread).

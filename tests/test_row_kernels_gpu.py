@@ -1,0 +1,67 @@
+"""The tile kernels at the sizes where they can go wrong, against the CPU oracle."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from helpers import OracleSampler
+from molla_b200 import sampler as S, workloads as W
+from test_parity_gpu import compare
+
+pytestmark = pytest.mark.gpu
+
+
+def _kinds(w, B, V):
+    """Rows of every way through the kernels: greedy, top-k of one, sorted head, wide top-k, a nucleus past
+    the head, nothing sorted (with min-p too), typical-p."""
+    w["temperature"][:] = np.float32([0.0, 0.7, 0.7, 1.0, 1.4, 1.0, 1.2, 0.9])[np.arange(B) % 8]
+    w["top_k"][:] = np.int32([0, 1, 40, 1024, 0, 0, 0, 50])[np.arange(B) % 8]
+    w["top_p"][:] = np.float32([1, 1, 0.9, 0.99, 0.98, 1, 1, 0.95])[np.arange(B) % 8]
+    w["min_p"][:] = np.float32([0, 0, 0, 0, 0, 0, 1e-4, 0])[np.arange(B) % 8]
+    w["typical_p"][:] = np.float32([1, 1, 1, 1, 1, 1, 1, 0.9])[np.arange(B) % 8]
+    return w
+
+
+@pytest.mark.parametrize("V", [33, 1023, 1024, 1025, 4095, 4096, 4097, 8191, 8193, 16385, 50257])
+def test_tile_edges(dev, lib, oracle, V):
+    B = 16
+    w = _kinds(W.config3(seed=V, B=B, V=V, H=16), B, V)
+    compare(w, dev, oracle, f"V={V}", top_n=min(5, V), max_exception_frac=0.2)
+    compare(w, dev, oracle, f"V={V}, odd stride", stride=V + 3, offset=1, max_exception_frac=0.2)
+
+
+@pytest.mark.parametrize("V", [3000, 9000, 16000, 40000])
+def test_sums_that_stay_near_a_power_of_two(dev, lib, oracle, V):
+    """Hundreds of chunks whose sum may lie in either of two binades: some, more than have places for their
+    values, more than the row kernel takes."""
+    B = 16
+    rng = np.random.default_rng(V)
+    w = _kinds(W.config3(seed=V + 1, B=B, V=V, H=4), B, V)
+    w["temperature"][:] = np.where(w["temperature"] > 0, np.float32(1.0), np.float32(0.0))
+    x = (-15.5 + rng.standard_normal((B, V)) * 0.2).astype(np.float32)
+    x[:, 0] = 0.0
+    x[:, 1] = np.log(np.maximum(1.0 - 2.1e-7 * V * rng.random(B), 0.5)).astype(np.float32)
+    w["logits"] = x
+    compare(w, dev, oracle, f"near two, V={V}", max_exception_frac=0.3)
+
+
+@pytest.mark.parametrize("V", [1000, 4097])
+def test_pick_rows_in_place(dev, lib, oracle, V):
+    """Samplers on the host, logit rows in any order and twice, a block with a stride, biases and windows."""
+    rng = np.random.default_rng(V)
+    wide = torch.from_numpy((3 * rng.standard_normal((6, V + 5))).astype(np.float32)).to(dev)
+    block = wide[:, 2:V + 2]
+    rows = [4, 0, 4, 5, 1]
+    mine, ref = [], []
+    for i in range(len(rows)):
+        kw = dict(temperature=0.3 * i, top_k=20 * (i % 2), repeat_penalty=1.2, repeat_last_n=8 * i, seed=i)
+        mine.append(S.Sampler(S.SamplerConfig(**kw), V, dev))
+        ref.append(OracleSampler(oracle, V, **kw))
+        for t in range(i):
+            mine[i].bias(7 * t + 1, 1.5 - t)
+            ref[i].bias(7 * t + 1, 1.5 - t)
+    host = block.cpu().numpy()
+    for _ in range(12):
+        got = S.pick_rows(block, mine, rows)
+        assert got == [r.pick(host, row) for r, row in zip(ref, rows)]
+        assert [m.recent[: m.filled] for m in mine] == [r.recent[: r.filled] for r in ref]
