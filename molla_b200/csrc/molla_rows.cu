@@ -897,7 +897,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     SpanShared *S = reinterpret_cast<SpanShared *>(smem_raw);
     pdl_next();
     pdl_wait();
-    const int rr = blockIdx.x / A.nspan, span = blockIdx.x - rr * A.nspan, r = A.r0 + rr;
+    // (the last spans first: of a block larger than the L2 they are what tile_stats has left there)
+    const int b = (int)(gridDim.x - 1u - blockIdx.x), rr = b / A.nspan, span = b - rr * A.nspan, r = A.r0 + rr;
     RowHead *head = A.head(rr);
     const RowPlan pl = head->plan;
     if (pl.kind == PLAN_DONE) return;
