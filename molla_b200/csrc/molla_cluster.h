@@ -1,0 +1,14 @@
+// The launch of the one-row-per-cluster kernel (molla_cluster.cu), called by the entry points
+// in molla_sample.cu.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+struct BatchArgs;
+
+// Whether B rows of V logits are better off there than in the tile kernels.
+bool molla_cluster_better(int V, int B);
+
+// Enqueues the sampling of `a.B` rows, for which molla_cluster_better holds, on `st`. Returns MOLLA_OK or
+// a MOLLA_ERR_* code with its message in `err`.
+int molla_cluster_launch(const BatchArgs &a, cudaStream_t st, char *err, size_t errlen);

@@ -47,6 +47,7 @@ struct BatchArgs {
     // vocab-sharded form: this GPU holds columns [col0, col0 + V) of a vocabulary of Vg
     int n_logit_rows, n_slots;   // bounds of rows[] and slot[] values (0 = not given)
     const unsigned int *mask; long long mask_stride;  // grammar mask: bit t of row r's words = token t allowed (nullptr = all)
+    int G, Vc, L;                // one row per thread-block cluster: blocks per cluster, logits per block, logits per thread
     int layout_B;                // rows of the call as its caller made it (0 = B)
     int mode;                    // 0 whole pipeline; 1, 2, 3 the stages around the two all-gathers
     int col0, Vg;

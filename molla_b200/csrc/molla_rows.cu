@@ -469,7 +469,7 @@ __device__ __forceinline__ float block_excl_scan_plus(float v, float *ws, float 
 // went wrong somewhere. They are made for ranges of oL logits, 32 ranges to a group, with a prefix over
 // the groups of a block that is taken by subtracting a group's own sum, in double precision; where that
 // sum is more than 2^40 times everything before it, too few bits are left of what came before. This finds the
-// groups where that may be: the estimated sum of their tiles (or of as many of the group's largest logit)
+// groups where that may be: the estimated sum of their tiles
 // against the largest term before them. Only sharp rows (low temperatures) have one.
 // Block of NT threads, 4 to a group; hit[q] is set for group q (block q / 16 of the layout, warp q % 16).
 __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, float xmax, JumpShared &J) {
@@ -494,7 +494,10 @@ __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, floa
 #pragma unroll 4
             for (int t = a / TILE; t <= (b - 1) / TILE; t++) {
                 const TileStat st = A.ts[(size_t)rr * A.ntile + t];
-                if (st.tmax > -INFINITY) own += st.tsum * ex2_approx(fminf((st.tmax - over) * f, 60.0f));
+                if (st.tmax > over) {   // (a tile that reaches out of the group: its lanes' maxima bound what is inside)
+#pragma unroll 8
+                    for (int k = max(t * 32, a >> 5); k < min(t * 32 + 32, ((b - 1) >> 5) + 1); k++) own += 32.0f * ex2_approx(fminf((gm[k] - over) * f, 0.0f));
+                } else if (st.tmax > -INFINITY) own += st.tsum * ex2_approx((st.tmax - over) * f);
             }
         J.in[q] = in; J.over[q] = over; J.own[q] = log2f(fminf(own, (float)(b - a))); J.hit[q] = 0;
     }

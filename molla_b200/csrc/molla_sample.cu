@@ -1,7 +1,7 @@
 // The C ABI (declared in include/molla_sample.h) and the streaming kernel.
 //
-// The ordinary entry points' rows go through the kernels of molla_rows.cu, their logprobs
-// through those of molla_logprob.cu. What follows here serves the forms that take no scratch
+// The ordinary entry points' rows go through the kernel of molla_cluster.cu or those of
+// molla_rows.cu, their logprobs through those of molla_logprob.cu. What follows here serves the forms that take no scratch
 // of that size or stop between stages: the one without allocations, the dump of penalised
 // logits, and the stages of the vocab-sharded form. One CTA owns one logit row at a time and
 // streams it twice through shared memory: pass A reads it from HBM and finds the maximum;
@@ -48,6 +48,7 @@
 #endif
 #include "molla_device.cuh"
 #include "molla_exact.cuh"
+#include "molla_cluster.h"
 #include "molla_logprob.h"
 #include "molla_rows.h"
 
@@ -1741,6 +1742,7 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
 int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
+    if (molla_cluster_better(a.V, a.layout_B > 0 ? a.layout_B : a.B)) return molla_cluster_launch(a, st, g_err, sizeof(g_err));
     return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err));
 }
 
