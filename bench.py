@@ -262,11 +262,16 @@ class Timed:
         return self.out["tokens"].cpu().numpy(), self.out["row_status"].cpu().numpy()
 
     def launches_per_step(self):
-        # seven row kernels for every 2^27 logits of the block (rows go in equal parts), and three
-        # logprob kernels (one for rows too short for tiles)
+        # one row kernel where the clusters of all rows are resident at once (the smallest cluster whose
+        # blocks hold 38400 logits each), else seven for every 2^27 logits of the block (rows go in equal
+        # parts); and three logprob kernels (one for rows too short for tiles)
+        sms = self.torch.cuda.get_device_properties(self.dev).multi_processor_count
+        lp = (3 if self.V >= 4096 else 1) if (self.logprob or self.top_n) else 0
+        groups = next((g for g in (1, 2, 4, 8) if self.V <= 38400 * g), None)
+        if groups and self.B * groups * 9 <= sms * 8:
+            return 1 + lp
         per_row = -(-self.V // 1024) * 1024
         parts = -(-self.B // max(1, (1 << 27) // per_row))
-        lp = (3 if self.V >= 4096 else 1) if (self.logprob or self.top_n) else 0
         return 7 * parts + lp
 
 

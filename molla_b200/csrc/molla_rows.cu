@@ -1008,6 +1008,10 @@ __device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *
     return b + inc - v;
 }
 
+// A key's value in units of 2^-60, as bits: subnormal values spread over their binades like all others (in one
+// bin, the 600 subnormals that a short row of a low temperature can keep took 100 us to be counted).
+__device__ __forceinline__ unsigned int spread_bits(unsigned long long key) { return __float_as_uint(__fmul_rn(key_val(key), 1152921504606846976.0f)); }
+
 // Sorts S->cand[0..n) (descending value, ascending id; zeros behind them up to a multiple of 16) and leaves the values in S->p.pc, padded with zeros
 // to a multiple of eight. Up to HT keys: every key counts the keys above it. More go through bins of value
 // first (a few keys each) and count within their bin.
@@ -1036,7 +1040,7 @@ __device__ void head_sort(HeadShared *S, int n) {
         for (int u = 0; u < KPT; u++) {
             const int i = tid + u * HT;
             k[u] = i < n ? S->cand[i] : 0ull;
-            if (i < n) { lo = min(lo, (unsigned int)(k[u] >> 32)); hi = max(hi, (unsigned int)(k[u] >> 32)); }
+            if (i < n) { const unsigned int b = spread_bits(k[u]); lo = min(lo, b); hi = max(hi, b); }
         }
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
@@ -1048,7 +1052,7 @@ __device__ void head_sort(HeadShared *S, int n) {
         for (int w = 0; w < HW; w++) { lo = min(lo, S->ws[w]); hi = max(hi, S->ws2[w]); }
         const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
         unsigned int slot[KPT];
-        auto bin_of = [&](unsigned long long key) { return NBINS - 1 - (((unsigned int)(key >> 32) - lo) >> shift); };   // descending
+        auto bin_of = [&](unsigned long long key) { return NBINS - 1 - ((spread_bits(key) - lo) >> shift); };   // descending
 #pragma unroll
         for (int u = 0; u < KPT; u++)
             if (tid + u * HT < n) slot[u] = atomicAdd(&S->sbin[bin_of(k[u])], 1u);
