@@ -1,4 +1,5 @@
-// The ordinary entry points' path: a batch of logit rows through seven small kernels.
+// The ordinary entry points' path for batches whose rows do not all fit the chip at once in thread-block
+// clusters: seven small kernels.
 //
 //   tile_stats   every tile of 1024 logits: its maximum, where it lies, and an estimate of the tile's
 //                sum of exponentials                                     (reads the block from HBM)
