@@ -264,9 +264,9 @@ class Timed:
     def launches_per_step(self):
         # one row kernel where the clusters of all rows are resident at once (the smallest cluster whose
         # blocks hold 38400 logits each), else seven for every 2^27 logits of the block (rows go in equal
-        # parts); and three logprob kernels (one for rows too short for tiles)
+        # parts); and two logprob kernels (one for rows too short for tiles)
         sms = self.torch.cuda.get_device_properties(self.dev).multi_processor_count
-        lp = (3 if self.V >= 4096 else 1) if (self.logprob or self.top_n) else 0
+        lp = (2 if self.V >= 4096 and self.V // 1024 >= self.top_n else 1) if (self.logprob or self.top_n) else 0
         groups = next((g for g in (1, 2, 4, 8) if self.V <= 38400 * g), None)
         if groups and self.B * groups * 9 <= sms * 8:
             return 1 + lp

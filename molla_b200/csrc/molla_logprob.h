@@ -4,7 +4,7 @@
 #include <stddef.h>
 
 // Whether rows of V logits go this way; shorter ones are one block's work.
-bool molla_logprob_tiled(int V);
+bool molla_logprob_tiled(int V, int top_n);
 size_t molla_logprob_workspace_bytes(int B, int V);
 
 // The chosen tokens' and the top N's logprobs (workspace of molla_logprob_workspace_bytes), or with

@@ -1751,7 +1751,7 @@ int launch_logprobs(const float *logits, int64_t row_stride, int B, int V, const
                     float *top_lps, const int *rows, int n_logit_rows, float softcap, void *d_workspace, cudaStream_t st) {
     if (!chosen && top_n == 0) return MOLLA_OK;
     cudaError_t e;
-    if (molla_logprob_tiled(V)) {
+    if (molla_logprob_tiled(V, top_n)) {
         e = molla_logprob_launch(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, rows, n_logit_rows, softcap,
                                  d_workspace, nullptr, st);
     } else {
@@ -2411,7 +2411,7 @@ int32_t molla_sample_logprobs(const float *d_logits, int64_t row_stride, int32_t
     g_err[0] = 0;
     if (!d_logits || !d_out || B < 0 || V <= 0 || row_stride < V) return fail(MOLLA_ERR_ARGUMENT, "bad arguments to logprobs%s");
     if (B == 0) return MOLLA_OK;
-    if (molla_logprob_tiled(V)) {
+    if (molla_logprob_tiled(V, top_n)) {
         const cudaError_t e = molla_logprob_launch(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0.0f,
                                                    nullptr, d_out, (cudaStream_t)stream);
         return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
