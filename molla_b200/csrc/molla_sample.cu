@@ -2411,7 +2411,7 @@ int32_t molla_sample_logprobs(const float *d_logits, int64_t row_stride, int32_t
     g_err[0] = 0;
     if (!d_logits || !d_out || B < 0 || V <= 0 || row_stride < V) return fail(MOLLA_ERR_ARGUMENT, "bad arguments to logprobs%s");
     if (B == 0) return MOLLA_OK;
-    if (molla_logprob_tiled(V, top_n)) {
+    if (molla_logprob_tiled(V, 0)) {
         const cudaError_t e = molla_logprob_launch(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0.0f,
                                                    nullptr, d_out, (cudaStream_t)stream);
         return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
