@@ -87,6 +87,7 @@ struct __align__(16) RowCfg {
     const long long *histp;
     long long n_lim;
     bool greedy, topp_on, pure, open_row;
+    bool late;              // the row is looked at again once it is answered (F_JUMP): its state moves on behind that
     unsigned int status;
 };
 
@@ -139,6 +140,7 @@ __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch
 __device__ __forceinline__ RowCfg row_cfg(const BatchArgs &a, int r) {
     RowCfg c;
     c.status = 0;
+    c.late = false;
     c.q = a.slot ? a.slot[r] : r;
     c.lrow = a.rows ? (long long)a.rows[r] : (long long)r;
     const bool idx_ok = (!a.slot || (c.q >= 0 && (a.n_slots <= 0 || c.q < a.n_slots))) &&
@@ -183,7 +185,25 @@ __device__ __forceinline__ RowCfg row_cfg(const BatchArgs &a, int r) {
     return c;
 }
 
-// The end of every row, one thread: the answer, then `_took` (sample.mojo:361-363).
+// `_took` (sample.mojo:361-363), one thread: the picked token into the slot's window, the draw counter on.
+__device__ __noinline__ void took_row(const BatchArgs &a, int r, const RowCfg &c, int token) {
+    if (!a.ring || token < 0) return;
+    // (all loads before the stores: one round trip instead of four)
+    const bool seen = c.ring_n > 0;
+    const int q = c.q, hd = seen ? a.ring_head[q] : 0, f = seen ? a.ring_filled[q] : 0;
+    const unsigned long long dn = a.drawn_rw[q];
+    const long long stop = a.stopped && a.stop_token ? a.stop_token[q] : -1ll;
+    if (seen) {  // `observe` (:246-258)
+        const int at = (hd >= 0 && hd < c.ring_n) ? hd : 0;
+        a.ring[(size_t)q * (size_t)a.ring_cap + at] = (long long)token;
+        a.ring_head[q] = (at + 1) % c.ring_n;
+        a.ring_filled[q] = f < c.ring_n ? f + 1 : c.ring_n;
+    }
+    a.drawn_rw[q] = dn + 1ull;
+    if (a.stopped) a.stopped[r] = (a.stop_token && stop == (long long)token) ? 1 : 0;
+}
+
+// The end of every row, one thread: the answer, then `_took`.
 __device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
                            float dtarget, float dp) {
     if (status & 0x80000000u) {  // a stale index
@@ -191,23 +211,9 @@ __device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg 
         return;
     }
     if (status & (MOLLA_ROW_LOAD_TIMEOUT | MOLLA_ROW_DEGENERATE | MOLLA_ROW_INVALID_CONFIG | MOLLA_ROW_UNSUPPORTED | MOLLA_ROW_EMPTY)) token = -1;
-    // (all loads before the stores: one round trip instead of four)
-    const bool took = a.ring && token >= 0, seen = took && c.ring_n > 0;
-    const int q = c.q, hd = seen ? a.ring_head[q] : 0, f = seen ? a.ring_filled[q] : 0;
-    const unsigned long long dn = took ? a.drawn_rw[q] : 0ull;
-    const long long stop = took && a.stopped && a.stop_token ? a.stop_token[q] : -1ll;
     a.tokens[r] = token;
     a.row_status[r] = status;
-    if (took) {
-        if (seen) {  // `observe` (:246-258)
-            const int at = (hd >= 0 && hd < c.ring_n) ? hd : 0;
-            a.ring[(size_t)q * (size_t)a.ring_cap + at] = (long long)token;
-            a.ring_head[q] = (at + 1) % c.ring_n;
-            a.ring_filled[q] = f < c.ring_n ? f + 1 : c.ring_n;
-        }
-        a.drawn_rw[q] = dn + 1ull;
-        if (a.stopped) a.stopped[r] = (a.stop_token && stop == (long long)token) ? 1 : 0;
-    }
+    if (!c.late) took_row(a, r, c, token);
     if (a.diag) { a.diag[4 * r] = dZ; a.diag[4 * r + 1] = dsum; a.diag[4 * r + 2] = dtarget; a.diag[4 * r + 3] = dp; }
 }
 
@@ -689,6 +695,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         // (too few lanes to bound the head: row_finish narrows it down from the list)
         pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
                    ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
+        pl.c.late = jump;
         pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
         pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
         store_plan(A, rr, pl);
@@ -3292,8 +3299,10 @@ __global__ void __launch_bounds__(NT, 1) row_tail_kernel(const __grid_constant__
         if (R.head(rr)->state != ST_DONE) tail_row(R, rr);
         __syncthreads();
         if (R.head(rr)->plan.flags & F_JUMP) {
+            // (with the window that the row was sampled with: the token goes into it afterwards)
             jump_status(R, rr);
             __syncthreads();
+            if (threadIdx.x == 0) { const int r = R.r0 + rr; took_row(R.a, r, R.head(rr)->plan.c, R.a.tokens[r]); }
         }
     }
 }

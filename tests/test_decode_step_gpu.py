@@ -166,3 +166,36 @@ def test_a_wait_that_ran_out_fails_the_row_and_keeps_its_state(dev, lib):
     torch.cuda.synchronize()
     assert not np.any(got["row_status"].cpu().numpy().astype(np.uint32) & capi.ROW_ERROR_BITS)
     assert np.all(ds.drawn.cpu().numpy() == 1)
+
+
+def test_status_words_follow_the_window_the_row_was_sampled_with(dev, lib):
+    """Rows whose running sum jumps (2^-48 before the largest term) are looked at once more after their token is
+    known, for MOLLA_ROW_SLOW_PATH. The window is full and holds one token, which the answer replaces: it is
+    ten above everything else unless its penalty is taken off. The same rows with their windows as lists, which no
+    call writes to, say what the status words are."""
+    B, V = 256, 8192   # (more rows than the chip holds clusters: the tile kernels)
+    rng = np.random.default_rng(11)
+    x = rng.uniform(-47.0, -40.0, (B, V)).astype(np.float32)
+    top = rng.integers(V // 4, V, B)
+    old = rng.integers(0, V // 4, B)
+    x[np.arange(B), top] = 0.0
+    x[np.arange(B), old] = 10.0
+    logits = torch.from_numpy(x).to(dev)
+    ds = S.DeviceSamplers(B, V, ring_cap=1, device=dev)
+    for r in range(B):
+        ds.assign(r, S.SamplerConfig(temperature=1.0, top_k=[40, 0, 0][r % 3], top_p=[0.9, 1.0, 0.999][r % 3],
+                                     presence_penalty=60.0, repeat_last_n=1, seed=r))
+    ds.ring.copy_(torch.from_numpy(old[:, None]))
+    ds.ring_filled.fill_(1)
+    p = dict(temperature=ds.temperature, top_k=ds.top_k, top_p=ds.top_p, presence_penalty=ds.presence_penalty, seed=ds.seed,
+             hist=torch.from_numpy(old).to(dev), hist_off=torch.arange(B + 1, dtype=torch.int32, device=dev))
+    ref = S.sample_batch(logits, p)
+    got = ds.step(logits, None, None)
+    torch.cuda.synchronize()
+    st = ref["row_status"].cpu().numpy()
+    slow = int(((st & capi.ROW_SLOW_PATH) != 0).sum())
+    assert 4 <= slow < B and not np.any(st & capi.ROW_ERROR_BITS), slow
+    assert np.array_equal(got["row_status"].cpu().numpy(), st)
+    assert torch.equal(got["tokens"], ref["tokens"])
+    # and the state has moved on
+    assert torch.equal(ds.ring[:, 0], got["tokens"].long()) and bool((ds.drawn == 1).all()) and bool((ds.ring_filled == 1).all())
