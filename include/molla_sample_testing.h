@@ -1,7 +1,7 @@
 /* Testing aids of libmolla_sample_testing.so: the same library compiled with
  * -DMOLLA_SAMPLE_TESTING. None of them has a counterpart in the reference, and none exists in
  * libmolla_sample.so: the production kernels carry no profiling stamps and take no experiment
- * switches. The three switches are process-wide and not thread-safe: set, call, reset. */
+ * switches. The switches are process-wide and not thread-safe: set, call, reset. */
 #ifndef MOLLA_SAMPLE_TESTING_H
 #define MOLLA_SAMPLE_TESTING_H
 
@@ -11,7 +11,8 @@
 extern "C" {
 #endif
 
-/* Experiment switches of the row kernels. Streaming kernel: bit 1 no last-use hint on the second
+/* Experiment switches of the row kernels. The ordinary entry points: bit 32 sends all rows through the tile
+ * kernels, bit 64 all rows that fit a thread-block cluster (V <= 307200) through the cluster kernel. Streaming kernel: bit 1 no last-use hint on the second
  * pass over a row, bit 2 no keep hint on list traffic. All of them: bit 4 pretends, after the row has arrived, that one warp's bounded wait ran out
  * (nothing is withheld and nothing is left waiting): the row must come back with
  * MOLLA_ROW_LOAD_TIMEOUT, token -1 and its sampler state untouched. 0 = production behaviour. */
@@ -25,6 +26,10 @@ void molla_sample_debug_profile(void *d_stamps);
  * 1 < top_k < 128, the ids that survive top-k (`_top_k`, sample.mojo:485-490) in descending
  * probability, padded with -1 (NULL switches it off again). */
 void molla_sample_debug_topk(void *d_ids, int32_t cap);
+
+/* How often the ordinary entry points launched the cluster kernel (counts[0]) and the tile kernels
+ * (counts[1]) since the last call of this function. */
+void molla_sample_debug_launches(int64_t *counts);
 
 #ifdef __cplusplus
 }

@@ -40,7 +40,7 @@ EXPORTS = (
     "molla_sample_nccl_unique_id", "molla_sample_nccl_comm_create", "molla_sample_nccl_comm_destroy",
     "molla_sample_sharded_last_error", "molla_sample_sharded_workspace_bytes", "molla_sample_sharded_step",
 )
-TESTING_EXPORTS = ("molla_sample_debug_knobs", "molla_sample_debug_profile", "molla_sample_debug_topk")
+TESTING_EXPORTS = ("molla_sample_debug_knobs", "molla_sample_debug_profile", "molla_sample_debug_topk", "molla_sample_debug_launches")
 TESTING_LIB_PATH = os.path.join(_HERE, "lib", "libmolla_sample_testing.so")
 
 
@@ -153,6 +153,8 @@ def _load(path, testing):
         L.molla_sample_debug_profile.argtypes = [vp]
         L.molla_sample_debug_topk.restype = None
         L.molla_sample_debug_topk.argtypes = [vp, i32]
+        L.molla_sample_debug_launches.restype = None
+        L.molla_sample_debug_launches.argtypes = [C.POINTER(i64)]
     return L
 
 

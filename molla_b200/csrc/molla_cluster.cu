@@ -1454,11 +1454,11 @@ bool cluster_fits(int dev, int G) {
 // 80 for walks, of up to 73000 logits (the tile kernels: 29, 36 to 47, 90 to 150). A second round of
 // clusters doubles that and the tile kernels pass it: 128 rows of 73000 with a top-k 62 against 97 us,
 // with a top-k of 1024 85 against 430.
-bool molla_cluster_better(int V, int B) {
+bool molla_cluster_better(int V, int B, int call_B) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const ClusterShape cs = cluster_shape(V, B, sms);
+    const ClusterShape cs = cluster_shape(V, call_B, sms);
     return cs.G != 0 && (long long)B * cs.G * 9 <= (long long)sms * 8 && cluster_fits(dev, cs.G);
 }
 

@@ -6,8 +6,8 @@
 
 struct BatchArgs;
 
-// Whether B rows of V logits are better off there than in the tile kernels.
-bool molla_cluster_better(int V, int B);
+// Whether B rows of V logits, of a call of `call_B`, are better off there than in the tile kernels.
+bool molla_cluster_better(int V, int B, int call_B);
 
 // Enqueues the sampling of `a.B` rows, for which molla_cluster_better holds, on `st`. Returns MOLLA_OK or
 // a MOLLA_ERR_* code with its message in `err`.

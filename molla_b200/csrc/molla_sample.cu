@@ -1672,6 +1672,7 @@ long long *g_prof = nullptr;
 int g_knobs = 0;
 int *g_topk = nullptr;
 int g_topk_cap = 0;
+int64_t g_launched[2] = {0, 0};   // launches of the cluster kernel and of the tile kernels
 #define MOLLA_SET_TESTING_ARGS(a) do { (a).prof = g_prof; (a).knobs = g_knobs; (a).topk_out = g_topk; (a).topk_cap = g_topk_cap; } while (0)
 #else
 #define MOLLA_SET_TESTING_ARGS(a) do { } while (0)
@@ -1738,11 +1739,23 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
     return MOLLA_OK;
 }
 
+// Which of the two the rows of a launch go through (the testing build can ask for either).
+bool takes_clusters(const BatchArgs &a) {
+    const int call = a.layout_B > 0 ? a.layout_B : a.B;
+    if (MOLLA_KNOB(a, 32)) return false;
+    if (MOLLA_KNOB(a, 64)) return molla_cluster_better(a.V, 1, call);
+    return molla_cluster_better(a.V, call, call);
+}
+
 // The ordinary entry points' launch.
 int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
-    if (molla_cluster_better(a.V, a.layout_B > 0 ? a.layout_B : a.B)) return molla_cluster_launch(a, st, g_err, sizeof(g_err));
+    const bool clusters = takes_clusters(a);
+#ifdef MOLLA_SAMPLE_TESTING
+    g_launched[clusters ? 0 : 1]++;
+#endif
+    if (clusters) return molla_cluster_launch(a, st, g_err, sizeof(g_err));
     return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err));
 }
 
@@ -2450,6 +2463,9 @@ int32_t molla_sample_logf(const float *d_x, int64_t n, void *stream, float *d_ou
 void molla_sample_debug_profile(void *d_stamps) { g_prof = (long long *)d_stamps; }
 void molla_sample_debug_knobs(int32_t k) { g_knobs = k; }
 void molla_sample_debug_topk(void *d_ids, int32_t cap) { g_topk = (int *)d_ids; g_topk_cap = d_ids ? cap : 0; }
+void molla_sample_debug_launches(int64_t *counts) {
+    for (int i = 0; i < 2; i++) { counts[i] = g_launched[i]; g_launched[i] = 0; }
+}
 #endif
 
 int32_t molla_sample_sync(void *stream) {

@@ -40,3 +40,27 @@ def dev():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     return torch.device("cuda:0")
+
+
+@pytest.fixture(params=["chosen", "tiles", "clusters"])
+def route(request, lib, dev):
+    """Which row kernels a test's calls go through: those that the library chooses for their size, or one and
+    the same kind for all of them. The latter takes the testing build, which counts its launches: a test that did
+    not run what its name says fails."""
+    if request.param == "chosen":
+        yield request.param
+        return
+    import ctypes as C
+    from helpers import ROUTES
+    from molla_b200 import capi
+    counts = (C.c_int64 * 2)()
+    with capi.testing_library() as T:
+        T.molla_sample_debug_launches(counts)
+        T.molla_sample_debug_knobs(ROUTES[request.param])
+        try:
+            yield request.param
+        finally:
+            T.molla_sample_debug_knobs(0)
+            T.molla_sample_debug_launches(counts)
+    cluster, tiles = counts
+    assert (cluster > 0, tiles > 0) == (request.param == "clusters", request.param == "tiles"), (cluster, tiles)

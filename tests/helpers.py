@@ -4,6 +4,8 @@ from __future__ import annotations
 
 import numpy as np
 
+ROUTES = {"tiles": 32, "clusters": 64}   # the switches of include/molla_sample_testing.h
+
 
 class OracleSampler:
     """`Sampler` of src/molla/engine/sample.mojo over the C oracle: keeps the ring window

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import OracleSampler
+from helpers import ROUTES, OracleSampler
 from molla_b200 import capi, sampler as S
 
 pytestmark = pytest.mark.gpu
@@ -42,6 +42,7 @@ def make(dev, oracle, V, ring_cap):
     return ds, host
 
 
+@pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("softcap", [0.0, 30.0])
 def test_decode_steps_match_host_kept_samplers(dev, lib, oracle, softcap):
     V, ring_cap, n_block = 3000, 16, 14
@@ -80,6 +81,7 @@ def test_decode_steps_match_host_kept_samplers(dev, lib, oracle, softcap):
             assert ring[slot, : h.filled].tolist() == h.recent[: h.filled]
 
 
+@pytest.mark.usefixtures("route")
 def test_softcap_alone_is_bit_identical_to_the_oracle(dev, lib, oracle):
     """Penalised-value dump of a capped row = oracle softcap of the row (no penalties, no bias)."""
     V = 5000
@@ -110,6 +112,7 @@ def test_bad_arguments_are_refused_before_any_launch(dev, lib):
         ds.step(torch.zeros((2, 100), device=dev), None, None, final_softcap=-1.0)
 
 
+@pytest.mark.usefixtures("route")
 def test_stale_row_and_slot_indices_touch_nothing(dev, lib):
     """`pick` refuses a row outside the block (sample.mojo:316-322). The device form reports such a
     row (and a slot outside the samplers) in its status word and reads and writes nothing of it.
@@ -138,7 +141,8 @@ def test_stale_row_and_slot_indices_touch_nothing(dev, lib):
     assert np.all(got["top_ids"].cpu().numpy()[[1, 3]] == -1)
 
 
-def test_a_wait_that_ran_out_fails_the_row_and_keeps_its_state(dev, lib):
+@pytest.mark.parametrize("switch", [0, ROUTES["tiles"], ROUTES["clusters"]])
+def test_a_wait_that_ran_out_fails_the_row_and_keeps_its_state(dev, lib, switch):
     """The bounded wait on a row's load reports in one warp only. The testing build can pretend
     that it ran out (nothing is withheld, nothing is left waiting): every such row must come back
     with MOLLA_ROW_LOAD_TIMEOUT and token -1, and the sampler in its slot must be as it was."""
@@ -150,7 +154,7 @@ def test_a_wait_that_ran_out_fails_the_row_and_keeps_its_state(dev, lib):
     block = torch.randn((4, V), device=dev)
     before = {k: getattr(ds, k).clone() for k in ("drawn", "ring", "ring_head", "ring_filled")}
     with capi.testing_library() as T:
-        T.molla_sample_debug_knobs(16)
+        T.molla_sample_debug_knobs(16 | switch)
         try:
             got = ds.step(block, None, None)
             torch.cuda.synchronize()

@@ -110,6 +110,7 @@ def test_logf_is_bit_identical_to_the_oracle(dev, lib, oracle):
 
 # ---- golden vectors ------------------------------------------------------------------------
 
+@pytest.mark.usefixtures("route")
 def test_golden_vectors(dev, lib, golden):
     for name in golden["names"]:
         w, c = golden_as_batch(golden, str(name))
@@ -229,6 +230,7 @@ def test_reference_properties(dev, lib):
     assert gpu_reachable(dev, [1.0] * V, 400, temperature=1.0, seed=17, min_p=0.9) == V
 
 
+@pytest.mark.usefixtures("route")
 def test_device_argmax_cases(dev, lib):
     """tests/test_gpu_ops.mojo:365-407: planted maximum, all-equal tie, all-negative row."""
     x = np.array([(i * 37 % 101) * 0.01 for i in range(777)], np.float32)
@@ -240,6 +242,7 @@ def test_device_argmax_cases(dev, lib):
     assert got["tokens"].tolist() == [513, 0, int(np.argmax(neg))]
 
 
+@pytest.mark.usefixtures("route")
 def test_min_p_against_the_oracle(dev, lib, oracle):
     """sample.mojo:508-523 after every combination of the earlier filters, vocabulary order included."""
     B = 96
@@ -261,6 +264,7 @@ def test_min_p_against_the_oracle(dev, lib, oracle):
     compare(w, dev, oracle, "min_p long", max_exception_frac=0.2)
 
 
+@pytest.mark.usefixtures("route")
 def test_typical_p_against_the_oracle(dev, lib, oracle):
     """sample.mojo:525-567 on the set top-k / top-p / min-p left, when that set lies in the sorted head."""
     B = 96
@@ -295,6 +299,7 @@ def test_typical_p_against_the_oracle(dev, lib, oracle):
     assert np.all(got["row_status"] & np.uint32(capi.ROW_UNSUPPORTED)) and np.all(got["tokens"] == -1)
 
 
+@pytest.mark.usefixtures("route")
 def test_top_k_around_the_sorted_head_limits(dev, lib, oracle):
     """A top-k up to 1025 is answered from the sorted head, a larger one by the walk past it: the values
     on both sides of the limits (128 in the streaming kernel, 1026 candidates in the cluster kernel)."""
@@ -307,19 +312,20 @@ def test_top_k_around_the_sorted_head_limits(dev, lib, oracle):
     compare(w, dev, oracle, "top-k around the head's limits", max_exception_frac=0.2)
 
 
+@pytest.mark.usefixtures("route")
 def test_long_lists_shared_with_idle_blocks(dev, lib, oracle):
-    """Rows whose list is most of the vocabulary next to rows that finish at once: the blocks of the
-    latter take segments of the former's list passes. Results must not depend on who did what."""
+    """Rows whose list is most of the vocabulary next to rows that finish at once: the tiles of the former are
+    spread over blocks in any order. Results must not depend on who did what."""
     B = 48
     w = W.config3(seed=41, B=B, V=151936, H=32)
     hot = np.arange(B) % 2 == 0
     w["temperature"][hot] = np.float32(1.25) + np.float32(0.01) * np.arange(hot.sum(), dtype=np.float32)
     w["top_k"][hot] = 0
     w["top_p"][hot] = np.float32([0.8, 0.95, 0.99, 0.999] * (hot.sum() // 4))
-    w["temperature"][~hot] = 0.0     # greedy: done after one pass, then helping
+    w["temperature"][~hot] = 0.0     # greedy: done after one pass
     r = compare(w, dev, oracle, "shared list passes", max_exception_frac=0.2)
     assert r["rows"] == B
-    # the same rows twice in a row give the same answers (who helps whom differs from run to run)
+    # the same rows twice in a row give the same answers (which block takes which tile differs from run to run)
     a = run_gpu(w, dev)
     b = run_gpu(w, dev)
     assert np.array_equal(a["tokens"], b["tokens"]) and np.array_equal(a["row_status"], b["row_status"])
@@ -392,17 +398,20 @@ def test_topk_sets_are_bit_exact(dev, lib, oracle):
 
 # ---- edge cases ---------------------------------------------------------------------------------
 
+@pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("V", [5, 33, 1000, 11264, 11265, 22529, 32000])
 def test_vocabulary_sizes_and_tile_edges(dev, lib, oracle, V):
     compare(W.config3(seed=100 + V, B=24, V=V, H=16), dev, oracle, f"V={V}", max_exception_frac=0.2)
 
 
+@pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("stride_pad,offset", [(1, 0), (3, 1), (4, 2), (0, 3)])
 def test_unaligned_rows(dev, lib, oracle, stride_pad, offset):
     w = W.config3(seed=7, B=12, V=12001, H=32)
     compare(w, dev, oracle, "unaligned", stride=12001 + stride_pad, offset=offset, max_exception_frac=0.2)
 
 
+@pytest.mark.usefixtures("route")
 def test_extremes(dev, lib, oracle):
     V = 4096
     rng = np.random.default_rng(3)
@@ -441,6 +450,7 @@ def test_extremes(dev, lib, oracle):
     assert np.array_equal(got["diag"][sampled, 0].view(np.uint32), ref["z_sum"][sampled].view(np.uint32))
 
 
+@pytest.mark.usefixtures("route")
 def test_invalid_and_unsupported_rows_are_reported_not_run(dev, lib):
     V = 64
     w = W._base(6, V, 0)
@@ -459,6 +469,7 @@ def test_invalid_and_unsupported_rows_are_reported_not_run(dev, lib):
     assert st[5] == 0 and got["tokens"][5] == V - 1  # greedy ignores min_p, as the reference does
 
 
+@pytest.mark.usefixtures("route")
 def test_window_edge_cases(dev, lib, oracle):
     V = 2000
     w = W.config3(seed=11, B=8, V=V, H=40)
@@ -529,6 +540,7 @@ def test_host_buffer_entry_matches_device_entry(dev, lib):
         assert np.array_equal(hb.top_ids.numpy(), got["top_ids"])
 
 
+@pytest.mark.usefixtures("route")
 def test_grammar_mask_against_the_oracle(dev, lib, oracle):
     """`_mask` (sample.mojo:371-379): tokens a grammar forbids are dropped ahead of every other
     filter. Dense and sparse masks, masks that hide the maximum, bias and penalties on hidden

@@ -1,4 +1,5 @@
-"""The tile kernels at the sizes where they can go wrong, against the CPU oracle."""
+"""The row kernels at the sizes where they can go wrong, against the CPU oracle: as the library chooses
+between them, and all sizes through the tile kernels and through the cluster kernel."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,7 @@ from helpers import OracleSampler
 from molla_b200 import sampler as S, workloads as W
 from test_parity_gpu import compare
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("route")]
 
 
 def _kinds(w, B, V):
