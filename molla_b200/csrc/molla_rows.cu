@@ -846,8 +846,9 @@ struct TileEval { int total; unsigned int keep; };
 // The exponentials (temperature and softmax numerator, sample.mojo:419-434) of a tile's logits that
 // reach `thr`, packed into the tile's list (over the logits: entry e never lies behind a logit that is
 // still to be read). The warp first lists what is kept and then evaluates it in full warps, two of them
-// at a time; a tile that keeps three quarters and more keeps all (a value too small to matter adds
-// nothing). `idx` holds 1024 positions.
+// at a time (take(value's bits, entry) by the lane that evaluates it, entry % 32); a tile that keeps three
+// quarters and more keeps all, and no other has 1024 entries (a value too small to matter adds nothing).
+// `idx` holds 1024 positions.
 template <class TAKE>
 __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, float thr, float T, float rT, float top, bool fast, TAKE take) {
     const int lane = threadIdx.x & 31;
@@ -885,8 +886,8 @@ __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, 
         const float x = tile[p + 4 * (p >> 5)], y = tile[q + 4 * (q >> 5)];
         const float ex = value(x), ey = value(y);
         __syncwarp();
-        if (i < r.total) { tile[skew(i)] = ex; take(__float_as_uint(ex), p); }
-        if (j < r.total) { tile[skew(j)] = ey; take(__float_as_uint(ey), q); }
+        if (i < r.total) { tile[skew(i)] = ex; take(__float_as_uint(ex), i); }
+        if (j < r.total) { tile[skew(j)] = ey; take(__float_as_uint(ey), j); }
         __syncwarp();
     }
     return r;
@@ -923,15 +924,25 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     const TilePlan tp = A.tp[gt];
     float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = pl.tau_bits;
-    unsigned long long *cand = A.cand(rr);
-    const TileEval t = tile_eval(list, reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top,
-        (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
-        [&](unsigned int eb, int i) {
-            if (eb >= tau) {
-                const int pos = atomicAdd(&head->ncand, 1);
-                if (pos < HEADCAP) cand[pos] = make_key(eb, tile * TILE + i);
-            }
-        });
+    unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
+    unsigned int wanted = 0u;   // this lane's candidates among the entries it evaluates
+    const TileEval t = tile_eval(list, idx, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
+        [&](unsigned int eb, int e) { wanted |= (eb >= tau ? 1u : 0u) << (e >> 5); });
+    // A tile asks for its candidates' places once. (One request per value, each waited for before the next two
+    // are evaluated, took 0.7 us each: up to 22 us a tile in short rows, whose few tiles hold all candidates.)
+    const unsigned int any = __reduce_or_sync(0xffffffffu, wanted);
+    if (any) {
+        unsigned long long *cand = A.cand(rr);
+        const int n = __popc(wanted), inc = warp_incl_scan(n, lane);
+        int pos = 0;
+        if (lane == 31) pos = atomicAdd(&head->ncand, inc);
+        pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
+#pragma unroll 1
+        for (; wanted; wanted &= wanted - 1u, pos++) {
+            const int e = (__ffs((int)wanted) - 1) * 32 + lane;
+            if (pos < HEADCAP) cand[pos] = make_key(__float_as_uint(list[skew(e)]), tile * TILE + (t.total == TILE ? e : (int)idx[e]));
+        }
+    }
     const TileChunk ch = tile_chunk(list, t.total);
     bool care;
     int my_place, c0 = CARE_PLACES;
