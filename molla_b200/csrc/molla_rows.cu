@@ -105,7 +105,7 @@ constexpr int PICKS = 8, PICK_CAP = NC;
 struct __align__(16) WalkPicks { int n, arrived, pad[2]; int bin[PICKS]; int cnt[PICKS]; };
 constexpr size_t WALK_BYTES = WALK_BINADES * (NBINS * sizeof(unsigned long long) + sizeof(WalkTies)) + sizeof(WalkPicks) + (size_t)PICKS * PICK_CAP * sizeof(unsigned long long);
 
-struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; int pad[4]; };
+struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; unsigned int hits[4]; };   // hits: see F_JUMP
 
 struct RowsArgs {
     BatchArgs a;
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
 // Kernel 2: one block per row. Bound: latency (two rounds of loads, one histogram, code that runs once):
 // 7 to 10 us for up to 148 rows, 13 for 256, 22 for 512.
 // =============================================================================
-struct JumpShared { float in[128], over[128], own[128], pref[128]; int hit[128]; };
+struct JumpShared { float in[128], over[128], own[128]; unsigned int hits[4]; };
 struct PlanShared {
     union { unsigned int hist[PLAN_BINS]; JumpShared jump; };
     int edge;
@@ -478,7 +478,7 @@ __device__ __forceinline__ float block_excl_scan_plus(float v, float *ws, float 
 // sum is more than 2^40 times everything before it, too few bits are left of what came before. This finds the
 // groups where that may be: the estimated sum of their tiles
 // against the largest term before them. Only sharp rows (low temperatures) have one.
-// Block of NT threads, 4 to a group; hit[q] is set for group q (block q / 16 of the layout, warp q % 16).
+// Block of NT threads, 4 to a group; bit q of J.hits is set for group q (block q / 16 of the layout, warp q % 16).
 __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, float xmax, JumpShared &J) {
     const int tid = threadIdx.x, lane = tid & 31, q = tid >> 2, part = tid & 3, g = q >> 4, w = q & 15, V = A.a.V;
     const float *gm = A.gmax + (size_t)rr * A.ntile * 32;
@@ -506,7 +506,7 @@ __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, floa
                     for (int k = max(t * 32, a >> 5); k < min(t * 32 + 32, ((b - 1) >> 5) + 1); k++) own += 32.0f * ex2_approx(fminf((gm[k] - over) * f, 0.0f));
                 } else if (st.tmax > -INFINITY) own += st.tsum * ex2_approx((st.tmax - over) * f);
             }
-        J.in[q] = in; J.over[q] = over; J.own[q] = log2f(fminf(own, (float)(b - a))); J.hit[q] = 0;
+        J.in[q] = in; J.over[q] = over; J.own[q] = log2f(fminf(own, (float)(b - a)));
     }
     __syncthreads();
     bool any = false;
@@ -516,10 +516,10 @@ __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, floa
         for (int o = 1; o < 32; o <<= 1) { const float v = __shfl_up_sync(0xffffffffu, pf, o); if (lane >= o) pf = fmaxf(pf, v); }
 #pragma unroll 4
         for (int i = 0; i < (tid & ~31); i++) pf = fmaxf(pf, J.in[i]);
-        J.pref[tid] = pf;
         // (e^-105 and less is zero)
         any = (tid & 15) != 0 && J.over[tid] > -INFINITY && pf > -INFINITY && (J.over[tid] - pf) * f + J.own[tid] > 39.9f && (xmax - pf) * f < 152.0f;
-        J.hit[tid] = any ? 1 : 0;
+        const unsigned int m = __ballot_sync(0xffffffffu, any);
+        if (lane == 0) J.hits[tid >> 5] = m;
     }
     return __syncthreads_or(any) != 0;
 }
@@ -680,6 +680,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     if (A.oG > 0 && !((xmax - first) * f <= 29.0f)) {
         __syncthreads();
         jump = find_jumps(A, rr, f, xmax, S.jump);
+        if (jump && tid < 4) A.head(rr)->hits[tid] = S.jump.hits[tid];
     }
     const float tv = (c.T == 1.0f) ? tau_x : __fdiv_rn(tau_x, c.T);
     const unsigned int tb = c.pure ? 0xffffffffu : __float_as_uint(expf_pinned(__fsub_rn(tv, top)));
@@ -3185,117 +3186,144 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
 
 // A row that find_jumps has marked: is a guess of its sum's binade wrong? Every marked group's guesses are
 // made here as they would be made from that prefix, and held against the sum before them (in double precision,
-// added without a subtraction). Pure rows add up twice, exponentials and then probabilities.
+// added without a subtraction). Pure rows add up twice, exponentials and then probabilities. Bound: latency of code
+// that runs once. What comes before is row_plan's estimate but for the tiles that the block and the group
+// begin in, so a group takes one or two stretches of logits, evaluated by the whole block; each lane's range is
+// added up by four threads. (With whole spans, and a thread for 32 logits or a range, a group took 20 to 45 us:
+// row_tail of 160 mixed rows of 2000 31 us where this takes 14, of 256 rows of 151936 76 where this takes 49.)
+struct JumpWork { double sum[4][NWARP]; float csum[32]; int jl[32]; int flags[32]; };
+static_assert(sizeof(JumpWork) <= ITEM_CAP * sizeof(Item), "the work on a jump uses the items' space");
 __device__ __noinline__ void jump_status(const RowsArgs &R, int rr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     AuxF *A = reinterpret_cast<AuxF *>(smem_raw);
-    JumpShared &J = *reinterpret_cast<JumpShared *>(A->items);
-    static_assert(sizeof(JumpShared) <= sizeof(A->items), "the groups' maxima use the items' space");
+    JumpWork &W = *reinterpret_cast<JumpWork *>(A->items);
     const RowHead *head = R.head(rr);
     const RowPlan pl = head->plan;
     const RowCfg &cfg = pl.c;
     const float T = cfg.T, Z = head->Z, f = fminf(1.44269504f / T, 1.0e30f);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = R.r0 + rr, L = R.oL;
-    float *list = R.elist + (size_t)rr * R.ntile * TILE;   // (the row is done: its list is free)
-    unsigned int minp = 0u;
-    if (cfg.minp > 0.0f) minp = __float_as_uint(__fmul_rn(__fdiv_rn(expf_pinned(__fsub_rn(pl.top, pl.top)), Z), cfg.minp));
+    const TilePlan *tp = R.tp + (size_t)rr * R.ntile;
+    float minp = 0.0f;   // (nobody's but a pure row's probabilities)
+    if (cfg.pure && cfg.minp > 0.0f) minp = __fmul_rn(__fdiv_rn(expf_pinned(__fsub_rn(pl.top, pl.top)), Z), cfg.minp);
     auto prob = [&](float e) -> float {
         const float p = __fdiv_rn(e, Z);
-        return __float_as_uint(p) < minp ? 0.0f : p;
+        return p < minp ? 0.0f : p;
     };
-    __syncthreads();
-    if (!find_jumps(R, rr, f, pl.xmax, J)) return;
+    const int npass = cfg.pure ? 2 : 1, nsum = minp > 0.0f ? 4 : 2;
     bool slow = false;
 #pragma unroll 1
-    for (int q = 1; q < 128 && !slow; q++) {
-        if (!J.hit[q]) continue;
+    for (int q = 0; q < 128 && !slow; q++) {
+        const unsigned int left_q = head->hits[q >> 5] >> (q & 31);
+        if (!left_q) { q |= 31; continue; }
+        q += __ffs((int)left_q) - 1;
         const int blk0 = (q >> 4) * R.oVc, e = min(R.a.V, blk0 + R.oVc), ga = blk0 + (q & 15) * 32 * L, gb = min(e, ga + 32 * L);
-        const float least = J.pref[q] - 40.0f / f;   // tiles below this are nothing beside what comes before the group
+        const int t0 = ga / TILE, tb = blk0 / TILE;
+        const bool split = tb < t0 && blk0 % TILE != 0;   // the block begins inside a tile before the group's
         double sum[4] = {0.0, 0.0, 0.0, 0.0};   // before the block, in the block before the group; of the probabilities
-        // What comes before is known from row_plan's estimates but for the spans that the block and the group
-        // begin in (unless min-p takes some of it away): three spans to look at where eighteen took 100 us.
-        const int s_b = blk0 / SPAN, s_g = ga / SPAN;
-        const bool known = minp == 0u;
-        if (known && tid == 0) {
-            const TilePlan *tp = R.tp + (size_t)rr * R.ntile;
-            constexpr int TPS = SPAN / TILE;
-            sum[0] = (double)tp[s_b * TPS].est;
-            if (s_g > s_b) sum[1] = (double)tp[s_g * TPS].est - (double)tp[(s_b + 1) * TPS].est;
-            sum[2] = sum[0] / (double)Z; sum[3] = sum[1] / (double)Z;
+        if (tid == 0) {
+            sum[0] = (double)tp[tb].est;
+            if (tb < t0) sum[1] = (double)tp[t0].est - (double)tp[tb + (split ? 1 : 0)].est;
         }
+        // the stretches [c0, c1): the block's first tile; where min-p takes something away, everything that it leaves; the group
+        const int stop = minp > 0.0f ? t0 * TILE : (split ? (tb + 1) * TILE : 0), step = minp > 0.0f ? SPAN : TILE;
+        int c0 = minp > 0.0f ? 0 : tb * TILE;
 #pragma unroll 1
-        for (int span = 0; span * SPAN < gb; span++) {
-            bool want = (span + 1) * SPAN > ga;
-            for (int t = 0; t < SPAN / TILE && !want; t++) want = R.ts[(size_t)rr * R.ntile + span * (SPAN / TILE) + t].tmax >= least;
-            if (known) want = span == s_b || span >= s_g;
-            if (!want) continue;
-            __syncthreads();
-            if (tid < SPAN_THREADS) span_fetch(R.a, cfg.lrow, span * SPAN, A->tile);
-            span_ready(R.a, cfg, r, span * SPAN, A->tile, reinterpret_cast<SpanScratch *>(A->tile + SPAN_THREADS * PITCH), tid < SPAN_THREADS);
-            if (tid < SPAN_THREADS)
+        for (bool last = false; !last;) {
+            last = c0 >= stop;
+            if (last) c0 = t0 * TILE;
+            const int c1 = last ? gb : min(c0 + step, stop);
+            bool want = last || (split && tb >= c0 / TILE && tb < (c1 + TILE - 1) / TILE);
+            for (int t = c0 / TILE; t * TILE < c1 && !want; t++)
+                want = ex2_approx((R.ts[(size_t)rr * R.ntile + t].tmax - pl.xmax) * f) >= 0.99f * minp * Z;
+            if (want) {
+                __syncthreads();
+                if (warp < SPAN / TILE && warp * TILE < c1 - c0) span_fetch(R.a, cfg.lrow, c0, A->tile);
+                span_ready(R.a, cfg, r, c0, A->tile, reinterpret_cast<SpanScratch *>(A->tile + SPAN_THREADS * PITCH), tid < SPAN_THREADS);
+                __syncthreads();
 #pragma unroll 1
-                for (int j = 0; j < 32; j++) {
-                    const int i = span * SPAN + tid * 32 + j;
-                    const float x = A->tile[tid * PITCH + j];
-                    if (i >= gb) break;
+                for (int i = tid; i < c1 - c0; i += NT) {
+                    float &x = A->tile[(i >> 5) * PITCH + (i & 31)];
                     const float ev = x > -INFINITY ? expf_pinned_nonpos(__fsub_rn(T == 1.0f ? x : div_slow(x, T), pl.top)) : 0.0f;
-                    if (i >= ga) list[i - ga] = ev;
-                    else if (ev != 0.0f) {
-                        sum[i < blk0 ? 0 : 1] += (double)ev;
-                        if (cfg.pure) sum[i < blk0 ? 2 : 3] += (double)prob(ev);
+                    x = ev;
+                    if (c0 + i < ga) {
+                        const bool own = c0 + i >= blk0;
+                        if (last || (c0 + i) / TILE == tb) sum[own ? 1 : 0] += (double)ev;
+                        if (minp > 0.0f) sum[own ? 3 : 2] += (double)prob(ev);
                     }
                 }
+            }
+            if (!last) c0 = c1;
         }
-        __syncthreads();
-        for (int i = tid; i < gb - ga; i += NT) A->tile[i] = list[i];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            double v = sum[k];
+#pragma unroll 1
+        for (int k = 0; k < nsum; k++) {
+            double v = k == 0 ? sum[0] : k == 1 ? sum[1] : k == 2 ? sum[2] : sum[3];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0 && warp < 8) A->wsd[k * 8 + warp] = v;
+            if (lane == 0) W.sum[k][warp] = v;
         }
         __syncthreads();
-        bool wrong = false;
-        if (warp == 0) {
 #pragma unroll 1
-            for (int pass = 0; pass < (cfg.pure ? 2 : 1); pass++) {
+        for (int pass = 0; pass < npass && !slow; pass++) {
+            // lane l's range is [i0, i1) of the group, added up four apart, what is left over with the first
+            const int n = gb - ga, l = (tid >> 2) & 31, part = tid & 3, i0 = min(n, l * L), i1 = min(n, i0 + L), n4 = (i1 - i0) & ~3;
+            auto val = [&](int i) { const int at = ga - c0 + i; const float v = A->tile[(at >> 5) * PITCH + (at & 31)]; return pass ? prob(v) : v; };
+            if (tid < 128) {
+                float c = 0.0f;
+#pragma unroll 1
+                for (int i = i0 + part; i < i1; i += i < i0 + n4 ? 4 : 1)
+                    if (i < i0 + n4 || part == 0) c = __fadd_rn(c, val(i));
+                c = __fadd_rn(c, __shfl_xor_sync(0xffffffffu, c, 1));
+                c = __fadd_rn(c, __shfl_xor_sync(0xffffffffu, c, 2));
+                if (part == 0) W.csum[l] = c;
+            }
+            __syncthreads();
+            double s0 = 0.0, s1 = 0.0;
+            if (warp == 0) {
                 double base = 0.0, before = 0.0;
-                for (int w = 0; w < 8; w++) { base += A->wsd[pass * 16 + w]; before += A->wsd[pass * 16 + 8 + w]; }
-                const int n = gb - ga, i0 = min(n, lane * L), i1 = min(n, i0 + L);
-                auto val = [&](int i) { return pass ? prob(A->tile[i]) : A->tile[i]; };
-                float c4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                const int k = pass && minp > 0.0f ? 2 : 0;
 #pragma unroll 1
-                for (int i = i0; i < i1; i++) { const int k = (i - i0) < ((i1 - i0) & ~3) ? (i - i0) & 3 : 0; const float v = val(i);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) if (k == u) c4[u] = __fadd_rn(c4[u], v); }
-                const float csum = __fadd_rn(__fadd_rn(c4[0], c4[1]), __fadd_rn(c4[2], c4[3]));
+                for (int w = 0; w < NWARP; w++) { base += W.sum[k][w]; before += W.sum[k + 1][w]; }
+                if (pass && !(minp > 0.0f)) { base /= (double)Z; before /= (double)Z; }
+                const float csum = W.csum[lane];
                 const double inc = warp_incl_scan((double)csum, lane), own = __shfl_sync(0xffffffffu, inc, 31);
                 double ex = __shfl_up_sync(0xffffffffu, inc, 1);
                 if (lane == 0) ex = 0.0;
                 const double left = (before + own) - own;   // what the subtraction leaves of `before`
                 const double sst = base + (left + (inc - (double)csum));
                 const float lo = (float)(sst * (1.0 - 1.0 / 4096.0)), hi = (float)((sst + (double)csum) * (1.0 + 1.0 / 4096.0));
-                if (!(lo > 0.0f) || csum == 0.0f) continue;
                 const int jl = fexpo(lo), j2 = fexpo(hi);
-                if (!(j2 <= jl + 1 && jl >= -100 && j2 <= 100)) continue;
-                const bool two = j2 == jl + 1;
-                bool bad = false, some = false;
-                const float C1 = __fmul_rn(1.5f, fpow2(jl)), C2 = __fmul_rn(1.5f, fpow2(jl + 1));
-#pragma unroll 1
-                for (int i = i0; i < i1; i++) {
-                    const float v = val(i);
-                    const float k1 = __fsub_rn(__fadd_rn(v, C1), C1), k2 = __fsub_rn(__fadd_rn(v, C2), C2);
-                    bad |= fabsf(__fsub_rn(v, k1)) == fpow2(jl - 24) || v >= fpow2(jl - 1) || (two && fabsf(__fsub_rn(v, k2)) == fpow2(jl - 23));
-                    some |= k1 != 0.0f || (two && k2 != 0.0f);
-                }
-                if (bad || !some) continue;
-                const double s0 = base + before + ex, s1 = s0 + (double)csum;
-                const int js = fexpo((float)s0);
-                const bool held = two ? (js == jl || js == jl + 1) && s1 < (double)fpow2(jl + 2) : js == jl && s1 < (double)fpow2(jl + 1);
-                wrong |= !held;
+                const bool guessed = lo > 0.0f && csum != 0.0f && j2 <= jl + 1 && jl >= -100 && j2 <= 100;
+                W.jl[lane] = jl;
+                W.flags[lane] = !guessed ? 0 : (j2 == jl + 1 ? 3 : 1);   // bit 0: there is a guess; bit 1: it spans two binades
+                s0 = base + before + ex;
+                s1 = s0 + (double)csum;
             }
+            __syncthreads();
+            if (tid < 128) {   // would the range go by itself in the guessed binades, and does it add anything?
+                const int jl = W.jl[l];
+                const bool guessed = W.flags[l] != 0, two = W.flags[l] == 3;
+                bool bad = false, some = false;
+                if (guessed) {
+                    const float C1 = __fmul_rn(1.5f, fpow2(jl)), C2 = __fmul_rn(1.5f, fpow2(jl + 1));
+#pragma unroll 1
+                    for (int i = i0 + part; i < i1; i += 4) {
+                        const float v = val(i);
+                        const float k1 = __fsub_rn(__fadd_rn(v, C1), C1), k2 = __fsub_rn(__fadd_rn(v, C2), C2);
+                        bad |= fabsf(__fsub_rn(v, k1)) == fpow2(jl - 24) || v >= fpow2(jl - 1) || (two && fabsf(__fsub_rn(v, k2)) == fpow2(jl - 23));
+                        some |= k1 != 0.0f || (two && k2 != 0.0f);
+                    }
+                }
+                const unsigned int four = 0xfu << (lane & ~3), bm = __ballot_sync(0xffffffffu, bad), sm = __ballot_sync(0xffffffffu, some);
+                if (part == 0 && ((bm & four) || !(sm & four))) W.flags[l] = 0;
+            }
+            __syncthreads();
+            bool wrong = false;
+            if (warp == 0 && W.flags[lane]) {
+                const int jl = W.jl[lane], js = fexpo((float)s0);
+                const bool held = W.flags[lane] == 3 ? (js == jl || js == jl + 1) && s1 < (double)fpow2(jl + 2) : js == jl && s1 < (double)fpow2(jl + 1);
+                wrong = !held;
+            }
+            slow = __syncthreads_or(wrong) != 0;
         }
-        slow = __syncthreads_or(wrong) != 0;
     }
     if (slow && tid == 0) R.a.row_status[r] |= MOLLA_ROW_SLOW_PATH;
 }
