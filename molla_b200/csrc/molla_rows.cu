@@ -186,7 +186,7 @@ __device__ __forceinline__ RowCfg row_cfg(const BatchArgs &a, int r) {
 }
 
 // `_took` (sample.mojo:361-363), one thread: the picked token into the slot's window, the draw counter on.
-__device__ __noinline__ void took_row(const BatchArgs &a, int r, const RowCfg &c, int token) {
+__device__ __forceinline__ void took_row(const BatchArgs &a, int r, const RowCfg &c, int token) {
     if (!a.ring || token < 0) return;
     // (all loads before the stores: one round trip instead of four)
     const bool seen = c.ring_n > 0;
@@ -203,18 +203,24 @@ __device__ __noinline__ void took_row(const BatchArgs &a, int r, const RowCfg &c
     if (a.stopped) a.stopped[r] = (a.stop_token && stop == (long long)token) ? 1 : 0;
 }
 
-// The end of every row, one thread: the answer, then `_took`.
-__device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
-                           float dtarget, float dp) {
+// A row's answer, one thread; returns the token, -1 where there is none.
+__device__ __forceinline__ int answer_row(const BatchArgs &a, int r, unsigned int status, int token, float dZ, float dsum, float dtarget, float dp) {
     if (status & 0x80000000u) {  // a stale index
         a.tokens[r] = -1; a.row_status[r] = status & 0x7fffffffu;
-        return;
+        return -1;
     }
     if (status & (MOLLA_ROW_LOAD_TIMEOUT | MOLLA_ROW_DEGENERATE | MOLLA_ROW_INVALID_CONFIG | MOLLA_ROW_UNSUPPORTED | MOLLA_ROW_EMPTY)) token = -1;
     a.tokens[r] = token;
     a.row_status[r] = status;
-    if (!c.late) took_row(a, r, c, token);
     if (a.diag) { a.diag[4 * r] = dZ; a.diag[4 * r + 1] = dsum; a.diag[4 * r + 2] = dtarget; a.diag[4 * r + 3] = dp; }
+    return token;
+}
+
+// The end of a row, one thread: the answer, then `_took`.
+__device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg &c, unsigned int status, int token, float dZ, float dsum,
+                           float dtarget, float dp) {
+    token = answer_row(a, r, status, token, dZ, dsum, dtarget, dp);
+    if (!c.late) took_row(a, r, c, token);
 }
 
 // ---- arithmetic -------------------------------------------------------------------------------
@@ -530,6 +536,10 @@ __device__ __forceinline__ void store_plan(const RowsArgs &A, int rr, const RowP
     h->ncand = 0; h->nitem = 0; h->ncare = 0; h->state = 0;
     if (rr == 0) A.queue[0] = 0;
 }
+__device__ __forceinline__ void store_done(const RowsArgs &A, int rr) {   // (nothing else of such a row is looked at)
+    A.head(rr)->plan.kind = PLAN_DONE;
+    if (rr == 0) A.queue[0] = 0;
+}
 
 __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ RowsArgs A) {
     __shared__ PlanShared S;
@@ -539,11 +549,8 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     pdl_wait();
     RowCfg c = row_cfg(a, r);
     if (MOLLA_KNOB(a, 16) && !c.status) c.status |= MOLLA_ROW_LOAD_TIMEOUT;  // testing build: a wait that ran out
-    RowPlan pl;
-    pl.c = c;
-    pl.kind = PLAN_DONE; pl.flags = 0; pl.top = 0; pl.tau_bits = 1u; pl.xmax = 0; pl.imax = 0; pl.need = 0; pl.pad = 0;
     if (c.status) {
-        if (tid == 0) { finish_row(a, r, c, c.status, -1, 0, 0, 0, 0); store_plan(A, rr, pl); }
+        if (tid == 0) { answer_row(a, r, c.status, -1, 0, 0, 0, 0); store_done(A, rr); }
         return;
     }
     // the maximum and its first index (kernel.mojo:571-585, sample.mojo:342-346)
@@ -584,7 +591,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         if (eq > 1) status |= MOLLA_ROW_TOPK_TIE;
     }
     if (done) {
-        if (tid == 0) { finish_row(a, r, c, status, imax, 0, 0, 0, 0); store_plan(A, rr, pl); }
+        if (tid == 0) { took_row(a, r, c, answer_row(a, r, status, imax, 0, 0, 0, 0)); store_done(A, rr); }
         return;
     }
     const float top = (c.T == 1.0f) ? xmax : __fdiv_rn(xmax, c.T);
@@ -691,7 +698,9 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         if (t < A.ntile) { TilePlan p; p.thr = fminf(thr_of(est[u]), tau_x); p.est = est[u]; tp[t] = p; }
     }
     if (tid == 0) {
-        pl.kind = PLAN_SAMPLED;
+        RowPlan pl;
+        pl.c = c;
+        pl.kind = PLAN_SAMPLED; pl.pad = 0;
         const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
         // (too few lanes to bound the head: row_finish narrows it down from the list)
         pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
