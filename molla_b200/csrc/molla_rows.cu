@@ -530,9 +530,10 @@ __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, floa
     return __syncthreads_or(any) != 0;
 }
 
-__device__ __forceinline__ void store_plan(const RowsArgs &A, int rr, const RowPlan &pl) {
+// (the settings as soon as the row is known to be sampled: they are not kept in registers to the end)
+__device__ __forceinline__ void store_settings(const RowsArgs &A, int rr, const RowCfg &c) {
     RowHead *h = A.head(rr);
-    h->plan = pl;
+    h->plan.c = c;
     h->ncand = 0; h->nitem = 0; h->ncare = 0; h->state = 0;
     if (rr == 0) A.queue[0] = 0;
 }
@@ -594,6 +595,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         if (tid == 0) { took_row(a, r, c, answer_row(a, r, status, imax, 0, 0, 0, 0)); store_done(A, rr); }
         return;
     }
+    if (tid == 0) store_settings(A, rr, c);
     const float top = (c.T == 1.0f) ? xmax : __fdiv_rn(xmax, c.T);
     const bool filter_ok = fabsf(top) < 1.0e5f;
     long long need = c.open_row ? (long long)HEAD_NEED : c.n_lim + 1;
@@ -698,17 +700,15 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         if (t < A.ntile) { TilePlan p; p.thr = fminf(thr_of(est[u]), tau_x); p.est = est[u]; tp[t] = p; }
     }
     if (tid == 0) {
-        RowPlan pl;
-        pl.c = c;
-        pl.kind = PLAN_SAMPLED; pl.pad = 0;
+        RowPlan &pl = A.head(rr)->plan;
+        pl.kind = PLAN_SAMPLED;
         const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
         // (too few lanes to bound the head: row_finish narrows it down from the list)
         pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
                    ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
-        pl.c.late = jump;
+        if (jump) pl.c.late = true;
         pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
         pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
-        store_plan(A, rr, pl);
     }
 }
 
@@ -856,9 +856,9 @@ struct TileEval { int total; unsigned int keep; };
 // The exponentials (temperature and softmax numerator, sample.mojo:419-434) of a tile's logits that
 // reach `thr`, packed into the tile's list (over the logits: entry e never lies behind a logit that is
 // still to be read). The warp first lists what is kept and then evaluates it in full warps, two of them
-// at a time (take(value's bits, entry) by the lane that evaluates it, entry % 32); a tile that keeps three
-// quarters and more keeps all, and no other has 1024 entries (a value too small to matter adds nothing).
-// `idx` holds 1024 positions.
+// at a time (take(value's bits, second of the two, bit of the time) by the lane that evaluates it); a tile that
+// keeps three quarters and more keeps all, and no other has 1024 entries (a value too small to matter adds
+// nothing). `idx` holds 1024 positions.
 template <class TAKE>
 __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, float thr, float T, float rT, float top, bool fast, TAKE take) {
     const int lane = threadIdx.x & 31;
@@ -889,15 +889,16 @@ __device__ __forceinline__ TileEval tile_eval(float *tile, unsigned short *idx, 
         const float v = one ? x : (fast ? div_by(fmaxf(x, -1.0e20f), T, rT) : div_slow(x, T));
         return expf_pinned_nonpos(__fsub_rn(v, top));  // no logit of the row exceeds its maximum
     };
+    unsigned int bit = 1u;
 #pragma unroll 1
-    for (int i0 = 0; i0 < r.total; i0 += 64) {
+    for (int i0 = 0; i0 < r.total; i0 += 64, bit <<= 1) {
         const int i = i0 + lane, j = i + 32;
         const int p = all ? i : (i < r.total ? (int)idx[i] : 0), q = all ? j : (j < r.total ? (int)idx[j] : 0);
         const float x = tile[p + 4 * (p >> 5)], y = tile[q + 4 * (q >> 5)];
         const float ex = value(x), ey = value(y);
         __syncwarp();
-        if (i < r.total) { tile[skew(i)] = ex; take(__float_as_uint(ex), i); }
-        if (j < r.total) { tile[skew(j)] = ey; take(__float_as_uint(ey), j); }
+        if (i < r.total) { tile[skew(i)] = ex; take(__float_as_uint(ex), false, bit); }
+        if (j < r.total) { tile[skew(j)] = ey; take(__float_as_uint(ey), true, bit); }
         __syncwarp();
     }
     return r;
@@ -935,13 +936,13 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = pl.tau_bits;
     unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
-    unsigned int wanted = 0u;   // this lane's candidates among the entries it evaluates
+    unsigned int w0 = 0u, w1 = 0u;   // this lane's candidates among the entries it evaluates
     const TileEval t = tile_eval(list, idx, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
-        [&](unsigned int eb, int e) { wanted |= (eb >= tau ? 1u : 0u) << (e >> 5); });
+        [&](unsigned int eb, bool second, unsigned int bit) { if (eb >= tau) { if (second) w1 |= bit; else w0 |= bit; } });
     // A tile asks for its candidates' places once. (One request per value, each waited for before the next two
     // are evaluated, took 0.7 us each: up to 22 us a tile in short rows, whose few tiles hold all candidates.)
-    const unsigned int any = __reduce_or_sync(0xffffffffu, wanted);
-    if (any) {
+    unsigned int wanted = w0 | (w1 << 16);
+    if (__any_sync(0xffffffffu, wanted != 0u)) {
         unsigned long long *cand = A.cand(rr);
         const int n = __popc(wanted), inc = warp_incl_scan(n, lane);
         int pos = 0;
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
         pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
 #pragma unroll 1
         for (; wanted; wanted &= wanted - 1u, pos++) {
-            const int e = (__ffs((int)wanted) - 1) * 32 + lane;
+            const int b = __ffs((int)wanted) - 1, e = (b & 15) * 64 + (b & 16) * 2 + lane;
             if (pos < HEADCAP) cand[pos] = make_key(__float_as_uint(list[skew(e)]), tile * TILE + (t.total == TILE ? e : (int)idx[e]));
         }
     }
@@ -1954,7 +1955,7 @@ __device__ __noinline__ void tile_again(CtxF &c, int t0, int t1, float *dst, boo
         const float thr = R.tp[(size_t)c.rr * R.ntile + t].thr;
         float *list = A->tile + (size_t)c.warp * 32 * PITCH;
         const TileEval e = tile_eval(list, reinterpret_cast<unsigned short *>(s->cnt) + c.warp * TILE, thr, c.cfg.T, __fdiv_rn(1.0f, c.cfg.T), c.pl.top,
-                                     (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, int) {});
+                                     (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, bool, unsigned int) {});
         float *to = to_list ? c.list + (size_t)t * TILE : dst;
 #pragma unroll 1
         for (int i = c.lane; i < e.total; i += 32) to[i] = list[skew(i)];
