@@ -51,7 +51,18 @@ constexpr int PLAN_BINS = 1024;            // row_plan: bins of the lanes' maxim
 constexpr float PLAN_RES = 32.0f;          // 32 per unit of logit
 
 enum { PLAN_DONE = 0, PLAN_SAMPLED = 1 };
-enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8, F_JUMP = 16 };
+enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8, F_JUMP = 16, F_FAR = 32, F_ALLNEAR = 64 };
+
+// The far head. A row without a top-k sorts what at least HEAD_NEED lanes' maxima reach and walks on through
+// tables of its list where top-p lies behind that: three more kernels, 60 to 80 us however short the row. In
+// rows of up to FAR_MOST_V logits most nuclei end within about FAR_HEAD elements, so their candidates go further
+// down: those the head has had all along (near) in one list, the others in a second one, used where both fit the
+// head's buffer together. Longer rows keep the near head: at 151936 seven nuclei in ten end behind either.
+// F_ALLNEAR: the row has fewer lanes than its head wants elements, so all it keeps is near, mostly too much; the
+// second list, of what all lanes' maxima reach, is then the head alone, if it holds what a top-k asks for.
+// Without and with it, us: 512 rows with mixed settings, 4000 logits 156 / 139, 8000 158 / 142, 20000 193 / 175;
+// 256 rows with a nucleus, 4000 logits 169 / 64, 8000 150 / 69, 20000 192 / 131, 50257 266 / 200.
+constexpr int FAR_MOST_V = 65536, FAR_HEAD = 1000;
 
 struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
 struct __align__(8) TilePlan { float thr, est; };
@@ -92,7 +103,7 @@ struct __align__(16) RowCfg {
 };
 
 // What row_plan hands to the kernels behind it.
-struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; int pad; };
+struct __align__(16) RowPlan { RowCfg c; int kind, flags; float top; unsigned int tau_bits; float xmax; int imax; int need; unsigned int tau_far; };
 
 // A row's small results, together in memory: the kernels that read them wait once.
 //   RowHead | TileOut[ntile] | candidates[HEADCAP] | prefix sums[HEADCAP] | values of careful chunks[CARE_PLACES][32] | items
@@ -105,13 +116,14 @@ constexpr int PICKS = 8, PICK_CAP = NC;
 struct __align__(16) WalkPicks { int n, arrived, pad[2]; int bin[PICKS]; int cnt[PICKS]; };
 constexpr size_t WALK_BYTES = WALK_BINADES * (NBINS * sizeof(unsigned long long) + sizeof(WalkTies)) + sizeof(WalkPicks) + (size_t)PICKS * PICK_CAP * sizeof(unsigned long long);
 
-struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; unsigned int hits[4]; };   // hits: see F_JUMP
+struct __align__(16) RowHead { RowPlan plan; int ncand, nitem, ncare, state; float Z, head_s; long long head_pos; unsigned int hits[4]; int nfar, pad[3]; };   // hits: see F_JUMP
 
 struct RowsArgs {
     BatchArgs a;
     int r0, rows;            // batch rows [r0, r0 + rows) are in flight
     int ntile, nspan;
     int oG, oVc, oL;         // see F_NARROW
+    int need_far;            // lanes' maxima that reach a far head's edge; 0: rows of this length have none
     TileStat *ts;            // [rows][ntile]
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
     TilePlan *tp;            // [rows][ntile]
@@ -124,6 +136,7 @@ struct RowsArgs {
     __device__ __forceinline__ WalkTies *ties(int rr) const { return reinterpret_cast<WalkTies *>(table(rr, WALK_BINADES)); }
     __device__ __forceinline__ WalkPicks *picks(int rr) const { return reinterpret_cast<WalkPicks *>(ties(rr) + WALK_BINADES); }
     __device__ __forceinline__ unsigned long long *picked(int rr, int i) const { return reinterpret_cast<unsigned long long *>(picks(rr) + 1) + (size_t)i * PICK_CAP; }
+    __device__ __forceinline__ unsigned long long *far(int rr) const { return picked(rr, 0); }   // (row_head has read it before tile_pick writes there)
     __device__ __forceinline__ RowHead *head(int rr) const { return reinterpret_cast<RowHead *>(box + (long long)rr * box_stride); }
     __device__ __forceinline__ TileOut *to(int rr) const { return reinterpret_cast<TileOut *>(head(rr) + 1); }
     __device__ __forceinline__ unsigned long long *cand(int rr) const { return reinterpret_cast<unsigned long long *>(to(rr) + ((ntile + 1) & ~1)); }
@@ -454,7 +467,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
 struct JumpShared { float in[128], over[128], own[128]; unsigned int hits[4]; };
 struct PlanShared {
     union { unsigned int hist[PLAN_BINS]; JumpShared jump; };
-    int edge;
+    int edge, edge_far;
     float wsf[NWARP + 1];
     int wsi[NWARP + 1];
 };
@@ -534,7 +547,7 @@ __device__ __noinline__ bool find_jumps(const RowsArgs &A, int rr, float f, floa
 __device__ __forceinline__ void store_settings(const RowsArgs &A, int rr, const RowCfg &c) {
     RowHead *h = A.head(rr);
     h->plan.c = c;
-    h->ncand = 0; h->nitem = 0; h->ncare = 0; h->state = 0;
+    h->ncand = 0; h->nfar = 0; h->nitem = 0; h->ncare = 0; h->state = 0;
     if (rr == 0) A.queue[0] = 0;
 }
 __device__ __forceinline__ void store_done(const RowsArgs &A, int rr) {   // (nothing else of such a row is looked at)
@@ -620,15 +633,15 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
     };
     // The head: a value that at least `need` of the lanes' maxima reach bounds the need-th largest
     // element from below, and few more elements than that reach it.
-    float tau_x = INFINITY;
-    bool narrow = false;
+    float tau_x = INFINITY, far_x = INFINITY;
+    bool narrow = false, far = false;
     if (!c.pure) {
         const int ng = A.ntile * 32;
         const float *gm = A.gmax + (size_t)rr * ng;
         // one histogram of the lanes' maxima by distance below the row's
 #pragma unroll 1
         for (int i = tid; i < PLAN_BINS; i += NT) S.hist[i] = 0u;
-        if (tid == 0) S.edge = -1;
+        if (tid == 0) S.edge = S.edge_far = -1;
         __syncthreads();
 #pragma unroll 1
         for (int i0 = 0; i0 < ng; i0 += 8 * NT) {
@@ -647,14 +660,21 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
 #pragma unroll
         for (int i = 0; i < PER; i++) { n[i] = (int)S.hist[PER * tid + i]; sum += n[i]; }
         int run = block_excl_scan<int>(sum, S.wsi, &tot);
+        // (typical-p works on what the near head holds, and refuses more)
+        const int need_far = A.need_far == 0 ? 0 : (c.open_row ? (c.topp_on && !(c.typ < 1.0f) ? min(A.need_far, tot) : 0) : (tot < need ? tot : 0));
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             if (run < need && run + n[i] >= need) S.edge = PER * tid + i;
+            if (run < need_far && run + n[i] >= need_far) S.edge_far = PER * tid + i;
             run += n[i];
         }
         __syncthreads();
         // (a bin's lower end, and a little below it: the subtraction and the product above were rounded)
-        tau_x = (S.edge >= 0 && fabsf(xmax) < 65536.0f) ? xmax - ((float)(S.edge + 1) + 0.25f) * (1.0f / PLAN_RES) : -INFINITY;
+        auto below_bin = [&](int b) { return fabsf(xmax) < 65536.0f ? xmax - ((float)(b + 1) + 0.25f) * (1.0f / PLAN_RES) : -INFINITY; };
+        tau_x = S.edge >= 0 ? below_bin(S.edge) : -INFINITY;
+        // (what cannot matter to the whole sum is no use to an open row's head: a sharp row has few elements that can)
+        far_x = S.edge_far >= 0 ? fmaxf(below_bin(S.edge_far), c.open_row ? thr_of(total) : -INFINITY) : -INFINITY;
+        far = far_x > -INFINITY && far_x < (tau_x > -INFINITY ? tau_x : INFINITY);
         // F_NARROW: a top-k so wide for the vocabulary that fewer ranges than candidates exist (one range
         // per thread of the widest layout: oG blocks of NT threads with oL logits each). Such rows report
         // the order of equal probabilities the way the descending walk sees it.
@@ -691,13 +711,16 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         jump = find_jumps(A, rr, f, xmax, S.jump);
         if (jump && tid < 4) A.head(rr)->hits[tid] = S.jump.hits[tid];
     }
-    const float tv = (c.T == 1.0f) ? tau_x : __fdiv_rn(tau_x, c.T);
-    const unsigned int tb = c.pure ? 0xffffffffu : __float_as_uint(expf_pinned(__fsub_rn(tv, top)));
+    auto bits_of = [&](float x) -> unsigned int {
+        const unsigned int b = __float_as_uint(expf_pinned(__fsub_rn((c.T == 1.0f) ? x : __fdiv_rn(x, c.T), top)));
+        return b > 5u ? b - 4u : 1u;
+    };
+    const float keep_x = far && far_x < tau_x ? far_x : tau_x;
     TilePlan *tp = A.tp + (size_t)rr * A.ntile;
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         const int t = 2 * tid + u;
-        if (t < A.ntile) { TilePlan p; p.thr = fminf(thr_of(est[u]), tau_x); p.est = est[u]; tp[t] = p; }
+        if (t < A.ntile) { TilePlan p; p.thr = fminf(thr_of(est[u]), keep_x); p.est = est[u]; tp[t] = p; }
     }
     if (tid == 0) {
         RowPlan &pl = A.head(rr)->plan;
@@ -705,9 +728,10 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
         // (too few lanes to bound the head: row_finish narrows it down from the list)
         pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
-                   ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
+                   (far ? F_FAR | (tau_x > -INFINITY ? 0 : F_ALLNEAR) : 0) | ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
         if (jump) pl.c.late = true;
-        pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : (tb > 5u ? tb - 4u : 1u);
+        pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : bits_of(tau_x);
+        pl.tau_far = far ? bits_of(far_x) : pl.tau_bits;
         pl.xmax = xmax; pl.imax = imax; pl.need = (int)need;
     }
 }
@@ -934,25 +958,39 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     const size_t gt = (size_t)rr * A.ntile + tile;
     const TilePlan tp = A.tp[gt];
     float *list = S->x + (size_t)warp * 32 * PITCH;
-    const unsigned int tau = pl.tau_bits;
+    const unsigned int tau = min(pl.tau_bits, pl.tau_far);
     unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
     unsigned int w0 = 0u, w1 = 0u;   // this lane's candidates among the entries it evaluates
     const TileEval t = tile_eval(list, idx, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
         [&](unsigned int eb, bool second, unsigned int bit) { if (eb >= tau) { if (second) w1 |= bit; else w0 |= bit; } });
     // A tile asks for its candidates' places once. (One request per value, each waited for before the next two
     // are evaluated, took 0.7 us each: up to 22 us a tile in short rows, whose few tiles hold all candidates.)
-    unsigned int wanted = w0 | (w1 << 16);
+    const unsigned int wanted = w0 | (w1 << 16);
     if (__any_sync(0xffffffffu, wanted != 0u)) {
-        unsigned long long *cand = A.cand(rr);
-        const int n = __popc(wanted), inc = warp_incl_scan(n, lane);
-        int pos = 0;
-        if (lane == 31) pos = atomicAdd(&head->ncand, inc);
-        pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
+        auto entry = [&](unsigned int m) { const int b = __ffs((int)m) - 1; return (b & 15) * 64 + (b & 16) * 2 + lane; };
+        auto put = [&](unsigned int m, int *count, unsigned long long *to) {
+            const int n = __popc(m), inc = warp_incl_scan(n, lane);
+            int pos = 0;
+            if (lane == 31 && inc) pos = atomicAdd(count, inc);
+            pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
 #pragma unroll 1
-        for (; wanted; wanted &= wanted - 1u, pos++) {
-            const int b = __ffs((int)wanted) - 1, e = (b & 15) * 64 + (b & 16) * 2 + lane;
-            if (pos < HEADCAP) cand[pos] = make_key(__float_as_uint(list[skew(e)]), tile * TILE + (t.total == TILE ? e : (int)idx[e]));
+            for (; m; m &= m - 1u, pos++) {
+                const int e = entry(m);
+                if (pos < HEADCAP) to[pos] = make_key(__float_as_uint(list[skew(e)]), tile * TILE + (t.total == TILE ? e : (int)idx[e]));
+            }
+        };
+        unsigned int near = wanted;
+        if (pl.flags & F_FAR) {
+            unsigned int beyond = 0u;
+#pragma unroll 1
+            for (unsigned int m = wanted; m; m &= m - 1u) {
+                const unsigned int eb = __float_as_uint(list[skew(entry(m))]), one = m & (0u - m);
+                if (eb < pl.tau_bits) near ^= one;
+                if (eb >= pl.tau_far && ((pl.flags & F_ALLNEAR) || eb < pl.tau_bits)) beyond |= one;
+            }
+            put(beyond, &head->nfar, A.far(rr));
         }
+        put(near, &head->ncand, A.cand(rr));
     }
     const TileChunk ch = tile_chunk(list, t.total);
     bool care;
@@ -1402,6 +1440,11 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     unsigned long long key = R.cand(rr)[tid];
     if (kind == PLAN_DONE) return;
     const RowCfg &g = pl.c;
+    const bool all_near = (pl.flags & F_ALLNEAR) != 0;
+    const int nfar = (pl.flags & F_FAR) ? head->nfar : 0, nfirst = all_near ? 0 : ncand;   // of the near list, with the far one
+    const bool far = nfar > 0 && nfirst + nfar <= HEADCAP && (!all_near || (ncand > HEADCAP && (g.open_row || nfar >= pl.need)));
+    const int nc = far ? nfirst + nfar : ncand;
+    const int nwalk = far && g.open_row ? (all_near ? HEAD_NEED : ncand) : nc;   // the near head alone would have walked on from here
     const bool narrow = (pl.flags & F_NARROW) != 0;
     auto queue_row = [&](int state, int why = 0) {
 #ifdef MOLLA_SAMPLE_TESTING
@@ -1409,7 +1452,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
 #endif
         if (tid == 0) { head->state = state; R.queue[1 + atomicAdd(&R.queue[0], 1)] = rr; }
     };
-    if (nitem > H_ITEMS || (!g.pure && ncand > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
+    if (nitem > H_ITEMS || (!g.pure && nc > HEADCAP)) { queue_row(ST_NOTHING, 1); return; }
     const unsigned long long seed = a.seed ? a.seed[g.q] : 0ull, drawn = a.drawn ? a.drawn[g.q] : 0ull;   // (not needed before the end)
     if (tid == 0) S->n_ge = 0;
     const unsigned int nrec = wl.order(&S->w, ntile, nitem);
@@ -1431,10 +1474,10 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         return;
     }
     // ---- sorted order: the head's candidates as probabilities
-    const int nc = ncand;
 #pragma unroll 1
     for (int i = tid; i < nc; i += HT) {
-        if (i >= HT) key = R.cand(rr)[i];
+        if (far && i >= nfirst) key = R.far(rr)[i - nfirst];
+        else if (i >= HT) key = R.cand(rr)[i];
         S->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(key), Z, yZ)) << 32) | (key & 0xFFFFFFFFull);
     }
     if (tid < 16 && nc + tid < HEADCAP) S->cand[nc + tid] = 0ull;
@@ -1503,14 +1546,16 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         __syncwarp();
         const int pos = cut >= 0 ? cut : lim;
         auto equal_next_to = [&](int i) { return (i > 0 && pc[i - 1] == pc[i]) || (i + 1 < nc && pc[i + 1] == pc[i]); };
+        // behind the near head, equal probabilities are reported the way the walk from there sees them
+        const bool walked = narrow || cut > nwalk || (cut < 0 && (long long)lim >= n_use && lim > nwalk);
         if (by_mass) {
-            if (narrow ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
+            if (walked ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
         } else if (lim > 0 && (long long)lim >= n_use) {
             cut = lim;  // the count limit
-            if (narrow && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
+            if (walked && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
         }
         if (cut < 0 && !p3row) cut = nc;  // everything that can matter is in the head
-        if (!narrow && n_use < (long long)a.V && (long long)nc > n_use && pc[n_use] == pc[n_use - 1]) tie |= MOLLA_ROW_TOPK_TIE;
+        if (!narrow && n_use < (long long)a.V && (long long)nwalk > n_use && pc[n_use] == pc[n_use - 1]) tie |= MOLLA_ROW_TOPK_TIE;
         if (g.typ < 1.0f) {
             // the typical-p filter takes over from here
         } else if (cut > 0) {
@@ -1522,7 +1567,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
                 const int mid = (at + hi) >> 1;
                 if (target < pre[mid]) hi = mid; else at = mid + 1;
             }
-            if (narrow ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at])))
+            if (walked ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at])))
                 tie |= MOLLA_ROW_CHOSEN_TIE;
             if (lane == 0)
                 finish_row(a, r, g, (unsigned int)tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), key_idx(S->cand[at]), Z, sum, target, pc[at]);
@@ -1552,6 +1597,7 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     }
 #pragma unroll 1
     for (int i = tid; i < nc; i += HT) { R.cand(rr)[i] = S->cand[i]; R.pre(rr)[i] = S->p.pre[i]; }
+    if (far && tid == 0) { head->ncand = nc; head->plan.tau_bits = pl.tau_far; }
     queue_row(ST_HEAD, 6);
 }
 
@@ -3439,6 +3485,8 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     A.a.Vg = a.V; A.a.col0 = 0; A.a.mode = 0;
     A.ntile = (a.V + TILE - 1) / TILE;
     A.nspan = (a.V + SPAN - 1) / SPAN;
+    // of V logits in no order, FAR_HEAD reach the value that this share of the lanes' maxima reaches
+    A.need_far = a.V > HEADCAP && a.V <= FAR_MOST_V ? (int)ceil((a.V + 31) / 32 * (1.0 - pow(1.0 - (double)FAR_HEAD / a.V, 32.0))) : 0;
     narrow_layout(a.V, a.layout_B > 0 ? a.layout_B : a.B, sms, A.oG, A.oVc, A.oL);
     const int rows = rows_in_flight(a.B, a.V);
     lay_out(A, (char *)d_workspace, rows, a.V);
