@@ -1449,6 +1449,8 @@ bool cluster_fits(int dev, int G) {
 
 }  // namespace
 
+bool molla_cluster_is_block(int V) { return V <= CL_CAPF; }
+
 // A row in the shared memory of its cluster is worked on in one launch, so as long as the clusters of all
 // rows are resident together the call is one row long: 19 us for greedy rows, 30 to 40 for a top-k, 60 to
 // 80 for walks, of up to 73000 logits (the tile kernels: 29, 36 to 47, 90 to 150). A second round of

@@ -1739,19 +1739,24 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
     return MOLLA_OK;
 }
 
-// Which of the two the rows of a launch go through (the testing build can ask for either).
-bool takes_clusters(const BatchArgs &a) {
+// Which of the two the rows of a launch go through (the testing build can ask for either). `piece`: a piece of a
+// host block, sampled alone however large the block, in which nobody asks for a top-k wider than 128. Where its own
+// clusters, of one thread block each, are resident together, it goes there though the block's would not be. Measured
+// through the host form (tiles / clusters, us): 200 rows of 20000 in five pieces, top-k 40 433 / 423, mixed settings
+// 484 / 479, 400 of 10000 mixed 642 / 567, 400 of 20000 mixed 826 / 732, nucleus 899 / 841; with clusters of two,
+// 100 rows of 60000, nothing sorted 562 / 766, mixed 636 / 707; with a top-k of 1024 in 400 rows of 20000 1201 / 1424.
+bool takes_clusters(const BatchArgs &a, bool piece) {
     const int call = a.layout_B > 0 ? a.layout_B : a.B;
     if (MOLLA_KNOB(a, 32)) return false;
     if (MOLLA_KNOB(a, 64)) return molla_cluster_better(a.V, 1, call);
-    return molla_cluster_better(a.V, call, call);
+    return molla_cluster_better(a.V, call, call) || (piece && molla_cluster_is_block(a.V) && molla_cluster_better(a.V, a.B, call));
 }
 
 // The ordinary entry points' launch.
-int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st) {
+int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool piece = false) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
-    const bool clusters = takes_clusters(a);
+    const bool clusters = takes_clusters(a, piece);
 #ifdef MOLLA_SAMPLE_TESTING
     g_launched[clusters ? 0 : 1]++;
 #endif
@@ -2299,7 +2304,9 @@ int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32
         }
         BatchArgs a = device_params(h, L, w, r0, r1);
         a.logits = (const float *)(w + L.logits) + (size_t)r0 * V; a.row_stride = V; a.V = V; a.layout_B = layout_B;
-        rc = launch_sampling(a, w, st);
+        bool wide = false;
+        for (int r = r0; top_k && r < r1; r++) wide |= temperature[r] > 0.0f && top_k[r] > 128;
+        rc = launch_sampling(a, w, st, npiece > 1 && !wide);
         if (rc == MOLLA_OK)
             rc = launch_logprobs(a.logits, V, a.B, V, a.tokens, top_n, h_chosen_logprob ? (float *)(w + L.chosen) + r0 : nullptr,
                                  top_n > 0 ? (int32_t *)(w + L.top_ids) + (size_t)r0 * top_n : nullptr,

@@ -540,6 +540,26 @@ def test_host_buffer_entry_matches_device_entry(dev, lib):
         assert np.array_equal(hb.top_ids.numpy(), got["top_ids"])
 
 
+@pytest.mark.parametrize("top_k,clusters", [(40, True), (500, False)])
+def test_host_pieces_are_routed_by_their_own_rows(dev, lib, top_k, clusters):
+    """A host block goes up in pieces that are sampled one by one: 200 rows at once go through the tile kernels, the 40 of
+    a piece through the cluster kernel, unless one of them asks for a wide top-k."""
+    w = W.config3(seed=23, B=200, V=20000, H=16)
+    w["top_k"][:] = np.minimum(w["top_k"], 40)
+    w["temperature"][::40] = 0.9
+    w["top_k"][::40] = top_k   # one such row in every piece
+    got = run_gpu(w, dev)
+    hb = S.HostBlock(w, dev)
+    counts = (C.c_int64 * 2)()
+    with capi.testing_library() as T:
+        T.molla_sample_debug_launches(counts)
+        S.sample_batch_host(hb)
+        T.molla_sample_debug_launches(counts)
+    assert (counts[0] > 1, counts[1] > 1) == (clusters, not clusters), list(counts)
+    assert np.array_equal(hb.tokens.numpy(), got["tokens"])
+    assert np.array_equal(hb.status.numpy().astype(np.uint32), got["row_status"])
+
+
 @pytest.mark.usefixtures("route")
 def test_grammar_mask_against_the_oracle(dev, lib, oracle):
     """`_mask` (sample.mojo:371-379): tokens a grammar forbids are dropped ahead of every other
