@@ -1699,11 +1699,21 @@ int region_floats(int V) { return (((V + NWARP - 1) / NWARP) + 3) & ~3; }
 // scratch layout: [row counter and finished-rows counter, 256 bytes][row order][per CTA: 16 per-warp
 // list segments + one contiguous copy, each entry an (exp bits, token id) pair]
 constexpr size_t WS_HEADER = 256 + (size_t)ORDER_CAP * 4;
+// What the ordinary entry points' own launches use: nothing where the rows go through the cluster kernel.
+size_t sampling_workspace_bytes(int B, int V, bool pieces, bool logprobs) {
+    bool clusters = !pieces && molla_cluster_better(V, B, B);
+#ifdef MOLLA_SAMPLE_TESTING
+    if (g_knobs & 32) clusters = false;
+#endif
+    const size_t rows = clusters ? 0 : molla_rows_workspace_bytes(B, V), lp = logprobs ? molla_logprob_workspace_bytes(B, V) : 0;
+    return rows > lp ? rows : lp;
+}
+
+// ... and the streaming kernel's lists (penalised rows, the sharded stages), for the workspace that serves all.
 size_t batch_workspace_bytes(int B, int V, int sms) {
     const size_t ctas = (size_t)(B < sms ? B : sms);
     const size_t lists = WS_HEADER + ctas * 2 * (size_t)NWARP * (size_t)region_floats(V) * 8;
-    const size_t rows = molla_rows_workspace_bytes(B, V), lp = molla_logprob_workspace_bytes(B, V);
-    const size_t most = rows > lp ? rows : lp;
+    const size_t most = sampling_workspace_bytes(B, V, true, true);
     return lists > most ? lists : most;
 }
 
@@ -2128,9 +2138,9 @@ struct HostLayout {
     size_t logits, f[8], win, seed, drawn, k, rows, hist, hist_off, bias_ids, bias_vals, bias_off;
     size_t tokens, status, chosen, top_ids, top_lps, total, inner;
 };
-HostLayout host_layout(int B, int V, long long n_hist, long long n_bias, int top_n, int sms, bool with_logits = true) {
+HostLayout host_layout(int B, int V, long long n_hist, long long n_bias, int top_n, bool with_logits = true) {
     HostLayout L;
-    size_t o = al256(batch_workspace_bytes(B, V, sms));  // the batched call's own workspace comes first
+    size_t o = al256(sampling_workspace_bytes(B, V, with_logits, with_logits));  // the batched call's own workspace comes first
     L.inner = o;
     L.logits = o; o += with_logits ? al256((size_t)B * V * 4) : 0;
     for (int i = 0; i < 8; i++) { L.f[i] = o; o += al256((size_t)B * 4); }
@@ -2232,7 +2242,7 @@ int64_t molla_sample_host_workspace_bytes(int32_t B, int32_t V, int64_t n_hist, 
         return fail(MOLLA_ERR_ARGUMENT, "bad shape for the workspace query%s");
     const int sms = sm_count();
     if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
-    return (int64_t)host_layout(B, V, n_hist, n_bias, top_n, sms).total;
+    return (int64_t)host_layout(B, V, n_hist, n_bias, top_n).total;
 }
 
 int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32_t B, int32_t V,
@@ -2259,7 +2269,7 @@ int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32
     const long long n_hist = hist_off ? hist_off[B] : 0, n_bias = bias_off ? bias_off[B] : 0;
     const int sms = sm_count();
     if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
-    const HostLayout L = host_layout(B, V, n_hist, n_bias, top_n, sms);
+    const HostLayout L = host_layout(B, V, n_hist, n_bias, top_n);
     if (!d_workspace || workspace_bytes < (int64_t)L.total) return fail(MOLLA_ERR_WORKSPACE, "workspace missing or too small%s");
     char *w = (char *)d_workspace;
     cudaStream_t st = (cudaStream_t)stream;
@@ -2353,7 +2363,7 @@ int64_t molla_sample_pick_workspace_bytes(int32_t B, int32_t V, int64_t n_hist, 
     if (B < 0 || V <= 0 || n_hist < 0 || n_bias < 0) return fail(MOLLA_ERR_ARGUMENT, "bad shape for the workspace query%s");
     const int sms = sm_count();
     if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
-    return (int64_t)host_layout(B, V, n_hist, n_bias, 0, sms, false).total;
+    return (int64_t)host_layout(B, V, n_hist, n_bias, 0, false).total;
 }
 
 int32_t molla_sample_pick_rows(const float *d_logits, int64_t row_stride, int32_t n_logit_rows, int32_t V, const int32_t *rows, int32_t B,
@@ -2378,7 +2388,7 @@ int32_t molla_sample_pick_rows(const float *d_logits, int64_t row_stride, int32_
     const long long n_hist = hist_off ? hist_off[B] : 0, n_bias = bias_off ? bias_off[B] : 0;
     const int sms = sm_count();
     if (sms <= 0) return fail(MOLLA_ERR_CUDA, "cannot query the device%s");
-    const HostLayout L = host_layout(B, V, n_hist, n_bias, 0, sms, false);
+    const HostLayout L = host_layout(B, V, n_hist, n_bias, 0, false);
     if (!d_workspace || workspace_bytes < (int64_t)L.total) return fail(MOLLA_ERR_WORKSPACE, "workspace missing or too small%s");
     char *w = (char *)d_workspace;
     cudaStream_t st = (cudaStream_t)stream;

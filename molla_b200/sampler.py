@@ -418,7 +418,8 @@ def params_of(samplers: Sequence[Sampler]) -> dict:
 
 
 # Each thread's device scratch for `pick_rows`, per device: a call ends with its stream idle, so the next
-# one in the thread may use the same memory on any stream. Kept up to 64 MB, given back with the thread.
+# one in the thread may use the same memory on any stream. Kept up to 64 MB, given back with the thread; what
+# a larger call needs beside it comes from PyTorch's own pool and goes back there. (Nothing in it has to be zero.)
 _scratch = threading.local()
 _SCRATCH_MOST = 64 << 20
 
@@ -427,8 +428,7 @@ def _pick_scratch(dev, need: int) -> torch.Tensor:
     kept = _scratch.__dict__.setdefault("bufs", {})
     buf = kept.get(dev)
     if buf is None or buf.numel() < need:
-        kept.pop(dev, None)
-        buf = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
+        buf = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=dev)
         if buf.numel() <= _SCRATCH_MOST:
             kept[dev] = buf
     return buf

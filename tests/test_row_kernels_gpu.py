@@ -71,6 +71,25 @@ def test_pick_rows_in_place(dev, lib, oracle, V):
         assert [m.recent[: m.filled] for m in mine] == [r.recent[: r.filled] for r in ref]
 
 
+@pytest.mark.parametrize("B,V,per_logit", [(32, 131072, 0.01), (16, 262144, 0.01), (64, 131072, 8.0), (200, 3000, 100.0)])
+def test_pick_rows_asks_for_what_its_kernels_use(dev, lib, B, V, per_logit):
+    """Rows in thread-block clusters need no scratch; the tile kernels' is some 6 bytes a logit and, a row, 250 KB of
+    lists and tables. It may hold anything: two calls, one of them on a buffer of 0xff."""
+    need = lib.molla_sample_pick_workspace_bytes(B, V, 0, 0)
+    assert 0 < need <= B * V * per_logit + (1 << 20) and (per_logit < 1 or need > 4 * B * V), need
+    block = torch.randn((B, V), device=dev) * 3
+    cfg = [S.SamplerConfig(temperature=1.2, top_k=[40, 0, 0][i % 3], top_p=[0.9, 1.0, 0.97][i % 3], seed=i) for i in range(B)]
+    got = []
+    for fill in (0xff, 0):
+        S._scratch.__dict__.clear()
+        S._scratch.bufs = {block.device: torch.full((max(need, 1 << 20),), fill, dtype=torch.uint8, device=dev)}
+        kept = S._scratch.bufs[block.device].data_ptr()
+        got.append(S.pick_rows(block, [S.Sampler(c, V, dev) for c in cfg]))
+        assert S._scratch.bufs[block.device].data_ptr() == kept   # large enough
+    S._scratch.__dict__.clear()
+    assert got[0] == got[1]
+
+
 @pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("steps", [0, 16])
 @pytest.mark.parametrize("V", [2049, 3000, 4064, 4097, 20000, 65536, 65537])
