@@ -1080,77 +1080,82 @@ __device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *
 // bin, the 600 subnormals that a short row of a low temperature can keep took 100 us to be counted).
 __device__ __forceinline__ unsigned int spread_bits(unsigned long long key) { return __float_as_uint(__fmul_rn(key_val(key), 1152921504606846976.0f)); }
 
-// Sorts S->cand[0..n) (descending value, ascending id; zeros behind them up to a multiple of 16) and leaves the values in S->p.pc, padded with zeros
-// to a multiple of eight. Up to HT keys: every key counts the keys above it. More go through bins of value
-// first (a few keys each) and count within their bin.
-__device__ void head_sort(HeadShared *S, int n) {
+// Sorts cand[0..n) (descending value, ascending id) with N threads and leaves the values in pc, padded with zeros
+// to a multiple of eight; tmp may lie over pc. Up to FEW keys: every key counts the keys above it. More go through
+// bins of value first (a few keys each: about four to a bin at n = 1400) and count within their bin: 1.4 us for
+// 1400 keys, where a sorting network over the block took 17 us. Ends with a barrier.
+template <int N, int FEW>
+__device__ __forceinline__ void sort_keys(int n, unsigned long long *cand, unsigned long long *tmp, float *pc, unsigned int *sbin, unsigned int *ws, unsigned int *ws2) {
+    static_assert(FEW <= N && HEADCAP % 16 == 0, "a key per thread, sixteen at a time");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int KPT = HEADCAP / HT, PER = NBINS / HT;
-    if (n <= HT) {
-        const unsigned long long mine = tid < n ? S->cand[tid] : 0ull;
+    constexpr int KPT = HEADCAP / N, PER = NBINS / N;
+    if (n <= FEW) {
+        if (tid < 16 && n + tid < HEADCAP) cand[n + tid] = 0ull;
+        __syncthreads();
+        const unsigned long long mine = tid < n ? cand[tid] : 0ull;
         int rank = 0;
         if (warp * 32 < n) {
 #pragma unroll 1
-            for (int j = 0; j < n; j += 16) {   // (padded to a multiple of 16; eight loads at a time)
+            for (int j = 0; j < n; j += 16) {   // (eight loads at a time)
                 ulonglong2 o[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) o[u] = *reinterpret_cast<const ulonglong2 *>(S->cand + j + 2 * u);
+                for (int u = 0; u < 8; u++) o[u] = *reinterpret_cast<const ulonglong2 *>(cand + j + 2 * u);
 #pragma unroll
                 for (int u = 0; u < 8; u++) rank += (o[u].x > mine ? 1 : 0) + (o[u].y > mine ? 1 : 0);
             }
         }
         __syncthreads();
-        if (tid < n) { S->cand[rank] = mine; S->p.pc[rank] = key_val(mine); }
+        if (tid < n) { cand[rank] = mine; pc[rank] = key_val(mine); }
     } else {
         unsigned long long k[KPT];
         unsigned int lo = 0xffffffffu, hi = 0u;
 #pragma unroll
         for (int u = 0; u < KPT; u++) {
-            const int i = tid + u * HT;
-            k[u] = i < n ? S->cand[i] : 0ull;
+            const int i = tid + u * N;
+            k[u] = i < n ? cand[i] : 0ull;
             if (i < n) { const unsigned int b = spread_bits(k[u]); lo = min(lo, b); hi = max(hi, b); }
         }
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) { S->ws[warp] = lo; S->ws2[warp] = hi; }
+        if (lane == 0) { ws[warp] = lo; ws2[warp] = hi; }
 #pragma unroll
-        for (int i = 0; i < PER; i++) S->sbin[tid + i * HT] = 0u;
+        for (int i = 0; i < PER; i++) sbin[tid + i * N] = 0u;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < HW; w++) { lo = min(lo, S->ws[w]); hi = max(hi, S->ws2[w]); }
+        for (int w = 0; w < N / 32; w++) { lo = min(lo, ws[w]); hi = max(hi, ws2[w]); }
         const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
         unsigned int slot[KPT];
         auto bin_of = [&](unsigned long long key) { return NBINS - 1 - ((spread_bits(key) - lo) >> shift); };   // descending
 #pragma unroll
         for (int u = 0; u < KPT; u++)
-            if (tid + u * HT < n) slot[u] = atomicAdd(&S->sbin[bin_of(k[u])], 1u);
+            if (tid + u * N < n) slot[u] = atomicAdd(&sbin[bin_of(k[u])], 1u);
         __syncthreads();
         unsigned int cnt[PER], sum = 0u, tot;
 #pragma unroll
-        for (int i = 0; i < PER; i++) { cnt[i] = S->sbin[PER * tid + i]; sum += cnt[i]; }
-        unsigned int at = head_scan<HT>(sum, S->ws, &tot);
+        for (int i = 0; i < PER; i++) { cnt[i] = sbin[PER * tid + i]; sum += cnt[i]; }
+        unsigned int at = head_scan<N>(sum, ws, &tot);
 #pragma unroll
-        for (int i = 0; i < PER; i++) { S->sbin[PER * tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
+        for (int i = 0; i < PER; i++) { sbin[PER * tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < KPT; u++)
-            if (tid + u * HT < n) S->tmp[(S->sbin[bin_of(k[u])] & 0xffffu) + slot[u]] = k[u];
+            if (tid + u * N < n) tmp[(sbin[bin_of(k[u])] & 0xffffu) + slot[u]] = k[u];
         __syncthreads();
         unsigned int rank[KPT];
 #pragma unroll
         for (int u = 0; u < KPT; u++)
-            if (tid + u * HT < n) {
-                const unsigned int b = S->sbin[bin_of(k[u])], b0 = b & 0xffffu, m = b >> 16;
+            if (tid + u * N < n) {
+                const unsigned int b = sbin[bin_of(k[u])], b0 = b & 0xffffu, m = b >> 16;
                 rank[u] = b0;
 #pragma unroll 1
-                for (unsigned int j = 0; j < m; j++) rank[u] += S->tmp[b0 + j] > k[u] ? 1u : 0u;
+                for (unsigned int j = 0; j < m; j++) rank[u] += tmp[b0 + j] > k[u] ? 1u : 0u;
             }
-        __syncthreads();   // the values take the space of the keys being read
+        __syncthreads();   // the values may take the space of the keys being read
 #pragma unroll
         for (int u = 0; u < KPT; u++)
-            if (tid + u * HT < n) { S->cand[rank[u]] = k[u]; S->p.pc[rank[u]] = key_val(k[u]); }
+            if (tid + u * N < n) { cand[rank[u]] = k[u]; pc[rank[u]] = key_val(k[u]); }
     }
-    if (tid < 8 && n + tid < HEADCAP) S->p.pc[n + tid] = 0.0f;
+    if (tid < 8 && n + tid < HEADCAP) pc[n + tid] = 0.0f;
     __syncthreads();
 }
 
@@ -1480,9 +1485,8 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
         else if (i >= HT) key = R.cand(rr)[i];
         S->cand[i] = ((unsigned long long)__float_as_uint(prob_of(key_val(key), Z, yZ)) << 32) | (key & 0xFFFFFFFFull);
     }
-    if (tid < 16 && nc + tid < HEADCAP) S->cand[nc + tid] = 0ull;
     __syncthreads();
-    head_sort(S, nc);
+    sort_keys<HT, HT>(nc, S->cand, S->tmp, S->p.pc, S->sbin, S->ws, S->ws2);
     // min-p (sample.mojo:508-523) keeps a prefix of the sorted order: what reaches p_max * min_p
     long long n_use = g.n_lim;
     bool all_above = false;   // every candidate does: how many others do is not known here
@@ -2200,72 +2204,12 @@ __device__ __forceinline__ void for_list4(const CtxF &c, F f) {
     }
 }
 
-// Sorts A->cand[0..n) (descending value, ascending id) and leaves the values in A->pc, padded with zeros
-// to a multiple of eight. Short lists: every key counts the keys above it. Longer ones go through bins of
-// value first (a few keys each: about four keys to a bin at n = 1400) and count within their bin: 1.4 us
-// for 1400 keys, where a sorting network over the block took 17 us.
 __device__ __noinline__ void sort_head(CtxF &c, int n) {
     AuxF *A = c.A;
     IN_SHARED(A);
+    static_assert(HEADCAP <= NC, "the sorted keys fit the candidates' space");
     __syncthreads();
-    if (n <= 96) {
-        const unsigned long long mine = (c.tid < n) ? A->cand[c.tid] : 0ull;
-        int rank = 0;
-        if (c.tid < n)
-#pragma unroll 1
-            for (int j = 0; j < n; j++) rank += A->cand[j] > mine ? 1 : 0;
-        __syncthreads();
-        if (c.tid < n) { A->cand[rank] = mine; A->pc[rank] = key_val(mine); }
-    } else {
-        constexpr int KPT = NC / NT;
-        unsigned long long k[KPT];
-        unsigned int lo = 0xffffffffu, hi = 0u;
-#pragma unroll
-        for (int u = 0; u < KPT; u++) {
-            const int i = c.tid + u * NT;
-            k[u] = i < n ? A->cand[i] : 0ull;
-            if (i < n) { lo = min(lo, (unsigned int)(k[u] >> 32)); hi = max(hi, (unsigned int)(k[u] >> 32)); }
-        }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (c.lane == 0) { A->wsi[c.warp] = (int)lo; A->wsf[c.warp] = __uint_as_float(hi); }
-#pragma unroll
-        for (int i = 0; i < BPT; i++) A->sbin[c.tid + i * NT] = 0u;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < NWARP; w++) { lo = min(lo, (unsigned int)A->wsi[w]); hi = max(hi, __float_as_uint(A->wsf[w])); }
-        const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
-        unsigned int bin[KPT], slot[KPT];
-#pragma unroll
-        for (int u = 0; u < KPT; u++) {
-            bin[u] = NBINS - 1 - (((unsigned int)(k[u] >> 32) - lo) >> shift);   // descending
-            if (c.tid + u * NT < n) slot[u] = atomicAdd(&A->sbin[bin[u]], 1u);
-        }
-        __syncthreads();
-        unsigned int cnt[BPT], sum = 0u, tot;
-#pragma unroll
-        for (int i = 0; i < BPT; i++) { cnt[i] = A->sbin[BPT * c.tid + i]; sum += cnt[i]; }
-        unsigned int at = block_excl_scan<unsigned int>(sum, reinterpret_cast<unsigned int *>(A->wsi), &tot);
-#pragma unroll
-        for (int i = 0; i < BPT; i++) { A->sbin[BPT * c.tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < KPT; u++)
-            if (c.tid + u * NT < n) A->tmp[(A->sbin[bin[u]] & 0xffffu) + slot[u]] = k[u];
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < KPT; u++)
-            if (c.tid + u * NT < n) {
-                const unsigned int b = A->sbin[bin[u]], b0 = b & 0xffffu, m = b >> 16;
-                unsigned int rank = b0;
-#pragma unroll 1
-                for (unsigned int j = 0; j < m; j++) rank += A->tmp[b0 + j] > k[u] ? 1u : 0u;
-                A->cand[rank] = k[u];
-                A->pc[rank] = key_val(k[u]);
-            }
-    }
-    if (c.tid < 8 && n + c.tid < NC) A->pc[n + c.tid] = 0.0f;
-    __syncthreads();
+    sort_keys<NT, 96>(n, A->cand, A->tmp, A->pc, A->sbin, reinterpret_cast<unsigned int *>(A->wsi), reinterpret_cast<unsigned int *>(A->wsf));
 }
 
 // More candidates than the head holds (few lanes for a wide top-k, or many equal values): a finer
