@@ -1159,6 +1159,71 @@ __device__ __forceinline__ void sort_keys(int n, unsigned long long *cand, unsig
     __syncthreads();
 }
 
+// The sorted head's pc[0..nc) by one warp: its prefix sums (sample.mojo:497-506) into pre, eight at a time, at most
+// n_use elements of them; where top-p or the count ends the set (cut, or -1: behind the head); the draw from it
+// (:580-590, unless typical-p takes over); the marks of equal probabilities at either end.
+// From nwalk on, and everywhere with `narrow`, they are those of a walk past the head; with `overflow` there is no head.
+struct HeadEnd { float s; int pos, cut, at; float sum, target; unsigned int tie; };   // s, pos: the sum and the count so far; at: the drawn one, or -1
+__device__ __forceinline__ HeadEnd head_end(const RowCfg &g, int V, const float *pc, float *pre, int nc, int nwalk, long long n_use, bool narrow, bool overflow, float u01) {
+    const int lane = threadIdx.x & 31;
+    const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST), topp_on = g.topp_on;
+    const float P = g.P;
+    HeadEnd e;
+    e.at = -1; e.sum = 0.0f; e.target = 0.0f; e.tie = 0u;
+    float s = 0.0f;
+    int cut = -1;
+    bool by_mass = false;
+    const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
+    const float4 *p4 = reinterpret_cast<const float4 *>(pc);
+    float4 x = p4[0], y = p4[1];
+#pragma unroll 1
+    for (int i = 0; i < lim && cut < 0; i += 8) {
+        const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        if (i + 8 < lim) { x = p4[(i >> 2) + 2]; y = p4[(i >> 2) + 3]; }
+        float t[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
+        if (lane == 0) {
+            float4 *o4 = reinterpret_cast<float4 *>(pre + i);
+            o4[0] = make_float4(t[0], t[1], t[2], t[3]);
+            o4[1] = make_float4(t[4], t[5], t[6], t[7]);
+        }
+        if (topp_on && s >= P) {
+#pragma unroll
+            for (int q = 7; q >= 0; q--)
+                if (t[q] >= P) { cut = i + q + 1; s = t[q]; }   // the first one wins
+            by_mass = true;
+        }
+    }
+    __syncwarp();
+    e.s = s;
+    e.pos = cut >= 0 ? cut : lim;
+    auto equal_next_to = [&](int i) { return (i > 0 && pc[i - 1] == pc[i]) || (i + 1 < nc && pc[i + 1] == pc[i]); };
+    const bool walked = narrow || cut > nwalk || (cut < 0 && (long long)lim >= n_use && lim > nwalk);
+    if (by_mass) {
+        if (walked ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) e.tie |= MOLLA_ROW_TOPP_TIE;
+    } else if (lim > 0 && (long long)lim >= n_use) {
+        cut = lim;  // the count limit
+        if (walked && equal_next_to(cut - 1)) e.tie |= MOLLA_ROW_TOPK_TIE;
+    }
+    if (cut < 0 && !p3row && !overflow) cut = nc;  // everything that can matter is in the head
+    if (!narrow && n_use < (long long)V && (long long)nwalk > n_use && pc[n_use] == pc[n_use - 1]) e.tie |= MOLLA_ROW_TOPK_TIE;
+    if (!(g.typ < 1.0f) && cut > 0) {
+        e.sum = pre[cut - 1];
+        e.target = __fmul_rn(u01, e.sum);
+        // the first prefix sum above the target (they never fall), or the last one kept
+        int at = 0, hi = cut - 1;
+        while (at < hi) {
+            const int mid = (at + hi) >> 1;
+            if (e.target < pre[mid]) hi = mid; else at = mid + 1;
+        }
+        if (walked ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at]))) e.tie |= MOLLA_ROW_CHOSEN_TIE;
+        e.at = at;
+    }
+    e.cut = cut;
+    return e;
+}
+
 // Everything about a row's items, in one round of loads by N threads (what lies past the counts is not used).
 template <int N>
 struct WalkLoads {
@@ -1515,70 +1580,15 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     }
 #endif
     if (warp == 0) {
-        // the prefix sums of the sorted head (sample.mojo:497-506), eight at a time; at most n_use
-        // elements are added
-        const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST);
-        const bool topp_on = g.topp_on;
-        const float P = g.P;
-        const float *pc = S->p.pc;
-        float *pre = S->p.pre;
-        float s = 0.0f;
-        int cut = -1, tie = 0;
-        bool by_mass = false;
-        const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
-        const float4 *p4 = reinterpret_cast<const float4 *>(pc);
-        float4 x = p4[0], y = p4[1];
-#pragma unroll 1
-        for (int i = 0; i < lim && cut < 0; i += 8) {
-            const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            if (i + 8 < lim) { x = p4[(i >> 2) + 2]; y = p4[(i >> 2) + 3]; }
-            float t[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
-            if (lane == 0) {
-                float4 *o4 = reinterpret_cast<float4 *>(pre + i);
-                o4[0] = make_float4(t[0], t[1], t[2], t[3]);
-                o4[1] = make_float4(t[4], t[5], t[6], t[7]);
+        const HeadEnd e = head_end(g, a.V, S->p.pc, S->p.pre, nc, nwalk, n_use, narrow, false, draw01(seed, drawn));
+        if (lane == 0) {
+            if (e.at >= 0)
+                finish_row(a, r, g, e.tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), key_idx(S->cand[e.at]), Z, e.sum, e.target, S->p.pc[e.at]);
+            else if (!(g.typ < 1.0f)) {
+                head->head_s = e.s; head->head_pos = e.pos;
             }
-            if (topp_on && s >= P) {
-#pragma unroll
-                for (int q = 7; q >= 0; q--)
-                    if (t[q] >= P) { cut = i + q + 1; s = t[q]; }   // the first one wins
-                by_mass = true;
-            }
+            S->cut = e.cut; S->tie = e.tie;
         }
-        __syncwarp();
-        const int pos = cut >= 0 ? cut : lim;
-        auto equal_next_to = [&](int i) { return (i > 0 && pc[i - 1] == pc[i]) || (i + 1 < nc && pc[i + 1] == pc[i]); };
-        // behind the near head, equal probabilities are reported the way the walk from there sees them
-        const bool walked = narrow || cut > nwalk || (cut < 0 && (long long)lim >= n_use && lim > nwalk);
-        if (by_mass) {
-            if (walked ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
-        } else if (lim > 0 && (long long)lim >= n_use) {
-            cut = lim;  // the count limit
-            if (walked && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
-        }
-        if (cut < 0 && !p3row) cut = nc;  // everything that can matter is in the head
-        if (!narrow && n_use < (long long)a.V && (long long)nwalk > n_use && pc[n_use] == pc[n_use - 1]) tie |= MOLLA_ROW_TOPK_TIE;
-        if (g.typ < 1.0f) {
-            // the typical-p filter takes over from here
-        } else if (cut > 0) {
-            const float sum = pre[cut - 1];
-            const float target = __fmul_rn(draw01(seed, drawn), sum);
-            // the first prefix sum above the target (they never fall), or the last one kept
-            int at = 0, hi = cut - 1;
-            while (at < hi) {
-                const int mid = (at + hi) >> 1;
-                if (target < pre[mid]) hi = mid; else at = mid + 1;
-            }
-            if (walked ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at])))
-                tie |= MOLLA_ROW_CHOSEN_TIE;
-            if (lane == 0)
-                finish_row(a, r, g, (unsigned int)tie | (narrow ? MOLLA_ROW_SLOW_PATH : 0u), key_idx(S->cand[at]), Z, sum, target, pc[at]);
-        } else if (lane == 0) {
-            head->head_s = s; head->head_pos = pos;
-        }
-        if (lane == 0) { S->cut = cut; S->tie = (unsigned int)tie; }
     }
     __syncthreads();
     if (g.typ < 1.0f) {
@@ -3012,63 +3022,18 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
             a.topk_out[(long long)c.r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? (int)(A->hidx[i] & 0x7fffffffu) : -1;
     }
 #endif
-    const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST);
     const bool typ_on = g.typ < 1.0f;
     FSTAMP(5);
-    if (c.tid == 0) {
-        float s = 0.0f;
-        int cut = -1, tie = 0;
-        bool by_mass = false;
-        // the prefix sums of the sorted head (sample.mojo:497-506), eight at a time; at most n_use
-        // elements are added
-        const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
-#pragma unroll 1
-        for (int i = 0; i < lim && cut < 0; i += 8) {
-            const float4 *p4 = reinterpret_cast<const float4 *>(A->pc + i);
-            const float4 x = p4[0], y = p4[1];
-            const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-            float t[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
-            float4 *o4 = reinterpret_cast<float4 *>(A->pre + i);
-            o4[0] = make_float4(t[0], t[1], t[2], t[3]);
-            o4[1] = make_float4(t[4], t[5], t[6], t[7]);
-            if (g.topp_on && s >= g.P) {
-#pragma unroll
-                for (int q = 7; q >= 0; q--)
-                    if (t[q] >= g.P) { cut = i + q + 1; s = t[q]; }   // the first one wins
-                by_mass = true;
+    if (c.warp == 0) {
+        const HeadEnd e = head_end(g, a.V, A->pc, A->pre, nc, nc, n_use, narrow, head_overflow, u01);
+        if (c.lane == 0) {
+            A->b_s = e.s; A->b_pos = e.pos; A->b_event = EV_NONE; A->b_idx = -1; A->b_p = 0.0f; A->b_aux = (int)e.tie;
+            if (typ_on) A->ncand = narrow ? -1 : e.cut;  // the typical-p filter takes over from here
+            if (e.at >= 0) {
+                A->b_event = EV_DRAW; A->b_idx = (int)(A->hidx[e.at] & 0x7fffffffu); A->b_p = A->pc[e.at];
+                A->b_sum = e.sum; A->b_target = e.target;
             }
         }
-        const long long pos = (cut >= 0) ? (long long)cut : (long long)lim;
-        auto equal_next_to = [&](int x) { return (A->hidx[x] & 0x80000000u) != 0u; };
-        if (by_mass) {
-            if (narrow ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && A->pc[cut] == A->pc[cut - 1])) tie |= MOLLA_ROW_TOPP_TIE;
-        } else if (lim > 0 && (long long)lim >= n_use) {
-            cut = lim;  // the count limit
-            if (narrow && equal_next_to(cut - 1)) tie |= MOLLA_ROW_TOPK_TIE;
-        }
-        if (cut < 0 && !p3row && !head_overflow) cut = nc;  // everything that can matter is in the head
-        if (!narrow && n_use < (long long)a.V && (long long)nc > n_use && A->pc[n_use] == A->pc[n_use - 1])
-            tie |= MOLLA_ROW_TOPK_TIE;
-        A->b_s = s; A->b_pos = pos; A->b_event = EV_NONE; A->b_idx = -1; A->b_p = 0.0f;
-        if (typ_on) {
-            A->ncand = narrow ? -1 : cut;  // the typical-p filter takes over from here
-        } else if (cut > 0) {
-            const float sum = A->pre[cut - 1];
-            const float target = __fmul_rn(u01, sum);
-            // the first prefix sum above the target (they never fall), or the last one kept
-            int at = 0, hi = cut - 1;
-            while (at < hi) {
-                const int mid = (at + hi) >> 1;
-                if (target < A->pre[mid]) hi = mid; else at = mid + 1;
-            }
-            A->b_event = EV_DRAW; A->b_idx = (int)(A->hidx[at] & 0x7fffffffu); A->b_p = A->pc[at];
-            if (narrow ? equal_next_to(at) : ((at > 0 && A->pc[at - 1] == A->pc[at]) || (at + 1 < cut && A->pc[at + 1] == A->pc[at])))
-                tie |= MOLLA_ROW_CHOSEN_TIE;
-            A->b_sum = sum; A->b_target = target;
-        }
-        A->b_aux = tie;
     }
     __syncthreads();
     FSTAMP(6);
