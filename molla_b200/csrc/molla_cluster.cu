@@ -650,8 +650,7 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     g.G = a.G; g.rank = (int)cl.block_rank(); g.L = a.L;
     g.c0 = g.rank * a.Vc;
     g.nloc = max(0, min(a.Vc, a.V - g.c0));
-    const int row_i = (int)blockIdx.x / g.G;
-    const int r = a.order ? a.order[row_i] : row_i;
+    const int r = (int)blockIdx.x / g.G;
     const bool leader = g.rank == 0;
     AuxC *lead = cl.map_shared_rank(A, 0);
 
@@ -1472,7 +1471,6 @@ int molla_cluster_launch(const BatchArgs &args_in, cudaStream_t st, char *err, s
     const ClusterShape cs = cluster_shape(a.V, a.layout_B > 0 ? a.layout_B : a.B, sms);
     a.G = cs.G; a.Vc = cs.Vc; a.L = cs.L;
     a.Vg = a.V; a.col0 = 0; a.mode = 0;
-    a.order = nullptr;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     cluster_config(cfg, at, (unsigned)a.B * (unsigned)cs.G, cs.G, st);
