@@ -43,6 +43,24 @@ __device__ __forceinline__ long long logit_row(const LpArgs &a, int r) {
     return (a.rows && (l < 0 || (a.n_logit_rows > 0 && l >= a.n_logit_rows))) ? -1 : l;
 }
 __device__ __forceinline__ int tile_end(const LpArgs &a, int t) { return t == a.ntile - 1 ? a.V : (t + 1) * LTILE; }
+// A tile of n logits (the row's last one up to 64 more than LTILE) by one warp: by sixteen bytes a lane where `wide`
+// and the tile is whole, by words elsewhere; `none` for what is not there. Returns which.
+__device__ __forceinline__ bool load_tile(float (&x)[34], const float *z, int n, int lane, bool wide, float none) {
+    wide = wide && n >= LTILE;
+    if (wide) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(z) + lane + 32 * i);
+            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; i++) x[i] = lane + 32 * i < n ? __ldg(z + lane + 32 * i) : none;
+    }
+    x[32] = LTILE + lane < n ? __ldg(z + LTILE + lane) : none;
+    x[33] = LTILE + 32 + lane < n ? __ldg(z + LTILE + 32 + lane) : none;
+    return wide;
+}
 __device__ __forceinline__ float capped(const LpArgs &a, float x) { return a.softcap > 0.0f ? softcap_pinned(x, a.softcap) : x; }
 
 __global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
@@ -56,18 +74,7 @@ __global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a
     const float *z = a.logits + lrow * a.row_stride + (long long)t * LTILE;
     const int n = tile_end(a, t) - t * LTILE;
     float x[34];
-    if ((reinterpret_cast<uintptr_t>(z) & 15u) == 0 && n >= LTILE) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(z) + lane + 32 * i);
-            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; i++) x[i] = lane + 32 * i < n ? __ldg(z + lane + 32 * i) : -INFINITY;
-    }
-    x[32] = LTILE + lane < n ? __ldg(z + LTILE + lane) : -INFINITY;
-    x[33] = LTILE + 32 + lane < n ? __ldg(z + LTILE + 32 + lane) : -INFINITY;
+    (void)load_tile(x, z, n, lane, (reinterpret_cast<uintptr_t>(z) & 15u) == 0, -INFINITY);
     float m = -INFINITY;
     if (a.softcap > 0.0f) {
 #pragma unroll
@@ -248,19 +255,7 @@ __global__ void __launch_bounds__(LT_) lp_write(const __grid_constant__ LpArgs a
     const int n = tile_end(a, t) - t * LTILE;
     const float top = o[0], offset = o[1];
     float x[34];
-    const bool vec = (reinterpret_cast<uintptr_t>(z) & 15u) == 0 && (reinterpret_cast<uintptr_t>(o) & 15u) == 0 && n >= LTILE;
-    if (vec) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(z) + lane + 32 * i);
-            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; i++) x[i] = lane + 32 * i < n ? __ldg(z + lane + 32 * i) : 0.0f;
-    }
-    x[32] = LTILE + lane < n ? __ldg(z + LTILE + lane) : 0.0f;
-    x[33] = LTILE + 32 + lane < n ? __ldg(z + LTILE + 32 + lane) : 0.0f;
+    const bool vec = load_tile(x, z, n, lane, ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0, 0.0f);
 #pragma unroll
     for (int i = 0; i < 34; i++) x[i] = __fsub_rn(__fsub_rn(x[i], top), offset);
     __syncwarp();   // every lane has read the tile's copy
