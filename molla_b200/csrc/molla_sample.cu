@@ -1752,9 +1752,9 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
 // Which of the two the rows of a launch go through (the testing build can ask for either). `piece`: a piece of a
 // host block, sampled alone however large the block, in which nobody asks for a top-k wider than 128. Where its own
 // clusters, of one thread block each, are resident together, it goes there though the block's would not be. Measured
-// through the host form (tiles / clusters, us): 200 rows of 20000 in five pieces, top-k 40 433 / 423, mixed settings
-// 484 / 479, 400 of 10000 mixed 642 / 567, 400 of 20000 mixed 826 / 732, nucleus 899 / 841; with clusters of two,
-// 100 rows of 60000, nothing sorted 562 / 766, mixed 636 / 707; with a top-k of 1024 in 400 rows of 20000 1201 / 1424.
+// through the host form (tiles / clusters, us): 200 rows of 20000 in two pieces, mixed settings 445 / 412, a nucleus
+// 437 / 423; 400 rows of 20000 in four, mixed 755 / 708, a nucleus 748 / 713, top-k 40 722 / 719; with clusters of two,
+// 100 rows of 60000, nothing sorted 559 / 577; with a top-k of 1024, 200 rows of 38000 798 / 1073.
 bool takes_clusters(const BatchArgs &a, bool piece) {
     const int call = a.layout_B > 0 ? a.layout_B : a.B;
     if (MOLLA_KNOB(a, 32)) return false;
@@ -2275,12 +2275,15 @@ int32_t molla_sample_batch_host(const float *h_logits, int64_t row_stride, int32
     cudaStream_t st = (cudaStream_t)stream;
     CopyLane *lane = copy_lane();
     // A large block goes up in pieces on a stream of the library's own while the pieces that have arrived
-    // are sampled on the caller's stream. At the 55 GB/s of the link a piece of 3 MB takes the 55 us that a
-    // few rows take to be sampled: smaller ones would wait for the kernels, larger ones leave more of them
-    // behind the last copy (16 MB in one piece: 450 us, in pieces: 350).
+    // are sampled on the caller's stream. A piece is sampled in the 60 to 130 us of its longest row, however
+    // few its rows, so it should be no less on the link: 7 MB take 130 us at 55 GB/s. Pieces of 1 / 2 / 3 / 4 / 5 / 8 to a
+    // block, us: 16 MB (32 rows) mixed settings 439 / 391 / 411 / 416 / 432 / 528, a nucleus 428 / 431 / 433 / 494 / 564 /
+    // 810; 33 MB mixed 771 / 733 / 731 / 729 / 735 / 762; 66 MB mixed 1535 / 1389 / 1343 / 1328 / 1316 / 1301; 8 MB nucleus
+    // 284 / 266 / 319 / 391 / 434 / 643, mixed 276 / 283 / 310 / 336 / 372 / 500.
     constexpr int MAXPIECE = 8;
+    constexpr size_t PIECE_BYTES = (size_t)7 << 20;
     const size_t block = (size_t)B * V * 4;
-    int npiece = (int)(block / ((size_t)3 << 20) < MAXPIECE ? block / ((size_t)3 << 20) : MAXPIECE);
+    int npiece = (int)(block / PIECE_BYTES < MAXPIECE ? block / PIECE_BYTES : MAXPIECE);
     if (npiece > B) npiece = B;
     if (npiece < 2 || !lane || !lane->streams()) npiece = 1;
     cudaError_t e = cudaSuccess;

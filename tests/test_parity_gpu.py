@@ -542,7 +542,7 @@ def test_host_buffer_entry_matches_device_entry(dev, lib):
 
 @pytest.mark.parametrize("top_k,clusters", [(40, True), (500, False)])
 def test_host_pieces_are_routed_by_their_own_rows(dev, lib, top_k, clusters):
-    """A host block goes up in pieces that are sampled one by one: 200 rows at once go through the tile kernels, the 40 of
+    """A host block goes up in pieces that are sampled one by one: 200 rows at once go through the tile kernels, the 100 of
     a piece through the cluster kernel, unless one of them asks for a wide top-k."""
     w = W.config3(seed=23, B=200, V=20000, H=16)
     w["top_k"][:] = np.minimum(w["top_k"], 40)
