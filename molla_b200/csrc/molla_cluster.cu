@@ -1450,11 +1450,15 @@ bool cluster_fits(int dev, int G) {
 
 bool molla_cluster_is_block(int V) { return V <= CL_CAPF; }
 
-// A row in the shared memory of its cluster is worked on in one launch, so as long as the clusters of all
-// rows are resident together the call is one row long: 19 us for greedy rows, 30 to 40 for a top-k, 60 to
-// 80 for walks, of up to 73000 logits (the tile kernels: 29, 36 to 47, 90 to 150). A second round of
-// clusters doubles that and the tile kernels pass it: 128 rows of 73000 with a top-k 62 against 97 us,
-// with a top-k of 1024 85 against 430.
+// A row in the shared memory of its cluster is worked on in one launch, so as long as the clusters of all rows are
+// resident together the call is one row long: 32 rows of 8000 to 73000 logits take 10 to 14 us if greedy, 42 to 48
+// with a top-k of 40, 45 to 56 with mixed settings, 71 to 96 with a nucleus, 67 to 94 where nothing is sorted (the
+// tile kernels: 18 to 20, 44 to 54, 56 to 74, 52 to 121, 69 to 85). A second round of clusters doubles that and the
+// tile kernels pass it: 128 rows of 73000 with a top-k 75 against 96 us, nothing sorted 122 against 207; 256 rows of
+// 8000 with a top-k 53 against 67, a nucleus 69 against 121. Two kinds of batch the line cuts wrong, and as the
+// settings are on the device it cannot see them: up to 512 rows of 2500 to 20000 logits, each with its own settings
+// (256 of 8000: 108 us in tiles, 76 in clusters), and rows that all ask for a wide top-k (64 of 50257: 216 in clusters,
+// 77 in tiles).
 bool molla_cluster_better(int V, int B, int call_B) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;

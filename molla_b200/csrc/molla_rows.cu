@@ -21,7 +21,7 @@
 // so any number of rows, from one to thousands, fills the chip, and only the row kernels have serial
 // parts. A row per thread-block cluster, resident in its shared memory, read the block once but left 33 to 16
 // rows in flight on the chip, each as slow as its serial parts: 1024 rows of 262144 took 6316 us where this
-// takes 1024, 64 of 151936 with logprobs 300 where this takes 195. Seven launches cost 2 to 3 us each where
+// takes 930 to 1250 (by the longest row's careful chunks), 64 of 151936 with logprobs 300 where this takes 197. Seven launches cost 2 to 3 us each where
 // nothing else is to be done; they are chained so that a kernel's blocks are in place when the one before
 // ends. The reference's sequential fp32 sums are reproduced bit for bit: see "Items" below.
 #include <cuda_runtime.h>
@@ -462,7 +462,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
 
 // =============================================================================
 // Kernel 2: one block per row. Bound: latency (two rounds of loads, one histogram, code that runs once):
-// 7 to 10 us for up to 148 rows, 13 for 256, 22 for 512.
+// 5 us for 128 greedy rows, 9 for 64 sampled ones, 14 for 256, 21 for 512. The settings are stored as soon as the row
+// is known to be sampled: kept in registers to the end they spilled, and 512 rows took 3 us more.
 // =============================================================================
 struct JumpShared { float in[128], over[128], own[128]; unsigned int hits[4]; };
 struct PlanShared {
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
 // =============================================================================
 // Kernel 3: exponentials, candidates, items. Bound: instructions and shared memory latency, about 2300
 // warp instructions a tile that keeps two thirds (early tiles and warm rows keep nearly all, cold ones few):
-// 256 rows of 151936 take 73 us, 512 of 262144 260. Evaluating in full warps from a list of what
+// 256 rows of 151936 take 76 us, 512 of 262144 240, issuing in two thirds of the active cycles. Evaluating in full warps from a list of what
 // is kept, in place of each lane its own, gave 20 %.
 // =============================================================================
 // A tile's list in shared memory: entry e at list[skew(e)] (a word is left out after every 32, so that
@@ -1020,8 +1021,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // Kernel 4: one small block per sampled row. The items give the softmax denominator, the candidates the
 // sorted head; most rows end here. Rows that go on (nothing sorted, a nucleus past the head, typical-p,
 // anything unusual) are queued for the last kernel. Bound: the latency of one warp's dependent additions
-// and of one round of loads, so the block is small and three of them share an SM: 11 us for one row, 17 for
-// 64, 31 for 256, 60 for 512 with a top-k of 1024. (Run by the tail's 512 threads, one block an SM, the same
+// and of one round of loads, so the block is small and three of them share an SM: 11 us for one row, 18 for
+// 64, 32 for 256, 66 for 512 with a top-k of 1024. (Run by the tail's 512 threads, one block an SM, the same
 // rows took twice as long.)
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
@@ -1621,8 +1622,8 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
 // sorted head, the bin tables of the walk in the binades the sum will go through: an element adds
 // rne(p / ulp) units to whatever sum lies in the binade, so one histogram of those integers per binade
 // tells where the sum crosses anything. Blocks take spans from the queue as long as there are any.
-// Bound: shared-memory atomics and latency; 50 us for 58 rows of 151936 past the head, 14 for 48 rows of
-// 50257 that sort nothing. In the row's own block the same passes took 100 us and more.
+// Bound: the latency of dependent instructions, branches and loads (warps issue in 46 % of the active cycles); 48 us for 58
+// rows of 151936 past the head, 14 for 48 rows of 50257 that sort nothing. In the row's own block the same passes took 100 us and more.
 // =============================================================================
 union __align__(16) WalkTileShared {
     float x[SPAN_THREADS * PITCH];
