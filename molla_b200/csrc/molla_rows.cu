@@ -58,11 +58,13 @@ enum { F_LIST = 1, F_FASTDIV = 2, F_PURE = 4, F_NARROW = 8, F_JUMP = 16, F_FAR =
 // rows of up to FAR_MOST_V logits most nuclei end within about FAR_HEAD elements, so their candidates go further
 // down: those the head has had all along (near) in one list, the others in a second one, used where both fit the
 // head's buffer together. Longer rows keep the near head: at 151936 seven nuclei in ten end behind either.
-// F_ALLNEAR: the row has fewer lanes than its head wants elements, so all it keeps is near, mostly too much; the
-// second list, of what all lanes' maxima reach, is then the head alone, if it holds what a top-k asks for.
+// F_ALLNEAR: the row has fewer lanes than its head wants elements, or hardly more, so the near list mostly holds too
+// much; the second one, which ends higher up, is then the head alone, if it holds what a top-k asks for (aimed at
+// FAR_TOPK elements, between that and the buffer's size).
 // Without and with it, us: 512 rows with mixed settings, 4000 logits 156 / 139, 8000 158 / 142, 20000 193 / 175;
-// 256 rows with a nucleus, 4000 logits 169 / 64, 8000 150 / 69, 20000 192 / 131, 50257 266 / 200.
-constexpr int FAR_MOST_V = 65536, FAR_HEAD = 1000;
+// 256 rows with a nucleus, 4000 logits 169 / 64, 8000 150 / 69, 20000 192 / 131, 50257 266 / 200;
+// with a top-k of 1024, 8000 169 / 128, 20000 290 / 100.
+constexpr int FAR_MOST_V = 65536, FAR_HEAD = 1000, FAR_TOPK = 1450;
 
 struct __align__(16) TileStat { float tmax, tsum; int tidx, teq; };
 struct __align__(8) TilePlan { float thr, est; };
@@ -123,7 +125,7 @@ struct RowsArgs {
     int r0, rows;            // batch rows [r0, r0 + rows) are in flight
     int ntile, nspan;
     int oG, oVc, oL;         // see F_NARROW
-    int need_far;            // lanes' maxima that reach a far head's edge; 0: rows of this length have none
+    int need_far, need_topk; // lanes' maxima that reach a far head's edge, without a top-k and with one; 0: rows of this length have none
     TileStat *ts;            // [rows][ntile]
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
     TilePlan *tp;            // [rows][ntile]
@@ -662,7 +664,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         for (int i = 0; i < PER; i++) { n[i] = (int)S.hist[PER * tid + i]; sum += n[i]; }
         int run = block_excl_scan<int>(sum, S.wsi, &tot);
         // (typical-p works on what the near head holds, and refuses more)
-        const int need_far = A.need_far == 0 ? 0 : (c.open_row ? (c.topp_on && !(c.typ < 1.0f) ? min(A.need_far, tot) : 0) : (tot < need ? tot : 0));
+        const int need_far = A.need_far == 0 ? 0 : (c.open_row ? (c.topp_on && !(c.typ < 1.0f) ? min(A.need_far, tot) : 0) : min(A.need_topk, tot));
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             if (run < need && run + n[i] >= need) S.edge = PER * tid + i;
@@ -675,7 +677,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         tau_x = S.edge >= 0 ? below_bin(S.edge) : -INFINITY;
         // (what cannot matter to the whole sum is no use to an open row's head: a sharp row has few elements that can)
         far_x = S.edge_far >= 0 ? fmaxf(below_bin(S.edge_far), c.open_row ? thr_of(total) : -INFINITY) : -INFINITY;
-        far = far_x > -INFINITY && far_x < (tau_x > -INFINITY ? tau_x : INFINITY);
+        far = far_x > -INFINITY && (c.open_row ? far_x < (tau_x > -INFINITY ? tau_x : INFINITY) : far_x > tau_x);
         // F_NARROW: a top-k so wide for the vocabulary that fewer ranges than candidates exist (one range
         // per thread of the widest layout: oG blocks of NT threads with oL logits each). Such rows report
         // the order of equal probabilities the way the descending walk sees it.
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
         const bool past_head = c.n_lim + 1 > (c.open_row ? HEAD_NEED : HEAD_MOST);
         // (too few lanes to bound the head: row_finish narrows it down from the list)
         pl.flags = ((c.pure || past_head || !(tau_x > -INFINITY)) ? F_LIST : 0) | (c.pure ? F_PURE : 0) | (narrow ? F_NARROW : 0) | (jump ? F_JUMP : 0) |
-                   (far ? F_FAR | (tau_x > -INFINITY ? 0 : F_ALLNEAR) : 0) | ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
+                   (far ? F_FAR | (c.open_row && tau_x > -INFINITY ? 0 : F_ALLNEAR) : 0) | ((filter_ok && fabsf(top) > 1.0e-6f && c.T > 1.0e-9f && c.T < 1.0e9f) ? F_FASTDIV : 0);
         if (jump) pl.c.late = true;
         pl.top = top; pl.tau_bits = c.pure ? 0xffffffffu : bits_of(tau_x);
         pl.tau_far = far ? bits_of(far_x) : pl.tau_bits;
@@ -1515,7 +1517,8 @@ __global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__
     const int nfar = (pl.flags & F_FAR) ? head->nfar : 0, nfirst = all_near ? 0 : ncand;   // of the near list, with the far one
     const bool far = nfar > 0 && nfirst + nfar <= HEADCAP && (!all_near || (ncand > HEADCAP && (g.open_row || nfar >= pl.need)));
     const int nc = far ? nfirst + nfar : ncand;
-    const int nwalk = far && g.open_row ? (all_near ? HEAD_NEED : ncand) : nc;   // the near head alone would have walked on from here
+    // (the near head alone, or what the general form makes of it, would have walked on from here)
+    const int nwalk = far && g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST) ? (all_near ? pl.need : ncand) : nc;
     const bool narrow = (pl.flags & F_NARROW) != 0;
     auto queue_row = [&](int state, int why = 0) {
 #ifdef MOLLA_SAMPLE_TESTING
@@ -3395,8 +3398,11 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     A.a.Vg = a.V; A.a.col0 = 0; A.a.mode = 0;
     A.ntile = (a.V + TILE - 1) / TILE;
     A.nspan = (a.V + SPAN - 1) / SPAN;
-    // of V logits in no order, FAR_HEAD reach the value that this share of the lanes' maxima reaches
-    A.need_far = a.V > HEADCAP && a.V <= FAR_MOST_V ? (int)ceil((a.V + 31) / 32 * (1.0 - pow(1.0 - (double)FAR_HEAD / a.V, 32.0))) : 0;
+    // of V logits in no order, n reach the value that this share of the lanes' maxima reaches
+    const bool far = a.V > HEADCAP && a.V <= FAR_MOST_V;
+    auto lanes_for = [&](double n) { return far ? (int)ceil((a.V + 31) / 32 * (1.0 - pow(1.0 - n / a.V, 32.0))) : 0; };
+    A.need_far = lanes_for(FAR_HEAD);
+    A.need_topk = lanes_for(FAR_TOPK);
     narrow_layout(a.V, a.layout_B > 0 ? a.layout_B : a.B, sms, A.oG, A.oVc, A.oL);
     const int rows = rows_in_flight(a.B, a.V);
     lay_out(A, (char *)d_workspace, rows, a.V);

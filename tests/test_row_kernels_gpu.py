@@ -92,7 +92,7 @@ def test_pick_rows_asks_for_what_its_kernels_use(dev, lib, B, V, per_logit):
 
 @pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("steps", [0, 16])
-@pytest.mark.parametrize("V", [2049, 3000, 4064, 4097, 20000, 65536, 65537])
+@pytest.mark.parametrize("V", [2049, 3000, 4064, 4097, 20000, 40000, 65536, 65537])
 def test_heads_of_short_rows(dev, lib, oracle, V, steps):
     """Nuclei that end in the head's near list, in its far one and behind both; a top-k that asks for more
     elements than the row has lanes; min-p; logits of many values and of few (whole sixteenths: equal values at
@@ -101,10 +101,10 @@ def test_heads_of_short_rows(dev, lib, oracle, V, steps):
     w = W.config3(seed=V + steps, B=B, V=V, H=16)
     rng = np.random.default_rng(V + steps)
     w["temperature"][:] = rng.uniform(0.2, 1.6, B)
-    w["top_k"][:] = np.int32([0, 0, 0, 100, 127])[np.arange(B) % 5]
+    w["top_k"][:] = np.int32([0, 0, 0, 100, 127, 0, 600, 1025, 1026, 1500])[np.arange(B) % 10]
     w["top_p"][:] = rng.choice(np.float32([0.3, 0.6, 0.9, 0.95, 0.999]), B)
     w["min_p"][::7] = rng.choice(np.float32([0.001, 0.05]), len(w["min_p"][::7]))
-    w["typical_p"][:] = np.where((w["top_k"] > 0) & (np.arange(B) % 4 == 0), np.float32(0.9), np.float32(1.0))
+    w["typical_p"][:] = np.where((w["top_k"] > 0) & (w["top_k"] < 128) & (np.arange(B) % 4 == 0), np.float32(0.9), np.float32(1.0))
     if steps:
         w["logits"] = (np.round(w["logits"] * steps) / steps).astype(np.float32)
     # (every mismatch has to be explained by a mark: with few values most rows have equal ones at an edge)
