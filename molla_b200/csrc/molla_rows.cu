@@ -71,16 +71,19 @@ struct __align__(8) TilePlan { float thr, est; };
 struct __align__(8) TileOut { unsigned int ioff; unsigned short cnt, nitem; };   // its items in the row's, entries in its list
 
 // Items: the exact sequential sum of a tile's values as a short program. While the running sum s
-// stays in one binade, fl(s + v) is s plus rne(v / ulp) units, an integer that does not depend on s;
-// in the bit pattern of s, adding k units is the integer addition of k. So a run of lanes whose
-// values all round by themselves is one number (kind RUN). A lane near the end of a binade carries
-// the numbers of both binades (DUAL); a lane with a rounding tie, a value of a quarter of the sum or
-// a guess that spans more is added value by value (STEP). The binades are guessed from the estimated
+// stays in one binade, fl(s + v) is s plus rne(v / ulp) units; in the bit pattern of s, adding k units is
+// the integer addition of k. Only where v / ulp ends in a half (a rounding tie) does the integer depend on s,
+// and then only on the parity of its bit pattern. So any stretch of values is two numbers, the units it adds to
+// an even and to an odd pattern; they differ by one at most (fl does not change the order of two sums, and two
+// that have become equally even stay in step), and two stretches make one. A stretch of lanes whose
+// binade is certain is one such pair (kind RUN). A lane near the end of a binade carries
+// the pairs of both binades (DUAL); a lane that outgrows a binade by itself or whose
+// guess spans more is added value by value (STEP). The binades are guessed from the estimated
 // sum before the tile; whoever runs the items checks every guess against the exact sum and adds the
 // values one by one where it was wrong.
 enum { K_RUN = 0, K_DUAL = 1, K_STEP = 2 };
 struct __align__(16) Item {
-    unsigned int ka, kb;   // units of binade jb (RUN, DUAL) and of the next one (DUAL)
+    unsigned int ka, kb;   // units of binade jb (RUN, DUAL) and of the next one (DUAL), see units()
     unsigned int meta;     // biased exponent of the binade (8 bits), kind (2), place of the values (8; 255: the list), tile (10)
     unsigned int oc;       // entries (11 bits), first entry in the tile's list (10), number of the item in its tile (7)
     __device__ __forceinline__ unsigned int jb() const { return meta & 0xffu; }
@@ -91,6 +94,18 @@ struct __align__(16) Item {
     __device__ __forceinline__ int off() const { return (int)((oc >> 11) & 0x3ffu); }
     __device__ __forceinline__ int num() const { return (int)(oc >> 21); }
 };
+// A pair of units in one word: those added to an even pattern (30 bits; they stay below 2^25) and what an odd one
+// gets more of them (-1, 0 or 1).
+__device__ __forceinline__ unsigned int pair_of(unsigned int even, unsigned int odd) { return even | ((odd - even) << 30); }
+__device__ __forceinline__ bool parity_free(unsigned int pair) { return (pair >> 30) == 0u; }
+__device__ __forceinline__ unsigned int units(unsigned int pair, unsigned int sb) {   // added to the pattern sb
+    return (pair & 0x3fffffffu) + ((sb & 1u) ? (unsigned int)((int)pair >> 30) : 0u);
+}
+// Stretch a, then stretch b (even: to an even pattern, odd: to an odd one).
+struct Units { unsigned int even, odd; };
+__device__ __forceinline__ Units then(const Units &a, const Units &b) {
+    return Units{a.even + ((a.even & 1u) ? b.odd : b.even), a.odd + ((a.odd & 1u) ? b.even : b.odd)};
+}
 
 // ---- settings ---------------------------------------------------------------------------------
 struct __align__(16) RowCfg {
@@ -309,7 +324,7 @@ __device__ __forceinline__ void span_fetch(const BatchArgs &a, long long lrow, i
 // Waits for what span_fetch asked for and caps, masks, biases and penalises it. Threads
 // 0..SPAN_THREADS-1 work (`active`), all threads of the block take part in the barriers; each warp may
 // then use its own tile.
-__device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, float *sx, SpanScratch *s, bool active) {
+__device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, float *sx, SpanScratch *s, bool active, bool mine_on = true) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(SPAN, a.V - c0);
     const int e0 = warp * TILE;
@@ -338,7 +353,7 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
     if (active) {
         cp_wait();
         __syncwarp();
-        const int m = n - (e0 + lane * 32);  // this lane's logits that exist
+        const int m = mine_on ? n - (e0 + lane * 32) : 0;  // this lane's logits that exist
         if (a.softcap > 0.0f) {
 #pragma unroll 1
             for (int j = 0; j < min(32, m); j++) mine[j] = softcap_slow(mine[j], a.softcap);
@@ -740,10 +755,11 @@ __global__ void __launch_bounds__(NT) row_plan_kernel(const __grid_constant__ Ro
 }
 
 // =============================================================================
-// Kernel 3: exponentials, candidates, items. Bound: instructions and shared memory latency, about 2300
-// warp instructions a tile that keeps two thirds (early tiles and warm rows keep nearly all, cold ones few):
-// 256 rows of 151936 take 76 us, 512 of 262144 240, issuing in two thirds of the active cycles. Evaluating in full warps from a list of what
-// is kept, in place of each lane its own, gave 20 %.
+// Kernel 3: exponentials, candidates, items. Bound: instructions, and the latency of the plan's and the tile's loads:
+// about 1000 warp instructions a tile of a row whose list nobody wants (near_units), 2300 where it is wanted and two
+// thirds are kept. 256 rows of 151936, mixed, take 64 us (all evaluated in full and every tile cut into chunks: 74),
+// 512 of 262144 with a top-k of 1024 200 (245), issuing in 60 % of the active cycles. Evaluating in full warps from
+// a list of what is kept, in place of each lane its own, gave 20 %.
 // =============================================================================
 // A tile's list in shared memory: entry e at list[skew(e)] (a word is left out after every 32, so that
 // lanes that read their own chunks meet different banks). Lane l's chunk is entries [off, off + cnt):
@@ -766,6 +782,14 @@ __device__ __forceinline__ TileChunk tile_chunk(const float *list, int total) {
     return c;
 }
 
+__device__ __forceinline__ Item run_item(unsigned int pair, int j, int tile, int cnt, int off, int num) {
+    Item it;
+    it.ka = pair; it.kb = 0u;
+    it.meta = (unsigned int)(j + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18);
+    it.oc = (unsigned int)cnt | ((unsigned int)off << 11) | ((unsigned int)num << 21);
+    return it;
+}
+
 // The items of a tile's list cut into chunks, `est` = the estimated sum before the tile. Returns the
 // number of items; `care` = this lane's values are wanted one by one.
 // `alloc(n, c)` is called by all lanes with the number of items and of careful chunks among them and
@@ -785,32 +809,33 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     const int jl = fexpo(lo), jh = fexpo(hi);
     const bool usable = nonempty && lo > 0.0f && jh <= jl + 1 && jl >= -100 && jh <= 100;
     const bool two = usable && jh == jl + 1;
+    // the lane's values added to the smallest even and the smallest odd pattern of the binade (and of the next):
+    // the true sum rounds as the one of its parity does, as long as it stays in the binade
+    const unsigned int A1 = (unsigned int)(jl + 127) << 23, A2 = A1 + (1u << 23);
+    Units da{0u, 0u}, db{0u, 0u};
     bool bad = false;
-    float da = 0.0f, db = 0.0f;
     if (__any_sync(0xffffffffu, two)) {
         if (usable) {
-            const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
-            const float C2 = __fmul_rn(1.5f, fpow2(jl + 1)), h2 = fpow2(jl - 23);
+            float s0 = __uint_as_float(A1), s1 = __uint_as_float(A1 + 1u), t0 = __uint_as_float(A2), t1 = __uint_as_float(A2 + 1u);
 #pragma unroll 1
             for (int i = 0; i < cnt; i++) {
                 const float v = list[skew(off + i)];
-                const float q = __fsub_rn(__fadd_rn(v, C1), C1);
-                bad |= (fabsf(__fsub_rn(v, q)) == h1) | (v >= b1);
-                da = __fadd_rn(da, q);
-                const float q2 = __fsub_rn(__fadd_rn(v, C2), C2);
-                bad |= two & (fabsf(__fsub_rn(v, q2)) == h2);
-                db = __fadd_rn(db, q2);
+                s0 = __fadd_rn(s0, v); s1 = __fadd_rn(s1, v);
+                t0 = __fadd_rn(t0, v); t1 = __fadd_rn(t1, v);
             }
+            da = Units{__float_as_uint(s0) - A1, __float_as_uint(s1) - A1 - 1u};
+            db = Units{__float_as_uint(t0) - A2, __float_as_uint(t1) - A2 - 1u};
+            bad = __float_as_uint(s1) >= A2 || (two && __float_as_uint(t1) >= A2 + (1u << 23));
         }
     } else if (usable) {
-        const float C1 = __fmul_rn(1.5f, fpow2(jl)), h1 = fpow2(jl - 24), b1 = fpow2(jl - 1);
+        float s0 = __uint_as_float(A1), s1 = __uint_as_float(A1 + 1u);
 #pragma unroll 4
         for (int i = 0; i < cnt; i++) {
             const float v = list[skew(off + i)];
-            const float q = __fsub_rn(__fadd_rn(v, C1), C1);
-            bad |= (fabsf(__fsub_rn(v, q)) == h1) | (v >= b1);
-            da = __fadd_rn(da, q);
+            s0 = __fadd_rn(s0, v); s1 = __fadd_rn(s1, v);
         }
+        da = Units{__float_as_uint(s0) - A1, __float_as_uint(s1) - A1 - 1u};
+        bad = __float_as_uint(s1) >= A2;
     }
     const bool step = nonempty && (!usable || bad);
     const unsigned int ne = __ballot_sync(0xffffffffu, nonempty);
@@ -822,31 +847,46 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     const bool prev_alone = ((__ballot_sync(0xffffffffu, step || two) >> prev) & 1u) != 0u;
     care = step || two || (nonempty && below && !prev_alone && pj != jl);
     const unsigned int cm = __ballot_sync(0xffffffffu, care);
-    const float units = fpow2(max(min(23 - jl, 127), -126));
-    const unsigned int ka = (usable && !bad) ? __float2uint_rn(__fmul_rn(da, units)) : 0u;   // da is a multiple of 2^(jl-23), below 2^24 of them
     my_place = 255;
-    if (cm == 0u) {
-        const unsigned int k = __reduce_add_sync(0xffffffffu, ka);
-        if (k == 0u) return 0;
-        const int j0 = __shfl_sync(0xffffffffu, jl, __ffs((int)ne) - 1);
-        Item *out = alloc(1, 0);
-        if (lane == 0) {
-            Item it;
-            it.ka = k; it.kb = 0; it.meta = (unsigned int)(j0 + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18); it.oc = (unsigned int)total;
-            out[0] = it;
+    const int j0 = __shfl_sync(0xffffffffu, jl, max(__ffs((int)ne) - 1, 0));
+    if (__popc(ne) >= 4 && __all_sync(0xffffffffu, !nonempty || (two && !bad && jl == j0))) {
+        // A sum that stays near a power of two for long: most such tiles do not cross it, so several lanes make an item,
+        // of 128 values at most, which are in the list. (With an item a lane, one row in some hundreds of 262144 had more
+        // careful chunks than row_head takes, and row_tail took 200 us for it.)
+        const int lg = total <= 128 ? 5 : (total <= 256 ? 4 : (total <= 512 ? 3 : 2)), in = lane & ((1 << lg) - 1);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const Units a{__shfl_up_sync(0xffffffffu, da.even, o), __shfl_up_sync(0xffffffffu, da.odd, o)};
+            const Units b{__shfl_up_sync(0xffffffffu, db.even, o), __shfl_up_sync(0xffffffffu, db.odd, o)};
+            if (in >= o) { da = then(a, da); db = then(b, db); }
         }
-        return 1;
+        const int first = __shfl_sync(0xffffffffu, off, lane - in), n = 32 >> lg;
+        Item *out = alloc(n, 0);
+        if (in == (1 << lg) - 1) {
+            Item it;
+            it.ka = pair_of(da.even, da.odd); it.kb = pair_of(db.even, db.odd);
+            it.meta = (unsigned int)(j0 + 127) | (K_DUAL << 8) | (255u << 10) | ((unsigned int)tile << 18);
+            it.oc = (unsigned int)(off + cnt - first) | ((unsigned int)first << 11) | ((unsigned int)(lane >> lg) << 21);
+            out[lane >> lg] = it;
+        }
+        return n;
     }
     // the runs between the careful lanes: a run goes with the careful lane behind it, or closes the tile
-    const unsigned int kin = warp_incl_scan(care ? 0u : ka, lane);
     const unsigned int lt = (1u << lane) - 1u, cb = cm & lt;
-    const int lastc = cb ? 31 - __clz((int)cb) : -1, last = 31 - __clz((int)cm);
-    const unsigned int kprev = __shfl_sync(0xffffffffu, kin, lastc < 0 ? 0 : lastc);
-    const unsigned int kin_up = __shfl_up_sync(0xffffffffu, kin, 1);
-    const unsigned int kr = (lane == 0 ? 0u : kin_up) - (lastc < 0 ? 0u : kprev);   // units of the run that ends before this lane
+    const int lastc = cb ? 31 - __clz((int)cb) : -1, last = cm ? 31 - __clz((int)cm) : -1;
+    Units k = care || !usable ? Units{0u, 0u} : da;   // of the run up to this lane and with it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Units before{__shfl_up_sync(0xffffffffu, k.even, o), __shfl_up_sync(0xffffffffu, k.odd, o)};
+        if (lane - o > lastc && !care) k = then(before, k);
+    }
+    const unsigned int kp = pair_of(k.even, k.odd);
+    unsigned int kr = __shfl_up_sync(0xffffffffu, kp, 1);    // of the run that ends before this lane
+    if (lane == 0) kr = 0u;
     const unsigned int runm = __ballot_sync(0xffffffffu, care && kr != 0u);          // careful lanes with a run before them
-    const unsigned int ktail = __shfl_sync(0xffffffffu, kin, 31) - __shfl_sync(0xffffffffu, kin, last);
+    const unsigned int ktail = last == 31 ? 0u : __shfl_sync(0xffffffffu, kp, 31);
     const int ncare = __popc(cm), n = ncare + __popc(runm) + (ktail ? 1 : 0);
+    if (n == 0) return 0;
     Item *out = alloc(n, ncare);
     // the first lane of a run that holds anything, for its binade and its first entry
     auto first_in = [&](int from) { const unsigned int m = ne & ~(from < 0 ? 0u : (from == 31 ? 0xffffffffu : ((2u << from) - 1u))); return m ? __ffs((int)m) - 1 : 31; };
@@ -855,26 +895,17 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     const int tj = __shfl_sync(0xffffffffu, jl, tl), to = __shfl_sync(0xffffffffu, off, tl);
     if (care) {
         int i = __popc(cb) + __popc(runm & lt);
-        Item it;
-        if ((runm >> lane) & 1u) {
-            it.ka = kr; it.kb = 0; it.meta = (unsigned int)(fj + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18);
-            it.oc = (unsigned int)(off - fo) | ((unsigned int)fo << 11) | ((unsigned int)i << 21);
-            out[i++] = it;
-        }
+        if ((runm >> lane) & 1u) { out[i] = run_item(kr, fj, tile, off - fo, fo, i); i++; }
         my_place = place(__popc(cb));
         const bool dual = two && !bad;
-        it.ka = dual ? ka : 0u;
-        it.kb = dual ? __float2uint_rn(__fmul_rn(db, fpow2(max(min(22 - jl, 127), -126)))) : 0u;
+        Item it;
+        it.ka = dual ? pair_of(da.even, da.odd) : 0u;
+        it.kb = dual ? pair_of(db.even, db.odd) : 0u;
         it.meta = (dual ? ((unsigned int)(jl + 127) | (K_DUAL << 8)) : (unsigned int)(K_STEP << 8)) | ((unsigned int)my_place << 10) | ((unsigned int)tile << 18);
         it.oc = (unsigned int)cnt | ((unsigned int)off << 11) | ((unsigned int)i << 21);
         out[i] = it;
     }
-    if (ktail && lane == 0) {
-        Item it;
-        it.ka = ktail; it.kb = 0; it.meta = (unsigned int)(tj + 127) | (K_RUN << 8) | (255u << 10) | ((unsigned int)tile << 18);
-        it.oc = (unsigned int)(total - to) | ((unsigned int)to << 11) | ((unsigned int)(n - 1) << 21);
-        out[n - 1] = it;
-    }
+    if (ktail && lane == 0) out[n - 1] = run_item(ktail, tj, tile, total - to, to, n - 1);
     return n;
 }
 
@@ -942,6 +973,73 @@ __device__ __forceinline__ void store_care(float *care, const float *list, const
     }
 }
 
+// A tile's candidates for the head to their list, or to the second one of F_FAR: `wanted` names, per lane, entries
+// entry(b) for every set bit b, with the bits value(e) and the token token(e). A tile asks for its places once. (One
+// request per value, each waited for before the next two are evaluated, took 0.7 us each: up to 22 us a tile in short
+// rows, whose few tiles hold all candidates.)
+template <class ENTRY, class VALUE, class TOKEN>
+__device__ __forceinline__ void put_candidates(const RowsArgs &A, int rr, const RowPlan &pl, unsigned int wanted, ENTRY entry, VALUE value, TOKEN token) {
+    if (!__any_sync(0xffffffffu, wanted != 0u)) return;
+    const int lane = threadIdx.x & 31;
+    RowHead *head = A.head(rr);
+    auto put = [&](unsigned int m, int *count, unsigned long long *to) {
+        const int n = __popc(m), inc = warp_incl_scan(n, lane);
+        int pos = 0;
+        if (lane == 31 && inc) pos = atomicAdd(count, inc);
+        pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
+#pragma unroll 1
+        for (; m; m &= m - 1u, pos++) {
+            const int e = entry(__ffs((int)m) - 1);
+            if (pos < HEADCAP) to[pos] = make_key(value(e), token(e));
+        }
+    };
+    unsigned int near = wanted;
+    if (pl.flags & F_FAR) {
+        unsigned int beyond = 0u;
+#pragma unroll 1
+        for (unsigned int m = wanted; m; m &= m - 1u) {
+            const unsigned int eb = value(entry(__ffs((int)m) - 1)), one = m & (0u - m);
+            if (eb < pl.tau_bits) near ^= one;
+            if (eb >= pl.tau_far && ((pl.flags & F_ALLNEAR) || eb < pl.tau_bits)) beyond |= one;
+        }
+        put(beyond, &head->nfar, A.far(rr));
+    }
+    put(near, &head->ncand, A.cand(rr));
+}
+
+// The units of binade j that a lane's 32 logits add to a sum there, from hardware exponentials: those whose number
+// is certain, added up in `k`; returns which of them are not (and those that reach `tau`, whose value is wanted).
+//
+// y = ex2(x f + g), f = log2 e / T, g = 23 - j - top log2 e, against Y = expf_pinned(fl(fl(x / T) - top)) 2^(23 - j), of
+// which fl adds rne(Y) units. Relative errors in units of 2^-24, for what reaches a quarter of a unit (further down both
+// round to nothing), with P = |top| and D = 26 + |j|, the width in powers of two between a quarter of a unit and
+// the maximum: f is off by 2, so x f, at most 1.443 P + D, by twice that; g by 1.443 P + D; the sum, of 24 at most where
+// it matters, by 24; times ln 2: 3 P + 2.1 D + 17. ex2 by 4. Y itself against exact arithmetic: the quotient by
+// P + 0.7 D, the difference by 0.7 D, the exponential by 3. Together 4 P + 3.5 D + 24, and a quarter more here. A y whose
+// distance to the nearest integer plus its error stays below a half has the same integer as Y.
+constexpr int EXACT_MOST = 256;   // of a tile evaluated in full at most; else all that it keeps is
+__device__ __forceinline__ unsigned int near_units(const float *tile, int lane, float T, float top, int j, unsigned int tau, unsigned int &k) {
+    const float f = 1.44269504f / T, g = (float)((double)(23 - j) - (double)top * 1.4426950408889634);
+    const float err = (5.0f * fabsf(top) + 4.4f * (float)(26 + abs(j)) + 30.0f) * (1.0f / 16777216.0f);
+    // (a candidate near the smallest floats is not known by y to within a thousandth: all are evaluated then)
+    const float edge = tau < (27u << 23) ? -1.0f : (0.999f - 2.0f * err) * __uint_as_float(tau) * fpow2(min(23 - j, 127)), magic = 12582912.0f;
+    const float4 *mine = reinterpret_cast<const float4 *>(tile + lane * PITCH);
+    unsigned int m = 0u, sum = 0u;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const float4 v = mine[q];
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float y = ex2_approx(__fmaf_rn(x[u], f, g)), t = __fadd_rn(y, magic), r = __fsub_rn(y, __fsub_rn(t, magic));
+            const bool sure = __fmaf_rn(y, err, fabsf(r)) < 0.49999f && y < edge;   // (false for infinities and NaN)
+            if (sure) sum += __float_as_uint(t) - __float_as_uint(magic); else m |= 1u << (4 * q + u);
+        }
+    }
+    k = sum;
+    return m;
+}
+
 __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_constant__ RowsArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SpanShared *S = reinterpret_cast<SpanShared *>(smem_raw);
@@ -950,73 +1048,134 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     // (the last spans first: of a block larger than the L2 they are what tile_stats has left there)
     const int b = (int)(gridDim.x - 1u - blockIdx.x), rr = b / A.nspan, span = b - rr * A.nspan, r = A.r0 + rr;
     RowHead *head = A.head(rr);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
+    const size_t gt = (size_t)rr * A.ntile + min(tile, A.ntile - 1);
+    const TilePlan tp = A.tp[gt];
+    const bool hot = tile < A.ntile && A.ts[gt].tmax >= tp.thr;
     const RowPlan pl = head->plan;
     if (pl.kind == PLAN_DONE) return;
+    auto store_cold = [&]() {
+        if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = 0u;
+        if (lane == 0) { TileOut o; o.ioff = 0u; o.cnt = 0; o.nitem = 0; A.to(rr)[tile] = o; }
+    };
     const BatchArgs &a = A.a;
     const RowCfg &c = pl.c;
-    span_fetch(a, c.lrow, span * SPAN, S->x);
-    span_ready(a, c, r, span * SPAN, S->x, &S->s, true);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
+    // a tile whose maximum does not reach its bound keeps nothing
+    if (c.npatch > 0 ? !__syncthreads_or(hot) : !hot) {
+        if (tile < A.ntile) store_cold();
+        return;
+    }
+    if (hot) span_fetch(a, c.lrow, span * SPAN, S->x);
+    span_ready(a, c, r, span * SPAN, S->x, &S->s, true, hot);
     if (tile >= A.ntile) return;
-    const size_t gt = (size_t)rr * A.ntile + tile;
-    const TilePlan tp = A.tp[gt];
+    if (!hot) { store_cold(); return; }
     float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = min(pl.tau_bits, pl.tau_far);
     unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
-    unsigned int w0 = 0u, w1 = 0u;   // this lane's candidates among the entries it evaluates
-    const TileEval t = tile_eval(list, idx, tp.thr, c.T, __fdiv_rn(1.0f, c.T), pl.top, (pl.flags & F_FASTDIV) && tp.thr > -INFINITY,
-        [&](unsigned int eb, bool second, unsigned int bit) { if (eb >= tau) { if (second) w1 |= bit; else w0 |= bit; } });
-    // A tile asks for its candidates' places once. (One request per value, each waited for before the next two
-    // are evaluated, took 0.7 us each: up to 22 us a tile in short rows, whose few tiles hold all candidates.)
-    const unsigned int wanted = w0 | (w1 << 16);
-    if (__any_sync(0xffffffffu, wanted != 0u)) {
-        auto entry = [&](unsigned int m) { const int b = __ffs((int)m) - 1; return (b & 15) * 64 + (b & 16) * 2 + lane; };
-        auto put = [&](unsigned int m, int *count, unsigned long long *to) {
-            const int n = __popc(m), inc = warp_incl_scan(n, lane);
-            int pos = 0;
-            if (lane == 31 && inc) pos = atomicAdd(count, inc);
-            pos = __shfl_sync(0xffffffffu, pos, 31) + inc - n;
-#pragma unroll 1
-            for (; m; m &= m - 1u, pos++) {
-                const int e = entry(m);
-                if (pos < HEADCAP) to[pos] = make_key(__float_as_uint(list[skew(e)]), tile * TILE + (t.total == TILE ? e : (int)idx[e]));
-            }
-        };
-        unsigned int near = wanted;
-        if (pl.flags & F_FAR) {
-            unsigned int beyond = 0u;
-#pragma unroll 1
-            for (unsigned int m = wanted; m; m &= m - 1u) {
-                const unsigned int eb = __float_as_uint(list[skew(entry(m))]), one = m & (0u - m);
-                if (eb < pl.tau_bits) near ^= one;
-                if (eb >= pl.tau_far && ((pl.flags & F_ALLNEAR) || eb < pl.tau_bits)) beyond |= one;
-            }
-            put(beyond, &head->nfar, A.far(rr));
+    // Most tiles lie inside one binade and hold no tie: their sum is a number of its units, in any order, added up
+    // on the way. (Chunks and items for all tiles took half again as many instructions.)
+    const float qlo = tp.est * (1.0f - 1.0f / 1024.0f);
+    const int qj = fexpo(qlo);
+    bool quick = qlo > 0.0f && qj >= -100;
+    const float qc = __fmul_rn(1.5f, fpow2(quick ? qj : 0)), qh = fpow2(quick ? qj - 24 : -24), qb = fpow2(quick ? qj - 1 : -1);
+    unsigned int qk = 0u;
+    bool qbad = false;
+    auto add_units = [&](float e) {
+        const float s = __fadd_rn(e, qc);
+        qk += __float_as_uint(s) - __float_as_uint(qc);
+        qbad |= (fabsf(__fsub_rn(e, __fsub_rn(s, qc))) == qh) | (e >= qb);
+    };
+    auto quick_sum = [&]() {   // is the sum that of one binade's units? (qk: all of them)
+        if (!quick || __any_sync(0xffffffffu, qbad)) return false;
+        qk = __reduce_add_sync(0xffffffffu, qk);
+        const float end = tp.est + (float)qk * fpow2(max(qj - 23, -126));
+        return fexpo(end * (1.0f + 1.0f / 2048.0f)) == qj;
+    };
+    int ni = 0, cnt = TILE;
+    unsigned int i0 = 0u;
+    auto store_out = [&]() {
+        if (lane != 0) return;
+        TileOut o;
+        o.ioff = i0; o.cnt = (unsigned short)cnt; o.nitem = (unsigned short)ni;
+        A.to(rr)[tile] = o;
+    };
+    auto store_run = [&]() {
+        ni = qk ? 1 : 0;
+        if (lane == 0 && qk) {
+            i0 = (unsigned int)atomicAdd(&head->nitem, 1);
+            A.items(rr)[i0] = run_item(qk, qj, tile, cnt, 0, 0);
         }
-        put(near, &head->ncand, A.cand(rr));
+    };
+    const bool fast = (pl.flags & F_FASTDIV) && tp.thr > -INFINITY;
+    const float rT = __fdiv_rn(1.0f, c.T);
+    if (quick && fast && !(pl.flags & F_LIST)) {
+        // Nobody asks for this row's list, only for its sum and its candidates, and nearly all that is kept adds
+        // few units, whose number a hardware exponential tells unless it is near a half: see near_units. The others
+        // are evaluated as they have to be. Per tile 600 instructions, where evaluating all that is kept takes 1300
+        // (at a fifth of the logits kept: 1024 rows of 262144 with a top-k of 1024, 450 us).
+        const unsigned int m = near_units(list, lane, c.T, pl.top, qj, tau, qk);
+        const int mine = __popc(m), inc = warp_incl_scan(mine, lane), total = __shfl_sync(0xffffffffu, inc, 31);
+        if (total <= EXACT_MOST) {
+            float *val = reinterpret_cast<float *>(idx + EXACT_MOST);
+            unsigned short *o = idx + (inc - mine);
+#pragma unroll 1
+            for (unsigned int w = m; w; w &= w - 1u) *o++ = (unsigned short)(lane * 32 + __ffs((int)w) - 1);
+            __syncwarp();
+            unsigned int wanted = 0u, bit = 1u;
+            const bool one = c.T == 1.0f;
+#pragma unroll 1
+            for (int i = lane; i - lane < total; i += 32, bit <<= 1) {
+                const int p = i < total ? (int)idx[i] : 0;
+                const float x = list[p + 4 * (p >> 5)];
+                if (i < total && x >= tp.thr) {   // (not a number: never kept)
+                    const float e = expf_pinned_nonpos(__fsub_rn(one ? x : div_by(x, c.T, rT), pl.top));
+                    add_units(e);
+                    val[i] = e;
+                    if (__float_as_uint(e) >= tau) wanted |= bit;
+                }
+            }
+            __syncwarp();
+            if (quick_sum()) {
+                put_candidates(A, rr, pl, wanted, [&](int b) { return b * 32 + lane; }, [&](int e) { return __float_as_uint(val[e]); },
+                               [&](int e) { return tile * TILE + (int)idx[e]; });
+                store_run();
+                store_out();
+                return;
+            }
+            __syncwarp();
+        }
+        qk = 0u; qbad = false;
     }
-    const TileChunk ch = tile_chunk(list, t.total);
-    bool care;
-    int my_place, c0 = CARE_PLACES;
-    unsigned int i0 = 0;
-    const int ni = tile_items(list, ch, tp.est, tile,
-        [&](int n, int nc) -> Item * {
-            if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, n); if (nc) c0 = atomicAdd(&head->ncare, nc); }
-            i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
-            return A.items(rr) + i0;
-        },
-        [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
-    store_care(A.care(rr), list, ch, my_place);
-    const bool whole = (pl.flags & F_LIST) || __any_sync(0xffffffffu, care && my_place == 255);
+    unsigned int w0 = 0u, w1 = 0u;   // this lane's candidates among the entries it evaluates
+    const TileEval t = tile_eval(list, idx, tp.thr, c.T, rT, pl.top, fast,
+        [&](unsigned int eb, bool second, unsigned int bit) {
+            if (eb >= tau) { if (second) w1 |= bit; else w0 |= bit; }
+            add_units(__uint_as_float(eb));
+        });
+    cnt = t.total;
+    put_candidates(A, rr, pl, w0 | (w1 << 16), [&](int b) { return (b & 15) * 64 + (b & 16) * 2 + lane; },
+                   [&](int e) { return __float_as_uint(list[skew(e)]); }, [&](int e) { return tile * TILE + (t.total == TILE ? e : (int)idx[e]); });
+    bool whole = (pl.flags & F_LIST) != 0;
+    if (quick_sum()) store_run();
+    else {
+        const TileChunk ch = tile_chunk(list, t.total);
+        bool care;
+        int my_place, c0 = CARE_PLACES;
+        ni = tile_items(list, ch, tp.est, tile,
+            [&](int n, int nc) -> Item * {
+                if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, n); if (nc) c0 = atomicAdd(&head->ncare, nc); }
+                i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
+                return A.items(rr) + i0;
+            },
+            [&](int i) { return c0 + i < CARE_PLACES ? c0 + i : 255; }, care, my_place);
+        store_care(A.care(rr), list, ch, my_place);
+        whole = whole || __any_sync(0xffffffffu, care && my_place == 255);
+    }
     if (whole)
 #pragma unroll 1
         for (int i = lane; i < t.total; i += 32) A.elist[gt * TILE + i] = list[skew(i)];
     if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = t.keep;
-    if (lane == 0) {
-        TileOut o;
-        o.ioff = i0; o.cnt = (unsigned short)t.total; o.nitem = (unsigned short)ni;
-        A.to(rr)[tile] = o;
-    }
+    store_out();
 }
 
 // =============================================================================
@@ -1278,7 +1437,7 @@ struct WalkLoads {
                 const bool run = it[u].kind() == K_RUN;
                 bool prev_run = false;
                 if (i > 0) { const Item p = W->items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
-                if (!run || (prev_run && pj[u] != it[u].jb())) { care |= 1u << u; n++; }   // (a change of binade between two runs: a wrong guess)
+                if (!run || !parity_free(it[u].ka) || (prev_run && pj[u] != it[u].jb())) { care |= 1u << u; n++; }   // (a change of binade between two runs: a wrong guess)
                 else k += it[u].ka;
             }
         }
@@ -1326,21 +1485,35 @@ __device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsig
     if (q + lane < nrec) c = W->rec[q + lane];
     unsigned int kp = __shfl_up_sync(0xffffffffu, c.k, 1);
     if (lane == 0) kp = kdone;
-    const unsigned int runs = c.k - kp, jb = (c.meta >> 16) & 0xffu, d = runs + (e == jb ? c.ka : c.kb);
-    const bool can = q + lane < nrec && kind_of(c) == K_DUAL && (e == jb || e == jb + 1u) &&
+    const unsigned int runs = c.k - kp, jb = (c.meta >> 16) & 0xffu, kind = kind_of(c), own = e == jb ? c.ka : c.kb;
+    const bool can = q + lane < nrec && (kind == K_DUAL ? (e == jb || e == jb + 1u) : (kind == K_RUN && e == jb && (own & 0x3fffffffu) < (1u << 24))) &&
                      (runs == 0u || ((c.meta & 0xffu) == e && runs < (1u << 24)));
-    const unsigned int inc = warp_incl_scan(can ? d : 0u, lane);
+    Units d{0u, 0u};
+    if (can) d = Units{runs + units(own, runs), runs + units(own, runs + 1u)};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Units before{__shfl_up_sync(0xffffffffu, d.even, o), __shfl_up_sync(0xffffffffu, d.odd, o)};
+        if (lane >= o) d = then(before, d);
+    }
+    const unsigned int inc = (sb & 1u) ? d.odd : d.even;
     const unsigned int stop = __ballot_sync(0xffffffffu, !can || ((sb + inc) >> 23) != e);
     const int n = stop ? __ffs((int)stop) - 1 : 32;
-    if (lane < n) W->sbs[q + lane] = sb + inc - d;
+    unsigned int before = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) before = 0u;
+    if (lane < n) W->sbs[q + lane] = sb + before;
     if (n > 0) sb += __shfl_sync(0xffffffffu, inc, n - 1);
     return make_uint2(sb, (unsigned int)n);
 }
 __device__ __noinline__ float add_listed(float s, const float *v, int n) {
     const int lane = threadIdx.x & 31;
-    const float mine = lane < n ? v[lane] : 0.0f;
+    float next = lane < n ? v[lane] : 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < n; i += 32) {
+        const float mine = next;
+        next = i + 32 + lane < n ? v[i + 32 + lane] : 0.0f;
 #pragma unroll 8
-    for (int e = 0; e < 32; e++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+        for (int e = 0; e < 32; e++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+    }
     return s;
 }
 __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, const float *list, int nrec, float &Z) {
@@ -1366,13 +1539,12 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
         kdone = c.k;
         sb = to;
         if (q == nrec) break;
-        const unsigned int e = sb >> 23, ta = sb + c.ka, tb = sb + c.kb;
-        const bool run = kind == K_RUN, low = e == jb;
-        if (run && (!low || (ta >> 23) != jb)) { fine = false; break; }
-        const unsigned int td = low ? ta : tb;
+        const bool run = kind == K_RUN, low = (sb >> 23) == jb;
+        const unsigned int e = sb >> 23, td = sb + units(low ? c.ka : c.kb, sb);
+        if (run && (!low || (td >> 23) != jb)) { fine = false; break; }
         if (run || (kind == K_DUAL && (low || e == jb + 1u) && (td >> 23) == e)) {
             sb = td;
-            if (kind_of(r) == K_DUAL && q + 1 < nrec) {
+            if (kind_of(r) != K_STEP && q + 1 < nrec) {
                 const uint2 t = dual_stretch(W, nrec, q + 1, sb, kdone);
                 sb = t.x;
                 q += (int)t.y;
@@ -1386,7 +1558,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
             continue;
         }
         if (place >= H_CARE) {   // (a row with many: their values are still in L2)
-            if (place == 255u) {   // (past CARE_PLACES: in its tile's list)
+            if (place == 255u) {   // (past CARE_PLACES, or several lanes' values: in its tile's list)
                 const Item it = W->items[W->ritem[q]];
                 sb = __float_as_uint(add_listed(__uint_as_float(sb), list + (size_t)it.tile() * TILE + it.off(), it.cnt()));
 #pragma unroll
@@ -2022,8 +2194,11 @@ __device__ __noinline__ void tile_again(CtxF &c, int t0, int t1, float *dst, boo
                                      (c.pl.flags & F_FASTDIV) && thr > -INFINITY, [](unsigned int, bool, unsigned int) {});
         float *to = to_list ? c.list + (size_t)t * TILE : dst;
 #pragma unroll 1
-        for (int i = c.lane; i < e.total; i += 32) to[i] = list[skew(i)];
-        if (to_list) const_cast<unsigned int *>(c.kmask)[(size_t)t * 32 + c.lane] = e.keep;
+        for (int i = c.lane; i < (to_list ? e.total : TILE); i += 32) to[i] = i < e.total ? list[skew(i)] : 0.0f;
+        if (to_list) {
+            const_cast<unsigned int *>(c.kmask)[(size_t)t * 32 + c.lane] = e.keep;
+            if (c.lane == 0) A->tcnt[t] = (unsigned short)e.total;   // (kernel 3 need not have counted them)
+        }
     }
     __syncthreads();
 }
@@ -2068,13 +2243,13 @@ __device__ void run_items(AuxF *A, int n, bool locate, float target) {
         it.ka = 0u; it.kb = 0u; it.meta = 0u; it.oc = 0u;
         if (i0 + lane < n) it = A->items[i0 + lane];
         const unsigned int jb = it.jb(), kind = it.kind();
-        const bool exists = i0 + lane < n;
-        const unsigned int incl = warp_incl_scan(kind == K_RUN ? it.ka : 0u, lane);
+        const bool plain = i0 + lane < n && kind == K_RUN && parity_free(it.ka);
+        const unsigned int incl = warp_incl_scan(plain ? it.ka : 0u, lane);
         int at = 0;
         unsigned int base = 0u;      // units of the runs before `at`
         while (at < 32 && i0 + at < n && need < 0 && !found) {
             const unsigned int j = sb >> 23, to = sb + (incl - base);
-            const bool fits = exists && kind == K_RUN && jb == j && (to >> 23) == j && !(locate && target < __uint_as_float(to));
+            const bool fits = plain && jb == j && (to >> 23) == j && !(locate && target < __uint_as_float(to));
             const unsigned int stop = ~__ballot_sync(0xffffffffu, fits) & ~((1u << at) - 1u);
             const int f = stop ? __ffs((int)stop) - 1 : 32;
             if (f > at) { sb = __shfl_sync(0xffffffffu, to, f - 1); at = f; }
@@ -2085,9 +2260,9 @@ __device__ void run_items(AuxF *A, int n, bool locate, float target) {
             const unsigned int kd = (meta >> 8) & 3u, jx = meta & 0xffu, e = sb >> 23;
             bool ok = false;
             unsigned int nx = sb;
-            if (kd == K_DUAL) {
-                if (e == jx) { nx = sb + ka; ok = (nx >> 23) == e; }
-                else if (e == jx + 1u) { nx = sb + kb; ok = (nx >> 23) == e; }
+            if (kd != K_STEP) {
+                if (e == jx) { nx = sb + units(ka, sb); ok = (nx >> 23) == e; }
+                else if (kd == K_DUAL && e == jx + 1u) { nx = sb + units(kb, sb); ok = (nx >> 23) == e; }
             }
             if (ok && !(locate && target < __uint_as_float(nx))) { sb = nx; at++; continue; }
             const unsigned int src = A->isrc[i0 + at];
@@ -2137,7 +2312,7 @@ __device__ __noinline__ float exact_sum(CtxF &c, bool locate, float target) {
             }
             const Item it = c.gitems[A->tio[lo] + (b0 + i - A->toff[lo])];
             unsigned int slot = 255u;
-            if (it.kind() != K_RUN) {
+            if (it.kind() != K_RUN && it.cnt() <= 32) {
                 const int q = satom_add(&A->ncare, 1);
                 if (q < CARE_CAP) { slot = (unsigned int)q; A->careidx[q] = (unsigned short)i; }
             }
@@ -2746,7 +2921,8 @@ __device__ __noinline__ bool tail_pure(CtxF &c) {
             const Item it = W->items[i];
             rec = it.kind() != K_RUN;
             ka = it.ka;
-            if (!rec && i > 0) { const Item p = W->items[i - 1]; rec = p.kind() == K_RUN && p.jb() != it.jb(); }
+            if (!rec && !parity_free(it.ka)) rec = true;
+            else if (!rec && i > 0) { const Item p = W->items[i - 1]; rec = p.kind() == K_RUN && p.jb() != it.jb(); }
         }
         const unsigned int m = __ballot_sync(0xffffffffu, rec);
         int from = 0;
@@ -2776,25 +2952,33 @@ __device__ __noinline__ bool tail_pure(CtxF &c) {
         const float *v = c.list + (size_t)it.tile() * TILE + it.off();
         int n = it.cnt(), e0 = 0;
         float s = __uint_as_float(sb);
-        if (n > 32) {
-            // the values of a run round by themselves: each lane adds up the units of its share
-            const int j = fexpo(s), per = (n + 31) >> 5, b0 = min(n, c.lane * per), b1 = min(n, b0 + per);
-            const float Cm = __fmul_rn(1.5f, fpow2(j));
-            unsigned int k = 0u;
+        if (n > 32 && it.kind() == K_RUN) {   // it stays in the sum's binade: each lane adds up the units of its share
+            const int per = (n + 31) >> 5, b0 = min(n, c.lane * per), b1 = min(n, b0 + per);
+            const unsigned int base = sb & 0x7f800000u;
+            float s0 = __uint_as_float(base), s1 = __uint_as_float(base + 1u);
 #pragma unroll 8
-            for (int e = b0; e < b1; e++) k += __float_as_uint(__fadd_rn(v[e], Cm)) - __float_as_uint(Cm);
-            const unsigned int inc = warp_incl_scan(k, c.lane);
-            const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(sb + inc));
+            for (int e = b0; e < b1; e++) { s0 = __fadd_rn(s0, v[e]); s1 = __fadd_rn(s1, v[e]); }
+            Units k{__float_as_uint(s0) - base, __float_as_uint(s1) - base - 1u};
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const Units before{__shfl_up_sync(0xffffffffu, k.even, o), __shfl_up_sync(0xffffffffu, k.odd, o)};
+                if (c.lane >= o) k = then(before, k);
+            }
+            const unsigned int to = sb + ((sb & 1u) ? k.odd : k.even);
+            const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(to));
             const int l = hit ? __ffs((int)hit) - 1 : 31;
-            s = __uint_as_float(sb + __shfl_sync(0xffffffffu, inc - k, l));
+            if (l > 0) s = __uint_as_float(__shfl_sync(0xffffffffu, to, l - 1));
             e0 = min(n, l * per); n = min(n, e0 + per) - e0;
         }
-        const float mine = c.lane < n ? v[e0 + c.lane] : 0.0f;
         int first = -1;
+#pragma unroll 1
+        for (int g0 = 0; g0 < n && first < 0; g0 += 32) {
+            const float mine = g0 + c.lane < n ? v[e0 + g0 + c.lane] : 0.0f;
 #pragma unroll 8
-        for (int e = 0; e < 32; e++) {
-            s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
-            if (first < 0 && e < n && target < s) first = e;
+            for (int e = 0; e < 32; e++) {
+                s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+                if (first < 0 && g0 + e < n && target < s) first = g0 + e;
+            }
         }
         if (first >= 0) { tile = it.tile(); at = it.off() + e0 + first; }
     }

@@ -49,6 +49,25 @@ def test_sums_that_stay_near_a_power_of_two(dev, lib, oracle, V):
 
 
 @pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("low,high", [(18, 26), (0, 30), (22, 25)])
+@pytest.mark.parametrize("V", [33, 1025, 9000, 40000])
+def test_sums_full_of_rounding_ties(dev, lib, oracle, V, low, high):
+    """Exponentials that are powers of two, down to a quarter of the sum's last bit: most additions are rounding ties,
+    whose direction depends on the sum before them. Equal values at every edge, which the rows are marked for; the
+    softmax denominator and the draw in vocabulary order have to be the sequential ones all the same."""
+    B = 16
+    rng = np.random.default_rng(V + low)
+    w = _kinds(W.config3(seed=V + low, B=B, V=V, H=4), B, V)
+    w["temperature"][:] = np.where(w["temperature"] > 0, np.float32(1.0), np.float32(0.0))
+    w["typical_p"][:] = 1.0
+    k = rng.integers(low, high, (B, V))
+    k[np.arange(B), rng.integers(0, V, B)] = 0
+    k[::2, 0] = 0
+    w["logits"] = (-np.log(2.0) * k).astype(np.float32)
+    compare(w, dev, oracle, f"ties, V={V}", max_exception_frac=1.0)
+
+
+@pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("V", [1000, 4097])
 def test_pick_rows_in_place(dev, lib, oracle, V):
     """Samplers on the host, logit rows in any order and twice, a block with a stride, biases and windows."""
