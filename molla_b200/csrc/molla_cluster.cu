@@ -51,15 +51,29 @@ constexpr float TRES = (float)(NT / 32);     // bins per unit of logit: the bins
 #define CPROF_SLOTS(cond, first) nullptr
 #endif
 
+// A piece of a block's range as the exact sum goes through it: chunks (a thread's logits) whose binade is certain,
+// a chunk or a warp of them that may lie in either of two, or a chunk to be added value by value.
+struct __align__(16) Stretch {
+    unsigned int ka, kb;   // pairs of units in binade jb, and in the next one
+    unsigned int meta;     // biased exponent of the binade (8 bits; 255: value by value), it may be the next one (1 bit);
+                           // what was guessed: the binade (8 bits; 0: nothing), two of them (1); place of the values (8; 255: none)
+    unsigned int where;    // first chunk (9 bits), chunks (10 bits)
+    __device__ __forceinline__ unsigned int jb() const { return meta & 0xffu; }
+    __device__ __forceinline__ unsigned int both() const { return (meta >> 8) & 1u; }
+    __device__ __forceinline__ unsigned int guess() const { return (meta >> 9) & 0xffu; }
+    __device__ __forceinline__ bool guess_two() const { return (meta >> 17) & 1u; }
+    __device__ __forceinline__ int place() const { return (int)((meta >> 18) & 0xffu); }
+    __device__ __forceinline__ int first() const { return (int)(where & 511u); }
+    __device__ __forceinline__ int chunks() const { return (int)(where >> 9); }
+    __device__ __forceinline__ bool run() const { return jb() != 255u && !both(); }
+};
+constexpr int RECS = 64;                     // stretches of a block that the leader has at hand
+
 struct __align__(16) AuxC {
     union {
         struct {
-            double pa[NT + 1];
-            double pb[NT + 1];
-            float csum[NT];
-            short ja[NT];
-            unsigned char dual[NT];
-            unsigned long long segd[NT + 1];  // the walk's segments: first chunk, binade guess, flags
+            Stretch items[NWARP * 33];        // of this block's range, in order
+            Stretch recs[CL_MAX_G][RECS];     // leader: of every block, runs across warps as one
         } p1;
         struct {
             unsigned int hq[NBINS];
@@ -87,8 +101,9 @@ struct __align__(16) AuxC {
     float x2_total[CL_MAX_G];
     double x3_tot[CL_MAX_G]; int x3_n[CL_MAX_G];
     int x4_n[CL_MAX_G]; unsigned long long x5_key[CL_MAX_G];
-    float ch_s; int ch_found, ch_at, ch_slow;   // the exact sum on its way from range to range
-    int ch_flag;                                 // which hand-over of the row has arrived (the writer releases, thread 0 acquires)
+    int nitem, nrec[CL_MAX_G];                   // stretches of this block; leader: of every block
+    float first_s[CL_MAX_G];                     // leader: the sum before every block
+    float ch_s; int ch_at, ch_slow;              // the exact sum as the leader found it
     // elements of a walk that would round on a tie: their keys, bins, the mass before them
     long long rx[8];          // words fetched from the leader for the whole block
     int ngath, ngath_over;   // a bin's entries collected by this block; blocks whose own buffer overflowed (leader's)
@@ -113,31 +128,163 @@ struct ClGeo {          // where this thread block stands
 };
 
 // The exact sequential fp32 sum of the cluster's row (values `bits`, zero = absent), in vocabulary
-// order: every block builds the tables of its range from an estimate of the sum before it, then
-// the exact running sum travels from range to range. With `locate`, stops at the first entry
-// whose running sum exceeds `target`; its token id is returned in `at`.
-struct ClSum { float s; int found; int at; int slow; bool timeout; };
+// order. Every thread turns its chunk of the range into units of the binade (or two) in which the estimated sum
+// before it says the sum will be, every warp its chunks into stretches, every block its warps' into as few as may be,
+// which go to the leader with the values of the chunks that may have to be added one by one. One warp of the leader
+// goes through them: a stretch inside a binade is one addition, the chunk in which the sum leaves a binade is added
+// value by value. A guess that the exact sum shows to be wrong is made good for from the values.
+struct ClSum { float s; int slow; };
 
-// cluster-scope release / acquire of one word of (possibly another block's) shared memory
-__device__ __forceinline__ void st_release_cluster(int *p, int v) {
-    asm volatile("st.release.cluster.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ int ld_acquire_cluster(const int *p) {
-    int v;
-    asm volatile("ld.acquire.cluster.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
+// (every lane of the warp calls these and gets the same answer)
+__device__ __noinline__ unsigned int add_chunk(const float *v, int n, unsigned int sb) {
+    const int lane = threadIdx.x & 31;
+    float s = __uint_as_float(sb);
+#pragma unroll 1
+    for (int i = 0; i < n; i += 32) {
+        const float mine = i + lane < n ? v[i + lane] : 0.0f;
+#pragma unroll 8
+        for (int e = 0; e < 32; e++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, mine, e));
+    }
+    return __float_as_uint(s);
 }
 
-// `epoch` counts the sums of a row (the same in every block): the hand-over from range to range
-// is a word released into the next block's shared memory, on which only that block's thread 0
-// waits (with a bound); everybody else waits once, at the cluster barrier after the last range.
-__device__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, const ClGeo &g, const unsigned int *bits,
-                                   bool locate, float target, int &epoch, long long *stamps = nullptr, long long *stamps2 = nullptr) {
+// MOLLA_ROW_SLOW_PATH tells a caller that a guess of the sum's binade went wrong: whether that is said of a chunk
+// whose guess (binade jb, or that and the next one) did not hold. Not where nothing was added, and not where the
+// chunk held a rounding tie or a value of a quarter of the binade: such chunks never went by their guess.
+__device__ __noinline__ bool guess_counts(const float *v, int n, unsigned int jb, bool two) {
+    const int j = (int)jb - 127;
+    const float C1 = __fmul_rn(1.5f, fpow2(j)), C2 = __fmul_rn(1.5f, fpow2(j + 1));
+    bool bad = false, some = false;
+    for (int i = 0; i < n; i++) {
+        const float x = v[i], k1 = __fsub_rn(__fadd_rn(x, C1), C1), k2 = __fsub_rn(__fadd_rn(x, C2), C2);
+        bad |= fabsf(__fsub_rn(x, k1)) == fpow2(j - 24) || x >= fpow2(j - 1) || (two && fabsf(__fsub_rn(x, k2)) == fpow2(j - 23));
+        some |= k1 != 0.0f || (two && k2 != 0.0f);
+    }
+    return some && !bad;
+}
+__device__ __forceinline__ bool guess_held(unsigned int jb, bool two, unsigned int before, unsigned int after) {
+    const unsigned int e = before >> 23, f = after >> 23;
+    return jb == 0u || ((e == jb || (two && e == jb + 1u)) && f <= jb + (two ? 1u : 0u));
+}
+
+// One thread's units: its values added to the smallest even and the smallest odd pattern of the binade with biased exponent e.
+template <class V>
+__device__ __forceinline__ Units chunk_units(V lst, int i0, int i1, unsigned int e) {
+    const unsigned int base = e << 23;
+    float s0 = __uint_as_float(base), s1 = __uint_as_float(base + 1u);
+#pragma unroll 4
+    for (int i = i0; i < i1; i++) { const float v = lst(i); s0 = __fadd_rn(s0, v); s1 = __fadd_rn(s1, v); }
+    return Units{__float_as_uint(s0) - base, __float_as_uint(s1) - base - 1u};
+}
+
+struct ChunksSum { unsigned int sb; bool slow; };
+// Chunks [first, first + n) of a block's values, whatever was guessed about them.
+__device__ __noinline__ ChunksSum add_chunks(const float *vals, int nloc, int L, int first, int n, unsigned int sb, unsigned int jb, bool two) {
+    const int lane = threadIdx.x & 31;
+    ChunksSum r{sb, false};
+#pragma unroll 1
+    for (int c0 = first; c0 < first + n; c0 += 32) {
+        const int m = min(32, first + n - c0), i0 = min(nloc, (c0 + lane) * L), i1 = lane < m ? min(nloc, i0 + L) : i0;
+        bool wrong = false;
+        int at = 0;
+#pragma unroll 1
+        while (at < m) {
+            const unsigned int e = r.sb >> 23;
+            const Units d = units_scan(lane < at ? Units{0u, 0u} : chunk_units([&](int i) { return vals[i]; }, i0, i1, e), lane, 0);
+            const unsigned int to = r.sb + ((r.sb & 1u) ? d.odd : d.even);
+            unsigned int from = __shfl_up_sync(0xffffffffu, to, 1);
+            if (lane == 0) from = r.sb;
+            const unsigned int stop = __ballot_sync(0xffffffffu, lane >= at && lane < m && (to >> 23) != e);
+            const int f = stop ? __ffs((int)stop) - 1 : m;
+            if (lane >= at && lane < f) wrong |= !guess_held(jb, two, from, to);
+            if (f > at) r.sb = __shfl_sync(0xffffffffu, to, f - 1);
+            at = f;
+            if (at < m) {
+                const int o = min(nloc, (c0 + at) * L);
+                const unsigned int q = add_chunk(vals + o, min(nloc, o + L) - o, r.sb);
+                if (lane == at) wrong |= !guess_held(jb, two, r.sb, q);
+                r.sb = q;
+                at++;
+            }
+        }
+        if (__any_sync(0xffffffffu, wrong)) r.slow |= __any_sync(0xffffffffu, wrong && guess_counts(vals + i0, i1 - i0, jb, two)) != 0;
+    }
+    return r;
+}
+
+// Where the values of chunks to be added one by one wait for the leader's walk, `pitch` floats each: over pc, pre and
+// hidx, half of the places for the leader's own range, in which most binades are crossed.
+__device__ __forceinline__ int care_pitch(int L) { return (L + 3) & ~3; }
+__device__ __forceinline__ void care_places(int L, int rank, int &first, int &n) {
+    static_assert(offsetof(AuxC, pre) == offsetof(AuxC, pc) + sizeof(AuxC::pc) && offsetof(AuxC, hidx) == offsetof(AuxC, pre) + sizeof(AuxC::pre), "one area");
+    static_assert(offsetof(AuxC, pc) % 16 == 0, "read four at a time");
+    const int all = min(255, (int)((sizeof(AuxC::pc) + sizeof(AuxC::pre) + sizeof(AuxC::hidx)) / sizeof(float)) / care_pitch(L));
+    const int own = all / 2, others = (all - own) / (CL_MAX_G - 1);
+    first = rank == 0 ? 0 : own + (rank - 1) * others;
+    n = rank == 0 ? own : others;
+}
+
+// The leader's first warp, all lanes alike: through the stretches of blocks h0 and up, the sum before them sb. With
+// `locate`, ends with the stretch behind which the sum exceeds `target`: its block, place and the sum before it.
+struct Walked { unsigned int sb; bool slow; int h, first, chunks; };
+__device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, int h0, unsigned int sb, bool locate, float target) {
+    AuxC *A = c.A;
+    IN_SHARED(A);
+    Walked w{sb, false, -1, 0, 0};
+    const int pitch4 = care_pitch(g.L) / 4;
+#pragma unroll 1
+    for (int h = h0; h < g.G; h++) {
+        const int nrec = A->nrec[h];
+        const bool far = nrec > RECS;   // (too many: where the block has left them)
+        const int n = far ? cl.map_shared_rank(A, h)->nitem : nrec;
+        const Stretch *list = far ? cl.map_shared_rank(A, h)->u.p1.items : A->u.p1.recs[h];
+        if (!locate && c.lane == 0) A->first_s[h] = __uint_as_float(w.sb);
+        if (n == 0) continue;
+        Stretch nx = list[0];
+#pragma unroll 1
+        for (int i = 0; i < n; i++) {
+            const Stretch it = nx;
+            nx = list[min(i + 1, n - 1)];
+            const unsigned int before = w.sb, e = before >> 23, d = e - it.jb(), to = before + units(d ? it.kb : it.ka, before);
+            if (d <= it.both() && (to >> 23) == e) w.sb = to;
+            else {
+                const int nloc = max(0, min(Vc, V - h * Vc)), o = min(nloc, it.first() * g.L), len = min(nloc, o + g.L) - o;
+                const float *vals = reinterpret_cast<const float *>(h == 0 ? bits : cl.map_shared_rank(const_cast<unsigned int *>(bits), h));
+                if (it.chunks() > 1) {
+                    const ChunksSum q = add_chunks(vals, nloc, g.L, it.first(), it.chunks(), before, it.guess(), it.guess_two());
+                    w.sb = q.sb; w.slow |= q.slow;
+                } else {
+                    if (it.place() == 255) w.sb = add_chunk(vals + o, len, before);
+                    else {
+                        const float4 *v = reinterpret_cast<const float4 *>(A->pc) + it.place() * pitch4;
+                        float s = __uint_as_float(before);
+                        float4 x = v[0], y = v[1];   // (a pitch is eight floats at least where chunks are longer than four)
+#pragma unroll 1
+                        for (int k = 0; k < pitch4; k++) {
+                            const float4 z = v[min(k + 2, pitch4 - 1)];
+                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x.x), x.y), x.z), x.w);
+                            x = y; y = z;
+                        }
+                        w.sb = __float_as_uint(s);
+                    }
+                    if (!guess_held(it.guess(), it.guess_two(), before, w.sb)) w.slow |= guess_counts(vals + o, len, it.guess(), it.guess_two());
+                }
+            }
+            if (locate && target < __uint_as_float(w.sb)) {
+                w.sb = before; w.h = h; w.first = it.first(); w.chunks = it.chunks();
+                return w;
+            }
+        }
+    }
+    return w;
+}
+
+__device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, long long *stamps = nullptr) {
     AuxC *A = c.A;
     IN_SHARED(A);
     IN_SHARED(bits);
+    AuxC *lead = cl.map_shared_rank(A, 0);
     ValBits vals{bits};
-    epoch++;
     __syncthreads();
     const float csum = p1_csum(vals, g.nloc, g.L, c.tid);
     double tot;
@@ -147,41 +294,182 @@ __device__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, const ClGeo &
     double sbase = 0.0;
     for (int h = 0; h < g.rank; h++) sbase += A->x3_tot[h];
     if (stamps && c.tid == 0) stamps[0] = clock64();
-    p1_tables(c, vals, g.nloc, g.L, csum, sbase + ex);
-    if (stamps && c.tid == 0) stamps[1] = clock64();
-    if (c.tid == 0) {
-        Walker w;
-        int timed_out = 0;
-        if (g.rank == 0) { w.s = 0.0f; w.found = 0; w.at = -1; w.slow = 0; }
-        else {
-            bool here = false;
-            for (int spin = 0; spin < (1 << 22); spin++)
-                if (ld_acquire_cluster(&A->ch_flag) == epoch) { here = true; break; }
-            if (!here) timed_out = 4;
-            w.s = A->ch_s; w.found = A->ch_found; w.at = A->ch_at; w.slow = A->ch_slow;
-        }
-        if (!(locate && w.found)) {
-            const long long tw0 = clock64();
-            p1_walk(c, vals, g.nloc, g.L, locate, target, w);
-            if (w.found) w.at += g.c0;
-            if (stamps2) { stamps2[g.rank] = clock64() - tw0; stamps2[4 + g.rank] = w.nsim * 100000ll + w.nel; stamps2[8 + g.rank] = A->nseg; }
-        }
-        w.slow |= timed_out;
-        if (g.rank + 1 < g.G) {
-            AuxC *nx = cl.map_shared_rank(A, g.rank + 1);
-            nx->ch_s = w.s; nx->ch_found = w.found; nx->ch_at = w.at; nx->ch_slow = w.slow;
-            st_release_cluster(&nx->ch_flag, epoch);
-        } else {
-            for (int o = 0; o < g.G; o++) {
-                AuxC *ox = cl.map_shared_rank(A, o);
-                ox->ch_s = w.s; ox->ch_found = w.found; ox->ch_at = w.at; ox->ch_slow = w.slow;
+    const double sst = sbase + ex;
+    // the binade of the sum before and behind this chunk; 2^-12 covers the rounding of the true one
+    const float EPS = 1.0f / 4096.0f;
+    const float lo = (float)(sst * (1.0 - (double)EPS)), hi = (float)((sst + (double)csum) * (1.0 + (double)EPS));
+    const int i0 = min(g.nloc, c.tid * g.L), i1 = min(g.nloc, (c.tid + 1) * g.L), lane = c.lane;
+    const int jl = fexpo(lo), jh = fexpo(hi);
+    const bool nonempty = i1 > i0 && csum != 0.0f;
+    const bool usable = nonempty && lo > 0.0f && jh <= jl + 1 && jl >= -100 && jh <= 100, two = usable && jh == jl + 1;
+    const unsigned int jb = (unsigned int)(jl + 127);
+    Units da{0u, 0u}, db{0u, 0u};
+    bool over = false;   // outgrows a binade by itself
+    if (usable) {
+        da = chunk_units(vals, i0, i1, jb);
+        over = ((jb << 23) + 1u + da.odd) >> 23 != jb;
+    }
+    if (__any_sync(0xffffffffu, two) && two) {
+        db = chunk_units(vals, i0, i1, jb + 1u);
+        over |= (((jb + 1u) << 23) + 1u + db.odd) >> 23 != jb + 1u;
+    }
+    const bool step = nonempty && (!usable || over);
+    const unsigned int ne = __ballot_sync(0xffffffffu, nonempty), lt = (1u << lane) - 1u, below = ne & lt;
+    const int prev = below ? 31 - __clz((int)below) : lane;
+    const int pj = __shfl_sync(0xffffffffu, jl, prev);
+    const bool prev_alone = ((__ballot_sync(0xffffffffu, step || two) >> prev) & 1u) != 0u;
+    const int j0 = __shfl_sync(0xffffffffu, jl, max(__ffs((int)ne) - 1, 0));
+    // (chunks that all may lie in the same two binades are one stretch: a sum that stays near a power of two for long)
+    const bool merged = __popc(ne) >= 8 && __all_sync(0xffffffffu, !nonempty || (two && !over && jl == j0));
+    const bool care = !merged && (step || two || (nonempty && below && !prev_alone && pj != jl));
+    const unsigned int cm = __ballot_sync(0xffffffffu, care), cb = cm & lt;
+    const int lastc = cb ? 31 - __clz((int)cb) : -1, last = cm ? 31 - __clz((int)cm) : -1;
+    const Units ra = units_scan(care || !usable ? Units{0u, 0u} : da, lane, care ? lane : lastc + 1);
+    const unsigned int kp = pair_of(ra.even, ra.odd);
+    unsigned int kr = __shfl_up_sync(0xffffffffu, kp, 1);
+    if (lane == 0) kr = 0u;
+    // (a run that adds nothing is none: whatever its guess was, it would not count)
+    const unsigned int runm = __ballot_sync(0xffffffffu, care && kr != 0u);
+    const unsigned int ktail = last == 31 || merged ? 0u : __shfl_sync(0xffffffffu, kp, 31);
+    const int n = merged ? 1 : __popc(cm) + __popc(runm) + (ktail ? 1 : 0);
+    if (lane == 0) A->wsi[c.warp] = n | (__popc(cm) << 16);
+    Units rb{0u, 0u};
+    if (merged) rb = units_scan(db, lane, 0);
+    auto first_in = [&](int from) { const unsigned int m = ne & ~(from < 0 ? 0u : (from == 31 ? 0xffffffffu : ((2u << from) - 1u))); return m ? __ffs((int)m) - 1 : 31; };
+    const int fj = __shfl_sync(0xffffffffu, jl, first_in(lastc)), tj = __shfl_sync(0xffffffffu, jl, first_in(last));
+    __syncthreads();
+    int at = 0;
+    for (int w = 0; w < c.warp; w++) at += A->wsi[w];
+    int place0, places;
+    care_places(g.L, g.rank, place0, places);
+    const int care0 = at >> 16;
+    at &= 0xffff;
+    if (c.tid == NT - 1) A->nitem = at + n;
+    Stretch *out = A->u.p1.items + at;
+    const unsigned int w0 = (unsigned int)c.warp * 32u;
+    auto stretch = [&](unsigned int ka, unsigned int kb, unsigned int match, bool both, int guess, bool guess_two, int place, unsigned int first, unsigned int chunks) {
+        Stretch it;
+        it.ka = ka; it.kb = kb;
+        it.meta = match | (both ? 1u << 8 : 0u) | ((unsigned int)(guess + 127) << 9) | (guess_two ? 1u << 17 : 0u) | ((unsigned int)place << 18);
+        it.where = (w0 + first) | (chunks << 9);
+        return it;
+    };
+    int place = 255;
+    if (care) {
+        int i = __popc(cb) + __popc(runm & lt);
+        const int nth = care0 + __popc(cb);
+        place = nth < places ? place0 + nth : 255;
+        if ((runm >> lane) & 1u) out[i++] = stretch(kr, 0u, (unsigned int)(fj + 127), false, fj, false, 255, (unsigned int)(lastc + 1), (unsigned int)(lane - lastc - 1));
+        const bool known = usable && !over;
+        out[i] = stretch(known ? pair_of(da.even, da.odd) : 0u, known && two ? pair_of(db.even, db.odd) : 0u, known ? jb : 255u, known && two, usable ? jl : -127, two, place,
+                         (unsigned int)lane, 1u);
+    }
+    if (lane == 31 && merged) out[0] = stretch(kp, pair_of(rb.even, rb.odd), (unsigned int)(j0 + 127), true, j0, true, 255, 0u, 32u);
+    if (lane == 31 && ktail) out[n - 1] = stretch(ktail, 0u, (unsigned int)(tj + 127), false, tj, false, 255, (unsigned int)(last + 1), (unsigned int)(31 - last));
+    // the careful chunks' values to the leader, padded with zeros
+    const int pitch = care_pitch(g.L);
+    for (unsigned int left = __ballot_sync(0xffffffffu, place != 255); left; left &= left - 1u) {
+        const int l = __ffs((int)left) - 1, o = __shfl_sync(0xffffffffu, i0, l), len = __shfl_sync(0xffffffffu, i1, l) - o;
+        float *to = lead->pc + __shfl_sync(0xffffffffu, place, l) * pitch;
+        for (int i = lane; i < pitch; i += 32) to[i] = i < len ? vals(o + i) : 0.0f;
+    }
+    __syncthreads();
+    if (c.warp == 0) {   // the block's stretches to the leader, runs of one binade across warps as one
+        const int total = A->nitem;
+        int nrec = 0;
+        for (int b = 0; b < total; b += 32) {
+            const bool have = b + lane < total;
+            Stretch it;
+            it.ka = it.kb = it.where = 0u; it.meta = 255u;
+            if (have) it = A->u.p1.items[b + lane];
+            const bool run = it.run(), before = __shfl_up_sync(0xffffffffu, run, 1);
+            const unsigned int mj = it.jb(), bj = __shfl_up_sync(0xffffffffu, mj, 1);
+            const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || !run || !before || bj != mj);
+            const int s0 = 31 - __clz((int)(starts & (lt | (1u << lane))));
+            const unsigned int w_first = __shfl_sync(0xffffffffu, it.where, s0) & 511u;
+            Units u{units(it.ka, 0u), units(it.ka, 1u)};
+            if (__any_sync(0xffffffffu, run && !parity_free(it.ka))) u = units_scan(u, lane, s0);
+            else {
+                const unsigned int inc = warp_incl_scan(run ? u.even : 0u, lane), b0 = __shfl_sync(0xffffffffu, inc, max(s0 - 1, 0));
+                u.even = u.odd = inc - (s0 > 0 ? b0 : 0u);
             }
+            const bool ends = have && (lane == 31 || ((starts >> (lane + 1)) & 1u) || b + lane + 1 == total);
+            const unsigned int em = __ballot_sync(0xffffffffu, ends);
+            const int i = nrec + __popc(em & lt);
+            if (run) {
+                it.ka = pair_of(u.even, u.odd);
+                it.where = w_first | (((it.where & 511u) + (it.where >> 9) - w_first) << 9);
+            }
+            if (ends && i < RECS) lead->u.p1.recs[g.rank][i] = it;
+            nrec += __popc(em);
+        }
+        if (lane == 0) lead->nrec[g.rank] = nrec;
+    }
+    if (stamps && c.tid == 0) stamps[1] = clock64();
+    cl.sync();
+    if (g.rank == 0 && c.warp == 0) {
+        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, 0, 0u, false, 0.0f);
+        if (lane < g.G) { AuxC *ox = cl.map_shared_rank(A, lane); ox->ch_s = __uint_as_float(w.sb); ox->ch_slow = w.slow ? 1 : 0; }
+    }
+    cl.sync();
+    return ClSum{A->ch_s, A->ch_slow};
+}
+
+// The token at which the running sum of the last cluster_exact_sum (`total`) first exceeds `target`, or -1. Its
+// stretches and the values they stand for are where it left them.
+__device__ __noinline__ int cluster_locate(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, float total, float target) {
+    AuxC *A = c.A;
+    IN_SHARED(A);
+    IN_SHARED(bits);
+    if (!(target < total)) return -1;   // (the same in every block)
+    if (g.rank == 0 && c.warp == 0) {
+        int h = 0;
+        for (int k = 1; k < g.G; k++) if (!(target < A->first_s[k])) h = k;   // (the sums never fall)
+        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, h, __float_as_uint(A->first_s[h]), true, target);
+        if (c.lane < g.G) {
+            AuxC *ox = cl.map_shared_rank(A, c.lane);
+            ox->r_kind = w.h; ox->r_idx = w.first | (w.chunks << 16); ox->r_s = __uint_as_float(w.sb);
+            ox->ch_at = -1;
         }
     }
     cl.sync();
-    ClSum out;
-    out.s = A->ch_s; out.found = A->ch_found; out.at = A->ch_at; out.slow = A->ch_slow & 1; out.timeout = (A->ch_slow & 4) != 0;
-    return out;
+    if (A->r_kind == g.rank) {   // the block that holds it: every thread the sum before its chunk, the first one past the target looks into it
+        const int first = A->r_idx & 0xffff, n = A->r_idx >> 16;
+        const unsigned int sb = __float_as_uint(A->r_s), e = sb >> 23;
+        const int i0 = min(g.nloc, c.tid * g.L), i1 = min(g.nloc, i0 + g.L);
+        ValBits vals{bits};
+        const bool mine = c.tid >= first && c.tid < first + n;
+        unsigned int before = sb, to = sb;
+        if (n > 1) {
+            const Units d = units_scan(mine ? chunk_units(vals, i0, i1, e) : Units{0u, 0u}, c.lane, 0);
+            __syncthreads();
+            if (c.lane == 31) A->wsu[c.warp] = (unsigned long long)d.even | ((unsigned long long)d.odd << 32);
+            __syncthreads();
+            Units base{0u, 0u};
+            for (int w = 0; w < c.warp; w++) base = then(base, Units{(unsigned int)A->wsu[w], (unsigned int)(A->wsu[w] >> 32)});
+            const Units all = then(base, d), up{__shfl_up_sync(0xffffffffu, all.even, 1), __shfl_up_sync(0xffffffffu, all.odd, 1)}, mb = c.lane == 0 ? base : up;
+            to = sb + ((sb & 1u) ? all.odd : all.even);
+            before = sb + ((sb & 1u) ? mb.odd : mb.even);
+        }
+        if (c.tid == 0) A->evt_thread = 0x7fffffff;
+        __syncthreads();
+        // (a sum that leaves the binade inside: the guess was wrong, or it is one chunk; then from the first of them on)
+        const bool left = n == 1 || __syncthreads_or(mine && (to >> 23) != e) != 0;
+        if (left) { if (c.tid == first) { A->evt_thread = first; before = sb; } }
+        else if (mine && target < __uint_as_float(to)) atomicMin(&A->evt_thread, c.tid);
+        __syncthreads();
+        if (A->evt_thread == c.tid) {
+            float s = __uint_as_float(before);
+            int found = -1;
+            for (int i = i0; i < (left ? min(g.nloc, (first + n) * g.L) : i1); i++) {
+                s = __fadd_rn(s, vals(i));
+                if (target < s) { found = i; break; }
+            }
+            for (int o = 0; o < g.G; o++) cl.map_shared_rank(A, o)->ch_at = found < 0 ? -1 : g.c0 + found;
+        }
+    }
+    cl.sync();
+    return A->ch_at;
 }
 
 // Token id of the (nth+1)-th entry, in vocabulary order, whose bits equal `eb` (eb below tau).
@@ -876,7 +1164,7 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
         ox->x1_max[g.rank] = cmax; ox->x1_idx[g.rank] = cidx; ox->x1_eq[g.rank] = ceq; ox->x1_status[g.rank] = c.status;
         ox->x2_total[g.rank] = etot;
     }
-    if (c.tid == 0) { A->ncand = 0; A->evt_thread = 0x7fffffff; A->ch_flag = 0; }
+    if (c.tid == 0) { A->ncand = 0; A->evt_thread = 0x7fffffff; }
     CSTAMP(13);
     cl.sync();
     float xmax = -INFINITY;
@@ -1070,11 +1358,9 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     if (c.tid < g.G) cl.map_shared_rank(A, c.tid)->x3_n[g.rank] = A->ncand;
 
     // ---- 5. the softmax denominator, exactly as the sequential loop rounds it
-    int epoch = 0;
-    const ClSum zs = cluster_exact_sum(cl, c, g, rowbits, false, 0.0f, epoch, CPROF_SLOTS(leader, 14), CPROF_SLOTS(!p3row, 20));
+    const ClSum zs = cluster_exact_sum(cl, c, g, a.Vc, a.V, rowbits, CPROF_SLOTS(leader, 14));
     const float Z = zs.s;
     if (zs.slow) c.status |= MOLLA_ROW_SLOW_PATH;
-    if (zs.timeout) { c.status |= MOLLA_ROW_LOAD_TIMEOUT; finish(); return; }  // (the same word in every block)
     dZ = Z;
 
     CSTAMP(6);
@@ -1123,14 +1409,13 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
             if (pb < minp_pbits) pb = 0u;
             rowbits[i] = pb;
         }
-        const ClSum s1 = cluster_exact_sum(cl, c, g, rowbits, false, 0.0f, epoch);
+        const ClSum s1 = cluster_exact_sum(cl, c, g, a.Vc, a.V, rowbits);
         const float sum = s1.s;
         const float target = __fmul_rn(u01, sum);
-        const ClSum s2 = cluster_exact_sum(cl, c, g, rowbits, true, target, epoch);
-        if (s1.slow || s2.slow) c.status |= MOLLA_ROW_SLOW_PATH;
-        if (s1.timeout || s2.timeout) { c.status |= MOLLA_ROW_LOAD_TIMEOUT; finish(); return; }
+        const int drawn = cluster_locate(cl, c, g, a.Vc, a.V, rowbits, sum, target);
+        if (s1.slow) c.status |= MOLLA_ROW_SLOW_PATH;
         dsum = sum; dtarget = target;
-        if (s2.found) token = s2.at;
+        if (drawn >= 0) token = drawn;
         else {
             // the walk fell off the end: the reference returns the last token of the vocabulary,
             // whether or not it could matter to any sum ... or the last one min-p left

@@ -155,6 +155,31 @@ __device__ __forceinline__ unsigned long long make_key(unsigned int ebits, int i
 
 __device__ __forceinline__ int hslot(int tok) { return (int)(((unsigned int)tok * 2654435761u) >> 21); }
 
+// While the running sum s stays in one binade, fl(s + v) is s plus rne(v / ulp) units, and in the bit pattern of s adding k
+// units is the integer addition of k. Only where v / ulp ends in a half does the integer depend on s, and then on
+// the parity of its pattern alone: a stretch of values is what it adds to an even and to an odd pattern.
+// A pair of units in one word: those added to an even pattern (30 bits; they stay below 2^25) and what an odd one
+// gets more of them (-1, 0 or 1).
+__device__ __forceinline__ unsigned int pair_of(unsigned int even, unsigned int odd) { return even | ((odd - even) << 30); }
+__device__ __forceinline__ bool parity_free(unsigned int pair) { return (pair >> 30) == 0u; }
+__device__ __forceinline__ unsigned int units(unsigned int pair, unsigned int sb) {   // added to the pattern sb
+    return (pair & 0x3fffffffu) + ((sb & 1u) ? (unsigned int)((int)pair >> 30) : 0u);
+}
+struct Units { unsigned int even, odd; };
+// Stretch a, then stretch b.
+__device__ __forceinline__ Units then(const Units &a, const Units &b) {
+    return Units{a.even + ((a.even & 1u) ? b.odd : b.even), a.odd + ((a.odd & 1u) ? b.even : b.odd)};
+}
+// The stretches of the lanes from number `from` (of each lane its own) up to this one, as one.
+__device__ __forceinline__ Units units_scan(Units k, int lane, int from) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Units before{__shfl_up_sync(0xffffffffu, k.even, o), __shfl_up_sync(0xffffffffu, k.odd, o)};
+        if (lane - o >= from) k = then(before, k);
+    }
+    return k;
+}
+
 // =============================================================================
 // The exact sequential fp32 sum of the list's values, in list (= vocabulary) order.
 // =============================================================================

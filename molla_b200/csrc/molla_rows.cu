@@ -76,7 +76,7 @@ struct __align__(8) TileOut { unsigned int ioff; unsigned short cnt, nitem; };  
 // and then only on the parity of its bit pattern. So any stretch of values is two numbers, the units it adds to
 // an even and to an odd pattern; they differ by one at most (fl does not change the order of two sums, and two
 // that have become equally even stay in step), and two stretches make one. A stretch of lanes whose
-// binade is certain is one such pair (kind RUN). A lane near the end of a binade carries
+// binade is certain is one such pair (kind RUN; Units in molla_exact.cuh). A lane near the end of a binade carries
 // the pairs of both binades (DUAL); a lane that outgrows a binade by itself or whose
 // guess spans more is added value by value (STEP). The binades are guessed from the estimated
 // sum before the tile; whoever runs the items checks every guess against the exact sum and adds the
@@ -94,19 +94,6 @@ struct __align__(16) Item {
     __device__ __forceinline__ int off() const { return (int)((oc >> 11) & 0x3ffu); }
     __device__ __forceinline__ int num() const { return (int)(oc >> 21); }
 };
-// A pair of units in one word: those added to an even pattern (30 bits; they stay below 2^25) and what an odd one
-// gets more of them (-1, 0 or 1).
-__device__ __forceinline__ unsigned int pair_of(unsigned int even, unsigned int odd) { return even | ((odd - even) << 30); }
-__device__ __forceinline__ bool parity_free(unsigned int pair) { return (pair >> 30) == 0u; }
-__device__ __forceinline__ unsigned int units(unsigned int pair, unsigned int sb) {   // added to the pattern sb
-    return (pair & 0x3fffffffu) + ((sb & 1u) ? (unsigned int)((int)pair >> 30) : 0u);
-}
-// Stretch a, then stretch b (even: to an even pattern, odd: to an odd one).
-struct Units { unsigned int even, odd; };
-__device__ __forceinline__ Units then(const Units &a, const Units &b) {
-    return Units{a.even + ((a.even & 1u) ? b.odd : b.even), a.odd + ((a.odd & 1u) ? b.even : b.odd)};
-}
-
 // ---- settings ---------------------------------------------------------------------------------
 struct __align__(16) RowCfg {
     long long lrow;
@@ -854,12 +841,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
         // of 128 values at most, which are in the list. (With an item a lane, one row in some hundreds of 262144 had more
         // careful chunks than row_head takes, and row_tail took 200 us for it.)
         const int lg = total <= 128 ? 5 : (total <= 256 ? 4 : (total <= 512 ? 3 : 2)), in = lane & ((1 << lg) - 1);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const Units a{__shfl_up_sync(0xffffffffu, da.even, o), __shfl_up_sync(0xffffffffu, da.odd, o)};
-            const Units b{__shfl_up_sync(0xffffffffu, db.even, o), __shfl_up_sync(0xffffffffu, db.odd, o)};
-            if (in >= o) { da = then(a, da); db = then(b, db); }
-        }
+        da = units_scan(da, lane, lane - in); db = units_scan(db, lane, lane - in);
         const int first = __shfl_sync(0xffffffffu, off, lane - in), n = 32 >> lg;
         Item *out = alloc(n, 0);
         if (in == (1 << lg) - 1) {
@@ -874,12 +856,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     // the runs between the careful lanes: a run goes with the careful lane behind it, or closes the tile
     const unsigned int lt = (1u << lane) - 1u, cb = cm & lt;
     const int lastc = cb ? 31 - __clz((int)cb) : -1, last = cm ? 31 - __clz((int)cm) : -1;
-    Units k = care || !usable ? Units{0u, 0u} : da;   // of the run up to this lane and with it
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const Units before{__shfl_up_sync(0xffffffffu, k.even, o), __shfl_up_sync(0xffffffffu, k.odd, o)};
-        if (lane - o > lastc && !care) k = then(before, k);
-    }
+    const Units k = units_scan(care || !usable ? Units{0u, 0u} : da, lane, care ? lane : lastc + 1);   // of the run up to this lane and with it
     const unsigned int kp = pair_of(k.even, k.odd);
     unsigned int kr = __shfl_up_sync(0xffffffffu, kp, 1);    // of the run that ends before this lane
     if (lane == 0) kr = 0u;
@@ -1490,11 +1467,7 @@ __device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsig
                      (runs == 0u || ((c.meta & 0xffu) == e && runs < (1u << 24)));
     Units d{0u, 0u};
     if (can) d = Units{runs + units(own, runs), runs + units(own, runs + 1u)};
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const Units before{__shfl_up_sync(0xffffffffu, d.even, o), __shfl_up_sync(0xffffffffu, d.odd, o)};
-        if (lane >= o) d = then(before, d);
-    }
+    d = units_scan(d, lane, 0);
     const unsigned int inc = (sb & 1u) ? d.odd : d.even;
     const unsigned int stop = __ballot_sync(0xffffffffu, !can || ((sb + inc) >> 23) != e);
     const int n = stop ? __ffs((int)stop) - 1 : 32;
@@ -2958,12 +2931,7 @@ __device__ __noinline__ bool tail_pure(CtxF &c) {
             float s0 = __uint_as_float(base), s1 = __uint_as_float(base + 1u);
 #pragma unroll 8
             for (int e = b0; e < b1; e++) { s0 = __fadd_rn(s0, v[e]); s1 = __fadd_rn(s1, v[e]); }
-            Units k{__float_as_uint(s0) - base, __float_as_uint(s1) - base - 1u};
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const Units before{__shfl_up_sync(0xffffffffu, k.even, o), __shfl_up_sync(0xffffffffu, k.odd, o)};
-                if (c.lane >= o) k = then(before, k);
-            }
+            const Units k = units_scan(Units{__float_as_uint(s0) - base, __float_as_uint(s1) - base - 1u}, c.lane, 0);
             const unsigned int to = sb + ((sb & 1u) ? k.odd : k.even);
             const unsigned int hit = __ballot_sync(0xffffffffu, target < __uint_as_float(to));
             const int l = hit ? __ffs((int)hit) - 1 : 31;
