@@ -69,11 +69,19 @@ struct __align__(16) Stretch {
 };
 constexpr int RECS = 64;                     // stretches of a block that the leader has at hand
 
+// walk_fast's own.
+constexpr int FAST_RECS = 160;
+// units of all plain stretches before it, its own; binade of the last of those (8 bits), guess (8), two binades guessed (1), place (8), whether it has units (1)
+struct __align__(16) FastRec { unsigned int k, ka, kb, meta; };
+
 struct __align__(16) AuxC {
     union {
         struct {
             Stretch items[NWARP * 33];        // of this block's range, in order
             Stretch recs[CL_MAX_G][RECS];     // leader: of every block, runs across warps as one
+            FastRec fast[FAST_RECS];          // leader: see walk_fast
+            float after[FAST_RECS];           // the sum behind each of them,
+            unsigned short org[FAST_RECS];    // and which stretch it is: block (3 bits), number (9)
         } p1;
         struct {
             unsigned int hq[NBINS];
@@ -101,7 +109,7 @@ struct __align__(16) AuxC {
     float x2_total[CL_MAX_G];
     double x3_tot[CL_MAX_G]; int x3_n[CL_MAX_G];
     int x4_n[CL_MAX_G]; unsigned long long x5_key[CL_MAX_G];
-    int nitem, nrec[CL_MAX_G];                   // stretches of this block; leader: of every block
+    int nitem, nrec[CL_MAX_G], nfast;            // stretches of this block; leader: of every block; of walk_fast, or -1
     float first_s[CL_MAX_G];                     // leader: the sum before every block
     float ch_s; int ch_at, ch_slow;              // the exact sum as the leader found it
     // elements of a walk that would round on a tie: their keys, bins, the mass before them
@@ -214,7 +222,7 @@ __device__ __noinline__ ChunksSum add_chunks(const float *vals, int nloc, int L,
 
 // Where the values of chunks to be added one by one wait for the leader's walk, `pitch` floats each: over pc, pre and
 // hidx, half of the places for the leader's own range, in which most binades are crossed.
-__device__ __forceinline__ int care_pitch(int L) { return (L + 3) & ~3; }
+__device__ __forceinline__ int care_pitch(int L) { return (L + 11) / 12 * 12; }   // (whole steps of add_place)
 __device__ __forceinline__ void care_places(int L, int rank, int &first, int &n) {
     static_assert(offsetof(AuxC, pre) == offsetof(AuxC, pc) + sizeof(AuxC::pc) && offsetof(AuxC, hidx) == offsetof(AuxC, pre) + sizeof(AuxC::pre), "one area");
     static_assert(offsetof(AuxC, pc) % 16 == 0, "read four at a time");
@@ -224,10 +232,108 @@ __device__ __forceinline__ void care_places(int L, int rank, int &first, int &n)
     n = rank == 0 ? own : others;
 }
 
-// The leader's first warp, all lanes alike: through the stretches of blocks h0 and up, the sum before them sb. With
+// A place's values added to s, twelve at a time with the next twelve's loads ahead. (Addresses as numbers: through
+// pointers the loads were generic ones, with 64-bit arithmetic around them.)
+__device__ __forceinline__ float4 lds4(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ float add_place(const AuxC *A, int place, int pitch4, float s) {
+    uint32_t at = smem_u32(A->pc) + (uint32_t)(place * pitch4) * 16u;
+    const uint32_t last = at + (uint32_t)(pitch4 - 3) * 16u;
+    float4 x[3] = {lds4(at), lds4(at + 16u), lds4(at + 32u)};
+#pragma unroll 2
+    for (; at <= last; at += 48u) {
+        const uint32_t n = min(at + 48u, last);
+        const float4 y[3] = {lds4(n), lds4(n + 16u), lds4(n + 32u)};
+#pragma unroll
+        for (int u = 0; u < 3; u++) { s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[u].x), x[u].y), x[u].z), x[u].w); x[u] = y[u]; }
+    }
+    return s;
+}
+
+// The usual row: no guess is wrong. The leader's first warp first strings the stretches of all blocks together, 32 at a
+// time: those that are plain additions become part of what lies before the next that is not, and only
+// these (ten or twenty: mostly the chunks in which the sum leaves a binade) are gone through one by one. (Every
+// instruction of that loop is one of a lone warp's, eight cycles or so: with the plain ones in it, it took 14 thousand.)
+// Returns false, and nothing else, where something does not hold.
+__device__ __noinline__ bool walk_fast(CtxC &c, const ClGeo &g, float &sum) {
+    AuxC *A = c.A;
+    IN_SHARED(A);
+    const int lane = c.lane, pitch4 = care_pitch(g.L) / 4;
+    const unsigned int lt = (1u << lane) - 1u;
+    const int cnt = lane < g.G ? A->nrec[lane] : 0, incl = warp_incl_scan(cnt, lane), total = __shfl_sync(0xffffffffu, incl, 31);
+    if (lane == 0) A->nfast = -1;
+    if (__any_sync(0xffffffffu, cnt > RECS)) return false;
+    FastRec *out = A->u.p1.fast;
+    int ncare = 0;
+    unsigned int k = 0u, carry = 0u;   // of the record before this batch: its binade, 0 where it was not a run
+#pragma unroll 1
+    for (int b = 0; b < total; b += 32) {
+        const int idx = b + lane;
+        int h = 0, at = idx;
+#pragma unroll
+        for (int o = 0; o < CL_MAX_G - 1; o++) {
+            const int end = __shfl_sync(0xffffffffu, incl, o);
+            if (o < g.G - 1 && idx >= end) { h = o + 1; at = idx - end; }
+        }
+        const bool have = idx < total;
+        Stretch it;
+        it.ka = it.kb = it.where = 0u; it.meta = 255u;
+        if (have) it = A->u.p1.recs[h][at];
+        const unsigned int rj = it.run() ? it.jb() : 0u;
+        unsigned int pj = __shfl_up_sync(0xffffffffu, rj, 1);
+        if (lane == 0) pj = carry;
+        carry = __shfl_sync(0xffffffffu, rj, 31);
+        const bool care = have && (!it.run() || !parity_free(it.ka) || (pj != 0u && pj != rj));
+        const unsigned int inc = warp_incl_scan(have && !care ? it.ka : 0u, lane), cm = __ballot_sync(0xffffffffu, care);
+        const int i = ncare + __popc(cm & lt);
+        if (care && i < FAST_RECS - 1) {
+            FastRec r;
+            r.k = k + inc; r.ka = it.ka; r.kb = it.kb;
+            r.meta = pj | (it.guess() << 8) | (it.guess_two() ? 1u << 16 : 0u) | ((unsigned int)(it.chunks() > 1 ? 255 : it.place()) << 17) | (it.jb() != 255u ? 1u << 25 : 0u);
+            out[i] = r;
+            A->u.p1.org[i] = (unsigned short)(h << 9 | at);
+        }
+        ncare += __popc(cm);
+        k += __shfl_sync(0xffffffffu, inc, 31);
+        if (b + 32 >= total) carry = __shfl_sync(0xffffffffu, rj, (total - 1) & 31);
+    }
+    if (ncare >= FAST_RECS - 1) return false;
+    if (lane == 0) { FastRec r; r.k = k; r.ka = r.kb = 0u; r.meta = carry; out[ncare] = r; }
+    __syncwarp();
+    unsigned int sb = 0u, kdone = 0u;
+    FastRec nx = out[0];
+#pragma unroll 1
+    for (int q = 0; ; q++) {
+        const FastRec r = nx;
+        nx = out[min(q + 1, ncare)];
+        const unsigned int to = sb + (r.k - kdone), jr = r.meta & 0xffu, e = to >> 23;
+        if (r.k != kdone && ((sb >> 23) != jr || e != jr)) return false;
+        kdone = r.k;
+        sb = to;
+        if (q == ncare) break;
+        const unsigned int jb = (r.meta >> 8) & 0xffu, both = (r.meta >> 16) & 1u, d = e - jb, td = to + units(d ? r.kb : r.ka, to);
+        if (((r.meta >> 25) & 1u) && d <= both && (td >> 23) == e) sb = td;
+        else {
+            const int place = (int)((r.meta >> 17) & 0xffu);
+            if (place == 255) return false;
+            sb = __float_as_uint(add_place(A, place, pitch4, __uint_as_float(to)));
+            // (where a binade was guessed: the guess held?)
+            if (jb != 0u && !(d <= both && (sb >> 23) <= jb + both)) return false;
+        }
+        if (lane == 0) A->u.p1.after[q] = __uint_as_float(sb);
+    }
+    if (lane == 0) A->nfast = ncare;
+    sum = __uint_as_float(sb);
+    return true;
+}
+
+// The leader's first warp, all lanes alike, whatever was guessed: through the stretches from number i0 of block h0 on, the sum before them sb. With
 // `locate`, ends with the stretch behind which the sum exceeds `target`: its block, place and the sum before it.
 struct Walked { unsigned int sb; bool slow; int h, first, chunks; };
-__device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, int h0, unsigned int sb, bool locate, float target) {
+__device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, int h0, int i0, unsigned int sb, bool locate, float target) {
     AuxC *A = c.A;
     IN_SHARED(A);
     Walked w{sb, false, -1, 0, 0};
@@ -239,10 +345,11 @@ __device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, co
         const int n = far ? cl.map_shared_rank(A, h)->nitem : nrec;
         const Stretch *list = far ? cl.map_shared_rank(A, h)->u.p1.items : A->u.p1.recs[h];
         if (!locate && c.lane == 0) A->first_s[h] = __uint_as_float(w.sb);
-        if (n == 0) continue;
-        Stretch nx = list[0];
+        const int from = h == h0 ? i0 : 0;
+        if (from >= n) continue;
+        Stretch nx = list[from];
 #pragma unroll 1
-        for (int i = 0; i < n; i++) {
+        for (int i = from; i < n; i++) {
             const Stretch it = nx;
             nx = list[min(i + 1, n - 1)];
             const unsigned int before = w.sb, e = before >> 23, d = e - it.jb(), to = before + units(d ? it.kb : it.ka, before);
@@ -256,15 +363,7 @@ __device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, co
                 } else {
                     if (it.place() == 255) w.sb = add_chunk(vals + o, len, before);
                     else {
-                        const float4 *v = reinterpret_cast<const float4 *>(A->pc) + it.place() * pitch4;
-                        float s = __uint_as_float(before);
-                        float4 x = v[0], y = v[1];   // (a pitch is eight floats at least where chunks are longer than four)
-#pragma unroll 1
-                        for (int k = 0; k < pitch4; k++) {
-                            const float4 z = v[min(k + 2, pitch4 - 1)];
-                            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x.x), x.y), x.z), x.w);
-                            x = y; y = z;
-                        }
+                        const float s = add_place(A, it.place(), pitch4, __uint_as_float(before));
                         w.sb = __float_as_uint(s);
                     }
                     if (!guess_held(it.guess(), it.guess_two(), before, w.sb)) w.slow |= guess_counts(vals + o, len, it.guess(), it.guess_two());
@@ -408,7 +507,10 @@ __device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, 
     if (stamps && c.tid == 0) stamps[1] = clock64();
     cl.sync();
     if (g.rank == 0 && c.warp == 0) {
-        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, 0, 0u, false, 0.0f);
+        Walked w{0u, false, -1, 0, 0};
+        float sum;
+        if (walk_fast(c, g, sum)) w.sb = __float_as_uint(sum);
+        else w = walk_stretches(cl, c, g, Vc, V, bits, 0, 0, 0u, false, 0.0f);
         if (lane < g.G) { AuxC *ox = cl.map_shared_rank(A, lane); ox->ch_s = __uint_as_float(w.sb); ox->ch_slow = w.slow ? 1 : 0; }
     }
     cl.sync();
@@ -423,9 +525,18 @@ __device__ __noinline__ int cluster_locate(cg::cluster_group &cl, CtxC &c, const
     IN_SHARED(bits);
     if (!(target < total)) return -1;   // (the same in every block)
     if (g.rank == 0 && c.warp == 0) {
-        int h = 0;
-        for (int k = 1; k < g.G; k++) if (!(target < A->first_s[k])) h = k;   // (the sums never fall)
-        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, h, __float_as_uint(A->first_s[h]), true, target);
+        // from behind the last careful stretch, or from the last block, that the sum did not exceed the target at (it never falls)
+        int h = 0, i = 0;
+        float s = 0.0f;
+        if (A->nfast >= 0) {
+            int n = 0;
+            for (int q = c.lane; q < A->nfast; q += 32) if (!(target < A->u.p1.after[q])) n = q + 1;
+            n = __reduce_max_sync(0xffffffffu, n);
+            if (n > 0) { const int o = A->u.p1.org[n - 1]; h = o >> 9; i = (o & 511) + 1; s = A->u.p1.after[n - 1]; }
+        } else {
+            for (int k = 0; k < g.G; k++) if (!(target < A->first_s[k])) { h = k; s = A->first_s[k]; }
+        }
+        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, h, i, __float_as_uint(s), true, target);
         if (c.lane < g.G) {
             AuxC *ox = cl.map_shared_rank(A, c.lane);
             ox->r_kind = w.h; ox->r_idx = w.first | (w.chunks << 16); ox->r_s = __uint_as_float(w.sb);
@@ -1029,7 +1140,14 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
                 bulk_g2s_last_use(rowbuf + o, src + o, (uint32_t)min(CL_PIECE, nbulk - o) * 4u, &A->mbar);
         }
     }
-    // meanwhile: the tokens a bias or a penalty touches (sample.mojo:381-417), those of this range.
+    // meanwhile: this range's words of the grammar mask, where the tables will be
+    unsigned int *mwords = reinterpret_cast<unsigned int *>(&A->u);
+    static_assert(sizeof(A->u) >= (CL_CAPF / 32 + 2) * sizeof(unsigned int), "the mask's words fit");
+    if (a.mask && g.nloc > 0) {
+        const unsigned int *mrow = a.mask + (long long)r * a.mask_stride + (g.c0 >> 5);
+        for (int i = c.tid; i < (((g.c0 & 31) + g.nloc + 31) >> 5); i += NT) mwords[i] = __ldg(mrow + i);
+    }
+    // and the tokens a bias or a penalty touches (sample.mojo:381-417), those of this range.
     // A small hash (keys and window counts) in the space the candidates use later.
     int *hkey = reinterpret_cast<int *>(A->cand);
     int *hcnt = hkey + HSLOTS;
@@ -1064,17 +1182,27 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     if (__syncthreads_or((c.status & MOLLA_ROW_LOAD_TIMEOUT) ? 1 : 0)) c.status |= MOLLA_ROW_LOAD_TIMEOUT;
     CSTAMP(1);
     if (a.softcap > 0.0f) {
-        for (int i = c.tid; i < g.nloc; i += NT) rowbuf[i] = softcap_pinned(rowbuf[i], a.softcap);
+        const float rcap = softcap_plain(a.softcap) ? __frcp_rn(a.softcap) : 0.0f;
+        for (int i = c.tid; i < g.nloc; i += 4 * NT) {
+            float x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = i + u * NT < g.nloc ? rowbuf[i + u * NT] : 0.0f;
+            softcap4(x, a.softcap, rcap);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (i + u * NT < g.nloc) rowbuf[i + u * NT] = x[u];
+        }
         __syncthreads();
     }
-    if (a.mask) {
+    if (a.mask && g.nloc > 0) {
         // `_mask` (sample.mojo:371-379): what the grammar forbids is no candidate at all. A logit of
         // -inf is exactly that here: it wins no maximum, takes no bias or penalty that could bring it
         // back, its exponential is zero, and zeros are absent from every sum, count and walk.
-        const unsigned int *mrow = a.mask + (long long)r * a.mask_stride;
-        for (int i = c.tid; i < g.nloc; i += NT) {
-            const int t = g.c0 + i;
-            if (!((__ldg(mrow + (t >> 5)) >> (t & 31)) & 1u)) rowbuf[i] = -INFINITY;
+        const int shift = g.c0 & 31;   // (a multiple of four: four logits' bits are in one word)
+        for (int i = 4 * c.tid; i < g.nloc; i += 4 * NT) {
+            const unsigned int w = mwords[(shift + i) >> 5] >> ((shift + i) & 31);
+            float4 &x = *reinterpret_cast<float4 *>(rowbuf + i);
+            x = make_float4((w & 1u) ? x.x : -INFINITY, (w & 2u) ? x.y : -INFINITY, (w & 4u) ? x.z : -INFINITY, (w & 8u) ? x.w : -INFINITY);
         }
         __syncthreads();
     }
@@ -1713,22 +1841,22 @@ void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, unsigned i
     cfg.attrs = at; cfg.numAttrs = 1;
 }
 
-// Whether this device can hold a cluster of G of the kernel's blocks (asked once per device and size).
-bool cluster_fits(int dev, int G) {
-    static int known[CL_MAX_DEVICES][CL_MAX_G + 1] = {};  // 0 unknown, 1 yes, -1 no
-    if (dev < 0 || dev >= CL_MAX_DEVICES) return false;
-    if (known[dev][G]) return known[dev][G] > 0;
+// How many clusters of G of the kernel's blocks this device holds at a time (asked once per device and size).
+int clusters_resident(int dev, int G) {
+    static int known[CL_MAX_DEVICES][CL_MAX_G + 1] = {};  // 0 unknown, -1 none
+    if (dev < 0 || dev >= CL_MAX_DEVICES) return 0;
+    if (known[dev][G]) return known[dev][G] > 0 ? known[dev][G] : 0;
+    int n = 0;
     bool ok = cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL_SMEM) == cudaSuccess;
     if (ok) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at[1];
         cluster_config(cfg, at, (unsigned)G, G, nullptr);
-        int n = 0;
         ok = cudaOccupancyMaxActiveClusters(&n, sample_rows_cluster_kernel, &cfg) == cudaSuccess && n > 0;
     }
     if (!ok) (void)cudaGetLastError();
-    known[dev][G] = ok ? 1 : -1;
-    return ok;
+    known[dev][G] = ok ? n : -1;
+    return ok ? n : 0;
 }
 
 }  // namespace
@@ -1749,7 +1877,18 @@ bool molla_cluster_better(int V, int B, int call_B) {
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const ClusterShape cs = cluster_shape(V, call_B, sms);
-    return cs.G != 0 && (long long)B * cs.G * 9 <= (long long)sms * 8 && cluster_fits(dev, cs.G);
+    return cs.G != 0 && (long long)B * cs.G * 9 <= (long long)sms * 8 && clusters_resident(dev, cs.G) > 0;
+}
+
+// Whether the clusters of all B rows fit the device at the same time. Of those of eight blocks 15 or 16 do, depending
+// on which of its SMs a device has: 16 rows of 262144 in two rounds took 133 to 140 us with mixed settings, 95 with a
+// top-k and 141 with nothing sorted, where the tile kernels take 115, 61 and 93.
+bool molla_cluster_resident(int V, int B, int call_B) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const ClusterShape cs = cluster_shape(V, call_B, sms);
+    return cs.G != 0 && B <= clusters_resident(dev, cs.G);
 }
 
 int molla_cluster_launch(const BatchArgs &args_in, cudaStream_t st, char *err, size_t errlen) {

@@ -241,18 +241,7 @@ __device__ __noinline__ void finish_row(const BatchArgs &a, int r, const RowCfg 
 }
 
 // ---- arithmetic -------------------------------------------------------------------------------
-// x / d, correctly rounded, for many x and one d: two steps of the division by a reciprocal with
-// fused multiply-adds of Markstein (IBM J. Res. Dev. 34, 1990): with y = RN(1/d) the first step is
-// within an ulp, its remainder is exact, and the second step rounds correctly. Five operations in
-// place of a division's own sequence. Holds while nothing under- or overflows on the way: the
-// callers see to that (F_FASTDIV).
-__device__ __forceinline__ float div_by(float x, float d, float y) {
-    const float q0 = __fmul_rn(x, y);
-    const float q1 = __fmaf_rn(__fmaf_rn(-q0, d, x), y, q0);
-    return __fmaf_rn(__fmaf_rn(-q1, d, x), y, q1);
-}
 // (out of line: the compiler's division is long, and a row's code is read from L2 once per SM)
-__device__ __noinline__ float softcap_slow(float x, float cap) { return softcap_pinned(x, cap); }
 __device__ __noinline__ float div_slow(float x, float d) { return __fdiv_rn(x, d); }
 // a probability e / Z (Z between 1 and the vocabulary's size; e in [0, 1])
 __device__ __forceinline__ float prob_of(float e, float Z, float y) {
@@ -342,8 +331,14 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
         __syncwarp();
         const int m = mine_on ? n - (e0 + lane * 32) : 0;  // this lane's logits that exist
         if (a.softcap > 0.0f) {
+            const float rcap = softcap_plain(a.softcap) ? __frcp_rn(a.softcap) : 0.0f;
 #pragma unroll 1
-            for (int j = 0; j < min(32, m); j++) mine[j] = softcap_slow(mine[j], a.softcap);
+            for (int j = 0; j < min(32, m); j += 4) {   // (what lies past the row's end stays -inf)
+                float4 &v = *reinterpret_cast<float4 *>(mine + j);
+                float x[4] = {v.x, v.y, v.z, v.w};
+                softcap4(x, a.softcap, rcap);
+                v = make_float4(x[0], j + 1 < m ? x[1] : -INFINITY, j + 2 < m ? x[2] : -INFINITY, j + 3 < m ? x[3] : -INFINITY);
+            }
             __syncwarp();
         }
         if (a.mask && m > 0) {
