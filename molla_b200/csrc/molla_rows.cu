@@ -1824,12 +1824,11 @@ __device__ __forceinline__ void plan_want(PlanFind &F, int b) {   // one thread
 // What is left out here is only slower: row_tail then looks for it in the list.
 __device__ __noinline__ void plan_picks(const RowsArgs &R, int rr, float hs, int j0, int nb) {
     __shared__ PlanFind F;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     const RowCfg &g = R.head(rr)->plan.c;
-    const double slack = 96.0;
     double start[WALK_BINADES];
     int hi_of[WALK_BINADES], low_of[WALK_BINADES];
-    double s = (double)hs, sum_lo = s, sum_hi = s;
+    double s = (double)hs, sum_lo = s, sum_hi = s, unsure = 0.0;   // unsure: how far s may be off
     int hi = NBINS, phases = 0;
     if (tid == 0) F.n = 0;
     // stretch p: the running sum in binade j0 + p
@@ -1847,12 +1846,24 @@ __device__ __noinline__ void plan_picks(const RowsArgs &R, int rr, float hs, int
         const int hb = F.hit;
         if (hb < 0) { s = s + F.total * unit; sum_lo = sum_hi = s; hi = 0; continue; }
         low_of[p] = hb;
+        // the ties down to that bin add to the sum but are not in the table
+        const WalkTies *t = R.ties(rr) + p;
+        const int nt = min(__ldcg(&t->n), TIE_CAP);
+        float tied = 0.0f;
+#pragma unroll 1
+        for (int i = lane; i < nt; i += 32) {
+            const unsigned int b = (unsigned int)(__ldcg(&t->key[i]) >> 32);
+            if ((int)(b >> BIN_SHIFT) >= hb && (int)(b >> BIN_SHIFT) < hi) tied += __uint_as_float(b);
+        }
+        const double more = (double)warp_sum(tied) * inv, slack = 96.0 + unsure * inv;
         if (tid == 0) {
             plan_want(F, hb);
-            if (x - F.before < slack) plan_want(F, (int)F.prev);
+            if (x - F.before < slack + more) plan_want(F, (int)F.prev);
             if (F.end - x < slack) plan_want(F, F.next);
         }
-        s = F.end * unit;
+        s = F.end * unit + more * unit;
+        // the elements of that bin behind the crossing add units of the next binade
+        if (!by_cut && p + 1 < nb) unsure += fabs((double)__ldcg(R.table(rr, p) + hb) * unit - (double)__ldcg(R.table(rr, p + 1) + hb) * 2.0 * unit);
         sum_lo = sum_hi = s;
         if (by_cut) { sum_lo = x * unit; sum_hi = fmin(s, (x + slack) * unit + (double)__uint_as_float((unsigned int)(hb + 1) << BIN_SHIFT)); }
         hi = by_cut ? 0 : hb;
@@ -1905,18 +1916,30 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_next();
     pdl_wait();
-    const int work = R.queue[0] * R.nspan;
+    // a block takes neighbouring spans of a row, as many as make one round of blocks, and adds their tables up once
+    const int queued = R.queue[0], each = max(1, min(R.nspan, (queued * R.nspan + (int)gridDim.x - 1) / (int)gridDim.x)), groups = (R.nspan + each - 1) / each;
 #pragma unroll 1
-    for (int wi = blockIdx.x; wi < work; wi += gridDim.x) {
-        const int rr = R.queue[1 + wi / R.nspan], span = wi % R.nspan, tile = span * (SPAN / TILE) + warp;
+    for (int wi = blockIdx.x; wi < queued * groups; wi += gridDim.x) {
+        const int rr = R.queue[1 + wi / groups], span0 = wi % groups * each, span1 = min(R.nspan, span0 + each);
         RowHead *head = R.head(rr);
         const int state = head->state;
         if (state != ST_HEAD && state != ST_PURE) continue;
         const float Z = head->Z, yZ = __fdiv_rn(1.0f, Z);
+        const unsigned int tau = head->plan.tau_bits;
+        const float hs = head->head_s;
+        const int j0 = hs > 0.0f ? fexpo(hs) : 0, nb = (hs > 0.0f && j0 >= -30 && j0 < 0) ? min(WALK_BINADES, -j0) : 0;
+        __syncthreads();
+        if (state == ST_HEAD) {
+#pragma unroll 1
+            for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) { (&S->hq[0][0])[i] = 0u; (&S->hqh[0][0])[i] = 0u; }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int span = span0; span < span1; span++) {
+        const int tile = span * (SPAN / TILE) + warp;
         const size_t gt = (size_t)rr * R.ntile + tile;
         const int n = tile < R.ntile ? (int)R.to(rr)[tile].cnt : 0;
         float4 *src = reinterpret_cast<float4 *>(R.elist + gt * TILE);
-        __syncthreads();
         if (state == ST_PURE) {
             if (tile >= R.ntile) continue;
             float *list = S->x + (size_t)warp * 32 * PITCH;
@@ -1952,15 +1975,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             continue;
         }
         // ---- past a sorted head: what it took is consumed
-        const unsigned int tau = head->plan.tau_bits;
-        const float hs = head->head_s;
-        const int j0 = hs > 0.0f ? fexpo(hs) : 0, nb = (hs > 0.0f && j0 >= -30 && j0 < 0) ? min(WALK_BINADES, -j0) : 0;
-        __syncthreads();
-#pragma unroll 1
-        for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) { (&S->hq[0][0])[i] = 0u; (&S->hqh[0][0])[i] = 0u; }
-        __syncthreads();
         float4 nx = 4 * lane < n ? src[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float half0 = fpow2(j0 - 24);   // below half a unit of the first binade: adds nothing from here on
 #pragma unroll 1
         for (int e0 = 4 * lane; e0 < n; e0 += 128) {
             const float4 v = nx;
@@ -1969,15 +1984,16 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 p[u] = (e0 + u < n && __float_as_uint(p[u]) < tau) ? prob_of(p[u], Z, yZ) : 0.0f;
-                if (!(p[u] >= half0)) continue;
                 const unsigned int pb = __float_as_uint(p[u]);
                 const int bin = (int)(pb >> BIN_SHIFT);
-#pragma unroll 1
-                for (int b = 0; b < nb; b++) {
+#pragma unroll
+                for (int b = 0; b < WALK_BINADES; b++) {
+                    const float half = fpow2(j0 + b - 24);   // below half a unit of a binade: adds nothing there, nor in the ones above
+                    if (b >= nb || !(p[u] >= half)) break;
                     const float Cm = __fmul_rn(1.5f, fpow2(j0 + b));
                     const float tq = __fadd_rn(p[u], Cm);
                     const float rr_ = __fsub_rn(p[u], __fsub_rn(tq, Cm));
-                    if (fabsf(rr_) == fpow2(j0 + b - 24) || p[u] >= fpow2(j0 + b - 1)) {
+                    if (fabsf(rr_) == half || p[u] >= fpow2(j0 + b - 1)) {
                         // a rounding tie: listed (an element of a quarter of the sum cannot follow a whole head)
                         WalkTies *t = R.ties(rr) + b;
                         const int at = atomicAdd(&t->n, 1);
@@ -1993,6 +2009,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             }
             src[e0 >> 2] = make_float4(p[0], p[1], p[2], p[3]);
         }
+        }
+        if (state == ST_PURE) continue;
         __syncthreads();
 #pragma unroll 1
         for (int i = tid; i < nb * NBINS; i += SPAN_THREADS) {
@@ -2002,7 +2020,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
         // the block that finishes a row's tables works out which bins the walk will want
         __threadfence();
         __syncthreads();
-        if (tid == 0) S_last = atomicAdd(&R.picks(rr)->arrived, 1) == R.nspan - 1 ? 1 : 0;
+        if (tid == 0) S_last = atomicAdd(&R.picks(rr)->arrived, 1) == groups - 1 ? 1 : 0;
         __syncthreads();
         if (S_last && nb > 0) {
             __threadfence();
@@ -2966,21 +2984,56 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
         if (tail_pure(c)) return;
         __syncthreads();
     }
-    c.pl = head->plan;
+    // what the row will look up, in one round of loads: its tiles' entries and items; behind a head that row_head has
+    // sorted, the candidates, the walk's ties, the gathered bins and the first binade's table too
+    static_assert(MAX_TILES <= 2 * NT && sizeof(AuxF::ties) / 16 <= NT && sizeof(AuxF::u.h) >= NBINS * sizeof(unsigned long long), "a load or two a thread");
     const BatchArgs &a = R.a;
+    const int ntile = R.ntile, nhead = state == ST_HEAD ? head->ncand : 0;
+    unsigned long long *gcand = R.cand(rr);
+    {
+        TileOut o[2];
+        uint4 vt = make_uint4(0u, 0u, 0u, 0u), vp = vt, x[NBINS / 2 / NT];
+        unsigned long long k = 0ull, k0 = 0ull, k1 = 0ull;
+        float pre = 0.0f;
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+            if (c.tid + u * NT < ntile) o[u] = R.to(rr)[c.tid + u * NT];
+        if (state == ST_HEAD) {
+            if (c.tid < (int)(sizeof(A->ties) / 16)) vt = reinterpret_cast<const uint4 *>(R.ties(rr))[c.tid];
+            if (c.tid < (int)(sizeof(WalkPicks) / 16)) vp = reinterpret_cast<const uint4 *>(R.picks(rr))[c.tid];
+#pragma unroll
+            for (int i = 0; i < NBINS / 2 / NT; i++) x[i] = reinterpret_cast<const uint4 *>(R.table(rr, 0))[c.tid + i * NT];
+            k = gcand[c.tid]; k0 = c.tid > 0 ? gcand[c.tid - 1] : 0ull; k1 = gcand[c.tid + 1]; pre = R.pre(rr)[c.tid];
+        }
+        c.pl = head->plan;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int t = c.tid + u * NT;
+            if (t < ntile) { A->tcnt[t] = o[u].cnt; A->tni[t] = o[u].nitem; A->tio[t] = o[u].ioff; }
+        }
+        if (state == ST_HEAD) {
+            if (c.tid < (int)(sizeof(A->ties) / 16)) reinterpret_cast<uint4 *>(A->ties)[c.tid] = vt;
+            if (c.tid < (int)(sizeof(WalkPicks) / 16)) reinterpret_cast<uint4 *>(&A->picks)[c.tid] = vp;
+#pragma unroll
+            for (int i = 0; i < NBINS / 2 / NT; i++) reinterpret_cast<uint4 *>(&A->u.h)[c.tid + i * NT] = x[i];
+            auto store = [&](int i, unsigned long long key, unsigned long long before, unsigned long long behind, float sum) {
+                const unsigned int p = (unsigned int)(key >> 32);
+                const bool eq = (i > 0 && (unsigned int)(before >> 32) == p) || (i + 1 < nhead && (unsigned int)(behind >> 32) == p);
+                A->pre[i] = sum;
+                A->hidx[i] = (unsigned int)key_idx(key) | (eq ? 0x80000000u : 0u);
+            };
+            if (c.tid < nhead) store(c.tid, k, k0, k1, pre);
+#pragma unroll 1
+            for (int i = c.tid + NT; i < nhead; i += NT) store(i, gcand[i], gcand[i - 1], i + 1 < nhead ? gcand[i + 1] : 0ull, R.pre(rr)[i]);
+        }
+    }
     c.cfg = c.pl.c;
     c.list = R.elist + (size_t)c.rr * R.ntile * TILE;
     c.gitems = R.items(rr);
     c.kmask = R.kmask + (size_t)c.rr * R.ntile * 32;
     const RowCfg &g = c.cfg;
-    const int ntile = R.ntile, imax = c.pl.imax;
-#pragma unroll 1
-    for (int t = c.tid; t < ntile; t += NT) {
-        const TileOut o = R.to(rr)[t];
-        A->tcnt[t] = o.cnt; A->tni[t] = o.nitem; A->tio[t] = o.ioff;
-    }
+    const int imax = c.pl.imax;
     __syncthreads();
-    unsigned long long *gcand = R.cand(rr);
     int nc_all = g.pure ? 0 : head->ncand;
     if (nc_all > HEADCAP) {
         __syncthreads();
@@ -3126,29 +3179,6 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
     long long head_pos;
     if (state == ST_HEAD) {   // row_head has sorted it and added it up
         head_s = head->head_s; head_pos = head->head_pos;
-        // what the walk will look up, all at once: its ties, the gathered bins, the first binade's table
-        static_assert(sizeof(A->u.h) >= NBINS * sizeof(unsigned long long), "a table takes the space of the walk's own histograms");
-        const uint4 *from = reinterpret_cast<const uint4 *>(R.ties(rr));
-        uint4 *to = reinterpret_cast<uint4 *>(A->ties);
-        for (int i = c.tid; i < (int)(sizeof(A->ties) / 16); i += NT) to[i] = from[i];
-        from = reinterpret_cast<const uint4 *>(R.picks(rr));
-        to = reinterpret_cast<uint4 *>(&A->picks);
-        if (c.tid < (int)(sizeof(WalkPicks) / 16)) to[c.tid] = from[c.tid];
-        from = reinterpret_cast<const uint4 *>(R.table(rr, 0));
-        to = reinterpret_cast<uint4 *>(&A->u.h);
-        uint4 x[NBINS / 2 / NT];
-#pragma unroll
-        for (int i = 0; i < NBINS / 2 / NT; i++) x[i] = from[c.tid + i * NT];
-#pragma unroll
-        for (int i = 0; i < NBINS / 2 / NT; i++) to[c.tid + i * NT] = x[i];
-#pragma unroll 1
-        for (int i = c.tid; i < nc; i += NT) {
-            const unsigned int p = (unsigned int)(gcand[i] >> 32);
-            const bool eq = (i > 0 && (unsigned int)(gcand[i - 1] >> 32) == p) || (i + 1 < nc && (unsigned int)(gcand[i + 1] >> 32) == p);
-            A->pre[i] = R.pre(rr)[i];
-            A->hidx[i] = (unsigned int)key_idx(gcand[i]) | (eq ? 0x80000000u : 0u);
-        }
-        __syncthreads();
     } else {
     {
 #pragma unroll 1
