@@ -115,7 +115,7 @@ struct __align__(16) AuxC {
     // elements of a walk that would round on a tie: their keys, bins, the mass before them
     long long rx[8];          // words fetched from the leader for the whole block
     int ngath, ngath_over;   // a bin's entries collected by this block; blocks whose own buffer overflowed (leader's)
-    int ntie[2]; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP]; unsigned long long tpqm[TIE_CAP], tabove[TIE_CAP], tc[TIE_CAP];
+    int ntie[2]; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned char tord[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP]; unsigned long long tpqm[TIE_CAP], tabove[TIE_CAP], tc[TIE_CAP];
     unsigned int tbits[NBINS / 32];
     int r_kind; int r_idx; float r_s; long long r_pos; unsigned int r_status;  // the leader's word after the head
 };
@@ -808,6 +808,7 @@ __device__ void descend_cluster(cg::cluster_group &cl, CtxC &c, const ClGeo &g, 
         qy.hq = A->u.h.hq; qy.hqh = A->u.h.hqh; qy.hc = A->u.h.hc;
         qy.pos0 = (unsigned long long)w.pos;
         qy.nstop = counting ? (unsigned long long)nstop : ~0ull;
+        qy.counts = counting || !binade_ok;
         qy.m0 = 0; qy.xq = ~0ull;
         if (binade_ok) {
             qy.m0 = (unsigned long long)((double)w.s * (double)inv_u);
@@ -877,15 +878,17 @@ __device__ void descend_cluster(cg::cluster_group &cl, CtxC &c, const ClGeo &g, 
                             if (A->tbin[t] == b) A->tabove[t] = run;
                         run += q[i];
                     }
+                    if (c.tid < ntie) {   // the ties' order from the top
+                        int rank = 0;
+                        for (int t = 0; t < ntie; t++) rank += A->tkey[t] > A->tkey[c.tid] ? 1 : 0;
+                        A->tord[rank] = (unsigned char)c.tid;
+                    }
                     __syncthreads();
                     if (c.tid == 0) {
                         // from the top down (what lies below an event never matters: the walk stops there)
-                        unsigned long long done = 0ull, carried = 0ull;
+                        unsigned long long carried = 0ull;
                         for (int round = 0; round < ntie; round++) {
-                            int best = -1;
-                            for (int t = 0; t < ntie; t++)
-                                if (!((done >> t) & 1ull) && (best < 0 || A->tkey[t] > A->tkey[best])) best = t;
-                            done |= 1ull << best;
+                            const int best = A->tord[round];
                             const float p = key_val(A->tkey[best]);
                             const float qf = __fsub_rn(__fadd_rn(p, Cm), Cm);
                             unsigned long long k = (unsigned long long)__float2uint_rn(__fmul_rn(qf, inv_u));

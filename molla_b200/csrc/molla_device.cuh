@@ -197,7 +197,14 @@ __device__ __forceinline__ T warp_incl_scan(T v, int lane) {
     return v;
 }
 // Exclusive scan over the NT threads of a CTA; `ws` is NWARP elements of shared
-// scratch. Every thread gets its exclusive prefix and the block total.
+// scratch. Every thread gets its exclusive prefix and the block total. Every warp scans the warps' totals for itself:
+// one barrier less than with one warp doing it for all.
+template <class T>
+__device__ __forceinline__ void warp_bases(T mine, int warp, int lane, T &base, T &total) {
+    const T wi = warp_incl_scan(mine, lane), ex = wi - mine;
+    base = __shfl_sync(0xffffffffu, ex, warp);
+    total = __shfl_sync(0xffffffffu, wi, NWARP - 1);
+}
 template <class T>
 __device__ __forceinline__ T block_excl_scan(T v, T *ws, T *total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -205,16 +212,9 @@ __device__ __forceinline__ T block_excl_scan(T v, T *ws, T *total) {
     __syncthreads();  // ws may still be read by an earlier call
     if (lane == 31) ws[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        T w = lane < NWARP ? ws[lane] : T(0);
-        T wi = warp_incl_scan(w, lane);
-        if (lane < NWARP) ws[lane] = wi - w;
-        if (lane == NWARP - 1) ws[NWARP] = wi;
-    }
-    __syncthreads();
-    T out = ws[warp] + (inc - v);
-    *total = ws[NWARP];
-    return out;
+    T base;
+    warp_bases<T>(lane < NWARP ? ws[lane] : T(0), warp, lane, base, *total);
+    return base + (inc - v);
 }
 
 // Exclusive scan of two doubles at once (one pass of barriers for both).
@@ -225,15 +225,10 @@ __device__ __forceinline__ void block_excl_scan2(double a, double b, double *ws 
     __syncthreads();
     if (lane == 31) { ws[warp] = ia; ws[NWARP + 1 + warp] = ib; }
     __syncthreads();
-    if (warp == 0) {
-        double wa = lane < NWARP ? ws[lane] : 0.0, wb = lane < NWARP ? ws[NWARP + 1 + lane] : 0.0;
-        double sa = warp_incl_scan(wa, lane), sb = warp_incl_scan(wb, lane);
-        if (lane < NWARP) { ws[lane] = sa - wa; ws[NWARP + 1 + lane] = sb - wb; }
-        if (lane == NWARP - 1) { ws[NWARP] = sa; ws[2 * NWARP + 1] = sb; }
-    }
-    __syncthreads();
-    ea = ws[warp] + (ia - a); eb = ws[NWARP + 1 + warp] + (ib - b);
-    ta = ws[NWARP]; tb = ws[2 * NWARP + 1];
+    double ba, bb;
+    warp_bases(lane < NWARP ? ws[lane] : 0.0, warp, lane, ba, ta);
+    warp_bases(lane < NWARP ? ws[NWARP + 1 + lane] : 0.0, warp, lane, bb, tb);
+    ea = ba + (ia - a); eb = bb + (ib - b);
 }
 
 // ---- mbarrier + bulk copy (TMA without a tensor map, never multicast) ---------

@@ -492,6 +492,7 @@ struct BinQuery {
     int specbin;                     // stop at this bin (-1 disables)
     int bin_hi;                      // only bins below this one count (NBINS = all)
     const unsigned int *spec_bits;   // or: stop at any bin whose bit is set here (nullptr = use specbin)
+    bool counts = true;              // whether anybody asks for counts (else they are all zero)
     const unsigned int *hq, *hqh, *hc;  // per bin: integer mass (low MASS_SPLIT bits summed, the rest summed) and count
 };
 
@@ -512,7 +513,7 @@ __device__ void find_event_bin_adj(CX &c, const BinQuery &qy, LD bin_load, ADJ a
         if (live) bin_load(b, q[i], n[i]);
         sq += q[i]; sn += n[i];
     }
-    unsigned long long tq, tc;
+    unsigned long long tq, tc = 0ull, ec = 0ull;
     unsigned long long eq = block_excl_scan<unsigned long long>(sq, A->wsu, &tq);
     if constexpr (!std::is_same<ADJ, NoAdjust>::value) if (adjust(q, eq)) {
         sq = 0;
@@ -520,10 +521,10 @@ __device__ void find_event_bin_adj(CX &c, const BinQuery &qy, LD bin_load, ADJ a
         for (int i = 0; i < BPT; i++) sq += q[i];
         eq = block_excl_scan<unsigned long long>(sq, A->wsu, &tq);
     }
-    const unsigned long long ec = block_excl_scan<unsigned long long>(sn, A->wsu, &tc);
-    __syncthreads();
-    if (c.tid == 0) { A->evt_thread = 0x7fffffff; A->tot_q = tq; A->tot_c = tc; A->hit_bin = -1; }
-    __syncthreads();
+    if (c.tid == 0) { A->evt_thread = 0x7fffffff; A->hit_bin = -1; }
+    if (qy.counts) ec = block_excl_scan<unsigned long long>(sn, A->wsu, &tc);
+    else __syncthreads();
+    if (c.tid == 0) { A->tot_q = tq; A->tot_c = tc; }
     int hit = -1;
     unsigned long long cq = eq, cc = ec, hq_before = 0, hc_before = 0;
 #pragma unroll

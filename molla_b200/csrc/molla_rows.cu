@@ -2116,7 +2116,7 @@ struct __align__(16) AuxF {
     float b_sum, b_target;
     unsigned int w_sb; int w_i, w_need, w_found, w_tile, w_at;   // the items' runner
     WalkTies ties[WALK_BINADES]; WalkPicks picks;   // row_tail's copies
-    int ntie; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP];
+    int ntie; unsigned long long tkey[TIE_CAP]; int tbin[TIE_CAP]; unsigned char tord[TIE_CAP]; unsigned int tpq_lo[TIE_CAP], tpq_hi[TIE_CAP];
     unsigned long long tpqm[TIE_CAP], tabove[TIE_CAP], tc[TIE_CAP];
     unsigned int tbits[NBINS / 32];
 };
@@ -2545,6 +2545,7 @@ __device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x
         qy.hq = A->u.h.hq; qy.hqh = A->u.h.hqh; qy.hc = A->u.h.hc;
         qy.pos0 = (unsigned long long)w.pos;
         qy.nstop = counting ? (unsigned long long)nstop : ~0ull;
+        qy.counts = counting || !binade_ok;
         qy.m0 = 0; qy.xq = ~0ull;
         if (binade_ok) {
             qy.m0 = (unsigned long long)((double)w.s * (double)inv_u);
@@ -2719,18 +2720,20 @@ __device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x
                         if (A->tbin[t] == b) A->tabove[t] = run;
                     run += q[i];
                 }
+                if (c.tid < ntie) {   // the ties' order from the top
+                    int rank = 0;
+#pragma unroll 1
+                    for (int t = 0; t < ntie; t++) rank += A->tkey[t] > A->tkey[c.tid] ? 1 : 0;
+                    A->tord[rank] = (unsigned char)c.tid;
+                }
                 __syncthreads();
                 if (c.tid == 0) {
                     // from the top down (what lies below an event never matters: the walk stops there)
-                    unsigned long long done = 0ull, carried = 0ull;
+                    unsigned long long carried = 0ull;
 #pragma unroll 1
-                    for (int round = 0; round < ntie; round++) {
-                        int best = -1;
-#pragma unroll 1
-                        for (int t = 0; t < ntie; t++)
-                            if (!((done >> t) & 1ull) && (best < 0 || A->tkey[t] > A->tkey[best])) best = t;
-                        done |= 1ull << best;
-                        const float p = key_val(A->tkey[best]);
+                        for (int round = 0; round < ntie; round++) {
+                            const int best = A->tord[round];
+                            const float p = key_val(A->tkey[best]);
                         const float qf = __fsub_rn(__fadd_rn(p, Cm), Cm);
                         unsigned long long k = (unsigned long long)__float2uint_rn(__fmul_rn(qf, inv_u));
                         if (qf > p) k -= 1ull;  // the multiple of the unit below p
