@@ -1,16 +1,15 @@
 // Logprobs of the raw logits (sample.mojo:268-293) for rows of 4096 logits and more: the chosen token's,
 // the top N's, or a whole row's. A tile of 1024 logits belongs to one warp, so a few rows fill the chip
 // as well as many: one block per row, as for short rows, took 97 us for 64 rows of 151936 logits and left
-// half of the SMs idle. Whole rows' logprobs, 64 of 128256: 109 us before, 22 now (3.0 TB/s of the 66 MB, which
-// the second pass finds in L2; floor 10 us). 4096 is where a row has four tiles, fewer would leave most of
-// a block of eight warps idle.
+// half of the SMs idle. 4096 is where a row has four tiles, fewer would leave most of a block of eight warps idle.
 //
 //   lp_tiles  every tile: its maximum and the sum of exp(z - maximum), accumulated in fp64
 //                                           (bound: HBM, 4 bytes per logit, and an exponential per logit)
 //   lp_rows   every row: maximum, logarithm of the sum, the chosen token, the top N. The N-th largest of
 //             the tiles' maxima bounds the N-th largest logit from below, so only tiles whose maximum
 //             reaches it, N of them but for ties, are looked at again
-//   lp_write  every tile of a whole row's logprobs: z - maximum - logarithm (bound: HBM, 8 bytes per logit)
+//   lp_whole  whole rows' logprobs, z - maximum - logarithm: a row per thread-block cluster
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -32,11 +31,11 @@ struct LpArgs {
     const int *tokens; int top_n; float *chosen; int *top_ids; float *top_lps;
     const int *rows; int n_logit_rows; float softcap;
     float *out;                   // whole rows' logprobs, or nullptr
-    float *stats; long long stats_row, stats_tile;   // tile t of row r: four floats at stats + r * stats_row + t * stats_tile
+    float *stats;                 // [rows][ntile] four floats
     int ntile;
 };
 
-__device__ __forceinline__ float *stat_of(const LpArgs &a, int r, int t) { return a.stats + (long long)r * a.stats_row + (long long)t * a.stats_tile; }
+__device__ __forceinline__ float *stat_of(const LpArgs &a, int r, int t) { return a.stats + ((long long)r * a.ntile + t) * 4; }
 // which row of the block batch row r reads; -1 for a stale index (the row's sampling call has reported it)
 __device__ __forceinline__ long long logit_row(const LpArgs &a, int r) {
     const long long l = a.rows ? (long long)a.rows[r] : (long long)r;
@@ -63,23 +62,9 @@ __device__ __forceinline__ bool load_tile(float (&x)[34], const float *z, int n,
 }
 __device__ __forceinline__ float capped(const LpArgs &a, float x) { return a.softcap > 0.0f ? softcap_pinned(x, a.softcap) : x; }
 
-__global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
-    const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
-    if (t >= a.ntile) return;
-    const long long lrow = logit_row(a, r);
-    if (lrow < 0) return;
-    const float *z = a.logits + lrow * a.row_stride + (long long)t * LTILE;
-    const int n = tile_end(a, t) - t * LTILE;
-    float x[34];
-    (void)load_tile(x, z, n, lane, (reinterpret_cast<uintptr_t>(z) & 15u) == 0, -INFINITY);
-    float m = -INFINITY;
-    if (a.softcap > 0.0f) {
-#pragma unroll
-        for (int i = 0; i < 34; i++) if (x[i] > -INFINITY) x[i] = softcap_pinned(x[i], a.softcap);
-    }
+// A tile's maximum and its sum of exp(z - maximum) in fp64, one warp.
+__device__ __forceinline__ void tile_stat(const float (&x)[34], float &m, double &sum) {
+    m = -INFINITY;
 #pragma unroll
     for (int i = 0; i < 34; i++) m = fmaxf(m, x[i]);
     m = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(m)));
@@ -94,7 +79,29 @@ __global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a
     s0 += s1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    if (lane == 0) {   // (whole rows' logprobs keep this in the tile's own output, which need not be aligned)
+    sum = s0;
+}
+
+__global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
+    const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
+    if (t >= a.ntile) return;
+    const long long lrow = logit_row(a, r);
+    if (lrow < 0) return;
+    const float *z = a.logits + lrow * a.row_stride + (long long)t * LTILE;
+    const int n = tile_end(a, t) - t * LTILE;
+    float x[34];
+    (void)load_tile(x, z, n, lane, (reinterpret_cast<uintptr_t>(z) & 15u) == 0, -INFINITY);
+    if (a.softcap > 0.0f) {
+#pragma unroll
+        for (int i = 0; i < 34; i++) if (x[i] > -INFINITY) x[i] = softcap_pinned(x[i], a.softcap);
+    }
+    float m;
+    double s0;
+    tile_stat(x, m, s0);
+    if (lane == 0) {
         float *o = stat_of(a, r, t);
         const unsigned long long b = (unsigned long long)__double_as_longlong(s0);
         o[0] = m; o[1] = __uint_as_float((unsigned int)b); o[2] = __uint_as_float((unsigned int)(b >> 32));
@@ -153,10 +160,6 @@ __global__ void __launch_bounds__(LT_) lp_rows(const __grid_constant__ LpArgs a)
 #pragma unroll
     for (int w = 0; w < LT_ / 32; w++) s += wsd[w];
     const float offset = (float)log(s);
-    if (a.out) {   // a copy for every tile, in the tile's own output
-        for (int t = tid; t < a.ntile; t += LT_) { float *o = stat_of(a, r, t); o[0] = top; o[1] = offset; }
-        return;
-    }
     if (a.chosen && a.tokens && tid == 0) {
         const int t = a.tokens[r];
         a.chosen[r] = (t >= 0 && t < a.V) ? __fsub_rn(__fsub_rn(capped(a, __ldg(z + t)), top), offset) : 0.0f;
@@ -244,40 +247,85 @@ __global__ void __launch_bounds__(LT_) lp_rows(const __grid_constant__ LpArgs a)
     }
 }
 
-__global__ void __launch_bounds__(LT_) lp_write(const __grid_constant__ LpArgs a) {
+// A whole row's logprobs, one cluster: every block its tiles' maxima and sums, those of all blocks through distributed
+// shared memory, then the same tiles again, which are in L2 (the clusters in flight hold some 300 bytes per logit of
+// the vocabulary), and the result. Bound: the exponentials' instructions, then the store. One launch: with a kernel
+// for the tiles, one for the rows and one for the result, 64 rows of 128256 took 22.0 us, now 19.3 (floor 10), 512 of
+// 262144 285 and 221, 16 of 32000 12.5 and 8.1. Clusters of sixteen where those of eight leave SMs without a block, or a
+// block with more than three rounds of tiles: 7 rows of 700000 took 21.8 us in clusters of eight, 13.8 of sixteen.
+constexpr int LG_MOST = 16;
+__global__ void __launch_bounds__(512, 2) lp_whole(const __grid_constant__ LpArgs a) {
+    namespace cg = cooperative_groups;
+    __shared__ float tm[LMAX_TILES], bm[LG_MOST], s_top, s_off;
+    __shared__ double ts[LMAX_TILES], bs[LG_MOST];
+    cg::cluster_group cl = cg::this_cluster();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
-    const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
-    if (t >= a.ntile) return;
-    const float *z = a.logits + (long long)r * a.row_stride + (long long)t * LTILE;
-    float *o = stat_of(a, r, t);   // this is also where the tile's logprobs go
-    const int n = tile_end(a, t) - t * LTILE;
-    const float top = o[0], offset = o[1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5, G = (int)cl.num_blocks(), rank = (int)cl.block_rank(), r = (int)blockIdx.x / G;
+    const int per = (a.ntile + G - 1) / G, t0 = rank * per, n = max(0, min(per, a.ntile - t0));
+    const float *z = a.logits + (long long)r * a.row_stride + (long long)t0 * LTILE;
+    float *o = a.out + (long long)r * a.V + (long long)t0 * LTILE;
+    const bool in16 = (reinterpret_cast<uintptr_t>(z) & 15u) == 0, out16 = (reinterpret_cast<uintptr_t>(o) & 15u) == 0;
     float x[34];
-    const bool vec = load_tile(x, z, n, lane, ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0, 0.0f);
-#pragma unroll
-    for (int i = 0; i < 34; i++) x[i] = __fsub_rn(__fsub_rn(x[i], top), offset);
-    __syncwarp();   // every lane has read the tile's copy
-    if (vec) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) __stcs(reinterpret_cast<float4 *>(o) + lane + 32 * i, make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; i++)
-            if (lane + 32 * i < n) __stcs(o + lane + 32 * i, x[i]);
+#pragma unroll 1
+    for (int t = warp; t < n; t += warps) {
+        (void)load_tile(x, z + t * LTILE, tile_end(a, t0 + t) - (t0 + t) * LTILE, lane, in16, -INFINITY);
+        float m;
+        double s;
+        tile_stat(x, m, s);
+        if (lane == 0) { tm[t] = m; ts[t] = s; }
     }
-    if (LTILE + lane < n) o[LTILE + lane] = x[32];
-    if (LTILE + 32 + lane < n) o[LTILE + 32 + lane] = x[33];
+    __syncthreads();
+    if (warp == 0) {
+        float m = -INFINITY;
+        for (int t = lane; t < n; t += 32) m = fmaxf(m, tm[t]);
+        m = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(m)));
+        double s = 0.0;
+        for (int t = lane; t < n; t += 32)
+            if (tm[t] > -INFINITY) s += ts[t] * exp((double)tm[t] - (double)m);
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) s += __shfl_xor_sync(0xffffffffu, s, i);
+        if (lane < G) { *cl.map_shared_rank(&bm[rank], lane) = m; *cl.map_shared_rank(&bs[rank], lane) = s; }
+    }
+    cl.sync();
+    if (warp == 0) {
+        const float m = lane < G ? bm[lane] : -INFINITY, top = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(m)));
+        double s = m > -INFINITY ? bs[lane] * exp((double)m - (double)top) : 0.0;
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) s += __shfl_xor_sync(0xffffffffu, s, i);
+        if (lane == 0) { s_top = top; s_off = (float)log(s); }
+    }
+    __syncthreads();
+    const float top = s_top, offset = s_off;
+#pragma unroll 1
+    for (int t = warp; t < n; t += warps) {
+        const int e = tile_end(a, t0 + t) - (t0 + t) * LTILE;
+        float *to = o + t * LTILE;
+        const bool vec = load_tile(x, z + t * LTILE, e, lane, in16 && out16, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 34; i++) x[i] = __fsub_rn(__fsub_rn(x[i], top), offset);
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) __stcs(reinterpret_cast<float4 *>(to) + lane + 32 * i, make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                if (lane + 32 * i < e) __stcs(to + lane + 32 * i, x[i]);
+        }
+        if (LTILE + lane < e) to[LTILE + lane] = x[32];
+        if (LTILE + 32 + lane < e) to[LTILE + 32 + lane] = x[33];
+    }
 }
 
-cudaError_t lp_launch(void (*kernel)(LpArgs), unsigned int blocks, cudaStream_t st, const LpArgs &a) {
+cudaError_t lp_launch(void (*kernel)(LpArgs), unsigned int blocks, unsigned int threads, unsigned int cluster, cudaStream_t st, const LpArgs &a) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(LT_); cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(threads); cfg.stream = st;
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
@@ -301,11 +349,25 @@ cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int 
     a.tokens = tokens; a.top_n = top_n; a.chosen = chosen; a.top_ids = top_ids; a.top_lps = top_lps;
     a.rows = rows; a.n_logit_rows = n_logit_rows; a.softcap = softcap; a.out = full_out;
     a.ntile = tiles_of(V);
-    if (full_out) { a.stats = full_out; a.stats_row = V; a.stats_tile = LTILE; }
-    else { a.stats = (float *)workspace; a.stats_row = 4ll * a.ntile; a.stats_tile = 4; }
+    if (full_out) {
+        // a block for eight tiles, up to eight of them; twice as many for the widest rows and for few; as many warps as
+        // share a block's tiles evenly in rounds of at most eight, of sixteen where there are not two blocks an SM
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+        int G = 1;
+        while (G < 8 && 8 * G < a.ntile) G *= 2;
+        if (a.ntile > 24 * 8 || (a.ntile > 8 * 8 && (long long)B * G <= 2 * sms)) G = LG_MOST;
+        const long long n = (long long)B * G;
+        const int each = (a.ntile + G - 1) / G, most = n <= 2 * sms ? 16 : 8, rounds = (each + most - 1) / most;
+        if (G > 8) {
+            const cudaError_t e = cudaFuncSetAttribute(lp_whole, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+        }
+        return lp_launch(lp_whole, (unsigned int)n, 32u * (unsigned int)((each + rounds - 1) / rounds), (unsigned int)G, st, a);
+    }
+    a.stats = (float *)workspace;
     const unsigned int blocks = (unsigned int)B * (unsigned int)((a.ntile + 7) / 8);
-    cudaError_t e = lp_launch(lp_tiles, blocks, st, a);
-    if (e == cudaSuccess) e = lp_launch(lp_rows, (unsigned int)B, st, a);
-    if (e == cudaSuccess && full_out) e = lp_launch(lp_write, blocks, st, a);
+    cudaError_t e = lp_launch(lp_tiles, blocks, LT_, 1, st, a);
+    if (e == cudaSuccess) e = lp_launch(lp_rows, (unsigned int)B, LT_, 1, st, a);
     return e;
 }

@@ -632,3 +632,19 @@ def test_pick_rows_is_the_batched_decode_step(dev, lib, oracle):
         toks = S.pick_rows(block, batch)
         assert toks == [s.pick(block, row=i) for i, s in enumerate(solo)]
         assert all(s.drawn == step + 1 for s in batch)
+
+
+@pytest.mark.parametrize("B,V", [(3, 4096), (2, 5121), (40, 8191), (3, 20000), (5, 65600), (20, 50257), (2, 262144), (1, 720896)])
+def test_whole_rows_logprobs_against_fp64(dev, lib, B, V):
+    """Rows of every cluster size and both block sizes, on and off 16-byte boundaries, with logits of minus infinity."""
+    rng = np.random.default_rng(V)
+    x = (3 * rng.standard_normal((B, V + 1))).astype(np.float32)
+    x[0, 5:V // 2] = -np.inf
+    block = torch.from_numpy(x).to(dev)
+    for logits in (block[:, :V], block[:, 1:]):
+        got = S.logprobs_block(logits)
+        ref = torch.log_softmax(logits.double(), 1)
+        assert torch.equal(torch.isneginf(got), torch.isneginf(ref))
+        keep = ~torch.isneginf(ref)
+        # the maximum and the logarithm's rounding, each half an ulp of numbers below 32
+        assert (got.double() - ref)[keep].abs().max().item() <= 2 ** -18
