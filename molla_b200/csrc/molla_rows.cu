@@ -423,14 +423,9 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_stats_kernel(const __gri
     for (int j = 1; j < 32; j++) m = fmaxf(m, x[j]);
     const float tmax = warp_max_key(m);
     const unsigned int who = __ballot_sync(0xffffffffu, m == tmax);
-    const int first = who ? __ffs((int)who) - 1 : 0;
-    int at = 0;
-    if (lane == first) {
-#pragma unroll
-        for (int j = 31; j >= 0; j--)
-            if (x[j] == tmax) at = j;
-    }
-    at = __shfl_sync(0xffffffffu, at, first) + first * 32 + tile * TILE;
+    const int first = who ? __ffs((int)who) - 1 : 0;   // the first line that holds the maximum, and where in it (a lane looks at a logit)
+    const unsigned int where = __ballot_sync(0xffffffffu, S->x[((threadIdx.x & ~31) + first) * PITCH + lane] == tmax);
+    const int at = (where ? __ffs((int)where) - 1 : 0) + first * 32 + tile * TILE;
     const bool sampled = !c.greedy && c.n_lim > 1;
     int eq = 0;
     float sum = 0.0f;
@@ -1023,9 +1018,10 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tile = span * (SPAN / TILE) + warp;
     const size_t gt = (size_t)rr * A.ntile + min(tile, A.ntile - 1);
     const TilePlan tp = A.tp[gt];
-    const bool hot = tile < A.ntile && A.ts[gt].tmax >= tp.thr;
+    const float tmax = A.ts[gt].tmax;
+    if (head->plan.kind == PLAN_DONE) return;
+    const bool hot = tile < A.ntile && tmax >= tp.thr;
     const RowPlan pl = head->plan;
-    if (pl.kind == PLAN_DONE) return;
     auto store_cold = [&]() {
         if (pl.flags & F_LIST) A.kmask[gt * 32 + lane] = 0u;
         if (lane == 0) { TileOut o; o.ioff = 0u; o.cnt = 0; o.nitem = 0; A.to(rr)[tile] = o; }
@@ -1160,7 +1156,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
 constexpr int H_ITEMS = 1024;              // items of a row
-constexpr int H_CARE = 64, H_REC = 704;    // careful chunks whose values are at hand, and all of them
+constexpr int H_CARE = 64, H_REC = 512;    // careful chunks whose values are at hand, and all of them
 // What a queued row has: nothing; its denominator; its head too (tile_walk prepares the walk past it);
 // its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
 enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3, ST_DONE = 4 };
@@ -1179,14 +1175,18 @@ struct __align__(16) WalkShared {
 struct __align__(16) HeadShared {
     union {
         WalkShared w;
-        unsigned int sbin[NBINS];
-        struct { unsigned long long keys[HEADC]; float lg[HEADC], tt[HEADC]; } typ;
+        struct {   // once the sum is known
+            union {
+                unsigned int sbin[NBINS];
+                struct { unsigned long long keys[HEADC]; float lg[HEADC], tt[HEADC]; } typ;
+            };
+            union {
+                unsigned long long tmp[HEADCAP];
+                struct { float pc[HEADCAP]; float pre[HEADCAP]; } p;
+            };
+        };
     };
     unsigned long long cand[HEADCAP];
-    union {
-        unsigned long long tmp[HEADCAP];
-        struct { float pc[HEADCAP]; float pre[HEADCAP]; } p;
-    };
     unsigned int ws[HW + 1], ws2[HW + 1];
     float Z; int ok, cut, n_ge; unsigned int tie;
     float ent;
@@ -1635,7 +1635,7 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
     }
 }
 
-__global__ void __launch_bounds__(HT, 3) row_head_kernel(const __grid_constant__ RowsArgs R) {
+__global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__ RowsArgs R) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HeadShared *S = reinterpret_cast<HeadShared *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rr = blockIdx.x, r = R.r0 + rr;
