@@ -1884,8 +1884,9 @@ bool molla_cluster_better(int V, int B, int call_B) {
 }
 
 // Whether the clusters of all B rows fit the device at the same time. Of those of eight blocks 15 or 16 do, depending
-// on which of its SMs a device has: 16 rows of 262144 in two rounds took 133 to 140 us with mixed settings, 95 with a
-// top-k and 141 with nothing sorted, where the tile kernels take 115, 61 and 93.
+// on which of its SMs a device has. Where it is 15, 16 rows of 262144 take two rounds of clusters (clusters / tiles, us): a
+// top-k of 40 95 / 66, a nucleus 182 / 132, nothing sorted 155 / 98, a top-k of 1024 152 / 78, greedy 25 / 25; mixed
+// with a softcap, of which the tile kernels do every logit twice, 114 / 127.
 bool molla_cluster_resident(int V, int B, int call_B) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;

@@ -1755,18 +1755,20 @@ int launch_rows(const BatchArgs &args_in, void *d_workspace, cudaStream_t st, in
 // through the host form (tiles / clusters, us): 200 rows of 20000 in two pieces, mixed settings 445 / 412, a nucleus
 // 437 / 423; 400 rows of 20000 in four, mixed 755 / 708, a nucleus 748 / 713, top-k 40 722 / 719; with clusters of two,
 // 100 rows of 60000, nothing sorted 559 / 577; with a top-k of 1024, 200 rows of 38000 798 / 1073.
-bool takes_clusters(const BatchArgs &a, bool piece) {
+// `tiles`: the workspace has room for the tile kernels too (that of pick_rows has not where molla_cluster_better holds).
+bool takes_clusters(const BatchArgs &a, bool piece, bool tiles) {
     const int call = a.layout_B > 0 ? a.layout_B : a.B;
     if (MOLLA_KNOB(a, 32)) return false;
     if (MOLLA_KNOB(a, 64)) return molla_cluster_better(a.V, 1, call);
+    if (tiles && !molla_cluster_resident(a.V, a.B, call)) return false;
     return molla_cluster_better(a.V, call, call) || (piece && molla_cluster_is_block(a.V) && molla_cluster_better(a.V, a.B, call));
 }
 
 // The ordinary entry points' launch.
-int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool piece = false) {
+int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool piece = false, bool tiles = true) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
-    const bool clusters = takes_clusters(a, piece);
+    const bool clusters = takes_clusters(a, piece, tiles);
 #ifdef MOLLA_SAMPLE_TESTING
     g_launched[clusters ? 0 : 1]++;
 #endif
@@ -2405,7 +2407,7 @@ int32_t molla_sample_pick_rows(const float *d_logits, int64_t row_stride, int32_
     const size_t behind = al256(L.tokens - L.f[0]);
     unsigned char *pin = lane && lane->pin && lane->pin_bytes >= behind + (size_t)B * 8 ? lane->pin + behind : nullptr;
     if (pin) { a.tokens = (int *)pin; a.row_status = (unsigned int *)(pin + (size_t)B * 4); }
-    rc = launch_sampling(a, w, st);
+    rc = launch_sampling(a, w, st, false, false);
     if (rc != MOLLA_OK) { cudaStreamSynchronize(st); return rc; }  // (the pinned memory is still being read)
     if (!pin) {
         e = cudaMemcpyAsync(tokens, w + L.tokens, (size_t)B * 4, cudaMemcpyDeviceToHost, st);

@@ -157,3 +157,23 @@ def test_both_kinds_report_rows_that_jump_alike(dev, lib, V):
     assert np.array_equal(a["row_status"] & ~slow, b["row_status"] & ~slow)
     # (one row in some thousands has a sum so near a power of two that the rounding of the estimate decides)
     assert ((a["row_status"] ^ b["row_status"]) != 0).sum() <= 1 and np.any(b["row_status"] & slow)
+
+
+@pytest.mark.parametrize("B", [14, 15, 16, 17])
+def test_rows_around_what_is_resident_at_once(dev, lib, B):
+    """Clusters of eight blocks: 15 or 16 of them fit a device, the next row sends the batch to the tile kernels. The
+    library's choice and either kind for all rows: the same tokens, sums and status words."""
+    V = 262144
+    w = _kinds(W.config3(seed=B, B=B, V=V, H=16), B, V)
+    got = []
+    for knob in (0, *ROUTES.values()):
+        with capi.testing_library() as T:
+            T.molla_sample_debug_knobs(knob)
+            try:
+                got.append(run_gpu(w, dev))
+            finally:
+                T.molla_sample_debug_knobs(0)
+    for other in got[1:]:
+        for key in ("tokens", "row_status"):
+            assert np.array_equal(got[0][key], other[key]), key
+        assert np.array_equal(got[0]["diag"][:, :3].view(np.uint32), other["diag"][:, :3].view(np.uint32))
