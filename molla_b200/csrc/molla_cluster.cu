@@ -36,8 +36,8 @@ constexpr int CL_MAX_G = 8;                  // thread blocks per cluster at mos
 constexpr int CL_LMAX = 75;                  // logits per thread at most (odd: conflict-free strides)
 constexpr int CL_CAPF = NT * CL_LMAX;        // logits per thread block at most: 38400 (150 KB)
 constexpr int CL_PIECE = 4096;               // floats per bulk copy
-constexpr int CL_HEADC = 2048;                // candidates of the sorted head at most (the buffers of a gathered bin hold as many)
-constexpr int CL_HEAD_NEED = 1026;            // the sorted head covers top-k + 1 up to this many: a top-k up to 1025 never walks
+constexpr int CL_HEADC = HEADCAP;             // candidates of the sorted head at most (the buffers of a gathered bin hold as many)
+constexpr int CL_HEAD_NEED = HEAD_MOST;
 constexpr int TIE_CAP = 64;                   // rounding ties a walk resolves by parity; more send it the slow way
 constexpr int TBINS = NT;                    // bins of the threads' maxima by distance below the row's maximum
 constexpr float TRES = (float)(NT / 32);     // bins per unit of logit: the bins cover 32 units
@@ -1327,7 +1327,6 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     long long need = open_row ? (long long)HEAD_NEED : n_lim + 1;
     if (need > CL_HEAD_NEED) need = CL_HEAD_NEED;
     if (need > a.V) need = a.V;
-    const bool p3row = !pure && (open_row ? (n_lim + 1 > HEAD_NEED) : (n_lim + 1 > CL_HEAD_NEED));
 
     // ---- 3. the bound relative to the row's maximum, and the head's threshold: a value that at
     // least `need` of the threads' maxima reach bounds the need-th largest element from below.
@@ -1599,74 +1598,30 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     unsigned int tau_head = 0xFFFFFFFFu;
     if (head_overflow) c.status |= MOLLA_ROW_SLOW_PATH;  // no head: the descending walk takes everything from the top
     if (leader) {
-        sort_cands(c, nc);
-            for (int i = c.tid; i < nc; i += NT) {
-            const float p = A->pc[i];
-            const bool eq = (i > 0 && A->pc[i - 1] == p) || (i + 1 < nc && A->pc[i + 1] == p);
-            A->hidx[i] = (unsigned int)key_idx(A->cand[i]) | (eq ? 0x80000000u : 0u);
-        }
-        __syncthreads();
+        // (sorted through the tables' space and, where there are many, that of pc and pre)
+        static_assert(CL_HEADC <= NC && sizeof(A->u) >= NBINS * sizeof(unsigned int) &&
+                      offsetof(AuxC, pre) == offsetof(AuxC, pc) + sizeof(A->pc) && sizeof(A->pc) + sizeof(A->pre) >= CL_HEADC * sizeof(unsigned long long), "room for the sort");
+        sort_keys<NT, 256>(nc, A->cand, reinterpret_cast<unsigned long long *>(A->pc), A->pc, A->u.h.hq, reinterpret_cast<unsigned int *>(A->wsi), reinterpret_cast<unsigned int *>(A->wsf));
 #ifdef MOLLA_SAMPLE_TESTING
         if (a.topk_out) {
             for (int i = c.tid; i < a.topk_cap; i += NT)
-                a.topk_out[(long long)r * a.topk_cap + i] =
-                    (i < nc && (long long)i < n_use) ? (int)(A->hidx[i] & 0x7fffffffu) : -1;
+                a.topk_out[(long long)r * a.topk_cap + i] = (i < nc && (long long)i < n_use) ? key_idx(A->cand[i]) : -1;
         }
 #endif
-        if (c.tid == 0) {
-            float s = 0.0f;
-            int cut = -1, tie = 0;
-            bool by_mass = false;
-            // the prefix sums of the sorted head (sample.mojo:497-506), eight loads ahead of the
-            // additions; at most n_use elements are added
-            const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
-            int i = 0;
-            while (i < lim && cut < 0) {
-                float v[8];
-                const int m = min(8, lim - i);
-#pragma unroll
-                for (int q = 0; q < 8; q++) v[q] = (q < m) ? A->pc[i + q] : 0.0f;
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    if (q < m && cut < 0) {
-                        s = __fadd_rn(s, v[q]);
-                        A->pre[i + q] = s;
-                        if (topp_on && s >= P) { cut = i + q + 1; by_mass = true; }
-                    }
-                }
-                i += m;
+        if (c.warp == 0) {
+            const HeadEnd e = head_end(HeadRule{n_lim, P, open_row, topp_on, typ_on}, a.V, A->pc, A->pre, nc, nc, n_use, false, head_overflow, u01);
+            if (c.lane == 0) {
+                A->b_s = e.s; A->b_pos = e.pos; A->b_event = EV_NONE; A->b_idx = -1; A->b_p = 0.0f; A->b_aux = (int)e.tie;
+                if (typ_on) A->ncand = e.cut;  // the typical-p filter takes over from here
+                if (e.at >= 0) { A->b_event = EV_DRAW; A->b_idx = key_idx(A->cand[e.at]); A->b_p = A->pc[e.at]; A->b_sum = e.sum; A->b_target = e.target; }
             }
-            const long long pos = (cut >= 0) ? (long long)cut : (long long)lim;
-            if (by_mass) {
-                if (cut < nc && (long long)cut < n_use && A->pc[cut] == A->pc[cut - 1]) tie |= MOLLA_ROW_TOPP_TIE;
-            } else if (lim > 0 && (long long)lim >= n_use) {
-                cut = lim;  // the count limit
+        } else {   // what the walks behind the head ask of it
+            for (int i = c.tid - 32; i < nc; i += NT - 32) {
+                const float p = A->pc[i];
+                const bool eq = (i > 0 && A->pc[i - 1] == p) || (i + 1 < nc && A->pc[i + 1] == p);
+                A->hidx[i] = (unsigned int)key_idx(A->cand[i]) | (eq ? 0x80000000u : 0u);
             }
-            if (cut < 0 && !p3row && !head_overflow) cut = nc;  // everything that can matter is in the head
-            if (n_use < (long long)a.V && (long long)nc > n_use && A->pc[n_use] == A->pc[n_use - 1])
-                tie |= MOLLA_ROW_TOPK_TIE;
-            A->b_s = s; A->b_pos = pos; A->b_event = EV_NONE; A->b_idx = -1; A->b_p = 0.0f;
-            if (typ_on) {
-                A->ncand = cut;  // the typical-p filter takes over from here
-            } else if (cut > 0) {
-                const float sum = A->pre[cut - 1];
-                const float target = __fmul_rn(u01, sum);
-                int at = cut - 1;
-                for (int i0 = 0; i0 < cut && at == cut - 1; i0 += 8) {
-                    float v[8];
-#pragma unroll
-                    for (int q = 0; q < 8; q++) v[q] = (i0 + q < cut) ? A->pre[i0 + q] : 0.0f;
-#pragma unroll
-                    for (int q = 7; q >= 0; q--)
-                        if (i0 + q < cut && target < v[q]) at = i0 + q;  // the first one wins
-                }
-                A->b_event = EV_DRAW; A->b_idx = (int)(A->hidx[at] & 0x7fffffffu); A->b_p = A->pc[at];
-                if ((at > 0 && A->pc[at - 1] == A->pc[at]) || (at + 1 < cut && A->pc[at + 1] == A->pc[at]))
-                    tie |= MOLLA_ROW_CHOSEN_TIE;
-                A->b_sum = sum; A->b_target = target;
-            }
-            A->b_aux = tie;
-                }
+        }
         __syncthreads();
         c.status |= (unsigned int)A->b_aux;
         const float head_s = A->b_s;

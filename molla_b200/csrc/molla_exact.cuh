@@ -72,7 +72,9 @@ constexpr int BIN_SHIFT2 = BIN_SHIFT > NBINS_LOG2 ? BIN_SHIFT - NBINS_LOG2 : 0; 
 constexpr int BPT = NBINS / NT;      // bins per thread in the bin search
 constexpr int NC = MOLLA_NC;         // candidate-list capacity (gathered bins)
 constexpr int HEADC = 1024;          // head-list capacity
-constexpr int HEAD_NEED = 128;       // the sorted head covers top-k + 1 up to this many
+constexpr int HEAD_NEED = 128;       // the sorted head covers top-k + 1 up to this many, where a nucleus alone ends the row;
+constexpr int HEAD_MOST = 1026;      // up to this many where a top-k does: up to 1025 it never walks
+constexpr int HEADCAP = 2048;        // candidates of such a head at most
 constexpr int HSLOTS = 2048;         // hash slots for penalised / biased tokens
 constexpr int PATCH_MAX = 1024;      // window + bias entries per row
 constexpr short SUS = -32768;        // chunk that must be replayed sequentially
@@ -585,6 +587,173 @@ __device__ void sort_cands(CX &c, int n) {
     }
     for (int i = c.tid; i < n; i += NT) A->pc[i] = key_val(A->cand[i]);
     __syncthreads();
+}
+
+// exclusive scan over N threads
+template <int N>
+__device__ __forceinline__ unsigned int head_scan(unsigned int v, unsigned int *ws, unsigned int *total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned int inc = warp_incl_scan(v, lane);
+    __syncthreads();
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    unsigned int b = 0u, t = 0u;
+#pragma unroll
+    for (int w = 0; w < N / 32; w++) {
+        if (w == warp) b = t;
+        t += ws[w];
+    }
+    *total = t;
+    return b + inc - v;
+}
+
+// A key's value in units of 2^-60, as bits: subnormal values spread over their binades like all others (in one
+// bin, the 600 subnormals that a short row of a low temperature can keep took 100 us to be counted).
+__device__ __forceinline__ unsigned int spread_bits(unsigned long long key) { return __float_as_uint(__fmul_rn(key_val(key), 1152921504606846976.0f)); }
+
+// Sorts cand[0..n) (descending value, ascending id) with N threads and leaves the values in pc, padded with zeros
+// to a multiple of eight; tmp may lie over pc. Up to FEW keys: every key counts the keys above it. More go through
+// bins of value first (a few keys each: about four to a bin at n = 1400) and count within their bin: 1.4 us for
+// 1400 keys, where a sorting network over the block took 17 us. Ends with a barrier.
+template <int N, int FEW>
+__device__ __forceinline__ void sort_keys(int n, unsigned long long *cand, unsigned long long *tmp, float *pc, unsigned int *sbin, unsigned int *ws, unsigned int *ws2) {
+    static_assert(FEW <= N && HEADCAP % 16 == 0, "a key per thread, sixteen at a time");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int KPT = HEADCAP / N, PER = NBINS / N;
+    if (n <= FEW) {
+        if (tid < 16 && n + tid < HEADCAP) cand[n + tid] = 0ull;
+        __syncthreads();
+        const unsigned long long mine = tid < n ? cand[tid] : 0ull;
+        int rank = 0;
+        if (warp * 32 < n) {
+#pragma unroll 1
+            for (int j = 0; j < n; j += 16) {   // (eight loads at a time)
+                ulonglong2 o[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) o[u] = *reinterpret_cast<const ulonglong2 *>(cand + j + 2 * u);
+#pragma unroll
+                for (int u = 0; u < 8; u++) rank += (o[u].x > mine ? 1 : 0) + (o[u].y > mine ? 1 : 0);
+            }
+        }
+        __syncthreads();
+        if (tid < n) { cand[rank] = mine; pc[rank] = key_val(mine); }
+    } else {
+        unsigned long long k[KPT];
+        unsigned int lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+        for (int u = 0; u < KPT; u++) {
+            const int i = tid + u * N;
+            k[u] = i < n ? cand[i] : 0ull;
+            if (i < n) { const unsigned int b = spread_bits(k[u]); lo = min(lo, b); hi = max(hi, b); }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) { ws[warp] = lo; ws2[warp] = hi; }
+#pragma unroll
+        for (int i = 0; i < PER; i++) sbin[tid + i * N] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < N / 32; w++) { lo = min(lo, ws[w]); hi = max(hi, ws2[w]); }
+        const int shift = max(0, 32 - __clz((int)(hi - lo)) - NBINS_LOG2);   // (hi - lo) >> shift is below NBINS
+        unsigned int slot[KPT];
+        auto bin_of = [&](unsigned long long key) { return NBINS - 1 - ((spread_bits(key) - lo) >> shift); };   // descending
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * N < n) slot[u] = atomicAdd(&sbin[bin_of(k[u])], 1u);
+        __syncthreads();
+        unsigned int cnt[PER], sum = 0u, tot;
+#pragma unroll
+        for (int i = 0; i < PER; i++) { cnt[i] = sbin[PER * tid + i]; sum += cnt[i]; }
+        unsigned int at = head_scan<N>(sum, ws, &tot);
+#pragma unroll
+        for (int i = 0; i < PER; i++) { sbin[PER * tid + i] = at | (cnt[i] << 16); at += cnt[i]; }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * N < n) tmp[(sbin[bin_of(k[u])] & 0xffffu) + slot[u]] = k[u];
+        __syncthreads();
+        unsigned int rank[KPT];
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * N < n) {
+                const unsigned int b = sbin[bin_of(k[u])], b0 = b & 0xffffu, m = b >> 16;
+                rank[u] = b0;
+#pragma unroll 1
+                for (unsigned int j = 0; j < m; j++) rank[u] += tmp[b0 + j] > k[u] ? 1u : 0u;
+            }
+        __syncthreads();   // the values may take the space of the keys being read
+#pragma unroll
+        for (int u = 0; u < KPT; u++)
+            if (tid + u * N < n) { cand[rank[u]] = k[u]; pc[rank[u]] = key_val(k[u]); }
+    }
+    if (tid < 8 && n + tid < HEADCAP) pc[n + tid] = 0.0f;
+    __syncthreads();
+}
+
+// The sorted head's pc[0..nc) by one warp: its prefix sums (sample.mojo:497-506) into pre, eight at a time, at most
+// n_use elements of them; where top-p or the count ends the set (cut, or -1: behind the head); the draw from it
+// (:580-590, unless typical-p takes over); the marks of equal probabilities at either end.
+// From nwalk on, and everywhere with `narrow`, they are those of a walk past the head; with `overflow` there is no head.
+struct HeadEnd { float s; int pos, cut, at; float sum, target; unsigned int tie; };   // s, pos: the sum and the count so far; at: the drawn one, or -1
+struct HeadRule { long long n_lim; float P; bool open_row, topp_on, typ_on; };
+__device__ __forceinline__ HeadEnd head_end(const HeadRule &g, int V, const float *pc, float *pre, int nc, int nwalk, long long n_use, bool narrow, bool overflow, float u01) {
+    const int lane = threadIdx.x & 31;
+    const bool p3row = g.n_lim + 1 > (g.open_row ? HEAD_NEED : HEAD_MOST), topp_on = g.topp_on;
+    const float P = g.P;
+    HeadEnd e;
+    e.at = -1; e.sum = 0.0f; e.target = 0.0f; e.tie = 0u;
+    float s = 0.0f;
+    int cut = -1;
+    bool by_mass = false;
+    const int lim = (int)((long long)nc < n_use ? (long long)nc : n_use);
+    const float4 *p4 = reinterpret_cast<const float4 *>(pc);
+    float4 x = p4[0], y = p4[1];
+#pragma unroll 1
+    for (int i = 0; i < lim && cut < 0; i += 8) {
+        const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        if (i + 8 < lim) { x = p4[(i >> 2) + 2]; y = p4[(i >> 2) + 3]; }
+        float t[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) { s = __fadd_rn(s, i + q < lim ? v[q] : 0.0f); t[q] = s; }
+        if (lane == 0) {
+            float4 *o4 = reinterpret_cast<float4 *>(pre + i);
+            o4[0] = make_float4(t[0], t[1], t[2], t[3]);
+            o4[1] = make_float4(t[4], t[5], t[6], t[7]);
+        }
+        if (topp_on && s >= P) {
+#pragma unroll
+            for (int q = 7; q >= 0; q--)
+                if (t[q] >= P) { cut = i + q + 1; s = t[q]; }   // the first one wins
+            by_mass = true;
+        }
+    }
+    __syncwarp();
+    e.s = s;
+    e.pos = cut >= 0 ? cut : lim;
+    auto equal_next_to = [&](int i) { return (i > 0 && pc[i - 1] == pc[i]) || (i + 1 < nc && pc[i + 1] == pc[i]); };
+    const bool walked = narrow || cut > nwalk || (cut < 0 && (long long)lim >= n_use && lim > nwalk);
+    if (by_mass) {
+        if (walked ? equal_next_to(cut - 1) : (cut < nc && (long long)cut < n_use && pc[cut] == pc[cut - 1])) e.tie |= MOLLA_ROW_TOPP_TIE;
+    } else if (lim > 0 && (long long)lim >= n_use) {
+        cut = lim;  // the count limit
+        if (walked && equal_next_to(cut - 1)) e.tie |= MOLLA_ROW_TOPK_TIE;
+    }
+    if (cut < 0 && !p3row && !overflow) cut = nc;  // everything that can matter is in the head
+    if (!narrow && n_use < (long long)V && (long long)nwalk > n_use && pc[n_use] == pc[n_use - 1]) e.tie |= MOLLA_ROW_TOPK_TIE;
+    if (!g.typ_on && cut > 0) {
+        e.sum = pre[cut - 1];
+        e.target = __fmul_rn(u01, e.sum);
+        // the first prefix sum above the target (they never fall), or the last one kept
+        int at = 0, hi = cut - 1;
+        while (at < hi) {
+            const int mid = (at + hi) >> 1;
+            if (e.target < pre[mid]) hi = mid; else at = mid + 1;
+        }
+        if (walked ? equal_next_to(at) : ((at > 0 && pc[at - 1] == pc[at]) || (at + 1 < cut && pc[at + 1] == pc[at]))) e.tie |= MOLLA_ROW_CHOSEN_TIE;
+        e.at = at;
+    }
+    e.cut = cut;
+    return e;
 }
 
 // Adds the sorted candidates pc[0..nb) to the running sum `s0` in order, exactly as the
