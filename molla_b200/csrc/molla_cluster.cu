@@ -223,11 +223,11 @@ __device__ __noinline__ ChunksSum add_chunks(const float *vals, int nloc, int L,
 // Where the values of chunks to be added one by one wait for the leader's walk, `pitch` floats each: over pc, pre and
 // hidx, half of the places for the leader's own range, in which most binades are crossed.
 __device__ __forceinline__ int care_pitch(int L) { return (L + 11) / 12 * 12; }   // (whole steps of add_place)
-__device__ __forceinline__ void care_places(int L, int rank, int &first, int &n) {
+__device__ __forceinline__ void care_places(int L, int G, int rank, int &first, int &n) {
     static_assert(offsetof(AuxC, pre) == offsetof(AuxC, pc) + sizeof(AuxC::pc) && offsetof(AuxC, hidx) == offsetof(AuxC, pre) + sizeof(AuxC::pre), "one area");
     static_assert(offsetof(AuxC, pc) % 16 == 0, "read four at a time");
     const int all = min(255, (int)((sizeof(AuxC::pc) + sizeof(AuxC::pre) + sizeof(AuxC::hidx)) / sizeof(float)) / care_pitch(L));
-    const int own = all / 2, others = (all - own) / (CL_MAX_G - 1);
+    const int own = G == 1 ? all : all / 2, others = G == 1 ? 0 : (all - own) / (G - 1);
     first = rank == 0 ? 0 : own + (rank - 1) * others;
     n = rank == 0 ? own : others;
 }
@@ -258,7 +258,7 @@ __device__ __forceinline__ float add_place(const AuxC *A, int place, int pitch4,
 // these (ten or twenty: mostly the chunks in which the sum leaves a binade) are gone through one by one. (Every
 // instruction of that loop is one of a lone warp's, eight cycles or so: with the plain ones in it, it took 14 thousand.)
 // Returns false, and nothing else, where something does not hold.
-__device__ __noinline__ bool walk_fast(CtxC &c, const ClGeo &g, float &sum) {
+__device__ __noinline__ bool walk_fast(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, float &sum) {
     AuxC *A = c.A;
     IN_SHARED(A);
     const int lane = c.lane, pitch4 = care_pitch(g.L) / 4;
@@ -318,8 +318,20 @@ __device__ __noinline__ bool walk_fast(CtxC &c, const ClGeo &g, float &sum) {
         if (((r.meta >> 25) & 1u) && d <= both && (td >> 23) == e) sb = td;
         else {
             const int place = (int)((r.meta >> 17) & 0xffu);
-            if (place == 255) return false;
-            sb = __float_as_uint(add_place(A, place, pitch4, __uint_as_float(to)));
+            if (place != 255) sb = __float_as_uint(add_place(A, place, pitch4, __uint_as_float(to)));
+            else {   // several chunks, or one that found no place: out of its block's memory
+                const int o = A->u.p1.org[q], h = o >> 9, nloc = max(0, min(Vc, V - h * Vc));
+                const Stretch it = A->u.p1.recs[h][o & 511];
+                const float *vals = reinterpret_cast<const float *>(h == 0 ? bits : cl.map_shared_rank(const_cast<unsigned int *>(bits), h));
+                if (it.chunks() > 1) {
+                    const ChunksSum s = add_chunks(vals, nloc, g.L, it.first(), it.chunks(), to, it.guess(), it.guess_two());
+                    if (s.slow) return false;
+                    sb = s.sb;
+                } else {
+                    const int i0 = min(nloc, it.first() * g.L);
+                    sb = add_chunk(vals + i0, min(nloc, i0 + g.L) - i0, to);
+                }
+            }
             // (where a binade was guessed: the guess held?)
             if (jb != 0u && !(d <= both && (sb >> 23) <= jb + both)) return false;
         }
@@ -440,7 +452,7 @@ __device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, 
     int at = 0;
     for (int w = 0; w < c.warp; w++) at += A->wsi[w];
     int place0, places;
-    care_places(g.L, g.rank, place0, places);
+    care_places(g.L, g.G, g.rank, place0, places);
     const int care0 = at >> 16;
     at &= 0xffff;
     if (c.tid == NT - 1) A->nitem = at + n;
@@ -509,7 +521,7 @@ __device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, 
     if (g.rank == 0 && c.warp == 0) {
         Walked w{0u, false, -1, 0, 0};
         float sum;
-        if (walk_fast(c, g, sum)) w.sb = __float_as_uint(sum);
+        if (walk_fast(cl, c, g, Vc, V, bits, sum)) w.sb = __float_as_uint(sum);
         else w = walk_stretches(cl, c, g, Vc, V, bits, 0, 0, 0u, false, 0.0f);
         if (lane < g.G) { AuxC *ox = cl.map_shared_rank(A, lane); ox->ch_s = __uint_as_float(w.sb); ox->ch_slow = w.slow ? 1 : 0; }
     }
