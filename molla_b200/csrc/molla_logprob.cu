@@ -32,6 +32,7 @@ struct LpArgs {
     const int *rows; int n_logit_rows; float softcap;
     float *out;                   // whole rows' logprobs, or nullptr
     float *stats;                 // [rows][ntile] four floats
+    bool early;                   // see lp_tiles
     int ntile;
 };
 
@@ -82,9 +83,7 @@ __device__ __forceinline__ void tile_stat(const float (&x)[34], float &m, double
     sum = s0;
 }
 
-__global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+__device__ __forceinline__ void lp_tile(const LpArgs &a) {
     const int lane = threadIdx.x & 31, per = (a.ntile + 7) / 8;
     const int r = blockIdx.x / per, t = (blockIdx.x - r * per) * 8 + (threadIdx.x >> 5);
     if (t >= a.ntile) return;
@@ -106,6 +105,16 @@ __global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a
         const unsigned long long b = (unsigned long long)__double_as_longlong(s0);
         o[0] = m; o[1] = __uint_as_float((unsigned int)b); o[2] = __uint_as_float((unsigned int)(b >> 32));
     }
+}
+
+// `early`: this kernel may run beside the one before it, which nothing here depends on (the logits are older, and it does
+// not touch a.stats). The kernel behind this one needs that one's tokens: so it ends only when that one has, which
+// one block waits for.
+__global__ void __launch_bounds__(LT_) lp_tiles(const __grid_constant__ LpArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!a.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    lp_tile(a);
+    if (a.early && blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(LT_) lp_rows(const __grid_constant__ LpArgs a) {
@@ -342,7 +351,7 @@ bool molla_logprob_tiled(int V, int top_n) { return V >= 4096 && tiles_of(V) >= 
 size_t molla_logprob_workspace_bytes(int B, int V) { return (size_t)B * (size_t)tiles_of(V) * 4 * sizeof(float); }
 
 cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int B, int V, const int *tokens, int top_n, float *chosen,
-                                 int *top_ids, float *top_lps, const int *rows, int n_logit_rows, float softcap, void *workspace,
+                                 int *top_ids, float *top_lps, const int *rows, int n_logit_rows, float softcap, void *workspace, bool early,
                                  float *full_out, cudaStream_t st) {
     LpArgs a = {};
     a.logits = logits; a.row_stride = row_stride; a.B = B; a.V = V;
@@ -365,7 +374,7 @@ cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int 
         }
         return lp_launch(lp_whole, (unsigned int)n, 32u * (unsigned int)((each + rounds - 1) / rounds), (unsigned int)G, st, a);
     }
-    a.stats = (float *)workspace;
+    a.stats = (float *)workspace; a.early = early;
     const unsigned int blocks = (unsigned int)B * (unsigned int)((a.ntile + 7) / 8);
     cudaError_t e = lp_launch(lp_tiles, blocks, LT_, 1, st, a);
     if (e == cudaSuccess) e = lp_launch(lp_rows, (unsigned int)B, LT_, 1, st, a);

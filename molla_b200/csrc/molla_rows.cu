@@ -125,6 +125,7 @@ struct RowsArgs {
     int r0, rows;            // batch rows [r0, r0 + rows) are in flight
     int ntile, nspan;
     int oG, oVc, oL;         // see F_NARROW
+    bool late_next;          // row_tail lets the next kernel begin once it has begun itself, not before
     int need_far, need_topk; // lanes' maxima that reach a far head's edge, without a top-k and with one; 0: rows of this length have none
     TileStat *ts;            // [rows][ntile]
     float *gmax;             // [rows][ntile * 32] the lanes' maxima
@@ -3310,8 +3311,9 @@ __device__ __noinline__ void jump_status(const RowsArgs &R, int rr) {
 }
 
 __global__ void __launch_bounds__(NT, 1) row_tail_kernel(const __grid_constant__ RowsArgs R) {
-    pdl_next();
+    if (!R.late_next) pdl_next();
     pdl_wait();
+    if (R.late_next) pdl_next();   // (everything before this call's kernels is done by now)
     const int n = R.queue[0];
 #pragma unroll 1
     for (int q = blockIdx.x; q < n; q += gridDim.x) {
@@ -3392,7 +3394,7 @@ size_t molla_rows_workspace_bytes(int B, int V) {
     return lay_out(A, nullptr, (int)(B < 1 ? 1 : (B < most ? B : most)), V);
 }
 
-int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, char *err, size_t errlen) {
+int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, char *err, size_t errlen, float **spare) {
     static bool ready[64] = {};
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -3418,7 +3420,10 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
     narrow_layout(a.V, a.layout_B > 0 ? a.layout_B : a.B, sms, A.oG, A.oVc, A.oL);
     const int rows = rows_in_flight(a.B, a.V);
     lay_out(A, (char *)d_workspace, rows, a.V);
+    // (the lanes' maxima are done with when row_tail begins; 128 bytes a tile of the rows in flight)
+    if (spare) *spare = a.B <= 8 * rows ? A.gmax : nullptr;
     for (A.r0 = 0; A.r0 < a.B && e == cudaSuccess; A.r0 += rows) {
+        A.late_next = spare && *spare && A.r0 + rows >= a.B;
         A.rows = a.B - A.r0 < rows ? a.B - A.r0 : rows;
         const unsigned int spans = (unsigned int)A.rows * (unsigned int)A.nspan;
         e = launch(tile_stats_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);

@@ -9,4 +9,6 @@ struct BatchArgs;
 size_t molla_rows_workspace_bytes(int B, int V);
 
 // Enqueues the sampling of `a.B` rows on `st`. Returns MOLLA_OK or a MOLLA_ERR_* code with its message in `err`.
-int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, char *err, size_t errlen);
+// With `spare`, a kernel that is launched next as a programmatic dependent begins when the last of these has begun, and
+// *spare is workspace memory of 16 bytes per 1024 logits of every row that this last one does not use (or nullptr).
+int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, char *err, size_t errlen, float **spare);

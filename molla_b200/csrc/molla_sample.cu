@@ -1765,7 +1765,7 @@ bool takes_clusters(const BatchArgs &a, bool piece, bool tiles) {
 }
 
 // The ordinary entry points' launch.
-int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool piece = false, bool tiles = true) {
+int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool piece = false, bool tiles = true, float **spare = nullptr) {
     if (a.V > MAX_VOCAB) return fail(MOLLA_ERR_VOCAB, "vocabulary too wide%s");
     if (a.mask && a.V > MAX_MASKED_VOCAB) return fail(MOLLA_ERR_VOCAB, "a grammar mask is only done for vocabularies of at most 307200 logits%s");
     const bool clusters = takes_clusters(a, piece, tiles);
@@ -1773,17 +1773,17 @@ int launch_sampling(const BatchArgs &a, void *d_workspace, cudaStream_t st, bool
     g_launched[clusters ? 0 : 1]++;
 #endif
     if (clusters) return molla_cluster_launch(a, st, g_err, sizeof(g_err));
-    return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err));
+    return molla_rows_launch(a, d_workspace, st, g_err, sizeof(g_err), spare);
 }
 
 // The chosen tokens' and the top N's logprobs behind a sampling launch, which is done with the workspace.
 int launch_logprobs(const float *logits, int64_t row_stride, int B, int V, const int *tokens, int top_n, float *chosen, int *top_ids,
-                    float *top_lps, const int *rows, int n_logit_rows, float softcap, void *d_workspace, cudaStream_t st) {
+                    float *top_lps, const int *rows, int n_logit_rows, float softcap, void *d_workspace, cudaStream_t st, float *spare = nullptr) {
     if (!chosen && top_n == 0) return MOLLA_OK;
     cudaError_t e;
     if (molla_logprob_tiled(V, top_n)) {
         e = molla_logprob_launch(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, rows, n_logit_rows, softcap,
-                                 d_workspace, nullptr, st);
+                                 spare ? (void *)spare : d_workspace, spare != nullptr, nullptr, st);
     } else {
         const int sms = sm_count();
         logprob_kernel<<<sms > 0 && B > sms ? sms : B, NT, 0, st>>>(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, nullptr,
@@ -1848,10 +1848,12 @@ int32_t molla_sample_batch_masked(const uint32_t *d_mask, int64_t mask_stride_wo
     a.tokens = d_tokens; a.row_status = d_row_status; a.diag = d_diag;
     a.penalised = nullptr; a.penalised_only = 0;
     MOLLA_SET_TESTING_ARGS(a);
-    int rc = launch_sampling(a, d_workspace, st);
+    // (the logprobs' pass over the tiles runs beside the last of the tile kernels, which few of the SMs work on)
+    float *spare = nullptr;
+    int rc = launch_sampling(a, d_workspace, st, false, true, (d_chosen_logprob || top_n > 0) && molla_logprob_tiled(V, top_n) ? &spare : nullptr);
     if (rc != MOLLA_OK) return rc;
     return launch_logprobs(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob, d_top_ids, d_top_logprobs, nullptr, 0, 0.0f,
-                           d_workspace, st);
+                           d_workspace, st, spare);
 }
 
 int32_t molla_sample_batch(const float *d_logits, int64_t row_stride, int32_t B, int32_t V,
@@ -1919,10 +1921,12 @@ int32_t molla_sample_decode_step(const float *d_logits, int64_t row_stride, int3
         cudaError_t e0 = cudaMemsetAsync(d_stopped, 0, (size_t)B, st);
         if (e0 != cudaSuccess) return fail(MOLLA_ERR_CUDA, "clearing the stop flags failed: %s", cudaGetErrorString(e0));
     }
-    int rc = launch_sampling(a, d_workspace, st);
+    // (the logprobs' pass over the tiles runs beside the last of the tile kernels, which few of the SMs work on)
+    float *spare = nullptr;
+    int rc = launch_sampling(a, d_workspace, st, false, true, (d_chosen_logprob || top_n > 0) && molla_logprob_tiled(V, top_n) ? &spare : nullptr);
     if (rc != MOLLA_OK) return rc;
     return launch_logprobs(d_logits, row_stride, B, V, d_tokens, top_n, d_chosen_logprob, d_top_ids, d_top_logprobs, d_rows, n_logit_rows, final_softcap,
-                           d_workspace, st);
+                           d_workspace, st, spare);
 }
 
 int32_t molla_sample_batch_noalloc(const float *d_logits, int64_t row_stride, int32_t B, int32_t V,
@@ -2448,7 +2452,7 @@ int32_t molla_sample_logprobs(const float *d_logits, int64_t row_stride, int32_t
     if (B == 0) return MOLLA_OK;
     if (molla_logprob_tiled(V, 0)) {
         const cudaError_t e = molla_logprob_launch(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0.0f,
-                                                   nullptr, d_out, (cudaStream_t)stream);
+                                                   nullptr, false, d_out, (cudaStream_t)stream);
         return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
     }
     const int sms = sm_count();
