@@ -1853,13 +1853,15 @@ bool molla_cluster_better(int V, int B, int call_B) {
 // Whether the clusters of all B rows fit the device at the same time. Of those of eight blocks 15 or 16 do, depending
 // on which of its SMs a device has. Where it is 15, 16 rows of 262144 take two rounds of clusters (clusters / tiles, us): a
 // top-k of 40 95 / 66, a nucleus 182 / 132, nothing sorted 155 / 98, a top-k of 1024 152 / 78, greedy 25 / 25; mixed
-// with a softcap, of which the tile kernels do every logit twice, 114 / 127.
+// with a softcap, of which the tile kernels do every logit twice, 114 / 127. Rows of 131072 and less stay where they are:
+// at 128256 mixed settings take 76 / 95 there, a nucleus 119 / 132, a top-k 83 / 54 and nothing sorted 118 / 83.
+constexpr int TWO_ROUNDS_V = 131072;
 bool molla_cluster_resident(int V, int B, int call_B) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const ClusterShape cs = cluster_shape(V, call_B, sms);
-    return cs.G != 0 && B <= clusters_resident(dev, cs.G);
+    return cs.G != 0 && (V <= TWO_ROUNDS_V || B <= clusters_resident(dev, cs.G));
 }
 
 int molla_cluster_launch(const BatchArgs &args_in, cudaStream_t st, char *err, size_t errlen) {

@@ -21,7 +21,7 @@
 // so any number of rows, from one to thousands, fills the chip, and only the row kernels have serial
 // parts. A row per thread-block cluster, resident in its shared memory, read the block once but left 33 to 16
 // rows in flight on the chip, each as slow as its serial parts: 1024 rows of 262144 took 6316 us where this
-// takes 930 to 1250 (by the longest row's careful chunks), 64 of 151936 with logprobs 300 where this takes 197. Seven launches cost 2 to 3 us each where
+// takes 705 to 750, 64 of 151936 with a nucleus and logprobs 300 where this takes 172. Seven launches cost 2 to 3 us each where
 // nothing else is to be done; they are chained so that a kernel's blocks are in place when the one before
 // ends. The reference's sequential fp32 sums are reproduced bit for bit: see "Items" below.
 #include <cuda_runtime.h>
@@ -384,8 +384,8 @@ __device__ void span_ready(const BatchArgs &a, const RowCfg &c, int r, int c0, f
 }
 
 // =============================================================================
-// Kernel 1: the tiles' maxima and estimated sums. Bound: HBM (4 bytes per logit, once): 156 MB take 44 us
-// (3.6 TB/s), 537 MB 105 us (5.1 TB/s). A warp has its tile in shared memory by asynchronous copies,
+// Kernel 1: the tiles' maxima and estimated sums. Bound: HBM (4 bytes per logit, once): 156 MB take 43 us
+// (3.6 TB/s), 537 MB 98 us (5.5 TB/s). A warp has its tile in shared memory by asynchronous copies,
 // four blocks of 8192 logits an SM in flight; a tile per warp, because then nothing but a warp waits for
 // it, and of 1024 logits, because a lane's 32 are what the items' chunks are made of.
 // =============================================================================
@@ -842,6 +842,13 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
         }
         return n;
     }
+    if (cm == 0u && !__any_sync(0xffffffffu, usable && da.even != da.odd)) {   // one run without a tie
+        const unsigned int k = __reduce_add_sync(0xffffffffu, usable ? da.even : 0u);
+        if (k == 0u) return 0;
+        Item *out = alloc(1, 0);
+        if (lane == 0) out[0] = run_item(k, j0, tile, total, 0, 0);
+        return 1;
+    }
     // the runs between the careful lanes: a run goes with the careful lane behind it, or closes the tile
     const unsigned int lt = (1u << lane) - 1u, cb = cm & lt;
     const int lastc = cb ? 31 - __clz((int)cb) : -1, last = cm ? 31 - __clz((int)cm) : -1;
@@ -874,6 +881,33 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     if (ktail && lane == 0) out[n - 1] = run_item(ktail, tj, tile, total - to, to, n - 1);
     return n;
 }
+
+// Most tiles lie inside one binade and hold no tie: their sum is a number of its units, in any order, added up where
+// the values are made. (Chunks and items for all tiles took half again as many instructions.) One warp; `est` = the
+// estimated sum before the tile.
+struct QuickSum {
+    int j;               // the binade
+    bool usable, bad;
+    float C, half, big;
+    unsigned int k;      // this lane's units; all lanes' once holds() has been true
+    __device__ __forceinline__ QuickSum(float est) {
+        const float lo = est * (1.0f - 1.0f / 1024.0f);
+        j = fexpo(lo);
+        usable = lo > 0.0f && j >= -100;
+        C = __fmul_rn(1.5f, fpow2(usable ? j : 0)); half = fpow2(usable ? j - 24 : -24); big = fpow2(usable ? j - 1 : -1);
+        k = 0u; bad = false;
+    }
+    __device__ __forceinline__ void add(float e) {
+        const float s = __fadd_rn(e, C);
+        k += __float_as_uint(s) - __float_as_uint(C);
+        bad |= (fabsf(__fsub_rn(e, __fsub_rn(s, C))) == half) | (e >= big);
+    }
+    __device__ __forceinline__ bool holds(float est) {
+        if (!usable || __any_sync(0xffffffffu, bad)) return false;
+        k = __reduce_add_sync(0xffffffffu, k);
+        return fexpo((est + (float)k * fpow2(max(j - 23, -126))) * (1.0f + 1.0f / 2048.0f)) == j;
+    }
+};
 
 struct TileEval { int total; unsigned int keep; };
 
@@ -1039,25 +1073,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = min(pl.tau_bits, pl.tau_far);
     unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
-    // Most tiles lie inside one binade and hold no tie: their sum is a number of its units, in any order, added up
-    // on the way. (Chunks and items for all tiles took half again as many instructions.)
-    const float qlo = tp.est * (1.0f - 1.0f / 1024.0f);
-    const int qj = fexpo(qlo);
-    bool quick = qlo > 0.0f && qj >= -100;
-    const float qc = __fmul_rn(1.5f, fpow2(quick ? qj : 0)), qh = fpow2(quick ? qj - 24 : -24), qb = fpow2(quick ? qj - 1 : -1);
-    unsigned int qk = 0u;
-    bool qbad = false;
-    auto add_units = [&](float e) {
-        const float s = __fadd_rn(e, qc);
-        qk += __float_as_uint(s) - __float_as_uint(qc);
-        qbad |= (fabsf(__fsub_rn(e, __fsub_rn(s, qc))) == qh) | (e >= qb);
-    };
-    auto quick_sum = [&]() {   // is the sum that of one binade's units? (qk: all of them)
-        if (!quick || __any_sync(0xffffffffu, qbad)) return false;
-        qk = __reduce_add_sync(0xffffffffu, qk);
-        const float end = tp.est + (float)qk * fpow2(max(qj - 23, -126));
-        return fexpo(end * (1.0f + 1.0f / 2048.0f)) == qj;
-    };
+    QuickSum qs(tp.est);
+    auto add_units = [&](float e) { qs.add(e); };
     int ni = 0, cnt = TILE;
     unsigned int i0 = 0u;
     auto store_out = [&]() {
@@ -1067,20 +1084,20 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
         A.to(rr)[tile] = o;
     };
     auto store_run = [&]() {
-        ni = qk ? 1 : 0;
-        if (lane == 0 && qk) {
+        ni = qs.k ? 1 : 0;
+        if (lane == 0 && qs.k) {
             i0 = (unsigned int)atomicAdd(&head->nitem, 1);
-            A.items(rr)[i0] = run_item(qk, qj, tile, cnt, 0, 0);
+            A.items(rr)[i0] = run_item(qs.k, qs.j, tile, cnt, 0, 0);
         }
     };
     const bool fast = (pl.flags & F_FASTDIV) && tp.thr > -INFINITY;
     const float rT = __fdiv_rn(1.0f, c.T);
-    if (quick && fast && !(pl.flags & F_LIST)) {
+    if (qs.usable && fast && !(pl.flags & F_LIST)) {
         // Nobody asks for this row's list, only for its sum and its candidates, and nearly all that is kept adds
         // few units, whose number a hardware exponential tells unless it is near a half: see near_units. The others
         // are evaluated as they have to be. Per tile 600 instructions, where evaluating all that is kept takes 1300
         // (at a fifth of the logits kept: 1024 rows of 262144 with a top-k of 1024, 450 us).
-        const unsigned int m = near_units(list, lane, c.T, pl.top, qj, tau, qk);
+        const unsigned int m = near_units(list, lane, c.T, pl.top, qs.j, tau, qs.k);
         const int mine = __popc(m), inc = warp_incl_scan(mine, lane), total = __shfl_sync(0xffffffffu, inc, 31);
         if (total <= EXACT_MOST) {
             float *val = reinterpret_cast<float *>(idx + EXACT_MOST);
@@ -1102,7 +1119,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
                 }
             }
             __syncwarp();
-            if (quick_sum()) {
+            if (qs.holds(tp.est)) {
                 put_candidates(A, rr, pl, wanted, [&](int b) { return b * 32 + lane; }, [&](int e) { return __float_as_uint(val[e]); },
                                [&](int e) { return tile * TILE + (int)idx[e]; });
                 store_run();
@@ -1111,7 +1128,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
             }
             __syncwarp();
         }
-        qk = 0u; qbad = false;
+        qs.k = 0u; qs.bad = false;
     }
     unsigned int w0 = 0u, w1 = 0u;   // this lane's candidates among the entries it evaluates
     const TileEval t = tile_eval(list, idx, tp.thr, c.T, rT, pl.top, fast,
@@ -1123,7 +1140,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     put_candidates(A, rr, pl, w0 | (w1 << 16), [&](int b) { return (b & 15) * 64 + (b & 16) * 2 + lane; },
                    [&](int e) { return __float_as_uint(list[skew(e)]); }, [&](int e) { return tile * TILE + (t.total == TILE ? e : (int)idx[e]); });
     bool whole = (pl.flags & F_LIST) != 0;
-    if (quick_sum()) store_run();
+    if (qs.holds(tp.est)) store_run();
     else {
         const TileChunk ch = tile_chunk(list, t.total);
         bool care;
@@ -1149,8 +1166,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // Kernel 4: one small block per sampled row. The items give the softmax denominator, the candidates the
 // sorted head; most rows end here. Rows that go on (nothing sorted, a nucleus past the head, typical-p,
 // anything unusual) are queued for the last kernel. Bound: the latency of one warp's dependent additions
-// and of one round of loads, so the block is small and three of them share an SM: 11 us for one row, 18 for
-// 64, 32 for 256, 66 for 512 with a top-k of 1024. (Run by the tail's 512 threads, one block an SM, the same
+// and of one round of loads, so the block is small and four of them share an SM: 21 us for
+// 64 rows, 35 for 256, 42 for 512 with a top-k of 1024 (three an SM, two rounds of them: 60). (Run by the tail's 512 threads, one block an SM, the same
 // rows took twice as long.)
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
@@ -1345,7 +1362,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
         if (run && (!low || (td >> 23) != jb)) { fine = false; break; }
         if (run || (kind == K_DUAL && (low || e == jb + 1u) && (td >> 23) == e)) {
             sb = td;
-            if (kind_of(r) != K_STEP && q + 1 < nrec) {
+            if (q + 6 < nrec && kind_of(r) != K_STEP && kind_of(nx) != K_STEP && kind_of(W->rec[q + 6]) != K_STEP) {
                 const uint2 t = dual_stretch(W, nrec, q + 1, sb, kdone);
                 sb = t.x;
                 q += (int)t.y;
@@ -1468,7 +1485,9 @@ __device__ __noinline__ void typical_rows(HeadShared *S, const BatchArgs &a, int
     }
 }
 
-__global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__ RowsArgs R) {
+// (PER_SM blocks an SM: with four its registers spill, which 300 rows of 8000 with a top-k pay for, 54 us where three take 52)
+template <int PER_SM>
+__global__ void __launch_bounds__(HT, PER_SM) row_head_kernel(const __grid_constant__ RowsArgs R) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HeadShared *S = reinterpret_cast<HeadShared *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rr = blockIdx.x, r = R.r0 + rr;
@@ -1598,8 +1617,8 @@ __global__ void __launch_bounds__(HT, 4) row_head_kernel(const __grid_constant__
 // sorted head, the bin tables of the walk in the binades the sum will go through: an element adds
 // rne(p / ulp) units to whatever sum lies in the binade, so one histogram of those integers per binade
 // tells where the sum crosses anything. Blocks take spans from the queue as long as there are any.
-// Bound: the latency of dependent instructions, branches and loads (warps issue in 46 % of the active cycles); 48 us for 58
-// rows of 151936 past the head, 14 for 48 rows of 50257 that sort nothing. In the row's own block the same passes took 100 us and more.
+// Bound: the latency of dependent instructions, branches and loads; 37 us for 58
+// rows of 151936 past the head (with every element added to all three tables, and every block's tables to the row's: 48), 14 for 48 rows of 50257 that sort nothing. In the row's own block the same passes took 100 us and more.
 // =============================================================================
 union __align__(16) WalkTileShared {
     float x[SPAN_THREADS * PITCH];
@@ -1777,6 +1796,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             if (tile >= R.ntile) continue;
             float *list = S->x + (size_t)warp * 32 * PITCH;
             __syncwarp();
+            const float est = R.tp[gt].est * yZ;
+            QuickSum qs(est);
             float4 nx = 4 * lane < n ? src[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
             for (int e0 = 4 * lane; e0 < n; e0 += 128) {
@@ -1787,15 +1808,25 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
                 for (int u = 0; u < 4; u++) {
                     p[u] = e0 + u < n ? prob_of(p[u], Z, yZ) : 0.0f;
                     list[skew(e0 + u)] = p[u];
+                    qs.add(p[u]);
                 }
                 src[e0 >> 2] = make_float4(p[0], p[1], p[2], p[3]);
             }
             __syncwarp();
+            if (qs.holds(est)) {
+                if (lane == 0) {
+                    unsigned int i0 = 0u;
+                    if (qs.k) { i0 = (unsigned int)atomicAdd(&head->nitem, 1); R.items(rr)[i0] = run_item(qs.k, qs.j, tile, n, 0, 0); }
+                    R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = qs.k ? 1 : 0;
+                }
+                __syncwarp();
+                continue;
+            }
             const TileChunk ch = tile_chunk(list, n);
             bool care;
             int my_place, c0 = CARE_PLACES;
             unsigned int i0 = 0;
-            const int ni = tile_items(list, ch, R.tp[gt].est * yZ, tile,
+            const int ni = tile_items(list, ch, est, tile,
                 [&](int k, int nc) -> Item * {
                     if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, k); if (nc) c0 = atomicAdd(&head->ncare, nc); }
                     i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
@@ -1912,7 +1943,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_pick_kernel(const __grid
 // =============================================================================
 // Kernel 7: the rows that were queued, one block each: the general forms of everything kernel 4 does, and
 // what it does not. Bound: latency of code that runs once and of one warp's dependent additions: 24 us where
-// nothing is sorted, 56 for walks past the head, 200 for a row with more careful chunks than kernel 4 takes.
+// nothing is sorted, 39 for 58 walks past the head, 200 for a row with more careful chunks than kernel 4 takes.
 // =============================================================================
 struct __align__(16) AuxF {
     union {
@@ -3404,7 +3435,8 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_exp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpanShared));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(row_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AuxF));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tile_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkTileShared));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_head_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(row_head_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HeadShared));
         if (e == cudaSuccess && dev < 64) ready[dev] = true;
     }
     RowsArgs A;
@@ -3429,7 +3461,7 @@ int molla_rows_launch(const BatchArgs &a, void *d_workspace, cudaStream_t st, ch
         e = launch(tile_stats_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
         if (e == cudaSuccess) e = launch(row_plan_kernel, (unsigned int)A.rows, NT, 0, st, A);
         if (e == cudaSuccess) e = launch(tile_exp_kernel, spans, SPAN_THREADS, sizeof(SpanShared), st, A);
-        if (e == cudaSuccess) e = launch(row_head_kernel, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
+        if (e == cudaSuccess) e = launch(A.rows > 3 * sms ? row_head_kernel<4> : row_head_kernel<3>, (unsigned int)A.rows, HT, sizeof(HeadShared), st, A);
         if (e == cudaSuccess) e = launch(tile_walk_kernel, spans < 4u * (unsigned int)sms ? spans : 4u * (unsigned int)sms, SPAN_THREADS, sizeof(WalkTileShared), st, A);
         if (e == cudaSuccess) e = launch(tile_pick_kernel, spans < 4u * (unsigned int)sms ? spans : 4u * (unsigned int)sms, SPAN_THREADS, 0, st, A);
         if (e == cudaSuccess) e = launch(row_tail_kernel, (unsigned int)(A.rows < sms ? A.rows : sms), NT, sizeof(AuxF), st, A);
