@@ -1092,7 +1092,9 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     };
     const bool fast = (pl.flags & F_FASTDIV) && tp.thr > -INFINITY;
     const float rT = __fdiv_rn(1.0f, c.T);
-    if (qs.usable && fast && !(pl.flags & F_LIST)) {
+    // (a tile that is expected to leave the binade has to be cut into chunks anyway: in short rows nearly every one)
+    const bool stays = fexpo((tile + 1 < A.ntile ? A.tp[gt + 1].est : tp.est) * (1.0f + 1.0f / 2048.0f)) == qs.j;
+    if (qs.usable && stays && fast && !(pl.flags & F_LIST)) {
         // Nobody asks for this row's list, only for its sum and its candidates, and nearly all that is kept adds
         // few units, whose number a hardware exponential tells unless it is near a half: see near_units. The others
         // are evaluated as they have to be. Per tile 600 instructions, where evaluating all that is kept takes 1300
