@@ -903,7 +903,9 @@ struct QuickSum {
         bad |= (fabsf(__fsub_rn(e, __fsub_rn(s, C))) == half) | (e >= big);
     }
     __device__ __forceinline__ bool holds(float est) {
-        if (!usable || __any_sync(0xffffffffu, bad)) return false;
+        // (2^23 units, the binade's, or more in a lane: it leaves the binade whatever the others add. Below that 32 lanes do not
+        // reach 2^32, which a tile of 1024 values of 2^22 units would: they are no ties and each is below `big`.)
+        if (!usable || __any_sync(0xffffffffu, bad || k >= (1u << 23))) return false;
         k = __reduce_add_sync(0xffffffffu, k);
         return fexpo((est + (float)k * fpow2(max(j - 23, -126))) * (1.0f + 1.0f / 2048.0f)) == j;
     }

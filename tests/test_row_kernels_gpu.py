@@ -177,3 +177,28 @@ def test_rows_around_what_is_resident_at_once(dev, lib, B):
         for key in ("tokens", "row_status"):
             assert np.array_equal(got[0][key], other[key]), key
         assert np.array_equal(got[0]["diag"][:, :3].view(np.uint32), other["diag"][:, :3].view(np.uint32))
+
+
+@pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("V", [3072, 9000])
+def test_a_tile_of_equal_values_below_a_quarter_of_the_sum(dev, lib, oracle, V):
+    """1024 exponentials 2^(j-1) (1 - 2^-24) while the sum is expected in [2^j, 2^(j+1)): each rounds to 2^22 units without a
+    tie, all of them together are 2^32. Rows that sort nothing add their probabilities in the same way: Z is 2048 in the even
+    ones, 1 / 2048 before the tile three times."""
+    B = 32
+    w = _kinds(W.config3(seed=V, B=B, V=V, H=4), B, V)
+    w["temperature"][:] = np.where(w["temperature"] > 0, np.float32(1.0), np.float32(0.0))
+    w["typical_p"][:] = 1.0
+    w["repeat_penalty"][:] = 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    x = np.full((B, V), -200.0, np.float32)
+    x[:, [3, 500, 1000]] = 0.0
+    x[:, 1024:2048] = -2.0 ** -24
+    x[::2, 2048:2048 + 1021] = 0.0
+    half = np.arange(B) % 4 == 3   # the same at half the size, below a maximum that comes last
+    x[np.ix_(half, [3, 500, 1000])] = -np.log(2.0)
+    x[half, 1024:2048] = np.float32(-0.69314724)
+    x[half, 3000] = 0.0
+    assert oracle.expf(x[1, 1024:1025])[0] == 1.0 - 2.0 ** -24 and oracle.expf(x[3, 1024:1025])[0] == 0.5 - 2.0 ** -25
+    w["logits"] = x
+    compare(w, dev, oracle, f"equal values, V={V}", max_exception_frac=1.0)
