@@ -231,6 +231,12 @@ __device__ __forceinline__ void block_excl_scan2(double a, double b, double *ws 
     ea = ba + (ia - a); eb = bb + (ib - b);
 }
 
+// ---- thread-block clusters ------------------------------------------------------
+// A block's shared memory may be touched by the others of its cluster once it has begun: every thread says that it has,
+// and waits for all of them before the first access. Orders no memory: with a release the one row of 128256 took 0.6 us more.
+__device__ __forceinline__ void cluster_begun() { asm volatile("barrier.cluster.arrive.relaxed.aligned;"); }
+__device__ __forceinline__ void cluster_all_begun() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 // ---- mbarrier + bulk copy (TMA without a tensor map, never multicast) ---------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);

@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(512, 2) lp_whole(const __grid_constant__ LpArg
     __shared__ double ts[LMAX_TILES], bs[LG_MOST];
     cg::cluster_group cl = cg::this_cluster();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    cluster_begun();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5, G = (int)cl.num_blocks(), rank = (int)cl.block_rank(), r = (int)blockIdx.x / G;
     const int per = (a.ntile + G - 1) / G, t0 = rank * per, n = max(0, min(per, a.ntile - t0));
@@ -284,6 +285,8 @@ __global__ void __launch_bounds__(512, 2) lp_whole(const __grid_constant__ LpArg
         tile_stat(x, m, s);
         if (lane == 0) { tm[t] = m; ts[t] = s; }
     }
+    __syncwarp();
+    cluster_all_begun();   // (blocks without tiles get here at once)
     __syncthreads();
     if (warp == 0) {
         float m = -INFINITY;

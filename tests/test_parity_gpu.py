@@ -634,7 +634,7 @@ def test_pick_rows_is_the_batched_decode_step(dev, lib, oracle):
         assert all(s.drawn == step + 1 for s in batch)
 
 
-@pytest.mark.parametrize("B,V", [(3, 4096), (2, 5121), (40, 8191), (3, 20000), (5, 65600), (20, 50257), (2, 262144), (1, 720896)])
+@pytest.mark.parametrize("B,V", [(3, 4096), (2, 5121), (40, 8191), (3, 20000), (40, 33900), (5, 65600), (20, 50257), (2, 262144), (1, 720896)])
 def test_whole_rows_logprobs_against_fp64(dev, lib, B, V):
     """Rows of every cluster size and both block sizes, on and off 16-byte boundaries, with logits of minus infinity."""
     rng = np.random.default_rng(V)
