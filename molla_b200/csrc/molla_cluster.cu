@@ -1142,6 +1142,7 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
         a.prof[(long long)r * 32 + 10] = (long long)gt; a.prof[(long long)r * 32 + 12] = blockIdx.x;
     }
 #endif
+    cluster_begun();
     // ---- 1. this block's range of the row, HBM -> shared memory
     const float *src = a.logits + lrow * a.row_stride + g.c0;
     const bool aligned = ((reinterpret_cast<uintptr_t>(src) & 15u) == 0);
@@ -1195,6 +1196,7 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     }
     if (MOLLA_KNOB(a, 16) && c.warp == 3) c.status |= MOLLA_ROW_LOAD_TIMEOUT;  // testing build: one warp reports a wait that ran out
     if (__syncthreads_or((c.status & MOLLA_ROW_LOAD_TIMEOUT) ? 1 : 0)) c.status |= MOLLA_ROW_LOAD_TIMEOUT;
+    cluster_all_begun();
     CSTAMP(1);
     if (a.softcap > 0.0f) {
         const float rcap = softcap_plain(a.softcap) ? __frcp_rn(a.softcap) : 0.0f;
