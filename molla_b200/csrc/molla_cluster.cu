@@ -125,6 +125,14 @@ struct CtxC {
     AuxC *A;
     unsigned int status;
 };
+// (What is called out of line makes its own: a reference to the kernel's would put that on the stack, and every loop with an
+// atomic in it would load the thread's number from there again. The walks past the head took a tenth longer so.)
+__device__ __forceinline__ CtxC ctx_of(AuxC *A) {
+    CtxC c;
+    c.tid = threadIdx.x; c.lane = c.tid & 31; c.warp = c.tid >> 5; c.status = 0;
+    c.A = A;
+    return c;
+}
 
 struct ClWalk {
     float s; long long pos; unsigned int tau;
@@ -258,9 +266,10 @@ __device__ __forceinline__ float add_place(const AuxC *A, int place, int pitch4,
 // these (ten or twenty: mostly the chunks in which the sum leaves a binade) are gone through one by one. (Every
 // instruction of that loop is one of a lone warp's, eight cycles or so: with the plain ones in it, it took 14 thousand.)
 // Returns false, and nothing else, where something does not hold.
-__device__ __noinline__ bool walk_fast(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, float &sum) {
-    AuxC *A = c.A;
+__device__ __noinline__ bool walk_fast(AuxC *A, ClGeo g, int Vc, int V, const unsigned int *bits, float &sum) {
     IN_SHARED(A);
+    cg::cluster_group cl = cg::this_cluster();
+    const CtxC c = ctx_of(A);
     const int lane = c.lane, pitch4 = care_pitch(g.L) / 4;
     const unsigned int lt = (1u << lane) - 1u;
     const int cnt = lane < g.G ? A->nrec[lane] : 0, incl = warp_incl_scan(cnt, lane), total = __shfl_sync(0xffffffffu, incl, 31);
@@ -345,9 +354,10 @@ __device__ __noinline__ bool walk_fast(cg::cluster_group &cl, CtxC &c, const ClG
 // The leader's first warp, all lanes alike, whatever was guessed: through the stretches from number i0 of block h0 on, the sum before them sb. With
 // `locate`, ends with the stretch behind which the sum exceeds `target`: its block, place and the sum before it.
 struct Walked { unsigned int sb; bool slow; int h, first, chunks; };
-__device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, int h0, int i0, unsigned int sb, bool locate, float target) {
-    AuxC *A = c.A;
+__device__ __noinline__ Walked walk_stretches(AuxC *A, ClGeo g, int Vc, int V, const unsigned int *bits, int h0, int i0, unsigned int sb, bool locate, float target) {
     IN_SHARED(A);
+    cg::cluster_group cl = cg::this_cluster();
+    const CtxC c = ctx_of(A);
     Walked w{sb, false, -1, 0, 0};
     const int pitch4 = care_pitch(g.L) / 4;
 #pragma unroll 1
@@ -390,9 +400,10 @@ __device__ __noinline__ Walked walk_stretches(cg::cluster_group &cl, CtxC &c, co
     return w;
 }
 
-__device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, long long *stamps = nullptr) {
-    AuxC *A = c.A;
+__device__ __noinline__ ClSum cluster_exact_sum(AuxC *A, ClGeo g, int Vc, int V, const unsigned int *bits, long long *stamps = nullptr) {
     IN_SHARED(A);
+    cg::cluster_group cl = cg::this_cluster();
+    const CtxC c = ctx_of(A);
     IN_SHARED(bits);
     AuxC *lead = cl.map_shared_rank(A, 0);
     ValBits vals{bits};
@@ -521,8 +532,8 @@ __device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, 
     if (g.rank == 0 && c.warp == 0) {
         Walked w{0u, false, -1, 0, 0};
         float sum;
-        if (walk_fast(cl, c, g, Vc, V, bits, sum)) w.sb = __float_as_uint(sum);
-        else w = walk_stretches(cl, c, g, Vc, V, bits, 0, 0, 0u, false, 0.0f);
+        if (walk_fast(A, g, Vc, V, bits, sum)) w.sb = __float_as_uint(sum);
+        else w = walk_stretches(A, g, Vc, V, bits, 0, 0, 0u, false, 0.0f);
         if (lane < g.G) { AuxC *ox = cl.map_shared_rank(A, lane); ox->ch_s = __uint_as_float(w.sb); ox->ch_slow = w.slow ? 1 : 0; }
     }
     cl.sync();
@@ -531,9 +542,10 @@ __device__ __noinline__ ClSum cluster_exact_sum(cg::cluster_group &cl, CtxC &c, 
 
 // The token at which the running sum of the last cluster_exact_sum (`total`) first exceeds `target`, or -1. Its
 // stretches and the values they stand for are where it left them.
-__device__ __noinline__ int cluster_locate(cg::cluster_group &cl, CtxC &c, const ClGeo &g, int Vc, int V, const unsigned int *bits, float total, float target) {
-    AuxC *A = c.A;
+__device__ __noinline__ int cluster_locate(AuxC *A, ClGeo g, int Vc, int V, const unsigned int *bits, float total, float target) {
     IN_SHARED(A);
+    cg::cluster_group cl = cg::this_cluster();
+    const CtxC c = ctx_of(A);
     IN_SHARED(bits);
     if (!(target < total)) return -1;   // (the same in every block)
     if (g.rank == 0 && c.warp == 0) {
@@ -548,7 +560,7 @@ __device__ __noinline__ int cluster_locate(cg::cluster_group &cl, CtxC &c, const
         } else {
             for (int k = 0; k < g.G; k++) if (!(target < A->first_s[k])) { h = k; s = A->first_s[k]; }
         }
-        const Walked w = walk_stretches(cl, c, g, Vc, V, bits, h, i, __float_as_uint(s), true, target);
+        const Walked w = walk_stretches(A, g, Vc, V, bits, h, i, __float_as_uint(s), true, target);
         if (c.lane < g.G) {
             AuxC *ox = cl.map_shared_rank(A, c.lane);
             ox->r_kind = w.h; ox->r_idx = w.first | (w.chunks << 16); ox->r_s = __uint_as_float(w.sb);
@@ -1051,12 +1063,10 @@ __device__ void descend_cluster(cg::cluster_group &cl, CtxC &c, const ClGeo &g, 
 __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     cg::cluster_group cl = cg::this_cluster();
-    CtxC c;
-    c.tid = threadIdx.x; c.lane = c.tid & 31; c.warp = c.tid >> 5; c.status = 0;
     float *rowbuf = reinterpret_cast<float *>(smem_raw);
     unsigned int *rowbits = reinterpret_cast<unsigned int *>(smem_raw);
     AuxC *A = reinterpret_cast<AuxC *>(smem_raw + (size_t)CL_CAPF * 4);
-    c.A = A;
+    CtxC c = ctx_of(A);
     IN_SHARED(A);
     IN_SHARED(rowbuf);
     IN_SHARED(rowbits);
@@ -1502,7 +1512,7 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     if (c.tid < g.G) cl.map_shared_rank(A, c.tid)->x3_n[g.rank] = A->ncand;
 
     // ---- 5. the softmax denominator, exactly as the sequential loop rounds it
-    const ClSum zs = cluster_exact_sum(cl, c, g, a.Vc, a.V, rowbits, CPROF_SLOTS(leader, 14));
+    const ClSum zs = cluster_exact_sum(A, g, a.Vc, a.V, rowbits, CPROF_SLOTS(leader, 14));
     const float Z = zs.s;
     if (zs.slow) c.status |= MOLLA_ROW_SLOW_PATH;
     dZ = Z;
@@ -1553,10 +1563,10 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
             if (pb < minp_pbits) pb = 0u;
             rowbits[i] = pb;
         }
-        const ClSum s1 = cluster_exact_sum(cl, c, g, a.Vc, a.V, rowbits);
+        const ClSum s1 = cluster_exact_sum(A, g, a.Vc, a.V, rowbits);
         const float sum = s1.s;
         const float target = __fmul_rn(u01, sum);
-        const int drawn = cluster_locate(cl, c, g, a.Vc, a.V, rowbits, sum, target);
+        const int drawn = cluster_locate(A, g, a.Vc, a.V, rowbits, sum, target);
         if (s1.slow) c.status |= MOLLA_ROW_SLOW_PATH;
         dsum = sum; dtarget = target;
         if (drawn >= 0) token = drawn;
