@@ -793,7 +793,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     if (__any_sync(0xffffffffu, two)) {
         if (usable) {
             float s0 = __uint_as_float(A1), s1 = __uint_as_float(A1 + 1u), t0 = __uint_as_float(A2), t1 = __uint_as_float(A2 + 1u);
-#pragma unroll 1
+#pragma unroll 2
             for (int i = 0; i < cnt; i++) {
                 const float v = list[skew(off + i)];
                 s0 = __fadd_rn(s0, v); s1 = __fadd_rn(s1, v);
@@ -884,20 +884,22 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
 
 // Most tiles lie inside one binade and hold no tie: their sum is a number of its units, in any order, added up where
 // the values are made. (Chunks and items for all tiles took half again as many instructions.) One warp; `est` = the
-// estimated sum before the tile.
+// estimated sum before the tile, `behind` = the one behind it, as far as it is known: a tile that is expected to leave the binade
+// has to be cut into chunks anyway, in short rows nearly every one.
 struct QuickSum {
     int j;               // the binade
     bool usable, bad;
     float C, half, big;
     unsigned int k;      // this lane's units; all lanes' once holds() has been true
-    __device__ __forceinline__ QuickSum(float est) {
+    __device__ __forceinline__ QuickSum(float est, float behind) {
         const float lo = est * (1.0f - 1.0f / 1024.0f);
         j = fexpo(lo);
-        usable = lo > 0.0f && j >= -100;
+        usable = lo > 0.0f && j >= -100 && fexpo(behind * (1.0f + 1.0f / 2048.0f)) == j;
         C = __fmul_rn(1.5f, fpow2(usable ? j : 0)); half = fpow2(usable ? j - 24 : -24); big = fpow2(usable ? j - 1 : -1);
         k = 0u; bad = false;
     }
     __device__ __forceinline__ void add(float e) {
+        if (!usable) return;
         const float s = __fadd_rn(e, C);
         k += __float_as_uint(s) - __float_as_uint(C);
         bad |= (fabsf(__fsub_rn(e, __fsub_rn(s, C))) == half) | (e >= big);
@@ -1075,7 +1077,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     float *list = S->x + (size_t)warp * 32 * PITCH;
     const unsigned int tau = min(pl.tau_bits, pl.tau_far);
     unsigned short *idx = reinterpret_cast<unsigned short *>(S->s.cnt) + warp * TILE;
-    QuickSum qs(tp.est);
+    QuickSum qs(tp.est, tile + 1 < A.ntile ? A.tp[gt + 1].est : tp.est);
     auto add_units = [&](float e) { qs.add(e); };
     int ni = 0, cnt = TILE;
     unsigned int i0 = 0u;
@@ -1094,9 +1096,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
     };
     const bool fast = (pl.flags & F_FASTDIV) && tp.thr > -INFINITY;
     const float rT = __fdiv_rn(1.0f, c.T);
-    // (a tile that is expected to leave the binade has to be cut into chunks anyway: in short rows nearly every one)
-    const bool stays = fexpo((tile + 1 < A.ntile ? A.tp[gt + 1].est : tp.est) * (1.0f + 1.0f / 2048.0f)) == qs.j;
-    if (qs.usable && stays && fast && !(pl.flags & F_LIST)) {
+    if (qs.usable && fast && !(pl.flags & F_LIST)) {
         // Nobody asks for this row's list, only for its sum and its candidates, and nearly all that is kept adds
         // few units, whose number a hardware exponential tells unless it is near a half: see near_units. The others
         // are evaluated as they have to be. Per tile 600 instructions, where evaluating all that is kept takes 1300
@@ -1801,7 +1801,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             float *list = S->x + (size_t)warp * 32 * PITCH;
             __syncwarp();
             const float est = R.tp[gt].est * yZ;
-            QuickSum qs(est);
+            QuickSum qs(est, (tile + 1 < R.ntile ? R.tp[gt + 1].est : R.tp[gt].est) * yZ);
             float4 nx = 4 * lane < n ? src[lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
             for (int e0 = 4 * lane; e0 < n; e0 += 128) {
