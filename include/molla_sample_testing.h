@@ -31,6 +31,14 @@ void molla_sample_debug_topk(void *d_ids, int32_t cap);
  * (counts[1]) since the last call of this function. */
 void molla_sample_debug_launches(int64_t *counts);
 
+/* The final-logit softcap as the row kernels evaluate it, four logits at a time, of n values at d_x into d_out
+ * (device memory, the legacy default stream). Returns when it is done. */
+void molla_sample_debug_softcap(const float *d_x, int64_t n, float cap, float *d_out);
+
+/* For how many floats e from 0 to 1 its quotient (1 - e) / (1 + e), by a reciprocal, is not the division's
+ * (-1: the kernel could not be run). */
+int64_t molla_sample_debug_softcap_quotients(void);
+
 #ifdef __cplusplus
 }
 #endif

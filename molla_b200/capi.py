@@ -40,7 +40,8 @@ EXPORTS = (
     "molla_sample_nccl_unique_id", "molla_sample_nccl_comm_create", "molla_sample_nccl_comm_destroy",
     "molla_sample_sharded_last_error", "molla_sample_sharded_workspace_bytes", "molla_sample_sharded_step",
 )
-TESTING_EXPORTS = ("molla_sample_debug_knobs", "molla_sample_debug_profile", "molla_sample_debug_topk", "molla_sample_debug_launches")
+TESTING_EXPORTS = ("molla_sample_debug_knobs", "molla_sample_debug_profile", "molla_sample_debug_topk", "molla_sample_debug_launches",
+                   "molla_sample_debug_softcap", "molla_sample_debug_softcap_quotients")
 TESTING_LIB_PATH = os.path.join(_HERE, "lib", "libmolla_sample_testing.so")
 
 
@@ -155,6 +156,10 @@ def _load(path, testing):
         L.molla_sample_debug_topk.argtypes = [vp, i32]
         L.molla_sample_debug_launches.restype = None
         L.molla_sample_debug_launches.argtypes = [C.POINTER(i64)]
+        L.molla_sample_debug_softcap.restype = None
+        L.molla_sample_debug_softcap.argtypes = [vp, i64, f32, vp]
+        L.molla_sample_debug_softcap_quotients.restype = i64
+        L.molla_sample_debug_softcap_quotients.argtypes = []
     return L
 
 

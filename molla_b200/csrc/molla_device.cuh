@@ -140,9 +140,10 @@ __device__ __forceinline__ float div_by(float x, float d, float y) {
 
 // Four of them at a time without branches, bit for bit the same, for a cap between 2^-40 and 2^40 (softcap_plain; rcap
 // = RN(1 / cap)). Past 1024 caps the exponential is zero whatever the logit is, and a quotient so small that a step
-// of div_by is no longer exact has an exponential of one: neither comes out differently. 1 + e lies in [1, 2] and its
+// of div_by is no longer exact has an exponential of one: neither comes out differently, but for the sign of the zero that a
+// subnormal logit gives, which no comparison and no exponential sees. 1 + e lies in [1, 2] and its
 // reciprocal, from the hardware's by one step of Newton, is close enough for div_by: compared with the division for all
-// e in [0, 1]. (16 rows of 262144 in clusters: 25 thousand cycles with two divisions, one logit after the other.)
+// e in [0, 1] (tests/test_decode_step_gpu.py). (16 rows of 262144 in clusters: 25 thousand cycles with two divisions, one logit after the other.)
 __device__ __forceinline__ bool softcap_plain(float cap) { return cap > 9.1e-13f && cap < 1.1e12f; }
 __device__ __forceinline__ float softcap_quotient(float e) {   // (1 - e) / (1 + e), e in [0, 1]
     const float d = __fadd_rn(1.0f, e);

@@ -1668,6 +1668,23 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[MOLLA_NOALLOC_S
 constexpr int NOALLOC_MAX_DEVICES = 64;
 void *g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};  // device address of the array, per device ordinal
 #ifdef MOLLA_SAMPLE_TESTING
+__global__ void softcap4_kernel(const float *x, long long n, float cap, float *out) {
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    float v[4];
+    for (int u = 0; u < 4; u++) v[u] = i + u < n ? x[i + u] : 0.0f;
+    softcap4(v, cap, softcap_plain(cap) ? __frcp_rn(cap) : 0.0f);
+    for (int u = 0; u < 4; u++)
+        if (i + u < n) out[i + u] = v[u];
+}
+__device__ unsigned long long g_quotients_off;
+__global__ void softcap_quotient_kernel() {
+    unsigned int off = 0u;
+    for (unsigned int b = blockIdx.x * blockDim.x + threadIdx.x; b <= 0x3f800000u; b += gridDim.x * blockDim.x) {
+        const float e = __uint_as_float(b), q = __fdiv_rn(__fsub_rn(1.0f, e), __fadd_rn(1.0f, e));
+        off += __float_as_uint(softcap_quotient(e)) != __float_as_uint(q) ? 1u : 0u;
+    }
+    if (off) atomicAdd(&g_quotients_off, (unsigned long long)off);
+}
 long long *g_prof = nullptr;
 int g_knobs = 0;
 int *g_topk = nullptr;
@@ -2491,6 +2508,18 @@ void molla_sample_debug_knobs(int32_t k) { g_knobs = k; }
 void molla_sample_debug_topk(void *d_ids, int32_t cap) { g_topk = (int *)d_ids; g_topk_cap = d_ids ? cap : 0; }
 void molla_sample_debug_launches(int64_t *counts) {
     for (int i = 0; i < 2; i++) { counts[i] = g_launched[i]; g_launched[i] = 0; }
+}
+void molla_sample_debug_softcap(const float *d_x, int64_t n, float cap, float *d_out) {
+    softcap4_kernel<<<(unsigned)((n + 1023) / 1024), 256>>>(d_x, n, cap, d_out);
+    cudaDeviceSynchronize();
+}
+int64_t molla_sample_debug_softcap_quotients(void) {
+    unsigned long long n = 0;
+    cudaError_t e = cudaMemcpyToSymbol(g_quotients_off, &n, sizeof(n));
+    softcap_quotient_kernel<<<4096, 256>>>();
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(&n, g_quotients_off, sizeof(n));
+    return e == cudaSuccess ? (int64_t)n : -1;
 }
 #endif
 

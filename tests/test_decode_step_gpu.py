@@ -98,6 +98,28 @@ def test_softcap_alone_is_bit_identical_to_the_oracle(dev, lib, oracle):
     assert np.all(np.abs(capped) <= 50.0)
 
 
+def test_softcap_quotients_are_the_divisions(dev, lib):
+    """(1 - e) / (1 + e) by a reciprocal, for every float e from 0 to 1."""
+    with capi.testing_library() as T:
+        assert T.molla_sample_debug_softcap_quotients() == 0
+
+
+@pytest.mark.parametrize("cap", [1e-38, 9.0e-13, 9.2e-13, 1e-3, 1.0, 30.0, 50.0, 1e5, 1.09e12, 1.2e12, 1e38])
+def test_softcap_four_at_a_time_is_the_oracles(dev, lib, oracle, cap):
+    """Over every exponent, subnormal and infinite logits included, and around the cap. (Zeros are equal whatever their
+    sign: a subnormal logit's depends on how x / cap is rounded, and nothing distinguishes them.)"""
+    cap = np.float32(cap)
+    rng = np.random.default_rng(1)
+    bits = np.concatenate([np.arange(0, 2 ** 31, 20011, dtype=np.uint32), np.arange(300, dtype=np.uint32), [0x7f800000, 0x7f7fffff, 0x7fc00000]]).astype(np.uint32)
+    x = np.concatenate([bits, bits | np.uint32(1 << 31)]).view(np.float32)
+    x = np.concatenate([x, (min(float(cap), 1e37) * rng.uniform(-12, 12, 100001)).astype(np.float32)])
+    at, out = torch.from_numpy(x).to(dev), torch.empty(x.size, device=dev)
+    with capi.testing_library() as T:
+        T.molla_sample_debug_softcap(at.data_ptr(), x.size, float(cap), out.data_ptr())
+    got, ref = out.cpu().numpy(), oracle.softcap(x, float(cap))
+    assert np.array_equal(got, ref, equal_nan=True)   # (of finite floats only the two zeros are equal without being the same)
+
+
 def test_bad_arguments_are_refused_before_any_launch(dev, lib):
     ds = S.DeviceSamplers(2, 100, ring_cap=8, device=dev)
     ds.assign(0, S.SamplerConfig(repeat_last_n=8))
