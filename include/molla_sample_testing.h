@@ -12,7 +12,8 @@ extern "C" {
 #endif
 
 /* Experiment switches of the row kernels. The ordinary entry points: bit 32 sends all rows through the tile
- * kernels, bit 64 all rows that fit a thread-block cluster (V <= 307200) through the cluster kernel. Streaming kernel: bit 1 no last-use hint on the second
+ * kernels, bit 64 all rows that fit a thread-block cluster (V <= 307200) through the cluster kernel. Whole rows' logprobs:
+ * bit 128 pretends that the device takes no clusters of sixteen. Streaming kernel: bit 1 no last-use hint on the second
  * pass over a row, bit 2 no keep hint on list traffic. All of them: bit 4 pretends, after the row has arrived, that one warp's bounded wait ran out
  * (nothing is withheld and nothing is left waiting): the row must come back with
  * MOLLA_ROW_LOAD_TIMEOUT, token -1 and its sampler state untouched. 0 = production behaviour. */

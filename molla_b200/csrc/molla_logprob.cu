@@ -329,16 +329,38 @@ __global__ void __launch_bounds__(512, 2) lp_whole(const __grid_constant__ LpArg
     }
 }
 
-cudaError_t lp_launch(void (*kernel)(LpArgs), unsigned int blocks, unsigned int threads, unsigned int cluster, cudaStream_t st, const LpArgs &a) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[2];
+void lp_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, unsigned int blocks, unsigned int threads, unsigned int cluster, cudaStream_t st) {
+    cfg = cudaLaunchConfig_t{};
     cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(threads); cfg.stream = st;
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
+}
+cudaError_t lp_launch(void (*kernel)(LpArgs), unsigned int blocks, unsigned int threads, unsigned int cluster, cudaStream_t st, const LpArgs &a) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    lp_config(cfg, at, blocks, threads, cluster, st);
     return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// Whether this device takes lp_whole's clusters of sixteen, which no device has to (asked once per device).
+bool wide_clusters(int dev) {
+    constexpr int DEVICES = 64;
+    static int known[DEVICES] = {};  // 0 unknown, -1 no
+    if (dev < 0 || dev >= DEVICES) return false;
+    if (known[dev] == 0) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[2];
+        lp_config(cfg, at, LG_MOST, 512, LG_MOST, nullptr);
+        int n = 0;
+        const bool ok = cudaFuncSetAttribute(lp_whole, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, lp_whole, &cfg) == cudaSuccess && n > 0;
+        if (!ok) (void)cudaGetLastError();
+        known[dev] = ok ? 1 : -1;
+    }
+    return known[dev] > 0;
 }
 
 int tiles_of(int V) {
@@ -355,7 +377,7 @@ size_t molla_logprob_workspace_bytes(int B, int V) { return (size_t)B * (size_t)
 
 cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int B, int V, const int *tokens, int top_n, float *chosen,
                                  int *top_ids, float *top_lps, const int *rows, int n_logit_rows, float softcap, void *workspace, bool early,
-                                 float *full_out, cudaStream_t st) {
+                                 float *full_out, bool wide, cudaStream_t st) {
     LpArgs a = {};
     a.logits = logits; a.row_stride = row_stride; a.B = B; a.V = V;
     a.tokens = tokens; a.top_n = top_n; a.chosen = chosen; a.top_ids = top_ids; a.top_lps = top_lps;
@@ -365,16 +387,12 @@ cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int 
         // a block for eight tiles, up to eight of them; twice as many for the widest rows and for few; as many warps as
         // share a block's tiles evenly in rounds of at most eight, of sixteen where there are not two blocks an SM
         int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { dev = -1; sms = 0; }
         int G = 1;
         while (G < 8 && 8 * G < a.ntile) G *= 2;
-        if (a.ntile > 24 * 8 || (a.ntile > 8 * 8 && (long long)B * G <= 2 * sms)) G = LG_MOST;
+        if ((a.ntile > 24 * 8 || (a.ntile > 8 * 8 && (long long)B * G <= 2 * sms)) && wide && wide_clusters(dev)) G = LG_MOST;
         const long long n = (long long)B * G;
         const int each = (a.ntile + G - 1) / G, most = n <= 2 * sms ? 16 : 8, rounds = (each + most - 1) / most;
-        if (G > 8) {
-            const cudaError_t e = cudaFuncSetAttribute(lp_whole, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return e;
-        }
         return lp_launch(lp_whole, (unsigned int)n, 32u * (unsigned int)((each + rounds - 1) / rounds), (unsigned int)G, st, a);
     }
     a.stats = (float *)workspace; a.early = early;

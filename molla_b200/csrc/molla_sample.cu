@@ -1800,7 +1800,7 @@ int launch_logprobs(const float *logits, int64_t row_stride, int B, int V, const
     cudaError_t e;
     if (molla_logprob_tiled(V, top_n)) {
         e = molla_logprob_launch(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, rows, n_logit_rows, softcap,
-                                 spare ? (void *)spare : d_workspace, spare != nullptr, nullptr, st);
+                                 spare ? (void *)spare : d_workspace, spare != nullptr, nullptr, false, st);
     } else {
         const int sms = sm_count();
         logprob_kernel<<<sms > 0 && B > sms ? sms : B, NT, 0, st>>>(logits, row_stride, B, V, tokens, top_n, chosen, top_ids, top_lps, nullptr,
@@ -2468,8 +2468,12 @@ int32_t molla_sample_logprobs(const float *d_logits, int64_t row_stride, int32_t
     if (!d_logits || !d_out || B < 0 || V <= 0 || row_stride < V) return fail(MOLLA_ERR_ARGUMENT, "bad arguments to logprobs%s");
     if (B == 0) return MOLLA_OK;
     if (molla_logprob_tiled(V, 0)) {
+        bool wide = true;
+#ifdef MOLLA_SAMPLE_TESTING
+        if (g_knobs & 128) wide = false;
+#endif
         const cudaError_t e = molla_logprob_launch(d_logits, row_stride, B, V, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, 0.0f,
-                                                   nullptr, false, d_out, (cudaStream_t)stream);
+                                                   nullptr, false, d_out, wide, (cudaStream_t)stream);
         return e == cudaSuccess ? MOLLA_OK : fail(MOLLA_ERR_CUDA, "logprob launch failed: %s", cudaGetErrorString(e));
     }
     const int sms = sm_count();

@@ -648,3 +648,17 @@ def test_whole_rows_logprobs_against_fp64(dev, lib, B, V):
         keep = ~torch.isneginf(ref)
         # the maximum and the logarithm's rounding, each half an ulp of numbers below 32
         assert (got.double() - ref)[keep].abs().max().item() <= 2 ** -18
+
+
+@pytest.mark.parametrize("B,V", [(3, 65600), (2, 262144), (1, 720896)])
+def test_whole_rows_logprobs_without_clusters_of_sixteen(dev, lib, B, V):
+    """A device that takes clusters of at most eight: the same rows, the sum of a row's tiles in another order."""
+    x = 3 * torch.randn(B, V, generator=torch.Generator(dev).manual_seed(V), device=dev)
+    with capi.testing_library() as T:
+        T.molla_sample_debug_knobs(128)
+        try:
+            got = S.logprobs_block(x)
+        finally:
+            T.molla_sample_debug_knobs(0)
+    # as above
+    assert (got.double() - torch.log_softmax(x.double(), 1)).abs().max().item() <= 2 ** -18
