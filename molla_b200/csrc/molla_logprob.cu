@@ -384,16 +384,23 @@ cudaError_t molla_logprob_launch(const float *logits, long long row_stride, int 
     a.rows = rows; a.n_logit_rows = n_logit_rows; a.softcap = softcap; a.out = full_out;
     a.ntile = tiles_of(V);
     if (full_out) {
-        // a block for eight tiles, up to eight of them; twice as many for the widest rows and for few; as many warps as
-        // share a block's tiles evenly in rounds of at most eight, of sixteen where there are not two blocks an SM
+        // A block for eight tiles, up to eight of them; sixteen for the widest rows and for few; as many warps as
+        // share a block's tiles evenly in rounds of at most eight, of sixteen where there are not two blocks an SM.
+        // Few rows: those whose blocks, at eight a row, are three an SM at most on the SMs that clusters of eight reach (8/9 of
+        // them). (At two an SM, 48 rows of 140000 had clusters of eight, 18 tiles a block in three rounds of six: 24.0 us, where
+        // sixteen of nine tiles in two rounds take 18.3; 38 of 128256 18.2 and 14.7, 40 of 196000 25.4 and 19.8.) Where they are
+        // four an SM a block has seven warps at least, so that no SM takes a fifth: 64 of 140000 24.4 and 22.0, of 90000 17.4 and 15.2.
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { dev = -1; sms = 0; }
         int G = 1;
         while (G < 8 && 8 * G < a.ntile) G *= 2;
-        if ((a.ntile > 24 * 8 || (a.ntile > 8 * 8 && (long long)B * G <= 2 * sms)) && wide && wide_clusters(dev)) G = LG_MOST;
+        const long long reached = (long long)sms * 8 / 9;
+        if ((a.ntile > 24 * 8 || (a.ntile > 8 * 8 && (long long)B * G <= 3 * reached)) && wide && wide_clusters(dev)) G = LG_MOST;
         const long long n = (long long)B * G;
         const int each = (a.ntile + G - 1) / G, most = n <= 2 * sms ? 16 : 8, rounds = (each + most - 1) / most;
-        return lp_launch(lp_whole, (unsigned int)n, 32u * (unsigned int)((each + rounds - 1) / rounds), (unsigned int)G, st, a);
+        int warps = (each + rounds - 1) / rounds;
+        if (n > 3 * reached && n <= 4 * reached && warps < 7) warps = each < 7 ? each : 7;
+        return lp_launch(lp_whole, (unsigned int)n, 32u * (unsigned int)warps, (unsigned int)G, st, a);
     }
     a.stats = (float *)workspace; a.early = early;
     const unsigned int blocks = (unsigned int)B * (unsigned int)((a.ntile + 7) / 8);
