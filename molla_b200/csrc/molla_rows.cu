@@ -1176,7 +1176,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;
 constexpr int H_ITEMS = 1024;              // items of a row
-constexpr int H_CARE = 64, H_REC = 512;    // careful chunks whose values are at hand, and all of them
+constexpr int H_CARE = 64, H_REC = 704;    // careful chunks whose values are at hand, and all of them (what four blocks an SM have room for)
 // What a queued row has: nothing; its denominator; its head too (tile_walk prepares the walk past it);
 // its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
 enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3, ST_DONE = 4 };
@@ -1186,9 +1186,12 @@ struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of al
 struct __align__(16) WalkShared {
     Item items[H_ITEMS];
     float care[H_CARE * 32];
-    CareRec rec[H_REC + 1];
+    union {
+        unsigned short toff[MAX_TILES + 4];   // the tiles' first items, until these are in order
+        CareRec rec[H_REC + 1];
+    };
     unsigned int sbs[H_REC + 2];           // the sum before every record's runs
-    unsigned short toff[MAX_TILES + 4], ritem[H_REC];
+    unsigned short ritem[H_REC];
     unsigned int ws[NWARP + 1], ws2[NWARP + 1];
 };
 
@@ -1211,6 +1214,7 @@ struct __align__(16) HeadShared {
     float Z; int ok, cut, n_ge; unsigned int tie;
     float ent;
 };
+static_assert(4 * (sizeof(HeadShared) + 1024) <= 228 * 1024, "four blocks an SM");
 
 // Everything about a row's items, in one round of loads by N threads (what lies past the counts is not used).
 template <int N>
@@ -2735,6 +2739,7 @@ __device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x
 __device__ __noinline__ bool tail_pure(CtxF &c) {
     const RowsArgs &R = *c.R;
     WalkShared *W = reinterpret_cast<WalkShared *>(c.A->tile);
+    static_assert(sizeof(WalkShared) <= sizeof(AuxF::tile), "the walk fits the tiles' space");
     AuxF *A = c.A;
     const RowHead *head = R.head(c.rr);
     WalkLoads<NT> wl;

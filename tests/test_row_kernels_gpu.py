@@ -202,3 +202,32 @@ def test_a_tile_of_equal_values_below_a_quarter_of_the_sum(dev, lib, oracle, V):
     assert oracle.expf(x[1, 1024:1025])[0] == 1.0 - 2.0 ** -24 and oracle.expf(x[3, 1024:1025])[0] == 0.5 - 2.0 ** -25
     w["logits"] = x
     compare(w, dev, oracle, f"equal values, V={V}", max_exception_frac=1.0)
+
+
+@pytest.mark.parametrize("tiles,head", [(190, True), (225, True), (240, False)])
+def test_rows_of_many_careful_chunks_end_in_row_head(dev, lib, oracle, tiles, head):
+    """Three values a tile, each in a chunk of its own, while the sum stays near a power of two: three careful chunks a tile,
+    of which row_head takes 704. Rows of more go through the last kernel's general form, to the same result."""
+    B, V = 8, 1024 * tiles
+    rng = np.random.default_rng(tiles)
+    w = W.config3(seed=tiles, B=B, V=V, H=4)
+    w["temperature"][:] = 1.0
+    w["top_k"][:], w["top_p"][:], w["min_p"][:], w["typical_p"][:] = 40, 0.9, 0.0, 1.0
+    w["repeat_penalty"][:] = 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    x = np.full((B, V), -200.0, np.float32)
+    at = (1024 * np.arange(tiles)[:, None] + [70, 500, 990]).ravel()
+    x[:, at] = rng.uniform(-15.9, -14.5, (B, at.size))   # the sum grows by 2e-4 in all
+    x[:, 0] = 0.0
+    x[:, 1] = np.log(1.0 - 1e-4 * rng.random(B))
+    w["logits"] = x
+    stamps = torch.zeros((B, 32), dtype=torch.int64, device=dev)
+    with capi.testing_library() as T:
+        T.molla_sample_debug_knobs(ROUTES["tiles"])
+        T.molla_sample_debug_profile(stamps.data_ptr())
+        try:
+            compare(w, dev, oracle, f"{tiles} tiles", max_exception_frac=0.3)
+        finally:
+            T.molla_sample_debug_knobs(0)
+            T.molla_sample_debug_profile(None)
+    assert stamps[:, 24].tolist() == [0 if head else 2] * B   # why a row was queued: not at all, or for its records
