@@ -231,3 +231,21 @@ def test_rows_of_many_careful_chunks_end_in_row_head(dev, lib, oracle, tiles, he
             T.molla_sample_debug_knobs(0)
             T.molla_sample_debug_profile(None)
     assert stamps[:, 24].tolist() == [0 if head else 2] * B   # why a row was queued: not at all, or for its records
+
+
+@pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("top", [-9e4, -2e3, 3e2, 4e3, 9e4])
+def test_denominators_of_rows_far_from_zero(dev, lib, oracle, top):
+    """Maxima over temperature of up to 1e5, temperatures from 0.05 to 20: what a tile adds to the sum is told by hardware
+    exponentials where their error, which grows with both, leaves no doubt. The denominator is the sequential one, bit for bit."""
+    B, V = 24, 60000
+    w = W.config3(seed=7, B=B, V=V, H=4)
+    w["temperature"][:] = np.geomspace(0.05, 20.0, B).astype(np.float32)
+    w["temperature"][::6] = 1.0
+    w["top_k"][:], w["top_p"][:], w["min_p"][:], w["typical_p"][:] = 40, 0.95, 0.0, 1.0
+    w["repeat_penalty"][:] = 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    T = w["temperature"][:, None]
+    x = np.where(np.arange(B)[:, None] % 2 == 0, w["logits"], w["logits"] * T)   # (spread by the temperature, or as it is)
+    w["logits"] = (x - x.max(1, keepdims=True) + np.float32(top) * T).astype(np.float32)
+    compare(w, dev, oracle, f"top={top}", max_exception_frac=1.0)
