@@ -1862,18 +1862,22 @@ bool molla_cluster_better(int V, int B, int call_B) {
     return cs.G != 0 && (long long)B * cs.G * 9 <= (long long)sms * 8 && clusters_resident(dev, cs.G) > 0;
 }
 
-// Whether the clusters of all B rows fit the device at the same time. Of those of eight blocks 15 or 16 do, depending
-// on which of its SMs a device has. Where it is 15, 16 rows of 262144 take two rounds of clusters (clusters / tiles, us): a
-// top-k of 40 95 / 66, a nucleus 182 / 132, nothing sorted 155 / 98, a top-k of 1024 152 / 78, greedy 25 / 25; mixed
-// with a softcap, of which the tile kernels do every logit twice, 114 / 127. Rows of 131072 and less stay where they are:
-// at 128256 mixed settings take 76 / 95 there, a nucleus 119 / 132, a top-k 83 / 54 and nothing sorted 118 / 83.
-constexpr int TWO_ROUNDS_V = 131072;
-bool molla_cluster_resident(int V, int B, int call_B) {
+// Whether the clusters of all B rows fit the device at the same time, where it matters. Of those of eight blocks 15 or 16
+// fit, depending on which of its SMs a device has. Where it is 15, 16 rows take two rounds of clusters: whatever the length, calls
+// whose rows are all alike are then better off in the tile kernels, while mixed settings, of which the row that starts
+// late is seldom the dearest, are not (clusters / tiles, us): 151936 logits, a top-k of 40 67 / 48, a nucleus 134 / 120, nothing
+// sorted 97 / 79, mixed 82 / 99; 235000 72 / 53, 156 / 129, 115 / 84, 96 / 108; 262144 76 / 53, 160 / 129, 122 / 83, 103 / 107;
+// 290000 77 / 58, 168 / 131, 122 / 85, 107 / 109. A row's time in a cluster grows with its length and the tile
+// kernels' hardly does, so from 240000 on mixed rows lose next to nothing. With a softcap, of which the tile kernels do
+// every logit twice, they do (262144: 117 / 124), and stay.
+constexpr int TWO_ROUNDS_V = 240000;
+bool molla_cluster_resident(int V, int B, int call_B, bool capped) {
+    if (capped || V <= TWO_ROUNDS_V) return true;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const ClusterShape cs = cluster_shape(V, call_B, sms);
-    return cs.G != 0 && (V <= TWO_ROUNDS_V || B <= clusters_resident(dev, cs.G));
+    return cs.G != 0 && B <= clusters_resident(dev, cs.G);
 }
 
 int molla_cluster_launch(const BatchArgs &args_in, cudaStream_t st, char *err, size_t errlen) {

@@ -9,8 +9,9 @@ struct BatchArgs;
 // Whether B rows of V logits, of a call of `call_B`, are better off there than in the tile kernels.
 bool molla_cluster_better(int V, int B, int call_B);
 
-// Whether the clusters of all B rows, of a call of `call_B`, are on the device at the same time.
-bool molla_cluster_resident(int V, int B, int call_B);
+// Whether the clusters of all B rows, of a call of `call_B`, are on the device at the same time, or need not be (`capped`: the
+// logits have a softcap).
+bool molla_cluster_resident(int V, int B, int call_B, bool capped);
 
 // Whether a row of V logits fits one thread block.
 bool molla_cluster_is_block(int V);

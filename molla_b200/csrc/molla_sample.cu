@@ -1777,7 +1777,7 @@ bool takes_clusters(const BatchArgs &a, bool piece, bool tiles) {
     const int call = a.layout_B > 0 ? a.layout_B : a.B;
     if (MOLLA_KNOB(a, 32)) return false;
     if (MOLLA_KNOB(a, 64)) return molla_cluster_better(a.V, 1, call);
-    if (tiles && !molla_cluster_resident(a.V, a.B, call)) return false;
+    if (tiles && !molla_cluster_resident(a.V, a.B, call, a.softcap > 0.0f)) return false;
     return molla_cluster_better(a.V, call, call) || (piece && molla_cluster_is_block(a.V) && molla_cluster_better(a.V, a.B, call));
 }
 

@@ -1,5 +1,7 @@
 """The row kernels at the sizes where they can go wrong, against the CPU oracle: as the library chooses
 between them, and all sizes through the tile kernels and through the cluster kernel."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -177,6 +179,20 @@ def test_rows_around_what_is_resident_at_once(dev, lib, B):
         for key in ("tokens", "row_status"):
             assert np.array_equal(got[0][key], other[key]), key
         assert np.array_equal(got[0]["diag"][:, :3].view(np.uint32), other["diag"][:, :3].view(np.uint32))
+
+
+@pytest.mark.parametrize("V,softcap", [(140000, 0.0), (240000, 0.0), (262144, 30.0)])
+def test_two_rounds_of_clusters_where_tiles_would_lose(dev, lib, V, softcap):
+    """16 rows, of which 15 or 16 are resident: in clusters either way up to 240000 logits, and with a softcap."""
+    ds = S.DeviceSamplers(16, V, ring_cap=1, device=dev)
+    for slot in range(16):
+        ds.assign(slot, S.SamplerConfig(temperature=1.0, top_k=40, repeat_last_n=0))
+    counts = (C.c_int64 * 2)()
+    with capi.testing_library() as T:
+        T.molla_sample_debug_launches(counts)
+        ds.step(torch.randn(16, V, device=dev), None, None, final_softcap=softcap)
+        T.molla_sample_debug_launches(counts)
+    assert list(counts) == [1, 0]
 
 
 @pytest.mark.usefixtures("route")
