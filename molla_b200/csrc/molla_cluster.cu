@@ -97,10 +97,9 @@ struct __align__(16) AuxC {
     unsigned long long wsu[NWARP + 1];
     float wsf[NWARP + 1];
     int wsi[NWARP + 1];
-    int nseg, ncand, evt_thread, specbin, hit_bin;
+    int ncand, evt_thread, specbin, hit_bin;
     unsigned long long hit_qbefore, hit_cbefore, tot_q, tot_c;
-    float walk_s; int walk_found, walk_idx, walk_slow;
-    float b_s; unsigned int b_tau; int b_event; int b_idx; float b_p; long long b_pos; int b_aux;
+    float b_s; int b_event; int b_idx; float b_p; long long b_pos; int b_aux;
     float b_sum; float b_target;
     uint64_t mbar;
     unsigned int thist[TBINS];           // the threads' maxima by distance below the block's maximum
@@ -1518,9 +1517,6 @@ __global__ void __launch_bounds__(NT, 1) sample_rows_cluster_kernel(const __grid
     dZ = Z;
 
     CSTAMP(6);
-    const unsigned int tau_p = __float_as_uint(__fdiv_rn(__uint_as_float(tau_bits), Z));
-    const unsigned int tau_pb = tau_p > 1u ? tau_p : 1u;
-    (void)tau_pb;
 
     // min-p (sample.mojo:508-523): see the note at the same place in sample_rows_kernel
     long long n_use = n_lim;
