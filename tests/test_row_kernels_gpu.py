@@ -265,3 +265,52 @@ def test_denominators_of_rows_far_from_zero(dev, lib, oracle, top):
     x = np.where(np.arange(B)[:, None] % 2 == 0, w["logits"], w["logits"] * T)   # (spread by the temperature, or as it is)
     w["logits"] = (x - x.max(1, keepdims=True) + np.float32(top) * T).astype(np.float32)
     compare(w, dev, oracle, f"top={top}", max_exception_frac=1.0)
+
+
+@pytest.mark.parametrize("chunks,V", [(1, 131072), (3, 131072), (7, 131072), (7, 30000)])
+def test_cluster_sums_of_many_careful_chunks(dev, lib, oracle, chunks, V):
+    """Every warp with some chunks, too few to be one stretch, whose sum may lie in either of two binades. Of 131072 logits in
+    eight blocks: 128 of them, which the leader strings together; 384, more than it has records for, and 896, more than 64
+    of a block, which it goes through one by one. The same for 30000 logits in eight blocks, with chunks of nine."""
+    B = 8
+    rng = np.random.default_rng(chunks)
+    w = _kinds(W.config3(seed=V, B=B, V=V, H=4), B, V)
+    w["temperature"][:] = np.where(w["temperature"] > 0, np.float32(1.0), np.float32(0.0))
+    w["typical_p"][:] = 1.0
+    w["repeat_penalty"][:] = 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    per = {131072: 33, 30000: 9}[V]   # logits a thread: a range of V / 8 over 512 threads, odd
+    x = np.full((B, V), -200.0, np.float32)
+    for block in range(0, V, V // 8):
+        for warp in range(block, min(block + V // 8, V), 32 * per):
+            at = warp + 3 + per * np.linspace(1, 30, chunks).astype(int)
+            at = at[at < min(block + V // 8, V)]
+            x[:, at] = rng.uniform(-15.9, -14.5, (B, at.size))   # the sum grows by 3e-4 at most
+    x[:, 0] = 0.0
+    x[:, 1] = np.log(1.0 - 1e-4 * rng.random(B))
+    w["logits"] = x
+    counts = (C.c_int64 * 2)()
+    with capi.testing_library() as T:
+        T.molla_sample_debug_launches(counts)
+        compare(w, dev, oracle, f"{chunks} chunks, V={V}", max_exception_frac=0.5)
+        T.molla_sample_debug_launches(counts)
+    assert counts[0] > 0 and counts[1] == 0
+
+
+def test_logprobs_of_a_block_too_large_to_run_beside_it(dev, lib):
+    """More than eight times the rows that are in flight together: the logprobs' own pass has no memory to spare beside the last
+    kernels and comes behind them. Tokens and logprobs are those of the rows sampled a few at a time."""
+    B, V = 1500, 720896
+    x = torch.randn(B, V, generator=torch.Generator(dev).manual_seed(5), device=dev) * 3
+    w = W.config3(seed=5, B=B, V=64, H=16)
+    def sample(rows):
+        part = {k: (w[k][rows] if k not in ("hist", "hist_off", "bias_ids", "bias_vals", "bias_off") else w[k]) for k in W.SAMPLER_KEYS}
+        n = len(part["temperature"])
+        part["hist"], part["hist_off"] = w["hist"][rows.start * 16:(rows.start + n) * 16], np.arange(n + 1, dtype=np.int32) * 16
+        part["bias_ids"], part["bias_vals"], part["bias_off"] = np.zeros(0, np.int64), np.zeros(0, np.float32), np.zeros(n + 1, np.int32)
+        return S.sample_batch(x[rows], S.upload_params(part, dev), top_n=5, want_logprob=True)
+    whole = sample(slice(0, B))
+    for a in (0, 160, 1440):
+        part = sample(slice(a, a + 60))
+        for k in ("tokens", "chosen_logprob", "top_ids", "top_logprobs"):
+            assert torch.equal(whole[k][a:a + 60], part[k]), (a, k)
