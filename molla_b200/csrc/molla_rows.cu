@@ -1304,7 +1304,9 @@ struct WalkLoads {
 // between two chunks (337 cycles a record when each asked for its own; two sets of registers spill).
 // Chunks whose sum may lie in either of two binades come in stretches wherever a row's sum stays near a
 // power of two for long, 188 in one row of 196: while the binade holds, 32 of them are one prefix sum over
-// the lanes (173 cycles each one after the other), out of line, because most rows have none.
+// the lanes (173 cycles each one after the other), out of line, because most rows have none. Only behind four in a row:
+// most come by twos and threes before a crossing, and the prefix sum, tried there, took nothing and 700 cycles (100 rows
+// of 50257 9.3 thousand cycles where they now take 7.7, the longest 18.8 and 14.6).
 __device__ __forceinline__ unsigned int kind_of(const CareRec &c) { return (c.meta >> 8) & 3u; }
 // From record q on: how many records one prefix sum takes, and the sum behind them.
 __device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsigned int sb, unsigned int kdone) {
@@ -1353,6 +1355,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
         for (int i = 0; i < 8; i++) x[i] = v[i];
     }
     bool fine = true;
+    int inside = 0;   // records in a row that needed no additions
 #pragma unroll 1
     for (int q = 0; ; q++) {
         const float4 *v = values(nx);   // the next record's
@@ -1370,11 +1373,12 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
         if (run && (!low || (td >> 23) != jb)) { fine = false; break; }
         if (run || (kind == K_DUAL && (low || e == jb + 1u) && (td >> 23) == e)) {
             sb = td;
-            if (q + 6 < nrec && kind_of(r) != K_STEP && kind_of(nx) != K_STEP && kind_of(W->rec[q + 6]) != K_STEP) {
+            if (++inside >= 4 && q + 6 < nrec && kind_of(r) != K_STEP && kind_of(nx) != K_STEP && kind_of(W->rec[q + 6]) != K_STEP) {
                 const uint2 t = dual_stretch(W, nrec, q + 1, sb, kdone);
                 sb = t.x;
                 q += (int)t.y;
                 kdone = t.y ? W->rec[q].k : kdone;
+                if (t.y < 8u) inside = 0;
                 r = W->rec[q + 1];
                 nx = W->rec[min(q + 2, nrec)];
                 v = values(r);
@@ -1383,6 +1387,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
             for (int i = 0; i < 8; i++) x[i] = v[i];
             continue;
         }
+        inside = 0;
         if (place >= H_CARE) {   // (a row with many: their values are still in L2)
             if (place == 255u) {   // (past CARE_PLACES, or several lanes' values: in its tile's list)
                 const Item it = W->items[W->ritem[q]];
