@@ -647,6 +647,67 @@ __device__ __forceinline__ void fetch_from_leader(CtxC &c, int n, F word) {
     __syncthreads();
 }
 
+// This block's elements below `tau` and from `lo` on into the tables of a walk whose sum lies in binade j: those that add a
+// number of units that does not depend on the sum, by bin; a rounding tie to the leader's list, the bin of any
+// other to specbin. With `count_all`, their number too. Out of line, with registers of its own: in line the loop's
+// share of the kernel's depended on what else was in it (120 rows of 32000 with a top-k of 1024 42 to 51 thousand cycles).
+// Every thread's elements four at a time. The common case (an element that simply adds its
+// mass to its bin) runs without a branch; elements that need care and rounding ties are rare
+// and a warp turns to them only when one of its lanes has met one.
+__device__ __noinline__ void walk_tables(AuxC *A, AuxC *lead, const unsigned int *bits, int nloc, int c0, unsigned int tau, unsigned int lo, int shift, int j,
+                                         bool binade_ok, bool count_all, bool ties_listed, int ntie_slot) {
+    IN_SHARED(A);
+    IN_SHARED(bits);
+    const float Cm = __fmul_rn(1.5f, fpow2(j)), halfu = fpow2(j - 24), bigthr = fpow2(j - 1);
+    const unsigned int cm_bits = __float_as_uint(Cm);
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int i0 = threadIdx.x - lane; i0 < nloc; i0 += 4 * NT) {  // (the same trips for all lanes of a warp)
+        const int i4 = i0 + lane;
+        unsigned int ebs[4];
+        bool rare = false;
+#pragma unroll
+        for (int u = 0; u < 4; u++) ebs[u] = (i4 + u * NT < nloc) ? bits[i4 + u * NT] : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const unsigned int eb = ebs[u];
+            const bool live = eb != 0u && eb < tau && eb >= lo;
+            const int bin = (int)((eb - lo) >> shift);
+            const float p = __uint_as_float(eb);
+            const float tq = __fadd_rn(p, Cm);
+            const float q = __fsub_rn(tq, Cm);
+            const float rr = __fsub_rn(p, q);
+            const bool special = (fabsf(rr) == halfu) || (p >= bigthr);
+            // q in units: below bigthr, p + Cm stays in Cm's binade, whose unit is the sum's, so
+            // the difference of the two bit patterns is the count (a conversion would issue at
+            // a quarter of the rate)
+            const unsigned int qu = __float_as_uint(tq) - cm_bits;
+            if (live && count_all) sred_add(&A->u.h.hc[bin], 1u);
+            const bool plain = live && binade_ok && !special;
+            if (plain) sred_add(&A->u.h.hq[bin], qu & MASS_LO_MASK);
+            if (plain && (qu >> MASS_SPLIT)) sred_add(&A->u.h.hqh[bin], qu >> MASS_SPLIT);
+            rare |= live && binade_ok && special;
+        }
+        if (__any_sync(0xffffffffu, rare)) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const unsigned int eb = ebs[u];
+                if (!(eb != 0u && eb < tau && eb >= lo)) continue;
+                const int bin = (int)((eb - lo) >> shift);
+                const float p = __uint_as_float(eb);
+                const float q = __fsub_rn(__fadd_rn(p, Cm), Cm);
+                const bool tie = fabsf(__fsub_rn(p, q)) == halfu;
+                if ((p >= bigthr) || (tie && !ties_listed)) { sred_max(&A->specbin, bin); continue; }
+                if (tie) {
+                    const int pos = atomicAdd(&lead->ntie[ntie_slot], 1);
+                    if (pos < TIE_CAP) { lead->tkey[pos] = make_key(eb, c0 + i4 + u * NT); lead->tbin[pos] = bin; }
+                }
+            }
+        }
+    }
+}
+
+
 // The descending walk past the sorted head (sample.mojo:492-506 and :580-590) over the cluster's
 // row of probabilities. State as in `descend`: exact running sum, elements consumed, and tau:
 // everything with probability bits >= tau is consumed. Every phase histograms what remains by
@@ -714,56 +775,8 @@ __device__ void descend_cluster(cg::cluster_group &cl, CtxC &c, const ClGeo &g, 
         const bool ties_listed = tie_mode && lvl == 1 && binade_ok;
         int ntie = rs.ntie;
         if (!reuse) {
-        // Every thread's elements four at a time. The common case (an element that simply adds its
-        // mass to its bin) runs without a branch; elements that need care and rounding ties are rare
-        // and a warp turns to them only when one of its lanes has met one.
         const int ntie_slot = phase & 1;
-        const unsigned int wtau = w.tau;
-        const int nloc = g.nloc;
-        const bool count_all = counting || !binade_ok;
-        for (int i0 = c.tid - c.lane; i0 < nloc; i0 += 4 * NT) {  // (the same trips for all lanes of a warp)
-            const int i4 = i0 + c.lane;
-            unsigned int ebs[4];
-            bool rare = false;
-#pragma unroll
-            for (int u = 0; u < 4; u++) ebs[u] = (i4 + u * NT < nloc) ? bits[i4 + u * NT] : 0u;
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const unsigned int eb = ebs[u];
-                const bool live = eb != 0u && eb < wtau && eb >= lo;
-                const int bin = (int)((eb - lo) >> shift);
-                const float p = __uint_as_float(eb);
-                const float tq = __fadd_rn(p, Cm);
-                const float q = __fsub_rn(tq, Cm);
-                const float rr = __fsub_rn(p, q);
-                const bool special = (fabsf(rr) == halfu) || (p >= bigthr);
-                // q in units: below bigthr, p + Cm stays in Cm's binade, whose unit is the sum's, so
-                // the difference of the two bit patterns is the count (a conversion would issue at
-                // a quarter of the rate)
-                const unsigned int qu = __float_as_uint(tq) - cm_bits;
-                if (live && count_all) sred_add(&A->u.h.hc[bin], 1u);
-                const bool plain = live && binade_ok && !special;
-                if (plain) sred_add(&A->u.h.hq[bin], qu & MASS_LO_MASK);
-                if (plain && (qu >> MASS_SPLIT)) sred_add(&A->u.h.hqh[bin], qu >> MASS_SPLIT);
-                rare |= live && binade_ok && special;
-            }
-            if (__any_sync(0xffffffffu, rare)) {
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const unsigned int eb = ebs[u];
-                    if (!(eb != 0u && eb < wtau && eb >= lo)) continue;
-                    const int bin = (int)((eb - lo) >> shift);
-                    const float p = __uint_as_float(eb);
-                    const float q = __fsub_rn(__fadd_rn(p, Cm), Cm);
-                    const bool tie = fabsf(__fsub_rn(p, q)) == halfu;
-                    if ((p >= bigthr) || (tie && !ties_listed)) { sred_max(&A->specbin, bin); continue; }
-                    if (tie) {
-                        const int pos = atomicAdd(&lead->ntie[ntie_slot], 1);
-                        if (pos < TIE_CAP) { lead->tkey[pos] = make_key(eb, g.c0 + i4 + u * NT); lead->tbin[pos] = bin; }
-                    }
-                }
-            }
-        }
+        walk_tables(A, lead, bits, g.nloc, g.c0, w.tau, lo, shift, j, binade_ok, counting || !binade_ok, ties_listed, ntie_slot);
         cl.sync();
         fetch_from_leader(c, 1, [&](int) { return (long long)lead->ntie[ntie_slot]; });
         ntie = ties_listed ? (int)A->rx[0] : 0;
