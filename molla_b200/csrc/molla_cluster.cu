@@ -1855,14 +1855,14 @@ int clusters_resident(int dev, int G) {
 bool molla_cluster_is_block(int V) { return V <= CL_CAPF; }
 
 // A row in the shared memory of its cluster is worked on in one launch, so as long as the clusters of all rows are
-// resident together the call is one row long: 32 rows of 8000 to 151936 logits take 11 to 16 us if greedy, 41 to 54
-// with a top-k of 40, 47 to 59 with mixed settings, 73 to 114 with a nucleus, 49 to 83 where nothing is sorted (the
-// tile kernels: 19 to 23, 48 to 64, 61 to 74, 58 to 134, 73 to 99). A second round of clusters doubles that and the
-// tile kernels pass it: 128 rows of 73000 with a top-k 74 against 94 us, nothing sorted 126 against 142; 256 rows of
-// 8000 with a top-k 57 against 70, a nucleus 73 against 122. Two kinds of batch the line cuts wrong, and as the
+// resident together the call is one row long: 32 rows of 8000 to 151936 logits take 6 to 8 us if greedy, 28 to 43
+// with a top-k of 40, 33 to 74 with mixed settings, 48 to 92 with a nucleus, 36 to 69 where nothing is sorted (the
+// tile kernels: 11 to 14, 36 to 51, 51 to 78, 45 to 110, 57 to 82; all in CUDA graphs). A second round of clusters doubles that and the
+// tile kernels pass it: 128 rows of 73000 with a top-k 59 against 76 us, nothing sorted 102 against 125; 256 rows of
+// 8000 with a top-k 44 against 52, a nucleus 58 against 90. Two kinds of batch the line cuts wrong, and as the
 // settings are on the device it cannot see them: up to 512 rows of 2500 to 20000 logits, each with its own settings
-// (256 of 8000: 107 us in tiles, 78 in clusters), and rows that all ask for a wide top-k (64 of 50257: 229 in clusters,
-// 78 in tiles).
+// (256 of 8000: 95 us in tiles, 64 in clusters), and rows that all ask for a wide top-k (64 of 50257: 192 in clusters,
+// 63 in tiles).
 bool molla_cluster_better(int V, int B, int call_B) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;

@@ -259,9 +259,9 @@ __global__ void __launch_bounds__(LT_) lp_rows(const __grid_constant__ LpArgs a)
 // A whole row's logprobs, one cluster: every block its tiles' maxima and sums, those of all blocks through distributed
 // shared memory, then the same tiles again, which are in L2 (the clusters in flight hold some 300 bytes per logit of
 // the vocabulary), and the result. Bound: the exponentials' instructions, then the store. One launch: with a kernel
-// for the tiles, one for the rows and one for the result, 64 rows of 128256 took 22.0 us, now 19.3 (floor 10), 512 of
-// 262144 285 and 221, 16 of 32000 12.5 and 8.1. Clusters of sixteen where those of eight leave SMs without a block, or a
-// block with more than three rounds of tiles: 7 rows of 700000 took 21.8 us in clusters of eight, 13.8 of sixteen.
+// for the tiles, one for the rows and one for the result, 64 rows of 128256 took 22.0 us, now 19.5 (floor 10), 512 of
+// 262144 285 and 221, 16 of 32000 12.5 and 8.1. Clusters of sixteen where rows are few or
+// widest (molla_logprob_launch): 7 rows of 700000 took 21.8 us in clusters of eight, 13.8 of sixteen.
 constexpr int LG_MOST = 16;
 __global__ void __launch_bounds__(512, 2) lp_whole(const __grid_constant__ LpArgs a) {
     namespace cg = cooperative_groups;

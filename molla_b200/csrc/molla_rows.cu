@@ -21,7 +21,7 @@
 // so any number of rows, from one to thousands, fills the chip, and only the row kernels have serial
 // parts. A row per thread-block cluster, resident in its shared memory, read the block once but left 33 to 16
 // rows in flight on the chip, each as slow as its serial parts: 1024 rows of 262144 took 6316 us where this
-// takes 705 to 750, 64 of 151936 with a nucleus and logprobs 300 where this takes 172. Seven launches cost 2 to 3 us each where
+// takes 690 to 700, 64 of 151936 with a nucleus and logprobs 300 where this takes 168 to 184. Seven launches cost 2 to 3 us each where
 // nothing else is to be done; they are chained so that a kernel's blocks are in place when the one before
 // ends. The reference's sequential fp32 sums are reproduced bit for bit: see "Items" below.
 #include <cuda_runtime.h>
@@ -1170,8 +1170,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
 // Kernel 4: one small block per sampled row. The items give the softmax denominator, the candidates the
 // sorted head; most rows end here. Rows that go on (nothing sorted, a nucleus past the head, typical-p,
 // anything unusual) are queued for the last kernel. Bound: the latency of one warp's dependent additions
-// and of one round of loads, so the block is small and four of them share an SM: 21 us for
-// 64 rows, 35 for 256, 42 for 512 with a top-k of 1024 (three an SM, two rounds of them: 60). (Run by the tail's 512 threads, one block an SM, the same
+// and of one round of loads, so the block is small and four of them share an SM: 20 us for
+// 64 rows, 34 for 256, 42 for 512 with a top-k of 1024 (three an SM, two rounds of them: 60). (Run by the tail's 512 threads, one block an SM, the same
 // rows took twice as long.)
 // =============================================================================
 constexpr int HT = 256, HW = HT / 32;

@@ -82,8 +82,8 @@ def test_decode_steps_match_host_kept_samplers(dev, lib, oracle, softcap):
 
 
 @pytest.mark.usefixtures("route")
-def test_softcap_alone_is_bit_identical_to_the_oracle(dev, lib, oracle):
-    """Penalised-value dump of a capped row = oracle softcap of the row (no penalties, no bias)."""
+def test_softcap_alone_gives_the_oracles_tokens_and_logprobs(dev, lib, oracle):
+    """Greedy tokens and their logprobs of capped rows (no penalties, no bias). The capped values bit for bit: below."""
     V = 5000
     rng = np.random.default_rng(3)
     block = (40.0 * rng.standard_normal((4, V))).astype(np.float32)
