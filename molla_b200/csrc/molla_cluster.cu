@@ -318,7 +318,7 @@ __device__ __noinline__ bool walk_fast(AuxC *A, ClGeo g, int Vc, int V, const un
         const FastRec r = nx;
         nx = out[min(q + 1, ncare)];
         const unsigned int to = sb + (r.k - kdone), jr = r.meta & 0xffu, e = to >> 23;
-        if (r.k != kdone && ((sb >> 23) != jr || e != jr)) return false;
+        if (jr != 0u && ((sb >> 23) != jr || e != jr)) return false;   // (also where the runs add nothing)
         kdone = r.k;
         sb = to;
         if (q == ncare) break;
@@ -434,6 +434,9 @@ __device__ __noinline__ ClSum cluster_exact_sum(AuxC *A, ClGeo g, int Vc, int V,
         db = chunk_units(vals, i0, i1, jb + 1u);
         over |= (((jb + 1u) << 23) + 1u + db.odd) >> 23 != jb + 1u;
     }
+    // A run that adds nothing is none, unless the sum may still be in the binade below (each of the additions before took 2^-24
+    // of it at most), where it might add something: then it is a stretch of no units, by which the binade is checked.
+    const unsigned int um = __ballot_sync(0xffffffffu, usable && (da.even | da.odd) == 0u && fexpo(lo * (1.0f - (float)(g.c0 + i1) * (1.0f / 16777216.0f))) < jl);
     const bool step = nonempty && (!usable || over);
     const unsigned int ne = __ballot_sync(0xffffffffu, nonempty), lt = (1u << lane) - 1u, below = ne & lt;
     const int prev = below ? 31 - __clz((int)below) : lane;
@@ -449,10 +452,11 @@ __device__ __noinline__ ClSum cluster_exact_sum(AuxC *A, ClGeo g, int Vc, int V,
     const unsigned int kp = pair_of(ra.even, ra.odd);
     unsigned int kr = __shfl_up_sync(0xffffffffu, kp, 1);
     if (lane == 0) kr = 0u;
-    // (a run that adds nothing is none: whatever its guess was, it would not count)
-    const unsigned int runm = __ballot_sync(0xffffffffu, care && kr != 0u);
+    auto behind = [&](int l) { return l < 0 ? 0xffffffffu : ~((2u << l) - 1u); };   // the lanes past l
+    const unsigned int runm = __ballot_sync(0xffffffffu, care && (kr != 0u || (um & lt & behind(lastc)) != 0u));
     const unsigned int ktail = last == 31 || merged ? 0u : __shfl_sync(0xffffffffu, kp, 31);
-    const int n = merged ? 1 : __popc(cm) + __popc(runm) + (ktail ? 1 : 0);
+    const bool tail = ktail != 0u || (!merged && (um & behind(last)) != 0u);
+    const int n = merged ? 1 : __popc(cm) + __popc(runm) + (tail ? 1 : 0);
     if (lane == 0) A->wsi[c.warp] = n | (__popc(cm) << 16);
     Units rb{0u, 0u};
     if (merged) rb = units_scan(db, lane, 0);
@@ -486,7 +490,7 @@ __device__ __noinline__ ClSum cluster_exact_sum(AuxC *A, ClGeo g, int Vc, int V,
                          (unsigned int)lane, 1u);
     }
     if (lane == 31 && merged) out[0] = stretch(kp, pair_of(rb.even, rb.odd), (unsigned int)(j0 + 127), true, j0, true, 255, 0u, 32u);
-    if (lane == 31 && ktail) out[n - 1] = stretch(ktail, 0u, (unsigned int)(tj + 127), false, tj, false, 255, (unsigned int)(last + 1), (unsigned int)(31 - last));
+    if (lane == 31 && tail) out[n - 1] = stretch(ktail, 0u, (unsigned int)(tj + 127), false, tj, false, 255, (unsigned int)(last + 1), (unsigned int)(31 - last));
     // the careful chunks' values to the leader, padded with zeros
     const int pitch = care_pitch(g.L);
     for (unsigned int left = __ballot_sync(0xffffffffu, place != 255); left; left &= left - 1u) {

@@ -415,7 +415,7 @@ __device__ void p1_walk(CX &c, V lst, int n, int L, bool locate, float target, W
             continue;
         }
         const bool dual = ((d >> 32) & 0xffu) != 0;
-        if (pa1 == pa0 && pb1 == pb0) continue;  // every term rounds to nothing in either binade
+        if (pa1 == pa0 && pb1 == pb0 && w.s > 0.0f && fexpo(w.s) >= j) continue;  // every term rounds to nothing in the binade expected, and so in those above
         bool ok = false;
         if (w.s > 0.0f) {
             const int js = fexpo(w.s);

@@ -766,6 +766,9 @@ __device__ __forceinline__ Item run_item(unsigned int pair, int j, int tile, int
     return it;
 }
 
+// The running sum is at least this part of the exact one: each of the additions before it took 2^-24 at most.
+__device__ __forceinline__ float least_of(int tile) { return 1.0f - (float)(tile + 1) * ((float)TILE / 16777216.0f); }
+
 // The items of a tile's list cut into chunks, `est` = the estimated sum before the tile. Returns the
 // number of items; `care` = this lane's values are wanted one by one.
 // `alloc(n, c)` is called by all lanes with the number of items and of careful chunks among them and
@@ -813,6 +816,9 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
         da = Units{__float_as_uint(s0) - A1, __float_as_uint(s1) - A1 - 1u};
         bad = __float_as_uint(s1) >= A2;
     }
+    // A run that adds nothing has no item, unless the sum may still be in the binade below, where it might add something:
+    // then it has one of no units, by which the binade is checked.
+    const unsigned int um = __ballot_sync(0xffffffffu, usable && (da.even | da.odd) == 0u && fexpo(lo * least_of(tile)) < jl);
     const bool step = nonempty && (!usable || bad);
     const unsigned int ne = __ballot_sync(0xffffffffu, nonempty);
     // lanes that round by themselves inside one binade form runs; two neighbours that disagree about
@@ -844,7 +850,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     }
     if (cm == 0u && !__any_sync(0xffffffffu, usable && da.even != da.odd)) {   // one run without a tie
         const unsigned int k = __reduce_add_sync(0xffffffffu, usable ? da.even : 0u);
-        if (k == 0u) return 0;
+        if (k == 0u && um == 0u) return 0;
         Item *out = alloc(1, 0);
         if (lane == 0) out[0] = run_item(k, j0, tile, total, 0, 0);
         return 1;
@@ -856,9 +862,11 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     const unsigned int kp = pair_of(k.even, k.odd);
     unsigned int kr = __shfl_up_sync(0xffffffffu, kp, 1);    // of the run that ends before this lane
     if (lane == 0) kr = 0u;
-    const unsigned int runm = __ballot_sync(0xffffffffu, care && kr != 0u);          // careful lanes with a run before them
+    auto behind = [&](int l) { return l < 0 ? 0xffffffffu : ~((2u << l) - 1u); };   // the lanes past l
+    const unsigned int runm = __ballot_sync(0xffffffffu, care && (kr != 0u || (um & lt & behind(lastc)) != 0u));          // careful lanes with a run before them
     const unsigned int ktail = last == 31 ? 0u : __shfl_sync(0xffffffffu, kp, 31);
-    const int ncare = __popc(cm), n = ncare + __popc(runm) + (ktail ? 1 : 0);
+    const bool tail = ktail != 0u || (um & behind(last)) != 0u;
+    const int ncare = __popc(cm), n = ncare + __popc(runm) + (tail ? 1 : 0);
     if (n == 0) return 0;
     Item *out = alloc(n, ncare);
     // the first lane of a run that holds anything, for its binade and its first entry
@@ -878,7 +886,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
         it.oc = (unsigned int)cnt | ((unsigned int)off << 11) | ((unsigned int)i << 21);
         out[i] = it;
     }
-    if (ktail && lane == 0) out[n - 1] = run_item(ktail, tj, tile, total - to, to, n - 1);
+    if (tail && lane == 0) out[n - 1] = run_item(ktail, tj, tile, total - to, to, n - 1);
     return n;
 }
 
@@ -911,6 +919,8 @@ struct QuickSum {
         k = __reduce_add_sync(0xffffffffu, k);
         return fexpo((est + (float)k * fpow2(max(j - 23, -126))) * (1.0f + 1.0f / 2048.0f)) == j;
     }
+    // Whether it has an item: see tile_items.
+    __device__ __forceinline__ bool counts(float est, int tile) const { return k != 0u || fexpo(est * (1.0f - 1.0f / 1024.0f) * least_of(tile)) != j; }
 };
 
 struct TileEval { int total; unsigned int keep; };
@@ -1088,8 +1098,8 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
         A.to(rr)[tile] = o;
     };
     auto store_run = [&]() {
-        ni = qs.k ? 1 : 0;
-        if (lane == 0 && qs.k) {
+        ni = qs.counts(tp.est, tile) ? 1 : 0;
+        if (lane == 0 && ni) {
             i0 = (unsigned int)atomicAdd(&head->nitem, 1);
             A.items(rr)[i0] = run_item(qs.k, qs.j, tile, cnt, 0, 0);
         }
@@ -1181,7 +1191,7 @@ constexpr int H_CARE = 64, H_REC = 704;    // careful chunks whose values are at
 // its denominator, and nothing to be sorted (tile_walk prepares the sum of the probabilities).
 enum { ST_NOTHING = 0, ST_SUM = 1, ST_HEAD = 2, ST_PURE = 3, ST_DONE = 4 };
 
-struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the last of them | kind | own binade | place
+struct __align__(16) CareRec { unsigned int k, meta, ka, kb; };   // units of all runs before it; binade of the one right before it, or 0 | kind | own binade | place
 
 struct __align__(16) WalkShared {
     Item items[H_ITEMS];
@@ -1266,7 +1276,7 @@ struct WalkLoads {
                 it[u] = W->items[i];
                 const bool run = it[u].kind() == K_RUN;
                 bool prev_run = false;
-                if (i > 0) { const Item p = W->items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = p.jb(); }
+                if (i > 0) { const Item p = W->items[i - 1]; prev_run = p.kind() == K_RUN; pj[u] = prev_run ? p.jb() : 0u; }
                 if (!run || !parity_free(it[u].ka) || (prev_run && pj[u] != it[u].jb())) { care |= 1u << u; n++; }   // (a change of binade between two runs: a wrong guess)
                 else k += it[u].ka;
             }
@@ -1288,7 +1298,7 @@ struct WalkLoads {
             }
             if (tid == 0) {
                 CareRec c;
-                c.k = ktot; c.ka = c.kb = 0u; c.meta = nitem > 0 ? W->items[nitem - 1].jb() : 0u;
+                c.k = ktot; c.ka = c.kb = 0u; c.meta = nitem > 0 && W->items[nitem - 1].kind() == K_RUN ? W->items[nitem - 1].jb() : 0u;
                 W->rec[nrec] = c;
             }
         }
@@ -1319,7 +1329,7 @@ __device__ __noinline__ uint2 dual_stretch(WalkShared *W, int nrec, int q, unsig
     if (lane == 0) kp = kdone;
     const unsigned int runs = c.k - kp, jb = (c.meta >> 16) & 0xffu, kind = kind_of(c), own = e == jb ? c.ka : c.kb;
     const bool can = q + lane < nrec && (kind == K_DUAL ? (e == jb || e == jb + 1u) : (kind == K_RUN && e == jb && (own & 0x3fffffffu) < (1u << 24))) &&
-                     (runs == 0u || ((c.meta & 0xffu) == e && runs < (1u << 24)));
+                     ((c.meta & 0xffu) == 0u || ((c.meta & 0xffu) == e && runs < (1u << 24)));
     Units d{0u, 0u};
     if (can) d = Units{runs + units(own, runs), runs + units(own, runs + 1u)};
     d = units_scan(d, lane, 0);
@@ -1364,7 +1374,7 @@ __device__ __forceinline__ bool walk_records(WalkShared *W, const float *more, c
         nx = W->rec[min(q + 2, nrec)];
         W->sbs[q] = sb;
         const unsigned int to = sb + (c.k - kdone), j = c.meta & 0xffu, kind = kind_of(c), jb = (c.meta >> 16) & 0xffu, place = c.meta >> 24;
-        if (c.k != kdone && ((sb >> 23) != j || (to >> 23) != j)) { fine = false; break; }
+        if (j != 0u && ((sb >> 23) != j || (to >> 23) != j)) { fine = false; break; }   // (also where the runs add nothing)
         kdone = c.k;
         sb = to;
         if (q == nrec) break;
@@ -1835,8 +1845,9 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             if (qs.holds(est)) {
                 if (lane == 0) {
                     unsigned int i0 = 0u;
-                    if (qs.k) { i0 = (unsigned int)atomicAdd(&head->nitem, 1); R.items(rr)[i0] = run_item(qs.k, qs.j, tile, n, 0, 0); }
-                    R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = qs.k ? 1 : 0;
+                    const bool item = qs.counts(est, tile);
+                    if (item) { i0 = (unsigned int)atomicAdd(&head->nitem, 1); R.items(rr)[i0] = run_item(qs.k, qs.j, tile, n, 0, 0); }
+                    R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = item ? 1 : 0;
                 }
                 __syncwarp();
                 continue;

@@ -58,6 +58,23 @@ class OracleSampler:
         return t
 
 
+def half_a_unit_tails(w):
+    """Rows whose sum comes to within 5e-8 V of two with its first two values, and then a tail around half of its last bit:
+    what is below adds nothing, what is above adds a whole one, so the running sum gets up to half a percent away from the
+    exact one, which is past two long before it."""
+    B, V = w["logits"].shape
+    rng = np.random.default_rng(V)
+    w["temperature"][:] = np.where(w["temperature"] > 0, np.float32(1.0), np.float32(0.0))
+    w["typical_p"][:] = 1.0
+    w["repeat_penalty"][:] = 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    x = (rng.uniform(-17.1, -16.6, (B, 1)) + rng.normal(0, 0.3, (B, V))).astype(np.float32)
+    x[:, 0] = 0.0
+    x[:, 1] = np.log(1.0 - 5e-8 * V * rng.random(B))
+    w["logits"] = x
+    return w
+
+
 def golden_case(g, name):
     cfg = g[f"{name}/cfg"]
     return dict(

@@ -7,7 +7,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from helpers import ROUTES, OracleSampler
+from helpers import ROUTES, OracleSampler, half_a_unit_tails
 from molla_b200 import capi, sampler as S, workloads as W
 from test_parity_gpu import compare, run_gpu
 
@@ -68,6 +68,12 @@ def test_sums_full_of_rounding_ties(dev, lib, oracle, V, low, high):
     w["logits"] = (-np.log(2.0) * k).astype(np.float32)
     compare(w, dev, oracle, f"ties, V={V}", max_exception_frac=1.0)
 
+
+@pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("V", [9000, 30000, 60000, 131072, 262144])
+def test_tails_of_half_a_unit(dev, lib, oracle, V):
+    """Values that add nothing in the binade their chunk expects may add something in the one the sum is still in."""
+    compare(half_a_unit_tails(_kinds(W.config3(seed=V, B=64, V=V, H=4), 64, V)), dev, oracle, f"half a unit, V={V}", max_exception_frac=0.5)
 
 @pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("V", [1000, 4097])

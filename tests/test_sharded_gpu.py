@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 import torch
 
+from helpers import half_a_unit_tails
 from molla_b200 import capi, sampler as S, sharded, workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -68,6 +69,12 @@ def test_heterogeneous_rows_four_shards(dev, lib, oracle):
 
 def test_small_vocabulary_two_shards(dev, lib, oracle):
     check(W.config3(seed=5, B=16, V=64, H=8), 2, dev, oracle)
+
+
+@pytest.mark.parametrize("V", [60000, 131072])
+def test_tails_of_half_a_unit_two_shards(dev, lib, oracle, V):
+    """Values that add nothing in the binade their chunk expects may add something in the one the sum is still in."""
+    check(half_a_unit_tails(W.config3(seed=V, B=64, V=V, H=4)), 2, dev, oracle)
 
 
 def test_list_overflow_is_reported(dev, lib):
