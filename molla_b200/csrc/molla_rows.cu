@@ -2407,11 +2407,12 @@ __device__ __noinline__ void descend_list(CtxF &c, FWalk &w, float x_ge, float x
         const unsigned int cm_bits = __float_as_uint(Cm);
         const bool ties_listed = tie_mode && lvl == 1 && binade_ok;
         const unsigned int wtau = w.tau;
-        // tile_walk's tables hold whole bins: they serve while what is consumed ends at a bin's edge
+        // tile_walk's tables hold whole bins: they serve while what is consumed ends at a bin's edge (not where the walk before has left
+        // its own, with its ties and what precedes each of them)
         const WalkTies *tt = nullptr;
         const unsigned long long *tab = nullptr;
         int bin_hi = NBINS;
-        if (c.tnb > 0 && ties_listed && !counting && j >= c.tj0 && j < c.tj0 + c.tnb && (wtau == 0xFFFFFFFFu || (wtau & ((1u << BIN_SHIFT) - 1u)) == 0u)) {
+        if (!reuse && c.tnb > 0 && ties_listed && !counting && j >= c.tj0 && j < c.tj0 + c.tnb && (wtau == 0xFFFFFFFFu || (wtau & ((1u << BIN_SHIFT) - 1u)) == 0u)) {
             tt = A->ties + (j - c.tj0);
             if (tt->n <= TIE_CAP) {
                 tab = (j == c.tj0 && c.first_table) ? reinterpret_cast<const unsigned long long *>(&A->u.h) : c.R->table(c.rr, j - c.tj0);

@@ -320,3 +320,20 @@ def test_logprobs_of_a_block_too_large_to_run_beside_it(dev, lib):
         part = sample(slice(a, a + 60))
         for k in ("tokens", "chosen_logprob", "top_ids", "top_logprobs"):
             assert torch.equal(whole[k][a:a + 60], part[k]), (a, k)
+
+
+@pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("seed", [905217, 905230, 12])
+def test_draws_from_sets_that_end_by_count_past_the_head(dev, lib, oracle, seed):
+    """Flat rows and a top-k of some thousands: the cut is found by counting, and the draw starts from what that walk has left,
+    rounding ties among it. (Two rows of the first two seeds' draws fall behind such a tie.)"""
+    rng = np.random.default_rng(seed)
+    B, V = 48, int(round(np.exp(rng.uniform(np.log(3000), np.log(60000)))))
+    w = W.config3(seed=3, B=B, V=64, H=4)
+    w["logits"] = (rng.uniform(0.5, 4) * rng.standard_normal((B, V))).astype(np.float32)
+    w["temperature"][:] = rng.choice(np.float32([1.0, 2.0, 4.0, 10.0]), B)
+    w["top_k"][:] = rng.choice([0, 1100, 2000, 3000, 5000], B)
+    w["top_p"][:] = rng.choice(np.float32([1.0, 0.9, 0.95, 0.5, 0.99]), B)
+    w["min_p"][:], w["typical_p"][:], w["repeat_penalty"][:] = 0.0, 1.0, 1.0
+    w["seed"][:] = rng.integers(0, 2 ** 63, B).astype(np.uint64)
+    compare(w, dev, oracle, f"counted, V={V}", max_exception_frac=0.3)
