@@ -766,15 +766,18 @@ __device__ __forceinline__ Item run_item(unsigned int pair, int j, int tile, int
     return it;
 }
 
-// The running sum is at least this part of the exact one: each of the additions before it took 2^-24 at most.
-__device__ __forceinline__ float least_of(int tile) { return 1.0f - (float)(tile + 1) * ((float)TILE / 16777216.0f); }
+// The running sum is at least this part of the estimated one: each of the additions before took 2^-24 at most, and the
+// estimate does not know that a logit over the temperature and the maximum over it are rounded, by 2^-24 of either.
+__device__ __forceinline__ float least_of(int tile, float top) {
+    return fmaxf(1.0f - (float)(tile + 1) * ((float)TILE / 16777216.0f) - fabsf(top) * (1.0f / 4194304.0f), 1.0e-6f);
+}
 
 // The items of a tile's list cut into chunks, `est` = the estimated sum before the tile. Returns the
 // number of items; `care` = this lane's values are wanted one by one.
 // `alloc(n, c)` is called by all lanes with the number of items and of careful chunks among them and
 // returns where the items go; place(i) says where the i-th careful chunk's values go (255: nowhere).
 template <class ALLOC, class PLACE>
-__device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch, float est, int tile, ALLOC alloc, PLACE place, bool &care, int &my_place) {
+__device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch, float est, int tile, float top, ALLOC alloc, PLACE place, bool &care, int &my_place) {
     const int cnt = ch.cnt, off = ch.off, total = ch.total;
     const float csum = ch.csum;
     const int lane = threadIdx.x & 31;
@@ -818,7 +821,7 @@ __device__ __forceinline__ int tile_items(const float *list, const TileChunk &ch
     }
     // A run that adds nothing has no item, unless the sum may still be in the binade below, where it might add something:
     // then it has one of no units, by which the binade is checked.
-    const unsigned int um = __ballot_sync(0xffffffffu, usable && (da.even | da.odd) == 0u && fexpo(lo * least_of(tile)) < jl);
+    const unsigned int um = __ballot_sync(0xffffffffu, usable && (da.even | da.odd) == 0u && fexpo(lo * least_of(tile, top)) < jl);
     const bool step = nonempty && (!usable || bad);
     const unsigned int ne = __ballot_sync(0xffffffffu, nonempty);
     // lanes that round by themselves inside one binade form runs; two neighbours that disagree about
@@ -920,7 +923,7 @@ struct QuickSum {
         return fexpo((est + (float)k * fpow2(max(j - 23, -126))) * (1.0f + 1.0f / 2048.0f)) == j;
     }
     // Whether it has an item: see tile_items.
-    __device__ __forceinline__ bool counts(float est, int tile) const { return k != 0u || fexpo(est * (1.0f - 1.0f / 1024.0f) * least_of(tile)) != j; }
+    __device__ __forceinline__ bool counts(float est, int tile, float top) const { return k != 0u || fexpo(est * (1.0f - 1.0f / 1024.0f) * least_of(tile, top)) != j; }
 };
 
 struct TileEval { int total; unsigned int keep; };
@@ -1098,7 +1101,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
         A.to(rr)[tile] = o;
     };
     auto store_run = [&]() {
-        ni = qs.counts(tp.est, tile) ? 1 : 0;
+        ni = qs.counts(tp.est, tile, pl.top) ? 1 : 0;
         if (lane == 0 && ni) {
             i0 = (unsigned int)atomicAdd(&head->nitem, 1);
             A.items(rr)[i0] = run_item(qs.k, qs.j, tile, cnt, 0, 0);
@@ -1159,7 +1162,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_exp_kernel(const __grid_
         const TileChunk ch = tile_chunk(list, t.total);
         bool care;
         int my_place, c0 = CARE_PLACES;
-        ni = tile_items(list, ch, tp.est, tile,
+        ni = tile_items(list, ch, tp.est, tile, pl.top,
             [&](int n, int nc) -> Item * {
                 if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, n); if (nc) c0 = atomicAdd(&head->ncare, nc); }
                 i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
@@ -1845,7 +1848,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             if (qs.holds(est)) {
                 if (lane == 0) {
                     unsigned int i0 = 0u;
-                    const bool item = qs.counts(est, tile);
+                    const bool item = qs.counts(est, tile, head->plan.top);
                     if (item) { i0 = (unsigned int)atomicAdd(&head->nitem, 1); R.items(rr)[i0] = run_item(qs.k, qs.j, tile, n, 0, 0); }
                     R.to(rr)[tile].ioff = i0; R.to(rr)[tile].nitem = item ? 1 : 0;
                 }
@@ -1856,7 +1859,7 @@ __global__ void __launch_bounds__(SPAN_THREADS, 4) tile_walk_kernel(const __grid
             bool care;
             int my_place, c0 = CARE_PLACES;
             unsigned int i0 = 0;
-            const int ni = tile_items(list, ch, est, tile,
+            const int ni = tile_items(list, ch, est, tile, head->plan.top,
                 [&](int k, int nc) -> Item * {
                     if (lane == 0) { i0 = (unsigned int)atomicAdd(&head->nitem, k); if (nc) c0 = atomicAdd(&head->ncare, nc); }
                     i0 = __shfl_sync(0xffffffffu, i0, 0); c0 = __shfl_sync(0xffffffffu, c0, 0);
@@ -3037,7 +3040,7 @@ __device__ void tail_row(const RowsArgs &R, int rr) {
             const TileChunk ch = tile_chunk(list, n);
             bool care;
             int my_place;
-            const int ni = tile_items(list, ch, A->tsum[t], t, [&](int, int) { return c.gitems + (size_t)t * ITEMS_PER_TILE; }, [](int) { return 255; }, care, my_place);
+            const int ni = tile_items(list, ch, A->tsum[t], t, c.pl.top, [&](int, int) { return c.gitems + (size_t)t * ITEMS_PER_TILE; }, [](int) { return 255; }, care, my_place);
             if (c.lane == 0) { A->tni[t] = (unsigned short)ni; A->tio[t] = (unsigned int)(t * ITEMS_PER_TILE); }
             __syncwarp();
         }

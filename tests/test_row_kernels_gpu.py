@@ -76,6 +76,35 @@ def test_tails_of_half_a_unit(dev, lib, oracle, V):
     compare(half_a_unit_tails(_kinds(W.config3(seed=V, B=64, V=V, H=4), 64, V)), dev, oracle, f"half a unit, V={V}", max_exception_frac=0.5)
 
 @pytest.mark.usefixtures("route")
+@pytest.mark.parametrize("first", [-30000.0, -9000.0, 25000.0])
+def test_sums_of_rows_whose_scaled_logits_round_coarsely(dev, lib, oracle, first):
+    """A logit over a temperature of 0.05 is rounded to a sixteenth or so here, its exponential with it. First some values whose
+    exponentials are past two in all before that rounding and below two after it, then a tail that adds a unit each below two
+    and nothing above."""
+    B, V, T, x0 = 16, 6000, np.float32(0.05), np.float32(first)
+    rng = np.random.default_rng(int(abs(first)))
+    v = (x0 - np.arange(1, 800, dtype=np.float32) * np.spacing(np.float32(abs(first)))).astype(np.float32)
+    real = np.exp((v.astype(np.float64) - x0) / float(T))
+    got = np.exp((v / T).astype(np.float32).astype(np.float64) - np.float32(x0 / T))
+    low = np.argsort(got / real)[:200]
+    low = low[real[low] > 0.003]
+    w = _kinds(W.config3(seed=1, B=B, V=V, H=4), B, V)
+    w["temperature"][:] = T
+    w["typical_p"][:], w["repeat_penalty"][:], w["top_p"][:] = 1.0, 1.0, 1.0
+    w["frequency_penalty"][:] = w["presence_penalty"][:] = 0.0
+    x = np.full((B, V), x0 - 200.0, np.float32)
+    x[:, 0] = x0
+    for r in range(B):
+        while True:
+            some = rng.choice(low, rng.integers(3, 9), replace=False)
+            if real[some].sum() > 1 + 2 ** -8.5 and got[some].sum() < 1 - 2 ** -11:
+                break
+        x[r, 1:1 + len(some)] = v[some]
+    x[:, 1024:4000] = x0 - np.float32(16.3 * 0.05)
+    w["logits"] = x
+    compare(w, dev, oracle, f"coarse, first={first}", max_exception_frac=1.0)
+
+@pytest.mark.usefixtures("route")
 @pytest.mark.parametrize("V", [1000, 4097])
 def test_pick_rows_in_place(dev, lib, oracle, V):
     """Samplers on the host, logit rows in any order and twice, a block with a stride, biases and windows."""
